@@ -1,0 +1,452 @@
+// ggml_axpy for 2..32 tokens on the tensor cores (ggml.c:14314-14618 is the CPU path it matches), and the coefficients it reads.
+//
+// dst[t, c] = sum over listed rows r of coef[t, r] * Wt[r, c].  As a matrix product C[c, t] += A[c, r] * B[r, t]: A = the rows
+// of down_t read transposed, B = the coefficients, laid out by list position so that they load like a matrix.
+//   FP16 rows: coef = FP16(h) of a token's active rows, else 0; the products of two halves are exact, sums are FP32, as on
+//              the CPU.
+//   Q4_0 rows, columns a multiple of 1024: weight FP16(d * (q - 8)) (one rounding: q - 8 is exact), coef = FP16(b8 * d8) of the
+//              CPU path's int8 x scale pair: two roundings to 11 bits that the CPU path does not have, relative error <= 5e-4
+//              per term.
+//   Q4_0 rows, other widths: exact.  A = q - 8 (an integer, exact in BF16), B = b8 * d8 * d of a column block as the sum of
+//              three BF16 numbers (24 bits, FP32's exponent range): three mma for one, so three times the tensor time.
+// The nibbles become fragments in registers: a lane takes the same 4-byte word of two neighbouring rows, and one byte permute
+// and one logic operation make the pair {1024 + q of row r, 1024 + q of row r + 1} of a column, in the fragment's k order.
+// (Expanding a stage into an FP16 tile in shared memory first costs two barriers per 16 rows: 159 us where this takes 82,
+// 103 MB of rows, 32 tokens.)
+//
+// Work split: units of 256 columns x 64 (128) list rows, numbered slice by slice; every CTA takes an equal contiguous range,
+// so the chip is full whatever the number of columns.  The CTAs that meet in a column slice each write one partial vector
+// ("piece"); at most n_pieces of them per slice, the missing ones are written as zeros, and the norm (or the reduction)
+// that follows adds the pieces in order.  Rows arrive by 16-byte cp.async from all threads (they lie anywhere).
+#include "pi_common.cuh"
+
+namespace pi {
+
+static constexpr int AX_THREADS = 512, AX_CW = 256;      // 16 warps; columns of a unit
+static constexpr int AX_RED_PITCH = AX_CW + 4;           // conflict-free fragment stores
+static constexpr size_t AX_SMEM_MAX = 226 * 1024;
+static constexpr int AX_ROW_RING = 16;                   // stages whose row numbers are kept
+
+struct AxpyMmP {
+    const uint8_t * Wt; int64_t row_bytes; int nrows, ncols, nb, T, T_all;
+    const int32_t * list; const int32_t * count;
+    const void * coef; int64_t coef_stride;                           // FP16, or F32 in the exact mode
+    float * partial; int n_cs, n_pieces;
+};
+
+__device__ __forceinline__ void ax_cp16(uint32_t dst, const void * src, unsigned bytes) {       // the first `bytes` bytes, the rest zeros
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void ax_ldsm4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ax_ldsm4_trans(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ax_ldsm2(uint32_t & r0, uint32_t & r1, uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
+}
+__device__ __forceinline__ void ax_hmma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ax_bmma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t ax_bf2(float lo, float hi) { uint32_t r; asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo)); return r; }
+__device__ __forceinline__ uint32_t ax_badd2(uint32_t a, uint32_t b) { uint32_t r; asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
+// {x, y} as the sum of three pairs of BF16 numbers (each difference is exact in FP32)
+__device__ __forceinline__ void ax_split3(float x, float y, uint32_t (&b)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        b[i] = ax_bf2(x, y);
+        x -= __uint_as_float(b[i] << 16);
+        y -= __uint_as_float(b[i] & 0xFFFF0000u);
+    }
+}
+__device__ __forceinline__ uint32_t ax_mul2(uint32_t a, uint32_t b) { uint32_t r; asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
+__device__ __forceinline__ uint32_t ax_add2(uint32_t a, uint32_t b) { uint32_t r; asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
+__device__ __forceinline__ uint32_t ax_fma2(uint32_t a, uint32_t b, uint32_t c) { uint32_t r; asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c)); return r; }
+
+enum { AX_F16 = 0, AX_Q4 = 1, AX_Q4_EXACT = 2 };
+
+template <int MODE, int NT>
+struct AxShape {
+    static constexpr bool Q4 = MODE != AX_F16, EXACT = MODE == AX_Q4_EXACT;
+    static constexpr int TP = NT * 8;
+    static constexpr int RS = MODE == AX_Q4 ? 128 : 64;               // list rows of a stage
+    static constexpr int W_PITCH = Q4 ? 144 : AX_CW * 2 + 16;         // odd multiples of 16 bytes
+    static constexpr int CB = EXACT ? 4 : 2;                          // bytes of a coefficient
+    static constexpr int C_PITCH = RS * CB + (EXACT ? 32 : 16);
+    static constexpr int C_OFF = RS * W_PITCH;
+    static constexpr int STAGE = (C_OFF + TP * C_PITCH + 127) / 128 * 128;
+    static constexpr int RED = TP * AX_RED_PITCH * 4;
+    static constexpr int HEAD = (RED + AX_ROW_RING * RS * 4 + 127) / 128 * 128;
+    static constexpr int FIT = (int)((AX_SMEM_MAX - HEAD) / STAGE);
+    static constexpr int S = FIT > 8 ? 8 : FIT;
+    static constexpr int KPW = RS / 64;                               // 16-row steps of a warp per stage (4 warps share the rows)
+    static_assert(S >= 3 && S + 2 <= AX_ROW_RING, "ring");
+};
+
+template <int MODE, int NT>
+__global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
+    using Z = AxShape<MODE, NT>;
+    constexpr bool Q4 = Z::Q4, EXACT = Z::EXACT;
+    constexpr int TP = Z::TP, RS = Z::RS, S = Z::S, KPW = Z::KPW;
+    extern __shared__ __align__(128) unsigned char smem[];
+    float * red = reinterpret_cast<float *>(smem);                    // [TP][AX_RED_PITCH]
+    int * rows = reinterpret_cast<int *>(smem + Z::RED);              // [AX_ROW_RING][RS] row numbers of the stages ahead
+    const uint32_t ring_a = smem_u32(smem + Z::HEAD);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wc = warp & 3, wk = warp >> 2;                          // 64 columns, a quarter of the stage's rows
+    const int cta = blockIdx.x;
+
+    pdl_launch();
+    pdl_wait();
+    const int n = min(*p.count, p.nrows);
+    const int nst = (n + RS - 1) / RS;
+    const unsigned total = (unsigned)p.n_cs * (unsigned)nst;
+    if (total == 0) {                                                 // no active row: the result is zero
+        for (int cs = cta; cs < p.n_cs; cs += gridDim.x)
+            for (int e = tid; e < p.n_pieces * p.T * AX_CW; e += AX_THREADS) {
+                const int c = cs * AX_CW + e % AX_CW, t = e / AX_CW % p.T, k = e / AX_CW / p.T;
+                if (c < p.ncols) p.partial[((size_t)k * p.T_all + t) * p.ncols + c] = 0.f;
+            }
+        return;
+    }
+    const unsigned G = min((unsigned)gridDim.x, total);               // every CTA that takes part has a unit
+    if ((unsigned)cta >= G) return;
+    const int u0 = (int)((unsigned long long)total * (unsigned)cta / G), n_units = (int)((unsigned long long)total * (unsigned)(cta + 1) / G) - u0;
+
+    auto row_at = [&](int u, int r) {                                 // row number of list entry r of unit u's stage
+        const int li = (u % nst) * RS + r;
+        const int v = u < u0 + n_units && li < n ? p.list[li] : 0;
+        return (unsigned)v < (unsigned)p.nrows ? v : 0;
+    };
+    for (int e = tid; e < (S + 1) * RS; e += AX_THREADS) rows[e] = row_at(u0 + e / RS, e % RS);
+    __syncthreads();
+    auto issue = [&](int i) {                                         // unit u0 + i
+        const int u = u0 + i, cs = u / nst, st = u % nst;
+        const uint32_t base = ring_a + (uint32_t)(i % S) * Z::STAGE;
+        const int * rw = rows + (i % AX_ROW_RING) * RS;
+        if (!Q4) {
+            const int col = cs * AX_CW + lane * 8;
+#pragma unroll
+            for (int j = 0; j < RS / 16; j++) {
+                const int r = warp + j * 16;
+                const bool ok = st * RS + r < n && col < p.ncols;
+                ax_cp16(base + r * Z::W_PITCH + lane * 16, ok ? p.Wt + (size_t)rw[r] * p.row_bytes + (size_t)col * 2 : p.Wt, ok ? 16u : 0u);
+            }
+        } else {
+            constexpr int CT = 8 * RS / AX_THREADS;                   // pieces of a row slice per thread
+            const int r = tid / (8 / CT), qd = tid % (8 / CT);
+            const bool ok = st * RS + r < n;
+            const uint8_t * row = p.Wt + (size_t)rw[r] * p.row_bytes;
+#pragma unroll
+            for (int j = 0; j < CT; j++) ax_cp16(base + r * Z::W_PITCH + (qd * CT + j) * 16, row + (size_t)cs * 128 + (qd * CT + j) * 16, ok ? 16u : 0u);
+            if (qd == 0) ax_cp16(base + r * Z::W_PITCH + 128, row + (size_t)p.nb * 16 + (size_t)cs * 16, ok ? 16u : 0u);
+        }
+        constexpr int CPP = 16 / Z::CB;                               // coefficients of a 16-byte piece; positions past the list count as 0
+        for (int e = tid; e < TP * (RS / CPP); e += AX_THREADS) {
+            const int t = e / (RS / CPP), c = e % (RS / CPP), li = st * RS + c * CPP;
+            const int bytes = t < p.T ? max(0, min(CPP, n - li)) * Z::CB : 0;
+            ax_cp16(base + Z::C_OFF + t * Z::C_PITCH + c * 16, (const char *)p.coef + (bytes ? ((size_t)t * p.coef_stride + li) * Z::CB : 0), (unsigned)bytes);
+        }
+    };
+    for (int s = 0; s < S - 1; s++) { if (s < n_units) issue(s); asm volatile("cp.async.commit_group;" ::: "memory"); }
+
+    float acc[4][NT][4];
+    auto clear = [&]() {
+#pragma unroll
+        for (int m = 0; m < 4; m++)
+#pragma unroll
+            for (int t = 0; t < NT; t++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[m][t][j] = 0.f;
+    };
+    clear();
+    const int g = lane >> 2, q = lane & 3, j8 = lane >> 3;
+    // FP16: transposed 8x8 loads (k = list rows, m = columns).  Q4_0: word g of the warp's 64 columns, rows 2q, 2q + 1 (and + 8)
+    const uint32_t a_off = Q4 ? (uint32_t)((wk * KPW * 16 + 2 * q) * Z::W_PITCH + wc * 32 + g * 4)
+                              : (uint32_t)((wk * KPW * 16 + (j8 >> 1) * 8 + (lane & 7)) * Z::W_PITCH + (wc * 64 + (j8 & 1) * 8) * 2);
+    const uint32_t s_off = (uint32_t)((wk * KPW * 16 + 2 * q) * Z::W_PITCH + 128 + (wc * 2 + (g >> 2)) * 2);
+    const uint32_t b_off = (uint32_t)(Z::C_OFF + ((lane & 7) + (NT > 1 ? ((lane >> 4) & 1) * 8 : 0)) * Z::C_PITCH + (wk * KPW * 16 + ((lane >> 3) & 1) * 8) * 2);
+
+    int next_row = 0;
+    for (int i = 0; i < n_units; i++) {
+        asm volatile("cp.async.wait_group %0;" :: "n"(S - 2) : "memory");
+        // row numbers travel two units ahead of their use: read now, stored in the next round, used in the one after
+        if (i > 0 && tid < RS) rows[((i + S) % AX_ROW_RING) * RS + tid] = next_row;
+        __syncthreads();                                              // stage i has landed for everybody; stage i - 1 is consumed
+        if (i + S - 1 < n_units) issue(i + S - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (tid < RS) next_row = row_at(u0 + i + S + 1, tid);
+        const uint32_t base = ring_a + (uint32_t)(i % S) * Z::STAGE;
+#pragma unroll
+        for (int k = 0; k < KPW; k++) {
+            if (EXACT) {
+                // lane: bytes 2 * (g & 1) and the next of word g >> 1 of a block, so that an mma's rows lie in ONE column block
+                // and the block's scales can go into its B operand
+#pragma unroll
+                for (int bl = 0; bl < 2; bl++) {
+                    uint32_t w[4];
+                    float d[4];
+#pragma unroll
+                    for (int h = 0; h < 4; h++) {
+                        const uint32_t at = base + (uint32_t)((wk * 16 + 2 * q + (h >> 1) * 8 + (h & 1)) * Z::W_PITCH);
+                        unsigned short x;
+                        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[h]) : "r"(at + (wc * 2 + bl) * 16 + (g >> 1) * 4));
+                        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(x) : "r"(at + 128 + (wc * 2 + bl) * 2));
+                        d[h] = __half2float(__ushort_as_half(x));
+                    }
+                    uint32_t a[2][4];                                 // (bit patterns: 0x4300 = 128, 0xC308 = -136)
+#pragma unroll
+                    for (int m = 0; m < 2; m++) {
+                        const unsigned sel = 0x4400u + 0x1111u * (unsigned)(2 * (g & 1) + m);
+                        const uint32_t x = __byte_perm(w[0], w[1], sel), y = __byte_perm(w[2], w[3], sel);
+                        a[m][0] = ax_badd2((x & 0x000F000Fu) | 0x43004300u, 0xC308C308u);
+                        a[m][1] = ax_badd2(((x >> 4) & 0x000F000Fu) | 0x43004300u, 0xC308C308u);
+                        a[m][2] = ax_badd2((y & 0x000F000Fu) | 0x43004300u, 0xC308C308u);
+                        a[m][3] = ax_badd2(((y >> 4) & 0x000F000Fu) | 0x43004300u, 0xC308C308u);
+                    }
+#pragma unroll
+                    for (int t = 0; t < NT; t++) {
+                        const uint32_t at = base + (uint32_t)(Z::C_OFF + (t * 8 + g) * Z::C_PITCH + (wk * 16 + 2 * q) * 4);
+                        float c[4];
+                        asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(c[0]), "=f"(c[1]) : "r"(at));
+                        asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(c[2]), "=f"(c[3]) : "r"(at + 32));
+                        uint32_t b0[3], b1[3];
+                        ax_split3(c[0] * d[0], c[1] * d[1], b0);
+                        ax_split3(c[2] * d[2], c[3] * d[3], b1);
+#pragma unroll
+                        for (int m = 0; m < 2; m++)
+#pragma unroll
+                            for (int i3 = 0; i3 < 3; i3++) ax_bmma(acc[bl * 2 + m][t], a[m], b0[i3], b1[i3]);
+                    }
+                }
+                continue;
+            }
+            uint32_t b[NT][2];
+            if (NT == 1) ax_ldsm2(b[0][0], b[0][1], base + b_off + k * 32);
+            else {
+#pragma unroll
+                for (int t = 0; t + 1 < NT; t += 2) {
+                    uint32_t v[4];
+                    ax_ldsm4(v, base + b_off + t * 8 * Z::C_PITCH + k * 32);
+                    b[t][0] = v[0]; b[t][1] = v[1]; b[t + (NT > 1)][0] = v[2]; b[t + (NT > 1)][1] = v[3];
+                }
+            }
+            if (!Q4) {
+#pragma unroll
+                for (int m = 0; m < 4; m++) {
+                    uint32_t a[4];
+                    ax_ldsm4_trans(a, base + a_off + k * 16 * Z::W_PITCH + m * 32);
+#pragma unroll
+                    for (int t = 0; t < NT; t++) ax_hmma(acc[m][t], a, b[t][0], b[t][1]);
+                }
+            } else {
+                uint32_t w[4], sc[2];
+#pragma unroll
+                for (int h = 0; h < 4; h++)
+                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[h]) : "r"(base + a_off + (k * 16 + (h >> 1) * 8 + (h & 1)) * Z::W_PITCH));
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    unsigned short x, y;
+                    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(x) : "r"(base + s_off + (k * 16 + h * 8) * Z::W_PITCH));
+                    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(y) : "r"(base + s_off + (k * 16 + h * 8 + 1) * Z::W_PITCH));
+                    sc[h] = (uint32_t)x | ((uint32_t)y << 16);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++) {                         // byte j of the word: columns j (low nibble) and 16 + j (high)
+                    const unsigned sel = 0x4400u + 0x1111u * (unsigned)j;
+                    const uint32_t x = __byte_perm(w[0], w[1], sel), y = __byte_perm(w[2], w[3], sel);
+                    uint32_t a[4];                                    // (bit patterns: 0x6400 = 1024, 0x2C00 = 1/16, 0xE408 = -1032, 0xD480 = -72)
+                    a[0] = ax_mul2(ax_add2((x & 0x000F000Fu) | 0x64006400u, 0xE408E408u), sc[0]);
+                    a[1] = ax_mul2(ax_fma2((x & 0x00F000F0u) | 0x64006400u, 0x2C002C00u, 0xD480D480u), sc[0]);
+                    a[2] = ax_mul2(ax_add2((y & 0x000F000Fu) | 0x64006400u, 0xE408E408u), sc[1]);
+                    a[3] = ax_mul2(ax_fma2((y & 0x00F000F0u) | 0x64006400u, 0x2C002C00u, 0xD480D480u), sc[1]);
+#pragma unroll
+                    for (int t = 0; t < NT; t++) ax_hmma(acc[j][t], a, b[t][0], b[t][1]);
+                }
+            }
+        }
+        const int u = u0 + i, cs = u / nst;
+        if (u % nst == nst - 1 || i == n_units - 1) {
+            // ---- end of this CTA's share of the slice: the four row quarters are added in order
+#pragma unroll 1
+            for (int r = 0; r < 4; r++) {
+                if (wk == r) {
+#pragma unroll
+                    for (int m = 0; m < 4; m++)
+#pragma unroll
+                        for (int t = 0; t < NT; t++)
+#pragma unroll
+                            for (int j = 0; j < 4; j++) {
+                                // fragment row g (j < 2) or g + 8: FP16: column m * 16 + that; Q4_0: word g, byte m, nibble j >> 1;
+                                // exact: block m >> 1, word g >> 1, byte 2 * (g & 1) + (m & 1), nibble j >> 1
+                                const int c = wc * 64 + (EXACT ? (m >> 1) * 32 + (g >> 1) * 4 + 2 * (g & 1) + (m & 1) + (j >> 1) * 16
+                                                         : Q4 ? (g >> 2) * 32 + (g & 3) * 4 + m + (j >> 1) * 16 : m * 16 + g + (j >> 1) * 8);
+                                float * o = red + (t * 8 + 2 * q + (j & 1)) * AX_RED_PITCH + c;
+                                *o = r == 0 ? acc[m][t][j] : *o + acc[m][t][j];
+                            }
+                }
+                __syncthreads();
+            }
+            const int c_lo = (int)((((unsigned long long)cs * nst + 1u) * G - 1u) / total), c_hi = (int)(((unsigned long long)(cs + 1) * nst * G - 1u) / total);
+            const int piece = cta - c_lo, more = cta == c_hi ? p.n_pieces - 1 - piece : 0;      // the slice's last CTA also writes the missing pieces
+            for (int e = tid; e < p.T * AX_CW; e += AX_THREADS) {
+                const int c = e % AX_CW, t = e / AX_CW, col = cs * AX_CW + c;
+                if (col >= p.ncols) continue;
+                float * o = p.partial + ((size_t)piece * p.T_all + t) * p.ncols + col;
+                *o = red[t * AX_RED_PITCH + c];
+                for (int k = 1; k <= more; k++) o[(size_t)k * p.T_all * p.ncols] = 0.f;
+            }
+            clear();
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------- coefficients
+// h F32 [T, h_stride] (by global neuron id) -> coef [T, coef_stride] by list position: FP16(h), or for Q4_0 rows the int8
+// quant of h in its block of 32 neurons times that block's FP16 scale (ggml.c:14575-14581, quantize_row_q8_0), rounded to FP16
+// or (exact mode) as it is, in F32; 0 where the token is inactive.  One warp per 32 local rows (one word of the union masks); a
+// CTA counts the rows named by the words before its own to find its list positions, and writes its part of the list.
+struct CoefP {
+    const float * h; int64_t h_stride; const float * idx; int64_t idx_stride; float threshold;
+    const int32_t * bucket; const uint32_t * masks; int32_t * list; int32_t * count; int n_local, T;
+    const float * fill_bias; int h_uncleared;
+    void * coef; int64_t coef_stride; int exact;
+};
+
+template <bool Q4>
+__global__ void __launch_bounds__(256) k_coef(const CoefP p) {
+    __shared__ int s_sum[8];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_chunks = (p.n_local + 31) / 32;
+    const int c = blockIdx.x * 8 + warp;
+    pdl_launch();
+    pdl_wait();
+    int sum = 0;
+    for (int k = tid; k < (int)blockIdx.x * 8; k += 256) sum += __popc(__ldcg(p.masks + k));
+    uint32_t m = c < n_chunks ? __ldcg(p.masks + c) : 0u;
+    const int left = p.n_local - c * 32;                              // bits beyond the last row never count
+    if (left < 32) m &= left <= 0 ? 0u : (1u << left) - 1u;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0) s_sum[warp] = sum;
+    __syncthreads();
+    int base = 0;
+#pragma unroll
+    for (int w = 0; w < 8; w++) base += s_sum[w];
+    __syncthreads();
+    if (lane == 0) s_sum[warp] = __popc(m);
+    __syncthreads();
+    int total = base;
+#pragma unroll
+    for (int w = 0; w < 8; w++) { if (w < warp) base += s_sum[w]; total += s_sum[w]; }
+    if (blockIdx.x == gridDim.x - 1 && blockIdx.y == 0 && tid == 0) *p.count = total;
+    if (m == 0u) return;
+    const int pos = base + __popc(m & ((1u << lane) - 1u));
+    const bool mine = m >> lane & 1u;
+    const int r = c * 32 + lane;
+    const bool in = r < p.n_local;
+    if (mine && blockIdx.y == 0) p.list[pos] = r;
+    const int64_t g = in ? (p.bucket ? p.bucket[r] : r) : 0;
+    const float fill = Q4 && p.h_uncleared && p.fill_bias && in ? fmaxf(p.fill_bias[g], 0.f) : 0.f;
+    constexpr int UN = 8;
+    for (int t0 = blockIdx.y * UN; t0 < p.T; t0 += gridDim.y * UN) {
+        float v[UN], l[UN];
+#pragma unroll
+        for (int u = 0; u < UN; u++) {
+            v[u] = 0.f; l[u] = 0.f;
+            if (in && t0 + u < p.T) { v[u] = p.h[(size_t)(t0 + u) * p.h_stride + g]; l[u] = p.idx[(size_t)(t0 + u) * p.idx_stride + g]; }
+        }
+#pragma unroll
+        for (int u = 0; u < UN; u++) {
+            const int t = t0 + u;
+            if (t >= p.T) break;
+            const bool on = in && !(l[u] < p.threshold);              // (a NaN logit counts as active)
+            float o;
+            if (!Q4) {
+                o = on ? v[u] : 0.f;
+            } else {
+                const float x = on || !p.h_uncleared ? v[u] : fill;   // what the graph leaves at an inactive neuron
+                const float amax = warp_max(fabsf(x));
+                const float id = amax != 0.0f ? 127.0f / amax : 0.0f;
+                o = on ? (float)__float2int_rn(x * id) * round_f16(amax / 127.0f) : 0.f;
+            }
+            if (mine) {
+                if (Q4 && p.exact) reinterpret_cast<float *>(p.coef)[(size_t)t * p.coef_stride + pos] = o;
+                else reinterpret_cast<__half *>(p.coef)[(size_t)t * p.coef_stride + pos] = __float2half_rn(o);
+            }
+        }
+    }
+}
+
+int launch_coef(const CoefArgs & a, cudaStream_t st) {
+    CoefP p;
+    p.h = a.h; p.h_stride = a.h_stride; p.idx = a.idx; p.idx_stride = a.idx_stride; p.threshold = a.threshold;
+    p.bucket = a.bucket; p.masks = a.masks; p.list = a.list_out; p.count = a.count_out; p.n_local = (int)a.n_local; p.T = a.T;
+    p.fill_bias = a.fill_bias; p.h_uncleared = a.h_uncleared ? 1 : 0; p.coef = a.coef; p.coef_stride = a.coef_stride; p.exact = a.exact ? 1 : 0;
+    const int n_chunks = (int)((a.n_local + 31) / 32);
+    const dim3 grid((n_chunks + 7) / 8, (a.T + 7) / 8);
+    if (a.wtype == PI_TYPE_Q4_0) PI_CUDA(launch_k(k_coef<true>, grid, dim3(256), 0, st, a.pdl, p));
+    else                         PI_CUDA(launch_k(k_coef<false>, grid, dim3(256), 0, st, a.pdl, p));
+    return PI_OK;
+}
+
+// ---------------------------------------------------------------------------------------------- launch
+// At most 16 CTAs per column slice (a partial vector each): more would cost the reader of the pieces more than they save.
+static void axpy_mm_shape(int64_t ncols, int * n_cs, int * grid, int * n_pieces) {
+    *n_cs = (int)((ncols + AX_CW - 1) / AX_CW);
+    *grid = (int)imin64(sm_count(), (int64_t)*n_cs * 16);
+    *n_pieces = (*grid + *n_cs - 1) / *n_cs + 1;                      // ranges are not aligned to slices: one more than the quotient
+}
+
+// Q4_0 rows whose width is no multiple of 1024 take exact coefficients (F32): see the top of the file
+bool axpy_mm_exact(int wtype, int64_t ncols) { return wtype == PI_TYPE_Q4_0 && ncols % 1024 != 0; }
+
+int axpy_mm_pieces(int64_t ncols) { int cs, g, np; axpy_mm_shape(ncols, &cs, &g, &np); return np; }
+
+template <int MODE, int NT>
+static int axpy_mm_go(const AxpyMmP & p, int grid, bool pdl, cudaStream_t st) {
+    using Z = AxShape<MODE, NT>;
+    static bool attr_done[16] = {false};
+    int dev = 0;
+    PI_CUDA(cudaGetDevice(&dev));
+    auto kern = k_axpy_mm<MODE, NT>;
+    const int smem = Z::HEAD + Z::S * Z::STAGE;
+    if (dev >= 0 && dev < 16 && !attr_done[dev]) {
+        PI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        attr_done[dev] = true;
+    }
+    PI_CUDA(launch_k(kern, dim3(grid), dim3(AX_THREADS), (size_t)smem, st, pdl, p));
+    return PI_OK;
+}
+
+template <int MODE>
+static int axpy_mm_tokens(const AxpyMmP & p, int grid, bool pdl, cudaStream_t st) {
+    return p.T <= 8 ? axpy_mm_go<MODE, 1>(p, grid, pdl, st) : p.T <= 16 ? axpy_mm_go<MODE, 2>(p, grid, pdl, st) : axpy_mm_go<MODE, 4>(p, grid, pdl, st);
+}
+
+// PI_ERR_UNSUPPORTED: shape not eligible, the caller uses the CUDA-core kernel.  Tokens go in launches of at most 32.
+int launch_axpy_mm(const AxpyArgs & a, cudaStream_t st, int * pieces_used) {
+    const bool q4 = a.wtype == PI_TYPE_Q4_0, exact = axpy_mm_exact(a.wtype, a.ncols);
+    if (!a.coef || a.coef_stride % 8 != 0 || !a.list || (q4 ? a.ncols % 256 != 0 : a.ncols % 8 != 0)) return PI_ERR_UNSUPPORTED;
+    AxpyMmP p;
+    int grid;
+    axpy_mm_shape(a.ncols, &p.n_cs, &grid, &p.n_pieces);
+    if (p.n_pieces > a.n_groups) return PI_ERR_UNSUPPORTED;
+    p.Wt = (const uint8_t *)a.Wt; p.row_bytes = (int64_t)pi_row_bytes(a.wtype, a.ncols); p.nrows = (int)a.nrows; p.ncols = (int)a.ncols;
+    p.nb = (int)(a.ncols / 32); p.T_all = a.T; p.list = a.list; p.count = a.count; p.coef_stride = a.coef_stride;
+    if (pieces_used) *pieces_used = p.n_pieces;
+    for (int t0 = 0; t0 < a.T; t0 += 32) {
+        p.T = a.T - t0 < 32 ? a.T - t0 : 32;
+        p.coef = (const char *)a.coef + (size_t)t0 * a.coef_stride * (exact ? 4 : 2); p.partial = a.partial + (size_t)t0 * a.ncols;
+        const int rc = exact ? axpy_mm_tokens<AX_Q4_EXACT>(p, grid, a.pdl, st) : q4 ? axpy_mm_tokens<AX_Q4>(p, grid, a.pdl, st) : axpy_mm_tokens<AX_F16>(p, grid, a.pdl, st);
+        if (rc != PI_OK) return rc;
+    }
+    return PI_OK;
+}
+
+}  // namespace pi

@@ -43,18 +43,27 @@ static int check_w(int wtype, int64_t ncols, const void * W) {
     return PI_OK;
 }
 
-struct SparseScratch { int32_t * list; int32_t * count; unsigned int * ticket; unsigned int * status; uint32_t * masks; };
+struct SparseScratch {
+    int32_t * list; int32_t * count; unsigned int * ticket; unsigned int * status; uint32_t * masks;
+    void * coef; int64_t coef_stride;                                // 2+ tokens: axpy coefficients
+};
 
 // The control words come FIRST in every sparse operator's workspace (count, ticket, status at bytes 0, 4, 8), so that
-// pi_op_status can find the status word of whichever operator used the workspace last.
-static bool carve_sparse(Scratch & s, int64_t n_rows, SparseScratch & o) {
+// pi_op_status can find the status word of whichever operator used the workspace last.  coef_size: bytes of an axpy
+// coefficient (0: none needed).
+static bool carve_sparse(Scratch & s, int64_t n_rows, int T, int coef_size, SparseScratch & o) {
     int32_t * ct = (int32_t *)s.take(256);
     o.list = (int32_t *)s.take((size_t)n_rows * 4);
     o.masks = (uint32_t *)s.take((size_t)((n_rows + 31) / 32) * 4);
+    o.coef = nullptr; o.coef_stride = (n_rows + 7) / 8 * 8;
+    if (T > 1 && coef_size && !(o.coef = s.take((size_t)T * o.coef_stride * coef_size))) return false;
     if (!o.list || !ct || !o.masks) return false;
     o.count = ct; o.ticket = (unsigned int *)(ct + 1); o.status = (unsigned int *)(ct + 2);
     return true;
 }
+
+// The rows of a gather: activity bit masks, and the sorted list only where the kernel that follows wants one
+static bool wants_list(int T, int64_t n_rows) { return T == 1 || n_rows > MM_MAX_ROWS; }
 
 }  // namespace pi
 
@@ -77,7 +86,8 @@ size_t pi_workspace_bytes(int64_t ncols, int64_t nrows, int T) {
     size_t b = 0;
     b += act_bytes(PI_TYPE_Q4_0, (m + 31) / 32 * 32, T) + act_bytes(PI_TYPE_F16, m, T) * 2;   // activation planes, predictor hidden
     b += up((size_t)nrows * 4) + 256 + up((size_t)(nrows + 31) / 32 * 4);                    // list, count/ticket, masks
-    b += up((size_t)T * nrows) + up((size_t)T * (nrows / 32 + 1) * 4);                       // Q8 coefficients of h
+    if (T == 1) b += up((size_t)nrows) + up((size_t)(nrows / 32 + 1) * 4);                   // Q8 coefficients of h
+    else b += up((size_t)T * (nrows + 7) * 4);                                               // axpy coefficients
     b += up((size_t)T * nrows * 4);                                                          // hidden vector of pi_sparse_ffn
     b += up((size_t)256 * T * ncols * 4);                                                    // axpy partials (<= 256 groups)
     return b + 4096;
@@ -118,7 +128,7 @@ int pi_mul_mat(int wtype, const void * W, int64_t nrows, int64_t ncols, const fl
     GemvArgs g;
     g.wtype = wtype; g.W = W; g.nrows = nrows; g.ncols = ncols; g.x = act.view(); g.T = T;
     g.bias = bias; g.dst = dst; g.dst_stride = nrows;
-    if (workspace_bytes >= act_bytes(wtype, ncols, T) + 256) {       // room for a status word: the bulk-copy ring kernels are eligible
+    if (T == 1 && workspace_bytes >= act_bytes(wtype, ncols, T) + 256) {   // room for a status word: the bulk-copy ring kernels are eligible
         g.status = (unsigned int *)p;
         PI_CUDA(cudaMemsetAsync(g.status, 0, 4, st));
     }
@@ -141,9 +151,13 @@ int pi_predictor(const void * fc1, const void * fc2, int64_t d, int64_t rank, in
     if ((rc = launch_convert_act(PI_TYPE_F16, p_in, d, d, T, a_in, st))) return rc;
     GemvArgs g1;                                       // hidden = relu(fc1 . p), kept only in the FP16 form fc2 consumes
     g1.W = fc1; g1.nrows = rank; g1.ncols = d; g1.x = a_in.view(); g1.T = T; g1.relu = 1; g1.dst16 = a_h.h16; g1.dst_stride = rank;
-    if ((rc = launch_gemv(g1, st))) return rc;
     GemvArgs g2;
-    g2.W = fc2; g2.nrows = F; g2.ncols = rank; g2.x = a_h.view(); g2.T = T; g2.dst = idx; g2.dst_stride = F;
+    g2.W = fc2; g2.nrows = F; g2.ncols = rank; g2.x = a_h.view(); g2.T = T; g2.dst = idx; g2.dst_stride = F; g2.pdl = true;
+    if (T == 1 && workspace_bytes >= act_bytes(PI_TYPE_F16, d, T) + act_bytes(PI_TYPE_F16, rank, T) + 256) {     // as in pi_mul_mat
+        g1.status = g2.status = (unsigned int *)p;
+        PI_CUDA(cudaMemsetAsync(p, 0, 4, st));
+    }
+    if ((rc = launch_gemv(g1, st))) return rc;
     return launch_gemv(g2, st);
 }
 
@@ -175,7 +189,7 @@ int pi_mul_mat_idx(int wtype, const void * W, int64_t n_w_rows, int64_t ncols,
     cudaStream_t st = (cudaStream_t)stream;
     Scratch s(workspace, workspace_bytes);
     SparseScratch ss;
-    const bool carved = carve_sparse(s, n_w_rows, ss);
+    const bool carved = carve_sparse(s, n_w_rows, T, 0, ss);
     char * actp = (char *)s.take(act_bytes(wtype, ncols, T));
     if (!aligned(workspace, 256) || !actp || !carved) { set_error("mul_mat_idx: workspace too small or misaligned"); return PI_ERR_WORKSPACE; }
     ActBuf act = act_carve(wtype, ncols, T, &actp);
@@ -185,14 +199,16 @@ int pi_mul_mat_idx(int wtype, const void * W, int64_t n_w_rows, int64_t ncols,
     if ((rc = launch_convert_act(wtype, x, ncols, ncols, T, act, st))) return rc;
     CompactArgs c;
     c.idx = idx; c.idx_stride = idx_stride; c.T = T; c.threshold = threshold; c.n_local = n_w_rows; c.bucket = bucket;
-    c.list = ss.list; c.count = ss.count; c.masks = ss.masks; c.ticket = ss.ticket;
+    c.masks = ss.masks;
+    if (wants_list(T, n_w_rows)) { c.list = ss.list; c.count = ss.count; c.ticket = ss.ticket; }
     c.zero_dst = dst; c.zero_stride = n_dst_rows;
     if ((rc = launch_compact(c, st))) return rc;
     GemvArgs g;
     g.wtype = wtype; g.W = W; g.nrows = n_w_rows; g.ncols = ncols; g.x = act.view(); g.T = T;
-    g.list = ss.list; g.count = ss.count; g.bucket = bucket; g.idx = idx; g.idx_stride = idx_stride; g.threshold = threshold;
+    if (wants_list(T, n_w_rows)) { g.list = ss.list; g.count = ss.count; }
+    if (T == 1 || n_w_rows <= MM_MAX_ROWS) g.masks = ss.masks;
+    g.bucket = bucket; g.idx = idx; g.idx_stride = idx_stride; g.threshold = threshold;
     g.dst = dst; g.dst_stride = n_dst_rows; g.status = ss.status;
-    if (T == 1) g.masks = ss.masks;
     return launch_gemv(g, st);
 }
 
@@ -210,11 +226,11 @@ int pi_axpy(int wtype, const void * Wt, int64_t n_w_rows, int64_t ncols,
     Scratch s(workspace, workspace_bytes);
     SparseScratch ss;
     const int G = axpy_groups(wtype, ncols, T);
-    bool ok = aligned(workspace, 256) && carve_sparse(s, n_w_rows, ss);
+    bool ok = aligned(workspace, 256) && carve_sparse(s, n_w_rows, T, axpy_mm_exact(wtype, ncols) ? 4 : 2, ss);
     int8_t * cq = nullptr; float * cd = nullptr;
-    if (ok && wtype == PI_TYPE_Q4_0) {
-        cq = (int8_t *)s.take((size_t)T * h_stride);
-        cd = (float *)s.take((size_t)T * (h_stride / 32) * 4);
+    if (ok && wtype == PI_TYPE_Q4_0 && T == 1) {
+        cq = (int8_t *)s.take((size_t)h_stride);
+        cd = (float *)s.take((size_t)(h_stride / 32) * 4);
         ok = cq && cd;
     }
     float * partial = ok ? (float *)s.take((size_t)G * T * ncols * 4) : nullptr;
@@ -222,17 +238,26 @@ int pi_axpy(int wtype, const void * Wt, int64_t n_w_rows, int64_t ncols,
     PI_CUDA(cudaMemsetAsync(ss.count, 0, 12, st));                                      // count, ticket, status
     CompactArgs c;
     c.idx = idx; c.idx_stride = idx_stride; c.T = T; c.threshold = threshold; c.n_local = n_w_rows; c.bucket = bucket;
-    c.list = ss.list; c.count = ss.count; c.masks = ss.masks; c.ticket = ss.ticket;
+    c.masks = ss.masks;
+    if (T == 1) { c.list = ss.list; c.count = ss.count; c.ticket = ss.ticket; }              // (batches: launch_coef makes the list)
     if ((rc = launch_compact(c, st))) return rc;
-    if (wtype == PI_TYPE_Q4_0 && T > 1 && (rc = launch_neuron_q8(h, h_stride, h_stride, T, cq, cd, st))) return rc;
     AxpyArgs a;
+    if (T > 1) {
+        CoefArgs k;
+        k.pdl = true;
+        k.wtype = wtype; k.h = h; k.h_stride = h_stride; k.idx = idx; k.idx_stride = idx_stride; k.threshold = threshold; k.bucket = bucket;
+        k.masks = ss.masks; k.list_out = ss.list; k.count_out = ss.count; k.n_local = n_w_rows; k.T = T;
+        k.coef = ss.coef; k.coef_stride = ss.coef_stride; k.exact = axpy_mm_exact(wtype, ncols);
+        if ((rc = launch_coef(k, st))) return rc;
+        a.coef = ss.coef; a.coef_stride = ss.coef_stride; a.pdl = true;
+    }
     a.wtype = wtype; a.Wt = Wt; a.nrows = n_w_rows; a.ncols = ncols; a.h = h; a.h_stride = h_stride; a.T = T;
     a.list = ss.list; a.count = ss.count; a.bucket = bucket; a.idx = idx; a.idx_stride = idx_stride; a.threshold = threshold;
     a.cq = cq; a.cd = cd; a.c_stride = h_stride; a.partial = partial; a.n_groups = G; a.status = ss.status;
     if (T == 1) a.masks = ss.masks;
     int used = G;
     if ((rc = launch_axpy(a, st, &used))) return rc;
-    return launch_reduce_partials(partial, used, T, ncols, nullptr, nullptr, dst, st);
+    return launch_reduce_partials(partial, used, T, ncols, nullptr, nullptr, dst, st, true);
 }
 
 int pi_sparse_ffn(int wtype, const void * up, const void * gate, const void * down_t, int64_t n_w_rows, int64_t ncols,
@@ -250,21 +275,21 @@ int pi_sparse_ffn(int wtype, const void * up, const void * gate, const void * do
     Scratch s(workspace, workspace_bytes);
     SparseScratch ss;
     const int G = axpy_groups(wtype, ncols, T);
-    const bool carved = carve_sparse(s, n_w_rows, ss);
+    const bool carved = carve_sparse(s, n_w_rows, T, axpy_mm_exact(wtype, ncols) ? 4 : 2, ss);
     char * actp = (char *)s.take(act_bytes(wtype, ncols, T));
     bool ok = aligned(workspace, 256) && actp && carved;
     float * h = ok ? (float *)s.take((size_t)T * F * 4) : nullptr;
     int8_t * cq = nullptr; float * cd = nullptr;
-    if (ok && wtype == PI_TYPE_Q4_0) {
-        cq = (int8_t *)s.take((size_t)T * F);
-        cd = (float *)s.take((size_t)T * (F / 32) * 4);
+    if (ok && wtype == PI_TYPE_Q4_0 && T == 1) {
+        cq = (int8_t *)s.take((size_t)F);
+        cd = (float *)s.take((size_t)(F / 32) * 4);
         ok = cq && cd;
     }
     float * partial = ok && h ? (float *)s.take((size_t)G * T * ncols * 4) : nullptr;
     if (!ok || !h || !partial) { set_error("sparse_ffn: workspace too small or misaligned"); return PI_ERR_WORKSPACE; }
     ActBuf act = act_carve(wtype, ncols, T, &actp);
     PI_CUDA(cudaMemsetAsync(ss.count, 0, 12, st));                                      // count, ticket, status
-    if (bucket || T > 1 || wtype == PI_TYPE_Q4_0) PI_CUDA(cudaMemsetAsync(h, 0, (size_t)T * F * 4, st));
+    if (T == 1 && (bucket || wtype == PI_TYPE_Q4_0)) PI_CUDA(cudaMemsetAsync(h, 0, (size_t)F * 4, st));
     if ((rc = launch_convert_act(wtype, x, ncols, ncols, T, act, st))) return rc;
     // the kernels below are chained with programmatic dependent launch: each may start while its predecessor drains
     {
@@ -287,27 +312,42 @@ int pi_sparse_ffn(int wtype, const void * up, const void * gate, const void * do
     CompactArgs c;
     c.pdl = true;
     c.idx = idx; c.idx_stride = idx_stride; c.T = T; c.threshold = threshold; c.n_local = n_w_rows; c.bucket = bucket;
-    c.list = ss.list; c.count = ss.count; c.masks = ss.masks; c.ticket = ss.ticket;
-    if (wtype == PI_TYPE_Q4_0) { c.zero_dst = h; c.zero_stride = F; c.fill_bias = up_bias; c.fill_relu = 1; }
+    c.masks = ss.masks;
+    if (wants_list(T, n_w_rows)) { c.list = ss.list; c.count = ss.count; c.ticket = ss.ticket; }
+    if (wtype == PI_TYPE_Q4_0 && T == 1) { c.zero_dst = h; c.zero_stride = F; c.fill_bias = up_bias; c.fill_relu = 1; }
     if ((rc = launch_compact(c, st))) return rc;
     GemvArgs g;
     g.pdl = true;
     g.wtype = wtype; g.W = up; g.W2 = gate; g.nrows = n_w_rows; g.ncols = ncols; g.x = act.view(); g.T = T;
-    g.list = ss.list; g.count = ss.count; g.bucket = bucket; g.idx = idx; g.idx_stride = idx_stride; g.threshold = threshold;
+    if (wants_list(T, n_w_rows)) { g.list = ss.list; g.count = ss.count; }
+    if (T == 1 || n_w_rows <= MM_MAX_ROWS) g.masks = ss.masks;
+    g.bucket = bucket; g.idx = idx; g.idx_stride = idx_stride; g.threshold = threshold;
     g.bias = up_bias; g.relu = gate ? 0 : 1;
-    g.dst = h; g.dst_stride = F; g.status = ss.status;
-    if (T == 1) g.masks = ss.masks;
+    g.status = ss.status;
+    // a batch of FP16 rows needs the activations only as coefficients; Q4_0 coefficients are made from blocks of 32 neurons
+    const bool direct = T > 1 && wtype == PI_TYPE_F16 && n_w_rows <= MM_MAX_ROWS;
+    if (direct) { g.coef = (__half *)ss.coef; g.coef_stride = ss.coef_stride; g.list_out = ss.list; g.count_out = ss.count; } else { g.dst = h; g.dst_stride = F; }
     if ((rc = launch_gemv(g, st))) return rc;
-    if (wtype == PI_TYPE_Q4_0 && T > 1 && (rc = launch_neuron_q8(h, F, F, T, cq, cd, st))) return rc;
     AxpyArgs a;
-    a.pdl = !(wtype == PI_TYPE_Q4_0 && T > 1);
+    if (T > 1) {
+        if (!direct) {
+            CoefArgs k;
+            k.pdl = true;
+            k.wtype = wtype; k.h = h; k.h_stride = F; k.idx = idx; k.idx_stride = idx_stride; k.threshold = threshold; k.bucket = bucket;
+            k.masks = ss.masks; k.list_out = ss.list; k.count_out = ss.count; k.n_local = n_w_rows; k.T = T; k.h_uncleared = true; k.fill_bias = up_bias;
+            k.coef = ss.coef; k.coef_stride = ss.coef_stride; k.exact = axpy_mm_exact(wtype, ncols);
+            if ((rc = launch_coef(k, st))) return rc;
+        }
+        a.coef = ss.coef; a.coef_stride = ss.coef_stride;
+    }
+    a.pdl = true;
     a.wtype = wtype; a.Wt = down_t; a.nrows = n_w_rows; a.ncols = ncols; a.h = h; a.h_stride = F; a.T = T;
     a.list = ss.list; a.count = ss.count; a.bucket = bucket; a.idx = idx; a.idx_stride = idx_stride; a.threshold = threshold;
     a.cq = cq; a.cd = cd; a.c_stride = F; a.partial = partial; a.n_groups = G; a.status = ss.status;
     if (T == 1) a.masks = ss.masks;
     int used = G;
     if ((rc = launch_axpy(a, st, &used))) return rc;
-    return launch_reduce_partials(partial, used, T, ncols, nullptr, nullptr, dst, st, T == 1);
+    return launch_reduce_partials(partial, used, T, ncols, nullptr, nullptr, dst, st, true);
 }
 
 int pi_op_status(const void * workspace, void * stream) {

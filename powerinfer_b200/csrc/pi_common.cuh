@@ -106,21 +106,26 @@ struct GemvArgs {
     __half * dst16 = nullptr;          // optional FP16 copy of the result [T, dst_stride] (feeds an F16 mat-vec)
     // second matrix sharing the row selection (gate with up): dst = relu(W2 row . x) * (W row . x)
     const void * W2 = nullptr;
-    // one token: activity bit masks (one word per 32 LOCAL rows) instead of a list; selects the register-streaming kernel
+    // activity bit masks (one word per 32 LOCAL rows) instead of a list; selects the register-streaming kernel (one token) or the
+    // tensor-core kernel (2+ tokens: the union of the tokens' masks)
     const uint32_t * masks = nullptr;
     unsigned long long * rows_total = nullptr;   // with masks (optional): incremented by the number of active rows (statistics)
-    // dense, one token: also write the activity bit masks of the result, bit (row % 32) of word (row / 32) = !(result <
-    // masks_threshold): the predictor's mask, made where the logit is.  Room for (nrows + 63) / 64 * 2 words.
+    // dense: also write the activity bit masks of the result, bit (row % 32) of word (row / 32) = !(result < masks_threshold) for
+    // some token: the predictor's mask, made where the logit is.  Room for (nrows + 63) / 64 * 2 words.
     uint32_t * masks_out = nullptr; float masks_threshold = 0.f;
     int pre_stages = -1;               // ring kernels: stages of weights requested before the dependency wait (-1: the whole ring)
     unsigned int * status = nullptr;   // device status word; when given, T == 1 shapes use the bulk-copy ring kernel
+    // 2+ tokens with masks (their union over the tokens): optional list of the active local rows in order, and their number
+    int32_t * list_out = nullptr; int32_t * count_out = nullptr;
+    // 2+ tokens with masks (optional): the result as axpy coefficients, FP16 by LIST POSITION, 0 where the token is inactive
+    __half * coef = nullptr; int64_t coef_stride = 0;
     bool pdl = false;                  // launch with programmatic dependent launch (the kernel waits for its producer itself)
 };
 int launch_gemv(const GemvArgs & a, cudaStream_t st);
 // PI_ERR_UNSUPPORTED: not eligible; *wrote_masks: the kernel that ran honoured masks_out itself
 int launch_gemv_ring(const GemvArgs & a, unsigned int * status, bool pdl, cudaStream_t st, bool * wrote_masks = nullptr);
-int launch_gemv_mma(const GemvArgs & a, cudaStream_t st);                                     // FP16 rows, T <= 32; PI_ERR_UNSUPPORTED: not eligible
-int launch_gemv_mma_q4(const GemvArgs & a, cudaStream_t st);                                  // Q4_0 rows, T >= 2; PI_ERR_UNSUPPORTED: not eligible
+int launch_mm(const GemvArgs & a, cudaStream_t st);                                           // 2+ tokens; PI_ERR_UNSUPPORTED: not eligible
+static constexpr int64_t MM_MAX_ROWS = 262144;                                                // rows a gather of launch_mm can choose from
 
 // predictor logits -> compacted list of LOCAL rows active for >= 1 token; also writes zeros (or relu(bias)) into
 // h_init [T, h_stride] for rows that are inactive for a token when h_init != nullptr
@@ -151,6 +156,7 @@ struct AxpyArgs {
     const float * idx = nullptr; int64_t idx_stride = 0; float threshold = 0.f;
     // Q4_0: coefficient planes made by launch_neuron_q8 (int8 by global id, float scale per 32-neuron block)
     const int8_t * cq = nullptr; const float * cd = nullptr; int64_t c_stride = 0;
+    const void * coef = nullptr; int64_t coef_stride = 0;             // 2+ tokens: coefficients by list position (launch_coef, or GemvArgs::coef)
     float * partial = nullptr; int n_groups = 0;                      // [n_groups, T, ncols]: room for n_groups partial vectors
     unsigned int * status = nullptr;                                  // device status word (bit 1: a copy wait ran out); enables the
                                                                       // bulk-copy pipelined kernel for T == 1
@@ -158,7 +164,22 @@ struct AxpyArgs {
 };
 int axpy_groups(int wtype, int64_t ncols, int T);                     // row groups the launcher will use
 int launch_axpy(const AxpyArgs & a, cudaStream_t st, int * groups_used = nullptr);   // groups_used: partial vectors written
-int launch_axpy_mma(const AxpyArgs & a, cudaStream_t st, int * groups_used);         // FP16, 2..32 tokens; PI_ERR_UNSUPPORTED: not eligible
+int launch_axpy_mm(const AxpyArgs & a, cudaStream_t st, int * groups_used);          // 2+ tokens, needs coef; PI_ERR_UNSUPPORTED: not eligible
+bool axpy_mm_exact(int wtype, int64_t ncols);                                        // coefficients are F32, else FP16
+int axpy_mm_pieces(int64_t ncols);                                                   // partial vectors launch_axpy_mm writes
+// axpy coefficients by list position (pi_axpy_mm.cu): [T, coef_stride], FP16 or (exact) F32, from h F32 [T, h_stride] by global neuron id
+struct CoefArgs {
+    int wtype = PI_TYPE_F16;
+    const float * h = nullptr; int64_t h_stride = 0; const float * idx = nullptr; int64_t idx_stride = 0; float threshold = 0.f;
+    const int32_t * bucket = nullptr; const uint32_t * masks = nullptr;   // masks: union over the tokens
+    int32_t * list_out = nullptr; int32_t * count_out = nullptr;       // the active local rows in order, and their number
+    int64_t n_local = 0; int T = 1;
+    // h holds nothing where a token is inactive: Q4_0 block scales take 0 there, or relu(fill_bias) (what the graph's bias add leaves)
+    bool h_uncleared = false; const float * fill_bias = nullptr;
+    void * coef = nullptr; int64_t coef_stride = 0; bool exact = false;
+    bool pdl = false;
+};
+int launch_coef(const CoefArgs & a, cudaStream_t st);
 // one token, rows named by bit masks, weights streamed into registers (pi_rows.cu); PI_ERR_UNSUPPORTED: not eligible
 bool rows_eligible(int wtype, int64_t nrows, int64_t ncols);
 int launch_gather_rows(const GemvArgs & a, cudaStream_t st);

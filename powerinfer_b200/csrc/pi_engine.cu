@@ -104,12 +104,13 @@ struct pi_engine {
     std::vector<pi_layer_weights> layers;
     pi_model_weights g;
     int hd, dq, dkv, F, T_max;
-    int G;                                   // axpy row groups
+    int G, pieces;                           // axpy row groups (one token), partial vectors of a batch
     // device buffers carved from the caller's workspace
     int32_t * tokens, * pos, * seq_ids, * seq_pf, * argmax;   // seq_pf: the sequence of every token of a prompt chunk
     float * x, * x2, * attn_out, * ffn_vec, * qkv, * pred, * h, * partial, * logits, * cs;
     int32_t * list, * count; unsigned int * ticket; uint32_t * masks;
-    int8_t * cq; float * cd;
+    int8_t * cq; float * cd;                 // one token, shapes without a mask-driven axpy: Q8_0 coefficients of the hidden vector
+    void * coef; int64_t coef_stride;        // batches: axpy coefficients
     __half * hidden16;
     ActBuf act_a, act_q, act_p, act_o;       // FFN input, QKV input, predictor input (FP16), out-proj input
     __half * k_cache, * v_cache;             // [n_layer, max_batch, n_ctx, dkv]
@@ -161,12 +162,16 @@ static void carve(pi_engine * e, void * ws, size_t ws_bytes, bool dry, size_t * 
     e->x = cv.take<float>(T * d); e->x2 = cv.take<float>(T * d); e->attn_out = cv.take<float>(T * d); e->ffn_vec = cv.take<float>(T * d);
     e->qkv = cv.take<float>((size_t)T * (e->dq + 2 * e->dkv));
     e->pred = cv.take<float>(T * F); e->h = cv.take<float>(T * F);
-    e->partial = cv.take<float>((size_t)e->G * T * d);
+    e->pieces = axpy_mm_pieces(c.d);
+    const size_t vecs = (size_t)e->pieces * T;                       // partial vectors of a batch, of one token
+    e->partial = cv.take<float>((vecs > (size_t)e->G ? vecs : (size_t)e->G) * d);
     e->logits = cv.take<float>((size_t)T * c.n_vocab);
     e->cs = cv.take<float>((size_t)c.n_ctx * e->hd);
     e->list = cv.take<int32_t>(F); e->count = cv.take<int32_t>(1); e->ticket = cv.take<unsigned int>(1);
     e->masks = cv.take<uint32_t>((F + 63) / 64 * 2);
-    e->cq = cv.take<int8_t>(T * F); e->cd = cv.take<float>(T * (F / 32 + 1));
+    e->cq = cv.take<int8_t>(F); e->cd = cv.take<float>(F / 32 + 1);
+    e->coef = nullptr; e->coef_stride = ((int64_t)F + 7) / 8 * 8;
+    if (T > 1) e->coef = cv.take<float>((size_t)T * e->coef_stride);
     e->hidden16 = cv.take<__half>((size_t)T * c.rank);
     e->act_a = cv.act(c.wtype, c.d, T);
     e->act_q = cv.act(c.wtype, c.d, T);
@@ -414,7 +419,7 @@ int enqueue_step(pi_engine * e, int T, cudaStream_t st, StageTimer & tm, int mod
             g.status = e->status; g.pdl = pdl;
             g.wtype = out_t; g.W = e->g.output ? e->g.output : e->g.tok_embd; g.nrows = c.n_vocab; g.ncols = d;
             g.x = n1.act.view(); g.T = T; g.dst = e->logits; g.dst_stride = c.n_vocab;
-            STAGE(PI_STAGE_LM_HEAD, (T + 7) / 8, launch_gemv(g, st));
+            STAGE(PI_STAGE_LM_HEAD, 1, launch_gemv(g, st));
             if (!(e->skip_mask & (1u << PI_STAGE_OTHER))) {
                 if (tm.begin()) return PI_ERR_CUDA;
                 k_argmax<<<T, 1024, 0, st>>>(e->logits, c.n_vocab, e->argmax);
@@ -454,7 +459,7 @@ int enqueue_step(pi_engine * e, int T, cudaStream_t st, StageTimer & tm, int mod
             // while the norm before it is still reading the partial vectors; those reads then queue behind the burst
             // (measured: 5 us for 0.5 MB).  After such a norm the QKV mat-vec starts its ring only when its wait is over.
             g.pre_stages = n1_collects ? e->qkv_pre : -1;
-            STAGE(PI_STAGE_QKV, (T + 7) / 8, launch_gemv(g, st));
+            STAGE(PI_STAGE_QKV, 1, launch_gemv(g, st));
         }
         {
             AttnArgs a;
@@ -480,7 +485,7 @@ int enqueue_step(pi_engine * e, int T, cudaStream_t st, StageTimer & tm, int mod
             g.wtype = wt; g.W = L->wo; g.nrows = d; g.ncols = e->dq; g.x = e->act_o.view(); g.T = T;
             g.bias = c.rank_id == 0 ? L->bo : nullptr;                    // the bias enters the sum over ranks once
             g.dst = e->attn_out; g.dst_stride = d;
-            STAGE(PI_STAGE_WO, (T + 7) / 8, launch_gemv(g, st));
+            STAGE(PI_STAGE_WO, 1, launch_gemv(g, st));
         }
 
         // ---- FFN input.  llama / opt: ffn_inp = attn_out + x, then the FFN norm; the complete attention output is needed,
@@ -499,34 +504,35 @@ int enqueue_step(pi_engine * e, int T, cudaStream_t st, StageTimer & tm, int mod
 
         // ---- predictor: idx = fc2 . relu(fc1 . p)   (llama.cpp:4688-4695)
         float * pred = e->pred_trace ? e->pred_trace + (size_t)il * c.max_batch * F : e->pred;
-        // One token: the sparse kernels rank the active rows themselves from bit masks, which the predictor's second mat-vec
-        // writes in its epilogue (then no mask kernel runs at all).  Q4_0 rows with an up bias keep the mask kernel: it also
-        // writes relu(bias) into the hidden vector where a row is inactive, which the axpy's per-block quantisation must see.
-        const bool rows1 = T == 1 && e->rows1;
-        const bool masks1 = rows1 && e->fc2_masks && !(wt == PI_TYPE_Q4_0 && L->up_b);
+        // The sparse kernels rank the active rows themselves from bit masks (for a batch: the union of its tokens' masks), which
+        // the predictor's second mat-vec writes in its epilogue (then no mask kernel runs at all).  One token, Q4_0 rows with an
+        // up bias keeps the mask kernel: it also writes relu(bias) into the hidden vector where a row is inactive, which the
+        // axpy's per-block quantisation must see (batches: launch_coef).
+        const bool rows1 = T == 1 ? e->rows1 : F <= MM_MAX_ROWS;
+        const bool masks1 = rows1 && e->fc2_masks && !(T == 1 && wt == PI_TYPE_Q4_0 && L->up_b);
         {
             GemvArgs g1;
             g1.status = e->status; g1.pdl = pdl;
             g1.W = L->fc1; g1.nrows = c.rank; g1.ncols = d; g1.x = e->act_p.view(); g1.T = T; g1.relu = 1;
             g1.dst16 = e->hidden16; g1.dst_stride = c.rank;
-            STAGE(PI_STAGE_PRED, (T + 7) / 8, launch_gemv(g1, st));
+            STAGE(PI_STAGE_PRED, 1, launch_gemv(g1, st));
             Act hx; hx.h16 = e->hidden16;
             GemvArgs g2;
             g2.status = e->status; g2.pdl = pdl;
             g2.W = L->fc2; g2.nrows = F; g2.ncols = c.rank; g2.x = hx; g2.T = T; g2.dst = pred; g2.dst_stride = F;
             if (masks1) { g2.masks_out = e->masks; g2.masks_threshold = c.threshold; }
-            STAGE(PI_STAGE_PRED, (T + 7) / 8, launch_gemv(g2, st));
+            STAGE(PI_STAGE_PRED, 1, launch_gemv(g2, st));
         }
-        // ---- mask -> activity bit masks, and for batches the sorted list of rows active for at least one token.
-        //      Where a row is inactive for a token the dense hidden vector holds 0 (or relu(bias)): the Q4_0 axpy quantises
-        //      that vector per 32 neurons, and a union list leaves per-token holes.
+        // ---- mask -> activity bit masks where the predictor did not write them (and the list, where rows are named by one).
+        //      One token: where a row is inactive the dense hidden vector gets 0 (or relu(bias)); the Q4_0 axpy quantises it
+        //      per 32 neurons.
         if (!masks1) {
             CompactArgs ca;
             ca.pdl = pdl;
             ca.idx = pred; ca.idx_stride = F; ca.T = T; ca.threshold = c.threshold; ca.n_local = F;
             if (!rows1) { ca.list = e->list; ca.count = e->count; }
             ca.masks = e->masks; ca.ticket = e->ticket; ca.total = e->active_total;
-            if (wt == PI_TYPE_Q4_0) { ca.zero_dst = e->h; ca.zero_stride = F; ca.fill_bias = L->up_b; ca.fill_relu = 1; }
+            if (wt == PI_TYPE_Q4_0 && T == 1) { ca.zero_dst = e->h; ca.zero_stride = F; ca.fill_bias = L->up_b; ca.fill_relu = 1; }
             STAGE(PI_STAGE_COMPACT, 1, launch_compact(ca, st));
         }
         int used = e->G;
@@ -536,9 +542,11 @@ int enqueue_step(pi_engine * e, int T, cudaStream_t st, StageTimer & tm, int mod
         f.wtype = wt; f.up = L->up; f.gate = L->gate; f.down_t = L->down_t; f.nrows = F; f.ncols = d;
         f.x = e->act_a.view(); f.masks = e->masks; f.bias = L->up_b; f.relu = L->gate ? (e->gate_sym ? 1 : 0) : 1;
         f.h = e->h; f.partial = e->partial; f.n_groups = e->G < NORM_MAX_GROUPS ? e->G : NORM_MAX_GROUPS; f.rows_total = e->active_total;
-        if (masks1 && ffn_rows_eligible(f)) {                          // (the plan is cached: a table look-up after the first call)
+        if (T == 1 && masks1 && ffn_rows_eligible(f)) {                          // (the plan is cached: a table look-up after the first call)
             STAGE(PI_STAGE_FFN, 1, launch_ffn_rows(f, st, &used));
         } else {
+            // a batch of FP16 rows needs the activations only as coefficients; Q4_0 coefficients are made from blocks of 32 neurons
+            const bool direct = T > 1 && wt == PI_TYPE_F16 && F <= MM_MAX_ROWS;
             // ---- up (and gate) over the active rows: h = relu(gate.x) * (up.x) | relu(up.x + b)
             {
                 GemvArgs g;
@@ -547,19 +555,27 @@ int enqueue_step(pi_engine * e, int T, cudaStream_t st, StageTimer & tm, int mod
                 if (rows1) { g.masks = e->masks; if (masks1) g.rows_total = e->active_total; } else { g.list = e->list; g.count = e->count; }
                 g.idx = pred; g.idx_stride = F; g.threshold = c.threshold;
                 g.bias = L->up_b; g.relu = L->gate ? (e->gate_sym ? 1 : 0) : 1;
-                g.dst = e->h; g.dst_stride = F;
-                STAGE(PI_STAGE_UPGATE, (T + 7) / 8, launch_gemv(g, st));
+                if (direct) { g.coef = (__half *)e->coef; g.coef_stride = e->coef_stride; g.list_out = e->list; g.count_out = e->count; } else { g.dst = e->h; g.dst_stride = F; }
+                STAGE(PI_STAGE_UPGATE, 1, launch_gemv(g, st));
             }
             // ---- down: axpy over the same rows; the sum over row groups (and, sharded, over ranks) is left to the next norm
-            if (wt == PI_TYPE_Q4_0 && T > 1) STAGE(PI_STAGE_DOWN, 1, launch_neuron_q8(e->h, F, F, T, e->cq, e->cd, st));
+            if (T > 1 && !direct) {
+                CoefArgs k;
+                k.pdl = pdl;
+                k.wtype = wt; k.h = e->h; k.h_stride = F; k.idx = pred; k.idx_stride = F; k.threshold = c.threshold;
+                k.masks = e->masks; k.list_out = e->list; k.count_out = e->count; k.n_local = F; k.T = T; k.h_uncleared = true; k.fill_bias = L->up_b;
+                k.coef = e->coef; k.coef_stride = e->coef_stride; k.exact = axpy_mm_exact(wt, d);
+                STAGE(PI_STAGE_DOWN, 1, launch_coef(k, st));
+            }
             {
                 AxpyArgs a;
                 a.pdl = pdl;
                 a.wtype = wt; a.Wt = L->down_t; a.nrows = F; a.ncols = d; a.h = e->h; a.h_stride = F; a.T = T;
-                if (rows1) { a.masks = e->masks; a.h_uncleared = masks1; } else { a.list = e->list; a.count = e->count; }
+                if (T == 1 && rows1) { a.masks = e->masks; a.h_uncleared = masks1; } else { a.list = e->list; a.count = e->count; }
                 a.idx = pred; a.idx_stride = F; a.threshold = c.threshold;
-                a.cq = e->cq; a.cd = e->cd; a.c_stride = F; a.partial = e->partial; a.n_groups = e->G; a.status = e->status;
-                STAGE(PI_STAGE_DOWN, T == 1 ? 1 : (wt == PI_TYPE_Q4_0 ? (T + 1) / 2 : (T + 3) / 4), launch_axpy(a, st, &used));
+                a.cq = e->cq; a.cd = e->cd; a.c_stride = F; a.partial = e->partial; a.n_groups = T == 1 ? e->G : e->pieces; a.status = e->status;
+                if (T > 1) { a.coef = e->coef; a.coef_stride = e->coef_stride; }
+                STAGE(PI_STAGE_DOWN, 1, launch_axpy(a, st, &used));
             }
         }
         pend = Pending();
@@ -772,9 +788,9 @@ int pi_engine_set_trace(pi_engine * e, float * pred_trace) {
 int pi_engine_debug(pi_engine * e, float ** pred, int32_t ** list, int32_t ** count) {
     PI_REQUIRE(e, "engine_debug: null");
     float * p = e->pred_trace ? e->pred_trace + (size_t)(e->c.n_layer - 1) * e->c.max_batch * e->F : e->pred;
-    if (e->rows1 && (list || count)) {
-        // one-token steps make bit masks only: build the list of the last layer's logits (first sequence) here, on the
-        // default stream, after everything queued so far
+    if (list || count) {
+        // steps make bit masks only: build the list of the last layer's logits (first sequence) here, on the default stream,
+        // after everything queued so far
         PI_CUDA(cudaDeviceSynchronize());
         CompactArgs ca;
         ca.idx = p; ca.idx_stride = e->F; ca.T = 1; ca.threshold = e->c.threshold; ca.n_local = e->F;

@@ -283,7 +283,7 @@ static int launch_tt(const GemvP & p, bool sparse, bool gated, size_t smem, cuda
             return launch_inst<WT, 1, false, false, 2, 1>(p, smem, st, pdl);
         return launch_inst<WT, 1, false, false, 1, 2>(p, smem, st, pdl);
     }
-    if (!sparse) return launch_inst<WT, TT, false, false, 1, 1>(p, smem, st, pdl);
+    if (!sparse) { set_error("gemv: matrix too large"); return PI_ERR_UNSUPPORTED; }      // (more than 2^26 rows)
     if (gated)   return launch_inst<WT, TT, true, true, 1, 1>(p, smem, st, pdl);
     return launch_inst<WT, TT, true, false, 1, 1>(p, smem, st, pdl);
 }
@@ -306,9 +306,9 @@ int launch_gemv(const GemvArgs & a, cudaStream_t st) {
     bool wrote = false;
     const int rc = launch_gemv_main(a, st, &wrote);
     if (rc != PI_OK || !a.masks_out || wrote || a.T <= 0 || a.nrows <= 0) return rc;
-    if (a.T != 1 || a.list || a.masks || !a.dst) { set_error("gemv: masks_out needs a dense one-token mat-vec with an F32 result"); return PI_ERR_UNSUPPORTED; }
+    if (a.list || a.masks || !a.dst) { set_error("gemv: masks_out needs a dense mat-vec with an F32 result"); return PI_ERR_UNSUPPORTED; }
     CompactArgs ca;
-    ca.pdl = a.pdl; ca.idx = a.dst; ca.idx_stride = a.dst_stride; ca.T = 1; ca.threshold = a.masks_threshold; ca.n_local = a.nrows;
+    ca.pdl = a.pdl; ca.idx = a.dst; ca.idx_stride = a.dst_stride; ca.T = a.T; ca.threshold = a.masks_threshold; ca.n_local = a.nrows;
     ca.masks = a.masks_out;
     return launch_compact(ca, st);
 }
@@ -320,13 +320,10 @@ static int launch_gemv_main(const GemvArgs & a, cudaStream_t st, bool * wrote_ma
         if (rc != PI_ERR_UNSUPPORTED) return rc;
         if (!a.list) { set_error("gemv: masks given but the shape is not eligible and there is no list"); return PI_ERR_UNSUPPORTED; }
     }
-    if (a.wtype == PI_TYPE_F16 && a.status) {                      // FP16 rows, up to 32 tokens: tensor-core ring kernel
-        const int rc = launch_gemv_mma(a, st);
-        if (rc != PI_ERR_UNSUPPORTED) return rc;
-    }
-    if (a.wtype == PI_TYPE_Q4_0 && a.status && a.T > 1) {          // Q4_0 rows, 2+ tokens: integer tensor-core ring kernel
-        const int rc = launch_gemv_mma_q4(a, st);
-        if (rc != PI_ERR_UNSUPPORTED) return rc;
+    if (a.T > 1) {                                                 // 2+ tokens: tensor-core kernel
+        const int rc = launch_mm(a, st);
+        if (rc != PI_ERR_UNSUPPORTED) { if (wrote_masks) *wrote_masks = a.masks_out != nullptr; return rc; }
+        if (!a.list && a.masks) { set_error("gemv: masks given but the shape is not eligible and there is no list"); return PI_ERR_UNSUPPORTED; }
     }
     if (a.T == 1 && a.status) {
         const int rc = launch_gemv_ring(a, a.status, a.pdl, st, wrote_masks);
@@ -334,7 +331,7 @@ static int launch_gemv_main(const GemvArgs & a, cudaStream_t st, bool * wrote_ma
     }
     const bool q4 = a.wtype == PI_TYPE_Q4_0;
     const int nb = (int)(a.ncols / QK);
-    // tokens are processed in chunks of at most 8 (weights are re-read per chunk; decode batches are <= 32)
+    // (batches come here only with a list of more than MM_MAX_ROWS neurons: chunks of at most 8 tokens, weights re-read per chunk)
     for (int t0 = 0; t0 < a.T; ) {
         const int left = a.T - t0;
         const int tt = left >= 8 ? 8 : (left >= 4 ? 4 : (left >= 2 ? 2 : 1));

@@ -11,7 +11,8 @@ static constexpr int QK = 32;
 // __ballot_sync gives the 32-bit activity mask of the chunk.  Phase B (the CTA that finishes last, found with a
 // ticket counter): exclusive scan of popc(mask) over the chunks and expansion into a SORTED list of local rows.
 // No CTA ever waits for another one.  The ticket counter is left at zero for the next launch.
-static constexpr int COMPACT_THREADS = 256;
+static constexpr int COMPACT_THREADS = 512;
+static constexpr int COMPACT_TOK = 8;                 // logits of that many tokens in flight per lane
 
 struct CompactP {
     const float * idx; int64_t idx_stride; int T; float threshold;
@@ -39,10 +40,17 @@ __global__ void __launch_bounds__(COMPACT_THREADS) k_compact(const CompactP p) {
             const int64_t g = p.bucket ? p.bucket[r] : r;
             float fill = 0.f;
             if (p.zero_dst && p.fill_bias) { fill = p.fill_bias[g]; if (p.fill_relu) fill = fmaxf(fill, 0.f); }
-            for (int t = 0; t < p.T; t++) {
-                const bool a = !(p.idx[(size_t)t * p.idx_stride + g] < p.threshold);   // the reference skips on `<`: a NaN logit counts as active
-                any |= a;
-                if (p.zero_dst && !a) p.zero_dst[(size_t)t * p.zero_stride + g] = fill;
+            for (int t0 = 0; t0 < p.T; t0 += COMPACT_TOK) {         // loads first: the stores below may alias them for the compiler
+                float l[COMPACT_TOK];
+#pragma unroll
+                for (int u = 0; u < COMPACT_TOK; u++) if (t0 + u < p.T) l[u] = p.idx[(size_t)(t0 + u) * p.idx_stride + g];
+#pragma unroll
+                for (int u = 0; u < COMPACT_TOK; u++) {
+                    if (t0 + u >= p.T) break;
+                    const bool a = !(l[u] < p.threshold);           // the reference skips on `<`: a NaN logit counts as active
+                    any |= a;
+                    if (p.zero_dst && !a) p.zero_dst[(size_t)(t0 + u) * p.zero_stride + g] = fill;
+                }
             }
         }
         const uint32_t m = __ballot_sync(0xffffffffu, any);
@@ -289,46 +297,30 @@ int launch_axpy(const AxpyArgs & a, cudaStream_t st, int * groups_used) {
         if (!a.list) { set_error("axpy: masks given but the shape is not eligible and there is no list"); return PI_ERR_UNSUPPORTED; }
         if (groups_used) *groups_used = a.n_groups;
     }
-    if (a.T > 1 && a.status) {                                      // 2..32 tokens: tensor-core kernels
-        const int rc = launch_axpy_mma(a, st, groups_used);
+    if (a.T > 1 && a.coef) {                                        // 2+ tokens: tensor-core kernel
+        const int rc = launch_axpy_mm(a, st, groups_used);
         if (rc != PI_ERR_UNSUPPORTED) return rc;
         if (groups_used) *groups_used = a.n_groups;
     }
-    // CUDA-core kernels for what the kernels above decline.  Q4_0 rows read the coefficient planes (int8 quant of h per
-    // 32 neurons, block scale); callers fill them for batches, a single token gets them here.
-    if (q4 && a.T == 1) {
+    // CUDA-core kernels for the one-token shapes the kernel above declines.  Q4_0 rows read coefficient planes (int8 quant of
+    // h per 32 neurons, block scale).
+    if (q4) {
         PI_REQUIRE(a.cq && a.cd, "axpy: Q4_0 needs coefficient planes");
         const int rc = launch_neuron_q8(a.h, a.h_stride, a.h_stride, 1, const_cast<int8_t *>(a.cq), const_cast<float *>(a.cd), st);
         if (rc) return rc;
     }
+    if (a.T != 1) { set_error("axpy: %d tokens need coefficients by list position", a.T); return PI_ERR_UNSUPPORTED; }
     AxpyP p;
     p.Wt = (const uint8_t *)a.Wt; p.row_bytes = (int64_t)pi_row_bytes(a.wtype, a.ncols);
     p.nrows = (int)a.nrows; p.ncols = (int)a.ncols; p.nb = (int)(a.ncols / QK);
     p.h_stride = a.h_stride; p.list = a.list; p.count = a.count; p.bucket = a.bucket;
-    p.idx_stride = a.idx_stride; p.threshold = a.threshold; p.c_stride = a.c_stride; p.T = a.T;
+    p.idx_stride = a.idx_stride; p.threshold = a.threshold; p.c_stride = a.c_stride; p.T = 1;
+    p.h = a.h; p.idx = a.idx; p.cq = a.cq; p.cd = a.cd; p.partial = a.partial;
     const int tiles = q4 ? (p.nb + AXPY_Q4_THREADS - 1) / AXPY_Q4_THREADS : (p.ncols / 8 + AXPY_F16_THREADS - 1) / AXPY_F16_THREADS;
     const dim3 grid(tiles, a.n_groups);
-    const int max_tt = q4 ? 2 : 4;                                      // register budget: 32 (8) sums per token
-    for (int t0 = 0; t0 < a.T; ) {
-        const int left = a.T - t0;
-        int tt = 1;
-        while (tt * 2 <= left && tt * 2 <= max_tt) tt *= 2;
-        p.h = a.h ? a.h + (size_t)t0 * a.h_stride : nullptr;
-        p.idx = a.idx + (size_t)t0 * a.idx_stride;
-        p.cq = a.cq ? a.cq + (size_t)t0 * a.c_stride : nullptr;
-        p.cd = a.cd ? a.cd + (size_t)t0 * (a.c_stride / QK) : nullptr;
-        p.partial = a.partial + (size_t)t0 * a.ncols;                   // token t of group j lives at [j, t, :]
-        if (q4) {
-            if (tt == 2) k_axpy_q4<2><<<grid, AXPY_Q4_THREADS, 0, st>>>(p);
-            else         k_axpy_q4<1><<<grid, AXPY_Q4_THREADS, 0, st>>>(p);
-        } else {
-            if (tt == 4)      k_axpy_f16<4><<<grid, AXPY_F16_THREADS, 0, st>>>(p);
-            else if (tt == 2) k_axpy_f16<2><<<grid, AXPY_F16_THREADS, 0, st>>>(p);
-            else              k_axpy_f16<1><<<grid, AXPY_F16_THREADS, 0, st>>>(p);
-        }
-        PI_LAUNCH_CHECK("k_axpy");
-        t0 += tt;
-    }
+    if (q4) k_axpy_q4<1><<<grid, AXPY_Q4_THREADS, 0, st>>>(p);
+    else    k_axpy_f16<1><<<grid, AXPY_F16_THREADS, 0, st>>>(p);
+    PI_LAUNCH_CHECK("k_axpy");
     return PI_OK;
 }
 
