@@ -1,0 +1,305 @@
+// llm_build_kv_store + llm_build_kqv (llama.cpp:4383-4418, 4764-4850) for several tokens of a step, on the tensor cores.
+//
+// A CTA takes 16 query rows that read the same keys and values: the query heads that share a KV head, of one token (a batch of
+// sequences), or 16 consecutive tokens of one head (a prompt chunk).  The kernel with one CTA per (head, token) reads a KV
+// head once for every query head and token and keeps one CTA per SM: 57 us for 32 sequences of 190 positions with 32 heads
+// (92 MB of keys and values), 125 us for 32 prompt tokens with 64 heads.
+//
+// Bound: the bytes of the cached rows for batches, the chain scores -> maximum -> probabilities -> values for chunks.
+// Scores: mma.m16n8k16 with the keys straight from global memory: a lane loads 16 bytes (8 columns) of a row, which serve
+// as B operands of two mma whose k order is permuted in the same way on the query side; four tiles of 8 positions in
+// flight per warp.  Values travel to shared memory by cp.async (tiles of 64 positions, two in flight) while the scores are made and
+// are read transposed.  Every CTA rotates and stores the new keys and values it reads itself (CTAs that share a KV head store the
+// same bits), so no store pass runs before a chunk.
+// Numerics follow the CPU path as in k_attention: q, k, v and the probabilities in FP16, exp through FP16, the normaliser
+// summed in double.
+#include "pi_act.cuh"
+
+namespace pi {
+
+static constexpr int AM_THREADS = 256, AM_WARPS = 8, AM_VT = 64;      // positions of a value tile
+
+struct AttnMmP {
+    const float * q; const float * k; const float * v; __half * k_cache; __half * v_cache;
+    const int32_t * seq; const int32_t * pos; int T, n_head, n_head_kv, n_ctx;
+    const float * cs; int neox; int64_t q_stride, kv_stride;
+    float * out; ActBuf out_act; int out_act_type;
+    int chunk;                                                        // rows are tokens of one head, else heads of one token
+    int P, R;                                                         // positions (a multiple of 64) and rows that shared memory holds
+};
+
+__device__ __forceinline__ void am_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+template <int HC>                                                     // head_dim / 32
+__global__ void __launch_bounds__(AM_THREADS) k_attention_mm(const AttnMmP p) {
+    constexpr int HD = HC * 32, HALF = HD / 2;
+    constexpr int V_PITCH = HD + 8, Q_PITCH = HD + 8;                 // halves; odd multiples of 16 bytes
+    constexpr int NWC = HD / 16 < AM_WARPS ? HD / 16 : AM_WARPS;      // warps along the value columns, the rest split the positions
+    constexpr int KSPL = AM_WARPS / NWC, NCG = HD / 16 / NWC;         // column groups of 16 per warp
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ int s_pos[16];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+    const int group = p.n_head / p.n_head_kv, dkv = p.n_head_kv * HD;
+    // shared-memory map: scores [R][P + 4] F32 (later the output sums) | probabilities [R][P + 8] FP16 | queries [16][Q_PITCH] | values 2 x [64][V_PITCH]
+    const int S_PITCH = p.P + 4, P_PITCH = p.P + 8;
+    float * sc = reinterpret_cast<float *>(smem);
+    const size_t s_bytes = (size_t)max(p.R * S_PITCH * 4, KSPL * 16 * HD * 4);
+    __half * p16 = reinterpret_cast<__half *>(smem + (s_bytes + 127) / 128 * 128);
+    __half * qs = reinterpret_cast<__half *>(reinterpret_cast<unsigned char *>(p16) + ((size_t)p.R * P_PITCH * 2 + 127) / 128 * 128);
+    __half * vs = qs + 16 * Q_PITCH;
+
+    pdl_launch();
+    // ---- before the wait: positions, and L2 hints for the cached rows (earlier steps wrote them)
+    int t0, n_rows, head0, hk;
+    if (p.chunk) {
+        head0 = blockIdx.x; hk = head0 / group; t0 = blockIdx.y * 16; n_rows = min(16, p.T - t0);
+    } else {
+        const int ng = (group + 15) / 16, gi = blockIdx.x % ng;
+        hk = blockIdx.x / ng; head0 = hk * group + gi * 16; t0 = blockIdx.y; n_rows = min(16, group - gi * 16);
+    }
+    const int sq = p.seq ? p.seq[t0] : 0;
+    __half * kc = p.k_cache + ((size_t)sq * p.n_ctx * p.n_head_kv + hk) * HD;
+    __half * vc = p.v_cache + ((size_t)sq * p.n_ctx * p.n_head_kv + hk) * HD;
+    // tokens whose new keys and values this CTA stores: its own, or all of the chunk up to its last
+    const int s_lo = p.chunk ? 0 : t0, s_n = p.chunk ? t0 + n_rows : 1;
+    int n_keys = 0;                                                   // keys that any row sees
+    for (int r = 0; r < (p.chunk ? n_rows : 1); r++) { const int ps = p.pos[t0 + r]; if (ps >= 0 && ps < p.n_ctx) n_keys = max(n_keys, ps + 1); }
+    if (n_keys == 0) return;                                          // never index the cache out of range
+    if (tid < 16) {
+        const int ps = tid < n_rows ? p.pos[p.chunk ? t0 + tid : t0] : -1;
+        s_pos[tid] = ps < p.n_ctx ? ps : -1;
+    }
+    for (int j = tid; j < n_keys; j += AM_THREADS) {
+        const char * kr = reinterpret_cast<const char *>(kc + (size_t)j * dkv), * vr = reinterpret_cast<const char *>(vc + (size_t)j * dkv);
+#pragma unroll
+        for (int o = 0; o < HD * 2; o += 128) {
+            asm volatile("prefetch.global.L2 [%0];" :: "l"(kr + o));
+            asm volatile("prefetch.global.L2 [%0];" :: "l"(vr + o));
+        }
+    }
+    pdl_wait();
+
+    // ---- queries (rotated, FP16) to shared memory; the new keys and values to the cache
+    for (int e = tid; e < 16 * HALF; e += AM_THREADS) {
+        const int r = e / HALF, k = e % HALF;
+        const int t = p.chunk ? t0 + r : t0, h = p.chunk ? head0 : head0 + r;
+        const int i0 = p.cs && !p.neox ? 2 * k : k, i1 = p.cs && !p.neox ? 2 * k + 1 : k + HALF;
+        float o0 = 0.f, o1 = 0.f;
+        if (r < n_rows) {
+            const float * qh = p.q + (size_t)t * p.q_stride + (size_t)h * HD;
+            o0 = qh[i0]; o1 = qh[i1];
+            const int ps = p.pos[t];
+            if (p.cs && ps >= 0 && ps < p.n_ctx) {
+                const float2 a = reinterpret_cast<const float2 *>(p.cs)[(size_t)ps * HALF + k];
+                rope_pair(qh[i0], qh[i1], a.x, a.y, o0, o1);
+            }
+        }
+        qs[r * Q_PITCH + i0] = __float2half_rn(o0);
+        qs[r * Q_PITCH + i1] = __float2half_rn(o1);
+    }
+    for (int e = tid; e < s_n * HALF; e += AM_THREADS) {
+        const int t = s_lo + e / HALF, k = e % HALF, ps = p.pos[t];
+        if (ps < 0 || ps >= p.n_ctx) continue;
+        const float * kh = p.k + (size_t)t * p.kv_stride + (size_t)hk * HD, * vh = p.v + (size_t)t * p.kv_stride + (size_t)hk * HD;
+        const int i0 = p.cs && !p.neox ? 2 * k : k, i1 = p.cs && !p.neox ? 2 * k + 1 : k + HALF;
+        float o0 = kh[i0], o1 = kh[i1];
+        if (p.cs) {
+            const float2 a = reinterpret_cast<const float2 *>(p.cs)[(size_t)ps * HALF + k];
+            rope_pair(kh[i0], kh[i1], a.x, a.y, o0, o1);
+        }
+        kc[(size_t)ps * dkv + i0] = __float2half_rn(o0);
+        kc[(size_t)ps * dkv + i1] = __float2half_rn(o1);
+        vc[(size_t)ps * dkv + k] = __float2half_rn(vh[k]);
+        vc[(size_t)ps * dkv + k + HALF] = __float2half_rn(vh[k + HALF]);
+    }
+    __syncthreads();                                                  // this CTA's stores are visible to all of its threads
+
+    auto issue_v = [&](int tile) {
+        const uint32_t base = smem_u32(vs + (size_t)(tile & 1) * AM_VT * V_PITCH);
+        for (int e = tid; e < AM_VT * (HD / 8); e += AM_THREADS) {
+            const int r = e / (HD / 8), c = e % (HD / 8), j = tile * AM_VT + r;
+            const bool in = j < n_keys;                               // rows past the last key: zeros (their probabilities are 0)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(base + (uint32_t)(r * V_PITCH + c * 8) * 2), "l"(vc + (size_t)(in ? j : 0) * dkv + c * 8), "r"(in ? 16u : 0u) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int n_vt = (n_keys + AM_VT - 1) / AM_VT;
+    issue_v(0);
+    if (n_vt > 1) issue_v(1);
+
+    // ---- scores
+    {
+        uint32_t aq[HC][2][4];                                        // 8 columns of rows g and g + 8 per 32
+#pragma unroll
+        for (int c = 0; c < HC; c++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint4 v = *reinterpret_cast<const uint4 *>(qs + (g + 8 * h) * Q_PITCH + c * 32 + q * 8);
+                aq[c][h][0] = v.x; aq[c][h][1] = v.y; aq[c][h][2] = v.z; aq[c][h][3] = v.w;
+            }
+        const float scale = 1.0f / sqrtf((float)HD);
+        const int n_tiles = (n_keys + 7) / 8;
+        constexpr int UN = HC <= 4 ? 4 : 2;                           // tiles of 8 positions in flight
+        for (int nt0 = warp; nt0 < n_tiles; nt0 += AM_WARPS * UN) {
+            uint4 kv[UN][HC];
+#pragma unroll
+            for (int u = 0; u < UN; u++) {
+                const int j = min((nt0 + u * AM_WARPS) * 8 + g, n_keys - 1);
+#pragma unroll
+                for (int c = 0; c < HC; c++) kv[u][c] = __ldcg(reinterpret_cast<const uint4 *>(kc + (size_t)j * dkv + c * 32 + q * 8));
+            }
+#pragma unroll
+            for (int u = 0; u < UN; u++) {
+                const int nt = nt0 + u * AM_WARPS;
+                if (nt >= n_tiles) break;
+                float c4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int c = 0; c < HC; c++) {
+                    am_mma(c4, aq[c][0][0], aq[c][1][0], aq[c][0][1], aq[c][1][1], kv[u][c].x, kv[u][c].y);
+                    am_mma(c4, aq[c][0][2], aq[c][1][2], aq[c][0][3], aq[c][1][3], kv[u][c].z, kv[u][c].w);
+                }
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int r = g + 8 * h, j = nt * 8 + 2 * q;
+                    if (r >= p.R) continue;
+                    const int last = s_pos[r];
+                    sc[r * S_PITCH + j]     = j     <= last ? c4[2 * h] * scale     : -INFINITY;
+                    sc[r * S_PITCH + j + 1] = j + 1 <= last ? c4[2 * h + 1] * scale : -INFINITY;
+                }
+            }
+        }
+    }
+    __syncthreads();
+
+    // ---- softmax (ggml.c:10708-10777), a warp per row
+    const int k_end = (n_keys + 15) / 16 * 16;
+    for (int r = warp; r < p.R; r += AM_WARPS) {
+        const int last = s_pos[r];
+        float * row = sc + r * S_PITCH;
+        float mx = -INFINITY;
+        for (int j = lane; j <= last; j += 32) mx = fmaxf(mx, row[j]);
+        mx = warp_max(mx);
+        double part = 0.0;
+        for (int j = lane; j <= last; j += 32) {
+            const float e = round_f16(expf(round_f16(row[j] - mx)));
+            row[j] = e;
+            part += (double)e;
+        }
+        const float inv = (float)(1.0 / warp_sum_d(part));
+        for (int j = lane; j < k_end; j += 32) p16[r * P_PITCH + j] = __float2half_rn(j <= last ? row[j] * inv : 0.f);
+    }
+
+    // ---- values
+    float acc[NCG][2][4];
+#pragma unroll
+    for (int cg = 0; cg < NCG; cg++)
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc[cg][m][j] = 0.f;
+    const int wc = warp % NWC, wk = warp / NWC;
+    const int r0 = min(g, p.R - 1), r1 = min(g + 8, p.R - 1);         // (fragment rows beyond R repeat the last one and are dropped)
+    for (int tile = 0; tile < n_vt; tile++) {
+        if (tile + 1 < n_vt) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else                 asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                                              // the tile has landed for everybody (first time: the probabilities too)
+        const uint32_t base = smem_u32(vs + (size_t)(tile & 1) * AM_VT * V_PITCH);
+        for (int ks = wk; ks < AM_VT / 16; ks += KSPL) {
+            const int j = tile * AM_VT + ks * 16;
+            if (j >= k_end) break;
+            const uint32_t a0 = *reinterpret_cast<const uint32_t *>(p16 + r0 * P_PITCH + j + 2 * q), a1 = *reinterpret_cast<const uint32_t *>(p16 + r1 * P_PITCH + j + 2 * q);
+            const uint32_t a2 = *reinterpret_cast<const uint32_t *>(p16 + r0 * P_PITCH + j + 2 * q + 8), a3 = *reinterpret_cast<const uint32_t *>(p16 + r1 * P_PITCH + j + 2 * q + 8);
+#pragma unroll
+            for (int cg = 0; cg < NCG; cg++) {
+                const int col = (cg * NWC + wc) * 16;
+                uint32_t b[4];
+                asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3])
+                             : "r"(base + (uint32_t)((ks * 16 + (lane & 15)) * V_PITCH + col + (lane >> 4) * 8) * 2));
+                am_mma(acc[cg][0], a0, a1, a2, a3, b[0], b[1]);
+                am_mma(acc[cg][1], a0, a1, a2, a3, b[2], b[3]);
+            }
+        }
+        if (tile + 2 < n_vt) { __syncthreads(); issue_v(tile + 2); }
+    }
+    // ---- the output rows (scores are dead: their place takes the sums of each position share)
+    float * o = sc;
+#pragma unroll
+    for (int cg = 0; cg < NCG; cg++)
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) o[(wk * 16 + g + (j >> 1) * 8) * HD + (cg * NWC + wc) * 16 + m * 8 + 2 * q + (j & 1)] = acc[cg][m][j];
+    __syncthreads();
+    for (int r = warp; r < n_rows; r += AM_WARPS) {
+        if (s_pos[r] < 0) continue;
+        const int t = p.chunk ? t0 + r : t0, h = p.chunk ? head0 : head0 + r;
+        float y[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            y[j] = 0.f;
+            if (lane < HD / 8) {
+                y[j] = o[r * HD + lane * 8 + j];
+                if (KSPL > 1) y[j] += o[(16 + r) * HD + lane * 8 + j];
+                if (KSPL > 2) { y[j] += o[(32 + r) * HD + lane * 8 + j]; y[j] += o[(48 + r) * HD + lane * 8 + j]; }
+            }
+        }
+        if (p.out && lane < HD / 8) {
+            float * d = p.out + ((size_t)t * p.n_head + h) * HD + lane * 8;
+            *reinterpret_cast<float4 *>(d) = make_float4(y[0], y[1], y[2], y[3]);
+            *reinterpret_cast<float4 *>(d + 4) = make_float4(y[4], y[5], y[6], y[7]);
+        }
+        if (p.out_act_type) emit_act8(p.out_act_type, p.out_act, t, (int64_t)p.n_head * HD, h * (HD / 8) + lane, y, lane < HD / 8);
+    }
+}
+
+static constexpr size_t AM_SMEM_MAX = 220 * 1024;
+
+// rows and positions that shared memory holds, and its size
+static size_t attn_mm_smem(const AttnArgs & a, int * P, int * R) {
+    const int hd = a.head_dim, group = a.n_head / a.n_head_kv;
+    const int nwc = hd / 16 < AM_WARPS ? hd / 16 : AM_WARPS, kspl = AM_WARPS / nwc;
+    *P = (a.n_ctx + 63) / 64 * 64;
+    *R = a.store_mode != 0 || group > 16 ? 16 : group;
+    auto up = [](size_t v) { return (v + 127) / 128 * 128; };
+    const size_t scores = (size_t)*R * (*P + 4) * 4, sums = (size_t)kspl * 16 * hd * 4;
+    return up(scores > sums ? scores : sums) + up((size_t)*R * (*P + 8) * 2) + (size_t)16 * (hd + 8) * 2 + (size_t)2 * AM_VT * (hd + 8) * 2;
+}
+
+// Several tokens and head_dim 64 or 128 whose scores fit (16 rows: contexts of up to about 1900 positions); the others keep one
+// CTA per head and token.
+bool attention_mm_takes(const AttnArgs & a) {
+    int P, R;
+    return a.T >= 2 && (a.head_dim == 64 || a.head_dim == 128) && a.n_ctx > 0 && attn_mm_smem(a, &P, &R) <= AM_SMEM_MAX;
+}
+
+template <int HC>
+static int attn_mm_go(const AttnMmP & p, dim3 grid, size_t smem, bool pdl, cudaStream_t st) {
+    static bool attr_done[16] = {false};
+    int dev = 0;
+    PI_CUDA(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 16 && !attr_done[dev]) {
+        PI_CUDA(cudaFuncSetAttribute(k_attention_mm<HC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AM_SMEM_MAX));
+        attr_done[dev] = true;
+    }
+    PI_CUDA(launch_k(k_attention_mm<HC>, grid, dim3(AM_THREADS), smem, st, pdl, p));
+    return PI_OK;
+}
+
+int launch_attention_mm(const AttnArgs & a, cudaStream_t st) {
+    if (!attention_mm_takes(a)) return PI_ERR_UNSUPPORTED;
+    AttnMmP p;
+    p.q = a.q; p.k = a.k; p.v = a.v; p.k_cache = a.k_cache; p.v_cache = a.v_cache; p.seq = a.seq; p.pos = a.pos; p.T = a.T;
+    p.n_head = a.n_head; p.n_head_kv = a.n_head_kv; p.n_ctx = a.n_ctx; p.cs = a.cs; p.neox = a.neox;
+    p.q_stride = a.q_stride ? a.q_stride : (int64_t)a.n_head * a.head_dim;
+    p.kv_stride = a.kv_stride ? a.kv_stride : (int64_t)a.n_head_kv * a.head_dim;
+    p.out = a.out; p.out_act = a.out_act; p.out_act_type = a.out_act_type;
+    p.chunk = a.store_mode != 0;
+    const size_t smem = attn_mm_smem(a, &p.P, &p.R);
+    const dim3 grid = p.chunk ? dim3(a.n_head, (a.T + 15) / 16) : dim3(a.n_head_kv * ((a.n_head / a.n_head_kv + 15) / 16), a.T);
+    return a.head_dim == 64 ? attn_mm_go<2>(p, grid, smem, a.pdl, st) : attn_mm_go<4>(p, grid, smem, a.pdl, st);
+}
+
+}  // namespace pi

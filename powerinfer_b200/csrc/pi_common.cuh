@@ -251,6 +251,9 @@ struct AttnArgs {
     bool pdl = false;
 };
 int launch_attention(const AttnArgs & a, cudaStream_t st);
+// 2+ tokens on the tensor cores (pi_attn_mm.cu), a chunk's store pass included: store_mode 2 alone is enough where it takes the shape
+int launch_attention_mm(const AttnArgs & a, cudaStream_t st);
+bool attention_mm_takes(const AttnArgs & a);
 
 // ------------------------------------------------------------------------------------ device primitives
 #ifdef __CUDACC__

@@ -1,13 +1,11 @@
 // Dense decode nodes between the sparse operators: normalisation (with the residual / partial-sum reduction that
 // precedes it fused in), RoPE, KV store and one-token attention.  All are latency-bound at batch 1; they exist to
 // keep the residual stream on the device and to hand the next mat-vec its input already in FP16 / Q8_0 form.
-#include "pi_common.cuh"
+#include "pi_act.cuh"
 
 #include <cstdlib>
 
 namespace pi {
-
-static constexpr int QK = 32;
 
 // ------------------------------------------------------------------------------------------------
 // llm_build_norm (llama.cpp:4420-4450) = ggml_rms_norm | ggml_norm, * weight, + bias, with the CPU path's numerics
@@ -37,43 +35,6 @@ __device__ __forceinline__ double block_sum_d(double v, double * s_red) {
     double t = 0.0;
     for (int i = 0; i < nw; i++) t += s_red[i];
     return t;
-}
-
-// Emit 8 consecutive values (chunk index c8 = first column / 8) of token t as activation planes.
-// Must be called by every lane of a warp (it shuffles); `valid` gates the stores.  With n % 32 == 0 the 4 lanes that
-// share a Q8 block are valid or invalid together.
-__device__ __forceinline__ void emit_act8(int type, const ActBuf & a, int t, int64_t n, int c8, const float (&v)[8], bool valid) {
-    if (type == PI_TYPE_F16) {
-        if (!valid) return;
-        __half2 h[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) h[j] = __floats2half2_rn(v[2 * j], v[2 * j + 1]);
-        *reinterpret_cast<uint4 *>(a.h16 + (size_t)t * n + (size_t)c8 * 8) = *reinterpret_cast<uint4 *>(h);
-    } else if (type == PI_TYPE_Q4_0) {
-        // 4 consecutive threads (lanes 4k..4k+3) hold one block of 32 values
-        float amax = 0.f;
-#pragma unroll
-        for (int j = 0; j < 8; j++) amax = fmaxf(amax, fabsf(v[j]));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-        const float d  = amax / 127.0f;
-        const float id = amax != 0.0f ? 127.0f / amax : 0.0f;
-        int q[8], s = 0;
-#pragma unroll
-        for (int j = 0; j < 8; j++) { q[j] = __float2int_rn(v[j] * id); s += q[j]; }
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        const int nb = (int)(n / QK);
-        const size_t blk = (size_t)t * nb + (c8 >> 2);
-        const int part = c8 & 3;                                  // which 8 of the 32
-        uint2 packed;
-        packed.x = (uint32_t)(q[0] & 0xFF) | ((uint32_t)(q[1] & 0xFF) << 8) | ((uint32_t)(q[2] & 0xFF) << 16) | ((uint32_t)(q[3] & 0xFF) << 24);
-        packed.y = (uint32_t)(q[4] & 0xFF) | ((uint32_t)(q[5] & 0xFF) << 8) | ((uint32_t)(q[6] & 0xFF) << 16) | ((uint32_t)(q[7] & 0xFF) << 24);
-        if (!valid) return;
-        uint2 * plane = reinterpret_cast<uint2 *>(part < 2 ? a.lo + blk : a.hi + blk);
-        plane[part & 1] = packed;
-        if (part == 0) { a.d[blk] = __half2float(__float2half_rn(d)); a.s[blk] = s; }
-    }
 }
 
 // MAXT = the launch bound: 512 threads cover n <= 8192 with registers to spare for the weights, 1024 cover n <= 16384
@@ -477,11 +438,6 @@ int launch_norm(const NormArgs & a, cudaStream_t st) {
 // ------------------------------------------------------------------------------------------------
 // ggml_rope_custom, modes 0 and 2 (ggml.c:11163-11325), angles from a host-built table so that device and CPU path
 // rotate by the same float cos / sin.  Products and sums are rounded separately, as the CPU build does.
-__device__ __forceinline__ void rope_pair(float x0, float x1, float c, float s, float & o0, float & o1) {
-    o0 = __fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s));
-    o1 = __fadd_rn(__fmul_rn(x0, s), __fmul_rn(x1, c));
-}
-
 __global__ void k_rope(float * __restrict__ x, int n_heads, int head_dim, const int32_t * __restrict__ pos,
                        const float * __restrict__ cs, int neox) {
     const int t = blockIdx.y;
@@ -743,6 +699,7 @@ int launch_attention(const AttnArgs & a, cudaStream_t st) {
     if (a.T <= 0) return PI_OK;
     PI_REQUIRE(a.head_dim % 32 == 0 && a.head_dim <= 256, "attention: head_dim=%d must be a multiple of 32, <= 256", a.head_dim);
     PI_REQUIRE(a.n_head % a.n_head_kv == 0, "attention: n_head %% n_head_kv != 0");
+    if (attention_mm_takes(a)) return launch_attention_mm(a, st);      // several tokens: the tensor-core kernel where it takes the shape
     AttnP p;
     p.q = a.q; p.k = a.k; p.v = a.v; p.k_cache = a.k_cache; p.v_cache = a.v_cache; p.seq = a.seq; p.pos = a.pos;
     p.n_head = a.n_head; p.n_head_kv = a.n_head_kv; p.hd = a.head_dim; p.n_ctx = a.n_ctx;

@@ -474,7 +474,7 @@ int enqueue_step(pi_engine * e, int T, cudaStream_t st, StageTimer & tm, int mod
             a.out_act_type = wt; a.out_act = e->act_o;
             if (mode) {                                                   // prompt chunk: every token's K / V first, then attention
                 a.store_mode = 1;
-                STAGE(PI_STAGE_ATTN, 1, launch_attention(a, st));
+                if (!attention_mm_takes(a)) STAGE(PI_STAGE_ATTN, 1, launch_attention(a, st));
                 a.store_mode = 2;
             }
             STAGE(PI_STAGE_ATTN, 1, launch_attention(a, st));
