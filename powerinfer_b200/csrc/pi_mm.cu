@@ -16,9 +16,13 @@
 // KB of masks itself and takes the rows of its ranks, so no list has to be built first; it leaves its part of the list behind
 // for the axpy.  A dense product can write such masks (the predictor's second matrix does): no mask kernel in between.
 //
-// Inside a CTA 16 warps share a stage: TM / 32 groups of 32 rows, the others split the stage's columns; their sums meet in
-// shared memory at the end of a tile, in warp order.  Rows arrive by 16-byte cp.async from all threads: the rows of the active
-// list lie anywhere, and pieces of a few hundred bytes are too small for the bulk-copy engine (about 80 ns per copy).
+// Inside a CTA the 8 warps split the COLUMNS: a warp takes every eighth slice of 64 bytes of all rows of the tile, and the activation
+// of that slice, through a ring of its own.  Nothing is shared while a tile lasts: a warp waits for its own copies only, and there is
+// no barrier between the first slice and the last, where the 8 partial tiles meet in shared memory and are added in warp order.
+// (16 warps that shared a stage met in a barrier for each: 1900 clocks a stage, whatever it held.)
+// Rows arrive by 16-byte cp.async: the rows of the active list lie anywhere, and pieces of a few hundred bytes are too small for the
+// bulk-copy engine (about 80 ns per copy).  A row slice of 64 bytes is stored with its four 16-byte pieces permuted by
+// (row / 2) % 4, so that the eight rows of an 8x8 fragment lie in different banks without padding.
 // Dense weights do not depend on the kernel before: their first stages are requested before griddepcontrol.wait.
 //
 // Q4_0 arithmetic: a nibble q is placed in the high half of a byte and its top bit flipped, which is the int8 value
@@ -29,9 +33,9 @@
 
 namespace pi {
 
-static constexpr int MM_THREADS = 512, MM_WARPS = 16;
-static constexpr int MM_RED_PITCH = 36;                 // floats between tokens of a warp's sums: conflict-free fragment stores
-static constexpr size_t MM_SMEM_MAX = 226 * 1024;       // (leaves room for the static variables)
+static constexpr int MM_WARPS = 16, MM_THREADS = MM_WARPS * 32, MM_PAIRS = MM_WARPS / 2;
+static constexpr int MM_SMAX = 8;                       // stages of a ring at most
+static constexpr int MM_SMEM_MAX = 226 * 1024;          // (leaves room for the static variables)
 
 struct MmP {
     const uint8_t * W; const uint8_t * W2; int64_t row_bytes; int nrows, ncols, nb;
@@ -42,29 +46,40 @@ struct MmP {
     float * dst; __half * dst16; int64_t dst_stride;
     __half * coef; int64_t coef_stride;
     uint32_t * masks_out; float masks_threshold; int masks_or;
-    int n_slices, max_rows;
+    int n_slices, ring;                                               // slices of 64 bytes of a row; bytes of a warp's ring
 };
 
-__device__ __forceinline__ void mm_cp16(uint32_t dst, const void * src, unsigned bytes) {       // the first `bytes` bytes, the rest zeros
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(bytes) : "memory");
+__device__ __forceinline__ void mm_cp16(uint32_t dst, const void * src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ void mm_cp4(uint32_t dst, const void * src, unsigned bytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" :: "r"(dst), "l"(src), "r"(bytes) : "memory");
+__device__ __forceinline__ void mm_zero16(uint32_t dst) { asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" :: "r"(dst), "r"(0u) : "memory"); }
+__device__ __forceinline__ void mm_cp4(uint32_t dst, const void * src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void mm_cp8(uint32_t dst, const void * src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" :: "r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void mm_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void mm_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
+__device__ __forceinline__ void mm_wait(int pending) {                // all but the last `pending` (0 .. MM_SMAX - 2) groups have landed
+    switch (pending) {
+        case 0: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
+        case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
+        case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+        case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
+        case 4: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
+        case 5: asm volatile("cp.async.wait_group 5;" ::: "memory"); break;
+        default: asm volatile("cp.async.wait_group 6;" ::: "memory"); break;
+    }
+}
 __device__ __forceinline__ void mm_ldsm4(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
-__device__ __forceinline__ void mm_ldsm2(uint32_t & r0, uint32_t & r1, uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
-}
 __device__ __forceinline__ void mm_hmma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ void mm_imma(uint32_t (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1, uint32_t c) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
                  : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(c));
 }
 __device__ __forceinline__ unsigned long long mm_pack(float a, float b) {
@@ -77,178 +92,164 @@ __device__ __forceinline__ unsigned long long mm_packu(uint32_t a, uint32_t b) {
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
     return r;
 }
-// acc += (v - magic) * dd * d4, two tokens at a time (each lane of the pair rounds like the scalar operation)
-__device__ __forceinline__ void mm_scale_add(unsigned long long & acc, unsigned long long v, unsigned long long neg_magic, unsigned long long dd, unsigned long long d4) {
-    asm("{\n .reg .b64 t;\n add.rn.f32x2 t, %1, %2;\n mul.rn.f32x2 t, t, %3;\n fma.rn.f32x2 %0, t, %4, %0;\n}" : "+l"(acc) : "l"(v), "l"(neg_magic), "l"(dd), "l"(d4));
+__device__ __forceinline__ unsigned long long mm_mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// acc += (v * dd - magic * dd) * d4, two tokens at a time.  The first factor is (v - magic) * dd rounded once: dd holds 11 bits
+// (an FP16 number), so magic * dd = 1.5 * 2^23 * dd is exact.
+__device__ __forceinline__ void mm_scale_add(unsigned long long & acc, unsigned long long v, unsigned long long dd, unsigned long long md, unsigned long long d4) {
+    asm("{\n .reg .b64 t;\n fma.rn.f32x2 t, %1, %2, %3;\n fma.rn.f32x2 %0, t, %4, %0;\n}" : "+l"(acc) : "l"(v), "l"(dd), "l"(md), "l"(d4));
 }
 
-template <int WT, int NT, int TM>
+template <int WT, int NT>
 struct MmShape {
     static constexpr bool Q4 = WT == PI_TYPE_Q4_0;
     static constexpr int TP = NT * 8;                                 // token rows of a stage
-    static constexpr int WM = TM / 32, WK = MM_WARPS / WM;            // warps along the rows, along the columns
-    static constexpr int KPW = Q4 ? 2 : ((TM < 128 && NT == 4) || (TM == 32 && NT == 2) ? 1 : 2);   // 16-column steps (32-column blocks) of a warp per stage
-    static constexpr int NBS = KPW * WK;                              // steps / blocks of a stage
-    static constexpr int KS = NBS * (Q4 ? 32 : 16);
-    static constexpr int W_RAW = Q4 ? NBS * 18 : KS * 2;
-    static constexpr int W_PITCH = (W_RAW / 16) % 2 ? W_RAW : W_RAW + 16;              // odd multiples of 16 bytes: conflict-free ldmatrix
-    static constexpr int X_PITCH = Q4 ? NBS * 32 + 16 : KS * 2 + 16;
-    static constexpr int X_OFF = TM * W_PITCH, D_OFF = X_OFF + TP * X_PITCH;
-    static constexpr int STAGE = (D_OFF + (Q4 ? NBS * TP * 4 : 0) + 127) / 128 * 128;
-    static constexpr int RED = 4 * TP * MM_RED_PITCH * 4;             // sums of 4 warps
-    static constexpr int FIT = (int)((MM_SMEM_MAX - 8192 - RED) / STAGE);
-    static constexpr int S = FIT > 8 ? 8 : FIT;
-    static_assert(S >= 3, "ring too small");
+    static constexpr int MT = Q4 && NT == 4 ? 7 : 8;                  // fragments of 16 rows of a tile at most (two stages have to fit)
+    static constexpr int KS = Q4 ? 128 : 32;                          // columns of a slice
+    static constexpr int ROW = Q4 ? 72 : 64, TOK = Q4 ? 144 : 64;     // bytes of a stage per row and per token
+    static_assert(2 * (MT * 16 * ROW + TP * TOK) * MM_PAIRS <= MM_SMEM_MAX - 8192, "two stages");
 };
 
-template <int WT, int NT, int TM, bool SPARSE, bool GATED>
+template <int WT, int NT, bool SPARSE, bool GATED>
 __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
-    using Z = MmShape<WT, NT, TM>;
+    using Z = MmShape<WT, NT>;
     constexpr bool Q4 = Z::Q4;
-    constexpr int TP = Z::TP, WM = Z::WM, WK = Z::WK, KPW = Z::KPW, NBS = Z::NBS, KS = Z::KS, S = Z::S;
-    constexpr int IT = GATED ? TM / 2 : TM;                           // items (rows / neurons) of a tile
+    constexpr int TP = Z::TP, MT = Z::MT, MW = (MT + 1) / 2;           // fragments of a tile, of a warp
+    constexpr int IT = GATED ? MT * 8 : MT * 16;                      // items (rows / neurons) of a tile at most
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int s_warp[MM_WARPS];
-    float * red = reinterpret_cast<float *>(smem);                    // [4][TP][MM_RED_PITCH]
-    unsigned char * ring = smem + Z::RED;
-    int * rows = reinterpret_cast<int *>(ring + (size_t)S * Z::STAGE);   // [max_rows] rows of this CTA (sparse only)
+    __shared__ unsigned s_any[4];
+    int * rows = reinterpret_cast<int *>(smem + (size_t)MM_PAIRS * p.ring);      // rows of this CTA (sparse only)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wk = warp % WK, wm = warp / WK;                         // (warps w and w + 4 share a scheduler: rows a tile leaves unused idle on all four)
     const int G = gridDim.x, cta = blockIdx.x;
-    const uint32_t ring_a = smem_u32(ring);
+    const int pair = warp >> 1, half = warp & 1;
+    const uint32_t ring_a = smem_u32(smem) + (uint32_t)(pair * p.ring);
     pdl_launch();
 
-    int lo = 0, hi = 0, per_tile = 1, n_units = 0;                    // this CTA's items, items per tile
+    // this CTA's items, items per tile, fragment rows of a tile, bytes of a stage, stages of a ring
+    int lo = 0, hi = 0, per_tile = 1, n_tiles = 0, rt = 16, stage = 1, S = 2;
     auto set_range = [&](int n) {
         const int al = !SPARSE && p.masks_out ? 8 : 1;                // (a byte of the masks has one writer)
         const int gr = (n + al - 1) / al;
         lo = min(n, (int)((long long)gr * cta / G) * al);
         hi = min(n, (int)((long long)gr * (cta + 1) / G) * al);
-        const int tiles = (hi - lo + IT - 1) / IT;
-        if (tiles > 0) per_tile = ((hi - lo + tiles - 1) / tiles + al - 1) / al * al;
-        n_units = tiles * p.n_slices;
+        n_tiles = (hi - lo + IT - 1) / IT;
+        if (n_tiles > 0) per_tile = ((hi - lo + n_tiles - 1) / n_tiles + al - 1) / al * al;
+        rt = ((GATED ? 2 * per_tile : per_tile) + 15) / 16 * 16;
+        stage = rt * Z::ROW + TP * Z::TOK;
+        S = min(MM_SMAX, p.ring / stage);
     };
-    // ---- copies.  A thread's pieces of a stage lie in the same rows for a whole tile: it keeps their addresses and moves them along.
-    constexpr int CH = Q4 ? NBS : KS / 8;                             // 16-byte pieces of a row slice (Q4_0: of its nibbles)
-    constexpr int NW = TM * CH / MM_THREADS;                          // pieces per thread
-    constexpr int CS = Q4 ? NBS / 8 : 1;                              // Q4_0: pieces of 8 scales
-    constexpr int XP = Q4 ? TP * NBS * 2 : TP * CH;                   // activation pieces of a stage
-    constexpr int NX = (XP + MM_THREADS - 1) / MM_THREADS;
-    static_assert(MM_THREADS % CH == 0 && (TM * CH) % MM_THREADS == 0 && TM * CS <= MM_THREADS && (XP % MM_THREADS == 0 || NX == 1), "copy map");
-    const int c16 = tid % CH;                                         // my piece of a row
-    const uint8_t * wp[NW]; const uint8_t * sp = p.W;
-    unsigned w_ok = 0u;
-    int i_tile = 0, i_slice = 0;                                      // the unit that is requested next
-    auto tile_start = [&]() {
-        const int first = i_tile * per_tile, n_tile = min(per_tile, hi - lo - first);
-        auto row_ptr = [&](int r, bool & ok) -> const uint8_t * {
-            const int k = GATED ? r % IT : r;
-            ok = k < n_tile;
-            const int row = ok ? (SPARSE ? rows[first + k] : lo + first + k) : 0;
-            return (GATED && r >= IT ? p.W2 : p.W) + (size_t)row * p.row_bytes;
-        };
-        w_ok = 0u;
-#pragma unroll
-        for (int j = 0; j < NW; j++) {
-            bool ok;
-            wp[j] = row_ptr(tid / CH + j * (MM_THREADS / CH), ok) + c16 * 16;
-            if (ok) w_ok |= 1u << j;
-        }
-        if (Q4 && tid < TM * CS) {
-            bool ok;
-            sp = row_ptr(tid / CS, ok) + (size_t)p.nb * 16 + (tid % CS) * 16;
-            if (ok) w_ok |= 1u << NW;
-        }
+    const int n_mine = pair < p.n_slices ? (p.n_slices - pair + MM_PAIRS - 1) / MM_PAIRS : 0;       // slices of a tile that are the pair's
+    // A stage: row slices, activation slices (Q4_0: then the rows' scales and the activation's, [block][token])
+    int first = 0, n_rows = 0;                                        // current tile: first item, rows in all (gated: up 0, gate 0, up 1, ..)
+    const int r8 = lane >> 2, c4 = lane & 3;
+    const uint32_t w_dst = (uint32_t)(r8 * 64 + ((c4 ^ (r8 >> 1)) & 3) * 16);
+    auto row_ptr = [&](int r) -> const uint8_t * {
+        const int k = GATED ? r >> 1 : r;
+        return (GATED && (r & 1) ? p.W2 : p.W) + (size_t)(SPARSE ? rows[first + k] : lo + first + k) * p.row_bytes;
     };
-    auto issue_w = [&](int slot) {
-        if (i_slice == 0) tile_start();
-        const uint32_t base = ring_a + (uint32_t)slot * Z::STAGE + (tid / CH) * Z::W_PITCH + c16 * 16;
-        const int have = (Q4 ? p.nb : p.ncols / 8) - i_slice * CH;    // pieces of a row from this slice on
-        const unsigned bytes = c16 < have ? 16u : 0u;                 // past the end of a row: zeros
-#pragma unroll
-        for (int j = 0; j < NW; j++) {
-            if (w_ok >> j & 1u) mm_cp16(base + j * (MM_THREADS / CH) * Z::W_PITCH, bytes ? wp[j] : p.W, bytes);
-            wp[j] += CH * 16;
+    auto issue_w = [&](int j, int slot) {                             // the pair's slice number j: every other 8 rows
+        const int s = pair + j * MM_PAIRS;
+        const uint32_t base = ring_a + (uint32_t)(slot * stage);
+        const int off = s * 64 + c4 * 16;
+        if (!Q4 && off >= p.ncols * 2) {                              // past the end of a row: zeros
+            for (int r = half * 8 + r8; r < n_rows; r += 16) mm_zero16(base + w_dst + (r - r8) * 64);
+        } else if (!SPARSE) {
+            const uint8_t * src = row_ptr(half * 8 + r8) + off;
+            const size_t step = (size_t)p.row_bytes * 16;
+#pragma unroll 4
+            for (int r = half * 8 + r8; r < n_rows; r += 16, src += step) mm_cp16(base + w_dst + (r - r8) * 64, src);
+        } else {
+#pragma unroll 4
+            for (int r = half * 8 + r8; r < n_rows; r += 16) mm_cp16(base + w_dst + (r - r8) * 64, row_ptr(r) + off);
         }
         if (Q4) {
-            if (w_ok >> NW & 1u) {
-                const bool in = (tid % CS) * 8 < have;
-                mm_cp16(ring_a + (uint32_t)slot * Z::STAGE + (tid / CS) * Z::W_PITCH + NBS * 16 + (tid % CS) * 16, in ? sp : p.W, in ? 16u : 0u);
-            }
-            sp += NBS * 2;
+            const uint32_t sb = base + rt * 64 + TP * 128;
+            const int so = p.nb * 16 + s * 8;
+            for (int r = half * 32 + lane; r < n_rows; r += 64) mm_cp8(sb + r * 8, row_ptr(r) + so);
         }
     };
-    auto issue_x = [&](int slot) {
-        const uint32_t base = ring_a + (uint32_t)slot * Z::STAGE;
+    auto x_src = [&](int s, int e) -> const void * {                  // piece e of slice s: its address (nullptr: zeros)
+        if (!Q4) {
+            const int c = s * 32 + (e & 3) * 8;
+            return c < p.ncols ? p.x.h16 + (size_t)(e >> 2) * p.ncols + c : nullptr;
+        }
+        return (e & 1 ? p.x.hi : p.x.lo) + (size_t)(e >> 3) * p.nb + s * 4 + ((e >> 1) & 3);
+    };
+    auto x_dst = [&](int e) -> uint32_t {                             // where it lies behind the rows
+        return Q4 ? (uint32_t)((e >> 3) * 128 + ((e ^ (e >> 3)) & 7) * 16) : (uint32_t)((e >> 2) * 64 + ((e ^ (e >> 3)) & 3) * 16);
+    };
+    constexpr int XE = TP * (Q4 ? 8 : 4);                             // 16-byte pieces of an activation slice
+    const int x_n = p.T * (Q4 ? 8 : 4), pl = half * 32 + lane;
+    auto issue_x = [&](int j, int slot) {
+        const int s = pair + j * MM_PAIRS;
+        const uint32_t base = ring_a + (uint32_t)(slot * stage + rt * 64);
 #pragma unroll
-        for (int j = 0; j < NX; j++) {
-            const int e = tid + j * MM_THREADS;
-            if (!Q4) {
-                const int t = e / CH, c = i_slice * CH + c16;         // (512 is a multiple of CH: the piece is c16 again)
-                const bool in = c * 8 < p.ncols;
-                if (t < p.T) mm_cp16(base + Z::X_OFF + t * Z::X_PITCH + c16 * 16, p.x.h16 + (in ? (size_t)t * p.ncols + c * 8 : 0), in ? 16u : 0u);
-            } else {
-                const int h = e % 2, c = (e / 2) % NBS, t = e / (2 * NBS), b = i_slice * NBS + c;
-                const bool in = b < p.nb;
-                if (t < p.T) mm_cp16(base + Z::X_OFF + t * Z::X_PITCH + c * 32 + h * 16, (h ? p.x.hi : p.x.lo) + (in ? (size_t)t * p.nb + b : 0), in ? 16u : 0u);
+        for (int e0 = 0; e0 < XE; e0 += 64) {
+            const int e = e0 + pl;
+            if (e < x_n) {
+                const void * src = x_src(s, e);
+                if (src) mm_cp16(base + x_dst(e), src); else mm_zero16(base + x_dst(e));
             }
         }
         if (Q4) {
 #pragma unroll
-            for (int j = 0; j < (TP * NBS + MM_THREADS - 1) / MM_THREADS; j++) {
-                const int e = tid + j * MM_THREADS, c = e % NBS, t = e / NBS, b = i_slice * NBS + c;
-                const bool in = b < p.nb;
-                if (t < p.T) mm_cp4(base + Z::D_OFF + (c * TP + t) * 4, p.x.d + (in ? (size_t)t * p.nb + b : 0), in ? 4u : 0u);
+            for (int e0 = 0; e0 < TP * 4; e0 += 64) {
+                const int e = e0 + pl, t = e >> 2, k = e & 3;
+                if (t < p.T) mm_cp4(base + TP * 128 + rt * 8 + (k * TP + t) * 4, p.x.d + (size_t)t * p.nb + s * 4 + k);
             }
         }
     };
-    auto advance = [&]() { if (++i_slice == p.n_slices) { i_slice = 0; i_tile++; } };
+    auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" :: "r"(pair + 1) : "memory"); };
+    auto start_tile = [&](int tile) {
+        first = tile * per_tile;
+        n_rows = min(per_tile, hi - lo - first) * (GATED ? 2 : 1);
+    };
 
     if (!SPARSE) {
         set_range(p.nrows);
-        for (int s = 0; s < S - 1; s++) { if (s < n_units) { issue_w(s); advance(); } mm_commit(); }
+        start_tile(0);
+        const int ns = n_tiles > 0 ? min(S - 1, n_mine) : 0;
+        for (int j = 0; j < S - 1; j++) { if (j < ns) issue_w(j, j); mm_commit(); }
         pdl_wait();
         // The activation of the stages requested so far: plain loads, several in flight (as cp.async it would belong to a
         // later group than all the weights above, and the first stage would be waiting for the last)
-        const int ns = min(S - 1, n_units);
         constexpr int UN = 4;
-        const int PER = Q4 ? p.T * NBS * 2 : p.T * (KS / 8);
-        for (int e0 = tid; e0 < ns * PER; e0 += UN * MM_THREADS) {
+        const int n = ns * XE;
+        for (int e0 = pl; e0 < n; e0 += UN * 64) {
             uint4 v[UN];
-            uint32_t to[UN];
 #pragma unroll
-            for (int j = 0; j < UN; j++) {
-                const int ea = e0 + j * MM_THREADS, s = ea / PER, e = ea % PER, sl = s % p.n_slices;
-                v[j] = make_uint4(0u, 0u, 0u, 0u);
-                to[j] = 0u;
-                if (ea >= ns * PER) continue;
-                if (Q4) {
-                    const int h = e % 2, c = (e / 2) % NBS, t = e / (2 * NBS), b = sl * NBS + c;
-                    to[j] = ring_a + s * Z::STAGE + Z::X_OFF + t * Z::X_PITCH + c * 32 + h * 16;
-                    if (b < p.nb) v[j] = (h ? p.x.hi : p.x.lo)[(size_t)t * p.nb + b];
-                } else {
-                    const int t = e / (KS / 8), c = e % (KS / 8), col = sl * KS + c * 8;
-                    to[j] = ring_a + s * Z::STAGE + Z::X_OFF + t * Z::X_PITCH + c * 16;
-                    if (col < p.ncols) v[j] = *reinterpret_cast<const uint4 *>(p.x.h16 + (size_t)t * p.ncols + col);
+            for (int u = 0; u < UN; u++) {
+                const int ea = e0 + u * 64, j = ea / XE, e = ea % XE;
+                v[u] = make_uint4(0u, 0u, 0u, 0u);
+                if (ea < n && e < x_n) {
+                    const void * src = x_src(pair + j * MM_PAIRS, e);
+                    if (src) v[u] = *reinterpret_cast<const uint4 *>(src);
                 }
             }
 #pragma unroll
-            for (int j = 0; j < UN; j++)
-                if (e0 + j * MM_THREADS < ns * PER) asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" :: "r"(to[j]), "r"(v[j].x), "r"(v[j].y), "r"(v[j].z), "r"(v[j].w) : "memory");
+            for (int u = 0; u < UN; u++) {
+                const int ea = e0 + u * 64, j = ea / XE, e = ea % XE;
+                if (ea < n)
+                    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" :: "r"(ring_a + (uint32_t)(j * stage + rt * 64) + x_dst(e)), "r"(v[u].x), "r"(v[u].y), "r"(v[u].z), "r"(v[u].w) : "memory");
+            }
         }
         if (Q4) {
-            const int PD = p.T * NBS;
-            for (int e0 = tid; e0 < ns * PD; e0 += UN * MM_THREADS) {
+            const int nd = ns * TP * 4;
+            for (int e0 = pl; e0 < nd; e0 += UN * 64) {
                 float v[UN];
 #pragma unroll
-                for (int j = 0; j < UN; j++) {
-                    const int ea = e0 + j * MM_THREADS, s = ea / PD, e = ea % PD, sl = s % p.n_slices, c = e % NBS, t = e / NBS, b = sl * NBS + c;
-                    v[j] = ea < ns * PD && b < p.nb ? p.x.d[(size_t)t * p.nb + b] : 0.f;
+                for (int u = 0; u < UN; u++) {
+                    const int ea = e0 + u * 64, j = ea / (TP * 4), t = ea % (TP * 4) >> 2, k = ea & 3;
+                    v[u] = ea < nd && t < p.T ? p.x.d[(size_t)t * p.nb + (pair + j * MM_PAIRS) * 4 + k] : 0.f;
                 }
 #pragma unroll
-                for (int j = 0; j < UN; j++) {
-                    const int ea = e0 + j * MM_THREADS, s = ea / PD, e = ea % PD, c = e % NBS, t = e / NBS;
-                    if (ea < ns * PD) asm volatile("st.shared.f32 [%0], %1;" :: "r"(ring_a + s * Z::STAGE + Z::D_OFF + (c * TP + t) * 4), "f"(v[j]) : "memory");
+                for (int u = 0; u < UN; u++) {
+                    const int ea = e0 + u * 64, j = ea / (TP * 4), t = ea % (TP * 4) >> 2, k = ea & 3;
+                    if (ea < nd) asm volatile("st.shared.f32 [%0], %1;" :: "r"(ring_a + (uint32_t)(j * stage + rt * 72) + TP * 128 + (k * TP + t) * 4), "f"(v[u]) : "memory");
                 }
             }
         }
@@ -302,221 +303,222 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
             rank += n;
         }
         __syncthreads();
-        for (int s = 0; s < S - 1; s++) { if (s < n_units) { issue_w(s); issue_x(s); advance(); } mm_commit(); }
+        start_tile(0);
+        for (int j = 0; j < S - 1; j++) { if (j < n_mine && n_tiles > 0) { issue_w(j, j); issue_x(j, j); } mm_commit(); }
         if (p.list) for (int k = tid; k < hi - lo; k += MM_THREADS) p.list[lo + k] = rows[k];
     }
 
-    constexpr int NA = Q4 ? 1 : 2;                                    // (the accumulators of the two types have different shapes)
-    float acc[NA == 2 ? 2 : 1][NA == 2 ? NT : 1][4];
-    unsigned long long acq[Q4 ? 2 : 1][Q4 ? NT : 1][2];
-    auto clear = [&]() {
-        if (Q4) {
-#pragma unroll
-            for (int m = 0; m < (Q4 ? 2 : 1); m++)
-#pragma unroll
-                for (int n = 0; n < (Q4 ? NT : 1); n++) { acq[m][n][0] = 0ull; acq[m][n][1] = 0ull; }
-        } else {
-#pragma unroll
-            for (int m = 0; m < (Q4 ? 1 : 2); m++)
-#pragma unroll
-                for (int n = 0; n < (Q4 ? 1 : NT); n++)
-#pragma unroll
-                    for (int j = 0; j < 4; j++) acc[m][n][j] = 0.f;
-        }
-    };
-    clear();
     const int g = lane >> 2, q = lane & 3;
-    // ldmatrix row addresses inside a stage (fragment layouts of mma.m16n8k16 / m16n8k32)
-    const uint32_t a_off = Q4 ? (uint32_t)((wm * 32 + lane) * Z::W_PITCH + wk * KPW * 16)
-                              : (uint32_t)((wm * 32 + (lane & 7) + ((lane >> 3) & 1) * 8) * Z::W_PITCH + (wk * KPW * 16 + (lane >> 4) * 8) * 2);
-    const uint32_t s_off = (uint32_t)((wm * 32 + g) * Z::W_PITCH + NBS * 16 + wk * KPW * 2);
-    const uint32_t b_off = Q4 ? (uint32_t)(Z::X_OFF + (lane & 7) * Z::X_PITCH + wk * KPW * 32 + (lane >> 3) * 16)
-                              : (uint32_t)(Z::X_OFF + ((lane & 7) + (NT > 1 ? ((lane >> 4) & 1) * 8 : 0)) * Z::X_PITCH + (wk * KPW * 16 + ((lane >> 3) & 1) * 8) * 2);
-    const uint32_t d_off = (uint32_t)(Z::D_OFF + (wk * KPW * TP + 2 * q) * 4);
+    // ldmatrix addresses inside a stage (fragment layouts of mma.m16n8k16 / m16n8k32): two 16-byte pieces of 16 rows, four of 8 tokens
+    // (Q4_0: one block of 32 rows, one block of two groups of 8 tokens)
+    const int a_row = lane & 15;
+    const uint32_t a_up = (lane >> 4) * 32 * 64, b_up = NT > 1 ? (lane >> 4) * 8 * 128 : 0;   // (a warp's fragments are every other 16 rows)
+    const int b_row = Q4 ? (lane & 7) + (NT > 1 ? (lane >> 4) * 8 : 0) : (lane & 7);
     const uint32_t MAGIC = 0x4B400000u;
-    const unsigned long long neg_magic = mm_pack(-12582912.0f, -12582912.0f);
-
-    int tile = 0, slice = 0;
-    for (int i = 0; i < n_units; i++) {
-        mm_wait<S - 2>();
-        __syncthreads();                                              // stage i has landed for everybody; stage i - 1 is consumed
-        if (i + S - 1 < n_units) { const int slot = (i + S - 1) % S; issue_w(slot); issue_x(slot); advance(); }
-        mm_commit();
-        const uint32_t base = ring_a + (uint32_t)(i % S) * Z::STAGE;
-        const bool busy = (GATED ? wm * 32 % IT : wm * 32) < min(per_tile, hi - lo - tile * per_tile);      // my rows exist
-        if (!busy) {
-        } else if (!Q4) {
+    const unsigned long long neg_magic = mm_pack(-12582912.0f, -12582912.0f), sixteenth = mm_pack(0.0625f, 0.0625f);
+    uint32_t a_off[Q4 ? 4 : 2], b_off[Q4 ? 4 : 1];
 #pragma unroll
-            for (int k = 0; k < KPW; k++) {
-                uint32_t a[2][4];
-                mm_ldsm4(a[0], base + a_off + k * 32);
-                mm_ldsm4(a[1], base + a_off + 16 * Z::W_PITCH + k * 32);
-                if (NT == 1) {
-                    uint32_t b0, b1;
-                    mm_ldsm2(b0, b1, base + b_off + k * 32);
-                    mm_hmma(acc[0][0], a[0], b0, b1);
-                    mm_hmma(acc[NA - 1][0], a[1], b0, b1);
-                } else {
+    for (int k = 0; k < (Q4 ? 4 : 2); k++) a_off[k] = (uint32_t)(half * 1024 + a_row * 64 + (((Q4 ? k : k * 2 + (lane >> 4)) ^ ((lane & 7) >> 1)) & 3) * 16);
+#pragma unroll
+    for (int k = 0; k < (Q4 ? 4 : 1); k++)
+        b_off[k] = Q4 ? (uint32_t)(b_row * 128 + (((k * 2 + ((lane >> 3) & 1)) ^ (lane & 7)) & 7) * 16) : (uint32_t)(b_row * 64 + (((lane >> 3) ^ ((lane & 7) >> 1)) & 3) * 16);
+
+    for (int tile = 0; tile < n_tiles; tile++) {
+        if (tile > 0) {
+            start_tile(tile);
+            for (int j = 0; j < S - 1; j++) { if (j < n_mine) { issue_w(j, j); issue_x(j, j); } mm_commit(); }
+        }
+        // (the accumulators of the two types have different shapes)
+        float acc[Q4 ? 1 : MW][Q4 ? 1 : NT][4];
+        unsigned long long acq[Q4 ? MW : 1][Q4 ? NT : 1][2];
+#pragma unroll
+        for (int m = 0; m < MW; m++)
+#pragma unroll
+            for (int n = 0; n < NT; n++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) { if (Q4) acq[Q4 ? m : 0][Q4 ? n : 0][j >> 1] = 0ull; else acc[Q4 ? 0 : m][Q4 ? 0 : n][j] = 0.f; }
+        int slot = 0, next = S - 1;
+        for (int i = 0; i < n_mine; i++) {
+            mm_wait(S - 2);
+            pair_sync();                                              // stage i has landed for the pair, stage i - 1 is consumed
+            if (i + S - 1 < n_mine) { issue_w(i + S - 1, next); issue_x(i + S - 1, next); }
+            mm_commit();
+            if (++next == S) next = 0;
+            const uint32_t base = ring_a + (uint32_t)(slot * stage), xb = base + rt * 64;
+            if (++slot == S) slot = 0;
+            if (!Q4) {
+                uint32_t b[NT][4];
+#pragma unroll
+                for (int n = 0; n < NT; n++) mm_ldsm4(b[n], xb + b_off[0] + n * 8 * 64);
+#pragma unroll
+                for (int m = 0; m < MW; m++) {
+                    if (m * 32 + half * 16 >= rt) break;
+#pragma unroll
+                    for (int k = 0; k < 2; k++) {
+                        uint32_t a[4];
+                        mm_ldsm4(a, base + a_off[k] + m * 32 * 64);
+#pragma unroll
+                        for (int n = 0; n < NT; n++) mm_hmma(acc[Q4 ? 0 : m][Q4 ? 0 : n], a, b[n][2 * k], b[n][2 * k + 1]);
+                    }
+                }
+            } else {
+                const uint32_t sb = xb + TP * 128 + (half * 16 + g) * 8, db = xb + TP * 128 + rt * 8 + 2 * q * 4;
+#pragma unroll
+                for (int k = 0; k < (Q4 ? 4 : 0); k++) {              // block by block
+                    uint32_t b[NT + 1][2];
+                    unsigned long long dd[NT], md[NT];
 #pragma unroll
                     for (int n = 0; n < NT; n += 2) {
-                        uint32_t b[4];
-                        mm_ldsm4(b, base + b_off + n * 8 * Z::X_PITCH + k * 32);
-                        mm_hmma(acc[0][Q4 ? 0 : n], a[0], b[0], b[1]);
-                        mm_hmma(acc[NA - 1][Q4 ? 0 : n], a[1], b[0], b[1]);
-                        mm_hmma(acc[0][Q4 ? 0 : n + 1], a[0], b[2], b[3]);
-                        mm_hmma(acc[NA - 1][Q4 ? 0 : n + 1], a[1], b[2], b[3]);
+                        uint32_t v[4];
+                        mm_ldsm4(v, xb + b_off[k] + n * 8 * 128 - (n + 1 < NT ? 0u : b_up));      // (an odd last group is read twice)
+                        b[n][0] = v[0]; b[n][1] = v[1]; b[n + 1][0] = v[2]; b[n + 1][1] = v[3];
                     }
-                }
-            }
-        } else {
-            // scales of the warp's two blocks, rows g, g + 8, g + 16, g + 24 of its 32
-            unsigned long long d4[2][4];
 #pragma unroll
-            for (int r = 0; r < 4; r++) {
-                uint32_t w;
-                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(base + s_off + r * 8 * Z::W_PITCH));
-                const float2 f = h2f(w);
-                d4[0][r] = mm_pack(f.x * 0.0625f, f.x * 0.0625f);
-                d4[1][r] = mm_pack(f.y * 0.0625f, f.y * 0.0625f);
-            }
-            uint32_t al[2][4], ah[2][4];
-#pragma unroll
-            for (int k = 0; k < 2; k++) {
-                uint32_t w[4];
-                mm_ldsm4(w, base + a_off + k * 16);
-#pragma unroll
-                for (int r = 0; r < 4; r++) { al[k][r] = ((w[r] << 4) & 0xF0F0F0F0u) ^ 0x80808080u; ah[k][r] = (w[r] & 0xF0F0F0F0u) ^ 0x80808080u; }
-            }
-#pragma unroll
-            for (int n = 0; n < NT; n++) {
-                uint32_t b[4];
-                mm_ldsm4(b, base + b_off + n * 8 * Z::X_PITCH);
-#pragma unroll
-                for (int k = 0; k < 2; k++) {
-                    unsigned long long dd;
-                    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(dd) : "r"(base + d_off + (k * TP + n * 8) * 4));
-#pragma unroll
-                    for (int m = 0; m < 2; m++) {
-                        uint32_t c[4];
-                        mm_imma(c, al[k][2 * m], al[k][2 * m + 1], ah[k][2 * m], ah[k][2 * m + 1], b[2 * k], b[2 * k + 1], MAGIC);
-                        mm_scale_add(acq[Q4 ? m : 0][Q4 ? n : 0][0], mm_packu(c[0], c[1]), neg_magic, dd, d4[k][2 * m]);
-                        mm_scale_add(acq[Q4 ? m : 0][Q4 ? n : 0][1], mm_packu(c[2], c[3]), neg_magic, dd, d4[k][2 * m + 1]);
+                    for (int n = 0; n < NT; n++) {
+                        asm volatile("ld.shared.b64 %0, [%1];" : "=l"(dd[n]) : "r"(db + (k * TP + n * 8) * 4));
+                        dd[n] = mm_mul2(dd[n], sixteenth);
+                        md[n] = mm_mul2(dd[n], neg_magic);
                     }
-                }
-            }
-        }
-        if (slice == p.n_slices - 1) {
-            // ---- the warps' sums meet in shared memory: warps of one round write different slots, rounds in order
-            constexpr int SLOTS = WK / 4;
-            float * mine = red + (size_t)(wm * SLOTS + wk % SLOTS) * (TP * MM_RED_PITCH);
-#pragma unroll 1
-            for (int r = 0; r < 4; r++) {
-                if (wk / SLOTS == r) {
 #pragma unroll
-                    for (int m = 0; m < 2; m++)
+                    for (int m = 0; m < MW; m += 2) {
+                        if (m * 32 + half * 16 >= rt) break;
+                        uint32_t w[4];
+                        mm_ldsm4(w, base + a_off[k] + m * 32 * 64 + (m * 32 + half * 16 + 32 < rt ? a_up : 0u));      // (so is an odd last fragment)
 #pragma unroll
-                        for (int n = 0; n < NT; n++)
+                        for (int u = 0; u < 2; u++) {
+                            if (m + u >= MW || (m + u) * 32 + half * 16 >= rt) break;
+                            unsigned short h0, h1;
+                            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h0) : "r"(sb + (m + u) * 256 + k * 2));
+                            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h1) : "r"(sb + (m + u) * 256 + 64 + k * 2));
+                            const float e0 = __half2float(__ushort_as_half(h0)), e1 = __half2float(__ushort_as_half(h1));
+                            const unsigned long long d0 = mm_pack(e0, e0), d1 = mm_pack(e1, e1);
+                            const uint32_t w0 = w[2 * u], w1 = w[2 * u + 1];
+                            const uint32_t a0 = ((w0 << 4) & 0xF0F0F0F0u) ^ 0x80808080u, a1 = ((w1 << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
+                            const uint32_t a2 = (w0 & 0xF0F0F0F0u) ^ 0x80808080u, a3 = (w1 & 0xF0F0F0F0u) ^ 0x80808080u;
 #pragma unroll
-                            for (int j = 0; j < 4; j++) {
-                                float v;
-                                if (Q4) {
-                                    const unsigned long long w = acq[Q4 ? m : 0][Q4 ? n : 0][j >> 1];
-                                    v = __uint_as_float(j & 1 ? (unsigned)(w >> 32) : (unsigned)w);
-                                } else {
-                                    v = acc[Q4 ? 0 : m][Q4 ? 0 : n][j];
-                                }
-                                float * o = mine + (n * 8 + 2 * q + (j & 1)) * MM_RED_PITCH + m * 16 + g + (j >> 1) * 8;
-                                *o = r == 0 ? v : *o + v;
+                            for (int n = 0; n < NT; n++) {
+                                uint32_t c[4];
+                                mm_imma(c, a0, a1, a2, a3, b[n][0], b[n][1], MAGIC);
+                                mm_scale_add(acq[Q4 ? m + u : 0][Q4 ? n : 0][0], mm_packu(c[0], c[1]), dd[n], md[n], d0);
+                                mm_scale_add(acq[Q4 ? m + u : 0][Q4 ? n : 0][1], mm_packu(c[2], c[3]), dd[n], md[n], d1);
                             }
-                }
-                __syncthreads();
-            }
-            auto sum_of = [&](int r, int t) {                         // row r of the tile, token t: slots in order
-                const float * o = red + (size_t)(r >> 5) * SLOTS * (TP * MM_RED_PITCH) + t * MM_RED_PITCH + (r & 31);
-                float v = o[0];
-#pragma unroll
-                for (int s = 1; s < SLOTS; s++) v += o[(size_t)s * (TP * MM_RED_PITCH)];
-                return v;
-            };
-            const int first = tile * per_tile, n_tile = min(per_tile, hi - lo - first);
-            for (int e = tid; e < IT * p.T; e += MM_THREADS) {
-                const int k = e % IT, t = e / IT;                     // item k of the tile
-                if (k >= n_tile) continue;
-                const int item = lo + first + k;
-                const int r = SPARSE ? rows[first + k] : item;
-                const int64_t gid = SPARSE && p.bucket ? p.bucket[r] : r;
-                const float v = sum_of(k, t);
-                float o = GATED ? fmaxf(sum_of(IT + k, t), 0.f) * v : v;
-                if (SPARSE && p.idx[(size_t)t * p.idx_stride + gid] < p.threshold) {      // (a NaN logit counts as active)
-                    if (p.coef) { p.coef[(size_t)t * p.coef_stride + item] = __ushort_as_half((unsigned short)0); continue; }
-                    o = 0.f;
-                }
-                if (p.bias) o += p.bias[gid];
-                if (p.relu) o = fmaxf(o, 0.f);
-                if (p.dst)   p.dst[(size_t)t * p.dst_stride + gid] = o;
-                if (p.dst16) p.dst16[(size_t)t * p.dst_stride + gid] = __float2half_rn(o);
-                if (p.coef)  p.coef[(size_t)t * p.coef_stride + item] = __float2half_rn(o);
-            }
-            if (!SPARSE && p.masks_out) {                             // the union over the tokens of !(result < threshold), one bit per row
-                for (int k0 = warp * 32; k0 < n_tile; k0 += MM_WARPS * 32) {
-                    const int k = k0 + lane;
-                    bool any = false;
-                    for (int t = 0; t < p.T && k < n_tile; t++) {
-                        float o = sum_of(k, t);
-                        if (p.bias) o += p.bias[lo + first + k];
-                        if (p.relu) o = fmaxf(o, 0.f);
-                        any |= !(o < p.masks_threshold);
-                    }
-                    const uint32_t m = __ballot_sync(0xffffffffu, any);
-                    if (lane < 4 && k0 + lane * 8 < n_tile) {         // the range starts at a multiple of 8 rows
-                        unsigned char * o = reinterpret_cast<unsigned char *>(p.masks_out) + (lo + first + k0) / 8 + lane;
-                        const unsigned char bits = (unsigned char)(m >> (lane * 8));
-                        *o = p.masks_or ? (unsigned char)(*o | bits) : bits;
+                        }
                     }
                 }
             }
-            clear();
         }
-        if (++slice == p.n_slices) { slice = 0; tile++; }
+        // ---- the pairs' partial tiles: [token][row], each over its own ring (all copies have landed: the last stage was the last
+        // one requested); a pitch of 4 (20) mod 32 words keeps the fragment stores free of bank conflicts
+        pair_sync();
+        const int pitch = rt + 4;
+        float * mine = reinterpret_cast<float *>(smem + (size_t)pair * p.ring);
+#pragma unroll
+        for (int m = 0; m < MW; m++) {
+            if (m * 32 + half * 16 >= rt) break;
+#pragma unroll
+            for (int n = 0; n < NT; n++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    float v;
+                    if (Q4) {
+                        const unsigned long long w = acq[Q4 ? m : 0][Q4 ? n : 0][j >> 1];
+                        v = __uint_as_float(j & 1 ? (unsigned)(w >> 32) : (unsigned)w);
+                    } else {
+                        v = acc[Q4 ? 0 : m][Q4 ? 0 : n][j];
+                    }
+                    mine[(n * 8 + 2 * q + (j & 1)) * pitch + m * 32 + half * 16 + g + (j >> 1) * 8] = v;
+                }
+        }
+        if (tid < 4) s_any[tid] = 0u;
+        __syncthreads();
+        const float * sums = reinterpret_cast<const float *>(smem);
+        const int n_tile = GATED ? n_rows / 2 : n_rows;
+        for (int t = warp; t < p.T; t += MM_WARPS) {
+            for (int k0 = 0; k0 < n_tile; k0 += 32) {
+                const int k = k0 + lane;
+                const bool mine_k = k < n_tile;
+                float o = 0.f;
+                if (mine_k) {
+                    if (GATED) {
+                        float u = 0.f, v = 0.f;
+#pragma unroll
+                        for (int w = 0; w < MM_PAIRS; w++) {
+                            const float2 f = *reinterpret_cast<const float2 *>(sums + (size_t)w * (p.ring / 4) + t * pitch + 2 * k);
+                            u += f.x; v += f.y;
+                        }
+                        o = fmaxf(v, 0.f) * u;
+                    } else {
+#pragma unroll
+                        for (int w = 0; w < MM_PAIRS; w++) o += sums[(size_t)w * (p.ring / 4) + t * pitch + k];
+                    }
+                    const int item = lo + first + k;
+                    const int r = SPARSE ? rows[first + k] : item;
+                    const int64_t gid = SPARSE && p.bucket ? p.bucket[r] : r;
+                    const bool off = SPARSE && p.idx[(size_t)t * p.idx_stride + gid] < p.threshold;      // (a NaN logit counts as active)
+                    if (off && p.coef) {
+                        p.coef[(size_t)t * p.coef_stride + item] = __ushort_as_half((unsigned short)0);
+                    } else {
+                        if (off) o = 0.f;
+                        if (p.bias) o += p.bias[gid];
+                        if (p.relu) o = fmaxf(o, 0.f);
+                        if (p.dst)   p.dst[(size_t)t * p.dst_stride + gid] = o;
+                        if (p.dst16) p.dst16[(size_t)t * p.dst_stride + gid] = __float2half_rn(o);
+                        if (p.coef)  p.coef[(size_t)t * p.coef_stride + item] = __float2half_rn(o);
+                    }
+                }
+                if (!SPARSE && p.masks_out) {                         // the union over the tokens of !(result < threshold), one bit per row
+                    const unsigned m = __ballot_sync(0xffffffffu, mine_k && !(o < p.masks_threshold));
+                    if (lane == 0 && m) atomicOr(&s_any[k0 / 32], m);
+                }
+            }
+        }
+        if (!SPARSE && p.masks_out) {
+            __syncthreads();
+            if (tid < 16 && tid * 8 < n_tile) {                       // the range starts at a multiple of 8 rows
+                unsigned char * o = reinterpret_cast<unsigned char *>(p.masks_out) + (lo + first) / 8 + tid;
+                const unsigned char bits = (unsigned char)(s_any[tid / 4] >> (tid % 4 * 8));
+                *o = p.masks_or ? (unsigned char)(*o | bits) : bits;
+            }
+        }
+        if (tile + 1 < n_tiles) __syncthreads();                      // the sums are read, their rings may fill again
     }
 }
 
 // ---------------------------------------------------------------------------------------------- launch
-template <int WT, int NT, int TM, bool SPARSE, bool GATED>
+template <int WT, int NT, bool SPARSE, bool GATED>
 static int mm_go(MmP p, bool pdl, cudaStream_t st) {
-    using Z = MmShape<WT, NT, TM>;
+    using Z = MmShape<WT, NT>;
     p.n_slices = (p.ncols + Z::KS - 1) / Z::KS;
     // (8 rows are as little as is worth a CTA: its share of the activation costs more than its weights)
     const int G = (int)imin64(sm_count(), (p.nrows + 7) / 8);
-    p.max_rows = SPARSE ? (p.nrows + G - 1) / G + 1 : 0;
-    if (p.max_rows * 4 > 8192 - 256) return PI_ERR_UNSUPPORTED;       // (more than MM_MAX_ROWS rows)
-    const size_t smem = Z::RED + (size_t)Z::S * Z::STAGE + (size_t)p.max_rows * 4;
+    const int list = SPARSE ? ((p.nrows + G - 1) / G + 1) * 4 : 0;    // bytes
+    if (list > 8192 - 128) return PI_ERR_UNSUPPORTED;                 // (more than MM_MAX_ROWS rows)
+    p.ring = (MM_SMEM_MAX - list) / MM_PAIRS / 128 * 128;
     static bool attr_done[16] = {false};
     int dev = 0;
     PI_CUDA(cudaGetDevice(&dev));
-    auto kern = k_mm<WT, NT, TM, SPARSE, GATED>;
+    auto kern = k_mm<WT, NT, SPARSE, GATED>;
     if (dev >= 0 && dev < 16 && !attr_done[dev]) {
-        PI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MM_SMEM_MAX));
+        PI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MM_SMEM_MAX));
         attr_done[dev] = true;
     }
-    PI_CUDA(launch_k(kern, dim3(G), dim3(MM_THREADS), smem, st, pdl, p));
+    PI_CUDA(launch_k(kern, dim3(G), dim3(MM_THREADS), (size_t)p.ring * MM_PAIRS + list, st, pdl, p));
     return PI_OK;
 }
 
-template <int WT, int NT, int TM>
+template <int WT, int NT>
 static int mm_sel(const MmP & p, bool pdl, cudaStream_t st) {
-    if (!p.masks) return mm_go<WT, NT, TM, false, false>(p, pdl, st);
-    if (p.W2)     return mm_go<WT, NT, TM, true, true>(p, pdl, st);
-    return mm_go<WT, NT, TM, true, false>(p, pdl, st);
+    if (!p.masks) return mm_go<WT, NT, false, false>(p, pdl, st);
+    if (p.W2)     return mm_go<WT, NT, true, true>(p, pdl, st);
+    return mm_go<WT, NT, true, false>(p, pdl, st);
 }
 
-template <int WT, int NT>
-static int mm_tile(const MmP & p, bool pdl, cudaStream_t st) {
-    // the smallest tile that holds a CTA's share of the rows: less column splitting inside the CTA for the taller ones
-    const int64_t share = ((int64_t)p.nrows * (p.W2 ? 2 : 1) + sm_count() - 1) / sm_count();
-    if (share > 64) return mm_sel<WT, NT, 128>(p, pdl, st);
-    if (share > 32) return mm_sel<WT, NT, 64>(p, pdl, st);
-    return mm_sel<WT, NT, 32>(p, pdl, st);
+template <int WT>
+static int mm_tokens(const MmP & p, bool pdl, cudaStream_t st) {
+    if (p.T <= 8)  return mm_sel<WT, 1>(p, pdl, st);
+    if (p.T <= 16) return mm_sel<WT, 2>(p, pdl, st);
+    if (p.T <= 24) return mm_sel<WT, 3>(p, pdl, st);
+    return mm_sel<WT, 4>(p, pdl, st);
 }
 
 // PI_ERR_UNSUPPORTED: shape not eligible, the caller uses another kernel.  Tokens go in launches of at most 32.
@@ -541,10 +543,8 @@ int launch_mm(const GemvArgs & a, cudaStream_t st) {
         p.dst16 = a.dst16 ? a.dst16 + (size_t)t0 * a.dst_stride : nullptr; p.dst_stride = a.dst_stride;
         p.coef = a.coef ? a.coef + (size_t)t0 * a.coef_stride : nullptr; p.coef_stride = a.coef_stride;
         p.masks_out = a.masks_out; p.masks_threshold = a.masks_threshold; p.masks_or = t0 > 0;
-        p.n_slices = 0; p.max_rows = 0;
-        int rc;
-        if (q4) rc = p.T <= 8 ? mm_tile<PI_TYPE_Q4_0, 1>(p, a.pdl, st) : p.T <= 16 ? mm_tile<PI_TYPE_Q4_0, 2>(p, a.pdl, st) : mm_tile<PI_TYPE_Q4_0, 4>(p, a.pdl, st);
-        else    rc = p.T <= 8 ? mm_tile<PI_TYPE_F16, 1>(p, a.pdl, st) : p.T <= 16 ? mm_tile<PI_TYPE_F16, 2>(p, a.pdl, st) : mm_tile<PI_TYPE_F16, 4>(p, a.pdl, st);
+        p.n_slices = 0; p.ring = 0;
+        const int rc = q4 ? mm_tokens<PI_TYPE_Q4_0>(p, a.pdl, st) : mm_tokens<PI_TYPE_F16>(p, a.pdl, st);
         if (rc != PI_OK) return rc;
     }
     return PI_OK;
