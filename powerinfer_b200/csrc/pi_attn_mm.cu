@@ -10,7 +10,7 @@
 // as B operands of two mma whose k order is permuted in the same way on the query side; four tiles of 8 positions in
 // flight per warp.  Values travel to shared memory by cp.async (tiles of 64 positions, two in flight) while the scores are made and
 // are read transposed.  Every CTA rotates and stores the new keys and values it reads itself (CTAs that share a KV head store the
-// same bits), so no store pass runs before a chunk.
+// same bits), so no store pass runs before a chunk of up to AM_OWN_STORE tokens; beyond that the repeated work costs more than a launch.
 // Numerics follow the CPU path as in k_attention: q, k, v and the probabilities in FP16, exp through FP16, the normaliser
 // summed in double.
 #include "pi_act.cuh"
@@ -18,6 +18,7 @@
 namespace pi {
 
 static constexpr int AM_THREADS = 256, AM_WARPS = 8, AM_VT = 64;      // positions of a value tile
+static constexpr int AM_OWN_STORE = 32;
 
 struct AttnMmP {
     const float * q; const float * k; const float * v; __half * k_cache; __half * v_cache;
@@ -25,6 +26,7 @@ struct AttnMmP {
     const float * cs; int neox; int64_t q_stride, kv_stride;
     float * out; ActBuf out_act; int out_act_type;
     int chunk;                                                        // rows are tokens of one head, else heads of one token
+    int stored;                                                       // the new keys and values are in the cache already
     int P, R;                                                         // positions (a multiple of 64) and rows that shared memory holds
 };
 
@@ -64,7 +66,7 @@ __global__ void __launch_bounds__(AM_THREADS) k_attention_mm(const AttnMmP p) {
     __half * kc = p.k_cache + ((size_t)sq * p.n_ctx * p.n_head_kv + hk) * HD;
     __half * vc = p.v_cache + ((size_t)sq * p.n_ctx * p.n_head_kv + hk) * HD;
     // tokens whose new keys and values this CTA stores: its own, or all of the chunk up to its last
-    const int s_lo = p.chunk ? 0 : t0, s_n = p.chunk ? t0 + n_rows : 1;
+    const int s_lo = p.chunk ? 0 : t0, s_n = p.stored ? 0 : p.chunk ? t0 + n_rows : 1;
     int n_keys = 0;                                                   // keys that any row sees
     for (int r = 0; r < (p.chunk ? n_rows : 1); r++) { const int ps = p.pos[t0 + r]; if (ps >= 0 && ps < p.n_ctx) n_keys = max(n_keys, ps + 1); }
     if (n_keys == 0) return;                                          // never index the cache out of range
@@ -255,6 +257,28 @@ __global__ void __launch_bounds__(AM_THREADS) k_attention_mm(const AttnMmP p) {
     }
 }
 
+// new keys (rotated) and values of a chunk's tokens to the cache: one thread per pair of columns
+__global__ void __launch_bounds__(256) k_kv_store(const AttnMmP p, int hd) {
+    const int half = hd / 2, e = blockIdx.x * 256 + threadIdx.x, t = blockIdx.y;
+    pdl_launch();
+    pdl_wait();
+    if (e >= p.n_head_kv * half) return;
+    const int hk = e / half, k = e % half, ps = p.pos[t];
+    if (ps < 0 || ps >= p.n_ctx) return;
+    const size_t row = (((size_t)(p.seq ? p.seq[t] : 0) * p.n_ctx + ps) * p.n_head_kv + hk) * hd;
+    const float * kh = p.k + (size_t)t * p.kv_stride + (size_t)hk * hd, * vh = p.v + (size_t)t * p.kv_stride + (size_t)hk * hd;
+    const int i0 = p.cs && !p.neox ? 2 * k : k, i1 = p.cs && !p.neox ? 2 * k + 1 : k + half;
+    float o0 = kh[i0], o1 = kh[i1];
+    if (p.cs) {
+        const float2 a = reinterpret_cast<const float2 *>(p.cs)[(size_t)ps * half + k];
+        rope_pair(kh[i0], kh[i1], a.x, a.y, o0, o1);
+    }
+    p.k_cache[row + i0] = __float2half_rn(o0);
+    p.k_cache[row + i1] = __float2half_rn(o1);
+    p.v_cache[row + k] = __float2half_rn(vh[k]);
+    p.v_cache[row + k + half] = __float2half_rn(vh[k + half]);
+}
+
 static constexpr size_t AM_SMEM_MAX = 220 * 1024;
 
 // rows and positions that shared memory holds, and its size
@@ -297,7 +321,9 @@ int launch_attention_mm(const AttnArgs & a, cudaStream_t st) {
     p.kv_stride = a.kv_stride ? a.kv_stride : (int64_t)a.n_head_kv * a.head_dim;
     p.out = a.out; p.out_act = a.out_act; p.out_act_type = a.out_act_type;
     p.chunk = a.store_mode != 0;
+    p.stored = p.chunk && a.T > AM_OWN_STORE;
     const size_t smem = attn_mm_smem(a, &p.P, &p.R);
+    if (p.stored) PI_CUDA(launch_k(k_kv_store, dim3((unsigned)((a.n_head_kv * a.head_dim / 2 + 255) / 256), a.T), dim3(256), 0, st, a.pdl, p, a.head_dim));
     const dim3 grid = p.chunk ? dim3(a.n_head, (a.T + 15) / 16) : dim3(a.n_head_kv * ((a.n_head / a.n_head_kv + 15) / 16), a.T);
     return a.head_dim == 64 ? attn_mm_go<2>(p, grid, smem, a.pdl, st) : attn_mm_go<4>(p, grid, smem, a.pdl, st);
 }

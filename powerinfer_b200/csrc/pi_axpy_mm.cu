@@ -1,4 +1,4 @@
-// ggml_axpy for 2..32 tokens on the tensor cores (ggml.c:14314-14618 is the CPU path it matches), and the coefficients it reads.
+// ggml_axpy for 2 and more tokens on the tensor cores (ggml.c:14314-14618 is the CPU path it matches), and the coefficients it reads.
 //
 // dst[t, c] = sum over listed rows r of coef[t, r] * Wt[r, c].  As a matrix product C[c, t] += A[c, r] * B[r, t]: A = the rows
 // of down_t read transposed, B = the coefficients, laid out by list position so that they load like a matrix.
@@ -14,8 +14,9 @@
 // (Expanding a stage into an FP16 tile in shared memory first costs two barriers per 16 rows: 159 us where this takes 82,
 // 103 MB of rows, 32 tokens.)
 //
-// Work split: units of 256 columns x 64 (128) list rows, numbered slice by slice; every CTA takes an equal contiguous range,
-// so the chip is full whatever the number of columns.  The CTAs that meet in a column slice each write one partial vector
+// Work split: units of 256 columns x 64 (128) list rows x up to 32 tokens, numbered slice by slice (a slice: 256 columns of one group of
+// 32 tokens; the groups of a column range follow one another, so that they find its rows in L2); every CTA takes an equal contiguous
+// range, so the chip is full whatever the number of columns.  The CTAs that meet in a slice each write one partial vector
 // ("piece"); at most n_pieces of them per slice, the missing ones are written as zeros, and the norm (or the reduction)
 // that follows adds the pieces in order.  Rows arrive by 16-byte cp.async from all threads (they lie anywhere).
 #include "pi_common.cuh"
@@ -28,10 +29,10 @@ static constexpr size_t AX_SMEM_MAX = 226 * 1024;
 static constexpr int AX_ROW_RING = 16;                   // stages whose row numbers are kept
 
 struct AxpyMmP {
-    const uint8_t * Wt; int64_t row_bytes; int nrows, ncols, nb, T, T_all;
+    const uint8_t * Wt; int64_t row_bytes; int nrows, ncols, nb, T;
     const int32_t * list; const int32_t * count;
     const void * coef; int64_t coef_stride;                           // FP16, or F32 in the exact mode
-    float * partial; int n_cs, n_pieces;
+    float * partial; int n_cs, n_tg, n_pieces;                        // column ranges, token groups, partial vectors per slice
 };
 
 __device__ __forceinline__ void ax_cp16(uint32_t dst, const void * src, unsigned bytes) {       // the first `bytes` bytes, the rest zeros
@@ -106,12 +107,13 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
     pdl_wait();
     const int n = min(*p.count, p.nrows);
     const int nst = (n + RS - 1) / RS;
-    const unsigned total = (unsigned)p.n_cs * (unsigned)nst;
+    const int n_sl = p.n_cs * p.n_tg;
+    const unsigned total = (unsigned)n_sl * (unsigned)nst;
     if (total == 0) {                                                 // no active row: the result is zero
         for (int cs = cta; cs < p.n_cs; cs += gridDim.x)
             for (int e = tid; e < p.n_pieces * p.T * AX_CW; e += AX_THREADS) {
-                const int c = cs * AX_CW + e % AX_CW, t = e / AX_CW % p.T, k = e / AX_CW / p.T;
-                if (c < p.ncols) p.partial[((size_t)k * p.T_all + t) * p.ncols + c] = 0.f;
+                const int c = cs * AX_CW + e % AX_CW;
+                if (c < p.ncols) p.partial[(size_t)(e / AX_CW) * p.ncols + c] = 0.f;
             }
         return;
     }
@@ -127,7 +129,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
     for (int e = tid; e < (S + 1) * RS; e += AX_THREADS) rows[e] = row_at(u0 + e / RS, e % RS);
     __syncthreads();
     auto issue = [&](int i) {                                         // unit u0 + i
-        const int u = u0 + i, cs = u / nst, st = u % nst;
+        const int u = u0 + i, sl = u / nst, st = u % nst, cs = sl / p.n_tg, tok0 = sl % p.n_tg * 32, Tg = min(32, p.T - tok0);
         const uint32_t base = ring_a + (uint32_t)(i % S) * Z::STAGE;
         const int * rw = rows + (i % AX_ROW_RING) * RS;
         if (!Q4) {
@@ -150,8 +152,8 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
         constexpr int CPP = 16 / Z::CB;                               // coefficients of a 16-byte piece; positions past the list count as 0
         for (int e = tid; e < TP * (RS / CPP); e += AX_THREADS) {
             const int t = e / (RS / CPP), c = e % (RS / CPP), li = st * RS + c * CPP;
-            const int bytes = t < p.T ? max(0, min(CPP, n - li)) * Z::CB : 0;
-            ax_cp16(base + Z::C_OFF + t * Z::C_PITCH + c * 16, (const char *)p.coef + (bytes ? ((size_t)t * p.coef_stride + li) * Z::CB : 0), (unsigned)bytes);
+            const int bytes = t < Tg ? max(0, min(CPP, n - li)) * Z::CB : 0;
+            ax_cp16(base + Z::C_OFF + t * Z::C_PITCH + c * 16, (const char *)p.coef + (bytes ? ((size_t)(tok0 + t) * p.coef_stride + li) * Z::CB : 0), (unsigned)bytes);
         }
     };
     for (int s = 0; s < S - 1; s++) { if (s < n_units) issue(s); asm volatile("cp.async.commit_group;" ::: "memory"); }
@@ -271,8 +273,9 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
                 }
             }
         }
-        const int u = u0 + i, cs = u / nst;
+        const int u = u0 + i;
         if (u % nst == nst - 1 || i == n_units - 1) {
+            const int sl = u / nst, cs = sl / p.n_tg, tok0 = sl % p.n_tg * 32, Tg = min(32, p.T - tok0);
             // ---- end of this CTA's share of the slice: the four row quarters are added in order
 #pragma unroll 1
             for (int r = 0; r < 4; r++) {
@@ -293,14 +296,14 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
                 }
                 __syncthreads();
             }
-            const int c_lo = (int)((((unsigned long long)cs * nst + 1u) * G - 1u) / total), c_hi = (int)(((unsigned long long)(cs + 1) * nst * G - 1u) / total);
+            const int c_lo = (int)((((unsigned long long)sl * nst + 1u) * G - 1u) / total), c_hi = (int)(((unsigned long long)(sl + 1) * nst * G - 1u) / total);
             const int piece = cta - c_lo, more = cta == c_hi ? p.n_pieces - 1 - piece : 0;      // the slice's last CTA also writes the missing pieces
-            for (int e = tid; e < p.T * AX_CW; e += AX_THREADS) {
+            for (int e = tid; e < Tg * AX_CW; e += AX_THREADS) {
                 const int c = e % AX_CW, t = e / AX_CW, col = cs * AX_CW + c;
                 if (col >= p.ncols) continue;
-                float * o = p.partial + ((size_t)piece * p.T_all + t) * p.ncols + col;
+                float * o = p.partial + ((size_t)piece * p.T + tok0 + t) * p.ncols + col;
                 *o = red[t * AX_RED_PITCH + c];
-                for (int k = 1; k <= more; k++) o[(size_t)k * p.T_all * p.ncols] = 0.f;
+                for (int k = 1; k <= more; k++) o[(size_t)k * p.T * p.ncols] = 0.f;
             }
             clear();
         }
@@ -396,17 +399,19 @@ int launch_coef(const CoefArgs & a, cudaStream_t st) {
 }
 
 // ---------------------------------------------------------------------------------------------- launch
-// At most 16 CTAs per column slice (a partial vector each): more would cost the reader of the pieces more than they save.
-static void axpy_mm_shape(int64_t ncols, int * n_cs, int * grid, int * n_pieces) {
+// At most 16 CTAs per slice (a partial vector each): more would cost the reader of the pieces more than they save.
+static void axpy_mm_shape(int64_t ncols, int T, int * n_cs, int * n_tg, int * grid, int * n_pieces) {
     *n_cs = (int)((ncols + AX_CW - 1) / AX_CW);
-    *grid = (int)imin64(sm_count(), (int64_t)*n_cs * 16);
-    *n_pieces = (*grid + *n_cs - 1) / *n_cs + 1;                      // ranges are not aligned to slices: one more than the quotient
+    *n_tg = (T + 31) / 32;
+    const int n = *n_cs * *n_tg;
+    *grid = (int)imin64(sm_count(), (int64_t)n * 16);
+    *n_pieces = (*grid + n - 1) / n + 1;                              // ranges are not aligned to slices: one more than the quotient
 }
 
 // Q4_0 rows whose width is no multiple of 1024 take exact coefficients (F32): see the top of the file
 bool axpy_mm_exact(int wtype, int64_t ncols) { return wtype == PI_TYPE_Q4_0 && ncols % 1024 != 0; }
 
-int axpy_mm_pieces(int64_t ncols) { int cs, g, np; axpy_mm_shape(ncols, &cs, &g, &np); return np; }
+int axpy_mm_pieces(int64_t ncols, int T) { int cs, tg, g, np; axpy_mm_shape(ncols, T, &cs, &tg, &g, &np); return np; }
 
 template <int MODE, int NT>
 static int axpy_mm_go(const AxpyMmP & p, int grid, bool pdl, cudaStream_t st) {
@@ -429,24 +434,18 @@ static int axpy_mm_tokens(const AxpyMmP & p, int grid, bool pdl, cudaStream_t st
     return p.T <= 8 ? axpy_mm_go<MODE, 1>(p, grid, pdl, st) : p.T <= 16 ? axpy_mm_go<MODE, 2>(p, grid, pdl, st) : axpy_mm_go<MODE, 4>(p, grid, pdl, st);
 }
 
-// PI_ERR_UNSUPPORTED: shape not eligible, the caller uses the CUDA-core kernel.  Tokens go in launches of at most 32.
+// PI_ERR_UNSUPPORTED: shape not eligible, the caller uses the CUDA-core kernel.
 int launch_axpy_mm(const AxpyArgs & a, cudaStream_t st, int * pieces_used) {
     const bool q4 = a.wtype == PI_TYPE_Q4_0, exact = axpy_mm_exact(a.wtype, a.ncols);
     if (!a.coef || a.coef_stride % 8 != 0 || !a.list || (q4 ? a.ncols % 256 != 0 : a.ncols % 8 != 0)) return PI_ERR_UNSUPPORTED;
     AxpyMmP p;
     int grid;
-    axpy_mm_shape(a.ncols, &p.n_cs, &grid, &p.n_pieces);
+    axpy_mm_shape(a.ncols, a.T, &p.n_cs, &p.n_tg, &grid, &p.n_pieces);
     if (p.n_pieces > a.n_groups) return PI_ERR_UNSUPPORTED;
     p.Wt = (const uint8_t *)a.Wt; p.row_bytes = (int64_t)pi_row_bytes(a.wtype, a.ncols); p.nrows = (int)a.nrows; p.ncols = (int)a.ncols;
-    p.nb = (int)(a.ncols / 32); p.T_all = a.T; p.list = a.list; p.count = a.count; p.coef_stride = a.coef_stride;
+    p.nb = (int)(a.ncols / 32); p.T = a.T; p.list = a.list; p.count = a.count; p.coef = a.coef; p.coef_stride = a.coef_stride; p.partial = a.partial;
     if (pieces_used) *pieces_used = p.n_pieces;
-    for (int t0 = 0; t0 < a.T; t0 += 32) {
-        p.T = a.T - t0 < 32 ? a.T - t0 : 32;
-        p.coef = (const char *)a.coef + (size_t)t0 * a.coef_stride * (exact ? 4 : 2); p.partial = a.partial + (size_t)t0 * a.ncols;
-        const int rc = exact ? axpy_mm_tokens<AX_Q4_EXACT>(p, grid, a.pdl, st) : q4 ? axpy_mm_tokens<AX_Q4>(p, grid, a.pdl, st) : axpy_mm_tokens<AX_F16>(p, grid, a.pdl, st);
-        if (rc != PI_OK) return rc;
-    }
-    return PI_OK;
+    return exact ? axpy_mm_tokens<AX_Q4_EXACT>(p, grid, a.pdl, st) : q4 ? axpy_mm_tokens<AX_Q4>(p, grid, a.pdl, st) : axpy_mm_tokens<AX_F16>(p, grid, a.pdl, st);
 }
 
 }  // namespace pi

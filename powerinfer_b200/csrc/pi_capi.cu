@@ -63,7 +63,7 @@ static bool carve_sparse(Scratch & s, int64_t n_rows, int T, int coef_size, Spar
 }
 
 // The rows of a gather: activity bit masks, and the sorted list only where the kernel that follows wants one
-static bool wants_list(int T, int64_t n_rows) { return T == 1 || n_rows > MM_MAX_ROWS; }
+static bool wants_list(int wtype, int T, int64_t n_rows, int64_t ncols) { return T == 1 ? !rows_eligible(wtype, n_rows, ncols) : n_rows > MM_MAX_ROWS; }
 
 }  // namespace pi
 
@@ -124,14 +124,13 @@ int pi_mul_mat(int wtype, const void * W, int64_t nrows, int64_t ncols, const fl
     if (!aligned(workspace, 256) || workspace_bytes < act_bytes(wtype, ncols, T)) { set_error("mul_mat: workspace too small or misaligned"); return PI_ERR_WORKSPACE; }
     char * p = (char *)workspace;
     ActBuf act = act_carve(wtype, ncols, T, &p);
-    if ((rc = launch_convert_act(wtype, x, ncols, ncols, T, act, st))) return rc;
     GemvArgs g;
-    g.wtype = wtype; g.W = W; g.nrows = nrows; g.ncols = ncols; g.x = act.view(); g.T = T;
+    g.wtype = wtype; g.W = W; g.nrows = nrows; g.ncols = ncols; g.x = act.view(); g.T = T; g.pdl = true;
     g.bias = bias; g.dst = dst; g.dst_stride = nrows;
-    if (T == 1 && workspace_bytes >= act_bytes(wtype, ncols, T) + 256) {   // room for a status word: the bulk-copy ring kernels are eligible
-        g.status = (unsigned int *)p;
-        PI_CUDA(cudaMemsetAsync(g.status, 0, 4, st));
-    }
+    if (T == 1 && workspace_bytes >= act_bytes(wtype, ncols, T) + 256) g.status = (unsigned int *)p;   // room for a status word: the bulk-copy ring kernels are eligible
+    PrepArgs a;
+    a.wtype = wtype; a.T = T; a.x = x; a.n = ncols; a.act = act; a.words = g.status; a.n_words = 1;
+    if ((rc = launch_prep(a, st))) return rc;
     return launch_gemv(g, st);
 }
 
@@ -148,15 +147,17 @@ int pi_predictor(const void * fc1, const void * fc2, int64_t d, int64_t rank, in
     char * p = (char *)workspace;
     ActBuf a_in = act_carve(PI_TYPE_F16, d, T, &p);
     ActBuf a_h  = act_carve(PI_TYPE_F16, rank, T, &p);
-    if ((rc = launch_convert_act(PI_TYPE_F16, p_in, d, d, T, a_in, st))) return rc;
     GemvArgs g1;                                       // hidden = relu(fc1 . p), kept only in the FP16 form fc2 consumes
+    g1.pdl = true;
     g1.W = fc1; g1.nrows = rank; g1.ncols = d; g1.x = a_in.view(); g1.T = T; g1.relu = 1; g1.dst16 = a_h.h16; g1.dst_stride = rank;
     GemvArgs g2;
     g2.W = fc2; g2.nrows = F; g2.ncols = rank; g2.x = a_h.view(); g2.T = T; g2.dst = idx; g2.dst_stride = F; g2.pdl = true;
     if (T == 1 && workspace_bytes >= act_bytes(PI_TYPE_F16, d, T) + act_bytes(PI_TYPE_F16, rank, T) + 256) {     // as in pi_mul_mat
         g1.status = g2.status = (unsigned int *)p;
-        PI_CUDA(cudaMemsetAsync(p, 0, 4, st));
     }
+    PrepArgs a;
+    a.T = T; a.x = p_in; a.n = d; a.act = a_in; a.words = g1.status; a.n_words = 1;
+    if ((rc = launch_prep(a, st))) return rc;
     if ((rc = launch_gemv(g1, st))) return rc;
     return launch_gemv(g2, st);
 }
@@ -193,20 +194,24 @@ int pi_mul_mat_idx(int wtype, const void * W, int64_t n_w_rows, int64_t ncols,
     char * actp = (char *)s.take(act_bytes(wtype, ncols, T));
     if (!aligned(workspace, 256) || !actp || !carved) { set_error("mul_mat_idx: workspace too small or misaligned"); return PI_ERR_WORKSPACE; }
     ActBuf act = act_carve(wtype, ncols, T, &actp);
-    if (bucket) PI_CUDA(cudaMemsetAsync(dst, 0, (size_t)T * n_dst_rows * 4, st));      // rows held elsewhere read 0
-    PI_CUDA(cudaMemsetAsync(ss.count, 0, 12, st));                                      // count, ticket, status
-    if (n_w_rows == 0) return PI_OK;
-    if ((rc = launch_convert_act(wtype, x, ncols, ncols, T, act, st))) return rc;
-    CompactArgs c;
-    c.idx = idx; c.idx_stride = idx_stride; c.T = T; c.threshold = threshold; c.n_local = n_w_rows; c.bucket = bucket;
-    c.masks = ss.masks;
-    if (wants_list(T, n_w_rows)) { c.list = ss.list; c.count = ss.count; c.ticket = ss.ticket; }
-    c.zero_dst = dst; c.zero_stride = n_dst_rows;
-    if ((rc = launch_compact(c, st))) return rc;
+    if (n_w_rows == 0) { PI_CUDA(cudaMemsetAsync(dst, 0, (size_t)T * n_dst_rows * 4, st)); PI_CUDA(cudaMemsetAsync(ss.count, 0, 12, st)); return PI_OK; }
+    const bool list = wants_list(wtype, T, n_w_rows, ncols);
+    PrepArgs a;                                                       // rows that are inactive or held elsewhere read 0
+    a.wtype = wtype; a.T = T; a.x = x; a.n = ncols; a.act = act; a.zero = dst; a.n_zero = (int64_t)T * n_dst_rows;
+    a.words = (unsigned int *)ss.count; a.n_words = 3;                // count, ticket, status
+    if (!list) { a.idx = idx; a.idx_stride = idx_stride; a.threshold = threshold; a.n_local = n_w_rows; a.bucket = bucket; a.masks = ss.masks; }
+    if ((rc = launch_prep(a, st))) return rc;
+    if (list) {
+        CompactArgs c;
+        c.pdl = true;
+        c.idx = idx; c.idx_stride = idx_stride; c.T = T; c.threshold = threshold; c.n_local = n_w_rows; c.bucket = bucket;
+        c.masks = ss.masks; c.list = ss.list; c.count = ss.count; c.ticket = ss.ticket;
+        if ((rc = launch_compact(c, st))) return rc;
+    }
     GemvArgs g;
+    g.pdl = true;
     g.wtype = wtype; g.W = W; g.nrows = n_w_rows; g.ncols = ncols; g.x = act.view(); g.T = T;
-    if (wants_list(T, n_w_rows)) { g.list = ss.list; g.count = ss.count; }
-    if (T == 1 || n_w_rows <= MM_MAX_ROWS) g.masks = ss.masks;
+    if (list) { g.list = ss.list; g.count = ss.count; } else { g.masks = ss.masks; }
     g.bucket = bucket; g.idx = idx; g.idx_stride = idx_stride; g.threshold = threshold;
     g.dst = dst; g.dst_stride = n_dst_rows; g.status = ss.status;
     return launch_gemv(g, st);
@@ -235,12 +240,18 @@ int pi_axpy(int wtype, const void * Wt, int64_t n_w_rows, int64_t ncols,
     }
     float * partial = ok ? (float *)s.take((size_t)G * T * ncols * 4) : nullptr;
     if (!ok || !partial) { set_error("axpy: workspace too small or misaligned"); return PI_ERR_WORKSPACE; }
-    PI_CUDA(cudaMemsetAsync(ss.count, 0, 12, st));                                      // count, ticket, status
-    CompactArgs c;
-    c.idx = idx; c.idx_stride = idx_stride; c.T = T; c.threshold = threshold; c.n_local = n_w_rows; c.bucket = bucket;
-    c.masks = ss.masks;
-    if (T == 1) { c.list = ss.list; c.count = ss.count; c.ticket = ss.ticket; }              // (batches: launch_coef makes the list)
-    if ((rc = launch_compact(c, st))) return rc;
+    const bool rows1 = T == 1 && axpy_rows_eligible(wtype, n_w_rows, ncols, G);
+    PrepArgs pa;
+    pa.T = T; pa.words = (unsigned int *)ss.count; pa.n_words = 3;                      // count, ticket, status
+    if (T > 1 || rows1) { pa.idx = idx; pa.idx_stride = idx_stride; pa.threshold = threshold; pa.n_local = n_w_rows; pa.bucket = bucket; pa.masks = ss.masks; }
+    if ((rc = launch_prep(pa, st))) return rc;
+    if (T == 1 && !rows1) {                                                             // (batches: launch_coef makes the list)
+        CompactArgs c;
+        c.pdl = true;
+        c.idx = idx; c.idx_stride = idx_stride; c.T = T; c.threshold = threshold; c.n_local = n_w_rows; c.bucket = bucket;
+        c.masks = ss.masks; c.list = ss.list; c.count = ss.count; c.ticket = ss.ticket;
+        if ((rc = launch_compact(c, st))) return rc;
+    }
     AxpyArgs a;
     if (T > 1) {
         CoefArgs k;
@@ -254,7 +265,7 @@ int pi_axpy(int wtype, const void * Wt, int64_t n_w_rows, int64_t ncols,
     a.wtype = wtype; a.Wt = Wt; a.nrows = n_w_rows; a.ncols = ncols; a.h = h; a.h_stride = h_stride; a.T = T;
     a.list = ss.list; a.count = ss.count; a.bucket = bucket; a.idx = idx; a.idx_stride = idx_stride; a.threshold = threshold;
     a.cq = cq; a.cd = cd; a.c_stride = h_stride; a.partial = partial; a.n_groups = G; a.status = ss.status;
-    if (T == 1) a.masks = ss.masks;
+    if (rows1) { a.masks = ss.masks; a.pdl = true; }
     int used = G;
     if ((rc = launch_axpy(a, st, &used))) return rc;
     return launch_reduce_partials(partial, used, T, ncols, nullptr, nullptr, dst, st, true);
@@ -288,9 +299,9 @@ int pi_sparse_ffn(int wtype, const void * up, const void * gate, const void * do
     float * partial = ok && h ? (float *)s.take((size_t)G * T * ncols * 4) : nullptr;
     if (!ok || !h || !partial) { set_error("sparse_ffn: workspace too small or misaligned"); return PI_ERR_WORKSPACE; }
     ActBuf act = act_carve(wtype, ncols, T, &actp);
-    PI_CUDA(cudaMemsetAsync(ss.count, 0, 12, st));                                      // count, ticket, status
-    if (T == 1 && (bucket || wtype == PI_TYPE_Q4_0)) PI_CUDA(cudaMemsetAsync(h, 0, (size_t)F * 4, st));
-    if ((rc = launch_convert_act(wtype, x, ncols, ncols, T, act, st))) return rc;
+    PrepArgs pa;
+    pa.wtype = wtype; pa.T = T; pa.x = x; pa.n = ncols; pa.act = act; pa.words = (unsigned int *)ss.count; pa.n_words = 3;   // count, ticket, status
+    auto prep_masks = [&]() { pa.idx = idx; pa.idx_stride = idx_stride; pa.threshold = threshold; pa.n_local = n_w_rows; pa.bucket = bucket; pa.masks = ss.masks; };
     // the kernels below are chained with programmatic dependent launch: each may start while its predecessor drains
     {
         // one token, every row on this device, no bias that inactive rows would keep: masks, then the whole FFN in one launch
@@ -298,28 +309,32 @@ int pi_sparse_ffn(int wtype, const void * up, const void * gate, const void * do
         f.pdl = true;
         f.wtype = wtype; f.up = up; f.gate = gate; f.down_t = down_t; f.nrows = n_w_rows; f.ncols = ncols;
         f.x = act.view(); f.masks = ss.masks; f.bias = up_bias; f.relu = gate ? 0 : 1;
-        f.h = h; f.partial = partial; f.n_groups = G;
+        f.partial = partial; f.n_groups = G;
         if (T == 1 && !bucket && !(wtype == PI_TYPE_Q4_0 && up_bias) && ffn_rows_eligible(f)) {
-            CompactArgs cm;
-            cm.pdl = true;
-            cm.idx = idx; cm.idx_stride = idx_stride; cm.T = 1; cm.threshold = threshold; cm.n_local = n_w_rows; cm.masks = ss.masks;
-            if ((rc = launch_compact(cm, st))) return rc;
+            prep_masks();
+            if ((rc = launch_prep(pa, st))) return rc;
             int used1 = G;
             if ((rc = launch_ffn_rows(f, st, &used1))) return rc;
             return launch_reduce_partials(partial, used1, 1, ncols, nullptr, nullptr, dst, st, true);
         }
     }
-    CompactArgs c;
-    c.pdl = true;
-    c.idx = idx; c.idx_stride = idx_stride; c.T = T; c.threshold = threshold; c.n_local = n_w_rows; c.bucket = bucket;
-    c.masks = ss.masks;
-    if (wants_list(T, n_w_rows)) { c.list = ss.list; c.count = ss.count; c.ticket = ss.ticket; }
-    if (wtype == PI_TYPE_Q4_0 && T == 1) { c.zero_dst = h; c.zero_stride = F; c.fill_bias = up_bias; c.fill_relu = 1; }
-    if ((rc = launch_compact(c, st))) return rc;
+    if (T > 1 && n_w_rows <= MM_MAX_ROWS) {
+        prep_masks();
+        if ((rc = launch_prep(pa, st))) return rc;
+    } else {
+        if (T == 1 && (bucket || wtype == PI_TYPE_Q4_0)) { pa.zero = h; pa.n_zero = F; }
+        if ((rc = launch_prep(pa, st))) return rc;
+        CompactArgs c;
+        c.pdl = true;
+        c.idx = idx; c.idx_stride = idx_stride; c.T = T; c.threshold = threshold; c.n_local = n_w_rows; c.bucket = bucket;
+        c.masks = ss.masks; c.list = ss.list; c.count = ss.count; c.ticket = ss.ticket;
+        if (wtype == PI_TYPE_Q4_0 && T == 1) { c.zero_dst = h; c.zero_stride = F; c.fill_bias = up_bias; c.fill_relu = 1; }
+        if ((rc = launch_compact(c, st))) return rc;
+    }
     GemvArgs g;
     g.pdl = true;
     g.wtype = wtype; g.W = up; g.W2 = gate; g.nrows = n_w_rows; g.ncols = ncols; g.x = act.view(); g.T = T;
-    if (wants_list(T, n_w_rows)) { g.list = ss.list; g.count = ss.count; }
+    if (T == 1 || n_w_rows > MM_MAX_ROWS) { g.list = ss.list; g.count = ss.count; }
     if (T == 1 || n_w_rows <= MM_MAX_ROWS) g.masks = ss.masks;
     g.bucket = bucket; g.idx = idx; g.idx_stride = idx_stride; g.threshold = threshold;
     g.bias = up_bias; g.relu = gate ? 0 : 1;

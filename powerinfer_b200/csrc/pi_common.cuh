@@ -81,9 +81,16 @@ int launch_q4_0_repack(const void * src, void * dst, int64_t nrows, int64_t ncol
 int launch_dequantize_q4_0(const void * q4p, float * y, int64_t nrows, int64_t ncols, cudaStream_t st);
 int launch_quantize_q8_0_ggml(const float * x, void * q8, int64_t nrows, int64_t ncols, cudaStream_t st);
 
-// x F32 [T, n] (row stride x_stride) -> activation planes for `wtype` weights
-int launch_convert_act(int wtype, const float * x, int64_t x_stride, int64_t n, int T, ActBuf out, cudaStream_t st);
-
+// One launch in front of an operator's kernels (every part optional): x F32 [T, n] -> activation planes for `wtype` weights; predictor
+// logits -> activity bit masks (one word per 32 local rows, the union over the tokens); zeros; control words cleared.
+struct PrepArgs {
+    int wtype = PI_TYPE_F16; int T = 1;
+    const float * x = nullptr; int64_t n = 0; ActBuf act;
+    const float * idx = nullptr; int64_t idx_stride = 0; float threshold = 0.f; int64_t n_local = 0; const int32_t * bucket = nullptr; uint32_t * masks = nullptr;
+    float * zero = nullptr; int64_t n_zero = 0;
+    unsigned int * words = nullptr; int n_words = 0;
+};
+int launch_prep(const PrepArgs & a, cudaStream_t st);
 
 struct GemvArgs {
     int wtype = PI_TYPE_F16;
@@ -125,6 +132,7 @@ int launch_gemv(const GemvArgs & a, cudaStream_t st);
 // PI_ERR_UNSUPPORTED: not eligible; *wrote_masks: the kernel that ran honoured masks_out itself
 int launch_gemv_ring(const GemvArgs & a, unsigned int * status, bool pdl, cudaStream_t st, bool * wrote_masks = nullptr);
 int launch_mm(const GemvArgs & a, cudaStream_t st);                                           // 2+ tokens; PI_ERR_UNSUPPORTED: not eligible
+int launch_mm_wide(const GemvArgs & a, cudaStream_t st);                                      // 33+ tokens (called by launch_mm)
 static constexpr int64_t MM_MAX_ROWS = 262144;                                                // rows a gather of launch_mm can choose from
 
 // predictor logits -> compacted list of LOCAL rows active for >= 1 token; also writes zeros (or relu(bias)) into
@@ -166,7 +174,7 @@ int axpy_groups(int wtype, int64_t ncols, int T);                     // row gro
 int launch_axpy(const AxpyArgs & a, cudaStream_t st, int * groups_used = nullptr);   // groups_used: partial vectors written
 int launch_axpy_mm(const AxpyArgs & a, cudaStream_t st, int * groups_used);          // 2+ tokens, needs coef; PI_ERR_UNSUPPORTED: not eligible
 bool axpy_mm_exact(int wtype, int64_t ncols);                                        // coefficients are F32, else FP16
-int axpy_mm_pieces(int64_t ncols);                                                   // partial vectors launch_axpy_mm writes
+int axpy_mm_pieces(int64_t ncols, int T);                                            // partial vectors launch_axpy_mm writes
 // axpy coefficients by list position (pi_axpy_mm.cu): [T, coef_stride], FP16 or (exact) F32, from h F32 [T, h_stride] by global neuron id
 struct CoefArgs {
     int wtype = PI_TYPE_F16;
@@ -184,6 +192,7 @@ int launch_coef(const CoefArgs & a, cudaStream_t st);
 bool rows_eligible(int wtype, int64_t nrows, int64_t ncols);
 int launch_gather_rows(const GemvArgs & a, cudaStream_t st);
 int launch_axpy_rows(const AxpyArgs & a, cudaStream_t st, int * groups_used);
+bool axpy_rows_eligible(int wtype, int64_t nrows, int64_t ncols, int n_groups);
 int axpy_rows_groups(int64_t nrows, int64_t ncols);                                  // partial vectors launch_axpy_rows writes
 // one token, the whole sparse FFN in one launch (pi_ffn_rows.cu): h = act(up/gate rows . x) over the rows the masks name,
 // partial[c] = sum of the rows of down_t times their coefficients, one partial vector per cluster (groups_used of them, at

@@ -11,6 +11,7 @@
 
 #include <cmath>
 #include <cstdlib>
+#include <algorithm>
 #include <cstring>
 #include <new>
 #include <vector>
@@ -38,29 +39,78 @@ __global__ void k_embed(const __half * __restrict__ tok_embd, const __half * __r
     }
 }
 
-// llama_sample_token_greedy (llama.cpp:8617): first index of the maximum of the raw logits
-__global__ void __launch_bounds__(1024) k_argmax(const float * __restrict__ logits, int n, int32_t * __restrict__ out) {
-    __shared__ float s_v[32];
-    __shared__ int s_i[32];
-    const float * row = logits + (size_t)blockIdx.x * n;
-    float bv = -INFINITY; int bi = 0x7fffffff;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const float v = row[i];
-        if (v > bv) { bv = v; bi = i; }
+// llama_sample_token_greedy (llama.cpp:8617): first index of the maximum of the raw logits.
+// Latency: one CTA per row reads its 32000 logits in 32 dependent rounds (12 us; 26 us for 65000).  Here a row is cut into pieces of
+// ARG_PIECE logits, each read in one round; the pieces meet in one 64-bit word per row, (order-preserving bits of the value, ~index),
+// by atomicMax, and the CTA that arrives last writes the index and clears the word for the next step (3 us).
+static constexpr int ARG_THREADS = 256, ARG_UN = 8, ARG_PIECE = ARG_THREADS * ARG_UN;
+
+__global__ void __launch_bounds__(ARG_THREADS) k_argmax(const float * __restrict__ logits, int n, unsigned long long * __restrict__ best,
+                                                        unsigned int * __restrict__ ticket, int32_t * __restrict__ out, int32_t ** __restrict__ sink) {
+    __shared__ unsigned long long s_k[ARG_THREADS / 32];
+    const int t = blockIdx.y, lane = threadIdx.x & 31;
+    const float * row = logits + (size_t)t * n;
+    pdl_wait();
+    float v[ARG_UN];
+#pragma unroll
+    for (int u = 0; u < ARG_UN; u++) {
+        const int i = blockIdx.x * ARG_PIECE + u * ARG_THREADS + threadIdx.x;
+        v[u] = i < n ? row[i] : -INFINITY;
+    }
+    unsigned long long key = 0ull;                                    // (a NaN or -inf is never chosen: index 0 if there is nothing else)
+#pragma unroll
+    for (int u = 0; u < ARG_UN; u++) {
+        if (!(v[u] > -INFINITY)) continue;
+        const unsigned b = __float_as_uint(v[u] + 0.f);               // (-0 counts as 0)
+        const unsigned i = blockIdx.x * ARG_PIECE + u * ARG_THREADS + threadIdx.x;
+        const unsigned long long k = ((unsigned long long)(b >> 31 ? ~b : b | 0x80000000u) << 32) | ~i;
+        key = k > key ? k : key;
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-        const int   oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-    }
-    if ((threadIdx.x & 31) == 0) { s_v[threadIdx.x >> 5] = bv; s_i[threadIdx.x >> 5] = bi; }
+    for (int o = 16; o > 0; o >>= 1) { const unsigned long long k = __shfl_xor_sync(0xffffffffu, key, o); key = k > key ? k : key; }
+    if (lane == 0) s_k[threadIdx.x >> 5] = key;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); w++)
-            if (s_v[w] > bv || (s_v[w] == bv && s_i[w] < bi)) { bv = s_v[w]; bi = s_i[w]; }
-        out[blockIdx.x] = bi == 0x7fffffff ? 0 : bi;
-    }
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < ARG_THREADS / 32; w++) key = s_k[w] > key ? s_k[w] : key;
+    if (key) atomicMax(best + t, key);
+    __threadfence();
+    if (atomicAdd(ticket + t, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    const unsigned long long k = atomicExch(best + t, 0ull);
+    ticket[t] = 0u;
+    const int32_t i = k ? (int32_t)~(unsigned)k : 0;
+    out[t] = i;
+    int32_t * host = sink[t];                                         // (for this step only)
+    if (host) { *host = i; sink[t] = nullptr; }
+}
+
+// Tokens of a prompt that go through the layers together, whatever the engine's batch: a chunk reads the weights once, and 77 tokens of
+// the 7B shape in one chunk take 1.0 ms where three chunks of up to 32 took 3.5.  256: beyond it the products are all that is left.
+static constexpr int PROMPT_CHUNK = 256;
+
+// A step's token ids and positions travel as kernel arguments: one launch instead of two copies, and the caller's arrays are free again
+// as soon as it returns.  `sink`: where the greedy ids go besides the engine's own buffer (mapped host memory, or nowhere): a few bytes
+// written by the kernel that finds them, where a copy of their own is 6 us behind the logits'.
+struct Feed { int32_t token[PI_MAX_BATCH], pos[PI_MAX_BATCH]; int32_t * sink; };
+
+// a prompt chunk: consecutive positions of one sequence
+struct FeedPrompt { int32_t token[PROMPT_CHUNK]; };
+
+__global__ void __launch_bounds__(PROMPT_CHUNK) k_feed_prompt(const FeedPrompt f, int T, int pos0, int seq, int32_t * __restrict__ tokens, int32_t * __restrict__ pos,
+                                                              int32_t * __restrict__ seq_pf) {
+    const int t = threadIdx.x;
+    if (t >= T) return;
+    tokens[t] = f.token[t];
+    pos[t] = pos0 + t;
+    seq_pf[t] = seq;
+}
+
+__global__ void k_feed(const Feed f, int T, int32_t * __restrict__ tokens, int32_t * __restrict__ pos, int32_t ** __restrict__ sink) {
+    const int t = threadIdx.x;
+    if (t >= T) return;
+    sink[t] = f.sink ? f.sink + t : nullptr;
+    tokens[t] = f.token[t];
+    pos[t] = f.pos[t];
 }
 
 // Keeps the stream busy for a fixed time (profiling only): while it sleeps the host queues the whole step behind it, so
@@ -104,7 +154,8 @@ struct pi_engine {
     std::vector<pi_layer_weights> layers;
     pi_model_weights g;
     int hd, dq, dkv, F, T_max;
-    int G, pieces;                           // axpy row groups (one token), partial vectors of a batch
+    int P_max;                               // tokens of a prompt chunk (>= T_max)
+    int G;                                   // axpy row groups (one token)
     // device buffers carved from the caller's workspace
     int32_t * tokens, * pos, * seq_ids, * seq_pf, * argmax;   // seq_pf: the sequence of every token of a prompt chunk
     float * x, * x2, * attn_out, * ffn_vec, * qkv, * pred, * h, * partial, * logits, * cs;
@@ -114,6 +165,8 @@ struct pi_engine {
     __half * hidden16;
     ActBuf act_a, act_q, act_p, act_o;       // FFN input, QKV input, predictor input (FP16), out-proj input
     __half * k_cache, * v_cache;             // [n_layer, max_batch, n_ctx, dkv]
+    unsigned long long * amax_best; unsigned int * amax_ticket;   // k_argmax: a word per row, 0 between steps
+    int32_t ** sink;                         // per row: where the step's greedy id goes as well (null for steps fed on the device)
     unsigned int * status;                   // device word: bit 0 = an exchange wait ran out
     unsigned long long * active_total;       // device counter: sum of active-list lengths over layers and steps
     pi_exchange xch;
@@ -155,17 +208,18 @@ struct Carver {
 static void carve(pi_engine * e, void * ws, size_t ws_bytes, bool dry, size_t * need) {
     const pi_engine_config & c = e->c;
     Carver cv{(char *)ws, dry ? (char *)ws + (size_t(1) << 60) : (char *)ws + ws_bytes};
-    const int T = e->T_max;
+    const int T = e->P_max, B = e->T_max;                            // tokens of the largest step, of the largest decode step
     const size_t d = c.d, F = e->F;
-    e->tokens = cv.take<int32_t>(T); e->pos = cv.take<int32_t>(T); e->seq_ids = cv.take<int32_t>(T); e->seq_pf = cv.take<int32_t>(T); e->argmax = cv.take<int32_t>(T);
+    e->tokens = cv.take<int32_t>(T); e->pos = cv.take<int32_t>(T); e->seq_ids = cv.take<int32_t>(B); e->seq_pf = cv.take<int32_t>(T); e->argmax = cv.take<int32_t>(B);
+    e->amax_best = cv.take<unsigned long long>(B); e->amax_ticket = cv.take<unsigned int>(B); e->sink = cv.take<int32_t *>(B);
     e->status = cv.take<unsigned int>(1); e->active_total = cv.take<unsigned long long>(1);
     e->x = cv.take<float>(T * d); e->x2 = cv.take<float>(T * d); e->attn_out = cv.take<float>(T * d); e->ffn_vec = cv.take<float>(T * d);
     e->qkv = cv.take<float>((size_t)T * (e->dq + 2 * e->dkv));
     e->pred = cv.take<float>(T * F); e->h = cv.take<float>(T * F);
-    e->pieces = axpy_mm_pieces(c.d);
-    const size_t vecs = (size_t)e->pieces * T;                       // partial vectors of a batch, of one token
+    size_t vecs = 0;                                                 // partial vectors of 2+ tokens, of one token
+    for (int t = 2; t <= T; t++) vecs = std::max(vecs, (size_t)axpy_mm_pieces(c.d, t) * t);
     e->partial = cv.take<float>((vecs > (size_t)e->G ? vecs : (size_t)e->G) * d);
-    e->logits = cv.take<float>((size_t)T * c.n_vocab);
+    e->logits = cv.take<float>((size_t)B * c.n_vocab);
     e->cs = cv.take<float>((size_t)c.n_ctx * e->hd);
     e->list = cv.take<int32_t>(F); e->count = cv.take<int32_t>(1); e->ticket = cv.take<unsigned int>(1);
     e->masks = cv.take<uint32_t>((F + 63) / 64 * 2);
@@ -179,6 +233,11 @@ static void carve(pi_engine * e, void * ws, size_t ws_bytes, bool dry, size_t * 
     e->act_o = cv.act(c.wtype, e->dq, T);
     *need = (size_t)(cv.p - (char *)ws);
     if (!cv.ok && !dry) *need = (size_t)-1;
+}
+
+// (a sharded run exchanges whole steps through mailboxes sized for the batch)
+static int prompt_chunk(const pi_engine_config & c) {
+    return c.n_ranks > 1 ? c.max_batch : std::max(c.max_batch, std::min(PROMPT_CHUNK, c.n_ctx));
 }
 
 static int validate(const pi_engine_config & c) {
@@ -207,7 +266,7 @@ size_t pi_engine_workspace_bytes(const pi_engine_config * cfg) {
     pi_engine e{};
     e.c = *cfg;
     e.hd = cfg->d / cfg->n_head; e.dq = cfg->d / cfg->n_ranks; e.dkv = e.hd * cfg->n_head_kv / cfg->n_ranks;
-    e.F = cfg->n_ff / cfg->n_ranks; e.T_max = cfg->max_batch;
+    e.F = cfg->n_ff / cfg->n_ranks; e.T_max = cfg->max_batch; e.P_max = prompt_chunk(*cfg);
     e.G = axpy_groups(cfg->wtype, cfg->d, cfg->max_batch);
     size_t need = 0;
     carve(&e, nullptr, 0, true, &need);
@@ -236,7 +295,7 @@ int pi_engine_create(const pi_engine_config * cfg, const pi_model_weights * gw, 
     if (e->gate_sym) e->c.arch = PI_ARCH_LLAMA;
     e->layers.assign(lw, lw + cfg->n_layer);
     e->hd = cfg->d / cfg->n_head; e->dq = cfg->d / cfg->n_ranks; e->dkv = e->hd * cfg->n_head_kv / cfg->n_ranks;
-    e->F = cfg->n_ff / cfg->n_ranks; e->T_max = cfg->max_batch;
+    e->F = cfg->n_ff / cfg->n_ranks; e->T_max = cfg->max_batch; e->P_max = prompt_chunk(*cfg);
     e->G = axpy_groups(cfg->wtype, cfg->d, cfg->max_batch);
     size_t need = 0;
     carve(e, workspace, workspace_bytes, false, &need);
@@ -261,6 +320,9 @@ int pi_engine_create(const pi_engine_config * cfg, const pi_model_weights * gw, 
     cudaError_t ce = cudaMemcpyAsync(e->seq_ids, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice, st);
     if (ce == cudaSuccess) ce = cudaMemcpyAsync(e->cs, cs.data(), cs.size() * 4, cudaMemcpyHostToDevice, st);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(e->ticket, 0, 4, st);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(e->amax_best, 0, (size_t)e->T_max * 8, st);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(e->amax_ticket, 0, (size_t)e->T_max * 4, st);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(e->sink, 0, (size_t)e->T_max * sizeof *e->sink, st);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(e->count, 0, 4, st);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(e->status, 0, 4, st);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(e->active_total, 0, 8, st);
@@ -412,18 +474,28 @@ int enqueue_step(pi_engine * e, int T, cudaStream_t st, StageTimer & tm, int mod
         if (pend.any()) norm_inputs(e, pend, n1, &xch_index, xch_per_step); else n1.x = e->x;
         if (last && mode == 2) break;
         if (last) {
+            // a prompt chunk: only its last token's logits are wanted (a sharded run exchanges, and so normalises, all of them),
+            // and they stand in the first row
+            const int head = mode == 1 && !multi ? T - 1 : 0, HT = T - head;
+            if (head) {
+                n1.T = HT;
+                if (n1.partial) { n1.partial += (size_t)head * d; n1.partial_stride = (int64_t)T * d; } else { n1.x += (size_t)head * d; }
+                if (n1.residual) n1.residual += (size_t)head * d;
+                if (n1.residual2) n1.residual2 += (size_t)head * d;
+                if (n1.x_out) n1.x_out += (size_t)head * d;
+            }
             const int out_t = e->g.output ? wt : PI_TYPE_F16;            // opt: tied F16 embedding
             n1.act_type = out_t; n1.act = out_t == wt ? e->act_a : e->act_p;
             STAGE(PI_STAGE_NORM, 1, launch_norm(n1, st));
             GemvArgs g;
             g.status = e->status; g.pdl = pdl;
             g.wtype = out_t; g.W = e->g.output ? e->g.output : e->g.tok_embd; g.nrows = c.n_vocab; g.ncols = d;
-            g.x = n1.act.view(); g.T = T; g.dst = e->logits; g.dst_stride = c.n_vocab;
+            g.x = n1.act.view(); g.T = HT; g.dst = e->logits; g.dst_stride = c.n_vocab;
             STAGE(PI_STAGE_LM_HEAD, 1, launch_gemv(g, st));
             if (!(e->skip_mask & (1u << PI_STAGE_OTHER))) {
                 if (tm.begin()) return PI_ERR_CUDA;
-                k_argmax<<<T, 1024, 0, st>>>(e->logits, c.n_vocab, e->argmax);
-                PI_LAUNCH_CHECK("k_argmax");
+                PI_CUDA(launch_k(k_argmax, dim3((c.n_vocab + ARG_PIECE - 1) / ARG_PIECE, HT), dim3(ARG_THREADS), 0, st, pdl, e->logits,
+                                 c.n_vocab, e->amax_best, e->amax_ticket, e->argmax, e->sink));
                 if (tm.end(PI_STAGE_OTHER)) return PI_ERR_CUDA;
                 e->launches++;
             }
@@ -573,7 +645,7 @@ int enqueue_step(pi_engine * e, int T, cudaStream_t st, StageTimer & tm, int mod
                 a.wtype = wt; a.Wt = L->down_t; a.nrows = F; a.ncols = d; a.h = e->h; a.h_stride = F; a.T = T;
                 if (T == 1 && rows1) { a.masks = e->masks; a.h_uncleared = masks1; } else { a.list = e->list; a.count = e->count; }
                 a.idx = pred; a.idx_stride = F; a.threshold = c.threshold;
-                a.cq = e->cq; a.cd = e->cd; a.c_stride = F; a.partial = e->partial; a.n_groups = T == 1 ? e->G : e->pieces; a.status = e->status;
+                a.cq = e->cq; a.cd = e->cd; a.c_stride = F; a.partial = e->partial; a.n_groups = T == 1 ? e->G : axpy_mm_pieces(d, T); a.status = e->status;
                 if (T > 1) { a.coef = e->coef; a.coef_stride = e->coef_stride; }
                 STAGE(PI_STAGE_DOWN, 1, launch_axpy(a, st, &used));
             }
@@ -615,9 +687,18 @@ int count_kernel_nodes(cudaGraph_t graph) {
     return k;
 }
 
+// the device's address of pinned host memory, null for other memory
+int32_t * mapped(int32_t * host) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, host) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    return a.type == cudaMemoryTypeHost ? (int32_t *)a.devicePointer : nullptr;
+}
+
 // first call for a batch size: one plain run (fills every per-kernel attribute cache), then capture
 int run_step(pi_engine * e, int T, cudaStream_t st, int mode = 0) {
     StageTimer tm;
+    // A chunk beyond the batch: its length seldom comes again, and its kernels are longer than their launches
+    if (T > e->T_max) return enqueue_step(e, T, st, tm, mode);
     if (e->graphs[mode][T]) { PI_CUDA(cudaGraphLaunch(e->graphs[mode][T], st)); e->launches = e->graph_nodes[mode][T]; return PI_OK; }
     if (!e->warmed[mode][T]) {
         e->warmed[mode][T] = true;
@@ -665,11 +746,15 @@ int pi_engine_decode_host(pi_engine * e, const int32_t * host_tokens, const int3
     PI_REQUIRE(host_tokens && host_pos, "engine_decode_host: null input");
     cudaStream_t st = (cudaStream_t)stream;
     for (int t = 0; t < T; t++) PI_REQUIRE(host_pos[t] >= 0 && host_pos[t] < e->c.n_ctx, "engine_decode_host: position %d outside the context of %d", host_pos[t], e->c.n_ctx);
-    PI_CUDA(cudaMemcpyAsync(e->tokens, host_tokens, (size_t)T * 4, cudaMemcpyHostToDevice, st));
-    PI_CUDA(cudaMemcpyAsync(e->pos, host_pos, (size_t)T * 4, cudaMemcpyHostToDevice, st));
-    if ((rc = run_step(e, T, st))) return rc;
+    Feed f;
+    memcpy(f.token, host_tokens, (size_t)T * 4);
+    memcpy(f.pos, host_pos, (size_t)T * 4);
+    f.sink = host_argmax ? mapped(host_argmax) : nullptr;
+    k_feed<<<1, PI_MAX_BATCH, 0, st>>>(f, T, e->tokens, e->pos, e->sink);
+    PI_LAUNCH_CHECK("k_feed");
+    if ((rc = run_step(e, T, st))) { cudaMemsetAsync(e->sink, 0, (size_t)T * sizeof *e->sink, st); return rc; }
+    if (host_argmax && !f.sink) PI_CUDA(cudaMemcpyAsync(host_argmax, e->argmax, (size_t)T * 4, cudaMemcpyDeviceToHost, st));
     if (host_logits) PI_CUDA(cudaMemcpyAsync(host_logits, e->logits, (size_t)T * e->c.n_vocab * 4, cudaMemcpyDeviceToHost, st));
-    if (host_argmax) PI_CUDA(cudaMemcpyAsync(host_argmax, e->argmax, (size_t)T * 4, cudaMemcpyDeviceToHost, st));
     PI_CUDA(cudaStreamSynchronize(st));
     return PI_OK;
 }
@@ -682,22 +767,21 @@ int pi_engine_prefill_host(pi_engine * e, const int32_t * host_tokens, int n_tok
     int rc = check_T(e, 1);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    std::vector<int32_t> ids(e->T_max, seq), pos(e->T_max);
-    PI_CUDA(cudaMemcpyAsync(e->seq_pf, ids.data(), (size_t)e->T_max * 4, cudaMemcpyHostToDevice, st));
-    int last_T = 0;
-    for (int t0 = 0; t0 < n_tokens; t0 += e->T_max) {
-        const int T = n_tokens - t0 < e->T_max ? n_tokens - t0 : e->T_max;
+    const int most = e->pred_trace ? e->T_max : e->P_max;             // (a trace holds max_batch tokens of a step)
+    int row = 0;                                                      // of the last token's logits
+    for (int t0 = 0; t0 < n_tokens; t0 += most) {
+        const int T = n_tokens - t0 < most ? n_tokens - t0 : most;
         const bool final_chunk = t0 + T == n_tokens;
-        for (int t = 0; t < T; t++) pos[t] = pos0 + t0 + t;
-        PI_CUDA(cudaMemcpyAsync(e->tokens, host_tokens + t0, (size_t)T * 4, cudaMemcpyHostToDevice, st));
-        PI_CUDA(cudaMemcpyAsync(e->pos, pos.data(), (size_t)T * 4, cudaMemcpyHostToDevice, st));
-        PI_CUDA(cudaStreamSynchronize(st));                               // `pos` is rewritten for the next chunk
+        FeedPrompt f;
+        memcpy(f.token, host_tokens + t0, (size_t)T * 4);
+        k_feed_prompt<<<1, PROMPT_CHUNK, 0, st>>>(f, T, pos0 + t0, seq, e->tokens, e->pos, e->seq_pf);
+        PI_LAUNCH_CHECK("k_feed_prompt");
         const bool head = final_chunk && (host_logits_last || host_argmax_last);
         if ((rc = run_step(e, T, st, head ? 1 : 2))) return rc;
-        last_T = T;
+        row = e->c.n_ranks > 1 ? T - 1 : 0;
     }
-    if (host_logits_last) PI_CUDA(cudaMemcpyAsync(host_logits_last, e->logits + (size_t)(last_T - 1) * e->c.n_vocab, (size_t)e->c.n_vocab * 4, cudaMemcpyDeviceToHost, st));
-    if (host_argmax_last) PI_CUDA(cudaMemcpyAsync(host_argmax_last, e->argmax + (last_T - 1), 4, cudaMemcpyDeviceToHost, st));
+    if (host_logits_last) PI_CUDA(cudaMemcpyAsync(host_logits_last, e->logits + (size_t)row * e->c.n_vocab, (size_t)e->c.n_vocab * 4, cudaMemcpyDeviceToHost, st));
+    if (host_argmax_last) PI_CUDA(cudaMemcpyAsync(host_argmax_last, e->argmax + row, 4, cudaMemcpyDeviceToHost, st));
     PI_CUDA(cudaStreamSynchronize(st));
     return PI_OK;
 }

@@ -1,0 +1,450 @@
+// Mat-mat over FP16 and planar Q4_0 rows for MORE than 32 tokens (prompt chunks of up to 256): the same operators, row selection and
+// epilogue as pi_mm.cu, another split of the work.
+//
+// Bound: with 77 FP16 tokens the tensor pipe and HBM are about even (12288 x 4096: 17 us of mma.sync at 955 multiply-adds per clock
+// and SM, 15 us of weights); above that the products.  Q4_0 is bound by the scaling of its blocks: an mma of 16 rows x 32 columns x
+// 8 tokens and the four packed FP32 operations that apply its scales take 18 clocks of a scheduler together (they share a pipe).
+// What must not cost extra is shared memory: every warp reads its own fragments of both operands.
+//
+// Work split: as in pi_mm.cu every CTA takes an equal contiguous range of rows, in tiles of 32, 64 or 128; here the 16 warps share a
+// stage (128 bytes of every activation, 128 or 64 of every row) and split the TILE, WM ways along the rows and WN along the tokens:
+// no partial sums, so the accumulators of a tile exist once and the tile can be 128 x 256.  A stage holds enough products (2000
+// clocks of them at 128 x 128) for its barrier.  Warps without rows or tokens do nothing, and are spread over the four schedulers.
+// The accumulators go straight to global memory: the ring runs on across tiles.
+#include "pi_common.cuh"
+
+namespace pi {
+
+static constexpr int MW_THREADS = 512;
+static constexpr int MW_SMEM_MAX = 224 * 1024;
+static constexpr int MW_SMAX = 6;                       // stages at most
+static constexpr int MW_TOKENS = 256;                   // of a launch
+
+struct MwP {
+    const uint8_t * W; const uint8_t * W2; int64_t row_bytes; int nrows, ncols, nb;
+    Act x; int T;
+    const uint32_t * masks; const int32_t * bucket; int32_t * list; int32_t * count; unsigned long long * rows_total;
+    const float * idx; int64_t idx_stride; float threshold;
+    const float * bias; int relu;
+    float * dst; __half * dst16; int64_t dst_stride;
+    __half * coef; int64_t coef_stride;
+    uint32_t * masks_out; float masks_threshold; int masks_or;
+    int n_slices, stage, S;                             // column slices of a row; bytes of a stage; stages
+};
+
+__device__ __forceinline__ void mw_cp16(uint32_t dst, const void * src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void mw_cp8(uint32_t dst, const void * src)  { asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" :: "r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void mw_cp4(uint32_t dst, const void * src)  { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void mw_zero16(uint32_t dst) { asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" :: "r"(dst), "r"(0u) : "memory"); }
+__device__ __forceinline__ void mw_wait(int pending) {                // all but the last `pending` (0 .. MW_SMAX - 2) groups have landed
+    switch (pending) {
+        case 0: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
+        case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
+        case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+        case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
+        default: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
+    }
+}
+__device__ __forceinline__ void mw_ldsm4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void mw_hmma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mw_imma(uint32_t (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, uint32_t c) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c));
+}
+__device__ __forceinline__ unsigned long long mw_pack(float a, float b) { unsigned long long r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ unsigned long long mw_packu(uint32_t a, uint32_t b) { unsigned long long r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b)); return r; }
+__device__ __forceinline__ unsigned long long mw_mul2(unsigned long long a, unsigned long long b) { unsigned long long r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+// acc += (v * dd - magic * dd) * d4, two tokens at a time: exact up to the two roundings of (v - magic) * dd * d4 (see pi_mm.cu)
+__device__ __forceinline__ void mw_scale_add(unsigned long long & acc, unsigned long long v, unsigned long long dd, unsigned long long md, unsigned long long d4) {
+    asm("{\n .reg .b64 t;\n fma.rn.f32x2 t, %1, %2, %3;\n fma.rn.f32x2 %0, t, %4, %0;\n}" : "+l"(acc) : "l"(v), "l"(dd), "l"(md), "l"(d4));
+}
+
+// MT x 16 rows and NT x 8 tokens per warp; WM x WN warps
+template <int WT, int MT, int WM, int WN, int NT>
+struct MwShape {
+    static constexpr bool Q4 = WT == PI_TYPE_Q4_0;
+    static constexpr int TM = WM * MT * 16, TN = WN * NT * 8;
+    static constexpr int KS = Q4 ? 128 : 64;                          // columns of a stage
+    static constexpr int WB = Q4 ? 64 : 128;                          // bytes of a row in a stage (Q4_0: of its nibbles)
+    static_assert(WM * WN * 32 == MW_THREADS, "warps");
+};
+
+template <int WT, int MT, int WM, int WN, int NT, bool SPARSE, bool GATED>
+__global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
+    using Z = MwShape<WT, MT, WM, WN, NT>;
+    constexpr bool Q4 = Z::Q4;
+    constexpr int TM = Z::TM, WB = Z::WB;
+    constexpr int IT = GATED ? TM / 2 : TM;                           // items (rows / neurons) of a tile
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ int s_warp[MW_THREADS / 32];
+    __shared__ unsigned s_any[4];
+    int * rows = reinterpret_cast<int *>(smem + (size_t)p.S * p.stage);          // rows of this CTA (sparse only)
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wm = WM == 4 ? (warp + (warp >> 2)) & 3 : (warp + (warp >> 2)) & 1, wn = WM == 4 ? warp >> 2 : warp >> 1;
+    const int G = gridDim.x, cta = blockIdx.x, S = p.S;
+    const uint32_t ring = smem_u32(smem);
+    const int XR = (p.T + 15) / 16 * 16;                              // token rows of a stage
+    // a stage: rows [TM][WB], activations [XR][128], Q4_0: rows' scales [TM][4 halves], activation scales [4][XR] floats
+    const uint32_t x_off = TM * WB, s_off = x_off + XR * 128, d_off = s_off + TM * 8;
+    if (tid < 4) s_any[tid] = 0u;
+    pdl_launch();
+
+    int lo = 0, hi = 0, n_units = 0;
+    auto set_range = [&](int n) {
+        const int al = !SPARSE && p.masks_out ? 8 : 1;                // (a byte of the masks has one writer)
+        const int gr = (n + al - 1) / al;
+        lo = min(n, (int)((long long)gr * cta / G) * al);
+        hi = min(n, (int)((long long)gr * (cta + 1) / G) * al);
+        n_units = (hi - lo + IT - 1) / IT * p.n_slices;
+    };
+    // ---- copies: a thread's pieces of a stage lie in the same rows for a whole tile
+    constexpr int CW = WB / 16;                                       // 16-byte pieces of a row
+    constexpr int NW = (TM * CW + MW_THREADS - 1) / MW_THREADS;
+    const int cw = tid % CW;
+    const uint8_t * wp[NW]; const uint8_t * sp = nullptr;             // nullptr: no such row
+    int i_tile = 0, i_slice = 0;                                      // the unit that is requested next
+    auto row_ptr = [&](int r) -> const uint8_t * {                    // fragment row r of the tile (gated: 8 up rows, then their 8 gate rows)
+        const int k = i_tile * IT + (GATED ? (r >> 4) * 8 + (r & 7) : r);
+        if (r >= TM || lo + k >= hi) return nullptr;
+        return (GATED && (r & 8) ? p.W2 : p.W) + (size_t)(SPARSE ? rows[k] : lo + k) * p.row_bytes;
+    };
+    auto issue_w = [&](int slot) {
+        if (i_slice == 0) {
+#pragma unroll
+            for (int j = 0; j < NW; j++) wp[j] = row_ptr(tid / CW + j * (MW_THREADS / CW));
+            if (Q4) sp = row_ptr(tid);
+        }
+        const uint32_t base = ring + (uint32_t)(slot * p.stage);
+        const int off = i_slice * WB + cw * 16;
+        const bool in = Q4 || off < p.ncols * 2;                      // past the end of a row: zeros
+#pragma unroll
+        for (int j = 0; j < NW; j++) {
+            const int r = tid / CW + j * (MW_THREADS / CW);
+            const uint32_t to = base + r * WB + (Q4 ? (cw ^ (r >> 1)) & 3 : (cw ^ r) & 7) * 16;
+            if (wp[j]) { if (in) mw_cp16(to, wp[j] + off); else mw_zero16(to); }
+        }
+        if (Q4 && sp) mw_cp8(base + s_off + tid * 8, sp + (size_t)p.nb * 16 + i_slice * 8);
+    };
+    auto issue_x = [&](int slot) {
+        const uint32_t base = ring + (uint32_t)(slot * p.stage);
+        const int c = tid & 7;
+#pragma unroll
+        for (int j = 0; j < MW_TOKENS / 64; j++) {
+            const int t = (tid >> 3) + j * 64;
+            if (t >= p.T) break;
+            const uint32_t to = base + x_off + t * 128 + ((c ^ t) & 7) * 16;
+            if (Q4) {
+                mw_cp16(to, (c & 1 ? p.x.hi : p.x.lo) + (size_t)t * p.nb + i_slice * 4 + (c >> 1));
+            } else {
+                const int col = i_slice * 64 + c * 8;
+                if (col < p.ncols) mw_cp16(to, p.x.h16 + (size_t)t * p.ncols + col); else mw_zero16(to);
+            }
+        }
+        if (Q4) {
+#pragma unroll
+            for (int j = 0; j < MW_TOKENS / 128; j++) {
+                const int t = (tid >> 2) + j * 128, k = tid & 3;
+                if (t < p.T) mw_cp4(base + d_off + (k * XR + t) * 4, p.x.d + (size_t)t * p.nb + i_slice * 4 + k);
+            }
+        }
+    };
+    auto advance = [&]() { if (++i_slice == p.n_slices) { i_slice = 0; i_tile++; } };
+
+    if (!SPARSE) {
+        set_range(p.nrows);
+        pdl_wait();                                                   // (the stages are many and long: nothing to gain before the wait)
+    } else {
+        pdl_wait();
+        // ---- ranks of the active rows: thread t counts the words [c0, c1), a block scan gives the rank of its first row
+        constexpr int KEEP = 4;
+        const int n_chunks = (p.nrows + 31) / 32, per = (n_chunks + MW_THREADS - 1) / MW_THREADS;
+        const int c0 = min(tid * per, n_chunks), c1 = min(c0 + per, n_chunks);
+        auto word = [&](int c) {
+            const uint32_t m = __ldcg(p.masks + c);
+            const int left = p.nrows - c * 32;                        // bits beyond the last row never count
+            return left < 32 ? m & ((1u << left) - 1u) : m;
+        };
+        uint32_t mw[KEEP];
+        int mine = 0;
+#pragma unroll
+        for (int k = 0; k < KEEP; k++) { mw[k] = c0 + k < c1 ? word(c0 + k) : 0u; mine += __popc(mw[k]); }
+        for (int c = c0 + KEEP; c < c1; c++) mine += __popc(word(c));
+        int incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        int before = 0, total = 0;
+#pragma unroll
+        for (int w = 0; w < MW_THREADS / 32; w++) { if (w < warp) before += s_warp[w]; total += s_warp[w]; }
+        set_range(total);
+        if (cta == 0 && tid == 0) {
+            if (p.count) *p.count = total;
+            if (p.rows_total && total) atomicAdd(p.rows_total, (unsigned long long)total);      // statistics
+        }
+        int rank = before + incl - mine;
+        for (int c = c0; c < c1 && rank < hi; c++) {
+            uint32_t m = c - c0 < KEEP ? mw[0] : word(c);
+            if (c - c0 < KEEP) {
+#pragma unroll
+                for (int k = 1; k < KEEP; k++) if (c - c0 == k) m = mw[k];
+            }
+            const int n = __popc(m);
+            if (rank + n > lo) {
+                for (int k = rank; m; k++) {
+                    const int bit = __ffs(m) - 1;
+                    m &= m - 1;
+                    if (k >= lo && k < hi) rows[k - lo] = c * 32 + bit;
+                }
+            }
+            rank += n;
+        }
+        __syncthreads();
+        if (p.list) for (int k = tid; k < hi - lo; k += MW_THREADS) p.list[lo + k] = rows[k];
+    }
+    for (int s = 0; s < S - 1; s++) {
+        if (s < n_units) { issue_w(s); issue_x(s); advance(); }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+
+    float acc[Q4 ? 1 : MT][Q4 ? 1 : NT][4];                           // (the accumulators of the two types have different shapes)
+    unsigned long long acq[Q4 ? MT : 1][Q4 ? NT : 1][2];
+    auto clear = [&]() {
+#pragma unroll
+        for (int m = 0; m < MT; m++)
+#pragma unroll
+            for (int n = 0; n < NT; n++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) { if (Q4) acq[Q4 ? m : 0][Q4 ? n : 0][j >> 1] = 0ull; else acc[Q4 ? 0 : m][Q4 ? 0 : n][j] = 0.f; }
+    };
+    clear();
+    const int g = lane >> 2, q = lane & 3;
+    const int row0 = wm * MT * 16, tok0 = wn * NT * 8;                // this warp's part of the tile
+    const uint32_t MAGIC = 0x4B400000u;
+    const unsigned long long neg_magic = mw_pack(-12582912.0f, -12582912.0f), sixteenth = mw_pack(0.0625f, 0.0625f);
+    // ldmatrix row addresses inside a stage (fragment layouts of mma.m16n8k16 / m16n8k32); the piece is added per step
+    const uint32_t a_row = (uint32_t)((row0 + (Q4 && MT == 2 ? lane : lane & 15)) * WB);
+    const uint32_t b_row = x_off + (uint32_t)((tok0 + (lane & 7) + (lane >> 4) * 8) * 128);
+    const int a_swz = Q4 ? (lane >> 1) & 3 : lane & 7, b_swz = lane & 7;
+
+    int tile = 0, slice = 0, slot = 0, next = S - 1;
+    for (int i = 0; i < n_units; i++) {
+        mw_wait(S - 2);
+        __syncthreads();                                              // stage i has landed for everybody; stage i - 1 is consumed
+        if (i + S - 1 < n_units) { issue_w(next); issue_x(next); advance(); }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (++next == S) next = 0;
+        const uint32_t base = ring + (uint32_t)(slot * p.stage);
+        if (++slot == S) slot = 0;
+        const int n_tile = min(IT, hi - lo - tile * IT);
+        const bool busy = (GATED ? row0 / 2 : row0) < n_tile && tok0 < p.T;       // my rows and tokens exist
+        if (!busy) {
+        } else if (!Q4) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                uint32_t a[MT][4];
+#pragma unroll
+                for (int m = 0; m < MT; m++) mw_ldsm4(a[m], base + a_row + m * 16 * WB + (((2 * k + (lane >> 4)) ^ a_swz) & 7) * 16);
+#pragma unroll
+                for (int n = 0; n < NT; n += 2) {
+                    if (tok0 + n * 8 >= p.T) break;
+                    uint32_t b[4];
+                    mw_ldsm4(b, base + b_row + n * 8 * 128 + (((2 * k + ((lane >> 3) & 1)) ^ b_swz) & 7) * 16);
+#pragma unroll
+                    for (int m = 0; m < MT; m++) {
+                        mw_hmma(acc[Q4 ? 0 : m][Q4 ? 0 : n], a[m], b[0], b[1]);
+                        mw_hmma(acc[Q4 ? 0 : m][Q4 ? 0 : n + 1], a[m], b[2], b[3]);
+                    }
+                }
+            }
+        } else {
+            uint32_t w1[4];
+#pragma unroll
+            for (int k = 0; k < (Q4 ? 4 : 0); k++) {                  // block by block
+                uint32_t w[4];
+                if (MT == 2) {
+                    mw_ldsm4(w, base + a_row + ((k ^ a_swz) & 3) * 16);
+                } else {                                              // 16 rows: two blocks at a time
+                    if (!(k & 1)) mw_ldsm4(w1, base + a_row + (((k + (lane >> 4)) ^ ((lane & 7) >> 1)) & 3) * 16);
+                    w[0] = w1[2 * (k & 1)]; w[1] = w1[2 * (k & 1) + 1]; w[2] = w[3] = 0u;
+                }
+                uint32_t a[MT][4];
+                unsigned long long d4[MT][2];
+#pragma unroll
+                for (int m = 0; m < MT; m++) {
+                    const uint32_t w0 = w[2 * m], wh = w[2 * m + 1];
+                    a[m][0] = ((w0 << 4) & 0xF0F0F0F0u) ^ 0x80808080u; a[m][1] = ((wh << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
+                    a[m][2] = (w0 & 0xF0F0F0F0u) ^ 0x80808080u;        a[m][3] = (wh & 0xF0F0F0F0u) ^ 0x80808080u;
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        unsigned short s;
+                        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(s) : "r"(base + s_off + (row0 + m * 16 + g + h * 8) * 8 + k * 2));
+                        const float e = __half2float(__ushort_as_half(s));
+                        d4[m][h] = mw_pack(e, e);
+                    }
+                }
+#pragma unroll
+                for (int n = 0; n < NT; n += 2) {
+                    if (tok0 + n * 8 >= p.T) break;
+                    uint32_t b[4];
+                    mw_ldsm4(b, base + b_row + n * 8 * 128 + (((2 * k + ((lane >> 3) & 1)) ^ b_swz) & 7) * 16);
+#pragma unroll
+                    for (int u = 0; u < 2; u++) {
+                        unsigned long long dd;
+                        asm volatile("ld.shared.b64 %0, [%1];" : "=l"(dd) : "r"(base + d_off + (k * XR + tok0 + (n + u) * 8 + 2 * q) * 4));
+                        dd = mw_mul2(dd, sixteenth);
+                        const unsigned long long md = mw_mul2(dd, neg_magic);
+#pragma unroll
+                        for (int m = 0; m < MT; m++) {
+                            uint32_t c[4];
+                            mw_imma(c, a[m], b[2 * u], b[2 * u + 1], MAGIC);
+                            mw_scale_add(acq[Q4 ? m : 0][Q4 ? n + u : 0][0], mw_packu(c[0], c[1]), dd, md, d4[m][0]);
+                            mw_scale_add(acq[Q4 ? m : 0][Q4 ? n + u : 0][1], mw_packu(c[2], c[3]), dd, md, d4[m][1]);
+                        }
+                    }
+                }
+            }
+        }
+        if (slice == p.n_slices - 1) {
+            // ---- the tile is complete: a lane holds rows g and g + 8 of each fragment (gated: up and gate of one item), tokens 2q, 2q + 1
+            if (busy) {
+#pragma unroll
+                for (int m = 0; m < MT; m++) {
+#pragma unroll
+                    for (int h = 0; h < (GATED ? 1 : 2); h++) {
+                        const int k = GATED ? (row0 + m * 16) / 2 + g : row0 + m * 16 + g + h * 8;     // item of the tile
+                        bool any = false;
+                        if (k < n_tile) {
+                            const int item = lo + tile * IT + k;
+                            const int r = SPARSE ? rows[tile * IT + k] : item;
+                            const int64_t gid = SPARSE && p.bucket ? p.bucket[r] : r;
+                            const float bias = p.bias ? p.bias[gid] : 0.f;
+#pragma unroll
+                            for (int n = 0; n < NT; n++) {
+#pragma unroll
+                                for (int j = 0; j < 2; j++) {
+                                    const int t = tok0 + n * 8 + 2 * q + j;
+                                    if (t >= p.T) continue;
+                                    float v[2];
+#pragma unroll
+                                    for (int z = 0; z < 2; z++) {
+                                        if (Q4) {
+                                            const unsigned long long w = acq[Q4 ? m : 0][Q4 ? n : 0][z];
+                                            v[z] = __uint_as_float(j ? (unsigned)(w >> 32) : (unsigned)w);
+                                        } else {
+                                            v[z] = acc[Q4 ? 0 : m][Q4 ? 0 : n][2 * z + j];
+                                        }
+                                    }
+                                    float o = GATED ? fmaxf(v[1], 0.f) * v[0] : v[h];
+                                    const bool off = SPARSE && p.idx[(size_t)t * p.idx_stride + gid] < p.threshold;   // (a NaN logit counts as active)
+                                    if (off && p.coef) { p.coef[(size_t)t * p.coef_stride + item] = __ushort_as_half((unsigned short)0); continue; }
+                                    if (off) o = 0.f;
+                                    if (p.bias) o += bias;
+                                    if (p.relu) o = fmaxf(o, 0.f);
+                                    if (p.dst)   p.dst[(size_t)t * p.dst_stride + gid] = o;
+                                    if (p.dst16) p.dst16[(size_t)t * p.dst_stride + gid] = __float2half_rn(o);
+                                    if (p.coef)  p.coef[(size_t)t * p.coef_stride + item] = __float2half_rn(o);
+                                    any |= !(o < p.masks_threshold);
+                                }
+                            }
+                        }
+                        if (!SPARSE && p.masks_out && any) atomicOr(&s_any[k / 32], 1u << (k % 32));
+                    }
+                }
+            }
+            if (!SPARSE && p.masks_out) {                             // the union over the tokens of !(result < threshold), one bit per row
+                __syncthreads();
+                if (tid < TM / 8 && tid * 8 < n_tile) {               // the range starts at a multiple of 8 rows
+                    unsigned char * o = reinterpret_cast<unsigned char *>(p.masks_out) + (lo + tile * IT) / 8 + tid;
+                    const unsigned char bits = (unsigned char)(s_any[tid / 4] >> (tid % 4 * 8));
+                    *o = p.masks_or ? (unsigned char)(*o | bits) : bits;
+                }
+                __syncthreads();
+                if (tid < 4) s_any[tid] = 0u;
+            }
+            clear();
+        }
+        if (++slice == p.n_slices) { slice = 0; tile++; }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------- launch
+template <int WT, int MT, int WM, int WN, int NT, bool SPARSE, bool GATED>
+static int mw_go(MwP p, bool pdl, cudaStream_t st) {
+    using Z = MwShape<WT, MT, WM, WN, NT>;
+    p.n_slices = (p.ncols + Z::KS - 1) / Z::KS;
+    const int G = (int)imin64(sm_count(), (p.nrows + 7) / 8);
+    const int list = SPARSE ? ((p.nrows + G - 1) / G + 1) * 4 : 0;    // bytes
+    const int XR = (p.T + 15) / 16 * 16;
+    p.stage = Z::TM * Z::WB + XR * 128 + (Z::Q4 ? Z::TM * 8 + XR * 16 : 0);
+    p.S = (MW_SMEM_MAX - list) / p.stage;
+    if (p.S > MW_SMAX) p.S = MW_SMAX;
+    if (p.S < 2 || list > 8192) return PI_ERR_UNSUPPORTED;            // (more than MM_MAX_ROWS rows)
+    static bool attr_done[16] = {false};
+    int dev = 0;
+    PI_CUDA(cudaGetDevice(&dev));
+    auto kern = k_mm_wide<WT, MT, WM, WN, NT, SPARSE, GATED>;
+    if (dev >= 0 && dev < 16 && !attr_done[dev]) {
+        PI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MW_SMEM_MAX));
+        attr_done[dev] = true;
+    }
+    PI_CUDA(launch_k(kern, dim3(G), dim3(MW_THREADS), (size_t)p.S * p.stage + list, st, pdl, p));
+    return PI_OK;
+}
+
+template <int WT, int MT, int WM, int WN, int NT>
+static int mw_sel(const MwP & p, bool pdl, cudaStream_t st) {
+    if (!p.masks) return mw_go<WT, MT, WM, WN, NT, false, false>(p, pdl, st);
+    if (p.W2)     return mw_go<WT, MT, WM, WN, NT, true, true>(p, pdl, st);
+    return mw_go<WT, MT, WM, WN, NT, true, false>(p, pdl, st);
+}
+
+// The smallest tile that holds a CTA's share of the rows: with few rows more warps along the tokens.  Up to 128 tokens and up to 256.
+template <int WT>
+static int mw_tile(const MwP & p, bool pdl, cudaStream_t st) {
+    const int64_t share = ((int64_t)p.nrows * (p.W2 ? 2 : 1) + sm_count() - 1) / sm_count();
+    if (p.T <= 128) {
+        if (share <= 32) return mw_sel<WT, 1, 2, 8, 2>(p, pdl, st);
+        if (share <= 64) return mw_sel<WT, 1, 4, 4, 4>(p, pdl, st);
+        return mw_sel<WT, 2, 4, 4, 4>(p, pdl, st);
+    }
+    if (share <= 32) return mw_sel<WT, 1, 2, 8, 4>(p, pdl, st);
+    if (share <= 64) return mw_sel<WT, 1, 4, 4, 8>(p, pdl, st);
+    return mw_sel<WT, 2, 4, 4, 8>(p, pdl, st);
+}
+
+// Called by launch_mm, which has checked the arguments.  Tokens go in launches of at most 256.
+int launch_mm_wide(const GemvArgs & a, cudaStream_t st) {
+    const bool q4 = a.wtype == PI_TYPE_Q4_0;
+    for (int t0 = 0; t0 < a.T; t0 += MW_TOKENS) {
+        MwP p;
+        p.W = (const uint8_t *)a.W; p.W2 = (const uint8_t *)a.W2; p.row_bytes = (int64_t)pi_row_bytes(a.wtype, a.ncols);
+        p.nrows = (int)a.nrows; p.ncols = (int)a.ncols; p.nb = (int)(a.ncols / 32);
+        p.T = a.T - t0 < MW_TOKENS ? a.T - t0 : MW_TOKENS;
+        if (q4) {
+            p.x.lo = a.x.lo + (size_t)t0 * p.nb; p.x.hi = a.x.hi + (size_t)t0 * p.nb; p.x.d = a.x.d + (size_t)t0 * p.nb;
+        } else {
+            p.x.h16 = a.x.h16 + (size_t)t0 * a.ncols;
+        }
+        p.masks = a.masks; p.bucket = a.bucket; p.list = a.list_out; p.count = a.count_out; p.rows_total = t0 == 0 ? a.rows_total : nullptr;
+        p.idx = a.idx ? a.idx + (size_t)t0 * a.idx_stride : nullptr; p.idx_stride = a.idx_stride; p.threshold = a.threshold;
+        p.bias = a.bias; p.relu = a.relu;
+        p.dst = a.dst ? a.dst + (size_t)t0 * a.dst_stride : nullptr;
+        p.dst16 = a.dst16 ? a.dst16 + (size_t)t0 * a.dst_stride : nullptr; p.dst_stride = a.dst_stride;
+        p.coef = a.coef ? a.coef + (size_t)t0 * a.coef_stride : nullptr; p.coef_stride = a.coef_stride;
+        p.masks_out = a.masks_out; p.masks_threshold = a.masks_threshold; p.masks_or = t0 > 0;
+        const int rc = q4 ? mw_tile<PI_TYPE_Q4_0>(p, a.pdl, st) : mw_tile<PI_TYPE_F16>(p, a.pdl, st);
+        if (rc != PI_OK) return rc;
+    }
+    return PI_OK;
+}
+
+}  // namespace pi

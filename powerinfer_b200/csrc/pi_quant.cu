@@ -167,43 +167,87 @@ ActBuf act_carve(int wtype, int64_t n, int T, char ** p) {
     return a;
 }
 
-__global__ void k_act_f16(const float * __restrict__ x, int64_t x_stride, int64_t n, int T, __half * __restrict__ out) {
-    const int64_t total = (int64_t)T * n;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t t = i / n, c = i - t * n;
-        out[i] = __float2half_rn(x[t * x_stride + c]);
+// What an operator needs before its weight-streaming kernel, in one launch: activation planes of x, activity bit masks of the predictor
+// logits, zeros where nobody else will write, cleared control words.  Each is a few hundred KB at most, so they cost their launches
+// (2 us each, two memsets among them); the blocks of the grid are handed to the parts in turn.
+struct PrepP {
+    const float * x; int n, nb, T; ActBuf act;
+    const float * idx; int64_t idx_stride; float threshold; int n_local; const int32_t * bucket; uint32_t * masks;
+    float * zero; int64_t n_zero; unsigned int * words; int n_words;
+    int g_act, g_mask;                                                // blocks of the first two parts, the others zero
+};
+
+template <bool Q4>
+__global__ void __launch_bounds__(256) k_prep(const PrepP p) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int b = blockIdx.x;
+    pdl_wait();
+    pdl_launch();                                                     // (after the wait: a kernel that runs ahead may read weights that came before)
+    if (b == 0 && tid < p.n_words) p.words[tid] = 0u;
+    if (b < p.g_act) {
+        if (Q4) {
+            const int64_t n = (int64_t)p.T * p.nb;
+            for (int64_t i = (int64_t)b * 8 + warp; i < n; i += (int64_t)p.g_act * 8) {
+                int q, s; float d16;
+                q8_block(p.x[i * QK + lane], q, d16, s);
+                int8_t * plane = reinterpret_cast<int8_t *>(lane < 16 ? p.act.lo + i : p.act.hi + i);
+                plane[lane & 15] = (int8_t)q;
+                if (lane == 0) { p.act.d[i] = d16; p.act.s[i] = s; }
+            }
+        } else {
+            const int64_t n = (int64_t)p.T * p.n, step = (int64_t)p.g_act * 256;
+            int64_t i = (int64_t)b * 256 + tid;
+            for (; i + 3 * step < n; i += 4 * step) {
+                float v[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) v[u] = p.x[i + u * step];
+#pragma unroll
+                for (int u = 0; u < 4; u++) p.act.h16[i + u * step] = __float2half_rn(v[u]);
+            }
+            for (; i < n; i += step) p.act.h16[i] = __float2half_rn(p.x[i]);
+        }
+        return;
     }
+    b -= p.g_act;
+    if (b < p.g_mask) {                                               // one warp per 32 rows, as in k_compact
+        const int n_chunks = (p.n_local + 31) / 32;
+        constexpr int UN = 8;                                         // logits in flight per lane
+        for (int c = b * 8 + warp; c < n_chunks; c += p.g_mask * 8) {
+            const int r = c * 32 + lane;
+            bool any = false;
+            if (r < p.n_local) {
+                const float * row = p.idx + (p.bucket ? p.bucket[r] : r);
+                for (int t0 = 0; t0 < p.T; t0 += UN) {
+                    float l[UN];
+#pragma unroll
+                    for (int u = 0; u < UN; u++) l[u] = t0 + u < p.T ? row[(size_t)(t0 + u) * p.idx_stride] : 0.f;
+#pragma unroll
+                    for (int u = 0; u < UN; u++) any |= t0 + u < p.T && !(l[u] < p.threshold);      // (a NaN logit counts as active)
+                }
+            }
+            const uint32_t m = __ballot_sync(0xffffffffu, any);
+            if (lane == 0) p.masks[c] = m;
+        }
+        return;
+    }
+    b -= p.g_mask;
+    const int64_t step = (int64_t)(gridDim.x - p.g_act - p.g_mask) * 256;
+    for (int64_t i = (int64_t)b * 256 + tid; i < p.n_zero; i += step) p.zero[i] = 0.f;
 }
 
-__global__ void k_act_q8(const float * __restrict__ x, int64_t x_stride, int nb, int T, ActBuf out) {
-    const int lane = threadIdx.x & 31;
-    const int64_t nblocks = (int64_t)T * nb;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < nblocks; i += warps) {
-        const int64_t t = i / nb;
-        const int b = (int)(i - t * nb);
-        int q, s; float d16;
-        q8_block(x[t * x_stride + (int64_t)b * QK + lane], q, d16, s);
-        int8_t * plane = reinterpret_cast<int8_t *>(lane < 16 ? out.lo + i : out.hi + i);
-        plane[lane & 15] = (int8_t)q;
-        if (lane == 0) { out.d[i] = d16; out.s[i] = s; }
-    }
-}
-
-int launch_convert_act(int wtype, const float * x, int64_t x_stride, int64_t n, int T, ActBuf out, cudaStream_t st) {
-    if (T == 0 || n == 0) return PI_OK;
-    if (wtype == PI_TYPE_Q4_0) {
-        const int nb = (int)(n / QK);
-        const int64_t nblocks = (int64_t)T * nb;
-        const int grid = (int)imin64((nblocks + 7) / 8, (int64_t)sm_count() * 8);
-        k_act_q8<<<grid, 256, 0, st>>>(x, x_stride, nb, T, out);
-        PI_LAUNCH_CHECK("k_act_q8");
-    } else {
-        const int64_t total = (int64_t)T * n;
-        const int grid = (int)imin64((total + 255) / 256, (int64_t)sm_count() * 8);
-        k_act_f16<<<grid, 256, 0, st>>>(x, x_stride, n, T, out.h16);
-        PI_LAUNCH_CHECK("k_act_f16");
-    }
+int launch_prep(const PrepArgs & a, cudaStream_t st) {
+    PrepP p;
+    p.x = a.x; p.n = (int)a.n; p.nb = (int)(a.n / QK); p.T = a.T; p.act = a.act;
+    p.idx = a.idx; p.idx_stride = a.idx_stride; p.threshold = a.threshold; p.n_local = (int)a.n_local; p.bucket = a.bucket; p.masks = a.masks;
+    p.zero = a.zero; p.n_zero = a.zero ? a.n_zero : 0; p.words = a.words; p.n_words = a.words ? a.n_words : 0;
+    const bool q4 = a.wtype == PI_TYPE_Q4_0;
+    const int64_t most = (int64_t)sm_count() * 8;
+    p.g_act = !a.x ? 0 : (int)imin64(q4 ? ((int64_t)a.T * p.nb + 7) / 8 : ((int64_t)a.T * a.n + 1023) / 1024, most);
+    p.g_mask = !a.idx ? 0 : (int)imin64((a.n_local + 255) / 256, most);
+    const int g_zero = (int)imin64((p.n_zero + 1023) / 1024, most);
+    const int grid = p.g_act + p.g_mask + g_zero > 0 ? p.g_act + p.g_mask + g_zero : 1;
+    if (q4) PI_CUDA(launch_k(k_prep<true>, dim3(grid), dim3(256), 0, st, true, p));
+    else    PI_CUDA(launch_k(k_prep<false>, dim3(grid), dim3(256), 0, st, true, p));
     return PI_OK;
 }
 

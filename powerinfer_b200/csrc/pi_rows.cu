@@ -413,17 +413,21 @@ static int launch_axpy_rows_inst(const AxpyRowsP & p, size_t smem, bool pdl, cud
     return PI_OK;
 }
 
+bool axpy_rows_eligible(int wtype, int64_t nrows, int64_t ncols, int n_groups) {
+    int ns, rg, mr;
+    axpy_rows_shape(nrows, ncols, &ns, &rg, &mr);
+    return rows_eligible(wtype, nrows, ncols) && mr <= AXPY_MAX_CTA_ROWS && rg <= n_groups && axpy_rows_smem((int)((nrows + 31) / 32), mr) <= 160 * 1024;
+}
+
 int launch_axpy_rows(const AxpyArgs & a, cudaStream_t st, int * groups_used) {
-    if (a.T != 1 || !a.masks || !rows_eligible(a.wtype, a.nrows, a.ncols)) return PI_ERR_UNSUPPORTED;
+    if (a.T != 1 || !a.masks || !axpy_rows_eligible(a.wtype, a.nrows, a.ncols, a.n_groups)) return PI_ERR_UNSUPPORTED;
     if (a.h_uncleared && a.bucket) return PI_ERR_UNSUPPORTED;          // the masks are by local row, h by global id
     AxpyRowsP p;
     axpy_rows_shape(a.nrows, a.ncols, &p.n_slices, &p.n_rg, &p.max_rows);
-    if (p.max_rows > AXPY_MAX_CTA_ROWS || p.n_rg > a.n_groups) return PI_ERR_UNSUPPORTED;
     p.Wt = (const uint8_t *)a.Wt; p.row_bytes = (int64_t)pi_row_bytes(a.wtype, a.ncols); p.nrows = (int)a.nrows;
     p.ncols = (int)a.ncols; p.nb = (int)(a.ncols / QK); p.n_chunks = (int)((a.nrows + 31) / 32);
     p.h = a.h; p.masks = a.masks; p.bucket = a.bucket; p.h_uncleared = a.h_uncleared ? 1 : 0; p.partial = a.partial;
     const size_t smem = axpy_rows_smem(p.n_chunks, p.max_rows);
-    if (smem > 160 * 1024) return PI_ERR_UNSUPPORTED;
     if (groups_used) *groups_used = p.n_rg;
     return a.wtype == PI_TYPE_Q4_0 ? launch_axpy_rows_inst<PI_TYPE_Q4_0>(p, smem, a.pdl, st)
                                    : launch_axpy_rows_inst<PI_TYPE_F16>(p, smem, a.pdl, st);

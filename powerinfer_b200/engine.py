@@ -174,16 +174,18 @@ class DecodeEngine:
         self.h_pos = torch.zeros(max_batch, dtype=torch.int32).pin_memory()
         self.h_logits = torch.zeros(max_batch, spec.n_vocab, dtype=torch.float32).pin_memory()
         self.h_argmax = torch.zeros(max_batch, dtype=torch.int32).pin_memory()
+        self._host_io = (*(t.numpy() for t in (self.h_tokens, self.h_pos, self.h_logits, self.h_argmax)),
+                         tuple(t.data_ptr() for t in (self.h_tokens, self.h_pos, self.h_logits, self.h_argmax)))
         self._xch_mem = None
 
     # ---- llama_decode + llama_get_logits with host buffers
     def decode(self, tokens, pos, want_logits: bool = True):
         T = len(tokens)
-        self.h_tokens[:T] = torch.as_tensor(tokens, dtype=torch.int32)
-        self.h_pos[:T] = torch.as_tensor(pos, dtype=torch.int32)
-        check(lib.pi_engine_decode_host(self.handle, self.h_tokens.data_ptr(), self.h_pos.data_ptr(), T,
-                                        self.h_logits.data_ptr() if want_logits else None, self.h_argmax.data_ptr(), self.st))
-        return (self.h_logits[:T].numpy() if want_logits else None), self.h_argmax[:T].numpy()
+        n_tokens, n_pos, n_logits, n_argmax, (p_tokens, p_pos, p_logits, p_argmax) = self._host_io
+        n_tokens[:T] = tokens.cpu() if isinstance(tokens, torch.Tensor) else tokens
+        n_pos[:T] = pos.cpu() if isinstance(pos, torch.Tensor) else pos
+        check(lib.pi_engine_decode_host(self.handle, p_tokens, p_pos, T, p_logits if want_logits else None, p_argmax, self.st))
+        return (n_logits[:T] if want_logits else None), n_argmax[:T]
 
     def prefill(self, tokens, seq: int = 0, pos0: int = 0, want_logits: bool = True):
         """Prompt processing: `tokens` are consecutive tokens of sequence `seq` starting at position pos0; they go through

@@ -34,12 +34,27 @@ class Weight:
         return self.data.data_ptr()
 
 
+# An operator at one token lasts a few microseconds on the device, so what these wrappers do on the host is part of its time:
+# tensors that are float32 and contiguous already pass untouched, and sizes and addresses of the workspace are kept.
+
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _p(t):
     return None if t is None else t.data_ptr()
+
+
+def _f32(t: torch.Tensor) -> torch.Tensor:
+    return t if t.dtype is torch.float32 and t.is_contiguous() else t.contiguous().float()
+
+
+def _rows(t: torch.Tensor, T: int, n: int) -> torch.Tensor:
+    """t as contiguous float32 [T, n] (either may be -1)"""
+    t = _f32(t)
+    if t.dim() == 2 and (T < 0 or t.shape[0] == T) and (n < 0 or t.shape[1] == n):
+        return t
+    return t.reshape(T, n)
 
 
 class Workspace:
@@ -47,13 +62,20 @@ class Workspace:
 
     def __init__(self):
         self.buf = None
+        self.at = self.size = 0
+        self.need: dict = {}                 # (ncols, nrows, T) -> bytes
 
     def get(self, ncols: int, nrows: int, T: int):
-        need = lib.pi_workspace_bytes(ncols, nrows, T)
+        need = self.need.get((ncols, nrows, T))
+        if need is None:
+            if len(self.need) > 1024:
+                self.need.clear()
+            need = self.need[(ncols, nrows, T)] = lib.pi_workspace_bytes(ncols, nrows, T)
         if self.buf is None or self.buf.numel() < need:
             self.buf = torch.empty(need + 256, dtype=torch.uint8, device="cuda")
-        off = (-self.buf.data_ptr()) % 256
-        return self.buf.data_ptr() + off, self.buf.numel() - off
+            off = (-self.buf.data_ptr()) % 256
+            self.at, self.size = self.buf.data_ptr() + off, self.buf.numel() - off
+        return self.at, self.size
 
 
 _ws = Workspace()
@@ -63,8 +85,7 @@ def last_op_status() -> int:
     """Status of the last sparse operator issued through this module (pi_op_status): 0, or 5 (a bounded device-side wait ran out)."""
     if _ws.buf is None:
         return 0
-    off = (-_ws.buf.data_ptr()) % 256
-    return int(lib.pi_op_status(_ws.buf.data_ptr() + off, _stream()))
+    return int(lib.pi_op_status(_ws.at, _stream()))
 
 
 def upload_weight(host: np.ndarray, wtype: int, nrows: int, ncols: int) -> Weight:
@@ -105,7 +126,7 @@ def dequantize(w: Weight) -> torch.Tensor:
 
 def ggml_mul_mat(a: Weight, b: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
     """ggml_mul_mat(ctx, a, b): a [nrows, ncols] weights, b F32 [T, ncols] -> F32 [T, nrows]."""
-    b = b.contiguous().float().reshape(-1, a.ncols)
+    b = _rows(b, -1, a.ncols)
     T = b.shape[0]
     dst = torch.empty(T, a.nrows, dtype=torch.float32, device="cuda")
     ws, wsn = _ws.get(a.ncols, a.nrows, T)
@@ -120,9 +141,9 @@ def ggml_mul_mat_idx(a: Weight, b: torch.Tensor, sparse_idx: torch.Tensor, gpu_b
     a: rows of up / gate held on this device; b: F32 [T, ncols]; sparse_idx: F32 [T, F] predictor logits by
     global neuron id; gpu_bucket: int32 [a.nrows] global ids of a's rows (None: a holds all F rows);
     result_ne0: F when a bucket is given.  Returns F32 [T, F]."""
-    b = b.contiguous().float().reshape(-1, a.ncols)
+    b = _rows(b, -1, a.ncols)
     T = b.shape[0]
-    sparse_idx = sparse_idx.contiguous().float().reshape(T, -1)
+    sparse_idx = _rows(sparse_idx, T, -1)
     F = result_ne0 if gpu_bucket is not None else a.nrows
     assert F is not None and sparse_idx.shape[1] >= F
     dst = torch.empty(T, F, dtype=torch.float32, device="cuda")
@@ -137,8 +158,8 @@ def ggml_axpy(a: Weight, b: torch.Tensor, sparse_idx: torch.Tensor, hybrid_aux: 
     """ggml_axpy (ggml.h:1107-1112): a = rows of ffn_down_t on this device, b = F32 [T, F] hidden activations,
     hybrid_aux = gpu_bucket (int32 [a.nrows]) or None.  Returns F32 [T, ncols]."""
     T = b.shape[0] if b.dim() == 2 else 1
-    b = b.contiguous().float().reshape(T, -1)
-    sparse_idx = sparse_idx.contiguous().float().reshape(T, -1)
+    b = _rows(b, T, -1)
+    sparse_idx = _rows(sparse_idx, T, -1)
     dst = torch.empty(T, a.ncols, dtype=torch.float32, device="cuda")
     ws, wsn = _ws.get(a.ncols, max(a.nrows, b.shape[1]), T)
     check(lib.pi_axpy(a.wtype, a.ptr, a.nrows, a.ncols, b.data_ptr(), T, b.shape[1], sparse_idx.data_ptr(),
@@ -150,9 +171,9 @@ def sparse_ffn(up: Weight, gate: Weight | None, down_t: Weight, x: torch.Tensor,
                gpu_bucket: torch.Tensor | None = None, up_bias: torch.Tensor | None = None) -> torch.Tensor:
     """llm_build_ffn_sparse (llama.cpp:4652-4757) after the predictor, as one call: the two ggml_mul_mat_idx nodes, the
     relu / mul / bias nodes and ggml_axpy.  x F32 [T, d], sparse_idx F32 [T, F] -> F32 [T, d]."""
-    x = x.contiguous().float().reshape(-1, up.ncols)
+    x = _rows(x, -1, up.ncols)
     T = x.shape[0]
-    sparse_idx = sparse_idx.contiguous().float().reshape(T, -1)
+    sparse_idx = _rows(sparse_idx, T, -1)
     F = sparse_idx.shape[1]
     dst = torch.empty(T, up.ncols, dtype=torch.float32, device="cuda")
     ws, wsn = _ws.get(up.ncols, max(up.nrows, F), T)
@@ -164,7 +185,7 @@ def sparse_ffn(up: Weight, gate: Weight | None, down_t: Weight, x: torch.Tensor,
 
 def predictor(fc1: Weight, fc2: Weight, p: torch.Tensor) -> torch.Tensor:
     """idx = mul_mat(fc2, relu(mul_mat(fc1, p))) (llama.cpp:4688-4695); p F32 [T, d] -> F32 [T, F]."""
-    p = p.contiguous().float().reshape(-1, fc1.ncols)
+    p = _rows(p, -1, fc1.ncols)
     T = p.shape[0]
     idx = torch.empty(T, fc2.nrows, dtype=torch.float32, device="cuda")
     ws, wsn = _ws.get(max(fc1.ncols, fc2.ncols), max(fc1.nrows, fc2.nrows), T)
