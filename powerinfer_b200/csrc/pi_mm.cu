@@ -16,14 +16,17 @@
 // KB of masks itself and takes the rows of its ranks, so no list has to be built first; it leaves its part of the list behind
 // for the axpy.  A dense product can write such masks (the predictor's second matrix does): no mask kernel in between.
 //
-// Inside a CTA the 8 warps split the COLUMNS: a warp takes every eighth slice of 64 bytes of all rows of the tile, and the activation
-// of that slice, through a ring of its own.  Nothing is shared while a tile lasts: a warp waits for its own copies only, and there is
-// no barrier between the first slice and the last, where the 8 partial tiles meet in shared memory and are added in warp order.
-// (16 warps that shared a stage met in a barrier for each: 1900 clocks a stage, whatever it held.)
+// Inside a CTA 8 consumer warps split the COLUMNS: a warp takes every eighth slice of 64 bytes of all rows of the tile, and the
+// activation of that slice, from a ring of its own that a producer warp of its own fills.  Nothing is shared while a tile lasts, and
+// there is no barrier between the first slice and the last, where the 8 partial tiles meet in shared memory and are added in warp
+// order.  (16 warps that shared a stage met in a barrier for each: 1900 clocks a stage, whatever it held.  Warps that issued their own
+// copies spent half of the time in them: a cp.async waits while the SM's queue of outstanding loads is full, which with HBM as the
+// bound is always.)  Consumers get 200 registers, 128 of them accumulators, producers 56.
 // Rows arrive by 16-byte cp.async: the rows of the active list lie anywhere, and pieces of a few hundred bytes are too small for the
 // bulk-copy engine (about 80 ns per copy).  A row slice of 64 bytes is stored with its four 16-byte pieces permuted by
 // (row / 2) % 4, so that the eight rows of an 8x8 fragment lie in different banks without padding.
 // Dense weights do not depend on the kernel before: their first stages are requested before griddepcontrol.wait.
+// Every wait is bounded: when one runs out the warp sets bit 4 of *status (where given) and the CTA returns without a result, its copies landed.
 //
 // Q4_0 arithmetic: a nibble q is placed in the high half of a byte and its top bit flipped, which is the int8 value
 // 16 * (q - 8): one logic operation for four weights, no correction term.  The mma's C operand is the constant 0x4B400000, so
@@ -33,9 +36,10 @@
 
 namespace pi {
 
-static constexpr int MM_WARPS = 16, MM_THREADS = MM_WARPS * 32, MM_PAIRS = MM_WARPS / 2;
+static constexpr int MM_RINGS = 8, MM_WARPS = 2 * MM_RINGS, MM_THREADS = MM_WARPS * 32;      // consumer warps 0 .. 7, producer warps 8 .. 15
+static constexpr int MM_REGS_C = 200, MM_REGS_P = 56;   // 256 x (200 + 56) = the 512 x 128 of the launch
 static constexpr int MM_SMAX = 8;                       // stages of a ring at most
-static constexpr int MM_SMEM_MAX = 226 * 1024;          // (leaves room for the static variables)
+static constexpr int MM_SMEM_MAX = 225 * 1024;          // (leaves room for the static variables)
 
 struct MmP {
     const uint8_t * W; const uint8_t * W2; int64_t row_bytes; int nrows, ncols, nb;
@@ -46,6 +50,7 @@ struct MmP {
     float * dst; __half * dst16; int64_t dst_stride;
     __half * coef; int64_t coef_stride;
     uint32_t * masks_out; float masks_threshold; int masks_or;
+    unsigned int * status;
     int n_slices, ring;                                               // slices of 64 bytes of a row; bytes of a warp's ring
 };
 
@@ -59,18 +64,8 @@ __device__ __forceinline__ void mm_cp4(uint32_t dst, const void * src) {
 __device__ __forceinline__ void mm_cp8(uint32_t dst, const void * src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" :: "r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ void mm_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void mm_wait(int pending) {                // all but the last `pending` (0 .. MM_SMAX - 2) groups have landed
-    switch (pending) {
-        case 0: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
-        case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
-        case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
-        case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
-        case 4: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
-        case 5: asm volatile("cp.async.wait_group 5;" ::: "memory"); break;
-        default: asm volatile("cp.async.wait_group 6;" ::: "memory"); break;
-    }
-}
+// one arrival on `bar` when all copies this thread has issued so far have landed
+__device__ __forceinline__ void mm_arrive_copies(uint64_t * bar) { asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" :: "r"(smem_u32(bar)) : "memory"); }
 __device__ __forceinline__ void mm_ldsm4(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
@@ -110,24 +105,38 @@ struct MmShape {
     static constexpr int MT = Q4 && NT == 4 ? 7 : 8;                  // fragments of 16 rows of a tile at most (two stages have to fit)
     static constexpr int KS = Q4 ? 128 : 32;                          // columns of a slice
     static constexpr int ROW = Q4 ? 72 : 64, TOK = Q4 ? 144 : 64;     // bytes of a stage per row and per token
-    static_assert(2 * (MT * 16 * ROW + TP * TOK) * MM_PAIRS <= MM_SMEM_MAX - 8192, "two stages");
+    static_assert(2 * (MT * 16 * ROW + TP * TOK) * MM_RINGS <= MM_SMEM_MAX - 8192, "two stages");
 };
 
 template <int WT, int NT, bool SPARSE, bool GATED>
 __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
     using Z = MmShape<WT, NT>;
     constexpr bool Q4 = Z::Q4;
-    constexpr int TP = Z::TP, MT = Z::MT, MW = (MT + 1) / 2;           // fragments of a tile, of a warp
+    constexpr int TP = Z::TP, MT = Z::MT;
     constexpr int IT = GATED ? MT * 8 : MT * 16;                      // items (rows / neurons) of a tile at most
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int s_warp[MM_WARPS];
     __shared__ unsigned s_any[4];
-    int * rows = reinterpret_cast<int *>(smem + (size_t)MM_PAIRS * p.ring);      // rows of this CTA (sparse only)
+    __shared__ uint64_t s_full[MM_RINGS][MM_SMAX], s_empty[MM_RINGS][MM_SMAX], s_tile;
+    __shared__ volatile int s_dead;
+    int * rows = reinterpret_cast<int *>(smem + (size_t)MM_RINGS * p.ring);      // rows of this CTA (sparse only)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int G = gridDim.x, cta = blockIdx.x;
-    const int pair = warp >> 1, half = warp & 1;
-    const uint32_t ring_a = smem_u32(smem) + (uint32_t)(pair * p.ring);
+    const int me = warp & (MM_RINGS - 1);                             // my ring
+    const uint32_t ring_a = smem_u32(smem) + (uint32_t)(me * p.ring);
+    uint64_t * full = s_full[me], * empty = s_empty[me];
     pdl_launch();
+    if (tid < MM_RINGS * MM_SMAX) { mbar_init(&s_full[0][0] + tid, 64); mbar_init(&s_empty[0][0] + tid, 1); }
+    if (tid == 0) { mbar_init(&s_tile, MM_RINGS); s_dead = 0; }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    __syncthreads();
+    auto wait = [&](uint64_t * bar, unsigned parity) -> bool {        // warp-uniform; false: the wait ran out, here or elsewhere
+        bool ok = false;
+        for (int spins = 0; spins < (1 << 20) && !ok && !s_dead; spins++) ok = mbar_try_wait(bar, parity);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok && lane == 0) { s_dead = 1; if (p.status) atomicOr(p.status, 16u); }
+        return ok;
+    };
 
     // this CTA's items, items per tile, fragment rows of a tile, bytes of a stage, stages of a ring
     int lo = 0, hi = 0, per_tile = 1, n_tiles = 0, rt = 16, stage = 1, S = 2;
@@ -142,7 +151,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
         stage = rt * Z::ROW + TP * Z::TOK;
         S = min(MM_SMAX, p.ring / stage);
     };
-    const int n_mine = pair < p.n_slices ? (p.n_slices - pair + MM_PAIRS - 1) / MM_PAIRS : 0;       // slices of a tile that are the pair's
+    const int n_mine = me < p.n_slices ? (p.n_slices - me + MM_RINGS - 1) / MM_RINGS : 0;       // slices of a tile that are mine
     // A stage: row slices, activation slices (Q4_0: then the rows' scales and the activation's, [block][token])
     int first = 0, n_rows = 0;                                        // current tile: first item, rows in all (gated: up 0, gate 0, up 1, ..)
     const int r8 = lane >> 2, c4 = lane & 3;
@@ -151,59 +160,66 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
         const int k = GATED ? r >> 1 : r;
         return (GATED && (r & 1) ? p.W2 : p.W) + (size_t)(SPARSE ? rows[first + k] : lo + first + k) * p.row_bytes;
     };
-    auto issue_w = [&](int j, int slot) {                             // the pair's slice number j: every other 8 rows
-        const int s = pair + j * MM_PAIRS;
-        const uint32_t base = ring_a + (uint32_t)(slot * stage);
+    // Addresses are kept and moved along: a producer is one warp, and a chain of address arithmetic per copy costs it more than the copy.
+    const bool ragged = !Q4 && p.ncols % 32 != 0;                     // the last slice of a row is not whole
+    const uint8_t * w_src = nullptr; const uint8_t * s_src = nullptr; // dense: my piece of row r8 (Q4_0: my scales of row `lane`) of the next slice
+    const size_t w_step = (size_t)p.row_bytes * 8, s_step = (size_t)p.row_bytes * 32;
+    auto issue_w = [&](int j, int slot) {                             // my slice number j (asked for in order within a tile)
+        const int s = me + j * MM_RINGS;
+        const uint32_t base = ring_a + (uint32_t)(slot * stage), to = base + w_dst;
         const int off = s * 64 + c4 * 16;
-        if (!Q4 && off >= p.ncols * 2) {                              // past the end of a row: zeros
-            for (int r = half * 8 + r8; r < n_rows; r += 16) mm_zero16(base + w_dst + (r - r8) * 64);
+        if (!SPARSE && j == 0) { w_src = row_ptr(r8) + off; if (Q4) s_src = row_ptr(lane) + (size_t)p.nb * 16 + s * 8; }
+        if (ragged && off >= p.ncols * 2) {                           // past the end of a row: zeros
+            for (int r = r8; r < n_rows; r += 8) mm_zero16(to + (r - r8) * 64);
+            __threadfence_block();
         } else if (!SPARSE) {
-            const uint8_t * src = row_ptr(half * 8 + r8) + off;
-            const size_t step = (size_t)p.row_bytes * 16;
+            const uint8_t * src = w_src;
 #pragma unroll 4
-            for (int r = half * 8 + r8; r < n_rows; r += 16, src += step) mm_cp16(base + w_dst + (r - r8) * 64, src);
+            for (int r = r8; r < n_rows; r += 8, src += w_step) mm_cp16(to + (r - r8) * 64, src);
         } else {
 #pragma unroll 4
-            for (int r = half * 8 + r8; r < n_rows; r += 16) mm_cp16(base + w_dst + (r - r8) * 64, row_ptr(r) + off);
+            for (int r = r8; r < n_rows; r += 8) mm_cp16(to + (r - r8) * 64, row_ptr(r) + off);
         }
+        w_src += 64 * MM_RINGS;
         if (Q4) {
             const uint32_t sb = base + rt * 64 + TP * 128;
             const int so = p.nb * 16 + s * 8;
-            for (int r = half * 32 + lane; r < n_rows; r += 64) mm_cp8(sb + r * 8, row_ptr(r) + so);
+            const uint8_t * src = s_src;
+            for (int r = lane; r < n_rows; r += 32, src += s_step) mm_cp8(sb + r * 8, SPARSE ? row_ptr(r) + so : src);
+            s_src += 8 * MM_RINGS;
         }
     };
-    auto x_src = [&](int s, int e) -> const void * {                  // piece e of slice s: its address (nullptr: zeros)
-        if (!Q4) {
-            const int c = s * 32 + (e & 3) * 8;
-            return c < p.ncols ? p.x.h16 + (size_t)(e >> 2) * p.ncols + c : nullptr;
-        }
-        return (e & 1 ? p.x.hi : p.x.lo) + (size_t)(e >> 3) * p.nb + s * 4 + ((e >> 1) & 3);
-    };
-    auto x_dst = [&](int e) -> uint32_t {                             // where it lies behind the rows
-        return Q4 ? (uint32_t)((e >> 3) * 128 + ((e ^ (e >> 3)) & 7) * 16) : (uint32_t)((e >> 2) * 64 + ((e ^ (e >> 3)) & 3) * 16);
-    };
-    constexpr int XE = TP * (Q4 ? 8 : 4);                             // 16-byte pieces of an activation slice
-    const int x_n = p.T * (Q4 ? 8 : 4), pl = half * 32 + lane;
-    auto issue_x = [&](int j, int slot) {
-        const int s = pair + j * MM_PAIRS;
-        const uint32_t base = ring_a + (uint32_t)(slot * stage + rt * 64);
+    // The activation of a slice: 16-byte pieces, 8 (Q4_0: 4) tokens per instruction; tokens past the last one copy the last one again
+    constexpr int XN = Q4 ? 2 * NT : NT, XT = Q4 ? 4 : 8;             // instructions, tokens of one
+    const int xr = Q4 ? lane >> 3 : r8, xc = Q4 ? lane & 7 : c4;
+    const uint32_t x_dst = Q4 ? (uint32_t)(xr * 128 + ((xc ^ xr) & 7) * 16) : (uint32_t)(xr * 64 + ((xc ^ (xr >> 1)) & 3) * 16);
+    int x_at[XN], d_at[Q4 ? NT : 1];                                  // byte offsets of my tokens
+    const char * x_src = Q4 ? reinterpret_cast<const char *>((xc & 1 ? p.x.hi : p.x.lo) + (xc >> 1)) : reinterpret_cast<const char *>(p.x.h16 + xc * 8);
+    const char * d_src = reinterpret_cast<const char *>(p.x.d) + (lane & 3) * 4;
+    auto start_x = [&]() {
 #pragma unroll
-        for (int e0 = 0; e0 < XE; e0 += 64) {
-            const int e = e0 + pl;
-            if (e < x_n) {
-                const void * src = x_src(s, e);
-                if (src) mm_cp16(base + x_dst(e), src); else mm_zero16(base + x_dst(e));
-            }
+        for (int i = 0; i < XN; i++) x_at[i] = min(xr + i * XT, p.T - 1) * (Q4 ? p.nb * 16 : p.ncols * 2);
+#pragma unroll
+        for (int i = 0; i < (Q4 ? NT : 0); i++) d_at[i] = min((lane >> 2) + i * 8, p.T - 1) * p.nb * 4;
+    };
+    auto issue_x = [&](int j, int slot) {
+        const int s = me + j * MM_RINGS;
+        const uint32_t base = ring_a + (uint32_t)(slot * stage + rt * 64), to = base + x_dst;
+        if (ragged && s * 32 + xc * 8 >= p.ncols) {
+#pragma unroll
+            for (int i = 0; i < XN; i++) mm_zero16(to + i * 512);
+            __threadfence_block();
+        } else {
+            const char * src = x_src + s * 64;
+#pragma unroll
+            for (int i = 0; i < XN; i++) mm_cp16(Q4 && (i & 1) ? (to + i * 512) ^ 64u : to + i * 512, src + x_at[i]);      // (token + 4: piece ^ 4)
         }
         if (Q4) {
+            const uint32_t dt = base + TP * 128 + rt * 8 + ((lane & 3) * TP + (lane >> 2)) * 4;
 #pragma unroll
-            for (int e0 = 0; e0 < TP * 4; e0 += 64) {
-                const int e = e0 + pl, t = e >> 2, k = e & 3;
-                if (t < p.T) mm_cp4(base + TP * 128 + rt * 8 + (k * TP + t) * 4, p.x.d + (size_t)t * p.nb + s * 4 + k);
-            }
+            for (int i = 0; i < (Q4 ? NT : 0); i++) mm_cp4(dt + i * 32, d_src + s * 16 + d_at[i]);
         }
     };
-    auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" :: "r"(pair + 1) : "memory"); };
     auto start_tile = [&](int tile) {
         first = tile * per_tile;
         n_rows = min(per_tile, hi - lo - first) * (GATED ? 2 : 1);
@@ -211,48 +227,6 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
 
     if (!SPARSE) {
         set_range(p.nrows);
-        start_tile(0);
-        const int ns = n_tiles > 0 ? min(S - 1, n_mine) : 0;
-        for (int j = 0; j < S - 1; j++) { if (j < ns) issue_w(j, j); mm_commit(); }
-        pdl_wait();
-        // The activation of the stages requested so far: plain loads, several in flight (as cp.async it would belong to a
-        // later group than all the weights above, and the first stage would be waiting for the last)
-        constexpr int UN = 4;
-        const int n = ns * XE;
-        for (int e0 = pl; e0 < n; e0 += UN * 64) {
-            uint4 v[UN];
-#pragma unroll
-            for (int u = 0; u < UN; u++) {
-                const int ea = e0 + u * 64, j = ea / XE, e = ea % XE;
-                v[u] = make_uint4(0u, 0u, 0u, 0u);
-                if (ea < n && e < x_n) {
-                    const void * src = x_src(pair + j * MM_PAIRS, e);
-                    if (src) v[u] = *reinterpret_cast<const uint4 *>(src);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < UN; u++) {
-                const int ea = e0 + u * 64, j = ea / XE, e = ea % XE;
-                if (ea < n)
-                    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" :: "r"(ring_a + (uint32_t)(j * stage + rt * 64) + x_dst(e)), "r"(v[u].x), "r"(v[u].y), "r"(v[u].z), "r"(v[u].w) : "memory");
-            }
-        }
-        if (Q4) {
-            const int nd = ns * TP * 4;
-            for (int e0 = pl; e0 < nd; e0 += UN * 64) {
-                float v[UN];
-#pragma unroll
-                for (int u = 0; u < UN; u++) {
-                    const int ea = e0 + u * 64, j = ea / (TP * 4), t = ea % (TP * 4) >> 2, k = ea & 3;
-                    v[u] = ea < nd && t < p.T ? p.x.d[(size_t)t * p.nb + (pair + j * MM_PAIRS) * 4 + k] : 0.f;
-                }
-#pragma unroll
-                for (int u = 0; u < UN; u++) {
-                    const int ea = e0 + u * 64, j = ea / (TP * 4), t = ea % (TP * 4) >> 2, k = ea & 3;
-                    if (ea < nd) asm volatile("st.shared.f32 [%0], %1;" :: "r"(ring_a + (uint32_t)(j * stage + rt * 72) + TP * 128 + (k * TP + t) * 4), "f"(v[u]) : "memory");
-                }
-            }
-        }
     } else {
         pdl_wait();
         // ---- ranks of the active rows: thread t counts the words [c0, c1), a block scan gives the rank of its first row
@@ -303,66 +277,93 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
             rank += n;
         }
         __syncthreads();
-        start_tile(0);
-        for (int j = 0; j < S - 1; j++) { if (j < n_mine && n_tiles > 0) { issue_w(j, j); issue_x(j, j); } mm_commit(); }
         if (p.list) for (int k = tid; k < hi - lo; k += MM_THREADS) p.list[lo + k] = rows[k];
     }
 
+    if (warp >= MM_RINGS) {
+        // ================================================================= producers
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(MM_REGS_P));
+        start_x();
+        int slot = 0, ahead = 0;                                      // ahead: stages of tile 0 requested before the loop
+        unsigned phase = 1u;                                          // parity of the hand-back to wait for (first round: none)
+        if (!SPARSE) {
+            start_tile(0);
+            const int ns = n_tiles > 0 ? min(S, n_mine) : 0;
+            for (int j = 0; j < ns; j++) { issue_w(j, j); mm_arrive_copies(full + j); }
+            pdl_wait();
+            for (int j = 0; j < ns; j++) { issue_x(j, j); mm_arrive_copies(full + j); }
+            ahead = ns;
+            slot = ns == S ? 0 : ns;
+            if (ns == S) phase = 0u;
+        }
+        for (int tile = 0; tile < n_tiles; tile++) {
+            start_tile(tile);
+            if (tile > 0 && !wait(&s_tile, (unsigned)(tile - 1) & 1u)) break;      // the sums of the tile before lie over the rings
+            bool ok = true;
+            for (int j = tile == 0 ? ahead : 0; j < n_mine; j++) {
+                ok = wait(empty + slot, phase);
+                if (!ok) break;
+                issue_w(j, slot);
+                mm_arrive_copies(full + slot);
+                issue_x(j, slot);
+                mm_arrive_copies(full + slot);
+                if (++slot == S) { slot = 0; phase ^= 1u; }
+            }
+            if (!ok) break;
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        return;
+    }
+    // ===================================================================== consumers
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(MM_REGS_C));
     const int g = lane >> 2, q = lane & 3;
     // ldmatrix addresses inside a stage (fragment layouts of mma.m16n8k16 / m16n8k32): two 16-byte pieces of 16 rows, four of 8 tokens
     // (Q4_0: one block of 32 rows, one block of two groups of 8 tokens)
-    const int a_row = lane & 15;
-    const uint32_t a_up = (lane >> 4) * 32 * 64, b_up = NT > 1 ? (lane >> 4) * 8 * 128 : 0;   // (a warp's fragments are every other 16 rows)
+    const int a_row = Q4 ? lane : lane & 15;
+    const uint32_t a_up = (lane >> 4) * 16 * 64, b_up = NT > 1 ? (lane >> 4) * 8 * 128 : 0;
     const int b_row = Q4 ? (lane & 7) + (NT > 1 ? (lane >> 4) * 8 : 0) : (lane & 7);
     const uint32_t MAGIC = 0x4B400000u;
     const unsigned long long neg_magic = mm_pack(-12582912.0f, -12582912.0f), sixteenth = mm_pack(0.0625f, 0.0625f);
     uint32_t a_off[Q4 ? 4 : 2], b_off[Q4 ? 4 : 1];
 #pragma unroll
-    for (int k = 0; k < (Q4 ? 4 : 2); k++) a_off[k] = (uint32_t)(half * 1024 + a_row * 64 + (((Q4 ? k : k * 2 + (lane >> 4)) ^ ((lane & 7) >> 1)) & 3) * 16);
+    for (int k = 0; k < (Q4 ? 4 : 2); k++) a_off[k] = (uint32_t)(a_row * 64 + (((Q4 ? k : k * 2 + (lane >> 4)) ^ ((lane & 7) >> 1)) & 3) * 16);
 #pragma unroll
     for (int k = 0; k < (Q4 ? 4 : 1); k++)
         b_off[k] = Q4 ? (uint32_t)(b_row * 128 + (((k * 2 + ((lane >> 3) & 1)) ^ (lane & 7)) & 7) * 16) : (uint32_t)(b_row * 64 + (((lane >> 3) ^ ((lane & 7) >> 1)) & 3) * 16);
 
+    int slot = 0;
+    unsigned phase = 0u;
     for (int tile = 0; tile < n_tiles; tile++) {
-        if (tile > 0) {
-            start_tile(tile);
-            for (int j = 0; j < S - 1; j++) { if (j < n_mine) { issue_w(j, j); issue_x(j, j); } mm_commit(); }
-        }
+        start_tile(tile);
         // (the accumulators of the two types have different shapes)
-        float acc[Q4 ? 1 : MW][Q4 ? 1 : NT][4];
-        unsigned long long acq[Q4 ? MW : 1][Q4 ? NT : 1][2];
+        float acc[Q4 ? 1 : MT][Q4 ? 1 : NT][4];
+        unsigned long long acq[Q4 ? MT : 1][Q4 ? NT : 1][2];
 #pragma unroll
-        for (int m = 0; m < MW; m++)
+        for (int m = 0; m < MT; m++)
 #pragma unroll
             for (int n = 0; n < NT; n++)
 #pragma unroll
                 for (int j = 0; j < 4; j++) { if (Q4) acq[Q4 ? m : 0][Q4 ? n : 0][j >> 1] = 0ull; else acc[Q4 ? 0 : m][Q4 ? 0 : n][j] = 0.f; }
-        int slot = 0, next = S - 1;
         for (int i = 0; i < n_mine; i++) {
-            mm_wait(S - 2);
-            pair_sync();                                              // stage i has landed for the pair, stage i - 1 is consumed
-            if (i + S - 1 < n_mine) { issue_w(i + S - 1, next); issue_x(i + S - 1, next); }
-            mm_commit();
-            if (++next == S) next = 0;
+            if (!wait(full + slot, phase)) break;
             const uint32_t base = ring_a + (uint32_t)(slot * stage), xb = base + rt * 64;
-            if (++slot == S) slot = 0;
             if (!Q4) {
                 uint32_t b[NT][4];
 #pragma unroll
                 for (int n = 0; n < NT; n++) mm_ldsm4(b[n], xb + b_off[0] + n * 8 * 64);
 #pragma unroll
-                for (int m = 0; m < MW; m++) {
-                    if (m * 32 + half * 16 >= rt) break;
+                for (int m = 0; m < MT; m++) {
+                    if (m * 16 >= rt) break;
 #pragma unroll
                     for (int k = 0; k < 2; k++) {
                         uint32_t a[4];
-                        mm_ldsm4(a, base + a_off[k] + m * 32 * 64);
+                        mm_ldsm4(a, base + a_off[k] + m * 16 * 64);
 #pragma unroll
                         for (int n = 0; n < NT; n++) mm_hmma(acc[Q4 ? 0 : m][Q4 ? 0 : n], a, b[n][2 * k], b[n][2 * k + 1]);
                     }
                 }
             } else {
-                const uint32_t sb = xb + TP * 128 + (half * 16 + g) * 8, db = xb + TP * 128 + rt * 8 + 2 * q * 4;
+                const uint32_t sb = xb + TP * 128 + g * 8, db = xb + TP * 128 + rt * 8 + 2 * q * 4;
 #pragma unroll
                 for (int k = 0; k < (Q4 ? 4 : 0); k++) {              // block by block
                     uint32_t b[NT + 1][2];
@@ -380,16 +381,16 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
                         md[n] = mm_mul2(dd[n], neg_magic);
                     }
 #pragma unroll
-                    for (int m = 0; m < MW; m += 2) {
-                        if (m * 32 + half * 16 >= rt) break;
+                    for (int m = 0; m < MT; m += 2) {
+                        if (m * 16 >= rt) break;
                         uint32_t w[4];
-                        mm_ldsm4(w, base + a_off[k] + m * 32 * 64 + (m * 32 + half * 16 + 32 < rt ? a_up : 0u));      // (so is an odd last fragment)
+                        mm_ldsm4(w, base + a_off[k] + m * 16 * 64 - (m * 16 + 16 < rt ? 0u : a_up));      // (so is an odd last fragment)
 #pragma unroll
                         for (int u = 0; u < 2; u++) {
-                            if (m + u >= MW || (m + u) * 32 + half * 16 >= rt) break;
+                            if (m + u >= MT || (m + u) * 16 >= rt) break;
                             unsigned short h0, h1;
-                            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h0) : "r"(sb + (m + u) * 256 + k * 2));
-                            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h1) : "r"(sb + (m + u) * 256 + 64 + k * 2));
+                            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h0) : "r"(sb + (m + u) * 128 + k * 2));
+                            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h1) : "r"(sb + (m + u) * 128 + 64 + k * 2));
                             const float e0 = __half2float(__ushort_as_half(h0)), e1 = __half2float(__ushort_as_half(h1));
                             const unsigned long long d0 = mm_pack(e0, e0), d1 = mm_pack(e1, e1);
                             const uint32_t w0 = w[2 * u], w1 = w[2 * u + 1];
@@ -406,15 +407,17 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
                     }
                 }
             }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty + slot);                 // handed back
+            if (++slot == S) { slot = 0; phase ^= 1u; }
         }
-        // ---- the pairs' partial tiles: [token][row], each over its own ring (all copies have landed: the last stage was the last
+        // ---- the warps' partial tiles: [token][row], each over its own ring (all copies have landed: the last stage was the last
         // one requested); a pitch of 4 (20) mod 32 words keeps the fragment stores free of bank conflicts
-        pair_sync();
         const int pitch = rt + 4;
-        float * mine = reinterpret_cast<float *>(smem + (size_t)pair * p.ring);
+        float * mine = reinterpret_cast<float *>(smem + (size_t)me * p.ring);
 #pragma unroll
-        for (int m = 0; m < MW; m++) {
-            if (m * 32 + half * 16 >= rt) break;
+        for (int m = 0; m < MT; m++) {
+            if (m * 16 >= rt) break;
 #pragma unroll
             for (int n = 0; n < NT; n++)
 #pragma unroll
@@ -426,14 +429,18 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
                     } else {
                         v = acc[Q4 ? 0 : m][Q4 ? 0 : n][j];
                     }
-                    mine[(n * 8 + 2 * q + (j & 1)) * pitch + m * 32 + half * 16 + g + (j >> 1) * 8] = v;
+                    mine[(n * 8 + 2 * q + (j & 1)) * pitch + m * 16 + g + (j >> 1) * 8] = v;
                 }
         }
         if (tid < 4) s_any[tid] = 0u;
-        __syncthreads();
+        {                                                             // all partial tiles are there; the warps agree whether a wait ran out
+            int dead = s_dead;
+            asm volatile("{\n .reg .pred p, q;\n setp.ne.s32 p, %0, 0;\n bar.red.or.pred q, 1, 256, p;\n selp.s32 %0, 1, 0, q;\n}" : "+r"(dead) :: "memory");
+            if (dead) return;
+        }
         const float * sums = reinterpret_cast<const float *>(smem);
         const int n_tile = GATED ? n_rows / 2 : n_rows;
-        for (int t = warp; t < p.T; t += MM_WARPS) {
+        for (int t = warp; t < p.T; t += MM_RINGS) {
             for (int k0 = 0; k0 < n_tile; k0 += 32) {
                 const int k = k0 + lane;
                 const bool mine_k = k < n_tile;
@@ -442,14 +449,14 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
                     if (GATED) {
                         float u = 0.f, v = 0.f;
 #pragma unroll
-                        for (int w = 0; w < MM_PAIRS; w++) {
+                        for (int w = 0; w < MM_RINGS; w++) {
                             const float2 f = *reinterpret_cast<const float2 *>(sums + (size_t)w * (p.ring / 4) + t * pitch + 2 * k);
                             u += f.x; v += f.y;
                         }
                         o = fmaxf(v, 0.f) * u;
                     } else {
 #pragma unroll
-                        for (int w = 0; w < MM_PAIRS; w++) o += sums[(size_t)w * (p.ring / 4) + t * pitch + k];
+                        for (int w = 0; w < MM_RINGS; w++) o += sums[(size_t)w * (p.ring / 4) + t * pitch + k];
                     }
                     const int item = lo + first + k;
                     const int r = SPARSE ? rows[first + k] : item;
@@ -473,14 +480,15 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
             }
         }
         if (!SPARSE && p.masks_out) {
-            __syncthreads();
+            asm volatile("bar.sync 1, 256;" ::: "memory");
             if (tid < 16 && tid * 8 < n_tile) {                       // the range starts at a multiple of 8 rows
                 unsigned char * o = reinterpret_cast<unsigned char *>(p.masks_out) + (lo + first) / 8 + tid;
                 const unsigned char bits = (unsigned char)(s_any[tid / 4] >> (tid % 4 * 8));
                 *o = p.masks_or ? (unsigned char)(*o | bits) : bits;
             }
         }
-        if (tile + 1 < n_tiles) __syncthreads();                      // the sums are read, their rings may fill again
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_tile);                          // the sums are read: when all warps are here the rings may fill again
     }
 }
 
@@ -493,7 +501,7 @@ static int mm_go(MmP p, bool pdl, cudaStream_t st) {
     const int G = (int)imin64(sm_count(), (p.nrows + 7) / 8);
     const int list = SPARSE ? ((p.nrows + G - 1) / G + 1) * 4 : 0;    // bytes
     if (list > 8192 - 128) return PI_ERR_UNSUPPORTED;                 // (more than MM_MAX_ROWS rows)
-    p.ring = (MM_SMEM_MAX - list) / MM_PAIRS / 128 * 128;
+    p.ring = (MM_SMEM_MAX - list) / MM_RINGS / 128 * 128;
     static bool attr_done[16] = {false};
     int dev = 0;
     PI_CUDA(cudaGetDevice(&dev));
@@ -502,7 +510,7 @@ static int mm_go(MmP p, bool pdl, cudaStream_t st) {
         PI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MM_SMEM_MAX));
         attr_done[dev] = true;
     }
-    PI_CUDA(launch_k(kern, dim3(G), dim3(MM_THREADS), (size_t)p.ring * MM_PAIRS + list, st, pdl, p));
+    PI_CUDA(launch_k(kern, dim3(G), dim3(MM_THREADS), (size_t)p.ring * MM_RINGS + list, st, pdl, p));
     return PI_OK;
 }
 
@@ -545,7 +553,7 @@ int launch_mm(const GemvArgs & a, cudaStream_t st) {
         p.dst16 = a.dst16 ? a.dst16 + (size_t)t0 * a.dst_stride : nullptr; p.dst_stride = a.dst_stride;
         p.coef = a.coef ? a.coef + (size_t)t0 * a.coef_stride : nullptr; p.coef_stride = a.coef_stride;
         p.masks_out = a.masks_out; p.masks_threshold = a.masks_threshold; p.masks_or = t0 > 0;
-        p.n_slices = 0; p.ring = 0;
+        p.status = a.status; p.n_slices = 0; p.ring = 0;
         const int rc = q4 ? mm_tokens<PI_TYPE_Q4_0>(p, a.pdl, st) : mm_tokens<PI_TYPE_F16>(p, a.pdl, st);
         if (rc != PI_OK) return rc;
     }

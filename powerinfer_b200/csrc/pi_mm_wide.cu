@@ -106,51 +106,65 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
     constexpr int CW = WB / 16;                                       // 16-byte pieces of a row
     constexpr int NW = (TM * CW + MW_THREADS - 1) / MW_THREADS;
     const int cw = tid % CW;
-    const uint8_t * wp[NW]; const uint8_t * sp = nullptr;             // nullptr: no such row
+    const uint8_t * wp[NW]; const uint8_t * sp = nullptr;             // my pieces of the next slice
+    unsigned w_ok = 0u;                                               // which of these rows exist
     int i_tile = 0, i_slice = 0;                                      // the unit that is requested next
-    auto row_ptr = [&](int r) -> const uint8_t * {                    // fragment row r of the tile (gated: 8 up rows, then their 8 gate rows)
+    auto row_ptr = [&](int r, bool & ok) -> const uint8_t * {         // fragment row r of the tile (gated: 8 up rows, then their 8 gate rows)
         const int k = i_tile * IT + (GATED ? (r >> 4) * 8 + (r & 7) : r);
-        if (r >= TM || lo + k >= hi) return nullptr;
-        return (GATED && (r & 8) ? p.W2 : p.W) + (size_t)(SPARSE ? rows[k] : lo + k) * p.row_bytes;
+        ok = r < TM && lo + k < hi;
+        return (GATED && (r & 8) ? p.W2 : p.W) + (ok ? (size_t)(SPARSE ? rows[k] : lo + k) * p.row_bytes : 0);
     };
+    // Addresses are kept and moved along: a chain of address arithmetic per copy stalls the warp that should be at the products.
+    const bool ragged = !Q4 && p.ncols % 64 != 0;                     // the last slice of a row is not whole
+    const int wr = tid / CW, xt = tid >> 3, xc = tid & 7, dt = tid >> 2;
+    const uint32_t w_to = (uint32_t)(wr * WB + (Q4 ? (cw ^ (wr >> 1)) & 3 : (cw ^ wr) & 7) * 16), x_to = x_off + (uint32_t)(xt * 128 + ((xc ^ xt) & 7) * 16);
+    const uint32_t d_to = d_off + (uint32_t)(((tid & 3) * XR + dt) * 4);
+    const char * const x0 = Q4 ? reinterpret_cast<const char *>((xc & 1 ? p.x.hi : p.x.lo) + (size_t)xt * p.nb + (xc >> 1)) : reinterpret_cast<const char *>(p.x.h16 + (size_t)xt * p.ncols + xc * 8);
+    const char * const d0 = reinterpret_cast<const char *>(p.x.d + (size_t)dt * p.nb + (tid & 3));
+    const size_t x_step = (size_t)(Q4 ? p.nb * 16 : p.ncols * 2) * 64, d_step = (size_t)p.nb * 4 * 128;
+    constexpr int NX = Z::TN / 64, ND = (Z::TN + 127) / 128;
     auto issue_w = [&](int slot) {
         if (i_slice == 0) {
+            w_ok = 0u;
 #pragma unroll
-            for (int j = 0; j < NW; j++) wp[j] = row_ptr(tid / CW + j * (MW_THREADS / CW));
-            if (Q4) sp = row_ptr(tid);
+            for (int j = 0; j < NW; j++) {
+                bool ok;
+                wp[j] = row_ptr(wr + j * (MW_THREADS / CW), ok) + cw * 16;
+                if (ok) w_ok |= 1u << j;
+            }
+            if (Q4) {
+                bool ok;
+                sp = row_ptr(tid, ok) + (size_t)p.nb * 16;
+                if (ok) w_ok |= 1u << NW;
+            }
         }
         const uint32_t base = ring + (uint32_t)(slot * p.stage);
-        const int off = i_slice * WB + cw * 16;
-        const bool in = Q4 || off < p.ncols * 2;                      // past the end of a row: zeros
+        const bool in = !ragged || i_slice * 64 + cw * 8 < p.ncols;   // past the end of a row: zeros
 #pragma unroll
         for (int j = 0; j < NW; j++) {
-            const int r = tid / CW + j * (MW_THREADS / CW);
-            const uint32_t to = base + r * WB + (Q4 ? (cw ^ (r >> 1)) & 3 : (cw ^ r) & 7) * 16;
-            if (wp[j]) { if (in) mw_cp16(to, wp[j] + off); else mw_zero16(to); }
+            const uint32_t to = base + w_to + j * (MW_THREADS / CW) * WB;
+            if (w_ok >> j & 1u) { if (in) mw_cp16(to, wp[j]); else mw_zero16(to); }
+            wp[j] += WB;
         }
-        if (Q4 && sp) mw_cp8(base + s_off + tid * 8, sp + (size_t)p.nb * 16 + i_slice * 8);
+        if (Q4) {
+            if (w_ok >> NW & 1u) mw_cp8(base + s_off + tid * 8, sp);
+            sp += 8;
+        }
     };
     auto issue_x = [&](int slot) {
         const uint32_t base = ring + (uint32_t)(slot * p.stage);
-        const int c = tid & 7;
+        const char * src = x0 + (size_t)i_slice * (Q4 ? 64 : 128);
+        if (ragged && i_slice * 64 + xc * 8 >= p.ncols) {
 #pragma unroll
-        for (int j = 0; j < MW_TOKENS / 64; j++) {
-            const int t = (tid >> 3) + j * 64;
-            if (t >= p.T) break;
-            const uint32_t to = base + x_off + t * 128 + ((c ^ t) & 7) * 16;
-            if (Q4) {
-                mw_cp16(to, (c & 1 ? p.x.hi : p.x.lo) + (size_t)t * p.nb + i_slice * 4 + (c >> 1));
-            } else {
-                const int col = i_slice * 64 + c * 8;
-                if (col < p.ncols) mw_cp16(to, p.x.h16 + (size_t)t * p.ncols + col); else mw_zero16(to);
-            }
+            for (int j = 0; j < NX; j++) if (xt + j * 64 < p.T) mw_zero16(base + x_to + j * 64 * 128);
+        } else {
+#pragma unroll
+            for (int j = 0; j < NX; j++, src += x_step) if (xt + j * 64 < p.T) mw_cp16(base + x_to + j * 64 * 128, src);
         }
         if (Q4) {
+            const char * sd = d0 + (size_t)i_slice * 16;
 #pragma unroll
-            for (int j = 0; j < MW_TOKENS / 128; j++) {
-                const int t = (tid >> 2) + j * 128, k = tid & 3;
-                if (t < p.T) mw_cp4(base + d_off + (k * XR + t) * 4, p.x.d + (size_t)t * p.nb + i_slice * 4 + k);
-            }
+            for (int j = 0; j < ND; j++, sd += d_step) if (dt + j * 128 < p.T) mw_cp4(base + d_to + j * 128 * 4, sd);
         }
     };
     auto advance = [&]() { if (++i_slice == p.n_slices) { i_slice = 0; i_tile++; } };
