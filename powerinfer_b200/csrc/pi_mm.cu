@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
     __shared__ uint64_t s_full[MM_RINGS][MM_SMAX], s_empty[MM_RINGS][MM_SMAX], s_tile;
     __shared__ volatile int s_dead;
     int * rows = reinterpret_cast<int *>(smem + (size_t)MM_RINGS * p.ring);      // rows of this CTA (sparse only)
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);    // (uniform, also for the compiler: see the note)
     const int G = gridDim.x, cta = blockIdx.x;
     const int me = warp & (MM_RINGS - 1);                             // my ring
     const uint32_t ring_a = smem_u32(smem) + (uint32_t)(me * p.ring);
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
         int before = 0, total = 0;
 #pragma unroll
         for (int w = 0; w < MM_WARPS; w++) { if (w < warp) before += s_warp[w]; total += s_warp[w]; }
-        set_range(total);
+        set_range(__shfl_sync(0xffffffffu, total, 0));
         if (cta == 0 && tid == 0) {
             if (p.count) *p.count = total;
             if (p.rows_total && total) atomicAdd(p.rows_total, (unsigned long long)total);      // statistics

@@ -6,17 +6,22 @@
 // 8 tokens and the four packed FP32 operations that apply its scales take 18 clocks of a scheduler together (they share a pipe).
 // What must not cost extra is shared memory: every warp reads its own fragments of both operands.
 //
-// Work split: as in pi_mm.cu every CTA takes an equal contiguous range of rows, in tiles of 32, 64 or 128; here the 16 warps share a
-// stage (128 bytes of every activation, 128 or 64 of every row) and split the TILE, WM ways along the rows and WN along the tokens:
-// no partial sums, so the accumulators of a tile exist once and the tile can be 128 x 256.  A stage holds enough products (2000
-// clocks of them at 128 x 128) for its barrier.  Warps without rows or tokens do nothing, and are spread over the four schedulers.
+// Work split: as in pi_mm.cu every CTA takes an equal contiguous range of rows, in tiles of 96, and producer warps (4) copy for the
+// consumers (12) (a computing warp that issues cp.async waits while the SM's queue of outstanding loads is full: 700 to 2900 of the
+// clocks of a stage).  Here all consumers share a stage (128 bytes of every activation, 128 or 64 of every row) and split the TILE:
+// no partial sums, so the accumulators of a tile exist once and the tile can be 96 x 256.  Up to 128 tokens 6 x 2 consumers of 16 rows,
+// beyond that 3 x 4 consumers of 32 rows; the token count of a consumer is a template argument in steps of 8 or 16, because a branch
+// around every pair of products costs more than the products that it leaves out.
 // The accumulators go straight to global memory: the ring runs on across tiles.
+// Every wait is bounded, as in pi_mm.cu.
 #include "pi_common.cuh"
 
 namespace pi {
 
-static constexpr int MW_THREADS = 512;
-static constexpr int MW_SMEM_MAX = 224 * 1024;
+static constexpr int MW_THREADS = 512, MW_CONS = 12, MW_PROD = 128;       // warps 0 .. 11 consume, threads 384 .. 511 produce
+static constexpr int MW_REGS_C = 152, MW_REGS_P = 56;   // 384 x 152 + 128 x 56 = the 512 x 128 of the launch
+static constexpr int MW_TM = 96;                        // rows of a tile
+static constexpr int MW_SMEM_MAX = 224 * 1024;          // (leaves room for the static variables)
 static constexpr int MW_SMAX = 6;                       // stages at most
 static constexpr int MW_TOKENS = 256;                   // of a launch
 
@@ -29,22 +34,15 @@ struct MwP {
     float * dst; __half * dst16; int64_t dst_stride;
     __half * coef; int64_t coef_stride;
     uint32_t * masks_out; float masks_threshold; int masks_or;
-    int n_slices, stage, S;                             // column slices of a row; bytes of a stage; stages
+    unsigned int * status;
+    int n_slices, S;                                    // column slices of a row; stages
 };
 
 __device__ __forceinline__ void mw_cp16(uint32_t dst, const void * src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory"); }
 __device__ __forceinline__ void mw_cp8(uint32_t dst, const void * src)  { asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" :: "r"(dst), "l"(src) : "memory"); }
 __device__ __forceinline__ void mw_cp4(uint32_t dst, const void * src)  { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(dst), "l"(src) : "memory"); }
 __device__ __forceinline__ void mw_zero16(uint32_t dst) { asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" :: "r"(dst), "r"(0u) : "memory"); }
-__device__ __forceinline__ void mw_wait(int pending) {                // all but the last `pending` (0 .. MW_SMAX - 2) groups have landed
-    switch (pending) {
-        case 0: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
-        case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
-        case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
-        case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
-        default: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
-    }
-}
+__device__ __forceinline__ void mw_arrive_copies(uint64_t * bar) { asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" :: "r"(smem_u32(bar)) : "memory"); }
 __device__ __forceinline__ void mw_ldsm4(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
@@ -64,35 +62,48 @@ __device__ __forceinline__ void mw_scale_add(unsigned long long & acc, unsigned 
     asm("{\n .reg .b64 t;\n fma.rn.f32x2 t, %1, %2, %3;\n fma.rn.f32x2 %0, t, %4, %0;\n}" : "+l"(acc) : "l"(v), "l"(dd), "l"(md), "l"(d4));
 }
 
-// MT x 16 rows and NT x 8 tokens per warp; WM x WN warps
-template <int WT, int MT, int WM, int WN, int NT>
+// WM x WN consumers of MT x 16 rows and NT x 8 tokens
+template <int WT, int WM, int WN, int NT>
 struct MwShape {
     static constexpr bool Q4 = WT == PI_TYPE_Q4_0;
-    static constexpr int TM = WM * MT * 16, TN = WN * NT * 8;
+    static constexpr int MT = MW_TM / 16 / WM, TN = WN * NT * 8;
     static constexpr int KS = Q4 ? 128 : 64;                          // columns of a stage
     static constexpr int WB = Q4 ? 64 : 128;                          // bytes of a row in a stage (Q4_0: of its nibbles)
-    static_assert(WM * WN * 32 == MW_THREADS, "warps");
+    // a stage: rows [MW_TM][WB], activations [TN][128], Q4_0: rows' scales [MW_TM][4 halves], activation scales [4][TN] floats
+    static constexpr int X_OFF = MW_TM * WB, S_OFF = X_OFF + TN * 128, D_OFF = S_OFF + (Q4 ? MW_TM * 8 : 0), STAGE = D_OFF + (Q4 ? TN * 16 : 0);
+    static_assert(WM * WN == MW_CONS && MT * WM * 16 == MW_TM && STAGE % 128 == 0, "split");
 };
 
-template <int WT, int MT, int WM, int WN, int NT, bool SPARSE, bool GATED>
+template <int WT, int WM, int WN, int NT, bool SPARSE, bool GATED>
 __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
-    using Z = MwShape<WT, MT, WM, WN, NT>;
+    using Z = MwShape<WT, WM, WN, NT>;
     constexpr bool Q4 = Z::Q4;
-    constexpr int TM = Z::TM, WB = Z::WB;
+    constexpr int TM = MW_TM, WB = Z::WB, MT = Z::MT;
     constexpr int IT = GATED ? TM / 2 : TM;                           // items (rows / neurons) of a tile
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int s_warp[MW_THREADS / 32];
     __shared__ unsigned s_any[4];
-    int * rows = reinterpret_cast<int *>(smem + (size_t)p.S * p.stage);          // rows of this CTA (sparse only)
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = WM == 4 ? (warp + (warp >> 2)) & 3 : (warp + (warp >> 2)) & 1, wn = WM == 4 ? warp >> 2 : warp >> 1;
+    __shared__ uint64_t s_full[MW_SMAX], s_empty[MW_SMAX], s_bits[2];
+    __shared__ volatile int s_dead;
+    int * rows = reinterpret_cast<int *>(smem + (size_t)p.S * Z::STAGE);          // rows of this CTA (sparse only)
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);    // (uniform, also for the compiler: see the note)
+    const int wm = warp % WM, wn = warp / WM;
     const int G = gridDim.x, cta = blockIdx.x, S = p.S;
     const uint32_t ring = smem_u32(smem);
-    const int XR = (p.T + 15) / 16 * 16;                              // token rows of a stage
-    // a stage: rows [TM][WB], activations [XR][128], Q4_0: rows' scales [TM][4 halves], activation scales [4][XR] floats
-    const uint32_t x_off = TM * WB, s_off = x_off + XR * 128, d_off = s_off + TM * 8;
+    constexpr uint32_t x_off = Z::X_OFF, s_off = Z::S_OFF, d_off = Z::D_OFF;
     if (tid < 4) s_any[tid] = 0u;
+    if (tid < MW_SMAX) { mbar_init(s_full + tid, MW_PROD); mbar_init(s_empty + tid, MW_CONS); }
+    if (tid == 0) { mbar_init(s_bits, MW_CONS); mbar_init(s_bits + 1, MW_CONS); s_dead = 0; }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    __syncthreads();
     pdl_launch();
+    auto wait = [&](uint64_t * bar, unsigned parity) -> bool {        // warp-uniform; false: the wait ran out, here or elsewhere
+        bool ok = false;
+        for (int spins = 0; spins < (1 << 20) && !ok && !s_dead; spins++) ok = mbar_try_wait(bar, parity);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok && lane == 0) { s_dead = 1; if (p.status) atomicOr(p.status, 16u); }
+        return ok;
+    };
 
     int lo = 0, hi = 0, n_units = 0;
     auto set_range = [&](int n) {
@@ -104,8 +115,9 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
     };
     // ---- copies: a thread's pieces of a stage lie in the same rows for a whole tile
     constexpr int CW = WB / 16;                                       // 16-byte pieces of a row
-    constexpr int NW = (TM * CW + MW_THREADS - 1) / MW_THREADS;
-    const int cw = tid % CW;
+    constexpr int NW = (TM * CW + MW_PROD - 1) / MW_PROD, WS = MW_PROD / CW;     // pieces of a thread, rows between them
+    const int pt = tid - MW_CONS * 32;                              // producer thread
+    const int cw = pt % CW;
     const uint8_t * wp[NW]; const uint8_t * sp = nullptr;             // my pieces of the next slice
     unsigned w_ok = 0u;                                               // which of these rows exist
     int i_tile = 0, i_slice = 0;                                      // the unit that is requested next
@@ -116,55 +128,55 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
     };
     // Addresses are kept and moved along: a chain of address arithmetic per copy stalls the warp that should be at the products.
     const bool ragged = !Q4 && p.ncols % 64 != 0;                     // the last slice of a row is not whole
-    const int wr = tid / CW, xt = tid >> 3, xc = tid & 7, dt = tid >> 2;
+    const int wr = pt / CW, xt = pt >> 3, xc = pt & 7, dt = pt >> 2;
     const uint32_t w_to = (uint32_t)(wr * WB + (Q4 ? (cw ^ (wr >> 1)) & 3 : (cw ^ wr) & 7) * 16), x_to = x_off + (uint32_t)(xt * 128 + ((xc ^ xt) & 7) * 16);
-    const uint32_t d_to = d_off + (uint32_t)(((tid & 3) * XR + dt) * 4);
+    const uint32_t d_to = d_off + (uint32_t)(((pt & 3) * Z::TN + dt) * 4);
     const char * const x0 = Q4 ? reinterpret_cast<const char *>((xc & 1 ? p.x.hi : p.x.lo) + (size_t)xt * p.nb + (xc >> 1)) : reinterpret_cast<const char *>(p.x.h16 + (size_t)xt * p.ncols + xc * 8);
-    const char * const d0 = reinterpret_cast<const char *>(p.x.d + (size_t)dt * p.nb + (tid & 3));
-    const size_t x_step = (size_t)(Q4 ? p.nb * 16 : p.ncols * 2) * 64, d_step = (size_t)p.nb * 4 * 128;
-    constexpr int NX = Z::TN / 64, ND = (Z::TN + 127) / 128;
+    const char * const d0 = reinterpret_cast<const char *>(p.x.d + (size_t)dt * p.nb + (pt & 3));
+    const size_t x_step = (size_t)(Q4 ? p.nb * 16 : p.ncols * 2) * 16, d_step = (size_t)p.nb * 4 * 32;
+    constexpr int NX = Z::TN / 16, ND = (Z::TN + 31) / 32;
     auto issue_w = [&](int slot) {
         if (i_slice == 0) {
             w_ok = 0u;
 #pragma unroll
             for (int j = 0; j < NW; j++) {
                 bool ok;
-                wp[j] = row_ptr(wr + j * (MW_THREADS / CW), ok) + cw * 16;
+                wp[j] = row_ptr(wr + j * WS, ok) + cw * 16;
                 if (ok) w_ok |= 1u << j;
             }
             if (Q4) {
                 bool ok;
-                sp = row_ptr(tid, ok) + (size_t)p.nb * 16;
+                sp = row_ptr(pt, ok) + (size_t)p.nb * 16;
                 if (ok) w_ok |= 1u << NW;
             }
         }
-        const uint32_t base = ring + (uint32_t)(slot * p.stage);
+        const uint32_t base = ring + (uint32_t)(slot * Z::STAGE);
         const bool in = !ragged || i_slice * 64 + cw * 8 < p.ncols;   // past the end of a row: zeros
 #pragma unroll
         for (int j = 0; j < NW; j++) {
-            const uint32_t to = base + w_to + j * (MW_THREADS / CW) * WB;
+            const uint32_t to = base + w_to + j * WS * WB;
             if (w_ok >> j & 1u) { if (in) mw_cp16(to, wp[j]); else mw_zero16(to); }
             wp[j] += WB;
         }
         if (Q4) {
-            if (w_ok >> NW & 1u) mw_cp8(base + s_off + tid * 8, sp);
+            if (w_ok >> NW & 1u) mw_cp8(base + s_off + pt * 8, sp);
             sp += 8;
         }
     };
     auto issue_x = [&](int slot) {
-        const uint32_t base = ring + (uint32_t)(slot * p.stage);
+        const uint32_t base = ring + (uint32_t)(slot * Z::STAGE);
         const char * src = x0 + (size_t)i_slice * (Q4 ? 64 : 128);
         if (ragged && i_slice * 64 + xc * 8 >= p.ncols) {
 #pragma unroll
-            for (int j = 0; j < NX; j++) if (xt + j * 64 < p.T) mw_zero16(base + x_to + j * 64 * 128);
+            for (int j = 0; j < NX; j++) if (xt + j * 16 < p.T) mw_zero16(base + x_to + j * 16 * 128);
         } else {
 #pragma unroll
-            for (int j = 0; j < NX; j++, src += x_step) if (xt + j * 64 < p.T) mw_cp16(base + x_to + j * 64 * 128, src);
+            for (int j = 0; j < NX; j++, src += x_step) if (xt + j * 16 < p.T) mw_cp16(base + x_to + j * 16 * 128, src);
         }
         if (Q4) {
             const char * sd = d0 + (size_t)i_slice * 16;
 #pragma unroll
-            for (int j = 0; j < ND; j++, sd += d_step) if (dt + j * 128 < p.T) mw_cp4(base + d_to + j * 128 * 4, sd);
+            for (int j = 0; j < ND; j++, sd += d_step) if (dt + j * 32 < p.T) mw_cp4(base + d_to + j * 32 * 4, sd);
         }
     };
     auto advance = [&]() { if (++i_slice == p.n_slices) { i_slice = 0; i_tile++; } };
@@ -199,7 +211,7 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
         int before = 0, total = 0;
 #pragma unroll
         for (int w = 0; w < MW_THREADS / 32; w++) { if (w < warp) before += s_warp[w]; total += s_warp[w]; }
-        set_range(total);
+        set_range(__shfl_sync(0xffffffffu, total, 0));
         if (cta == 0 && tid == 0) {
             if (p.count) *p.count = total;
             if (p.rows_total && total) atomicAdd(p.rows_total, (unsigned long long)total);      // statistics
@@ -224,11 +236,25 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
         __syncthreads();
         if (p.list) for (int k = tid; k < hi - lo; k += MW_THREADS) p.list[lo + k] = rows[k];
     }
-    for (int s = 0; s < S - 1; s++) {
-        if (s < n_units) { issue_w(s); issue_x(s); advance(); }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+    if (warp >= MW_CONS) {
+        // ================================================================= producers
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(MW_REGS_P));
+        int slot = 0;
+        unsigned phase = 1u;                                          // parity of the hand-back to wait for (first round: none)
+        for (int i = 0; i < n_units; i++) {
+            if (!wait(s_empty + slot, phase)) break;
+            issue_w(slot);
+            issue_x(slot);
+            if (ragged && i_slice == p.n_slices - 1) __threadfence_block();      // zeros were stored, not copied
+            mw_arrive_copies(s_full + slot);
+            advance();
+            if (++slot == S) { slot = 0; phase ^= 1u; }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        return;
     }
-
+    // ===================================================================== consumers
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(MW_REGS_C));
     float acc[Q4 ? 1 : MT][Q4 ? 1 : NT][4];                           // (the accumulators of the two types have different shapes)
     unsigned long long acq[Q4 ? MT : 1][Q4 ? NT : 1][2];
     auto clear = [&]() {
@@ -241,24 +267,20 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
     };
     clear();
     const int g = lane >> 2, q = lane & 3;
-    const int row0 = wm * MT * 16, tok0 = wn * NT * 8;                // this warp's part of the tile
     const uint32_t MAGIC = 0x4B400000u;
     const unsigned long long neg_magic = mw_pack(-12582912.0f, -12582912.0f), sixteenth = mw_pack(0.0625f, 0.0625f);
+    const int row0 = wm * MT * 16, tok0 = wn * NT * 8;                // this warp's part of the tile
     // ldmatrix row addresses inside a stage (fragment layouts of mma.m16n8k16 / m16n8k32); the piece is added per step
     const uint32_t a_row = (uint32_t)((row0 + (Q4 && MT == 2 ? lane : lane & 15)) * WB);
-    const uint32_t b_row = x_off + (uint32_t)((tok0 + (lane & 7) + (lane >> 4) * 8) * 128);
+    const uint32_t b_row = x_off + (uint32_t)((tok0 + (lane & 7) + (lane >> 4) * 8) * 128), b_last = x_off + (uint32_t)((tok0 + (NT - 1) * 8 + (lane & 7)) * 128);
     const int a_swz = Q4 ? (lane >> 1) & 3 : lane & 7, b_swz = lane & 7;
 
-    int tile = 0, slice = 0, slot = 0, next = S - 1;
+    int tile = 0, slice = 0, slot = 0;
+    unsigned phase = 0u;
     for (int i = 0; i < n_units; i++) {
-        mw_wait(S - 2);
-        __syncthreads();                                              // stage i has landed for everybody; stage i - 1 is consumed
-        if (i + S - 1 < n_units) { issue_w(next); issue_x(next); advance(); }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        if (++next == S) next = 0;
-        const uint32_t base = ring + (uint32_t)(slot * p.stage);
-        if (++slot == S) slot = 0;
-        const int n_tile = min(IT, hi - lo - tile * IT);
+        if (!wait(s_full + slot, phase)) break;
+        const uint32_t base = ring + (uint32_t)(slot * Z::STAGE);
+        const int n_tile = min(IT, hi - lo - tile * IT);              // items
         const bool busy = (GATED ? row0 / 2 : row0) < n_tile && tok0 < p.T;       // my rows and tokens exist
         if (!busy) {
         } else if (!Q4) {
@@ -269,13 +291,12 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
                 for (int m = 0; m < MT; m++) mw_ldsm4(a[m], base + a_row + m * 16 * WB + (((2 * k + (lane >> 4)) ^ a_swz) & 7) * 16);
 #pragma unroll
                 for (int n = 0; n < NT; n += 2) {
-                    if (tok0 + n * 8 >= p.T) break;
                     uint32_t b[4];
-                    mw_ldsm4(b, base + b_row + n * 8 * 128 + (((2 * k + ((lane >> 3) & 1)) ^ b_swz) & 7) * 16);
+                    mw_ldsm4(b, base + (n + 1 < NT ? b_row + n * 8 * 128 : b_last) + (((2 * k + ((lane >> 3) & 1)) ^ b_swz) & 7) * 16);
 #pragma unroll
                     for (int m = 0; m < MT; m++) {
                         mw_hmma(acc[Q4 ? 0 : m][Q4 ? 0 : n], a[m], b[0], b[1]);
-                        mw_hmma(acc[Q4 ? 0 : m][Q4 ? 0 : n + 1], a[m], b[2], b[3]);
+                        if (n + 1 < NT) mw_hmma(acc[Q4 ? 0 : m][Q4 ? 0 : (n + 1) % NT], a[m], b[2], b[3]);
                     }
                 }
             }
@@ -307,26 +328,29 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
                 }
 #pragma unroll
                 for (int n = 0; n < NT; n += 2) {
-                    if (tok0 + n * 8 >= p.T) break;
                     uint32_t b[4];
-                    mw_ldsm4(b, base + b_row + n * 8 * 128 + (((2 * k + ((lane >> 3) & 1)) ^ b_swz) & 7) * 16);
+                    mw_ldsm4(b, base + (n + 1 < NT ? b_row + n * 8 * 128 : b_last) + (((2 * k + ((lane >> 3) & 1)) ^ b_swz) & 7) * 16);
 #pragma unroll
                     for (int u = 0; u < 2; u++) {
+                        if (n + u >= NT) break;
                         unsigned long long dd;
-                        asm volatile("ld.shared.b64 %0, [%1];" : "=l"(dd) : "r"(base + d_off + (k * XR + tok0 + (n + u) * 8 + 2 * q) * 4));
+                        asm volatile("ld.shared.b64 %0, [%1];" : "=l"(dd) : "r"(base + d_off + (k * Z::TN + tok0 + (n + u) * 8 + 2 * q) * 4));
                         dd = mw_mul2(dd, sixteenth);
                         const unsigned long long md = mw_mul2(dd, neg_magic);
 #pragma unroll
                         for (int m = 0; m < MT; m++) {
                             uint32_t c[4];
                             mw_imma(c, a[m], b[2 * u], b[2 * u + 1], MAGIC);
-                            mw_scale_add(acq[Q4 ? m : 0][Q4 ? n + u : 0][0], mw_packu(c[0], c[1]), dd, md, d4[m][0]);
-                            mw_scale_add(acq[Q4 ? m : 0][Q4 ? n + u : 0][1], mw_packu(c[2], c[3]), dd, md, d4[m][1]);
+                            mw_scale_add(acq[Q4 ? m : 0][Q4 ? (n + u) % NT : 0][0], mw_packu(c[0], c[1]), dd, md, d4[m][0]);
+                            mw_scale_add(acq[Q4 ? m : 0][Q4 ? (n + u) % NT : 0][1], mw_packu(c[2], c[3]), dd, md, d4[m][1]);
                         }
                     }
                 }
             }
         }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_empty + slot);                   // handed back
+        if (++slot == S) { slot = 0; phase ^= 1u; }
         if (slice == p.n_slices - 1) {
             // ---- the tile is complete: a lane holds rows g and g + 8 of each fragment (gated: up and gate of one item), tokens 2q, 2q + 1
             if (busy) {
@@ -375,14 +399,19 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
                 }
             }
             if (!SPARSE && p.masks_out) {                             // the union over the tokens of !(result < threshold), one bit per row
-                __syncthreads();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(s_bits);
+                if (!wait(s_bits, (unsigned)tile & 1u)) break;
                 if (tid < TM / 8 && tid * 8 < n_tile) {               // the range starts at a multiple of 8 rows
                     unsigned char * o = reinterpret_cast<unsigned char *>(p.masks_out) + (lo + tile * IT) / 8 + tid;
                     const unsigned char bits = (unsigned char)(s_any[tid / 4] >> (tid % 4 * 8));
                     *o = p.masks_or ? (unsigned char)(*o | bits) : bits;
                 }
-                __syncthreads();
+                __syncwarp();
                 if (tid < 4) s_any[tid] = 0u;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(s_bits + 1);
+                if (!wait(s_bits + 1, (unsigned)tile & 1u)) break;
             }
             clear();
         }
@@ -391,48 +420,44 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
 }
 
 // ---------------------------------------------------------------------------------------------- launch
-template <int WT, int MT, int WM, int WN, int NT, bool SPARSE, bool GATED>
+template <int WT, int WM, int WN, int NT, bool SPARSE, bool GATED>
 static int mw_go(MwP p, bool pdl, cudaStream_t st) {
-    using Z = MwShape<WT, MT, WM, WN, NT>;
+    using Z = MwShape<WT, WM, WN, NT>;
     p.n_slices = (p.ncols + Z::KS - 1) / Z::KS;
     const int G = (int)imin64(sm_count(), (p.nrows + 7) / 8);
     const int list = SPARSE ? ((p.nrows + G - 1) / G + 1) * 4 : 0;    // bytes
-    const int XR = (p.T + 15) / 16 * 16;
-    p.stage = Z::TM * Z::WB + XR * 128 + (Z::Q4 ? Z::TM * 8 + XR * 16 : 0);
-    p.S = (MW_SMEM_MAX - list) / p.stage;
+    if (list > 8192) return PI_ERR_UNSUPPORTED;                       // (more than MM_MAX_ROWS rows)
+    p.S = (MW_SMEM_MAX - list) / Z::STAGE;
     if (p.S > MW_SMAX) p.S = MW_SMAX;
-    if (p.S < 2 || list > 8192) return PI_ERR_UNSUPPORTED;            // (more than MM_MAX_ROWS rows)
+    static_assert(2 * Z::STAGE <= MW_SMEM_MAX - 8192, "two stages");
     static bool attr_done[16] = {false};
     int dev = 0;
     PI_CUDA(cudaGetDevice(&dev));
-    auto kern = k_mm_wide<WT, MT, WM, WN, NT, SPARSE, GATED>;
+    auto kern = k_mm_wide<WT, WM, WN, NT, SPARSE, GATED>;
     if (dev >= 0 && dev < 16 && !attr_done[dev]) {
         PI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MW_SMEM_MAX));
         attr_done[dev] = true;
     }
-    PI_CUDA(launch_k(kern, dim3(G), dim3(MW_THREADS), (size_t)p.S * p.stage + list, st, pdl, p));
+    PI_CUDA(launch_k(kern, dim3(G), dim3(MW_THREADS), (size_t)p.S * Z::STAGE + list, st, pdl, p));
     return PI_OK;
 }
 
-template <int WT, int MT, int WM, int WN, int NT>
+template <int WT, int WM, int WN, int NT>
 static int mw_sel(const MwP & p, bool pdl, cudaStream_t st) {
-    if (!p.masks) return mw_go<WT, MT, WM, WN, NT, false, false>(p, pdl, st);
-    if (p.W2)     return mw_go<WT, MT, WM, WN, NT, true, true>(p, pdl, st);
-    return mw_go<WT, MT, WM, WN, NT, true, false>(p, pdl, st);
+    if (!p.masks) return mw_go<WT, WM, WN, NT, false, false>(p, pdl, st);
+    if (p.W2)     return mw_go<WT, WM, WN, NT, true, true>(p, pdl, st);
+    return mw_go<WT, WM, WN, NT, true, false>(p, pdl, st);
 }
 
-// The smallest tile that holds a CTA's share of the rows: with few rows more warps along the tokens.  Up to 128 tokens and up to 256.
+// the narrowest tile that holds the tokens
 template <int WT>
-static int mw_tile(const MwP & p, bool pdl, cudaStream_t st) {
-    const int64_t share = ((int64_t)p.nrows * (p.W2 ? 2 : 1) + sm_count() - 1) / sm_count();
-    if (p.T <= 128) {
-        if (share <= 32) return mw_sel<WT, 1, 2, 8, 2>(p, pdl, st);
-        if (share <= 64) return mw_sel<WT, 1, 4, 4, 4>(p, pdl, st);
-        return mw_sel<WT, 2, 4, 4, 4>(p, pdl, st);
-    }
-    if (share <= 32) return mw_sel<WT, 1, 2, 8, 4>(p, pdl, st);
-    if (share <= 64) return mw_sel<WT, 1, 4, 4, 8>(p, pdl, st);
-    return mw_sel<WT, 2, 4, 4, 8>(p, pdl, st);
+static int mw_tokens(const MwP & p, bool pdl, cudaStream_t st) {
+    if (p.T <= 64)  return mw_sel<WT, 6, 2, 4>(p, pdl, st);
+    if (p.T <= 80)  return mw_sel<WT, 6, 2, 5>(p, pdl, st);
+    if (p.T <= 96)  return mw_sel<WT, 6, 2, 6>(p, pdl, st);
+    if (p.T <= 128) return mw_sel<WT, 6, 2, 8>(p, pdl, st);
+    if (p.T <= 192) return mw_sel<WT, 3, 4, 6>(p, pdl, st);
+    return mw_sel<WT, 3, 4, 8>(p, pdl, st);
 }
 
 // Called by launch_mm, which has checked the arguments.  Tokens go in launches of at most 256.
@@ -454,8 +479,8 @@ int launch_mm_wide(const GemvArgs & a, cudaStream_t st) {
         p.dst = a.dst ? a.dst + (size_t)t0 * a.dst_stride : nullptr;
         p.dst16 = a.dst16 ? a.dst16 + (size_t)t0 * a.dst_stride : nullptr; p.dst_stride = a.dst_stride;
         p.coef = a.coef ? a.coef + (size_t)t0 * a.coef_stride : nullptr; p.coef_stride = a.coef_stride;
-        p.masks_out = a.masks_out; p.masks_threshold = a.masks_threshold; p.masks_or = t0 > 0;
-        const int rc = q4 ? mw_tile<PI_TYPE_Q4_0>(p, a.pdl, st) : mw_tile<PI_TYPE_F16>(p, a.pdl, st);
+        p.masks_out = a.masks_out; p.masks_threshold = a.masks_threshold; p.masks_or = t0 > 0; p.status = a.status;
+        const int rc = q4 ? mw_tokens<PI_TYPE_Q4_0>(p, a.pdl, st) : mw_tokens<PI_TYPE_F16>(p, a.pdl, st);
         if (rc != PI_OK) return rc;
     }
     return PI_OK;
