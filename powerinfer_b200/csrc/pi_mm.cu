@@ -40,6 +40,7 @@ static constexpr int MM_RINGS = 8, MM_WARPS = 2 * MM_RINGS, MM_THREADS = MM_WARP
 static constexpr int MM_REGS_C = 200, MM_REGS_P = 56;   // 256 x (200 + 56) = the 512 x 128 of the launch
 static constexpr int MM_SMAX = 8;                       // stages of a ring at most
 static constexpr int MM_SMEM_MAX = 225 * 1024;          // (leaves room for the static variables)
+static constexpr int MM_SLACK = 4096;                   // behind the last ring: fragments past a tile read up to 48 rows (3072 bytes, 384 of scales) on
 
 struct MmP {
     const uint8_t * W; const uint8_t * W2; int64_t row_bytes; int nrows, ncols, nb;
@@ -103,16 +104,20 @@ struct MmShape {
     static constexpr bool Q4 = WT == PI_TYPE_Q4_0;
     static constexpr int TP = NT * 8;                                 // token rows of a stage
     static constexpr int MT = Q4 && NT == 4 ? 7 : 8;                  // fragments of 16 rows of a tile at most (two stages have to fit)
+    // Fragments that are multiplied without a branch between them: a branch around every fragment left each one's chain of latencies
+    // (fragment, nibbles, product, scale: 150 clocks) in the open.  Few tokens leave the pipes idle anyway: fragments of 16 rows that
+    // the tile does not have are then cheaper multiplied (their rows are whatever lies behind the tile) than skipped.
+    static constexpr int MG = NT <= 2 ? 4 : 2, MA = (MT + MG - 1) / MG * MG;
     static constexpr int KS = Q4 ? 128 : 32;                          // columns of a slice
     static constexpr int ROW = Q4 ? 72 : 64, TOK = Q4 ? 144 : 64;     // bytes of a stage per row and per token
-    static_assert(2 * (MT * 16 * ROW + TP * TOK) * MM_RINGS <= MM_SMEM_MAX - 8192, "two stages");
+    static_assert(2 * (MT * 16 * ROW + TP * TOK) * MM_RINGS <= MM_SMEM_MAX - 8192 - MM_SLACK, "two stages");
 };
 
 template <int WT, int NT, bool SPARSE, bool GATED>
 __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
     using Z = MmShape<WT, NT>;
     constexpr bool Q4 = Z::Q4;
-    constexpr int TP = Z::TP, MT = Z::MT;
+    constexpr int TP = Z::TP, MT = Z::MT, MG = Z::MG, MA = Z::MA;
     constexpr int IT = GATED ? MT * 8 : MT * 16;                      // items (rows / neurons) of a tile at most
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int s_warp[MM_WARPS];
@@ -320,7 +325,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
     // ldmatrix addresses inside a stage (fragment layouts of mma.m16n8k16 / m16n8k32): two 16-byte pieces of 16 rows, four of 8 tokens
     // (Q4_0: one block of 32 rows, one block of two groups of 8 tokens)
     const int a_row = Q4 ? lane : lane & 15;
-    const uint32_t a_up = (lane >> 4) * 16 * 64, b_up = NT > 1 ? (lane >> 4) * 8 * 128 : 0;
+    const uint32_t b_up = NT > 1 ? (lane >> 4) * 8 * 128 : 0;
     const int b_row = Q4 ? (lane & 7) + (NT > 1 ? (lane >> 4) * 8 : 0) : (lane & 7);
     const uint32_t MAGIC = 0x4B400000u;
     const unsigned long long neg_magic = mm_pack(-12582912.0f, -12582912.0f), sixteenth = mm_pack(0.0625f, 0.0625f);
@@ -336,10 +341,10 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
     for (int tile = 0; tile < n_tiles; tile++) {
         start_tile(tile);
         // (the accumulators of the two types have different shapes)
-        float acc[Q4 ? 1 : MT][Q4 ? 1 : NT][4];
-        unsigned long long acq[Q4 ? MT : 1][Q4 ? NT : 1][2];
+        float acc[Q4 ? 1 : MA][Q4 ? 1 : NT][4];
+        unsigned long long acq[Q4 ? MA : 1][Q4 ? NT : 1][2];
 #pragma unroll
-        for (int m = 0; m < MT; m++)
+        for (int m = 0; m < MA; m++)
 #pragma unroll
             for (int n = 0; n < NT; n++)
 #pragma unroll
@@ -352,56 +357,66 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
 #pragma unroll
                 for (int n = 0; n < NT; n++) mm_ldsm4(b[n], xb + b_off[0] + n * 8 * 64);
 #pragma unroll
-                for (int m = 0; m < MT; m++) {
-                    if (m * 16 >= rt) break;
+                for (int m0 = 0; m0 < MA; m0 += MG) {
+                    if (m0 * 16 >= rt) break;
+                    uint32_t a[MG][2][4];
 #pragma unroll
-                    for (int k = 0; k < 2; k++) {
-                        uint32_t a[4];
-                        mm_ldsm4(a, base + a_off[k] + m * 16 * 64);
+                    for (int m = 0; m < MG; m++)
 #pragma unroll
-                        for (int n = 0; n < NT; n++) mm_hmma(acc[Q4 ? 0 : m][Q4 ? 0 : n], a, b[n][2 * k], b[n][2 * k + 1]);
-                    }
+                        for (int k = 0; k < 2; k++) mm_ldsm4(a[m][k], base + a_off[k] + (m0 + m) * 16 * 64);
+#pragma unroll
+                    for (int k = 0; k < 2; k++)
+#pragma unroll
+                        for (int m = 0; m < MG; m++)
+#pragma unroll
+                            for (int n = 0; n < NT; n++) mm_hmma(acc[Q4 ? 0 : m0 + m][Q4 ? 0 : n], a[m][k], b[n][2 * k], b[n][2 * k + 1]);
                 }
             } else {
                 const uint32_t sb = xb + TP * 128 + g * 8, db = xb + TP * 128 + rt * 8 + 2 * q * 4;
 #pragma unroll
-                for (int k = 0; k < (Q4 ? 4 : 0); k++) {              // block by block
-                    uint32_t b[NT + 1][2];
-                    unsigned long long dd[NT], md[NT];
+                for (int m0 = 0; m0 < (Q4 ? MA : 0); m0 += MG) {
+                    if (m0 * 16 >= rt) break;
+                    uint2 sc[MG][2];                                  // scales of the slice's four blocks, rows g and g + 8
 #pragma unroll
-                    for (int n = 0; n < NT; n += 2) {
-                        uint32_t v[4];
-                        mm_ldsm4(v, xb + b_off[k] + n * 8 * 128 - (n + 1 < NT ? 0u : b_up));      // (an odd last group is read twice)
-                        b[n][0] = v[0]; b[n][1] = v[1]; b[n + 1][0] = v[2]; b[n + 1][1] = v[3];
-                    }
+                    for (int m = 0; m < MG; m++)
 #pragma unroll
-                    for (int n = 0; n < NT; n++) {
-                        asm volatile("ld.shared.b64 %0, [%1];" : "=l"(dd[n]) : "r"(db + (k * TP + n * 8) * 4));
-                        dd[n] = mm_mul2(dd[n], sixteenth);
-                        md[n] = mm_mul2(dd[n], neg_magic);
-                    }
+                        for (int h = 0; h < 2; h++)
+                            asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(sc[m][h].x), "=r"(sc[m][h].y) : "r"(sb + (m0 + m) * 128 + h * 64));
 #pragma unroll
-                    for (int m = 0; m < MT; m += 2) {
-                        if (m * 16 >= rt) break;
-                        uint32_t w[4];
-                        mm_ldsm4(w, base + a_off[k] + m * 16 * 64 - (m * 16 + 16 < rt ? 0u : a_up));      // (so is an odd last fragment)
+                    for (int k = 0; k < 4; k++) {                     // block by block
+                        uint32_t w[MG][2], b[NT + 1][2];
+                        unsigned long long dd[NT], md[NT];
 #pragma unroll
-                        for (int u = 0; u < 2; u++) {
-                            if (m + u >= MT || (m + u) * 16 >= rt) break;
-                            unsigned short h0, h1;
-                            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h0) : "r"(sb + (m + u) * 128 + k * 2));
-                            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h1) : "r"(sb + (m + u) * 128 + 64 + k * 2));
-                            const float e0 = __half2float(__ushort_as_half(h0)), e1 = __half2float(__ushort_as_half(h1));
+                        for (int m = 0; m < MG; m += 2) {
+                            uint32_t v[4];
+                            mm_ldsm4(v, base + a_off[k] + (m0 + m) * 16 * 64);
+                            w[m][0] = v[0]; w[m][1] = v[1]; w[m + 1][0] = v[2]; w[m + 1][1] = v[3];
+                        }
+#pragma unroll
+                        for (int n = 0; n < NT; n += 2) {
+                            uint32_t v[4];
+                            mm_ldsm4(v, xb + b_off[k] + n * 8 * 128 - (n + 1 < NT ? 0u : b_up));      // (an odd last group is read twice)
+                            b[n][0] = v[0]; b[n][1] = v[1]; b[n + 1][0] = v[2]; b[n + 1][1] = v[3];
+                        }
+#pragma unroll
+                        for (int n = 0; n < NT; n++) {
+                            asm volatile("ld.shared.b64 %0, [%1];" : "=l"(dd[n]) : "r"(db + (k * TP + n * 8) * 4));
+                            dd[n] = mm_mul2(dd[n], sixteenth);
+                            md[n] = mm_mul2(dd[n], neg_magic);
+                        }
+#pragma unroll
+                        for (int m = 0; m < MG; m++) {
+                            const float2 f0 = h2f(k < 2 ? sc[m][0].x : sc[m][0].y), f1 = h2f(k < 2 ? sc[m][1].x : sc[m][1].y);
+                            const float e0 = k & 1 ? f0.y : f0.x, e1 = k & 1 ? f1.y : f1.x;
                             const unsigned long long d0 = mm_pack(e0, e0), d1 = mm_pack(e1, e1);
-                            const uint32_t w0 = w[2 * u], w1 = w[2 * u + 1];
-                            const uint32_t a0 = ((w0 << 4) & 0xF0F0F0F0u) ^ 0x80808080u, a1 = ((w1 << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
-                            const uint32_t a2 = (w0 & 0xF0F0F0F0u) ^ 0x80808080u, a3 = (w1 & 0xF0F0F0F0u) ^ 0x80808080u;
+                            const uint32_t a0 = ((w[m][0] << 4) & 0xF0F0F0F0u) ^ 0x80808080u, a1 = ((w[m][1] << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
+                            const uint32_t a2 = (w[m][0] & 0xF0F0F0F0u) ^ 0x80808080u, a3 = (w[m][1] & 0xF0F0F0F0u) ^ 0x80808080u;
 #pragma unroll
                             for (int n = 0; n < NT; n++) {
                                 uint32_t c[4];
                                 mm_imma(c, a0, a1, a2, a3, b[n][0], b[n][1], MAGIC);
-                                mm_scale_add(acq[Q4 ? m + u : 0][Q4 ? n : 0][0], mm_packu(c[0], c[1]), dd[n], md[n], d0);
-                                mm_scale_add(acq[Q4 ? m + u : 0][Q4 ? n : 0][1], mm_packu(c[2], c[3]), dd[n], md[n], d1);
+                                mm_scale_add(acq[Q4 ? m0 + m : 0][Q4 ? n : 0][0], mm_packu(c[0], c[1]), dd[n], md[n], d0);
+                                mm_scale_add(acq[Q4 ? m0 + m : 0][Q4 ? n : 0][1], mm_packu(c[2], c[3]), dd[n], md[n], d1);
                             }
                         }
                     }
@@ -440,43 +455,50 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
         }
         const float * sums = reinterpret_cast<const float *>(smem);
         const int n_tile = GATED ? n_rows / 2 : n_rows;
-        for (int t = warp; t < p.T; t += MM_RINGS) {
-            for (int k0 = 0; k0 < n_tile; k0 += 32) {
-                const int k = k0 + lane;
-                const bool mine_k = k < n_tile;
-                float o = 0.f;
-                if (mine_k) {
-                    if (GATED) {
-                        float u = 0.f, v = 0.f;
+        for (int k0 = 0; k0 < n_tile; k0 += 32) {                     // a lane per item; tokens warp, warp + 8, ... at once
+            const int k = min(k0 + lane, n_tile - 1);
+            const bool mine_k = k0 + lane < n_tile;
+            const int item = lo + first + k;
+            const int r = SPARSE ? rows[first + k] : item;
+            const int64_t gid = SPARSE && p.bucket ? p.bucket[r] : r;
+            const float bias = p.bias ? p.bias[gid] : 0.f;
+            float l[NT], o[NT];
 #pragma unroll
-                        for (int w = 0; w < MM_RINGS; w++) {
-                            const float2 f = *reinterpret_cast<const float2 *>(sums + (size_t)w * (p.ring / 4) + t * pitch + 2 * k);
-                            u += f.x; v += f.y;
-                        }
-                        o = fmaxf(v, 0.f) * u;
-                    } else {
+            for (int u = 0; u < NT; u++) { const int t = warp + u * 8; l[u] = SPARSE && t < p.T ? p.idx[(size_t)t * p.idx_stride + gid] : 0.f; }
 #pragma unroll
-                        for (int w = 0; w < MM_RINGS; w++) o += sums[(size_t)w * (p.ring / 4) + t * pitch + k];
+            for (int u = 0; u < NT; u++) {
+                const int t = warp + u * 8;                           // (sums of tokens past the last are read, and dropped)
+                if (GATED) {
+                    float up = 0.f, gt = 0.f;
+#pragma unroll
+                    for (int w = 0; w < MM_RINGS; w++) {
+                        const float2 f = *reinterpret_cast<const float2 *>(sums + (size_t)w * (p.ring / 4) + t * pitch + 2 * k);
+                        up += f.x; gt += f.y;
                     }
-                    const int item = lo + first + k;
-                    const int r = SPARSE ? rows[first + k] : item;
-                    const int64_t gid = SPARSE && p.bucket ? p.bucket[r] : r;
-                    const bool off = SPARSE && p.idx[(size_t)t * p.idx_stride + gid] < p.threshold;      // (a NaN logit counts as active)
-                    if (off && p.coef) {
-                        p.coef[(size_t)t * p.coef_stride + item] = __ushort_as_half((unsigned short)0);
-                    } else {
-                        if (off) o = 0.f;
-                        if (p.bias) o += p.bias[gid];
-                        if (p.relu) o = fmaxf(o, 0.f);
-                        if (p.dst)   p.dst[(size_t)t * p.dst_stride + gid] = o;
-                        if (p.dst16) p.dst16[(size_t)t * p.dst_stride + gid] = __float2half_rn(o);
-                        if (p.coef)  p.coef[(size_t)t * p.coef_stride + item] = __float2half_rn(o);
-                    }
+                    o[u] = fmaxf(gt, 0.f) * up;
+                } else {
+                    o[u] = 0.f;
+#pragma unroll
+                    for (int w = 0; w < MM_RINGS; w++) o[u] += sums[(size_t)w * (p.ring / 4) + t * pitch + k];
                 }
-                if (!SPARSE && p.masks_out) {                         // the union over the tokens of !(result < threshold), one bit per row
-                    const unsigned m = __ballot_sync(0xffffffffu, mine_k && !(o < p.masks_threshold));
-                    if (lane == 0 && m) atomicOr(&s_any[k0 / 32], m);
-                }
+            }
+            bool any = false;
+#pragma unroll
+            for (int u = 0; u < NT; u++) {
+                const int t = warp + u * 8;
+                if (!mine_k || t >= p.T) continue;
+                const bool off = SPARSE && l[u] < p.threshold;        // (a NaN logit counts as active)
+                float v = off ? 0.f : o[u];
+                if (p.bias) v += bias;
+                if (p.relu) v = fmaxf(v, 0.f);
+                if (p.dst)   p.dst[(size_t)t * p.dst_stride + gid] = v;
+                if (p.dst16) p.dst16[(size_t)t * p.dst_stride + gid] = __float2half_rn(v);
+                if (p.coef)  p.coef[(size_t)t * p.coef_stride + item] = __float2half_rn(off ? 0.f : v);
+                any |= !(v < p.masks_threshold);
+            }
+            if (!SPARSE && p.masks_out) {                             // the union over the tokens of !(result < threshold), one bit per row
+                const unsigned m = __ballot_sync(0xffffffffu, any);
+                if (lane == 0 && m) atomicOr(&s_any[k0 / 32], m);
             }
         }
         if (!SPARSE && p.masks_out) {
@@ -501,7 +523,7 @@ static int mm_go(MmP p, bool pdl, cudaStream_t st) {
     const int G = (int)imin64(sm_count(), (p.nrows + 7) / 8);
     const int list = SPARSE ? ((p.nrows + G - 1) / G + 1) * 4 : 0;    // bytes
     if (list > 8192 - 128) return PI_ERR_UNSUPPORTED;                 // (more than MM_MAX_ROWS rows)
-    p.ring = (MM_SMEM_MAX - list) / MM_RINGS / 128 * 128;
+    p.ring = (MM_SMEM_MAX - list - MM_SLACK) / MM_RINGS / 128 * 128;
     static bool attr_done[16] = {false};
     int dev = 0;
     PI_CUDA(cudaGetDevice(&dev));
@@ -510,7 +532,7 @@ static int mm_go(MmP p, bool pdl, cudaStream_t st) {
         PI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MM_SMEM_MAX));
         attr_done[dev] = true;
     }
-    PI_CUDA(launch_k(kern, dim3(G), dim3(MM_THREADS), (size_t)p.ring * MM_RINGS + list, st, pdl, p));
+    PI_CUDA(launch_k(kern, dim3(G), dim3(MM_THREADS), (size_t)p.ring * MM_RINGS + list + MM_SLACK, st, pdl, p));
     return PI_OK;
 }
 
