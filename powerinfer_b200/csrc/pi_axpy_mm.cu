@@ -18,20 +18,25 @@
 // 32 tokens; the groups of a column range follow one another, so that they find its rows in L2); every CTA takes an equal contiguous
 // range, so the chip is full whatever the number of columns.  The CTAs that meet in a slice each write one partial vector
 // ("piece"); at most n_pieces of them per slice, the missing ones are written as zeros, and the norm (or the reduction)
-// that follows adds the pieces in order.  Rows arrive by 16-byte cp.async from all threads (they lie anywhere).
+// that follows adds the pieces in order.  Rows arrive by 16-byte cp.async (they lie anywhere) from 8 producer warps; 8 consumer warps
+// share a stage, 4 along the columns and 2 along the rows, and meet at the end of a slice only.  (When all 16 warps did both, a stage
+// took 5500 clocks, of which its bytes need 1400: divisions for the unit's place, copies that wait while the queue of outstanding
+// loads is full, a barrier.)  Every wait is bounded: when one runs out bit 4 of *status is set (where given) and the rest of the work
+// is passed over.
 #include "pi_common.cuh"
 
 namespace pi {
 
-static constexpr int AX_THREADS = 512, AX_CW = 256;      // 16 warps; columns of a unit
+static constexpr int AX_THREADS = 512, AX_CONS = 8, AX_PROD = 256, AX_CW = 256;      // warps 0 .. 7 consume, threads 256 .. 511 produce; columns of a unit
+static constexpr int AX_SMAX = 8;                        // stages at most
 static constexpr int AX_RED_PITCH = AX_CW + 4;           // conflict-free fragment stores
 static constexpr size_t AX_SMEM_MAX = 226 * 1024;
-static constexpr int AX_ROW_RING = 16;                   // stages whose row numbers are kept
 
 struct AxpyMmP {
     const uint8_t * Wt; int64_t row_bytes; int nrows, ncols, nb, T;
     const int32_t * list; const int32_t * count;
     const void * coef; int64_t coef_stride;                           // FP16, or F32 in the exact mode
+    unsigned int * status;
     float * partial; int n_cs, n_tg, n_pieces;                        // column ranges, token groups, partial vectors per slice
 };
 
@@ -83,11 +88,11 @@ struct AxShape {
     static constexpr int C_OFF = RS * W_PITCH;
     static constexpr int STAGE = (C_OFF + TP * C_PITCH + 127) / 128 * 128;
     static constexpr int RED = TP * AX_RED_PITCH * 4;
-    static constexpr int HEAD = (RED + AX_ROW_RING * RS * 4 + 127) / 128 * 128;
+    static constexpr int HEAD = (RED + 127) / 128 * 128;
     static constexpr int FIT = (int)((AX_SMEM_MAX - HEAD) / STAGE);
-    static constexpr int S = FIT > 8 ? 8 : FIT;
-    static constexpr int KPW = RS / 64;                               // 16-row steps of a warp per stage (4 warps share the rows)
-    static_assert(S >= 3 && S + 2 <= AX_ROW_RING, "ring");
+    static constexpr int S = FIT > AX_SMAX ? AX_SMAX : FIT;
+    static constexpr int KPW = RS / 32;                               // 16-row steps of a warp per stage (2 warps share the rows)
+    static_assert(S >= 3, "ring");
 };
 
 template <int MODE, int NT>
@@ -97,12 +102,24 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
     constexpr int TP = Z::TP, RS = Z::RS, S = Z::S, KPW = Z::KPW;
     extern __shared__ __align__(128) unsigned char smem[];
     float * red = reinterpret_cast<float *>(smem);                    // [TP][AX_RED_PITCH]
-    int * rows = reinterpret_cast<int *>(smem + Z::RED);              // [AX_ROW_RING][RS] row numbers of the stages ahead
+    __shared__ uint64_t s_full[AX_SMAX], s_empty[AX_SMAX];
+    __shared__ volatile int s_dead;
     const uint32_t ring_a = smem_u32(smem + Z::HEAD);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wc = warp & 3, wk = warp >> 2;                          // 64 columns, a quarter of the stage's rows
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);    // (uniform for the compiler)
+    const int wc = warp & 3, wk = (warp >> 2) & 1;                    // consumers: 64 columns, a half of the stage's rows
     const int cta = blockIdx.x;
 
+    if (tid < AX_SMAX) { mbar_init(s_full + tid, AX_PROD); mbar_init(s_empty + tid, AX_CONS); }
+    if (tid == 0) s_dead = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    __syncthreads();
+    auto wait = [&](uint64_t * bar, unsigned parity) -> bool {        // warp-uniform; false: the wait ran out, here or elsewhere
+        bool ok = false;
+        for (int spins = 0; spins < (1 << 20) && !ok && !s_dead; spins++) ok = mbar_try_wait(bar, parity);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok && lane == 0) { s_dead = 1; if (p.status) atomicOr(p.status, 16u); }
+        return ok;
+    };
     pdl_launch();
     pdl_wait();
     const int n = min(*p.count, p.nrows);
@@ -121,43 +138,64 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
     if ((unsigned)cta >= G) return;
     const int u0 = (int)((unsigned long long)total * (unsigned)cta / G), n_units = (int)((unsigned long long)total * (unsigned)(cta + 1) / G) - u0;
 
-    auto row_at = [&](int u, int r) {                                 // row number of list entry r of unit u's stage
-        const int li = (u % nst) * RS + r;
-        const int v = u < u0 + n_units && li < n ? p.list[li] : 0;
-        return (unsigned)v < (unsigned)p.nrows ? v : 0;
+    // place of the current unit: stage of the slice, slice, its column range and token group
+    int st = u0 % nst, sl = u0 / nst, cs = sl / p.n_tg, tg = sl % p.n_tg;
+    auto advance = [&]() {
+        if (++st < nst) return;
+        st = 0; sl++;
+        if (++tg == p.n_tg) { tg = 0; cs++; }
     };
-    for (int e = tid; e < (S + 1) * RS; e += AX_THREADS) rows[e] = row_at(u0 + e / RS, e % RS);
-    __syncthreads();
-    auto issue = [&](int i) {                                         // unit u0 + i
-        const int u = u0 + i, sl = u / nst, st = u % nst, cs = sl / p.n_tg, tok0 = sl % p.n_tg * 32, Tg = min(32, p.T - tok0);
-        const uint32_t base = ring_a + (uint32_t)(i % S) * Z::STAGE;
-        const int * rw = rows + (i % AX_ROW_RING) * RS;
-        if (!Q4) {
-            const int col = cs * AX_CW + lane * 8;
-#pragma unroll
-            for (int j = 0; j < RS / 16; j++) {
-                const int r = warp + j * 16;
-                const bool ok = st * RS + r < n && col < p.ncols;
-                ax_cp16(base + r * Z::W_PITCH + lane * 16, ok ? p.Wt + (size_t)rw[r] * p.row_bytes + (size_t)col * 2 : p.Wt, ok ? 16u : 0u);
-            }
-        } else {
-            constexpr int CT = 8 * RS / AX_THREADS;                   // pieces of a row slice per thread
-            const int r = tid / (8 / CT), qd = tid % (8 / CT);
-            const bool ok = st * RS + r < n;
-            const uint8_t * row = p.Wt + (size_t)rw[r] * p.row_bytes;
-#pragma unroll
-            for (int j = 0; j < CT; j++) ax_cp16(base + r * Z::W_PITCH + (qd * CT + j) * 16, row + (size_t)cs * 128 + (qd * CT + j) * 16, ok ? 16u : 0u);
-            if (qd == 0) ax_cp16(base + r * Z::W_PITCH + 128, row + (size_t)p.nb * 16 + (size_t)cs * 16, ok ? 16u : 0u);
-        }
-        constexpr int CPP = 16 / Z::CB;                               // coefficients of a 16-byte piece; positions past the list count as 0
-        for (int e = tid; e < TP * (RS / CPP); e += AX_THREADS) {
-            const int t = e / (RS / CPP), c = e % (RS / CPP), li = st * RS + c * CPP;
-            const int bytes = t < Tg ? max(0, min(CPP, n - li)) * Z::CB : 0;
-            ax_cp16(base + Z::C_OFF + t * Z::C_PITCH + c * 16, (const char *)p.coef + (bytes ? ((size_t)(tok0 + t) * p.coef_stride + li) * Z::CB : 0), (unsigned)bytes);
-        }
-    };
-    for (int s = 0; s < S - 1; s++) { if (s < n_units) issue(s); asm volatile("cp.async.commit_group;" ::: "memory"); }
 
+    if (warp >= AX_CONS) {
+        // ================================================================= producers: a row of the stage per TR threads
+        const int pt = tid - AX_CONS * 32;
+        constexpr int TR = AX_PROD / RS, PW = (Q4 ? 8 : 32) / TR;      // 16-byte pieces of a row slice per thread
+        const int r = pt / TR, c0 = pt % TR;
+        constexpr int CPP = 16 / Z::CB, CPR = RS / CPP;               // coefficients of a 16-byte piece; pieces of a token
+        constexpr int NC = (TP * CPR + AX_PROD - 1) / AX_PROD;
+        auto row_at = [&](int s) {                                    // row number of my list entry in stage s of the slice
+            const int v = s * RS + r < n ? p.list[s * RS + r] : 0;
+            return (unsigned)v < (unsigned)p.nrows ? v : 0;
+        };
+        int slot = 0, row = row_at(st);
+        unsigned phase = 1u;                                          // parity of the hand-back to wait for (first round: none)
+        for (int i = 0; i < n_units; i++) {
+            const int next_row = row_at(st + 1 < nst ? st + 1 : 0);   // (one unit ahead: its latency passes while this unit is copied)
+            if (!wait(s_empty + slot, phase)) break;
+            const uint32_t base = ring_a + (uint32_t)(slot * Z::STAGE);
+            const bool live = st * RS + r < n;
+            const uint8_t * src = p.Wt + (size_t)row * p.row_bytes;
+            if (!Q4) {
+                const int col = cs * AX_CW + c0 * 8;
+                const uint8_t * at = src + (size_t)col * 2;
+#pragma unroll
+                for (int j = 0; j < PW; j++) {                        // (rows past the list: coefficients 0, but what they meet must be finite)
+                    const bool ok = live && col + j * TR * 8 < p.ncols;
+                    ax_cp16(base + r * Z::W_PITCH + (c0 + j * TR) * 16, ok ? at + j * TR * 16 : p.Wt, ok ? 16u : 0u);
+                }
+            } else {
+                const uint8_t * at = src + (size_t)cs * 128 + c0 * 16;
+#pragma unroll
+                for (int j = 0; j < PW; j++) ax_cp16(base + r * Z::W_PITCH + (c0 + j * TR) * 16, at + j * TR * 16, live ? 16u : 0u);
+                if (c0 == 0) ax_cp16(base + r * Z::W_PITCH + 128, src + (size_t)p.nb * 16 + (size_t)cs * 16, live ? 16u : 0u);
+            }
+            const int tok0 = tg * 32, Tg = min(32, p.T - tok0);
+#pragma unroll
+            for (int j = 0; j < NC; j++) {                            // coefficients; positions past the list count as 0
+                const int e = pt + j * AX_PROD, t = e / CPR, c = e % CPR, li = st * RS + c * CPP;
+                if (t >= TP) break;
+                const int bytes = t < Tg ? max(0, min(CPP, n - li)) * Z::CB : 0;
+                ax_cp16(base + Z::C_OFF + t * Z::C_PITCH + c * 16, (const char *)p.coef + (bytes ? ((size_t)(tok0 + t) * p.coef_stride + li) * Z::CB : 0), (unsigned)bytes);
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" :: "r"(smem_u32(s_full + slot)) : "memory");
+            row = next_row;
+            advance();
+            if (++slot == S) { slot = 0; phase ^= 1u; }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        return;
+    }
+    // ===================================================================== consumers
     float acc[4][NT][4];
     auto clear = [&]() {
 #pragma unroll
@@ -175,16 +213,13 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
     const uint32_t s_off = (uint32_t)((wk * KPW * 16 + 2 * q) * Z::W_PITCH + 128 + (wc * 2 + (g >> 2)) * 2);
     const uint32_t b_off = (uint32_t)(Z::C_OFF + ((lane & 7) + (NT > 1 ? ((lane >> 4) & 1) * 8 : 0)) * Z::C_PITCH + (wk * KPW * 16 + ((lane >> 3) & 1) * 8) * 2);
 
-    int next_row = 0;
+    int slot = 0;
+    unsigned phase = 0u;
+    bool ok = true;                                                   // (when a wait ran out the barriers below are still met)
     for (int i = 0; i < n_units; i++) {
-        asm volatile("cp.async.wait_group %0;" :: "n"(S - 2) : "memory");
-        // row numbers travel two units ahead of their use: read now, stored in the next round, used in the one after
-        if (i > 0 && tid < RS) rows[((i + S) % AX_ROW_RING) * RS + tid] = next_row;
-        __syncthreads();                                              // stage i has landed for everybody; stage i - 1 is consumed
-        if (i + S - 1 < n_units) issue(i + S - 1);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        if (tid < RS) next_row = row_at(u0 + i + S + 1, tid);
-        const uint32_t base = ring_a + (uint32_t)(i % S) * Z::STAGE;
+        ok = ok && wait(s_full + slot, phase);
+        const uint32_t base = ring_a + (uint32_t)(slot * Z::STAGE);
+        if (ok)
 #pragma unroll
         for (int k = 0; k < KPW; k++) {
             if (EXACT) {
@@ -196,7 +231,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
                     float d[4];
 #pragma unroll
                     for (int h = 0; h < 4; h++) {
-                        const uint32_t at = base + (uint32_t)((wk * 16 + 2 * q + (h >> 1) * 8 + (h & 1)) * Z::W_PITCH);
+                        const uint32_t at = base + (uint32_t)(((wk * KPW + k) * 16 + 2 * q + (h >> 1) * 8 + (h & 1)) * Z::W_PITCH);
                         unsigned short x;
                         asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[h]) : "r"(at + (wc * 2 + bl) * 16 + (g >> 1) * 4));
                         asm volatile("ld.shared.u16 %0, [%1];" : "=h"(x) : "r"(at + 128 + (wc * 2 + bl) * 2));
@@ -214,7 +249,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
                     }
 #pragma unroll
                     for (int t = 0; t < NT; t++) {
-                        const uint32_t at = base + (uint32_t)(Z::C_OFF + (t * 8 + g) * Z::C_PITCH + (wk * 16 + 2 * q) * 4);
+                        const uint32_t at = base + (uint32_t)(Z::C_OFF + (t * 8 + g) * Z::C_PITCH + ((wk * KPW + k) * 16 + 2 * q) * 4);
                         float c[4];
                         asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(c[0]), "=f"(c[1]) : "r"(at));
                         asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(c[2]), "=f"(c[3]) : "r"(at + 32));
@@ -273,12 +308,14 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
                 }
             }
         }
-        const int u = u0 + i;
-        if (u % nst == nst - 1 || i == n_units - 1) {
-            const int sl = u / nst, cs = sl / p.n_tg, tok0 = sl % p.n_tg * 32, Tg = min(32, p.T - tok0);
-            // ---- end of this CTA's share of the slice: the four row quarters are added in order
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_empty + slot);                   // handed back
+        if (++slot == S) { slot = 0; phase ^= 1u; }
+        if (st == nst - 1 || i == n_units - 1) {
+            // ---- end of this CTA's share of the slice: the row halves are added in order
+            const int tok0 = tg * 32, Tg = min(32, p.T - tok0);
 #pragma unroll 1
-            for (int r = 0; r < 4; r++) {
+            for (int r = 0; r < 2; r++) {
                 if (wk == r) {
 #pragma unroll
                     for (int m = 0; m < 4; m++)
@@ -294,11 +331,11 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
                                 *o = r == 0 ? acc[m][t][j] : *o + acc[m][t][j];
                             }
                 }
-                __syncthreads();
+                asm volatile("bar.sync 1, 256;" ::: "memory");
             }
             const int c_lo = (int)((((unsigned long long)sl * nst + 1u) * G - 1u) / total), c_hi = (int)(((unsigned long long)(sl + 1) * nst * G - 1u) / total);
             const int piece = cta - c_lo, more = cta == c_hi ? p.n_pieces - 1 - piece : 0;      // the slice's last CTA also writes the missing pieces
-            for (int e = tid; e < Tg * AX_CW; e += AX_THREADS) {
+            for (int e = tid; e < Tg * AX_CW; e += AX_CONS * 32) {
                 const int c = e % AX_CW, t = e / AX_CW, col = cs * AX_CW + c;
                 if (col >= p.ncols) continue;
                 float * o = p.partial + ((size_t)piece * p.T + tok0 + t) * p.ncols + col;
@@ -306,7 +343,9 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
                 for (int k = 1; k <= more; k++) o[(size_t)k * p.T * p.ncols] = 0.f;
             }
             clear();
+            asm volatile("bar.sync 1, 256;" ::: "memory");             // the sums are read
         }
+        advance();
     }
 }
 
@@ -443,7 +482,7 @@ int launch_axpy_mm(const AxpyArgs & a, cudaStream_t st, int * pieces_used) {
     axpy_mm_shape(a.ncols, a.T, &p.n_cs, &p.n_tg, &grid, &p.n_pieces);
     if (p.n_pieces > a.n_groups) return PI_ERR_UNSUPPORTED;
     p.Wt = (const uint8_t *)a.Wt; p.row_bytes = (int64_t)pi_row_bytes(a.wtype, a.ncols); p.nrows = (int)a.nrows; p.ncols = (int)a.ncols;
-    p.nb = (int)(a.ncols / 32); p.T = a.T; p.list = a.list; p.count = a.count; p.coef = a.coef; p.coef_stride = a.coef_stride; p.partial = a.partial;
+    p.nb = (int)(a.ncols / 32); p.T = a.T; p.list = a.list; p.count = a.count; p.coef = a.coef; p.coef_stride = a.coef_stride; p.partial = a.partial; p.status = a.status;
     if (pieces_used) *pieces_used = p.n_pieces;
     return exact ? axpy_mm_tokens<AX_Q4_EXACT>(p, grid, a.pdl, st) : q4 ? axpy_mm_tokens<AX_Q4>(p, grid, a.pdl, st) : axpy_mm_tokens<AX_F16>(p, grid, a.pdl, st);
 }
