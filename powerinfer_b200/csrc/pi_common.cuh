@@ -111,6 +111,7 @@ struct GemvArgs {
     float * dst = nullptr;             // F32 [T, dst_stride]; destination row = global id (sparse) or row (dense)
     int64_t dst_stride = 0;
     __half * dst16 = nullptr;          // optional FP16 copy of the result [T, dst_stride] (feeds an F16 mat-vec)
+    float * const * dst_host = nullptr;  // dense, 2..32 tokens: device word that points to host memory for another copy of dst, or is null
     // second matrix sharing the row selection (gate with up): dst = relu(W2 row . x) * (W row . x)
     const void * W2 = nullptr;
     // activity bit masks (one word per 32 LOCAL rows) instead of a list; selects the register-streaming kernel (one token) or the

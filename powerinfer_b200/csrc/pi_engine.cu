@@ -46,7 +46,8 @@ __global__ void k_embed(const __half * __restrict__ tok_embd, const __half * __r
 static constexpr int ARG_THREADS = 256, ARG_UN = 8, ARG_PIECE = ARG_THREADS * ARG_UN;
 
 __global__ void __launch_bounds__(ARG_THREADS) k_argmax(const float * __restrict__ logits, int n, unsigned long long * __restrict__ best,
-                                                        unsigned int * __restrict__ ticket, int32_t * __restrict__ out, int32_t ** __restrict__ sink) {
+                                                        unsigned int * __restrict__ ticket, int32_t * __restrict__ out, int32_t ** __restrict__ sink,
+                                                        float ** __restrict__ logits_sink, int copy) {
     __shared__ unsigned long long s_k[ARG_THREADS / 32];
     const int t = blockIdx.y, lane = threadIdx.x & 31;
     const float * row = logits + (size_t)t * n;
@@ -56,6 +57,16 @@ __global__ void __launch_bounds__(ARG_THREADS) k_argmax(const float * __restrict
     for (int u = 0; u < ARG_UN; u++) {
         const int i = blockIdx.x * ARG_PIECE + u * ARG_THREADS + threadIdx.x;
         v[u] = i < n ? row[i] : -INFINITY;
+    }
+    if (copy) {                                                       // the logits pass here anyway: a copy of their own costs 6 us more
+        float * host = logits_sink[t];
+        if (host) {
+#pragma unroll
+            for (int u = 0; u < ARG_UN; u++) {
+                const int i = blockIdx.x * ARG_PIECE + u * ARG_THREADS + threadIdx.x;
+                if (i < n) host[i] = v[u];
+            }
+        }
     }
     unsigned long long key = 0ull;                                    // (a NaN or -inf is never chosen: index 0 if there is nothing else)
 #pragma unroll
@@ -82,6 +93,7 @@ __global__ void __launch_bounds__(ARG_THREADS) k_argmax(const float * __restrict
     out[t] = i;
     int32_t * host = sink[t];                                         // (for this step only)
     if (host) { *host = i; sink[t] = nullptr; }
+    logits_sink[t] = nullptr;                                         // (every CTA of the row has read it)
 }
 
 // Tokens of a prompt that go through the layers together, whatever the engine's batch: a chunk reads the weights once, and 77 tokens of
@@ -89,9 +101,9 @@ __global__ void __launch_bounds__(ARG_THREADS) k_argmax(const float * __restrict
 static constexpr int PROMPT_CHUNK = 256;
 
 // A step's token ids and positions travel as kernel arguments: one launch instead of two copies, and the caller's arrays are free again
-// as soon as it returns.  `sink`: where the greedy ids go besides the engine's own buffer (mapped host memory, or nowhere): a few bytes
-// written by the kernel that finds them, where a copy of their own is 6 us behind the logits'.
-struct Feed { int32_t token[PI_MAX_BATCH], pos[PI_MAX_BATCH]; int32_t * sink; };
+// as soon as it returns.  `sink`, `logits`: where the greedy ids and the logits go besides the engine's own buffers (mapped host memory,
+// or nowhere): written by the kernels that make them, where copies of their own start 6 us after the last kernel.
+struct Feed { int32_t token[PI_MAX_BATCH], pos[PI_MAX_BATCH]; int32_t * sink; float * logits; int n_vocab; };
 
 // a prompt chunk: consecutive positions of one sequence
 struct FeedPrompt { int32_t token[PROMPT_CHUNK]; };
@@ -105,10 +117,11 @@ __global__ void __launch_bounds__(PROMPT_CHUNK) k_feed_prompt(const FeedPrompt f
     seq_pf[t] = seq;
 }
 
-__global__ void k_feed(const Feed f, int T, int32_t * __restrict__ tokens, int32_t * __restrict__ pos, int32_t ** __restrict__ sink) {
+__global__ void k_feed(const Feed f, int T, int32_t * __restrict__ tokens, int32_t * __restrict__ pos, int32_t ** __restrict__ sink, float ** __restrict__ logits_sink) {
     const int t = threadIdx.x;
     if (t >= T) return;
     sink[t] = f.sink ? f.sink + t : nullptr;
+    logits_sink[t] = f.logits ? f.logits + (size_t)t * f.n_vocab : nullptr;
     tokens[t] = f.token[t];
     pos[t] = f.pos[t];
 }
@@ -166,7 +179,7 @@ struct pi_engine {
     ActBuf act_a, act_q, act_p, act_o;       // FFN input, QKV input, predictor input (FP16), out-proj input
     __half * k_cache, * v_cache;             // [n_layer, max_batch, n_ctx, dkv]
     unsigned long long * amax_best; unsigned int * amax_ticket;   // k_argmax: a word per row, 0 between steps
-    int32_t ** sink;                         // per row: where the step's greedy id goes as well (null for steps fed on the device)
+    int32_t ** sink; float ** logits_sink;   // per row: where the step's greedy id and logits go as well (null for steps fed on the device)
     unsigned int * status;                   // device word: bit 0 = an exchange wait ran out
     unsigned long long * active_total;       // device counter: sum of active-list lengths over layers and steps
     pi_exchange xch;
@@ -211,7 +224,7 @@ static void carve(pi_engine * e, void * ws, size_t ws_bytes, bool dry, size_t * 
     const int T = e->P_max, B = e->T_max;                            // tokens of the largest step, of the largest decode step
     const size_t d = c.d, F = e->F;
     e->tokens = cv.take<int32_t>(T); e->pos = cv.take<int32_t>(T); e->seq_ids = cv.take<int32_t>(B); e->seq_pf = cv.take<int32_t>(T); e->argmax = cv.take<int32_t>(B);
-    e->amax_best = cv.take<unsigned long long>(B); e->amax_ticket = cv.take<unsigned int>(B); e->sink = cv.take<int32_t *>(B);
+    e->amax_best = cv.take<unsigned long long>(B); e->amax_ticket = cv.take<unsigned int>(B); e->sink = cv.take<int32_t *>(B); e->logits_sink = cv.take<float *>(B);
     e->status = cv.take<unsigned int>(1); e->active_total = cv.take<unsigned long long>(1);
     e->x = cv.take<float>(T * d); e->x2 = cv.take<float>(T * d); e->attn_out = cv.take<float>(T * d); e->ffn_vec = cv.take<float>(T * d);
     e->qkv = cv.take<float>((size_t)T * (e->dq + 2 * e->dkv));
@@ -323,6 +336,7 @@ int pi_engine_create(const pi_engine_config * cfg, const pi_model_weights * gw, 
     if (ce == cudaSuccess) ce = cudaMemsetAsync(e->amax_best, 0, (size_t)e->T_max * 8, st);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(e->amax_ticket, 0, (size_t)e->T_max * 4, st);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(e->sink, 0, (size_t)e->T_max * sizeof *e->sink, st);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(e->logits_sink, 0, (size_t)e->T_max * sizeof *e->logits_sink, st);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(e->count, 0, 4, st);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(e->status, 0, 4, st);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(e->active_total, 0, 8, st);
@@ -491,11 +505,12 @@ int enqueue_step(pi_engine * e, int T, cudaStream_t st, StageTimer & tm, int mod
             g.status = e->status; g.pdl = pdl;
             g.wtype = out_t; g.W = e->g.output ? e->g.output : e->g.tok_embd; g.nrows = c.n_vocab; g.ncols = d;
             g.x = n1.act.view(); g.T = HT; g.dst = e->logits; g.dst_stride = c.n_vocab;
+            if (HT > 1) g.dst_host = e->logits_sink;                  // (one row leaves a mat-vec value by value: k_argmax copies it)
             STAGE(PI_STAGE_LM_HEAD, 1, launch_gemv(g, st));
             if (!(e->skip_mask & (1u << PI_STAGE_OTHER))) {
                 if (tm.begin()) return PI_ERR_CUDA;
                 PI_CUDA(launch_k(k_argmax, dim3((c.n_vocab + ARG_PIECE - 1) / ARG_PIECE, HT), dim3(ARG_THREADS), 0, st, pdl, e->logits,
-                                 c.n_vocab, e->amax_best, e->amax_ticket, e->argmax, e->sink));
+                                 c.n_vocab, e->amax_best, e->amax_ticket, e->argmax, e->sink, e->logits_sink, HT > 1 ? 0 : 1));
                 if (tm.end(PI_STAGE_OTHER)) return PI_ERR_CUDA;
                 e->launches++;
             }
@@ -688,10 +703,10 @@ int count_kernel_nodes(cudaGraph_t graph) {
 }
 
 // the device's address of pinned host memory, null for other memory
-int32_t * mapped(int32_t * host) {
+void * mapped(void * host) {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, host) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-    return a.type == cudaMemoryTypeHost ? (int32_t *)a.devicePointer : nullptr;
+    return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
 }
 
 // first call for a batch size: one plain run (fills every per-kernel attribute cache), then capture
@@ -749,12 +764,18 @@ int pi_engine_decode_host(pi_engine * e, const int32_t * host_tokens, const int3
     Feed f;
     memcpy(f.token, host_tokens, (size_t)T * 4);
     memcpy(f.pos, host_pos, (size_t)T * 4);
-    f.sink = host_argmax ? mapped(host_argmax) : nullptr;
-    k_feed<<<1, PI_MAX_BATCH, 0, st>>>(f, T, e->tokens, e->pos, e->sink);
+    f.sink = host_argmax ? (int32_t *)mapped(host_argmax) : nullptr;
+    f.logits = host_logits ? (float *)mapped(host_logits) : nullptr;
+    f.n_vocab = e->c.n_vocab;
+    k_feed<<<1, PI_MAX_BATCH, 0, st>>>(f, T, e->tokens, e->pos, e->sink, e->logits_sink);
     PI_LAUNCH_CHECK("k_feed");
-    if ((rc = run_step(e, T, st))) { cudaMemsetAsync(e->sink, 0, (size_t)T * sizeof *e->sink, st); return rc; }
+    if ((rc = run_step(e, T, st))) {
+        cudaMemsetAsync(e->sink, 0, (size_t)T * sizeof *e->sink, st);
+        cudaMemsetAsync(e->logits_sink, 0, (size_t)T * sizeof *e->logits_sink, st);
+        return rc;
+    }
     if (host_argmax && !f.sink) PI_CUDA(cudaMemcpyAsync(host_argmax, e->argmax, (size_t)T * 4, cudaMemcpyDeviceToHost, st));
-    if (host_logits) PI_CUDA(cudaMemcpyAsync(host_logits, e->logits, (size_t)T * e->c.n_vocab * 4, cudaMemcpyDeviceToHost, st));
+    if (host_logits && !f.logits) PI_CUDA(cudaMemcpyAsync(host_logits, e->logits, (size_t)T * e->c.n_vocab * 4, cudaMemcpyDeviceToHost, st));
     PI_CUDA(cudaStreamSynchronize(st));
     return PI_OK;
 }

@@ -48,7 +48,7 @@ struct MmP {
     const uint32_t * masks; const int32_t * bucket; int32_t * list; int32_t * count; unsigned long long * rows_total;
     const float * idx; int64_t idx_stride; float threshold;
     const float * bias; int relu;
-    float * dst; __half * dst16; int64_t dst_stride;
+    float * dst; __half * dst16; int64_t dst_stride; float * const * dst_host;
     __half * coef; int64_t coef_stride;
     uint32_t * masks_out; float masks_threshold; int masks_or;
     unsigned int * status;
@@ -455,6 +455,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
         }
         const float * sums = reinterpret_cast<const float *>(smem);
         const int n_tile = GATED ? n_rows / 2 : n_rows;
+        float * const host = !SPARSE && p.dst_host ? *p.dst_host : nullptr;
         for (int k0 = 0; k0 < n_tile; k0 += 32) {                     // a lane per item; tokens warp, warp + 8, ... at once
             const int k = min(k0 + lane, n_tile - 1);
             const bool mine_k = k0 + lane < n_tile;
@@ -492,6 +493,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
                 if (p.bias) v += bias;
                 if (p.relu) v = fmaxf(v, 0.f);
                 if (p.dst)   p.dst[(size_t)t * p.dst_stride + gid] = v;
+                if (host)    host[(size_t)t * p.dst_stride + gid] = v;
                 if (p.dst16) p.dst16[(size_t)t * p.dst_stride + gid] = __float2half_rn(v);
                 if (p.coef)  p.coef[(size_t)t * p.coef_stride + item] = __float2half_rn(off ? 0.f : v);
                 any |= !(v < p.masks_threshold);
@@ -572,7 +574,7 @@ int launch_mm(const GemvArgs & a, cudaStream_t st) {
         p.idx = a.idx ? a.idx + (size_t)t0 * a.idx_stride : nullptr; p.idx_stride = a.idx_stride; p.threshold = a.threshold;
         p.bias = a.bias; p.relu = a.relu;
         p.dst = a.dst ? a.dst + (size_t)t0 * a.dst_stride : nullptr;
-        p.dst16 = a.dst16 ? a.dst16 + (size_t)t0 * a.dst_stride : nullptr; p.dst_stride = a.dst_stride;
+        p.dst16 = a.dst16 ? a.dst16 + (size_t)t0 * a.dst_stride : nullptr; p.dst_stride = a.dst_stride; p.dst_host = a.dst_host;
         p.coef = a.coef ? a.coef + (size_t)t0 * a.coef_stride : nullptr; p.coef_stride = a.coef_stride;
         p.masks_out = a.masks_out; p.masks_threshold = a.masks_threshold; p.masks_or = t0 > 0;
         p.status = a.status; p.n_slices = 0; p.ring = 0;
