@@ -12,9 +12,13 @@
 // no partial sums, so the accumulators of a tile exist once and the tile can be 96 x 256.  Up to 128 tokens 6 x 2 consumers of 16 rows,
 // beyond that 3 x 4 consumers of 32 rows; the token count of a consumer is a template argument in steps of 8 or 16, because a branch
 // around every pair of products costs more than the products that it leaves out.
+// Copies: the activations and dense rows come as TMA tiles (one instruction of one thread; with 16-byte cp.async the producers' own
+// instruction rate, 50 clocks per warp and copy, bound every launch of few rows), gathered rows and the Q4_0 rows' scales by cp.async.
 // The accumulators go straight to global memory: the ring runs on across tiles.
 // Every wait is bounded, as in pi_mm.cu.
 #include "pi_common.cuh"
+
+#include <cuda.h>
 
 namespace pi {
 
@@ -25,7 +29,9 @@ static constexpr int MW_SMEM_MAX = 224 * 1024;          // (leaves room for the 
 static constexpr int MW_SMAX = 6;                       // stages at most
 static constexpr int MW_TOKENS = 256;                   // of a launch
 
-struct MwP {
+struct alignas(64) MwP {
+    CUtensorMap m_w, m_x, m_x2, m_d;                    // dense rows; activation (Q4_0: its low and high planes, its scales)
+    int per_tile;                                       // dense: rows of a tile
     const uint8_t * W; const uint8_t * W2; int64_t row_bytes; int nrows, ncols, nb;
     Act x; int T;
     const uint32_t * masks; const int32_t * bucket; int32_t * list; int32_t * count; unsigned long long * rows_total;
@@ -40,7 +46,11 @@ struct MwP {
 
 __device__ __forceinline__ void mw_cp16(uint32_t dst, const void * src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory"); }
 __device__ __forceinline__ void mw_cp8(uint32_t dst, const void * src)  { asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" :: "r"(dst), "l"(src) : "memory"); }
-__device__ __forceinline__ void mw_cp4(uint32_t dst, const void * src)  { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(dst), "l"(src) : "memory"); }
+// the tile of `map` at columns x.., rows y.. (x times the element size a multiple of 16 bytes)
+__device__ __forceinline__ void mw_tma(void * dst, const CUtensorMap * map, int x, int y, uint64_t * bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 :: "r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ void mw_zero16(uint32_t dst) { asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" :: "r"(dst), "r"(0u) : "memory"); }
 __device__ __forceinline__ void mw_arrive_copies(uint64_t * bar) { asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" :: "r"(smem_u32(bar)) : "memory"); }
 __device__ __forceinline__ void mw_ldsm4(uint32_t (&r)[4], uint32_t addr) {
@@ -70,17 +80,21 @@ struct MwShape {
     static constexpr int KS = Q4 ? 128 : 64;                          // columns of a stage
     static constexpr int WB = Q4 ? 64 : 128;                          // bytes of a row in a stage (Q4_0: of its nibbles)
     // a stage: rows [MW_TM][WB], activations [TN][128], Q4_0: rows' scales [MW_TM][4 halves], activation scales [4][TN] floats
-    static constexpr int X_OFF = MW_TM * WB, S_OFF = X_OFF + TN * 128, D_OFF = S_OFF + (Q4 ? MW_TM * 8 : 0), STAGE = D_OFF + (Q4 ? TN * 16 : 0);
-    static_assert(WM * WN == MW_CONS && MT * WM * 16 == MW_TM && STAGE % 128 == 0, "split");
+    // (Q4_0: low plane [TN][64], high plane [TN][64]; activation scales [TN][4]).  TMA writes and ldmatrix reads with the 16-byte pieces of a
+    // row permuted by the row's number in groups of 8 (64-byte rows: pairs of rows in groups of 4), counted from 1024-byte boundaries.
+    static constexpr int X_OFF = MW_TM * WB, S_OFF = X_OFF + TN * 128, D_OFF = S_OFF + (Q4 ? MW_TM * 8 : 0), STAGE = (D_OFF + (Q4 ? TN * 16 : 0) + 1023) / 1024 * 1024;
+    static_assert(WM * WN == MW_CONS && MT * WM * 16 == MW_TM && X_OFF % 1024 == 0 && D_OFF % 128 == 0 && TN % 8 == 0 && TN <= 256, "split");
 };
 
 template <int WT, int WM, int WN, int NT, bool SPARSE, bool GATED>
-__global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
+__global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant__ MwP p) {
     using Z = MwShape<WT, WM, WN, NT>;
     constexpr bool Q4 = Z::Q4;
     constexpr int TM = MW_TM, WB = Z::WB, MT = Z::MT;
-    constexpr int IT = GATED ? TM / 2 : TM;                           // items (rows / neurons) of a tile
-    extern __shared__ __align__(128) unsigned char smem[];
+    const int IT = GATED ? TM / 2 : SPARSE ? TM : p.per_tile;         // items (rows / neurons) of a tile
+    constexpr bool COPIES = SPARSE || Q4;                             // some of a stage comes by cp.async
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     __shared__ int s_warp[MW_THREADS / 32];
     __shared__ unsigned s_any[4];
     __shared__ uint64_t s_full[MW_SMAX], s_empty[MW_SMAX], s_bits[2];
@@ -92,7 +106,7 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
     const uint32_t ring = smem_u32(smem);
     constexpr uint32_t x_off = Z::X_OFF, s_off = Z::S_OFF, d_off = Z::D_OFF;
     if (tid < 4) s_any[tid] = 0u;
-    if (tid < MW_SMAX) { mbar_init(s_full + tid, MW_PROD); mbar_init(s_empty + tid, MW_CONS); }
+    if (tid < MW_SMAX) { mbar_init(s_full + tid, COPIES ? MW_PROD + 1 : 1); mbar_init(s_empty + tid, MW_CONS); }
     if (tid == 0) { mbar_init(s_bits, MW_CONS); mbar_init(s_bits + 1, MW_CONS); s_dead = 0; }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncthreads();
@@ -126,20 +140,14 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
         ok = r < TM && lo + k < hi;
         return (GATED && (r & 8) ? p.W2 : p.W) + (ok ? (size_t)(SPARSE ? rows[k] : lo + k) * p.row_bytes : 0);
     };
-    // Addresses are kept and moved along: a chain of address arithmetic per copy stalls the warp that should be at the products.
     const bool ragged = !Q4 && p.ncols % 64 != 0;                     // the last slice of a row is not whole
-    const int wr = pt / CW, xt = pt >> 3, xc = pt & 7, dt = pt >> 2;
-    const uint32_t w_to = (uint32_t)(wr * WB + (Q4 ? (cw ^ (wr >> 1)) & 3 : (cw ^ wr) & 7) * 16), x_to = x_off + (uint32_t)(xt * 128 + ((xc ^ xt) & 7) * 16);
-    const uint32_t d_to = d_off + (uint32_t)(((pt & 3) * Z::TN + dt) * 4);
-    const char * const x0 = Q4 ? reinterpret_cast<const char *>((xc & 1 ? p.x.hi : p.x.lo) + (size_t)xt * p.nb + (xc >> 1)) : reinterpret_cast<const char *>(p.x.h16 + (size_t)xt * p.ncols + xc * 8);
-    const char * const d0 = reinterpret_cast<const char *>(p.x.d + (size_t)dt * p.nb + (pt & 3));
-    const size_t x_step = (size_t)(Q4 ? p.nb * 16 : p.ncols * 2) * 16, d_step = (size_t)p.nb * 4 * 32;
-    constexpr int NX = Z::TN / 16, ND = (Z::TN + 31) / 32;
-    auto issue_w = [&](int slot) {
+    const int wr = pt / CW;
+    const uint32_t w_to = (uint32_t)(wr * WB + (Q4 ? (cw ^ (wr >> 1)) & 3 : (cw ^ wr) & 7) * 16);
+    auto issue_w = [&](int slot) {                                    // cp.async: addresses are kept and moved along
         if (i_slice == 0) {
             w_ok = 0u;
 #pragma unroll
-            for (int j = 0; j < NW; j++) {
+            for (int j = 0; j < (SPARSE ? NW : 0); j++) {
                 bool ok;
                 wp[j] = row_ptr(wr + j * WS, ok) + cw * 16;
                 if (ok) w_ok |= 1u << j;
@@ -153,7 +161,7 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
         const uint32_t base = ring + (uint32_t)(slot * Z::STAGE);
         const bool in = !ragged || i_slice * 64 + cw * 8 < p.ncols;   // past the end of a row: zeros
 #pragma unroll
-        for (int j = 0; j < NW; j++) {
+        for (int j = 0; j < (SPARSE ? NW : 0); j++) {
             const uint32_t to = base + w_to + j * WS * WB;
             if (w_ok >> j & 1u) { if (in) mw_cp16(to, wp[j]); else mw_zero16(to); }
             wp[j] += WB;
@@ -163,20 +171,15 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
             sp += 8;
         }
     };
-    auto issue_x = [&](int slot) {
-        const uint32_t base = ring + (uint32_t)(slot * Z::STAGE);
-        const char * src = x0 + (size_t)i_slice * (Q4 ? 64 : 128);
-        if (ragged && i_slice * 64 + xc * 8 >= p.ncols) {
-#pragma unroll
-            for (int j = 0; j < NX; j++) if (xt + j * 16 < p.T) mw_zero16(base + x_to + j * 16 * 128);
-        } else {
-#pragma unroll
-            for (int j = 0; j < NX; j++, src += x_step) if (xt + j * 16 < p.T) mw_cp16(base + x_to + j * 16 * 128, src);
-        }
+    auto issue_tma = [&](int slot) {                                  // one thread
+        unsigned char * base = smem + (size_t)slot * Z::STAGE;
+        uint64_t * bar = s_full + slot;
+        mbar_expect_tx(bar, (unsigned)(Z::TN * 128 + (Q4 ? Z::TN * 16 : 0) + (SPARSE ? 0 : p.per_tile * WB)));
+        if (!SPARSE) mw_tma(base, &p.m_w, i_slice * 64, lo + i_tile * IT, bar);
+        mw_tma(base + x_off, &p.m_x, i_slice * 64, 0, bar);
         if (Q4) {
-            const char * sd = d0 + (size_t)i_slice * 16;
-#pragma unroll
-            for (int j = 0; j < ND; j++, sd += d_step) if (dt + j * 32 < p.T) mw_cp4(base + d_to + j * 32 * 4, sd);
+            mw_tma(base + x_off + Z::TN * 64, &p.m_x2, i_slice * 64, 0, bar);
+            mw_tma(base + d_off, &p.m_d, i_slice * 4, 0, bar);
         }
     };
     auto advance = [&]() { if (++i_slice == p.n_slices) { i_slice = 0; i_tile++; } };
@@ -241,16 +244,21 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(MW_REGS_P));
         int slot = 0;
         unsigned phase = 1u;                                          // parity of the hand-back to wait for (first round: none)
+        if (!COPIES && warp > MW_CONS) return;
         for (int i = 0; i < n_units; i++) {
             if (!wait(s_empty + slot, phase)) break;
-            issue_w(slot);
-            issue_x(slot);
-            if (ragged && i_slice == p.n_slices - 1) __threadfence_block();      // zeros were stored, not copied
-            mw_arrive_copies(s_full + slot);
+            if (pt == 0) issue_tma(slot);
+            if (COPIES) {
+                issue_w(slot);
+                if (ragged && i_slice == p.n_slices - 1) __threadfence_block();  // zeros were stored, not copied
+                mw_arrive_copies(s_full + slot);
+            }
             advance();
             if (++slot == S) { slot = 0; phase ^= 1u; }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
+        if (s_dead && pt == 0)                                        // do not exit with tiles still landing in shared memory
+            for (int t = 0; t < S; t++) { int spins = 0; while (!mbar_try_wait(s_full + t, 0) && !mbar_try_wait(s_full + t, 1) && ++spins < (1 << 16)) {} }
         return;
     }
     // ===================================================================== consumers
@@ -272,8 +280,10 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
     const int row0 = wm * MT * 16, tok0 = wn * NT * 8;                // this warp's part of the tile
     // ldmatrix row addresses inside a stage (fragment layouts of mma.m16n8k16 / m16n8k32); the piece is added per step
     const uint32_t a_row = (uint32_t)((row0 + (Q4 && MT == 2 ? lane : lane & 15)) * WB);
-    const uint32_t b_row = x_off + (uint32_t)((tok0 + (lane & 7) + (lane >> 4) * 8) * 128), b_last = x_off + (uint32_t)((tok0 + (NT - 1) * 8 + (lane & 7)) * 128);
-    const int a_swz = Q4 ? (lane >> 1) & 3 : lane & 7, b_swz = lane & 7;
+    constexpr int XB = Q4 ? 64 : 128;                                 // bytes of a token (Q4_0: of a plane)
+    const uint32_t plane = Q4 ? ((lane >> 3) & 1) * Z::TN * 64 : 0;
+    const uint32_t b_row = x_off + plane + (uint32_t)((tok0 + (lane & 7) + (lane >> 4) * 8) * XB), b_last = x_off + plane + (uint32_t)((tok0 + (NT - 1) * 8 + (lane & 7)) * XB);
+    const int a_swz = Q4 ? (lane >> 1) & 3 : lane & 7, b_swz = Q4 ? (lane & 7) >> 1 : lane & 7;
 
     int tile = 0, slice = 0, slot = 0;
     unsigned phase = 0u;
@@ -292,7 +302,7 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
 #pragma unroll
                 for (int n = 0; n < NT; n += 2) {
                     uint32_t b[4];
-                    mw_ldsm4(b, base + (n + 1 < NT ? b_row + n * 8 * 128 : b_last) + (((2 * k + ((lane >> 3) & 1)) ^ b_swz) & 7) * 16);
+                    mw_ldsm4(b, base + (n + 1 < NT ? b_row + n * 8 * XB : b_last) + (((2 * k + ((lane >> 3) & 1)) ^ b_swz) & 7) * 16);
 #pragma unroll
                     for (int m = 0; m < MT; m++) {
                         mw_hmma(acc[Q4 ? 0 : m][Q4 ? 0 : n], a[m], b[0], b[1]);
@@ -329,13 +339,14 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
 #pragma unroll
                 for (int n = 0; n < NT; n += 2) {
                     uint32_t b[4];
-                    mw_ldsm4(b, base + (n + 1 < NT ? b_row + n * 8 * 128 : b_last) + (((2 * k + ((lane >> 3) & 1)) ^ b_swz) & 7) * 16);
+                    mw_ldsm4(b, base + (n + 1 < NT ? b_row + n * 8 * XB : b_last) + ((k ^ b_swz) & 3) * 16);
 #pragma unroll
                     for (int u = 0; u < 2; u++) {
                         if (n + u >= NT) break;
-                        unsigned long long dd;
-                        asm volatile("ld.shared.b64 %0, [%1];" : "=l"(dd) : "r"(base + d_off + (k * Z::TN + tok0 + (n + u) * 8 + 2 * q) * 4));
-                        dd = mw_mul2(dd, sixteenth);
+                        float t0, t1;                                 // scales of tokens 2q, 2q + 1
+                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t0) : "r"(base + d_off + (tok0 + (n + u) * 8 + 2 * q) * 16 + k * 4));
+                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t1) : "r"(base + d_off + (tok0 + (n + u) * 8 + 2 * q + 1) * 16 + k * 4));
+                        const unsigned long long dd = mw_mul2(mw_pack(t0, t1), sixteenth);
                         const unsigned long long md = mw_mul2(dd, neg_magic);
 #pragma unroll
                         for (int m = 0; m < MT; m++) {
@@ -420,6 +431,27 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const MwP p) {
 }
 
 // ---------------------------------------------------------------------------------------------- launch
+typedef CUresult (*MwEncode)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
+                             CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// rows of `cols` elements, `pitch` bytes apart, in boxes of box_cols x box_rows; what lies past the ends reads as zeros
+static int mw_map(CUtensorMap * m, CUtensorMapDataType type, const void * base, int64_t cols, int64_t rows, int64_t pitch, int box_cols, int box_rows, CUtensorMapSwizzle swizzle) {
+    static MwEncode encode = nullptr;
+    if (!encode) {
+        void * f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        PI_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q));
+        PI_REQUIRE(f && q == cudaDriverEntryPointSuccess, "mm_wide: the driver has no cuTensorMapEncodeTiled");
+        encode = (MwEncode)f;
+    }
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)pitch};
+    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows}, steps[2] = {1, 1};
+    const CUresult rc = encode(m, type, 2, const_cast<void *>(base), dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    PI_REQUIRE(rc == CUDA_SUCCESS, "mm_wide: tensor map refused (%d): %lld x %lld, pitch %lld", (int)rc, (long long)rows, (long long)cols, (long long)pitch);
+    return PI_OK;
+}
+
 template <int WT, int WM, int WN, int NT, bool SPARSE, bool GATED>
 static int mw_go(MwP p, bool pdl, cudaStream_t st) {
     using Z = MwShape<WT, WM, WN, NT>;
@@ -427,9 +459,26 @@ static int mw_go(MwP p, bool pdl, cudaStream_t st) {
     const int G = (int)imin64(sm_count(), (p.nrows + 7) / 8);
     const int list = SPARSE ? ((p.nrows + G - 1) / G + 1) * 4 : 0;    // bytes
     if (list > 8192) return PI_ERR_UNSUPPORTED;                       // (more than MM_MAX_ROWS rows)
-    p.S = (MW_SMEM_MAX - list) / Z::STAGE;
+    p.S = (MW_SMEM_MAX - 1024 - list) / Z::STAGE;
     if (p.S > MW_SMAX) p.S = MW_SMAX;
-    static_assert(2 * Z::STAGE <= MW_SMEM_MAX - 8192, "two stages");
+    static_assert(2 * Z::STAGE <= MW_SMEM_MAX - 1024 - 8192, "two stages");
+    p.per_tile = 0;
+    int rc;
+    if (!SPARSE) {                                                    // equal tiles; whole bytes of the masks
+        const int share = (p.nrows + G - 1) / G + (p.masks_out ? 8 : 0), tiles = (share + MW_TM - 1) / MW_TM;
+        p.per_tile = p.masks_out ? (share / tiles + 8) / 8 * 8 : (share + tiles - 1) / tiles;
+        if (p.per_tile > MW_TM) p.per_tile = MW_TM;
+        if (Z::Q4) rc = mw_map(&p.m_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.W, (int64_t)p.nb * 16, p.nrows, p.row_bytes, 64, p.per_tile, CU_TENSOR_MAP_SWIZZLE_64B);
+        else       rc = mw_map(&p.m_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, p.W, p.ncols, p.nrows, p.row_bytes, 64, p.per_tile, CU_TENSOR_MAP_SWIZZLE_128B);
+        if (rc != PI_OK) return rc;
+    }
+    if (Z::Q4) {
+        if ((rc = mw_map(&p.m_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.x.lo, (int64_t)p.nb * 16, p.T, (int64_t)p.nb * 16, 64, Z::TN, CU_TENSOR_MAP_SWIZZLE_64B)) != PI_OK) return rc;
+        if ((rc = mw_map(&p.m_x2, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.x.hi, (int64_t)p.nb * 16, p.T, (int64_t)p.nb * 16, 64, Z::TN, CU_TENSOR_MAP_SWIZZLE_64B)) != PI_OK) return rc;
+        if ((rc = mw_map(&p.m_d, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, p.x.d, p.nb, p.T, (int64_t)p.nb * 4, 4, Z::TN, CU_TENSOR_MAP_SWIZZLE_NONE)) != PI_OK) return rc;
+    } else {
+        if ((rc = mw_map(&p.m_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, p.x.h16, p.ncols, p.T, (int64_t)p.ncols * 2, 64, Z::TN, CU_TENSOR_MAP_SWIZZLE_128B)) != PI_OK) return rc;
+    }
     static bool attr_done[16] = {false};
     int dev = 0;
     PI_CUDA(cudaGetDevice(&dev));
@@ -438,7 +487,7 @@ static int mw_go(MwP p, bool pdl, cudaStream_t st) {
         PI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MW_SMEM_MAX));
         attr_done[dev] = true;
     }
-    PI_CUDA(launch_k(kern, dim3(G), dim3(MW_THREADS), (size_t)p.S * Z::STAGE + list, st, pdl, p));
+    PI_CUDA(launch_k(kern, dim3(G), dim3(MW_THREADS), (size_t)p.S * Z::STAGE + list + 1024, st, pdl, p));
     return PI_OK;
 }
 
