@@ -3,7 +3,8 @@
 //
 // Bound: with 77 FP16 tokens the tensor pipe and HBM are about even (12288 x 4096: 17 us of mma.sync at 955 multiply-adds per clock
 // and SM, 15 us of weights); above that the products.  Q4_0 is bound by the scaling of its blocks: an mma of 16 rows x 32 columns x
-// 8 tokens and the four packed FP32 operations that apply its scales take 18 clocks of a scheduler together (they share a pipe).
+// 8 tokens takes 8 clocks of a scheduler, the eight fused multiply-adds that apply its scales another 8 (as four packed ones they were
+// slower, 259 us where these take 208: packed operations have half the pipes, and every row scale needed a copy).
 // What must not cost extra is shared memory: every warp reads its own fragments of both operands.
 //
 // Work split: as in pi_mm.cu every CTA takes an equal contiguous range of rows, in tiles of 96, and producer warps (4) copy for the
@@ -23,7 +24,7 @@
 namespace pi {
 
 static constexpr int MW_THREADS = 512, MW_CONS = 12, MW_PROD = 128;       // warps 0 .. 11 consume, threads 384 .. 511 produce
-static constexpr int MW_REGS_C = 152, MW_REGS_P = 56;   // 384 x 152 + 128 x 56 = the 512 x 128 of the launch
+static constexpr int MW_REGS_C = 160, MW_REGS_P = 32;   // 384 x 160 + 128 x 32 = the 512 x 128 of the launch
 static constexpr int MW_TM = 96;                        // rows of a tile
 static constexpr int MW_SMEM_MAX = 224 * 1024;          // (leaves room for the static variables)
 static constexpr int MW_SMAX = 6;                       // stages at most
@@ -60,17 +61,13 @@ __device__ __forceinline__ void mw_hmma(float (&c)[4], const uint32_t (&a)[4], u
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void mw_imma(uint32_t (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, uint32_t c) {
-    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c));
+// (the C operand: four registers of their own, kept: as one value four times over it was copied into place for every product)
+__device__ __forceinline__ void mw_imma(uint32_t (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, const uint32_t (&c)[4]) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]));
 }
-__device__ __forceinline__ unsigned long long mw_pack(float a, float b) { unsigned long long r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
-__device__ __forceinline__ unsigned long long mw_packu(uint32_t a, uint32_t b) { unsigned long long r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b)); return r; }
-__device__ __forceinline__ unsigned long long mw_mul2(unsigned long long a, unsigned long long b) { unsigned long long r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-// acc += (v * dd - magic * dd) * d4, two tokens at a time: exact up to the two roundings of (v - magic) * dd * d4 (see pi_mm.cu)
-__device__ __forceinline__ void mw_scale_add(unsigned long long & acc, unsigned long long v, unsigned long long dd, unsigned long long md, unsigned long long d4) {
-    asm("{\n .reg .b64 t;\n fma.rn.f32x2 t, %1, %2, %3;\n fma.rn.f32x2 %0, t, %4, %0;\n}" : "+l"(acc) : "l"(v), "l"(dd), "l"(md), "l"(d4));
-}
+// acc += (v - magic) * dd * d4: exact up to the two roundings of the products (see pi_mm.cu)
+__device__ __forceinline__ void mw_scale_add(float & acc, uint32_t v, float dd, float md, float d4) { acc = fmaf(fmaf(__uint_as_float(v), dd, md), d4, acc); }
 
 // WM x WN consumers of MT x 16 rows and NT x 8 tokens
 template <int WT, int WM, int WN, int NT>
@@ -263,20 +260,20 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
     }
     // ===================================================================== consumers
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(MW_REGS_C));
-    float acc[Q4 ? 1 : MT][Q4 ? 1 : NT][4];                           // (the accumulators of the two types have different shapes)
-    unsigned long long acq[Q4 ? MT : 1][Q4 ? NT : 1][2];
+    float acc[MT][NT][4];
     auto clear = [&]() {
 #pragma unroll
         for (int m = 0; m < MT; m++)
 #pragma unroll
             for (int n = 0; n < NT; n++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) { if (Q4) acq[Q4 ? m : 0][Q4 ? n : 0][j >> 1] = 0ull; else acc[Q4 ? 0 : m][Q4 ? 0 : n][j] = 0.f; }
+                for (int j = 0; j < 4; j++) acc[m][n][j] = 0.f;
     };
     clear();
     const int g = lane >> 2, q = lane & 3;
-    const uint32_t MAGIC = 0x4B400000u;
-    const unsigned long long neg_magic = mw_pack(-12582912.0f, -12582912.0f), sixteenth = mw_pack(0.0625f, 0.0625f);
+    uint32_t MAGIC[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) asm volatile("mov.u32 %0, 0x4B400000;" : "=r"(MAGIC[j]));
     const int row0 = wm * MT * 16, tok0 = wn * NT * 8;                // this warp's part of the tile
     // ldmatrix row addresses inside a stage (fragment layouts of mma.m16n8k16 / m16n8k32); the piece is added per step
     const uint32_t a_row = (uint32_t)((row0 + (Q4 && MT == 2 ? lane : lane & 15)) * WB);
@@ -305,8 +302,8 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
                     mw_ldsm4(b, base + (n + 1 < NT ? b_row + n * 8 * XB : b_last) + (((2 * k + ((lane >> 3) & 1)) ^ b_swz) & 7) * 16);
 #pragma unroll
                     for (int m = 0; m < MT; m++) {
-                        mw_hmma(acc[Q4 ? 0 : m][Q4 ? 0 : n], a[m], b[0], b[1]);
-                        if (n + 1 < NT) mw_hmma(acc[Q4 ? 0 : m][Q4 ? 0 : (n + 1) % NT], a[m], b[2], b[3]);
+                        mw_hmma(acc[m][n], a[m], b[0], b[1]);
+                        if (n + 1 < NT) mw_hmma(acc[m][(n + 1) % NT], a[m], b[2], b[3]);
                     }
                 }
             }
@@ -322,7 +319,7 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
                     w[0] = w1[2 * (k & 1)]; w[1] = w1[2 * (k & 1) + 1]; w[2] = w[3] = 0u;
                 }
                 uint32_t a[MT][4];
-                unsigned long long d4[MT][2];
+                float d4[MT][2];                                      // (the nibbles stand for 16 times their value)
 #pragma unroll
                 for (int m = 0; m < MT; m++) {
                     const uint32_t w0 = w[2 * m], wh = w[2 * m + 1];
@@ -332,8 +329,7 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
                     for (int h = 0; h < 2; h++) {
                         unsigned short s;
                         asm volatile("ld.shared.u16 %0, [%1];" : "=h"(s) : "r"(base + s_off + (row0 + m * 16 + g + h * 8) * 8 + k * 2));
-                        const float e = __half2float(__ushort_as_half(s));
-                        d4[m][h] = mw_pack(e, e);
+                        d4[m][h] = __half2float(__ushort_as_half(s)) * 0.0625f;
                     }
                 }
 #pragma unroll
@@ -346,14 +342,16 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
                         float t0, t1;                                 // scales of tokens 2q, 2q + 1
                         asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t0) : "r"(base + d_off + (tok0 + (n + u) * 8 + 2 * q) * 16 + k * 4));
                         asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t1) : "r"(base + d_off + (tok0 + (n + u) * 8 + 2 * q + 1) * 16 + k * 4));
-                        const unsigned long long dd = mw_mul2(mw_pack(t0, t1), sixteenth);
-                        const unsigned long long md = mw_mul2(dd, neg_magic);
+                        const float m0 = t0 * -12582912.0f, m1 = t1 * -12582912.0f;
 #pragma unroll
                         for (int m = 0; m < MT; m++) {
                             uint32_t c[4];
                             mw_imma(c, a[m], b[2 * u], b[2 * u + 1], MAGIC);
-                            mw_scale_add(acq[Q4 ? m : 0][Q4 ? (n + u) % NT : 0][0], mw_packu(c[0], c[1]), dd, md, d4[m][0]);
-                            mw_scale_add(acq[Q4 ? m : 0][Q4 ? (n + u) % NT : 0][1], mw_packu(c[2], c[3]), dd, md, d4[m][1]);
+                            float (&o)[4] = acc[m][(n + u) % NT];
+                            mw_scale_add(o[0], c[0], t0, m0, d4[m][0]);
+                            mw_scale_add(o[1], c[1], t1, m1, d4[m][0]);
+                            mw_scale_add(o[2], c[2], t0, m0, d4[m][1]);
+                            mw_scale_add(o[3], c[3], t1, m1, d4[m][1]);
                         }
                     }
                 }
@@ -382,16 +380,7 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
                                 for (int j = 0; j < 2; j++) {
                                     const int t = tok0 + n * 8 + 2 * q + j;
                                     if (t >= p.T) continue;
-                                    float v[2];
-#pragma unroll
-                                    for (int z = 0; z < 2; z++) {
-                                        if (Q4) {
-                                            const unsigned long long w = acq[Q4 ? m : 0][Q4 ? n : 0][z];
-                                            v[z] = __uint_as_float(j ? (unsigned)(w >> 32) : (unsigned)w);
-                                        } else {
-                                            v[z] = acc[Q4 ? 0 : m][Q4 ? 0 : n][2 * z + j];
-                                        }
-                                    }
+                                    const float v[2] = {acc[m][n][j], acc[m][n][2 + j]};
                                     float o = GATED ? fmaxf(v[1], 0.f) * v[0] : v[h];
                                     const bool off = SPARSE && p.idx[(size_t)t * p.idx_stride + gid] < p.threshold;   // (a NaN logit counts as active)
                                     if (off && p.coef) { p.coef[(size_t)t * p.coef_stride + item] = __ushort_as_half((unsigned short)0); continue; }
