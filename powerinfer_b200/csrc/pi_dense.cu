@@ -695,6 +695,212 @@ __global__ void __launch_bounds__(ATTN_THREADS) k_attention(const AttnP p) {
     PI_TL_MARK(4);
 }
 
+// The same for head_dim 64 and 128, one CTA per query head and token.  Latency-bound: what counts is the length of the chain
+// QKV -> scores -> maximum -> sum -> probabilities -> values -> planes (the kernel above: 8.6 us of 16500 clocks at 150 positions).
+//   scores   mma.m16n8k16 with 16 cached rows as A, straight from global memory (a lane loads 16 bytes of a row, which serve as A
+//            operands of two products whose k order is permuted in the same way on the query side), and the query as every column of B,
+//            so that every lane finds its rows' scores in place: 16 instructions per 16 rows where dot products take 400 and a
+//            shuffle tree per row.  The rows of the first 512 positions are loaded BEFORE the wait (earlier steps stored them).
+//   values   the first 12 rows of a thread are requested before the softmax and travel while it runs.
+//   sums     the numerators are FP16 numbers, i.e. multiples of 2^-24: their sum is exact in integers (redux.sync), as it is in double.
+//   planes   a warp owns one block of 32 columns and quantises it itself.
+template <int HC>                                                     // head_dim / 32
+__global__ void __launch_bounds__(ATTN_THREADS) k_attention_row(const AttnP p) {
+    constexpr int HD = HC * 32, HALF = HD / 2, CH = HD / 8, SL = ATTN_THREADS / CH, NW = ATTN_THREADS / 32;
+    constexpr int KU = 2, UV = 12;                                    // passes of 256 rows, value rows per thread in flight
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ __align__(16) __half q16[HD], k16[HD], v16[HD];
+    __shared__ float red[NW][HD];
+    __shared__ unsigned s_sum[NW];
+    __shared__ int s_max[NW];
+    float * sc = reinterpret_cast<float *>(smem_raw);                 // [n_ctx] scores
+    __half * p16 = reinterpret_cast<__half *>(sc + p.n_ctx);          // [n_ctx] probabilities
+    const int h = blockIdx.x, t = blockIdx.y, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, q = lane & 3;
+    const int group = p.n_head / p.n_head_kv, hk = h / group, dkv = p.n_head_kv * HD;
+    pdl_launch();
+    // ---- before the wait: everything that no kernel of this step writes
+    const int pos = p.pos[t];
+    const int sq = p.seq ? p.seq[t] : 0;
+    if (pos < 0 || pos >= p.n_ctx) return;                            // never index the cache out of range
+    __half * kc = p.k_cache + (size_t)sq * p.n_ctx * dkv + (size_t)hk * HD;
+    __half * vc = p.v_cache + (size_t)sq * p.n_ctx * dkv + (size_t)hk * HD;
+    const bool early = p.store_mode == 0;                             // (a prompt chunk's rows were stored by the launch before)
+    uint4 kv[KU][2][HC];
+    auto load_keys = [&]() {
+#pragma unroll
+        for (int u = 0; u < KU; u++)
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                const int j = (u * NW + wid) * 16 + g + 8 * r;
+#pragma unroll
+                for (int c = 0; c < HC; c++) kv[u][r][c] = j < pos ? *(reinterpret_cast<const uint4 *>(kc + (size_t)j * dkv) + c * 4 + q) : make_uint4(0u, 0u, 0u, 0u);
+            }
+    };
+    if (early) {
+        load_keys();
+        for (int j = tid; j < pos; j += ATTN_THREADS) {
+            const char * vr = reinterpret_cast<const char *>(vc + (size_t)j * dkv);
+#pragma unroll
+            for (int o = 0; o < HD * 2; o += 128) asm volatile("prefetch.global.L2 [%0];" :: "l"(vr + o));
+        }
+    }
+    float2 cs = make_float2(1.f, 0.f);
+    if (p.cs && tid < HALF) cs = reinterpret_cast<const float2 *>(p.cs)[(size_t)pos * HALF + tid];
+    pdl_wait();
+    if (!early) load_keys();
+
+    // ---- the query and the new key, rotated, and the new value, as FP16
+    if (tid < HALF) {
+        const float * qh = p.q + (size_t)t * p.q_stride + (size_t)h * HD;
+        const float * kh = p.k + (size_t)t * p.kv_stride + (size_t)hk * HD;
+        const int i0 = p.cs && !p.neox ? 2 * tid : tid, i1 = p.cs && !p.neox ? 2 * tid + 1 : tid + HALF;
+        float a0 = qh[i0], a1 = qh[i1], b0 = kh[i0], b1 = kh[i1];
+        if (p.cs) {
+            float o0, o1;
+            rope_pair(a0, a1, cs.x, cs.y, o0, o1); a0 = o0; a1 = o1;
+            rope_pair(b0, b1, cs.x, cs.y, o0, o1); b0 = o0; b1 = o1;
+        }
+        q16[i0] = __float2half_rn(a0); q16[i1] = __float2half_rn(a1);
+        k16[i0] = __float2half_rn(b0); k16[i1] = __float2half_rn(b1);
+    } else if (tid >= 256 && tid < 256 + HD) {
+        v16[tid - 256] = __float2half_rn(p.v[(size_t)t * p.kv_stride + (size_t)hk * HD + tid - 256]);
+    }
+    __syncthreads();
+    if (h % group == 0 && p.store_mode == 0 && tid < HD) {
+        kc[(size_t)pos * dkv + tid] = k16[tid];
+        vc[(size_t)pos * dkv + tid] = v16[tid];
+    }
+
+    // ---- scores
+    const float scale = 1.0f / sqrtf((float)HD);
+    uint4 bq[HC];
+#pragma unroll
+    for (int c = 0; c < HC; c++) bq[c] = *(reinterpret_cast<const uint4 *>(q16) + c * 4 + q);
+    float mx = -INFINITY;
+    auto mma = [&](float (&c4)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+            : "+f"(c4[0]), "+f"(c4[1]), "+f"(c4[2]), "+f"(c4[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+    };
+    auto score = [&](int j0, uint4 (&rw)[2][HC]) {                    // rows j0 .. j0 + 15, of which this lane holds g and g + 8
+#pragma unroll
+        for (int r = 0; r < 2; r++)
+            if (j0 + g + 8 * r == pos) {
+#pragma unroll
+                for (int c = 0; c < HC; c++) rw[r][c] = *(reinterpret_cast<const uint4 *>(k16) + c * 4 + q);
+            }
+        __syncwarp();
+        float x[4] = {0.f, 0.f, 0.f, 0.f}, y[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int c = 0; c < HC; c++) {
+            mma(x, rw[0][c].x, rw[1][c].x, rw[0][c].y, rw[1][c].y, bq[c].x, bq[c].y);
+            mma(y, rw[0][c].z, rw[1][c].z, rw[0][c].w, rw[1][c].w, bq[c].z, bq[c].w);
+        }
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const int j = j0 + g + 8 * r;
+            const float v = (x[2 * r] + y[2 * r]) * scale;
+            if (j <= pos) { mx = fmaxf(mx, v); if (q == 0) sc[j] = v; }
+        }
+    };
+#pragma unroll
+    for (int u = 0; u < KU; u++) if (__shfl_sync(0xffffffffu, (u * NW + wid) * 16, 0) <= pos) score((u * NW + wid) * 16, kv[u]);
+    for (int j0 = (KU * NW + wid) * 16; j0 <= pos; j0 += NW * 16) {
+        uint4 rw[2][HC];
+#pragma unroll
+        for (int r = 0; r < 2; r++)
+#pragma unroll
+            for (int c = 0; c < HC; c++) rw[r][c] = j0 + g + 8 * r < pos ? *(reinterpret_cast<const uint4 *>(kc + (size_t)(j0 + g + 8 * r) * dkv) + c * 4 + q) : make_uint4(0u, 0u, 0u, 0u);
+        score(j0, rw);
+    }
+    // ---- the first value rows of this thread: 8 columns c8 of rows sl, sl + SL, ...
+    const int c8 = tid % CH, sl = tid / CH;
+    uint4 vv[UV];
+#pragma unroll
+    for (int u = 0; u < UV; u++) {
+        const int j = sl + u * SL;
+        vv[u] = make_uint4(0u, 0u, 0u, 0u);
+        if (j < pos) vv[u] = *(reinterpret_cast<const uint4 *>(vc + (size_t)j * dkv) + c8);
+        else if (j == pos) vv[u] = reinterpret_cast<const uint4 *>(v16)[c8];
+    }
+    // (a float's bits, with the lower 31 flipped where it is negative, compare like the float)
+    auto ordered = [](int b) { return b ^ ((b >> 31) & 0x7fffffff); };
+    const int mi = __reduce_max_sync(0xffffffffu, ordered(__float_as_int(mx)));
+    if (lane == 0) s_max[wid] = mi;
+    __syncthreads();
+    int m = s_max[0];
+#pragma unroll
+    for (int i = 1; i < NW; i++) m = max(m, s_max[i]);
+    mx = __int_as_float(ordered(m));
+
+    // ---- softmax (ggml.c:10708-10777)
+    unsigned part = 0u;
+    for (int j = tid; j <= pos; j += ATTN_THREADS) {
+        const float e = round_f16(expf(round_f16(sc[j] - mx)));
+        sc[j] = e;
+        part += (unsigned)(e * 16777216.0f);                          // exact; 2^24 at most, for up to 7 positions of a thread (launch_attention)
+    }
+    const unsigned ws = __reduce_add_sync(0xffffffffu, part);
+    if (lane == 0) s_sum[wid] = ws;
+    __syncthreads();
+    {
+        unsigned long long tot = 0ull;
+#pragma unroll
+        for (int i = 0; i < NW; i++) tot += s_sum[i];
+        const float inv = (float)(1.0 / ((double)tot * (1.0 / 16777216.0)));
+        for (int j = tid; j <= pos; j += ATTN_THREADS) p16[j] = __float2half_rn(sc[j] * inv);
+    }
+    __syncthreads();
+
+    // ---- out[e] = sum_j p_j V[j, e]
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    auto add = [&](int j, const uint4 & v) {
+        const float pj = __half2float(p16[j]);
+        const float2 v0 = h2f(v.x), v1 = h2f(v.y), v2 = h2f(v.z), v3 = h2f(v.w);
+        acc[0] = fmaf(pj, v0.x, acc[0]); acc[1] = fmaf(pj, v0.y, acc[1]); acc[2] = fmaf(pj, v1.x, acc[2]); acc[3] = fmaf(pj, v1.y, acc[3]);
+        acc[4] = fmaf(pj, v2.x, acc[4]); acc[5] = fmaf(pj, v2.y, acc[5]); acc[6] = fmaf(pj, v3.x, acc[6]); acc[7] = fmaf(pj, v3.y, acc[7]);
+    };
+#pragma unroll
+    for (int u = 0; u < UV; u++) { const int j = sl + u * SL; if (j <= pos) add(j, vv[u]); }
+    for (int j0 = sl + UV * SL; j0 <= pos; j0 += SL * 4) {
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int j = j0 + u * SL;
+            v[u] = make_uint4(0u, 0u, 0u, 0u);
+            if (j < pos) v[u] = *(reinterpret_cast<const uint4 *>(vc + (size_t)j * dkv) + c8);
+            else if (j == pos) v[u] = reinterpret_cast<const uint4 *>(v16)[c8];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) if (j0 + u * SL <= pos) add(j0 + u * SL, v[u]);
+    }
+#pragma unroll
+    for (int o = CH; o < 32; o <<= 1)
+#pragma unroll
+        for (int j = 0; j < 8; j++) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+    if (lane < CH) {
+        *reinterpret_cast<float4 *>(&red[wid][lane * 8]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        *reinterpret_cast<float4 *>(&red[wid][lane * 8 + 4]) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+    }
+    __syncthreads();
+    if (tid >= HD) return;
+    float o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int w = 0; w < NW; w++) o[w & 3] += red[w][tid];
+    const float v = (o[0] + o[1]) + (o[2] + o[3]);
+    const int64_t n = (int64_t)p.n_head * HD, e = (int64_t)h * HD + tid;
+    if (p.out) p.out[(size_t)t * n + e] = v;
+    if (p.out_act_type == PI_TYPE_F16) {
+        p.out_act.h16[(size_t)t * n + e] = __float2half_rn(v);
+    } else if (p.out_act_type == PI_TYPE_Q4_0) {                      // as emit_act8, a block per warp
+        const float amax = warp_max(fabsf(v));
+        const float d = amax / 127.0f, id = amax != 0.0f ? 127.0f / amax : 0.0f;
+        const int qv = __float2int_rn(v * id), s = __reduce_add_sync(0xffffffffu, qv);
+        const size_t blk = (size_t)t * (n / QK) + (size_t)(e / QK);
+        reinterpret_cast<int8_t *>(lane < 16 ? p.out_act.lo + blk : p.out_act.hi + blk)[lane & 15] = (int8_t)qv;
+        if (lane == 0) { p.out_act.d[blk] = __half2float(__float2half_rn(d)); p.out_act.s[blk] = s; }
+    }
+}
+
 int launch_attention(const AttnArgs & a, cudaStream_t st) {
     if (a.T <= 0) return PI_OK;
     PI_REQUIRE(a.head_dim % 32 == 0 && a.head_dim <= 256, "attention: head_dim=%d must be a multiple of 32, <= 256", a.head_dim);
@@ -720,6 +926,13 @@ int launch_attention(const AttnArgs & a, cudaStream_t st) {
     }
     PI_REQUIRE(smem <= 200 * 1024, "attention: n_ctx=%d needs %zu bytes of shared memory", a.n_ctx, smem);
     const dim3 grid(a.n_head, a.T);
+    // (32 x 7 x 2^24 fits the 32 bits of a warp's sum)
+    if ((a.head_dim == 64 || a.head_dim == 128) && a.store_mode != 1 && a.n_ctx <= 7 * ATTN_THREADS) {
+        const size_t smem1 = (size_t)a.n_ctx * 6 + 16;
+        if (a.head_dim == 64) PI_CUDA(launch_k(k_attention_row<2>, grid, dim3(ATTN_THREADS), smem1, st, a.pdl, p));
+        else                  PI_CUDA(launch_k(k_attention_row<4>, grid, dim3(ATTN_THREADS), smem1, st, a.pdl, p));
+        return PI_OK;
+    }
     PI_CUDA(launch_k(k_attention, grid, dim3(ATTN_THREADS), smem, st, a.pdl, p));
     return PI_OK;
 }
