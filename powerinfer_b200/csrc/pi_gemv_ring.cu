@@ -564,7 +564,8 @@ static int launch_ring_g(const RingP & p, const RingPlan & pl, bool pdl, cudaStr
 }
 
 
-// Two 100 KB rings per SM rather than one big one (PI_RING_CPS / PI_RING_KB override): with a single 8-warp CTA the
+// Two rings of up to 106 KB per SM (three stages of four 8 KB rows: 7 % of a 7B step over two; the CTAs of the one-token attention
+// still fit beside them) rather than one big one (PI_RING_CPS / PI_RING_KB override): with a single 8-warp CTA the
 // consumers are issue-latency bound, and what matters for bandwidth is ~200 KB of copies in flight per SM; four 54 KB rings
 // measure the same, two 54 KB rings 30 % slower.
 static RingPlan ring_plan(int wtype, int64_t nrows, int64_t ncols, bool sparse, bool gated) {
@@ -576,7 +577,7 @@ static RingPlan ring_plan(int wtype, int64_t nrows, int64_t ncols, bool sparse, 
     const size_t x_bytes = wtype == PI_TYPE_F16 ? (size_t)ncols * 2 : (size_t)(ncols / QK) * 40;
     static int cps0 = 0, kb0 = 0, rw0 = 2;
     if (!cps0) { const char * w = getenv("PI_RING_RW"); rw0 = w ? atoi(w) : 2; if (rw0 != 1 && rw0 != 4) rw0 = 2; }
-    if (!cps0) { const char * v = getenv("PI_RING_CPS"); cps0 = v ? atoi(v) : 2; const char * k = getenv("PI_RING_KB"); kb0 = k ? atoi(k) : 100; }
+    if (!cps0) { const char * v = getenv("PI_RING_CPS"); cps0 = v ? atoi(v) : 2; const char * k = getenv("PI_RING_KB"); kb0 = k ? atoi(k) : 106; }
     for (int cps = cps0; cps >= 1; cps /= 2) {
         const size_t budget = (size_t)(cps == cps0 ? kb0 : (cps == 2 ? 110 : 200)) * 1024;
         const int G = sm_count() * cps;
