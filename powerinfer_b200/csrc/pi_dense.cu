@@ -411,7 +411,8 @@ int launch_norm(const NormArgs & a, cudaStream_t st) {
     p.y = a.y; p.act_type = a.act_type; p.act = a.act; p.act2_type = a.act2_type; p.act2 = a.act2; p.act2_src = a.act2_src;
     static int use_cluster = -1;
     if (use_cluster < 0) { const char * v = getenv("PI_NORM_CLUSTER"); use_cluster = !(v && v[0] == '0'); }
-    if ((use_cluster || xch) && (a.x || a.partial)) {
+    // (a cluster per token shortens one token's chain; many tokens fill the chip without, and clusters of 8 cost more to place than they save)
+    if (((use_cluster && a.T <= 32) || xch) && (a.x || a.partial)) {
         int cs = 0;
         for (int k = 8; k >= (xch ? 1 : 2); k /= 2) if (a.n % (k * 256) == 0 && a.n / k / 8 <= 256) { cs = k; break; }
         if (cs) {

@@ -335,18 +335,18 @@ __global__ void __launch_bounds__(RED_WARPS * 32) k_reduce_partials(const float 
                                                                      float * __restrict__ dst, const float * __restrict__ residual2,
                                                                      double * __restrict__ stats_out) {
     __shared__ float4 s_part[RED_WARPS][32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
     pdl_launch();
     pdl_wait();
     const int64_t i4 = (int64_t)blockIdx.x * 32 + lane;                // float4 index
     const bool ok = i4 * 4 < total;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (ok) {
-        for (int j0 = w; j0 < G; j0 += RED_WARPS * 8) {                // 8 loads in flight, added in group order
+        for (int j0 = w; j0 < G; j0 += W * 8) {                // 8 loads in flight, added in group order
             float4 a[8];
 #pragma unroll
             for (int u = 0; u < 8; u++) {
-                const int j = j0 + u * RED_WARPS;
+                const int j = j0 + u * W;
                 a[u] = j < G ? __ldcg(reinterpret_cast<const float4 *>(partial + (size_t)j * total) + i4) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
 #pragma unroll
@@ -356,8 +356,7 @@ __global__ void __launch_bounds__(RED_WARPS * 32) k_reduce_partials(const float 
     s_part[w][lane] = v;
     __syncthreads();
     if (w == 0 && ok) {
-#pragma unroll
-        for (int k = 1; k < RED_WARPS; k++) { const float4 a = s_part[k][lane]; v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w; }
+        for (int k = 1; k < W; k++) { const float4 a = s_part[k][lane]; v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w; }
         const int64_t i = i4 * 4;
         if (bias) { const int64_t c = i % n; v.x += bias[c]; v.y += bias[c + 1]; v.z += bias[c + 2]; v.w += bias[c + 3]; }
         if (residual2) { const float4 r = *reinterpret_cast<const float4 *>(residual2 + i); v.x += r.x; v.y += r.y; v.z += r.z; v.w += r.w; }
@@ -378,7 +377,10 @@ int launch_reduce_partials(const float * partial, int n_groups, int T, int64_t n
     if (total == 0) return PI_OK;
     PI_REQUIRE(n % 4 == 0, "reduce: n must be a multiple of 4");
     const int grid = (int)((total / 4 + 31) / 32);
-    PI_CUDA(launch_k(k_reduce_partials, dim3(grid), dim3(RED_WARPS * 32), 0, st, pdl, partial, n_groups, total, n, residual, bias, dst, residual2, stats_out));
+    // a warp per group as long as there are few CTAs (one token's 150 groups: one load round), else a few warps that take several groups
+    // each: 9 groups of 16 tokens x 5120 values took 7.7 us in 640 CTAs of 32 warps, most of them without a group
+    const int warps = grid <= 2 * sm_count() && n_groups > 8 ? RED_WARPS : 4;
+    PI_CUDA(launch_k(k_reduce_partials, dim3(grid), dim3(warps * 32), 0, st, pdl, partial, n_groups, total, n, residual, bias, dst, residual2, stats_out));
     return PI_OK;
 }
 
