@@ -267,7 +267,7 @@ int  pi_engine_decode_host(pi_engine * e, const int32_t * host_tokens, const int
 
 /* Prompt processing (llama_decode with a batch of n_tokens > 1 tokens of one sequence: llama.cpp:6764-7006; the reference's
  * batched sparse kernels are ggml-cuda.cu:4607-4682, 4758-4824): n_tokens consecutive tokens of sequence `seq`, the first
- * at position pos0, go through the engine in chunks of up to max_batch tokens per step.  A chunk's step stores the K / V of
+ * at position pos0, go through the engine in chunks of up to 256 tokens per step (max_batch in sharded runs).  A chunk's step stores the K / V of
  * all its tokens first and then attends causally, reads every weight row once for the whole chunk, and applies each
  * token's own predictor mask (union list for reading, per-token predicate for writing: ggml.c:14250-14259).  Only the last
  * token's logits are computed and copied back (host_logits_last F32 [n_vocab], host_argmax_last int32 [1]; both may be

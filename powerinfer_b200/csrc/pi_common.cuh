@@ -151,8 +151,6 @@ struct CompactArgs {
 };
 int launch_compact(const CompactArgs & a, cudaStream_t st);
 
-// pulls the byte ranges into L2 (a hint; nothing may depend on it)
-
 struct AxpyArgs {
     int wtype = PI_TYPE_F16;
     const void * Wt = nullptr; int64_t nrows = 0, ncols = 0;

@@ -50,7 +50,7 @@ struct MmP {
     const float * bias; int relu;
     float * dst; __half * dst16; int64_t dst_stride; float * const * dst_host;
     __half * coef; int64_t coef_stride;
-    uint32_t * masks_out; float masks_threshold; int masks_or;
+    uint32_t * masks_out; float masks_threshold;
     unsigned int * status;
     int n_slices, ring;                                               // slices of 64 bytes of a row; bytes of a warp's ring
 };
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
     __shared__ uint64_t s_full[MM_RINGS][MM_SMAX], s_empty[MM_RINGS][MM_SMAX], s_tile;
     __shared__ volatile int s_dead;
     int * rows = reinterpret_cast<int *>(smem + (size_t)MM_RINGS * p.ring);      // rows of this CTA (sparse only)
-    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);    // (uniform, also for the compiler: see the note)
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);    // (a shuffle: uniform for the compiler too; a branch it takes for divergent costs every mma behind it)
     const int G = gridDim.x, cta = blockIdx.x;
     const int me = warp & (MM_RINGS - 1);                             // my ring
     const uint32_t ring_a = smem_u32(smem) + (uint32_t)(me * p.ring);
@@ -508,7 +508,7 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
             if (tid < 16 && tid * 8 < n_tile) {                       // the range starts at a multiple of 8 rows
                 unsigned char * o = reinterpret_cast<unsigned char *>(p.masks_out) + (lo + first) / 8 + tid;
                 const unsigned char bits = (unsigned char)(s_any[tid / 4] >> (tid % 4 * 8));
-                *o = p.masks_or ? (unsigned char)(*o | bits) : bits;
+                *o = bits;
             }
         }
         __syncwarp();
@@ -553,35 +553,20 @@ static int mm_tokens(const MmP & p, bool pdl, cudaStream_t st) {
     return mm_sel<WT, 4>(p, pdl, st);
 }
 
-// PI_ERR_UNSUPPORTED: shape not eligible, the caller uses another kernel.  Tokens go in launches of at most 32.
+// PI_ERR_UNSUPPORTED: shape not eligible, the caller uses another kernel.
 int launch_mm(const GemvArgs & a, cudaStream_t st) {
     const bool q4 = a.wtype == PI_TYPE_Q4_0;
     if (q4 ? !a.x.lo || a.ncols % 256 != 0 : !a.x.h16 || a.ncols % 8 != 0) return PI_ERR_UNSUPPORTED;
     if (a.nrows > (a.masks ? MM_MAX_ROWS : (1 << 26)) || (a.W2 && !a.masks) || (a.list && !a.masks)) return PI_ERR_UNSUPPORTED;
     if (a.T > 32) return launch_mm_wide(a, st);
-    {
-        const int t0 = 0;
-        MmP p;
-        p.W = (const uint8_t *)a.W; p.W2 = (const uint8_t *)a.W2; p.row_bytes = (int64_t)pi_row_bytes(a.wtype, a.ncols);
-        p.nrows = (int)a.nrows; p.ncols = (int)a.ncols; p.nb = (int)(a.ncols / 32);
-        p.T = a.T - t0 < 32 ? a.T - t0 : 32;
-        if (q4) {
-            p.x.lo = a.x.lo + (size_t)t0 * p.nb; p.x.hi = a.x.hi + (size_t)t0 * p.nb; p.x.d = a.x.d + (size_t)t0 * p.nb;
-        } else {
-            p.x.h16 = a.x.h16 + (size_t)t0 * a.ncols;
-        }
-        p.masks = a.masks; p.bucket = a.bucket; p.list = a.list_out; p.count = a.count_out; p.rows_total = t0 == 0 ? a.rows_total : nullptr;
-        p.idx = a.idx ? a.idx + (size_t)t0 * a.idx_stride : nullptr; p.idx_stride = a.idx_stride; p.threshold = a.threshold;
-        p.bias = a.bias; p.relu = a.relu;
-        p.dst = a.dst ? a.dst + (size_t)t0 * a.dst_stride : nullptr;
-        p.dst16 = a.dst16 ? a.dst16 + (size_t)t0 * a.dst_stride : nullptr; p.dst_stride = a.dst_stride; p.dst_host = a.dst_host;
-        p.coef = a.coef ? a.coef + (size_t)t0 * a.coef_stride : nullptr; p.coef_stride = a.coef_stride;
-        p.masks_out = a.masks_out; p.masks_threshold = a.masks_threshold; p.masks_or = t0 > 0;
-        p.status = a.status; p.n_slices = 0; p.ring = 0;
-        const int rc = q4 ? mm_tokens<PI_TYPE_Q4_0>(p, a.pdl, st) : mm_tokens<PI_TYPE_F16>(p, a.pdl, st);
-        if (rc != PI_OK) return rc;
-    }
-    return PI_OK;
+    MmP p;
+    p.W = (const uint8_t *)a.W; p.W2 = (const uint8_t *)a.W2; p.row_bytes = (int64_t)pi_row_bytes(a.wtype, a.ncols);
+    p.nrows = (int)a.nrows; p.ncols = (int)a.ncols; p.nb = (int)(a.ncols / 32); p.x = a.x; p.T = a.T;
+    p.masks = a.masks; p.bucket = a.bucket; p.list = a.list_out; p.count = a.count_out; p.rows_total = a.rows_total;
+    p.idx = a.idx; p.idx_stride = a.idx_stride; p.threshold = a.threshold; p.bias = a.bias; p.relu = a.relu;
+    p.dst = a.dst; p.dst16 = a.dst16; p.dst_stride = a.dst_stride; p.dst_host = a.dst_host; p.coef = a.coef; p.coef_stride = a.coef_stride;
+    p.masks_out = a.masks_out; p.masks_threshold = a.masks_threshold; p.status = a.status; p.n_slices = 0; p.ring = 0;
+    return q4 ? mm_tokens<PI_TYPE_Q4_0>(p, a.pdl, st) : mm_tokens<PI_TYPE_F16>(p, a.pdl, st);
 }
 
 }  // namespace pi

@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
     __shared__ uint64_t s_full[MW_SMAX], s_empty[MW_SMAX], s_bits[2];
     __shared__ volatile int s_dead;
     int * rows = reinterpret_cast<int *>(smem + (size_t)p.S * Z::STAGE);          // rows of this CTA (sparse only)
-    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);    // (uniform, also for the compiler: see the note)
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);    // (a shuffle: uniform for the compiler too; a branch it takes for divergent costs every mma behind it)
     const int wm = warp % WM, wn = warp / WM;
     const int G = gridDim.x, cta = blockIdx.x, S = p.S;
     const uint32_t ring = smem_u32(smem);

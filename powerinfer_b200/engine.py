@@ -189,7 +189,7 @@ class DecodeEngine:
 
     def prefill(self, tokens, seq: int = 0, pos0: int = 0, want_logits: bool = True):
         """Prompt processing: `tokens` are consecutive tokens of sequence `seq` starting at position pos0; they go through
-        in chunks of up to max_batch tokens per step.  Returns (logits of the last token | None, its greedy id | None)."""
+        in chunks of up to 256 tokens per step (max_batch in sharded runs).  Returns (logits of the last token | None, its greedy id | None)."""
         toks = np.ascontiguousarray(np.asarray(tokens, np.int32))
         logits = np.empty(self.spec.n_vocab, np.float32) if want_logits else None
         amax = np.zeros(1, np.int32)
