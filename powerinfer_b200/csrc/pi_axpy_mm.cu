@@ -14,8 +14,8 @@
 // (Expanding a stage into an FP16 tile in shared memory first costs two barriers per 16 rows: 159 us where this takes 82,
 // 103 MB of rows, 32 tokens.)
 //
-// Work split: units of 256 columns x 64 (128) list rows x up to 32 tokens, numbered slice by slice (a slice: 256 columns of one group of
-// 32 tokens; the groups of a column range follow one another, so that they find its rows in L2); every CTA takes an equal contiguous
+// Work split: units of 256 columns x 64 (128) list rows x up to 64 tokens, numbered slice by slice (a slice: 256 columns of one group of
+// tokens, equal groups: fragments are expanded once for all tokens of a group, 256 tokens of 70B shape in groups of 32 took 454 us where 64 take 355; the groups of a column range follow one another, so that they find its rows in L2); every CTA takes an equal contiguous
 // range, so the chip is full whatever the number of columns.  The CTAs that meet in a slice each write one partial vector
 // ("piece"); at most n_pieces of them per slice, the missing ones are written as zeros, and the norm (or the reduction)
 // that follows adds the pieces in order.  Rows arrive by 16-byte cp.async (they lie anywhere) from 8 producer warps; 8 consumer warps
@@ -29,6 +29,7 @@ namespace pi {
 
 static constexpr int AX_THREADS = 512, AX_CONS = 8, AX_PROD = 256, AX_CW = 256;      // warps 0 .. 7 consume, threads 256 .. 511 produce; columns of a unit
 static constexpr int AX_SMAX = 8;                        // stages at most
+static constexpr int AX_REGS_C = 200, AX_REGS_P = 56;    // 256 x (200 + 56) = the 512 x 128 of the launch
 static constexpr int AX_RED_PITCH = AX_CW + 4;           // conflict-free fragment stores
 static constexpr size_t AX_SMEM_MAX = 226 * 1024;
 
@@ -148,6 +149,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
 
     if (warp >= AX_CONS) {
         // ================================================================= producers: a row of the stage per TR threads
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(AX_REGS_P));
         const int pt = tid - AX_CONS * 32;
         constexpr int TR = AX_PROD / RS, PW = (Q4 ? 8 : 32) / TR;      // 16-byte pieces of a row slice per thread
         const int r = pt / TR, c0 = pt % TR;
@@ -179,7 +181,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
                 for (int j = 0; j < PW; j++) ax_cp16(base + r * Z::W_PITCH + (c0 + j * TR) * 16, at + j * TR * 16, live ? 16u : 0u);
                 if (c0 == 0) ax_cp16(base + r * Z::W_PITCH + 128, src + (size_t)p.nb * 16 + (size_t)cs * 16, live ? 16u : 0u);
             }
-            const int tok0 = tg * 32, Tg = min(32, p.T - tok0);
+            const int tok0 = tg * TP, Tg = min(TP, p.T - tok0);
 #pragma unroll
             for (int j = 0; j < NC; j++) {                            // coefficients; positions past the list count as 0
                 const int e = pt + j * AX_PROD, t = e / CPR, c = e % CPR, li = st * RS + c * CPP;
@@ -196,6 +198,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
         return;
     }
     // ===================================================================== consumers
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(AX_REGS_C));
     float acc[4][NT][4];
     auto clear = [&]() {
 #pragma unroll
@@ -268,10 +271,11 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
             if (NT == 1) ax_ldsm2(b[0][0], b[0][1], base + b_off + k * 32);
             else {
 #pragma unroll
-                for (int t = 0; t + 1 < NT; t += 2) {
+                for (int t = 0; t < NT; t += 2) {
                     uint32_t v[4];
-                    ax_ldsm4(v, base + b_off + t * 8 * Z::C_PITCH + k * 32);
-                    b[t][0] = v[0]; b[t][1] = v[1]; b[t + (NT > 1)][0] = v[2]; b[t + (NT > 1)][1] = v[3];
+                    ax_ldsm4(v, base + b_off + t * 8 * Z::C_PITCH + k * 32 - (t + 1 < NT ? 0u : ((lane >> 4) & 1) * 8 * Z::C_PITCH));   // (an odd last group is read twice)
+                    b[t][0] = v[0]; b[t][1] = v[1];
+                    if (t + 1 < NT) { b[(t + 1) % NT][0] = v[2]; b[(t + 1) % NT][1] = v[3]; }
                 }
             }
             if (!Q4) {
@@ -313,7 +317,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
         if (++slot == S) { slot = 0; phase ^= 1u; }
         if (st == nst - 1 || i == n_units - 1) {
             // ---- end of this CTA's share of the slice: the row halves are added in order
-            const int tok0 = tg * 32, Tg = min(32, p.T - tok0);
+            const int tok0 = tg * TP, Tg = min(TP, p.T - tok0);
 #pragma unroll 1
             for (int r = 0; r < 2; r++) {
                 if (wk == r) {
@@ -439,9 +443,16 @@ int launch_coef(const CoefArgs & a, cudaStream_t st) {
 
 // ---------------------------------------------------------------------------------------------- launch
 // At most 16 CTAs per slice (a partial vector each): more would cost the reader of the pieces more than they save.
+static int axpy_mm_group(int T) {                                      // tokens of a group: 8, 16, 32, or the equal share of up to 64 rounded up
+    if (T <= 32) return T <= 8 ? 8 : T <= 16 ? 16 : 32;
+    const int n = (T + 63) / 64, share = (T + n - 1) / n;
+    return share <= 40 ? 40 : share <= 48 ? 48 : 64;
+}
+
 static void axpy_mm_shape(int64_t ncols, int T, int * n_cs, int * n_tg, int * grid, int * n_pieces) {
+    const int group = axpy_mm_group(T);
     *n_cs = (int)((ncols + AX_CW - 1) / AX_CW);
-    *n_tg = (T + 31) / 32;
+    *n_tg = (T + group - 1) / group;
     const int n = *n_cs * *n_tg;
     *grid = (int)imin64(sm_count(), (int64_t)n * 16);
     *n_pieces = (*grid + n - 1) / n + 1;                              // ranges are not aligned to slices: one more than the quotient
@@ -470,7 +481,14 @@ static int axpy_mm_go(const AxpyMmP & p, int grid, bool pdl, cudaStream_t st) {
 
 template <int MODE>
 static int axpy_mm_tokens(const AxpyMmP & p, int grid, bool pdl, cudaStream_t st) {
-    return p.T <= 8 ? axpy_mm_go<MODE, 1>(p, grid, pdl, st) : p.T <= 16 ? axpy_mm_go<MODE, 2>(p, grid, pdl, st) : axpy_mm_go<MODE, 4>(p, grid, pdl, st);
+    switch (axpy_mm_group(p.T)) {
+        case 8:  return axpy_mm_go<MODE, 1>(p, grid, pdl, st);
+        case 16: return axpy_mm_go<MODE, 2>(p, grid, pdl, st);
+        case 32: return axpy_mm_go<MODE, 4>(p, grid, pdl, st);
+        case 40: return axpy_mm_go<MODE, 5>(p, grid, pdl, st);
+        case 48: return axpy_mm_go<MODE, 6>(p, grid, pdl, st);
+        default: return axpy_mm_go<MODE, 8>(p, grid, pdl, st);
+    }
 }
 
 // PI_ERR_UNSUPPORTED: shape not eligible, the caller uses the CUDA-core kernel.
