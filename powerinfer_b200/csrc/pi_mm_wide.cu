@@ -7,11 +7,11 @@
 // slower, 259 us where these take 208: packed operations have half the pipes, and every row scale needed a copy).
 // What must not cost extra is shared memory: every warp reads its own fragments of both operands.
 //
-// Work split: as in pi_mm.cu every CTA takes an equal contiguous range of rows, in tiles of 96, and producer warps (4) copy for the
+// Work split: as in pi_mm.cu every CTA takes an equal contiguous range of rows, in tiles of 192 (96), and producer warps (4) copy for the
 // consumers (12) (a computing warp that issues cp.async waits while the SM's queue of outstanding loads is full: 700 to 2900 of the
 // clocks of a stage).  Here all consumers share a stage (128 bytes of every activation, 128 or 64 of every row) and split the TILE:
-// no partial sums, so the accumulators of a tile exist once and the tile can be 96 x 256.  Up to 128 tokens 6 x 2 consumers of 16 rows,
-// beyond that 3 x 4 consumers of 32 rows; the token count of a consumer is a template argument in steps of 8 or 16, because a branch
+// no partial sums, so the accumulators of a tile exist once and the tile can be 96 x 256.  Up to 128 tokens 6 x 2 consumers, beyond that 3 x 4,
+// of 2 x 16 rows, the second of which a tile of up to half its height goes without; the token count of a consumer is a template argument in steps of 8 or 16, because a branch
 // around every pair of products costs more than the products that it leaves out.
 // Copies: the activations and dense rows come as TMA tiles (one instruction of one thread; with 16-byte cp.async the producers' own
 // instruction rate, 50 clocks per warp and copy, bound every launch of few rows), gathered rows and the Q4_0 rows' scales by cp.async.
@@ -20,12 +20,12 @@
 #include "pi_common.cuh"
 
 #include <cuda.h>
+#include <type_traits>
 
 namespace pi {
 
 static constexpr int MW_THREADS = 512, MW_CONS = 12, MW_PROD = 128;       // warps 0 .. 11 consume, threads 384 .. 511 produce
-static constexpr int MW_REGS_C = 160, MW_REGS_P = 32;   // 384 x 160 + 128 x 32 = the 512 x 128 of the launch
-static constexpr int MW_TM = 96;                        // rows of a tile
+static constexpr int MW_MT = 2;                         // fragments of 16 rows of a consumer
 static constexpr int MW_SMEM_MAX = 224 * 1024;          // (leaves room for the static variables)
 static constexpr int MW_SMAX = 6;                       // stages at most
 static constexpr int MW_TOKENS = 256;                   // of a launch
@@ -73,27 +73,29 @@ __device__ __forceinline__ void mw_scale_add(float & acc, uint32_t v, float dd, 
 template <int WT, int WM, int WN, int NT>
 struct MwShape {
     static constexpr bool Q4 = WT == PI_TYPE_Q4_0;
-    static constexpr int MT = MW_TM / 16 / WM, TN = WN * NT * 8;
+    static constexpr int TM = WM * MW_MT * 16, TN = WN * NT * 8;       // rows and tokens of a tile
+    // 384 consumers + 128 producers share the 512 x 128 registers of the launch; producers of 192 gathered rows keep 12 addresses each
+    static constexpr int REGS_C = WM == 6 ? 152 : 160, REGS_P = WM == 6 ? 56 : 32;
     static constexpr int KS = Q4 ? 128 : 64;                          // columns of a stage
     static constexpr int WB = Q4 ? 64 : 128;                          // bytes of a row in a stage (Q4_0: of its nibbles)
-    // a stage: rows [MW_TM][WB], activations [TN][128], Q4_0: rows' scales [MW_TM][4 halves], activation scales [4][TN] floats
+    // a stage: rows [TM][WB], activations [TN][128], Q4_0: rows' scales [TM][4 halves], activation scales [4][TN] floats
     // (Q4_0: low plane [TN][64], high plane [TN][64]; activation scales [TN][4]).  TMA writes and ldmatrix reads with the 16-byte pieces of a
     // row permuted by the row's number in groups of 8 (64-byte rows: pairs of rows in groups of 4), counted from 1024-byte boundaries.
-    static constexpr int X_OFF = MW_TM * WB, S_OFF = X_OFF + TN * 128, D_OFF = S_OFF + (Q4 ? MW_TM * 8 : 0), STAGE = (D_OFF + (Q4 ? TN * 16 : 0) + 1023) / 1024 * 1024;
-    static_assert(WM * WN == MW_CONS && MT * WM * 16 == MW_TM && X_OFF % 1024 == 0 && D_OFF % 128 == 0 && TN % 8 == 0 && TN <= 256, "split");
+    static constexpr int X_OFF = TM * WB, S_OFF = X_OFF + TN * 128, D_OFF = S_OFF + (Q4 ? TM * 8 : 0), STAGE = (D_OFF + (Q4 ? TN * 16 : 0) + 1023) / 1024 * 1024;
+    static_assert(WM * WN == MW_CONS && X_OFF % 1024 == 0 && D_OFF % 128 == 0 && TN % 8 == 0 && TN <= 256, "split");
 };
 
 template <int WT, int WM, int WN, int NT, bool SPARSE, bool GATED>
 __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant__ MwP p) {
     using Z = MwShape<WT, WM, WN, NT>;
     constexpr bool Q4 = Z::Q4;
-    constexpr int TM = MW_TM, WB = Z::WB, MT = Z::MT;
+    constexpr int TM = Z::TM, WB = Z::WB, MT = MW_MT;
     const int IT = GATED ? TM / 2 : SPARSE ? TM : p.per_tile;         // items (rows / neurons) of a tile
     constexpr bool COPIES = SPARSE || Q4;                             // some of a stage comes by cp.async
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     __shared__ int s_warp[MW_THREADS / 32];
-    __shared__ unsigned s_any[4];
+    __shared__ unsigned s_any[8];
     __shared__ uint64_t s_full[MW_SMAX], s_empty[MW_SMAX], s_bits[2];
     __shared__ volatile int s_dead;
     int * rows = reinterpret_cast<int *>(smem + (size_t)p.S * Z::STAGE);          // rows of this CTA (sparse only)
@@ -102,7 +104,7 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
     const int G = gridDim.x, cta = blockIdx.x, S = p.S;
     const uint32_t ring = smem_u32(smem);
     constexpr uint32_t x_off = Z::X_OFF, s_off = Z::S_OFF, d_off = Z::D_OFF;
-    if (tid < 4) s_any[tid] = 0u;
+    if (tid < 8) s_any[tid] = 0u;
     if (tid < MW_SMAX) { mbar_init(s_full + tid, COPIES ? MW_PROD + 1 : 1); mbar_init(s_empty + tid, MW_CONS); }
     if (tid == 0) { mbar_init(s_bits, MW_CONS); mbar_init(s_bits + 1, MW_CONS); s_dead = 0; }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -129,7 +131,7 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
     constexpr int NW = (TM * CW + MW_PROD - 1) / MW_PROD, WS = MW_PROD / CW;     // pieces of a thread, rows between them
     const int pt = tid - MW_CONS * 32;                              // producer thread
     const int cw = pt % CW;
-    const uint8_t * wp[NW]; const uint8_t * sp = nullptr;             // my pieces of the next slice
+    const uint8_t * wp[NW]; const uint8_t * sp[2] = {nullptr, nullptr};   // my pieces of the next slice; scales of rows pt, pt + 128
     unsigned w_ok = 0u;                                               // which of these rows exist
     int i_tile = 0, i_slice = 0;                                      // the unit that is requested next
     auto row_ptr = [&](int r, bool & ok) -> const uint8_t * {         // fragment row r of the tile (gated: 8 up rows, then their 8 gate rows)
@@ -149,10 +151,11 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
                 wp[j] = row_ptr(wr + j * WS, ok) + cw * 16;
                 if (ok) w_ok |= 1u << j;
             }
-            if (Q4) {
+#pragma unroll
+            for (int j = 0; j < (Q4 ? 2 : 0); j++) {
                 bool ok;
-                sp = row_ptr(pt, ok) + (size_t)p.nb * 16;
-                if (ok) w_ok |= 1u << NW;
+                sp[j] = row_ptr(pt + j * MW_PROD, ok) + (size_t)p.nb * 16;
+                if (ok) w_ok |= 1u << (NW + j);
             }
         }
         const uint32_t base = ring + (uint32_t)(slot * Z::STAGE);
@@ -163,9 +166,10 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
             if (w_ok >> j & 1u) { if (in) mw_cp16(to, wp[j]); else mw_zero16(to); }
             wp[j] += WB;
         }
-        if (Q4) {
-            if (w_ok >> NW & 1u) mw_cp8(base + s_off + pt * 8, sp);
-            sp += 8;
+#pragma unroll
+        for (int j = 0; j < (Q4 ? 2 : 0); j++) {
+            if (w_ok >> (NW + j) & 1u) mw_cp8(base + s_off + (pt + j * MW_PROD) * 8, sp[j]);
+            sp[j] += 8;
         }
     };
     auto issue_tma = [&](int slot) {                                  // one thread
@@ -238,7 +242,7 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
     }
     if (warp >= MW_CONS) {
         // ================================================================= producers
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(MW_REGS_P));
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(Z::REGS_P));
         int slot = 0;
         unsigned phase = 1u;                                          // parity of the hand-back to wait for (first round: none)
         if (!COPIES && warp > MW_CONS) return;
@@ -259,7 +263,7 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
         return;
     }
     // ===================================================================== consumers
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(MW_REGS_C));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(Z::REGS_C));
     float acc[MT][NT][4];
     auto clear = [&]() {
 #pragma unroll
@@ -274,9 +278,14 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
     uint32_t MAGIC[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) asm volatile("mov.u32 %0, 0x4B400000;" : "=r"(MAGIC[j]));
-    const int row0 = wm * MT * 16, tok0 = wn * NT * 8;                // this warp's part of the tile
+    // This warp's part of the tile: 16 rows from row0 and 16 from row0 + MS.  6 consumers along the rows: the second fragments lie above all
+    // first ones, and a tile of up to 96 rows has none (104 gathered rows are one tile instead of a whole one and a nearly empty one).
+    // 3 consumers: neighbours, so that 56 rows are two consumers' work and not three's; always multiplied.
+    constexpr bool APART = WM == 6;
+    constexpr int MS = APART ? WM * 16 : 16;
+    const int row0 = wm * (APART ? 16 : 32), tok0 = wn * NT * 8;
     // ldmatrix row addresses inside a stage (fragment layouts of mma.m16n8k16 / m16n8k32); the piece is added per step
-    const uint32_t a_row = (uint32_t)((row0 + (Q4 && MT == 2 ? lane : lane & 15)) * WB);
+    const uint32_t a_row = (uint32_t)((row0 + (lane & 15) + (Q4 ? (lane >> 4) * MS : 0)) * WB);
     constexpr int XB = Q4 ? 64 : 128;                                 // bytes of a token (Q4_0: of a plane)
     const uint32_t plane = Q4 ? ((lane >> 3) & 1) * Z::TN * 64 : 0;
     const uint32_t b_row = x_off + plane + (uint32_t)((tok0 + (lane & 7) + (lane >> 4) * 8) * XB), b_last = x_off + plane + (uint32_t)((tok0 + (NT - 1) * 8 + (lane & 7)) * XB);
@@ -289,73 +298,74 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
         const uint32_t base = ring + (uint32_t)(slot * Z::STAGE);
         const int n_tile = min(IT, hi - lo - tile * IT);              // items
         const bool busy = (GATED ? row0 / 2 : row0) < n_tile && tok0 < p.T;       // my rows and tokens exist
-        if (!busy) {
-        } else if (!Q4) {
+        auto multiply = [&](auto mc) {                                // MC fragments of 16 rows
+            constexpr int MC = decltype(mc)::value;
+            if (!Q4) {
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                uint32_t a[MT][4];
+                for (int k = 0; k < 4; k++) {
+                    uint32_t a[MC][4];
 #pragma unroll
-                for (int m = 0; m < MT; m++) mw_ldsm4(a[m], base + a_row + m * 16 * WB + (((2 * k + (lane >> 4)) ^ a_swz) & 7) * 16);
+                    for (int m = 0; m < MC; m++) mw_ldsm4(a[m], base + a_row + m * MS * WB + (((2 * k + (lane >> 4)) ^ a_swz) & 7) * 16);
 #pragma unroll
-                for (int n = 0; n < NT; n += 2) {
-                    uint32_t b[4];
-                    mw_ldsm4(b, base + (n + 1 < NT ? b_row + n * 8 * XB : b_last) + (((2 * k + ((lane >> 3) & 1)) ^ b_swz) & 7) * 16);
+                    for (int n = 0; n < NT; n += 2) {
+                        uint32_t b[4];
+                        mw_ldsm4(b, base + (n + 1 < NT ? b_row + n * 8 * XB : b_last) + (((2 * k + ((lane >> 3) & 1)) ^ b_swz) & 7) * 16);
 #pragma unroll
-                    for (int m = 0; m < MT; m++) {
-                        mw_hmma(acc[m][n], a[m], b[0], b[1]);
-                        if (n + 1 < NT) mw_hmma(acc[m][(n + 1) % NT], a[m], b[2], b[3]);
+                        for (int m = 0; m < MC; m++) {
+                            mw_hmma(acc[m][n], a[m], b[0], b[1]);
+                            if (n + 1 < NT) mw_hmma(acc[m][(n + 1) % NT], a[m], b[2], b[3]);
+                        }
                     }
                 }
-            }
-        } else {
-            uint32_t w1[4];
+            } else {
 #pragma unroll
-            for (int k = 0; k < (Q4 ? 4 : 0); k++) {                  // block by block
-                uint32_t w[4];
-                if (MT == 2) {
+                for (int k = 0; k < (Q4 ? 4 : 0); k++) {              // block by block
+                    uint32_t w[4], a[MC][4];
                     mw_ldsm4(w, base + a_row + ((k ^ a_swz) & 3) * 16);
-                } else {                                              // 16 rows: two blocks at a time
-                    if (!(k & 1)) mw_ldsm4(w1, base + a_row + (((k + (lane >> 4)) ^ ((lane & 7) >> 1)) & 3) * 16);
-                    w[0] = w1[2 * (k & 1)]; w[1] = w1[2 * (k & 1) + 1]; w[2] = w[3] = 0u;
-                }
-                uint32_t a[MT][4];
-                float d4[MT][2];                                      // (the nibbles stand for 16 times their value)
+                    float d4[MC][2];                                  // (the nibbles stand for 16 times their value)
 #pragma unroll
-                for (int m = 0; m < MT; m++) {
-                    const uint32_t w0 = w[2 * m], wh = w[2 * m + 1];
-                    a[m][0] = ((w0 << 4) & 0xF0F0F0F0u) ^ 0x80808080u; a[m][1] = ((wh << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
-                    a[m][2] = (w0 & 0xF0F0F0F0u) ^ 0x80808080u;        a[m][3] = (wh & 0xF0F0F0F0u) ^ 0x80808080u;
+                    for (int m = 0; m < MC; m++) {
+                        const uint32_t w0 = w[2 * m], wh = w[2 * m + 1];
+                        a[m][0] = ((w0 << 4) & 0xF0F0F0F0u) ^ 0x80808080u; a[m][1] = ((wh << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
+                        a[m][2] = (w0 & 0xF0F0F0F0u) ^ 0x80808080u;        a[m][3] = (wh & 0xF0F0F0F0u) ^ 0x80808080u;
 #pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        unsigned short s;
-                        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(s) : "r"(base + s_off + (row0 + m * 16 + g + h * 8) * 8 + k * 2));
-                        d4[m][h] = __half2float(__ushort_as_half(s)) * 0.0625f;
+                        for (int h = 0; h < 2; h++) {
+                            unsigned short s;
+                            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(s) : "r"(base + s_off + (row0 + m * MS + g + h * 8) * 8 + k * 2));
+                            d4[m][h] = __half2float(__ushort_as_half(s)) * 0.0625f;
+                        }
                     }
-                }
 #pragma unroll
-                for (int n = 0; n < NT; n += 2) {
-                    uint32_t b[4];
-                    mw_ldsm4(b, base + (n + 1 < NT ? b_row + n * 8 * XB : b_last) + ((k ^ b_swz) & 3) * 16);
+                    for (int n = 0; n < NT; n += 2) {
+                        uint32_t b[4];
+                        mw_ldsm4(b, base + (n + 1 < NT ? b_row + n * 8 * XB : b_last) + ((k ^ b_swz) & 3) * 16);
 #pragma unroll
-                    for (int u = 0; u < 2; u++) {
-                        if (n + u >= NT) break;
-                        float t0, t1;                                 // scales of tokens 2q, 2q + 1
-                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t0) : "r"(base + d_off + (tok0 + (n + u) * 8 + 2 * q) * 16 + k * 4));
-                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t1) : "r"(base + d_off + (tok0 + (n + u) * 8 + 2 * q + 1) * 16 + k * 4));
-                        const float m0 = t0 * -12582912.0f, m1 = t1 * -12582912.0f;
+                        for (int u = 0; u < 2; u++) {
+                            if (n + u >= NT) break;
+                            float t0, t1;                             // scales of tokens 2q, 2q + 1
+                            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t0) : "r"(base + d_off + (tok0 + (n + u) * 8 + 2 * q) * 16 + k * 4));
+                            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t1) : "r"(base + d_off + (tok0 + (n + u) * 8 + 2 * q + 1) * 16 + k * 4));
+                            const float m0 = t0 * -12582912.0f, m1 = t1 * -12582912.0f;
 #pragma unroll
-                        for (int m = 0; m < MT; m++) {
-                            uint32_t c[4];
-                            mw_imma(c, a[m], b[2 * u], b[2 * u + 1], MAGIC);
-                            float (&o)[4] = acc[m][(n + u) % NT];
-                            mw_scale_add(o[0], c[0], t0, m0, d4[m][0]);
-                            mw_scale_add(o[1], c[1], t1, m1, d4[m][0]);
-                            mw_scale_add(o[2], c[2], t0, m0, d4[m][1]);
-                            mw_scale_add(o[3], c[3], t1, m1, d4[m][1]);
+                            for (int m = 0; m < MC; m++) {
+                                uint32_t c[4];
+                                mw_imma(c, a[m], b[2 * u], b[2 * u + 1], MAGIC);
+                                float (&o)[4] = acc[m][(n + u) % NT];
+                                mw_scale_add(o[0], c[0], t0, m0, d4[m][0]);
+                                mw_scale_add(o[1], c[1], t1, m1, d4[m][0]);
+                                mw_scale_add(o[2], c[2], t0, m0, d4[m][1]);
+                                mw_scale_add(o[3], c[3], t1, m1, d4[m][1]);
+                            }
                         }
                     }
                 }
             }
+        };
+        if (!busy) {
+        } else if (!APART || (GATED ? MS / 2 : MS) < n_tile) {
+            multiply(std::integral_constant<int, 2>());
+        } else {
+            multiply(std::integral_constant<int, APART ? 1 : 2>());
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(s_empty + slot);                   // handed back
@@ -367,7 +377,7 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
                 for (int m = 0; m < MT; m++) {
 #pragma unroll
                     for (int h = 0; h < (GATED ? 1 : 2); h++) {
-                        const int k = GATED ? (row0 + m * 16) / 2 + g : row0 + m * 16 + g + h * 8;     // item of the tile
+                        const int k = GATED ? (row0 + m * MS) / 2 + g : row0 + m * MS + g + h * 8;     // item of the tile
                         bool any = false;
                         if (k < n_tile) {
                             const int item = lo + tile * IT + k;
@@ -408,7 +418,7 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
                     *o = p.masks_or ? (unsigned char)(*o | bits) : bits;
                 }
                 __syncwarp();
-                if (tid < 4) s_any[tid] = 0u;
+                if (tid < 8) s_any[tid] = 0u;
                 __syncwarp();
                 if (lane == 0) mbar_arrive(s_bits + 1);
                 if (!wait(s_bits + 1, (unsigned)tile & 1u)) break;
@@ -454,9 +464,9 @@ static int mw_go(MwP p, bool pdl, cudaStream_t st) {
     p.per_tile = 0;
     int rc;
     if (!SPARSE) {                                                    // equal tiles; whole bytes of the masks
-        const int share = (p.nrows + G - 1) / G + (p.masks_out ? 8 : 0), tiles = (share + MW_TM - 1) / MW_TM;
+        const int share = (p.nrows + G - 1) / G + (p.masks_out ? 8 : 0), tiles = (share + Z::TM - 1) / Z::TM;
         p.per_tile = p.masks_out ? (share / tiles + 8) / 8 * 8 : (share + tiles - 1) / tiles;
-        if (p.per_tile > MW_TM) p.per_tile = MW_TM;
+        if (p.per_tile > Z::TM) p.per_tile = Z::TM;
         if (Z::Q4) rc = mw_map(&p.m_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.W, (int64_t)p.nb * 16, p.nrows, p.row_bytes, 64, p.per_tile, CU_TENSOR_MAP_SWIZZLE_64B);
         else       rc = mw_map(&p.m_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, p.W, p.ncols, p.nrows, p.row_bytes, 64, p.per_tile, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc != PI_OK) return rc;
