@@ -8,7 +8,7 @@
 // Bound: the bytes of the cached rows for batches, the chain scores -> maximum -> probabilities -> values for chunks.
 // Scores: mma.m16n8k16 with the keys straight from global memory: a lane loads 16 bytes (8 columns) of a row, which serve
 // as B operands of two mma whose k order is permuted in the same way on the query side; four tiles of 8 positions in
-// flight per warp.  Values travel to shared memory by cp.async (tiles of 64 positions, two in flight) while the scores are made and
+// flight per warp, or two where more than two CTAs per SM have work (attn_mm_go).  Values travel to shared memory by cp.async (tiles of 64 positions, two in flight) while the scores are made and
 // are read transposed.  Every CTA rotates and stores the new keys and values it reads itself (CTAs that share a KV head store the
 // same bits), so no store pass runs before a chunk of up to AM_OWN_STORE tokens; beyond that the repeated work costs more than a launch.
 // Numerics follow the CPU path as in k_attention: q, k, v and the probabilities in FP16, exp through FP16, the normaliser
@@ -35,8 +35,8 @@ __device__ __forceinline__ void am_mma(float (&c)[4], uint32_t a0, uint32_t a1, 
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-template <int HC>                                                     // head_dim / 32
-__global__ void __launch_bounds__(AM_THREADS) k_attention_mm(const AttnMmP p) {
+template <int HC, int UN>                                             // head_dim / 32; tiles of 8 positions in flight per warp
+__global__ void __launch_bounds__(AM_THREADS, UN == 2 ? 4 : HC == 2 ? 3 : 2) k_attention_mm(const AttnMmP p) {
     constexpr int HD = HC * 32, HALF = HD / 2;
     constexpr int V_PITCH = HD + 8, Q_PITCH = HD + 8;                 // halves; odd multiples of 16 bytes
     constexpr int NWC = HD / 16 < AM_WARPS ? HD / 16 : AM_WARPS;      // warps along the value columns, the rest split the positions
@@ -144,7 +144,6 @@ __global__ void __launch_bounds__(AM_THREADS) k_attention_mm(const AttnMmP p) {
             }
         const float scale = 1.0f / sqrtf((float)HD);
         const int n_tiles = (n_keys + 7) / 8;
-        constexpr int UN = HC <= 4 ? 4 : 2;                           // tiles of 8 positions in flight
         for (int nt0 = warp; nt0 < n_tiles; nt0 += AM_WARPS * UN) {
             uint4 kv[UN][HC];
 #pragma unroll
@@ -299,16 +298,20 @@ bool attention_mm_takes(const AttnArgs & a) {
     return a.T >= 2 && (a.head_dim == 64 || a.head_dim == 128) && a.n_ctx > 0 && attn_mm_smem(a, &P, &R) <= AM_SMEM_MAX;
 }
 
-template <int HC>
+// UN = 4 takes 126 registers with head_dim 128, two CTAs per SM.  Where the grid and shared memory give an SM more than two, half
+// the tiles in 64 registers let four run side by side, so that one's softmax covers the others' loads: eight layers of 32 sequences
+// of 191 positions with 32 heads, 1024 CTAs of 42 KB: 1318 -> 1236 us per pass (one tile 1275 us, three CTAs 1282 us).  A grid that
+// two CTAs per SM hold at once has no use for more and loses the loads in flight: 64 CTAs, 557 -> 570 us per pass.
+template <int HC, int UN>
 static int attn_mm_go(const AttnMmP & p, dim3 grid, size_t smem, bool pdl, cudaStream_t st) {
     static bool attr_done[16] = {false};
     int dev = 0;
     PI_CUDA(cudaGetDevice(&dev));
     if (dev >= 0 && dev < 16 && !attr_done[dev]) {
-        PI_CUDA(cudaFuncSetAttribute(k_attention_mm<HC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AM_SMEM_MAX));
+        PI_CUDA(cudaFuncSetAttribute(k_attention_mm<HC, UN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AM_SMEM_MAX));
         attr_done[dev] = true;
     }
-    PI_CUDA(launch_k(k_attention_mm<HC>, grid, dim3(AM_THREADS), smem, st, pdl, p));
+    PI_CUDA(launch_k(k_attention_mm<HC, UN>, grid, dim3(AM_THREADS), smem, st, pdl, p));
     return PI_OK;
 }
 
@@ -325,7 +328,8 @@ int launch_attention_mm(const AttnArgs & a, cudaStream_t st) {
     const size_t smem = attn_mm_smem(a, &p.P, &p.R);
     if (p.stored) PI_CUDA(launch_k(k_kv_store, dim3((unsigned)((a.n_head_kv * a.head_dim / 2 + 255) / 256), a.T), dim3(256), 0, st, a.pdl, p, a.head_dim));
     const dim3 grid = p.chunk ? dim3(a.n_head, (a.T + 15) / 16) : dim3(a.n_head_kv * ((a.n_head / a.n_head_kv + 15) / 16), a.T);
-    return a.head_dim == 64 ? attn_mm_go<2>(p, grid, smem, a.pdl, st) : attn_mm_go<4>(p, grid, smem, a.pdl, st);
+    if (a.head_dim == 64) return attn_mm_go<2, 4>(p, grid, smem, a.pdl, st);
+    return smem <= AM_SMEM_MAX / 3 && (int64_t)grid.x * grid.y > 2 * sm_count() ? attn_mm_go<4, 2>(p, grid, smem, a.pdl, st) : attn_mm_go<4, 4>(p, grid, smem, a.pdl, st);
 }
 
 }  // namespace pi

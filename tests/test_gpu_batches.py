@@ -91,6 +91,35 @@ def test_axpy(wtype, rows, cols):
             assert ((got - c @ w).abs() <= per_term * mass + 1e-30).all(), T
 
 
+@pytest.mark.parametrize("heads,kv,hd", [(8, 2, 128), (9, 9, 128), (20, 20, 128), (34, 2, 128), (40, 40, 64)])
+def test_attention_of_a_batch(heads, kv, hd):
+    """Up to 32 sequences at different positions, CTAs for one and for several per SM.  With x = maximum - score, the kernel rounds x, exp(-x)
+    and the probability to FP16 (2^-11 x, 2^-11, 2^-11 and 2^-25 for subnormals), and the normaliser carries the same errors averaged:
+    |error| <= sum p (x + mean x + 5) 2^-11 |v| + 2^-24 sum |v|, the 5 with one unit for what FP32 sums and second-order terms add."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from powerinfer_b200 import ggml_ops as ops
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(heads)
+    n_ctx, S = 160, 32
+    for T in (2, 8, 32):
+        kc = torch.randn(S, n_ctx, kv * hd, device="cuda", generator=gen).half()
+        vc = torch.randn(S, n_ctx, kv * hd, device="cuda", generator=gen).half()
+        q = torch.randn(T, heads * hd, device="cuda", generator=gen)
+        k, v = (torch.randn(T, kv * hd, device="cuda", generator=gen) for _ in range(2))
+        seq = torch.randperm(S, device="cuda", generator=gen)[:T].int()
+        pos = torch.tensor([(0, 7, 63, 64, 130, 159)[t % 6] for t in range(T)], dtype=torch.int32, device="cuda")
+        got = ops.attention_decode(q, k, v, kc, vc, pos, heads, kv, seq=seq).double().view(T, heads, hd)
+        for t in range(T):
+            s, n = int(seq[t]), int(pos[t]) + 1
+            assert torch.equal(kc[s, n - 1], k[t].half()) and torch.equal(vc[s, n - 1], v[t].half())
+            K, V = (c[s, :n].double().view(n, kv, hd).repeat_interleave(heads // kv, 1) for c in (kc, vc))
+            sc = torch.einsum("hd,nhd->hn", q[t].half().double().view(heads, hd), K) / hd ** 0.5
+            p, x = sc.softmax(1), sc.max(1, keepdim=True)[0] - sc
+            w = p * (x + (p * x).sum(1, keepdim=True) + 5) * 2.0 ** -11 + 2.0 ** -24
+            assert ((got[t] - torch.einsum("hn,nhd->hd", p, V)).abs() <= torch.einsum("hn,nhd->hd", w, V.abs())).all(), (T, t)
+
+
 @pytest.mark.parametrize("arch,wtype,heads,kv,d", [(synth.ARCH_LLAMA, synth.F16, 8, 2, 512), (synth.ARCH_LLAMA, synth.Q4_0, 4, 4, 512), (synth.ARCH_OPT, synth.F16, 4, 4, 512),
                                                    (synth.ARCH_FALCON, synth.Q4_0, 32, 1, 2048), (synth.ARCH_LLAMA, synth.F16, 16, 16, 512)])
 def test_prompt_chunks(arch, wtype, heads, kv, d):
