@@ -357,7 +357,11 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
 // h F32 [T, h_stride] (by global neuron id) -> coef [T, coef_stride] by list position: FP16(h), or for Q4_0 rows the int8
 // quant of h in its block of 32 neurons times that block's FP16 scale (ggml.c:14575-14581, quantize_row_q8_0), rounded to FP16
 // or (exact mode) as it is, in F32; 0 where the token is inactive.  One warp per 32 local rows (one word of the union masks); a
-// CTA counts the rows named by the words before its own to find its list positions, and writes its part of the list.
+// CTA takes 8 tokens, counts the rows named by the words before its own to find its list positions, and writes its part of the list.
+// Bound: the latency from the wait to the stores.  The hidden values are loaded before the count, whether the word names a row or
+// not, the count meets at one barrier, and the eight tokens' maxima and quotients run side by side: eight tokens, 28672 rows, 3 layers
+// 556 -> 543 us per pass; 16 tokens, 13824 rows 77.0 -> 73.5 us; 256 tokens, 28672 rows, 3 layers 5143 -> 5116 us.  (CTAs with several
+// groups of 8 tokens, which count once, took 5150 .. 5200 us.)
 struct CoefP {
     const float * h; int64_t h_stride; const float * idx; int64_t idx_stride; float threshold;
     const int32_t * bucket; const uint32_t * masks; int32_t * list; int32_t * count; int n_local, T;
@@ -367,65 +371,68 @@ struct CoefP {
 
 template <bool Q4>
 __global__ void __launch_bounds__(256) k_coef(const CoefP p) {
-    __shared__ int s_sum[8];
+    __shared__ int s_pre[8], s_cnt[8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_chunks = (p.n_local + 31) / 32;
-    const int c = blockIdx.x * 8 + warp;
+    const int c = blockIdx.x * 8 + warp, r = c * 32 + lane;
+    const bool in = r < p.n_local;
+    const int64_t g = in ? (p.bucket ? p.bucket[r] : r) : 0;
+    const float fill = Q4 && p.h_uncleared && p.fill_bias && in ? fmaxf(p.fill_bias[g], 0.f) : 0.f;
+    constexpr int UN = 8;
     pdl_launch();
     pdl_wait();
-    int sum = 0;
-    for (int k = tid; k < (int)blockIdx.x * 8; k += 256) sum += __popc(__ldcg(p.masks + k));
     uint32_t m = c < n_chunks ? __ldcg(p.masks + c) : 0u;
+    const int t0 = blockIdx.y * UN;
+    float v[UN], l[UN];                                               // (on their way while the positions are counted)
+#pragma unroll
+    for (int u = 0; u < UN; u++) {
+        v[u] = 0.f; l[u] = 0.f;
+        if (in && t0 + u < p.T) { v[u] = p.h[(size_t)(t0 + u) * p.h_stride + g]; l[u] = p.idx[(size_t)(t0 + u) * p.idx_stride + g]; }
+    }
+    int sum = 0;
+#pragma unroll 4
+    for (int k = tid; k < (int)blockIdx.x * 8; k += 256) sum += __popc(__ldcg(p.masks + k));
     const int left = p.n_local - c * 32;                              // bits beyond the last row never count
     if (left < 32) m &= left <= 0 ? 0u : (1u << left) - 1u;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (lane == 0) s_sum[warp] = sum;
+    if (lane == 0) { s_pre[warp] = sum; s_cnt[warp] = __popc(m); }
     __syncthreads();
-    int base = 0;
+    int base = 0, total = 0;
 #pragma unroll
-    for (int w = 0; w < 8; w++) base += s_sum[w];
-    __syncthreads();
-    if (lane == 0) s_sum[warp] = __popc(m);
-    __syncthreads();
-    int total = base;
-#pragma unroll
-    for (int w = 0; w < 8; w++) { if (w < warp) base += s_sum[w]; total += s_sum[w]; }
+    for (int w = 0; w < 8; w++) { base += s_pre[w] + (w < warp ? s_cnt[w] : 0); total += s_pre[w] + s_cnt[w]; }
     if (blockIdx.x == gridDim.x - 1 && blockIdx.y == 0 && tid == 0) *p.count = total;
     if (m == 0u) return;
     const int pos = base + __popc(m & ((1u << lane) - 1u));
     const bool mine = m >> lane & 1u;
-    const int r = c * 32 + lane;
-    const bool in = r < p.n_local;
     if (mine && blockIdx.y == 0) p.list[pos] = r;
-    const int64_t g = in ? (p.bucket ? p.bucket[r] : r) : 0;
-    const float fill = Q4 && p.h_uncleared && p.fill_bias && in ? fmaxf(p.fill_bias[g], 0.f) : 0.f;
-    constexpr int UN = 8;
-    for (int t0 = blockIdx.y * UN; t0 < p.T; t0 += gridDim.y * UN) {
-        float v[UN], l[UN];
+    float o[UN];                                                      // (tokens beyond T too: no branch keeps the eight chains apart)
+#pragma unroll
+    for (int u = 0; u < UN; u++) {
+        const bool on = in && !(l[u] < p.threshold);                  // (a NaN logit counts as active)
+        if (!Q4) { o[u] = on ? v[u] : 0.f; continue; }
+        o[u] = on || !p.h_uncleared ? v[u] : fill;                    // what the graph leaves at an inactive neuron
+    }
+    if (Q4) {
+        float amax[UN];
+#pragma unroll
+        for (int u = 0; u < UN; u++) amax[u] = fabsf(o[u]);
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1)
+#pragma unroll
+            for (int u = 0; u < UN; u++) amax[u] = fmaxf(amax[u], __shfl_xor_sync(0xffffffffu, amax[u], s));
 #pragma unroll
         for (int u = 0; u < UN; u++) {
-            v[u] = 0.f; l[u] = 0.f;
-            if (in && t0 + u < p.T) { v[u] = p.h[(size_t)(t0 + u) * p.h_stride + g]; l[u] = p.idx[(size_t)(t0 + u) * p.idx_stride + g]; }
+            const float id = amax[u] != 0.0f ? 127.0f / amax[u] : 0.0f;
+            const float q = (float)__float2int_rn(o[u] * id) * round_f16(amax[u] / 127.0f);
+            o[u] = in && !(l[u] < p.threshold) ? q : 0.f;
         }
+    }
+    if (!mine) return;
 #pragma unroll
-        for (int u = 0; u < UN; u++) {
-            const int t = t0 + u;
-            if (t >= p.T) break;
-            const bool on = in && !(l[u] < p.threshold);              // (a NaN logit counts as active)
-            float o;
-            if (!Q4) {
-                o = on ? v[u] : 0.f;
-            } else {
-                const float x = on || !p.h_uncleared ? v[u] : fill;   // what the graph leaves at an inactive neuron
-                const float amax = warp_max(fabsf(x));
-                const float id = amax != 0.0f ? 127.0f / amax : 0.0f;
-                o = on ? (float)__float2int_rn(x * id) * round_f16(amax / 127.0f) : 0.f;
-            }
-            if (mine) {
-                if (Q4 && p.exact) reinterpret_cast<float *>(p.coef)[(size_t)t * p.coef_stride + pos] = o;
-                else reinterpret_cast<__half *>(p.coef)[(size_t)t * p.coef_stride + pos] = __float2half_rn(o);
-            }
-        }
+    for (int u = 0; u < UN; u++) {
+        if (t0 + u >= p.T) break;
+        if (Q4 && p.exact) reinterpret_cast<float *>(p.coef)[(size_t)(t0 + u) * p.coef_stride + pos] = o[u];
+        else reinterpret_cast<__half *>(p.coef)[(size_t)(t0 + u) * p.coef_stride + pos] = __float2half_rn(o[u]);
     }
 }
 
