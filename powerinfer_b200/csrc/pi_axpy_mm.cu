@@ -4,11 +4,10 @@
 // of down_t read transposed, B = the coefficients, laid out by list position so that they load like a matrix.
 //   FP16 rows: coef = FP16(h) of a token's active rows, else 0; the products of two halves are exact, sums are FP32, as on
 //              the CPU.
-//   Q4_0 rows, columns a multiple of 1024: weight FP16(d * (q - 8)) (one rounding: q - 8 is exact), coef = FP16(b8 * d8) of the
-//              CPU path's int8 x scale pair: two roundings to 11 bits that the CPU path does not have, relative error <= 5e-4
-//              per term.
-//   Q4_0 rows, other widths: exact.  A = q - 8 (an integer, exact in BF16), B = b8 * d8 * d of a column block as the sum of
-//              three BF16 numbers (24 bits, FP32's exponent range): three mma for one, so three times the tensor time.
+//   Q4_0 rows, rounded: weight FP16(d * (q - 8)) (one rounding: q - 8 is exact), coef = FP16(b8 * d8) of the CPU path's int8 x
+//              scale pair: two roundings to 11 bits that the CPU path does not have, relative error up to 2^-10 per term.
+//   Q4_0 rows, exact: A = q - 8 (an integer, exact in BF16), B = b8 * d8 * d of a column block as the sum of
+//              three BF16 numbers (24 bits, FP32's exponent range): three mma for one.  axpy_mm_exact says which.
 // The nibbles become fragments in registers: a lane takes the same 4-byte word of two neighbouring rows, and one byte permute
 // and one logic operation make the pair {1024 + q of row r, 1024 + q of row r + 1} of a column, in the fragment's k order.
 // (Expanding a stage into an FP16 tile in shared memory first costs two barriers per 16 rows: 159 us where this takes 82,
@@ -465,8 +464,13 @@ static void axpy_mm_shape(int64_t ncols, int T, int * n_cs, int * n_tg, int * gr
     *n_pieces = (*grid + n - 1) / n + 1;                              // ranges are not aligned to slices: one more than the quotient
 }
 
-// Q4_0 rows whose width is no multiple of 1024 take exact coefficients (F32): see the top of the file
-bool axpy_mm_exact(int wtype, int64_t ncols) { return wtype == PI_TYPE_Q4_0 && ncols % 1024 != 0; }
+// Which Q4_0 batches keep the CPU path's FP32 factors.  This is a promise about precision, not a matter of what the kernel can do: steps
+// of 2..32 tokens over matrices of whole 1024 columns and at most 2^28 weights round weight and coefficient to FP16, everything else
+// is exact.  Rounding buys (exact -> rounded) three layers of 28672 x 8192 and 8 tokens 576 -> 541 us per pass, a layer of 13824 x 5120
+// and 16 tokens 85.9 -> 73.7 us.  A prompt keeps the factors that steps of the engine's batch have: exact where it takes one sequence.
+bool axpy_mm_exact(int wtype, int64_t nrows, int64_t ncols, int T) {
+    return wtype == PI_TYPE_Q4_0 && (T < 2 || T > 32 || ncols % 1024 != 0 || nrows * ncols > (int64_t)1 << 28);
+}
 
 int axpy_mm_pieces(int64_t ncols, int T) { int cs, tg, g, np; axpy_mm_shape(ncols, T, &cs, &tg, &g, &np); return np; }
 
@@ -500,7 +504,7 @@ static int axpy_mm_tokens(const AxpyMmP & p, int grid, bool pdl, cudaStream_t st
 
 // PI_ERR_UNSUPPORTED: shape not eligible, the caller uses the CUDA-core kernel.
 int launch_axpy_mm(const AxpyArgs & a, cudaStream_t st, int * pieces_used) {
-    const bool q4 = a.wtype == PI_TYPE_Q4_0, exact = axpy_mm_exact(a.wtype, a.ncols);
+    const bool q4 = a.wtype == PI_TYPE_Q4_0;
     if (!a.coef || a.coef_stride % 8 != 0 || !a.list || (q4 ? a.ncols % 256 != 0 : a.ncols % 8 != 0)) return PI_ERR_UNSUPPORTED;
     AxpyMmP p;
     int grid;
@@ -509,7 +513,7 @@ int launch_axpy_mm(const AxpyArgs & a, cudaStream_t st, int * pieces_used) {
     p.Wt = (const uint8_t *)a.Wt; p.row_bytes = (int64_t)pi_row_bytes(a.wtype, a.ncols); p.nrows = (int)a.nrows; p.ncols = (int)a.ncols;
     p.nb = (int)(a.ncols / 32); p.T = a.T; p.list = a.list; p.count = a.count; p.coef = a.coef; p.coef_stride = a.coef_stride; p.partial = a.partial; p.status = a.status;
     if (pieces_used) *pieces_used = p.n_pieces;
-    return exact ? axpy_mm_tokens<AX_Q4_EXACT>(p, grid, a.pdl, st) : q4 ? axpy_mm_tokens<AX_Q4>(p, grid, a.pdl, st) : axpy_mm_tokens<AX_F16>(p, grid, a.pdl, st);
+    return q4 && a.exact ? axpy_mm_tokens<AX_Q4_EXACT>(p, grid, a.pdl, st) : q4 ? axpy_mm_tokens<AX_Q4>(p, grid, a.pdl, st) : axpy_mm_tokens<AX_F16>(p, grid, a.pdl, st);
 }
 
 }  // namespace pi

@@ -231,7 +231,8 @@ int pi_axpy(int wtype, const void * Wt, int64_t n_w_rows, int64_t ncols,
     Scratch s(workspace, workspace_bytes);
     SparseScratch ss;
     const int G = axpy_groups(wtype, ncols, T);
-    bool ok = aligned(workspace, 256) && carve_sparse(s, n_w_rows, T, axpy_mm_exact(wtype, ncols) ? 4 : 2, ss);
+    const bool exact = axpy_mm_exact(wtype, n_w_rows, ncols, T);
+    bool ok = aligned(workspace, 256) && carve_sparse(s, n_w_rows, T, exact ? 4 : 2, ss);
     int8_t * cq = nullptr; float * cd = nullptr;
     if (ok && wtype == PI_TYPE_Q4_0 && T == 1) {
         cq = (int8_t *)s.take((size_t)h_stride);
@@ -258,9 +259,9 @@ int pi_axpy(int wtype, const void * Wt, int64_t n_w_rows, int64_t ncols,
         k.pdl = true;
         k.wtype = wtype; k.h = h; k.h_stride = h_stride; k.idx = idx; k.idx_stride = idx_stride; k.threshold = threshold; k.bucket = bucket;
         k.masks = ss.masks; k.list_out = ss.list; k.count_out = ss.count; k.n_local = n_w_rows; k.T = T;
-        k.coef = ss.coef; k.coef_stride = ss.coef_stride; k.exact = axpy_mm_exact(wtype, ncols);
+        k.coef = ss.coef; k.coef_stride = ss.coef_stride; k.exact = exact;
         if ((rc = launch_coef(k, st))) return rc;
-        a.coef = ss.coef; a.coef_stride = ss.coef_stride; a.pdl = true;
+        a.coef = ss.coef; a.coef_stride = ss.coef_stride; a.exact = exact; a.pdl = true;
     }
     a.wtype = wtype; a.Wt = Wt; a.nrows = n_w_rows; a.ncols = ncols; a.h = h; a.h_stride = h_stride; a.T = T;
     a.list = ss.list; a.count = ss.count; a.bucket = bucket; a.idx = idx; a.idx_stride = idx_stride; a.threshold = threshold;
@@ -286,7 +287,8 @@ int pi_sparse_ffn(int wtype, const void * up, const void * gate, const void * do
     Scratch s(workspace, workspace_bytes);
     SparseScratch ss;
     const int G = axpy_groups(wtype, ncols, T);
-    const bool carved = carve_sparse(s, n_w_rows, T, axpy_mm_exact(wtype, ncols) ? 4 : 2, ss);
+    const bool exact = axpy_mm_exact(wtype, n_w_rows, ncols, T);
+    const bool carved = carve_sparse(s, n_w_rows, T, exact ? 4 : 2, ss);
     char * actp = (char *)s.take(act_bytes(wtype, ncols, T));
     bool ok = aligned(workspace, 256) && actp && carved;
     float * h = ok ? (float *)s.take((size_t)T * F * 4) : nullptr;
@@ -350,10 +352,10 @@ int pi_sparse_ffn(int wtype, const void * up, const void * gate, const void * do
             k.pdl = true;
             k.wtype = wtype; k.h = h; k.h_stride = F; k.idx = idx; k.idx_stride = idx_stride; k.threshold = threshold; k.bucket = bucket;
             k.masks = ss.masks; k.list_out = ss.list; k.count_out = ss.count; k.n_local = n_w_rows; k.T = T; k.h_uncleared = true; k.fill_bias = up_bias;
-            k.coef = ss.coef; k.coef_stride = ss.coef_stride; k.exact = axpy_mm_exact(wtype, ncols);
+            k.coef = ss.coef; k.coef_stride = ss.coef_stride; k.exact = exact;
             if ((rc = launch_coef(k, st))) return rc;
         }
-        a.coef = ss.coef; a.coef_stride = ss.coef_stride;
+        a.coef = ss.coef; a.coef_stride = ss.coef_stride; a.exact = exact;
     }
     a.pdl = true;
     a.wtype = wtype; a.Wt = down_t; a.nrows = n_w_rows; a.ncols = ncols; a.h = h; a.h_stride = F; a.T = T;

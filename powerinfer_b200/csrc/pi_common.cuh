@@ -164,6 +164,7 @@ struct AxpyArgs {
     // Q4_0: coefficient planes made by launch_neuron_q8 (int8 by global id, float scale per 32-neuron block)
     const int8_t * cq = nullptr; const float * cd = nullptr; int64_t c_stride = 0;
     const void * coef = nullptr; int64_t coef_stride = 0;             // 2+ tokens: coefficients by list position (launch_coef, or GemvArgs::coef)
+    bool exact = false;                                               // they are F32 (axpy_mm_exact), else FP16
     float * partial = nullptr; int n_groups = 0;                      // [n_groups, T, ncols]: room for n_groups partial vectors
     unsigned int * status = nullptr;                                  // device status word (bit 1: a copy wait ran out); enables the
                                                                       // bulk-copy pipelined kernel for T == 1
@@ -172,7 +173,7 @@ struct AxpyArgs {
 int axpy_groups(int wtype, int64_t ncols, int T);                     // row groups the launcher will use
 int launch_axpy(const AxpyArgs & a, cudaStream_t st, int * groups_used = nullptr);   // groups_used: partial vectors written
 int launch_axpy_mm(const AxpyArgs & a, cudaStream_t st, int * groups_used);          // 2+ tokens, needs coef; PI_ERR_UNSUPPORTED: not eligible
-bool axpy_mm_exact(int wtype, int64_t ncols);                                        // coefficients are F32, else FP16
+bool axpy_mm_exact(int wtype, int64_t nrows, int64_t ncols, int T);                  // the batch's coefficients are to be F32, else FP16
 int axpy_mm_pieces(int64_t ncols, int T);                                            // partial vectors launch_axpy_mm writes
 // axpy coefficients by list position (pi_axpy_mm.cu): [T, coef_stride], FP16 or (exact) F32, from h F32 [T, h_stride] by global neuron id
 struct CoefArgs {

@@ -634,6 +634,7 @@ int enqueue_step(pi_engine * e, int T, cudaStream_t st, StageTimer & tm, int mod
         } else {
             // a batch of FP16 rows needs the activations only as coefficients; Q4_0 coefficients are made from blocks of 32 neurons
             const bool direct = T > 1 && wt == PI_TYPE_F16 && F <= MM_MAX_ROWS;
+            const bool exact = axpy_mm_exact(wt, F, d, mode ? e->T_max : T);   // (a prompt's FP32 factors do not depend on how it is cut)
             // ---- up (and gate) over the active rows: h = relu(gate.x) * (up.x) | relu(up.x + b)
             {
                 GemvArgs g;
@@ -651,7 +652,7 @@ int enqueue_step(pi_engine * e, int T, cudaStream_t st, StageTimer & tm, int mod
                 k.pdl = pdl;
                 k.wtype = wt; k.h = e->h; k.h_stride = F; k.idx = pred; k.idx_stride = F; k.threshold = c.threshold;
                 k.masks = e->masks; k.list_out = e->list; k.count_out = e->count; k.n_local = F; k.T = T; k.h_uncleared = true; k.fill_bias = L->up_b;
-                k.coef = e->coef; k.coef_stride = e->coef_stride; k.exact = axpy_mm_exact(wt, d);
+                k.coef = e->coef; k.coef_stride = e->coef_stride; k.exact = exact;
                 STAGE(PI_STAGE_DOWN, 1, launch_coef(k, st));
             }
             {
@@ -661,7 +662,7 @@ int enqueue_step(pi_engine * e, int T, cudaStream_t st, StageTimer & tm, int mod
                 if (T == 1 && rows1) { a.masks = e->masks; a.h_uncleared = masks1; } else { a.list = e->list; a.count = e->count; }
                 a.idx = pred; a.idx_stride = F; a.threshold = c.threshold;
                 a.cq = e->cq; a.cd = e->cd; a.c_stride = F; a.partial = e->partial; a.n_groups = T == 1 ? e->G : axpy_mm_pieces(d, T); a.status = e->status;
-                if (T > 1) { a.coef = e->coef; a.coef_stride = e->coef_stride; }
+                if (T > 1) { a.coef = e->coef; a.coef_stride = e->coef_stride; a.exact = exact; }
                 STAGE(PI_STAGE_DOWN, 1, launch_axpy(a, st, &used));
             }
         }

@@ -1,0 +1,82 @@
+"""Steps with several tokens where a kernel's promise ends or its input is out of the ordinary: which Q4_0 down projections keep the CPU
+path's 32-bit factors, rows of any bucket, values that are not finite, addresses that are aligned to one value only.
+
+References are float64 sums over the values that the kernels multiply (Q8_0 activations with dequantised Q4_0 weights, FP16 with FP16).
+"""
+import numpy as np
+import pytest
+
+from powerinfer_b200 import synth
+from test_gpu_batches import rounded, weight
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(scope="module")
+def ops():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from powerinfer_b200 import ggml_ops
+    return ggml_ops
+
+
+def generator(seed):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(seed)
+    return gen
+
+
+def few(gen, T, rows, n):
+    """predictor logits under which the same `n` rows are active for every token"""
+    idx = torch.full((T, rows), -1.0, device="cuda")
+    on = torch.randperm(rows, device="cuda", generator=gen)[:n]
+    idx[:, on] = 1.0
+    return idx, on
+
+
+@pytest.mark.parametrize("rows,T", [(64, 33), (64, 40), (96, 128), (64, 261), (262208, 2), (262208, 32)])
+def test_axpy_keeps_32_bit_factors(ops, rows, T):
+    """More than 32 tokens, or more than 2^28 weights, at a width where a smaller step rounds its factors to FP16.  Products of FP32 factors
+    summed in FP32 are off by at most one rounding of 2^-24 per term and a few for each factor; FP16 factors would be off by 2^-11."""
+    cols, n = 1024, 12
+    gen = generator(rows + T)
+    if rows > 10000:
+        raw = ops.quantize_q4_0(torch.randn(rows, cols, device="cuda", generator=gen) * 0.05)
+        planar = torch.empty_like(raw)
+        from powerinfer_b200._lib import check, lib
+        check(lib.pi_q4_0_repack(raw.data_ptr(), planar.data_ptr(), rows, cols, torch.cuda.current_stream().cuda_stream))
+        W = ops.Weight(synth.Q4_0, planar, rows, cols)
+    else:
+        W = weight(ops, synth.Q4_0, rows, cols, gen)
+    idx, on = few(gen, T, rows, n)
+    h = torch.zeros(T, rows, device="cuda")
+    h[:, on] = torch.rand(T, n, device="cuda", generator=gen) + 0.1
+    w = ops.dequantize(W)[on].double()
+    c = rounded(ops, synth.Q4_0, h)[:, on]
+    got = ops.ggml_axpy(W, h, idx).double()
+    assert ((got - c @ w).abs() <= (n + 8) * 2.0 ** -24 * (c.abs() @ w.abs())).all()
+
+
+@pytest.mark.parametrize("n", [20, 40])
+def test_prompt_of_an_engine_for_one_sequence_keeps_32_bit_factors(ops, n):
+    """A prompt against the same prompt token by token, in a model where nothing but the FFN's sum can differ: one layer, no attention
+    output, predictor logits far from the threshold.  Up to the axpy both make the same bits but for rare flips of an FP16 rounding in the
+    norms' outputs.  Two sums of 32-bit products that add in another order are 1e-6 apart; FP16 factors (2^-11 / sqrt(3) for two random
+    roundings of up to half a unit each) 2e-4."""
+    from powerinfer_b200 import engine
+    spec = synth.ModelSpec(arch=synth.ARCH_OPT, wtype=synth.Q4_0, n_layer=1, d=1024, n_ff=1024, n_head=8, n_head_kv=8, rank=64, n_vocab=512, n_ctx=64, firing=0.2, seed=5)
+    t = synth.build_model(spec)
+    rng = np.random.default_rng(5)
+    z = np.where(rng.random(spec.n_ff) < spec.firing, 5.0, -5.0)
+    w = rng.standard_normal((spec.n_ff, spec.rank)) * spec.sigma
+    t["blk.0.fc2.weight"] = (w + (spec.sigma / (0.564 * spec.rank ** 0.5) * z)[:, None]).astype(np.float16)
+    t["blk.0.attn_output.weight"] = np.zeros_like(t["blk.0.attn_output.weight"])
+    one, many = engine.DecodeEngine(spec, t, max_batch=1), engine.DecodeEngine(spec, t, max_batch=1)
+    toks = rng.integers(0, spec.n_vocab, n).astype(np.int32)
+    for pos in range(n):
+        ref, _ = one.decode([toks[pos]], [pos])
+    got, _ = many.prefill(toks)
+    one.close()
+    many.close()
+    assert np.linalg.norm(got - ref[0]) <= 4e-5 * np.linalg.norm(ref[0])
