@@ -355,7 +355,9 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
 // ---------------------------------------------------------------------------------------------- coefficients
 // h F32 [T, h_stride] (by global neuron id) -> coef [T, coef_stride] by list position: FP16(h), or for Q4_0 rows the int8
 // quant of h in its block of 32 neurons times that block's FP16 scale (ggml.c:14575-14581, quantize_row_q8_0), rounded to FP16
-// or (exact mode) as it is, in F32; 0 where the token is inactive.  One warp per 32 local rows (one word of the union masks); a
+// or (exact mode) as it is, in F32; 0 where the token is inactive.  The block is the one of the GLOBAL ids.  Where a warp's rows are one
+// whole block (always without a bucket) its maximum is the warp's; any other bucket's rows read their blocks from h, which then holds
+// something at every neuron (h_uncleared only without a bucket).  One warp per 32 local rows (one word of the union masks); a
 // CTA takes 8 tokens, counts the rows named by the words before its own to find its list positions, and writes its part of the list.
 // Bound: the latency from the wait to the stores.  The hidden values are loaded before the count, whether the word names a row or
 // not, the count meets at one barrier, and the eight tokens' maxima and quotients run side by side: eight tokens, 28672 rows, 3 layers
@@ -381,11 +383,16 @@ __global__ void __launch_bounds__(256) k_coef(const CoefP p) {
     pdl_wait();
     uint32_t m = c < n_chunks ? __ldcg(p.masks + c) : 0u;
     const int t0 = blockIdx.y * UN;
+    // (lanes past the last row stand for the rest of its block, which counts where h holds something there)
+    const int64_t first = __shfl_sync(0xffffffffu, g, 0);
+    const bool tail = Q4 && !p.h_uncleared && !in && c < n_chunks;
+    const bool whole = !Q4 || p.h_uncleared || __all_sync(0xffffffffu, (first & 31) == 0 && (!in || g == first + lane));
     float v[UN], l[UN];                                               // (on their way while the positions are counted)
 #pragma unroll
     for (int u = 0; u < UN; u++) {
         v[u] = 0.f; l[u] = 0.f;
         if (in && t0 + u < p.T) { v[u] = p.h[(size_t)(t0 + u) * p.h_stride + g]; l[u] = p.idx[(size_t)(t0 + u) * p.idx_stride + g]; }
+        if (tail && whole && t0 + u < p.T) v[u] = p.h[(size_t)(t0 + u) * p.h_stride + first + lane];
     }
     int sum = 0;
 #pragma unroll 4
@@ -418,7 +425,12 @@ __global__ void __launch_bounds__(256) k_coef(const CoefP p) {
 #pragma unroll
         for (int s = 16; s > 0; s >>= 1)
 #pragma unroll
-            for (int u = 0; u < UN; u++) amax[u] = fmaxf(amax[u], __shfl_xor_sync(0xffffffffu, amax[u], s));
+            for (int u = 0; u < UN; u++) { const float a = __shfl_xor_sync(0xffffffffu, amax[u], s); if (whole) amax[u] = fmaxf(amax[u], a); }
+        if (!whole && in) {                                           // a bucket that cuts blocks: every row looks its own up
+#pragma unroll
+            for (int u = 0; u < UN; u++)
+                for (int k = 0; k < 32 && t0 + u < p.T; k++) amax[u] = fmaxf(amax[u], fabsf(p.h[(size_t)(t0 + u) * p.h_stride + (g & ~(int64_t)31) + k]));
+        }
 #pragma unroll
         for (int u = 0; u < UN; u++) {
             const float id = amax[u] != 0.0f ? 127.0f / amax[u] : 0.0f;

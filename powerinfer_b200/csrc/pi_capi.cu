@@ -320,17 +320,21 @@ int pi_sparse_ffn(int wtype, const void * up, const void * gate, const void * do
             return launch_reduce_partials(partial, used1, 1, ncols, nullptr, nullptr, dst, st, true);
         }
     }
-    if (T > 1 && n_w_rows <= MM_MAX_ROWS) {
+    // Q4_0 coefficients need the whole block of 32 global neurons.  The rows of a bucket may be any part of one, so a batch's hidden vector
+    // is then cleared as at one token: zeros, relu(bias) where a held neuron is inactive
+    const bool cleared = T > 1 && bucket && wtype == PI_TYPE_Q4_0;
+    if (T > 1 && n_w_rows <= MM_MAX_ROWS && !cleared) {
         prep_masks();
         if ((rc = launch_prep(pa, st))) return rc;
     } else {
-        if (T == 1 && (bucket || wtype == PI_TYPE_Q4_0)) { pa.zero = h; pa.n_zero = F; }
+        if (cleared || (T == 1 && (bucket || wtype == PI_TYPE_Q4_0))) { pa.zero = h; pa.n_zero = (int64_t)T * F; }
         if ((rc = launch_prep(pa, st))) return rc;
         CompactArgs c;
         c.pdl = true;
         c.idx = idx; c.idx_stride = idx_stride; c.T = T; c.threshold = threshold; c.n_local = n_w_rows; c.bucket = bucket;
-        c.masks = ss.masks; c.list = ss.list; c.count = ss.count; c.ticket = ss.ticket;
-        if (wtype == PI_TYPE_Q4_0 && T == 1) { c.zero_dst = h; c.zero_stride = F; c.fill_bias = up_bias; c.fill_relu = 1; }
+        c.masks = ss.masks;
+        if (T == 1 || n_w_rows > MM_MAX_ROWS) { c.list = ss.list; c.count = ss.count; c.ticket = ss.ticket; }
+        if (cleared || (wtype == PI_TYPE_Q4_0 && T == 1)) { c.zero_dst = h; c.zero_stride = F; c.fill_bias = up_bias; c.fill_relu = 1; }
         if ((rc = launch_compact(c, st))) return rc;
     }
     GemvArgs g;
@@ -351,7 +355,7 @@ int pi_sparse_ffn(int wtype, const void * up, const void * gate, const void * do
             CoefArgs k;
             k.pdl = true;
             k.wtype = wtype; k.h = h; k.h_stride = F; k.idx = idx; k.idx_stride = idx_stride; k.threshold = threshold; k.bucket = bucket;
-            k.masks = ss.masks; k.list_out = ss.list; k.count_out = ss.count; k.n_local = n_w_rows; k.T = T; k.h_uncleared = true; k.fill_bias = up_bias;
+            k.masks = ss.masks; k.list_out = ss.list; k.count_out = ss.count; k.n_local = n_w_rows; k.T = T; k.h_uncleared = !cleared; k.fill_bias = cleared ? nullptr : up_bias;
             k.coef = ss.coef; k.coef_stride = ss.coef_stride; k.exact = exact;
             if ((rc = launch_coef(k, st))) return rc;
         }

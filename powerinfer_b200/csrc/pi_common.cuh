@@ -182,7 +182,8 @@ struct CoefArgs {
     const int32_t * bucket = nullptr; const uint32_t * masks = nullptr;   // masks: union over the tokens
     int32_t * list_out = nullptr; int32_t * count_out = nullptr;       // the active local rows in order, and their number
     int64_t n_local = 0; int T = 1;
-    // h holds nothing where a token is inactive: Q4_0 block scales take 0 there, or relu(fill_bias) (what the graph's bias add leaves)
+    // (without a bucket) h holds nothing where a token is inactive: Q4_0 block scales take 0 there, or relu(fill_bias) (what the graph's
+    // bias add leaves); else it holds something at every neuron, h_stride a multiple of 32
     bool h_uncleared = false; const float * fill_bias = nullptr;
     void * coef = nullptr; int64_t coef_stride = 0; bool exact = false;
     bool pdl = false;

@@ -80,3 +80,48 @@ def test_prompt_of_an_engine_for_one_sequence_keeps_32_bit_factors(ops, n):
     one.close()
     many.close()
     assert np.linalg.norm(got - ref[0]) <= 4e-5 * np.linalg.norm(ref[0])
+
+
+def axpy_close(got, c, w, cols, T):
+    per_term = (w.shape[0] + 8) * 2.0 ** -24 + (2.0 ** -10 if cols % 1024 == 0 and T <= 32 else 0.0)
+    assert ((got.double() - c @ w).abs() <= per_term * (c.abs() @ w.abs()) + 1e-30).all()
+
+
+@pytest.mark.parametrize("cols", [256, 1024])
+@pytest.mark.parametrize("T", [2, 9, 40])
+def test_q8_blocks_are_those_of_the_global_neurons(ops, cols, T):
+    """The coefficient's scale is that of the 32 neurons around it in h, whichever of them this device holds: any sorted bucket, a bucket of
+    whole blocks that ends inside one, and rows that end inside a block of h."""
+    gen = generator(cols + T)
+    F = 640
+    h = torch.randn(T, F, device="cuda", generator=gen) * torch.rand(1, F, device="cuda", generator=gen) ** 4
+    idx = torch.randn(T, F, device="cuda", generator=gen)
+    some = torch.sort(torch.randperm(F, device="cuda", generator=gen)[:333])[0]
+    blocks = torch.cat([torch.arange(b * 32, b * 32 + 32, device="cuda") for b in (0, 3, 4, 9, 17)])[:-11]
+    for ids in (some, blocks, torch.arange(600, device="cuda")):
+        W = weight(ops, synth.Q4_0, len(ids), cols, gen)
+        c = (rounded(ops, synth.Q4_0, h) * (idx >= 0))[:, ids]
+        got = ops.ggml_axpy(W, h, idx, None if len(ids) == 600 else ids.int())
+        axpy_close(got, c, ops.dequantize(W).double(), cols, T)
+
+
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("T", [2, 9, 40])
+def test_sparse_ffn_of_any_bucket(ops, gated, T):
+    """The whole FFN over any part of the neurons: neurons held elsewhere count as 0 in their blocks, held ones that are inactive as 0 or as
+    relu(bias), as the graph's nodes leave them."""
+    gen = generator(T)
+    F, d = 640, 256
+    ids = torch.sort(torch.randperm(F, device="cuda", generator=gen)[:333])[0]
+    up, gate, down = (weight(ops, synth.Q4_0, len(ids), d, gen) for _ in range(3))
+    x = torch.randn(T, d, device="cuda", generator=gen)
+    idx = torch.randn(T, F, device="cuda", generator=gen)
+    bias = None if gated else torch.randn(F, device="cuda", generator=gen)
+    got = ops.sparse_ffn(up, gate if gated else None, down, x, idx, gpu_bucket=ids.int(), up_bias=bias)
+    h = ops.ggml_mul_mat_idx(up, x, idx, ids.int(), F)
+    if gated:
+        h = torch.relu(ops.ggml_mul_mat_idx(gate, x, idx, ids.int(), F)) * h
+    else:
+        h[:, ids] = torch.relu(h[:, ids] + bias[ids])
+    c = (rounded(ops, synth.Q4_0, h) * (idx >= 0))[:, ids]
+    axpy_close(got, c, ops.dequantize(down).double(), d, T)
