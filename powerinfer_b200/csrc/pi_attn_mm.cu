@@ -265,10 +265,10 @@ __global__ void __launch_bounds__(AM_THREADS, UN == 2 ? 4 : HC == 2 ? 3 : 2) k_a
                 if (KSPL > 2) { y[j] += o[(32 + r) * HD + lane * 8 + j]; y[j] += o[(48 + r) * HD + lane * 8 + j]; }
             }
         }
-        if (p.out && lane < HD / 8) {
+        if (p.out && lane < HD / 8) {                                 // (a caller's address: aligned to a float, not more)
             float * d = p.out + ((size_t)t * p.n_head + h) * HD + lane * 8;
-            *reinterpret_cast<float4 *>(d) = make_float4(y[0], y[1], y[2], y[3]);
-            *reinterpret_cast<float4 *>(d + 4) = make_float4(y[4], y[5], y[6], y[7]);
+#pragma unroll
+            for (int j = 0; j < 8; j++) d[j] = y[j];
         }
         if (p.out_act_type) emit_act8(p.out_act_type, p.out_act, t, (int64_t)p.n_head * HD, h * (HD / 8) + lane, y, lane < HD / 8);
     }

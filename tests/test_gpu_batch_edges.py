@@ -125,3 +125,37 @@ def test_sparse_ffn_of_any_bucket(ops, gated, T):
         h[:, ids] = torch.relu(h[:, ids] + bias[ids])
     c = (rounded(ops, synth.Q4_0, h) * (idx >= 0))[:, ids]
     axpy_close(got, c, ops.dequantize(down).double(), d, T)
+
+
+def attention_reference(q, k, v, heads, kv):
+    """softmax(q k^T / sqrt(hd)) v of one token's heads in float64; k, v [n, kv * hd]"""
+    n, hd = k.shape[0], q.numel() // heads
+    K, V = (c.double().view(n, kv, hd).repeat_interleave(heads // kv, 1) for c in (k, v))
+    sc = torch.einsum("hd,nhd->hn", q.half().double().view(heads, hd), K) / hd ** 0.5
+    p, x = sc.softmax(1), sc.max(1, keepdim=True)[0] - sc
+    w = p * (x + (p * x).sum(1, keepdim=True) + 5) * 2.0 ** -11 + 2.0 ** -24      # the bound of test_gpu_batches.test_attention_of_a_batch
+    return torch.einsum("hn,nhd->hd", p, V), torch.einsum("hn,nhd->hd", w, V.abs())
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("T", [1, 3])
+def test_attention_result_at_any_float_address(ops, hd, T):
+    """The F32 result goes to any address that is aligned to a float."""
+    from powerinfer_b200._lib import check, lib
+    gen = generator(hd + T)
+    heads, kv, n_ctx = 4, 2, 64
+    kc, vc = (torch.randn(T, n_ctx, kv * hd, device="cuda", generator=gen).half() for _ in range(2))
+    q = torch.randn(T, heads * hd, device="cuda", generator=gen)
+    k, v = (torch.randn(T, kv * hd, device="cuda", generator=gen) for _ in range(2))
+    pos = torch.tensor([40, 3, 63][:T], dtype=torch.int32, device="cuda")
+    seq = torch.arange(T, dtype=torch.int32, device="cuda")
+    buf = torch.zeros(T * heads * hd + 8, device="cuda")
+    for off in (0, 1, 2, 3):
+        out = buf[off:off + T * heads * hd]
+        buf.zero_()
+        check(lib.pi_attention_decode(q.data_ptr(), k.data_ptr(), v.data_ptr(), kc.data_ptr(), vc.data_ptr(), seq.data_ptr(), pos.data_ptr(), T, heads, kv, hd, n_ctx,
+                                      out.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        for t in range(T):
+            ref, bound = attention_reference(q[t], kc[t, :int(pos[t]) + 1], vc[t, :int(pos[t]) + 1], heads, kv)
+            assert ((out.double().view(T, heads, hd)[t] - ref).abs() <= bound).all(), (off, t)
+        assert not buf[:off].any() and not buf[off + T * heads * hd:].any()
