@@ -265,6 +265,25 @@ __global__ void __launch_bounds__(AM_THREADS, UN == 2 ? 4 : HC == 2 ? 3 : 2) k_a
                 if (KSPL > 2) { y[j] += o[(32 + r) * HD + lane * 8 + j]; y[j] += o[(48 + r) * HD + lane * 8 + j]; }
             }
         }
+        if (p.chunk) {
+            // The rows of a chunk share their value tiles, so a row also multiplied the values of tokens after its own, by 0: one that is not
+            // finite left a NaN.  Such a sum is made again from the row's own positions (and is a NaN if it is one).
+            bool nan = false;
+#pragma unroll
+            for (int j = 0; j < 8; j++) nan |= y[j] != y[j];
+            if (nan) {
+#pragma unroll
+                for (int j = 0; j < 8; j++) y[j] = 0.f;
+                for (int i = 0; i <= s_pos[r]; i++) {
+                    const float pi = __half2float(p16[r * P_PITCH + i]);
+                    const uint4 w = __ldcg(reinterpret_cast<const uint4 *>(vc + (size_t)i * dkv) + lane);
+                    const float2 w0 = h2f(w.x), w1 = h2f(w.y), w2 = h2f(w.z), w3 = h2f(w.w);
+                    y[0] = fmaf(pi, w0.x, y[0]); y[1] = fmaf(pi, w0.y, y[1]); y[2] = fmaf(pi, w1.x, y[2]); y[3] = fmaf(pi, w1.y, y[3]);
+                    y[4] = fmaf(pi, w2.x, y[4]); y[5] = fmaf(pi, w2.y, y[5]); y[6] = fmaf(pi, w3.x, y[6]); y[7] = fmaf(pi, w3.y, y[7]);
+                }
+            }
+            __syncwarp();
+        }
         if (p.out && lane < HD / 8) {                                 // (a caller's address: aligned to a float, not more)
             float * d = p.out + ((size_t)t * p.n_head + h) * HD + lane * 8;
 #pragma unroll

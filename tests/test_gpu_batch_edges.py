@@ -159,3 +159,35 @@ def test_attention_result_at_any_float_address(ops, hd, T):
             ref, bound = attention_reference(q[t], kc[t, :int(pos[t]) + 1], vc[t, :int(pos[t]) + 1], heads, kv)
             assert ((out.double().view(T, heads, hd)[t] - ref).abs() <= bound).all(), (off, t)
         assert not buf[:off].any() and not buf[off + T * heads * hd:].any()
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("n", [20, 40])
+def test_a_value_that_overflows_stays_with_the_tokens_that_see_it(ops, hd, n):
+    """A prompt whose tenth token has values beyond FP16's range: the rows that the tokens before it leave in the next layer's cache are those
+    of the same prompt without it.  (Its column of the value matrix is 0 times 60000 for every other token.)"""
+    from powerinfer_b200 import engine
+    spec = synth.ModelSpec(arch=synth.ARCH_LLAMA, wtype=synth.F16, n_layer=2, d=512, n_ff=1024, n_head=512 // hd, n_head_kv=512 // hd, rank=64, n_vocab=64, n_ctx=64, firing=0.2, seed=9)
+    t = synth.build_model(spec)
+    rng = np.random.default_rng(9)
+    for il in range(spec.n_layer):
+        z = np.where(rng.random(spec.n_ff) < spec.firing, 5.0, -5.0)
+        w = rng.standard_normal((spec.n_ff, spec.rank)) * spec.sigma
+        t[f"blk.{il}.fc2.weight"] = (w + (spec.sigma / (0.564 * spec.rank ** 0.5) * z)[:, None]).astype(np.float16)
+    t["token_embd.weight"][:, 7] = 0
+    t["token_embd.weight"][63] = 0
+    t["token_embd.weight"][63, 7] = 1
+    t["blk.0.attn_v.weight"][:, 7] = 60000
+    toks = rng.integers(0, 63, n).astype(np.int32)
+    toks[9] = 63
+    rows = []
+    for prompt in (toks, toks[:9]):
+        eng = engine.DecodeEngine(spec, t, max_batch=1)
+        eng.prefill(prompt, want_logits=False)
+        torch.cuda.synchronize()
+        rows.append(eng.k_cache.view(2, spec.n_ctx, -1)[1, :9].float().clone())
+        assert torch.isinf(eng.v_cache.view(2, spec.n_ctx, -1)[0, 9]).all() == (len(prompt) > 9)
+        eng.close()
+    assert torch.isfinite(rows[0]).all()
+    # FP16 roundings between the nodes that flip by one level, as in test_gpu_batches.test_prompt_chunks
+    assert (rows[0] - rows[1]).norm() <= 3e-3 * rows[1].norm()
