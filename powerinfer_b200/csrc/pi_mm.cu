@@ -25,7 +25,8 @@
 // Rows arrive by 16-byte cp.async: the rows of the active list lie anywhere, and pieces of a few hundred bytes are too small for the
 // bulk-copy engine (about 80 ns per copy).  A row slice of 64 bytes is stored with its four 16-byte pieces permuted by
 // (row / 2) % 4, so that the eight rows of an 8x8 fragment lie in different banks without padding.
-// Dense weights do not depend on the kernel before: their first stages are requested before griddepcontrol.wait.
+// Dense weights do not depend on the kernel before: the producers request their first stages before griddepcontrol.wait, and every thread
+// waits there before its first bounded wait.
 // Every wait is bounded: when one runs out the warp sets bit 4 of *status (where given) and the CTA returns without a result, its copies landed.
 //
 // Q4_0 arithmetic: a nibble q is placed in the high half of a byte and its top bit flipped, which is the int8 value
@@ -321,6 +322,9 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
     }
     // ===================================================================== consumers
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(MM_REGS_C));
+    // The waits below are bounded in tries: they count this kernel's own copies only, not what is left of the kernel before (an exchange may
+    // wait for a late rank for a second), and do not take issue slots from it.
+    if (!SPARSE) pdl_wait();
     const int g = lane >> 2, q = lane & 3;
     // ldmatrix addresses inside a stage (fragment layouts of mma.m16n8k16 / m16n8k32): two 16-byte pieces of 16 rows, four of 8 tokens
     // (Q4_0: one block of 32 rows, one block of two groups of 8 tokens)

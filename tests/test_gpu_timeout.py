@@ -32,3 +32,42 @@ def test_exchange_wait_runs_out_and_the_engine_stays_usable():
     eng.status()                                               # clean
     assert np.isfinite(logits).all() and int(amax[0]) == int(logits[0].argmax())
     eng.close()
+
+
+def _sharded(max_batch, wtype=synth.Q4_0):
+    from powerinfer_b200 import engine
+    spec = synth.ModelSpec(arch=synth.ARCH_LLAMA, wtype=wtype, n_layer=2, d=512, n_ff=2048, n_head=4, n_head_kv=2, rank=64, firing=0.15, seed=41)
+    eng = engine.DecodeEngine(spec, synth.build_model(spec), max_batch=max_batch, n_ranks=2, rank=0)
+    eng.setup_exchange_loopback()
+    return eng
+
+
+def _status_word(eng):
+    """The engine's status word as a view of its workspace: the one word that pi_engine_status clears after a wait ran out."""
+    from powerinfer_b200._lib import lib
+    eng.set_wait_cycles(1_000_000)
+    eng.decode([7], [0])
+    off = (-eng.ws.data_ptr()) % 256
+    words = eng.ws[off:off + (eng.ws.numel() - off) // 4 * 4].view(torch.int32)
+    before = words.clone()
+    assert lib.pi_engine_status(eng.handle, eng.st) == 5
+    at = (before != words).nonzero()
+    assert at.numel() == 1 and before[at].item() == 1
+    return words[at.item():at.item() + 1]
+
+
+@pytest.mark.parametrize("wtype", [synth.F16, synth.Q4_0])
+def test_a_late_rank_runs_out_only_the_exchange_wait_of_a_batch(wtype):
+    """The dense products of a batch are resident while the exchange before them still polls.  Their own bounded waits start when it is
+    over, however long it took."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from powerinfer_b200._lib import lib
+    eng = _sharded(3, wtype)
+    word = _status_word(eng)
+    eng.set_wait_cycles(300_000_000)               # about 0.15 s per exchange
+    for step in range(3):                          # plain launch, graph capture, graph replay
+        eng.decode([7, 8, 9], [step] * 3)
+        assert word.item() == 1
+        assert lib.pi_engine_status(eng.handle, eng.st) == 5 and b"exchange" in lib.pi_last_error()
+    eng.close()
