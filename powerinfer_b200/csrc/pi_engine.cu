@@ -180,7 +180,7 @@ struct pi_engine {
     __half * k_cache, * v_cache;             // [n_layer, max_batch, n_ctx, dkv]
     unsigned long long * amax_best; unsigned int * amax_ticket;   // k_argmax: a word per row, 0 between steps
     int32_t ** sink; float ** logits_sink;   // per row: where the step's greedy id and logits go as well (null for steps fed on the device)
-    unsigned int * status;                   // device word: bit 0 = an exchange wait ran out
+    unsigned int * status;                   // device word: bit 0 = an exchange wait ran out, any other = a wait for a kernel's own copies
     unsigned long long * active_total;       // device counter: sum of active-list lengths over layers and steps
     pi_exchange xch;
     cudaGraphExec_t graphs[3][PI_MAX_BATCH + 1];   // [0] decode, [1] prompt chunk, [2] prompt chunk without the lm head
@@ -873,7 +873,7 @@ int pi_engine_status(pi_engine * e, void * stream) {
     if (s) PI_CUDA(cudaMemsetAsync(e->status, 0, 4, (cudaStream_t)stream));      // reported once
     PI_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
     if (s & 1u) { set_error("an exchange wait ran out: a peer rank did not deliver its partial vector"); return PI_ERR_TIMEOUT; }
-    if (s & 14u) { set_error("a bulk-copy wait ran out in a weight-streaming kernel (status %u)", s); return PI_ERR_TIMEOUT; }
+    if (s) { set_error("a copy's wait ran out in a weight-streaming kernel (status %u)", s); return PI_ERR_TIMEOUT; }
     return PI_OK;
 }
 

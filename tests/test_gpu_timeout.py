@@ -71,3 +71,18 @@ def test_a_late_rank_runs_out_only_the_exchange_wait_of_a_batch(wtype):
         assert word.item() == 1
         assert lib.pi_engine_status(eng.handle, eng.st) == 5 and b"exchange" in lib.pi_last_error()
     eng.close()
+
+
+@pytest.mark.parametrize("bit", [2, 4, 8, 16])
+def test_every_status_bit_is_reported(bit):
+    """Each kind of kernel sets a bit of its own when a wait runs out; the host puts it there in a kernel's place."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from powerinfer_b200._lib import lib
+    eng = _sharded(1)
+    word = _status_word(eng)
+    word.fill_(bit)
+    torch.cuda.synchronize()
+    assert lib.pi_engine_status(eng.handle, eng.st) == 5 and b"status %d" % bit in lib.pi_last_error()
+    assert word.item() == 0 and lib.pi_engine_status(eng.handle, eng.st) == 0
+    eng.close()
