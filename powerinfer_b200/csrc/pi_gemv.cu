@@ -283,7 +283,6 @@ static int launch_tt(const GemvP & p, bool sparse, bool gated, size_t smem, cuda
             return launch_inst<WT, 1, false, false, 2, 1>(p, smem, st, pdl);
         return launch_inst<WT, 1, false, false, 1, 2>(p, smem, st, pdl);
     }
-    if (!sparse) { set_error("gemv: matrix too large"); return PI_ERR_UNSUPPORTED; }      // (more than 2^26 rows)
     if (gated)   return launch_inst<WT, TT, true, true, 1, 1>(p, smem, st, pdl);
     return launch_inst<WT, TT, true, false, 1, 1>(p, smem, st, pdl);
 }
@@ -331,10 +330,12 @@ static int launch_gemv_main(const GemvArgs & a, cudaStream_t st, bool * wrote_ma
     }
     const bool q4 = a.wtype == PI_TYPE_Q4_0;
     const int nb = (int)(a.ncols / QK);
-    // (batches come here only with a list of more than MM_MAX_ROWS neurons: chunks of at most 8 tokens, weights re-read per chunk)
+    // Batches that launch_mm declines: a list of more than MM_MAX_ROWS neurons in chunks of at most 8 tokens,
+    // dense matrices of more than 2^26 rows token by token; weights are read again for each
+    if (a.T > 1 && a.dst_host) { set_error("gemv: no second copy of the result for this shape"); return PI_ERR_UNSUPPORTED; }
     for (int t0 = 0; t0 < a.T; ) {
         const int left = a.T - t0;
-        const int tt = left >= 8 ? 8 : (left >= 4 ? 4 : (left >= 2 ? 2 : 1));
+        const int tt = !a.list ? 1 : left >= 8 ? 8 : (left >= 4 ? 4 : (left >= 2 ? 2 : 1));
         GemvP p;
         p.W = (const uint8_t *)a.W; p.W2 = (const uint8_t *)a.W2;
         p.row_bytes = (int64_t)pi_row_bytes(a.wtype, a.ncols);

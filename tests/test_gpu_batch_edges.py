@@ -191,3 +191,47 @@ def test_a_value_that_overflows_stays_with_the_tokens_that_see_it(ops, hd, n):
     assert torch.isfinite(rows[0]).all()
     # FP16 roundings between the nodes that flip by one level, as in test_gpu_batches.test_prompt_chunks
     assert (rows[0] - rows[1]).norm() <= 3e-3 * rows[1].norm()
+
+
+def test_dense_matrix_of_more_rows_than_a_tile_grid_takes(ops):
+    """More than 2^26 rows and several tokens."""
+    rows, cols, T = 2 ** 26 + 9, 8, 2
+    gen = generator(1)
+    w = torch.randint(-3, 4, (rows, cols), device="cuda", generator=gen, dtype=torch.int8).half()
+    x = torch.randint(-3, 4, (T, cols), device="cuda", generator=gen, dtype=torch.int8).float()
+    got = ops.ggml_mul_mat(ops.Weight(synth.F16, w.view(torch.uint8).reshape(-1), rows, cols), x)      # (small whole numbers: exact)
+    assert torch.equal(got, x @ w.float().T)
+
+
+@pytest.mark.parametrize("wtype,gated", [(synth.F16, True), (synth.F16, False), (synth.Q4_0, True)])
+def test_gathers_of_more_rows_than_their_masks_are_scanned_for(ops, wtype, gated):
+    """More than 262144 rows and several tokens: rows from a list, for up to 8 tokens at a time."""
+    rows, cols = 262240, 64 if wtype == synth.F16 else 256
+    gen = generator(rows)
+    def w(rows, cols):
+        if wtype == synth.F16:
+            return ops.Weight(wtype, (torch.randn(rows, cols, device="cuda", generator=gen) * 0.05).half().view(torch.uint8).reshape(-1), rows, cols)
+        raw = ops.quantize_q4_0(torch.randn(rows, cols, device="cuda", generator=gen) * 0.05)
+        planar = torch.empty_like(raw)
+        from powerinfer_b200._lib import check, lib
+        check(lib.pi_q4_0_repack(raw.data_ptr(), planar.data_ptr(), rows, cols, torch.cuda.current_stream().cuda_stream))
+        return ops.Weight(wtype, planar, rows, cols)
+    up, gate, down = w(rows, cols), w(rows, cols), w(rows, cols)
+    U, G, D = (ops.dequantize(m).double() for m in (up, gate, down))
+    for T in (3, 13):
+        x = torch.randn(T, cols, device="cuda", generator=gen)
+        idx, on = few(gen, T, rows, 3000)
+        idx[:, on] -= torch.rand(T, len(on), device="cuda", generator=gen) * 1.5                   # active for some tokens
+        xr, keep = rounded(ops, wtype, x), (idx[:, on] >= 0).double()
+        got = ops.ggml_mul_mat_idx(up, x, idx)
+        bound = (cols + 8) * 2.0 ** -24 * (xr.abs() @ U[on].abs().T)
+        assert ((got[:, on].double() - (xr @ U[on].T) * keep).abs() <= bound + 1e-30).all()
+        other = torch.ones(rows, dtype=torch.bool, device="cuda")
+        other[on] = False
+        assert not got[:, other].any()
+        got = ops.sparse_ffn(up, gate if gated else None, down, x, idx).double()
+        h = torch.relu(ops.ggml_mul_mat_idx(gate, x, idx)) * ops.ggml_mul_mat_idx(up, x, idx) if gated else torch.relu(ops.ggml_mul_mat_idx(up, x, idx))
+        c = rounded(ops, wtype, h)[:, on] * keep
+        # sums in another order (2^-22 of a hidden value) flip the rounding of one coefficient in 2^11 (FP16) or 2^15 / 127 x 64 (Q8_0: 127
+        # levels), by 2^-11 of it or 2^-7 of its block's largest: 2^-11 / 45 and 2^-7 / 16 of a sum of random signs, three times over
+        assert (got - c @ D[on]).norm() <= (4e-5 if wtype == synth.F16 else 2e-3) * (c @ D[on]).norm()
