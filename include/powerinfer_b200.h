@@ -120,7 +120,8 @@ int pi_sparse_ffn(int wtype, const void * up, const void * gate, const void * do
  * overlap on the GPU (different streams, or different host threads) race on it, so serialise them. */
 size_t pi_axpy_static_max_bytes(void);
 
-/* Did the last pi_mul_mat_idx / pi_axpy / pi_sparse_ffn that used `workspace` finish all its bounded device-side waits (the
+/* Did the last pi_mul_mat / pi_predictor / pi_mul_mat_idx / pi_axpy / pi_sparse_ffn that used `workspace` (of at least
+ * pi_workspace_bytes) finish all its bounded device-side waits (the
  * batch kernels stream rows through rings of bulk copies guarded by waits that give up after a limit rather than hang)?
  * PI_OK, or PI_ERR_TIMEOUT with the status bits in pi_last_error(): the call's result is then incomplete.  workspace NULL:
  * the built-in array of pi_axpy_static on the current device.  Synchronises `stream`.  (The engine has pi_engine_status.) */
@@ -131,7 +132,7 @@ int pi_axpy_static(int wtype, const void * Wt, int64_t n_w_rows, int64_t ncols,
 
 /* ---- dense decode nodes ------------------------------------------------------------------------------ */
 
-/* ggml_mul_mat with a weight matrix and T <= 32 activation columns (ggml.c:9598-9807; CUDA ggml-cuda.cu:4310-4414):
+/* ggml_mul_mat with a weight matrix and T activation columns (ggml.c:9598-9807; CUDA ggml-cuda.cu:4310-4414):
  * dst[t, r] = W[r,:] . x[t,:] (+ bias[r]).  Same activation rounding as above. */
 int pi_mul_mat(int wtype, const void * W, int64_t nrows, int64_t ncols, const float * x, int T,
                const float * bias, float * dst, void * workspace, size_t workspace_bytes, void * stream);

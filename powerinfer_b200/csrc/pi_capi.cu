@@ -48,7 +48,7 @@ struct SparseScratch {
     void * coef; int64_t coef_stride;                                // 2+ tokens: axpy coefficients
 };
 
-// The control words come FIRST in every sparse operator's workspace (count, ticket, status at bytes 0, 4, 8), so that
+// The control words come FIRST in every operator's workspace (count, ticket, status at bytes 0, 4, 8), so that
 // pi_op_status can find the status word of whichever operator used the workspace last.  coef_size: bytes of an axpy
 // coefficient (0: none needed).
 static bool carve_sparse(Scratch & s, int64_t n_rows, int T, int coef_size, SparseScratch & o) {
@@ -60,6 +60,15 @@ static bool carve_sparse(Scratch & s, int64_t n_rows, int T, int coef_size, Spar
     if (!o.list || !ct || !o.masks) return false;
     o.count = ct; o.ticket = (unsigned int *)(ct + 1); o.status = (unsigned int *)(ct + 2);
     return true;
+}
+
+// The dense operators keep the same control words in the same place where their workspace has room for them beside the activations (as
+// pi_workspace_bytes gives it).  Without them (null) the kernels run that have no bounded waits.
+static unsigned int * carve_words(char *& p, size_t workspace_bytes, size_t planes) {
+    if (workspace_bytes < planes + 256) return nullptr;
+    unsigned int * w = (unsigned int *)p;
+    p += 256;
+    return w;
 }
 
 // The rows of a gather: activity bit masks, and the sorted list only where the kernel that follows wants one
@@ -123,13 +132,13 @@ int pi_mul_mat(int wtype, const void * W, int64_t nrows, int64_t ncols, const fl
     cudaStream_t st = (cudaStream_t)stream;
     if (!aligned(workspace, 256) || workspace_bytes < act_bytes(wtype, ncols, T)) { set_error("mul_mat: workspace too small or misaligned"); return PI_ERR_WORKSPACE; }
     char * p = (char *)workspace;
+    unsigned int * words = carve_words(p, workspace_bytes, act_bytes(wtype, ncols, T));
     ActBuf act = act_carve(wtype, ncols, T, &p);
     GemvArgs g;
     g.wtype = wtype; g.W = W; g.nrows = nrows; g.ncols = ncols; g.x = act.view(); g.T = T; g.pdl = true;
-    g.bias = bias; g.dst = dst; g.dst_stride = nrows;
-    if (T == 1 && workspace_bytes >= act_bytes(wtype, ncols, T) + 256) g.status = (unsigned int *)p;   // room for a status word: the bulk-copy ring kernels are eligible
+    g.bias = bias; g.dst = dst; g.dst_stride = nrows; g.status = words ? words + 2 : nullptr;
     PrepArgs a;
-    a.wtype = wtype; a.T = T; a.x = x; a.n = ncols; a.act = act; a.words = g.status; a.n_words = 1;
+    a.wtype = wtype; a.T = T; a.x = x; a.n = ncols; a.act = act; a.words = words; a.n_words = 3;
     if ((rc = launch_prep(a, st))) return rc;
     return launch_gemv(g, st);
 }
@@ -145,6 +154,7 @@ int pi_predictor(const void * fc1, const void * fc2, int64_t d, int64_t rank, in
         set_error("predictor: workspace too small or misaligned"); return PI_ERR_WORKSPACE;
     }
     char * p = (char *)workspace;
+    unsigned int * words = carve_words(p, workspace_bytes, act_bytes(PI_TYPE_F16, d, T) + act_bytes(PI_TYPE_F16, rank, T));
     ActBuf a_in = act_carve(PI_TYPE_F16, d, T, &p);
     ActBuf a_h  = act_carve(PI_TYPE_F16, rank, T, &p);
     GemvArgs g1;                                       // hidden = relu(fc1 . p), kept only in the FP16 form fc2 consumes
@@ -152,11 +162,9 @@ int pi_predictor(const void * fc1, const void * fc2, int64_t d, int64_t rank, in
     g1.W = fc1; g1.nrows = rank; g1.ncols = d; g1.x = a_in.view(); g1.T = T; g1.relu = 1; g1.dst16 = a_h.h16; g1.dst_stride = rank;
     GemvArgs g2;
     g2.W = fc2; g2.nrows = F; g2.ncols = rank; g2.x = a_h.view(); g2.T = T; g2.dst = idx; g2.dst_stride = F; g2.pdl = true;
-    if (T == 1 && workspace_bytes >= act_bytes(PI_TYPE_F16, d, T) + act_bytes(PI_TYPE_F16, rank, T) + 256) {     // as in pi_mul_mat
-        g1.status = g2.status = (unsigned int *)p;
-    }
+    g1.status = g2.status = words ? words + 2 : nullptr;
     PrepArgs a;
-    a.T = T; a.x = p_in; a.n = d; a.act = a_in; a.words = g1.status; a.n_words = 1;
+    a.T = T; a.x = p_in; a.n = d; a.act = a_in; a.words = words; a.n_words = 3;
     if ((rc = launch_prep(a, st))) return rc;
     if ((rc = launch_gemv(g1, st))) return rc;
     return launch_gemv(g2, st);
@@ -384,7 +392,7 @@ int pi_op_status(const void * workspace, void * stream) {
     unsigned int word = 0;
     PI_CUDA(cudaMemcpyAsync(&word, (const char *)ws + 8, 4, cudaMemcpyDeviceToHost, st));
     PI_CUDA(cudaStreamSynchronize(st));
-    if (word) { set_error("a bounded wait inside a kernel of the last sparse operator ran out (status bits 0x%x): its result is incomplete", word); return PI_ERR_TIMEOUT; }
+    if (word) { set_error("a bounded wait inside a kernel of the last operator ran out (status bits 0x%x): its result is incomplete", word); return PI_ERR_TIMEOUT; }
     return PI_OK;
 }
 

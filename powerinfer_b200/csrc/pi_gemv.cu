@@ -319,7 +319,8 @@ static int launch_gemv_main(const GemvArgs & a, cudaStream_t st, bool * wrote_ma
         if (rc != PI_ERR_UNSUPPORTED) return rc;
         if (!a.list) { set_error("gemv: masks given but the shape is not eligible and there is no list"); return PI_ERR_UNSUPPORTED; }
     }
-    if (a.T > 1) {                                                 // 2+ tokens: tensor-core kernel
+    // 2+ tokens: tensor-core kernel, which reports waits that run out in *status; who has no room for one gets the kernels without waits
+    if (a.T > 1 && a.status) {
         const int rc = launch_mm(a, st);
         if (rc != PI_ERR_UNSUPPORTED) { if (wrote_masks) *wrote_masks = a.masks_out != nullptr; return rc; }
         if (!a.list && a.masks) { set_error("gemv: masks given but the shape is not eligible and there is no list"); return PI_ERR_UNSUPPORTED; }
@@ -330,8 +331,8 @@ static int launch_gemv_main(const GemvArgs & a, cudaStream_t st, bool * wrote_ma
     }
     const bool q4 = a.wtype == PI_TYPE_Q4_0;
     const int nb = (int)(a.ncols / QK);
-    // Batches that launch_mm declines: a list of more than MM_MAX_ROWS neurons in chunks of at most 8 tokens,
-    // dense matrices of more than 2^26 rows token by token; weights are read again for each
+    // Batches that launch_mm declines or that have no status word: a list of more than MM_MAX_ROWS neurons in chunks of at most 8 tokens,
+    // dense matrices (of more than 2^26 rows) token by token; weights are read again for each
     if (a.T > 1 && a.dst_host) { set_error("gemv: no second copy of the result for this shape"); return PI_ERR_UNSUPPORTED; }
     for (int t0 = 0; t0 < a.T; ) {
         const int left = a.T - t0;

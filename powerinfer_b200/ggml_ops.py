@@ -82,7 +82,7 @@ _ws = Workspace()
 
 
 def last_op_status() -> int:
-    """Status of the last sparse operator issued through this module (pi_op_status): 0, or 5 (a bounded device-side wait ran out)."""
+    """Status of the last operator issued through this module (pi_op_status): 0, or 5 (a bounded device-side wait ran out)."""
     if _ws.buf is None:
         return 0
     return int(lib.pi_op_status(_ws.at, _stream()))

@@ -235,3 +235,42 @@ def test_gathers_of_more_rows_than_their_masks_are_scanned_for(ops, wtype, gated
         # sums in another order (2^-22 of a hidden value) flip the rounding of one coefficient in 2^11 (FP16) or 2^15 / 127 x 64 (Q8_0: 127
         # levels), by 2^-11 of it or 2^-7 of its block's largest: 2^-11 / 45 and 2^-7 / 16 of a sum of random signs, three times over
         assert (got - c @ D[on]).norm() <= (4e-5 if wtype == synth.F16 else 2e-3) * (c @ D[on]).norm()
+
+
+@pytest.mark.parametrize("T", [1, 4, 40])
+def test_dense_operators_keep_a_status_word(ops, T):
+    """pi_op_status finds the word of a dense product too, and it is clear: 0xFF bytes before, whatever the activations are."""
+    gen = generator(T)
+    x = torch.randn(T, 512, device="cuda", generator=gen)
+    for wtype in (synth.F16, synth.Q4_0):
+        W = weight(ops, wtype, 100, 512, gen)
+        ops.ggml_mul_mat(W, x)                                        # (the workspace has its size)
+        ops._ws.buf.fill_(255)
+        ops.ggml_mul_mat(W, x)
+        assert ops.last_op_status() == 0
+    fc1, fc2 = weight(ops, synth.F16, 64, 512, gen), weight(ops, synth.F16, 300, 64, gen)
+    ops._ws.buf.fill_(255)
+    ops.predictor(fc1, fc2, x)
+    assert ops.last_op_status() == 0
+
+
+@pytest.mark.parametrize("wtype", [synth.F16, synth.Q4_0])
+@pytest.mark.parametrize("T", [1, 2, 9, 40])
+def test_dense_product_in_a_workspace_for_the_activations_alone(ops, wtype, T):
+    """A workspace without room for control words is accepted; the kernels without waits give the same result."""
+    from powerinfer_b200._lib import check, lib
+    rows, cols = 333, 1024
+    gen = generator(T)
+    W = weight(ops, wtype, rows, cols, gen)
+    x = torch.randn(T, cols, device="cuda", generator=gen)
+    planes = [T * cols * 2] if wtype == synth.F16 else [T * cols // 2] * 2 + [T * cols // 8] * 2
+    need = sum((b + 255) // 256 * 256 for b in planes)
+    buf = torch.full((need + 512,), 255, dtype=torch.uint8, device="cuda")
+    at = (-buf.data_ptr()) % 256
+    out = torch.empty(T, rows, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    check(lib.pi_mul_mat(wtype, W.ptr, rows, cols, x.data_ptr(), T, None, out.data_ptr(), buf.data_ptr() + at, need, st))
+    assert (buf[at + need:] == 255).all() and (buf[:at] == 255).all()
+    xr, w = rounded(ops, wtype, x), ops.dequantize(W).double()
+    assert ((out.double() - xr @ w.T).abs() <= (cols + 8) * 2.0 ** -24 * (xr.abs() @ w.abs().T)).all()
+    assert lib.pi_mul_mat(wtype, W.ptr, rows, cols, x.data_ptr(), T, None, out.data_ptr(), buf.data_ptr() + at, need - 1, st) == 3
