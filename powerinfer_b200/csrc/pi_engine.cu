@@ -802,6 +802,12 @@ int pi_engine_prefill_host(pi_engine * e, const int32_t * host_tokens, int n_tok
         if ((rc = run_step(e, T, st, head ? 1 : 2))) return rc;
         row = e->c.n_ranks > 1 ? T - 1 : 0;
     }
+    if (e->T_max == 1 && n_tokens > 1) {                              // an engine for one sequence goes on from here (pi_engine_advance): its row is the last token's
+        FeedPrompt f;
+        f.token[0] = host_tokens[n_tokens - 1];
+        k_feed_prompt<<<1, PROMPT_CHUNK, 0, st>>>(f, 1, pos0 + n_tokens - 1, seq, e->tokens, e->pos, e->seq_pf);
+        PI_LAUNCH_CHECK("k_feed_prompt");
+    }
     if (host_logits_last) PI_CUDA(cudaMemcpyAsync(host_logits_last, e->logits + (size_t)row * e->c.n_vocab, (size_t)e->c.n_vocab * 4, cudaMemcpyDeviceToHost, st));
     if (host_argmax_last) PI_CUDA(cudaMemcpyAsync(host_argmax_last, e->argmax + row, 4, cudaMemcpyDeviceToHost, st));
     PI_CUDA(cudaStreamSynchronize(st));

@@ -69,3 +69,30 @@ def test_chunked_prompt_leaves_the_kv_cache_single_steps_leave(engine_mod, name)
     assert np.abs(got_l[0] - ref_l[0]).max() <= tol(spec)
     b.status()
     b.close()
+
+
+@pytest.mark.parametrize("n", [1, 21, 60])
+def test_decoding_goes_on_from_the_device_after_a_prompt(engine_mod, n):
+    """An engine for one sequence: after a prompt its I/O buffers hold the last token, its position and its greedy id, as after a step, so
+    that pi_engine_advance feeds the next step without the host."""
+    spec = mg.MODEL_CASES["llama_f16"]
+    t = synth.build_model(spec)
+    toks = [int(v) for v in np.random.default_rng(n).integers(3, spec.n_vocab, n)]
+    eng = engine_mod.DecodeEngine(spec, t, max_batch=1)
+    _, cur = eng.prefill(toks)
+    want = []
+    for pos in range(n, n + 4):
+        cur = int(eng.decode([cur], [pos])[1][0])
+        want.append(cur)
+    eng.k_cache.zero_(); eng.v_cache.zero_(); torch.cuda.synchronize()
+    eng.prefill(toks)
+    got = []
+    for pos in range(n, n + 4):
+        eng.advance(1)
+        eng.stream.synchronize()
+        assert int(eng.device_view("pos", 1).cpu()[0]) == pos
+        eng.step_device(1)
+        eng.stream.synchronize()
+        got.append(int(eng.device_view("argmax", 1).cpu()[0]))
+    assert got == want
+    eng.close()
