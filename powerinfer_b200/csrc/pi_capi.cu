@@ -273,7 +273,7 @@ int pi_axpy(int wtype, const void * Wt, int64_t n_w_rows, int64_t ncols,
     }
     a.wtype = wtype; a.Wt = Wt; a.nrows = n_w_rows; a.ncols = ncols; a.h = h; a.h_stride = h_stride; a.T = T;
     a.list = ss.list; a.count = ss.count; a.bucket = bucket; a.idx = idx; a.idx_stride = idx_stride; a.threshold = threshold;
-    a.cq = cq; a.cd = cd; a.c_stride = h_stride; a.partial = partial; a.n_groups = G; a.status = ss.status;
+    a.cq = cq; a.cd = cd; a.partial = partial; a.n_groups = G; a.status = ss.status;
     if (rows1) { a.masks = ss.masks; a.pdl = true; }
     int used = G;
     if ((rc = launch_axpy(a, st, &used))) return rc;
@@ -372,7 +372,7 @@ int pi_sparse_ffn(int wtype, const void * up, const void * gate, const void * do
     a.pdl = true;
     a.wtype = wtype; a.Wt = down_t; a.nrows = n_w_rows; a.ncols = ncols; a.h = h; a.h_stride = F; a.T = T;
     a.list = ss.list; a.count = ss.count; a.bucket = bucket; a.idx = idx; a.idx_stride = idx_stride; a.threshold = threshold;
-    a.cq = cq; a.cd = cd; a.c_stride = F; a.partial = partial; a.n_groups = G; a.status = ss.status;
+    a.cq = cq; a.cd = cd; a.partial = partial; a.n_groups = G; a.status = ss.status;
     if (T == 1) a.masks = ss.masks;
     int used = G;
     if ((rc = launch_axpy(a, st, &used))) return rc;

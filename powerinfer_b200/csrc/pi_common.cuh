@@ -161,13 +161,12 @@ struct AxpyArgs {
     // bucket == nullptr.  Only the Q4_0 coefficients look at such entries (the scale of a block of 32 neurons).
     bool h_uncleared = false;
     const float * idx = nullptr; int64_t idx_stride = 0; float threshold = 0.f;
-    // Q4_0: coefficient planes made by launch_neuron_q8 (int8 by global id, float scale per 32-neuron block)
-    const int8_t * cq = nullptr; const float * cd = nullptr; int64_t c_stride = 0;
+    // one token, Q4_0: room for coefficient planes (int8 by global id, float scale per 32-neuron block) where the shape needs them
+    int8_t * cq = nullptr; float * cd = nullptr;
     const void * coef = nullptr; int64_t coef_stride = 0;             // 2+ tokens: coefficients by list position (launch_coef, or GemvArgs::coef)
     bool exact = false;                                               // they are F32 (axpy_mm_exact), else FP16
     float * partial = nullptr; int n_groups = 0;                      // [n_groups, T, ncols]: room for n_groups partial vectors
-    unsigned int * status = nullptr;                                  // device status word (bit 1: a copy wait ran out); enables the
-                                                                      // bulk-copy pipelined kernel for T == 1
+    unsigned int * status = nullptr;                                  // device status word (2+ tokens; bit 4: a copy wait ran out)
     bool pdl = false;
 };
 int axpy_groups(int wtype, int64_t ncols, int T);                     // row groups the launcher will use
@@ -210,8 +209,8 @@ struct FfnRowsArgs {
 };
 int launch_ffn_rows(const FfnRowsArgs & a, cudaStream_t st, int * groups_used);
 bool ffn_rows_eligible(const FfnRowsArgs & a);      // up / gate / down_t (null or not), shape and n_groups as they will be passed
-// h F32 [T, stride] -> Q8_0 over 32-neuron blocks: cq int8 [T, stride], cd float [T, stride/32]
-int launch_neuron_q8(const float * h, int64_t stride, int64_t n, int T, int8_t * cq, float * cd, cudaStream_t st);
+// h F32 [n] -> Q8_0 over 32-neuron blocks: cq int8 [n], cd float [n/32]
+int launch_neuron_q8(const float * h, int64_t n, int8_t * cq, float * cd, cudaStream_t st);
 
 // sum partial [n_groups, T, n] in group order (+ residual + bias) -> dst [T, n]
 int static_scratch_address(void ** out);      // device address of pi_axpy_static's built-in scratch array on the current device

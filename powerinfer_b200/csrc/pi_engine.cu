@@ -661,7 +661,7 @@ int enqueue_step(pi_engine * e, int T, cudaStream_t st, StageTimer & tm, int mod
                 a.wtype = wt; a.Wt = L->down_t; a.nrows = F; a.ncols = d; a.h = e->h; a.h_stride = F; a.T = T;
                 if (T == 1 && rows1) { a.masks = e->masks; a.h_uncleared = masks1; } else { a.list = e->list; a.count = e->count; }
                 a.idx = pred; a.idx_stride = F; a.threshold = c.threshold;
-                a.cq = e->cq; a.cd = e->cd; a.c_stride = F; a.partial = e->partial; a.n_groups = T == 1 ? e->G : axpy_mm_pieces(d, T); a.status = e->status;
+                a.cq = e->cq; a.cd = e->cd; a.partial = e->partial; a.n_groups = T == 1 ? e->G : axpy_mm_pieces(d, T); a.status = e->status;
                 if (T > 1) { a.coef = e->coef; a.coef_stride = e->coef_stride; a.exact = exact; }
                 STAGE(PI_STAGE_DOWN, 1, launch_axpy(a, st, &used));
             }

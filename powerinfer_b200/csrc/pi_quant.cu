@@ -254,27 +254,21 @@ int launch_prep(const PrepArgs & a, cudaStream_t st) {
 // ------------------------------------------------------------------------------------------------
 // Coefficients of the Q4_0 axpy (ggml.c:14575-14581): the FFN hidden vector quantised to Q8_0 over blocks of
 // 32 consecutive NEURONS; neuron r contributes int8 b = cq[r] with scale cd[r/32].
-__global__ void k_neuron_q8(const float * __restrict__ h, int64_t stride, int nb, int T,
-                            int8_t * __restrict__ cq, float * __restrict__ cd) {
-    const int lane = threadIdx.x & 31;
-    const int64_t nblocks = (int64_t)T * nb;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < nblocks; i += warps) {
-        const int64_t t = i / nb;
-        const int b = (int)(i - t * nb);
+__global__ void k_neuron_q8(const float * __restrict__ h, int nb, int8_t * __restrict__ cq, float * __restrict__ cd) {
+    const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
+    for (int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); b < nb; b += warps) {
         int q, s; float d16;
-        q8_block(h[t * stride + (int64_t)b * QK + lane], q, d16, s);
-        cq[t * stride + (int64_t)b * QK + lane] = (int8_t)q;
-        if (lane == 0) cd[t * (stride / QK) + b] = d16;
+        q8_block(h[(int64_t)b * QK + lane], q, d16, s);
+        cq[(int64_t)b * QK + lane] = (int8_t)q;
+        if (lane == 0) cd[b] = d16;
     }
 }
 
-int launch_neuron_q8(const float * h, int64_t stride, int64_t n, int T, int8_t * cq, float * cd, cudaStream_t st) {
+int launch_neuron_q8(const float * h, int64_t n, int8_t * cq, float * cd, cudaStream_t st) {
     const int nb = (int)(n / QK);
-    const int64_t nblocks = (int64_t)T * nb;
-    if (nblocks == 0) return PI_OK;
-    const int grid = (int)imin64((nblocks + 7) / 8, (int64_t)sm_count() * 8);
-    k_neuron_q8<<<grid, 256, 0, st>>>(h, stride, nb, T, cq, cd);
+    if (nb == 0) return PI_OK;
+    const int grid = (int)imin64(((int64_t)nb + 7) / 8, (int64_t)sm_count() * 8);
+    k_neuron_q8<<<grid, 256, 0, st>>>(h, nb, cq, cd);
     PI_LAUNCH_CHECK("k_neuron_q8");
     return PI_OK;
 }

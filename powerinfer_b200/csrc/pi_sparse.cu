@@ -132,69 +132,53 @@ static constexpr int AXPY_UNROLL = 4;
 
 struct AxpyP {
     const uint8_t * Wt; int64_t row_bytes; int nrows; int ncols; int nb;
-    const float * h; int64_t h_stride;
+    const float * h;
     const int32_t * list; const int32_t * count; const int32_t * bucket;
-    const float * idx; int64_t idx_stride; float threshold;
-    const int8_t * cq; const float * cd; int64_t c_stride;
-    float * partial; int T;
+    const float * idx; float threshold;
+    const int8_t * cq; const float * cd;
+    float * partial;
 };
 
-template <int TT>
 __global__ void __launch_bounds__(AXPY_F16_THREADS) k_axpy_f16(const AxpyP p) {
     const int c = (blockIdx.x * AXPY_F16_THREADS + threadIdx.x) * 8;
     const bool col_ok = c < p.ncols;
     const int G = gridDim.y;
     const int n = min(*p.count, p.nrows);
-    float acc[TT][8];
-#pragma unroll
-    for (int t = 0; t < TT; t++)
-#pragma unroll
-        for (int j = 0; j < 8; j++) acc[t][j] = 0.f;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 
     for (int i0 = blockIdx.y; i0 < n; i0 += G * AXPY_UNROLL) {
         uint4 w[AXPY_UNROLL];
-        float a[AXPY_UNROLL][TT];
+        float a[AXPY_UNROLL];
 #pragma unroll
         for (int u = 0; u < AXPY_UNROLL; u++) {
             const int i = i0 + u * G;
-#pragma unroll
-            for (int t = 0; t < TT; t++) a[u][t] = 0.f;
+            a[u] = 0.f;
             w[u] = make_uint4(0u, 0u, 0u, 0u);
             if (i < n) {
                 const int r = p.list[i];
                 if ((unsigned)r < (unsigned)p.nrows) {
                     const int64_t g = p.bucket ? p.bucket[r] : r;
                     if (col_ok) w[u] = ldg_stream(p.Wt + (size_t)r * p.row_bytes + (size_t)c * 2);
-#pragma unroll
-                    for (int t = 0; t < TT; t++) {
-                        // the CPU path rounds h to FP16 and skips rows below the threshold (ggml.c:14422-14428)
-                        const float hv = round_f16(p.h[(size_t)t * p.h_stride + g]);
-                        const bool on = !(p.idx[(size_t)t * p.idx_stride + g] < p.threshold);
-                        a[u][t] = on ? hv : 0.f;
-                    }
+                    // the CPU path rounds h to FP16 and skips rows below the threshold (ggml.c:14422-14428)
+                    const float hv = round_f16(p.h[g]);
+                    a[u] = !(p.idx[g] < p.threshold) ? hv : 0.f;
                 }
             }
         }
 #pragma unroll
         for (int u = 0; u < AXPY_UNROLL; u++) {
             const float2 w0 = h2f(w[u].x), w1 = h2f(w[u].y), w2 = h2f(w[u].z), w3 = h2f(w[u].w);
-#pragma unroll
-            for (int t = 0; t < TT; t++) {
-                const float s = a[u][t];
-                acc[t][0] = fmaf(w0.x, s, acc[t][0]); acc[t][1] = fmaf(w0.y, s, acc[t][1]);
-                acc[t][2] = fmaf(w1.x, s, acc[t][2]); acc[t][3] = fmaf(w1.y, s, acc[t][3]);
-                acc[t][4] = fmaf(w2.x, s, acc[t][4]); acc[t][5] = fmaf(w2.y, s, acc[t][5]);
-                acc[t][6] = fmaf(w3.x, s, acc[t][6]); acc[t][7] = fmaf(w3.y, s, acc[t][7]);
-            }
+            const float s = a[u];
+            acc[0] = fmaf(w0.x, s, acc[0]); acc[1] = fmaf(w0.y, s, acc[1]);
+            acc[2] = fmaf(w1.x, s, acc[2]); acc[3] = fmaf(w1.y, s, acc[3]);
+            acc[4] = fmaf(w2.x, s, acc[4]); acc[5] = fmaf(w2.y, s, acc[5]);
+            acc[6] = fmaf(w3.x, s, acc[6]); acc[7] = fmaf(w3.y, s, acc[7]);
         }
     }
     if (col_ok) {
-#pragma unroll
-        for (int t = 0; t < TT; t++) {
-            float * o = p.partial + ((size_t)blockIdx.y * p.T + t) * p.ncols + c;
-            *reinterpret_cast<float4 *>(o)     = make_float4(acc[t][0], acc[t][1], acc[t][2], acc[t][3]);
-            *reinterpret_cast<float4 *>(o + 4) = make_float4(acc[t][4], acc[t][5], acc[t][6], acc[t][7]);
-        }
+        float * o = p.partial + (size_t)blockIdx.y * p.ncols + c;
+        *reinterpret_cast<float4 *>(o)     = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        *reinterpret_cast<float4 *>(o + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
     }
 }
 
@@ -210,26 +194,22 @@ __device__ __forceinline__ float nib_to_float(uint32_t bytes, int k) {      // b
     return __uint_as_float(bits) - 8388616.0f;
 }
 
-template <int TT>
 __global__ void __launch_bounds__(AXPY_Q4_THREADS) k_axpy_q4(const AxpyP p) {
     const int b = blockIdx.x * AXPY_Q4_THREADS + threadIdx.x;
     const bool col_ok = b < p.nb;
     const int G = gridDim.y;
     const int n = min(*p.count, p.nrows);
-    float acc[TT][32];
+    float acc[32];
 #pragma unroll
-    for (int t = 0; t < TT; t++)
-#pragma unroll
-        for (int j = 0; j < 32; j++) acc[t][j] = 0.f;
+    for (int j = 0; j < 32; j++) acc[j] = 0.f;
 
     for (int i0 = blockIdx.y; i0 < n; i0 += G * AXPY_UNROLL) {
         uint4 q[AXPY_UNROLL];
-        float s[AXPY_UNROLL][TT];
+        float s[AXPY_UNROLL];
 #pragma unroll
         for (int u = 0; u < AXPY_UNROLL; u++) {
             const int i = i0 + u * G;
-#pragma unroll
-            for (int t = 0; t < TT; t++) s[u][t] = 0.f;
+            s[u] = 0.f;
             q[u] = make_uint4(0u, 0u, 0u, 0u);
             if (i < n) {
                 const int r = p.list[i];
@@ -238,13 +218,9 @@ __global__ void __launch_bounds__(AXPY_Q4_THREADS) k_axpy_q4(const AxpyP p) {
                     const uint8_t * row = p.Wt + (size_t)r * p.row_bytes;
                     q[u] = ldg_stream(reinterpret_cast<const uint4 *>(row) + b);
                     const float d4 = __half2float(__ldg(reinterpret_cast<const __half *>(row + (size_t)p.nb * 16) + b));
-#pragma unroll
-                    for (int t = 0; t < TT; t++) {
-                        const bool on = !(p.idx[(size_t)t * p.idx_stride + g] < p.threshold);
-                        const int b8 = p.cq[(size_t)t * p.c_stride + g];
-                        const float d8 = p.cd[(size_t)t * (p.c_stride / QK) + g / QK];
-                        s[u][t] = on ? (float)b8 * (d4 * d8) : 0.f;
-                    }
+                    const int b8 = p.cq[g];
+                    const float d8 = p.cd[g / QK];
+                    s[u] = !(p.idx[g] < p.threshold) ? (float)b8 * (d4 * d8) : 0.f;
                 }
             }
         }
@@ -256,24 +232,16 @@ __global__ void __launch_bounds__(AXPY_Q4_THREADS) k_axpy_q4(const AxpyP p) {
                 const uint32_t lo = wds[wi] & 0x0F0F0F0Fu, hi = (wds[wi] >> 4) & 0x0F0F0F0Fu;
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
-                    const float vlo = nib_to_float(lo, k), vhi = nib_to_float(hi, k);
-#pragma unroll
-                    for (int t = 0; t < TT; t++) {
-                        acc[t][wi * 4 + k]      = fmaf(vlo, s[u][t], acc[t][wi * 4 + k]);
-                        acc[t][16 + wi * 4 + k] = fmaf(vhi, s[u][t], acc[t][16 + wi * 4 + k]);
-                    }
+                    acc[wi * 4 + k]      = fmaf(nib_to_float(lo, k), s[u], acc[wi * 4 + k]);
+                    acc[16 + wi * 4 + k] = fmaf(nib_to_float(hi, k), s[u], acc[16 + wi * 4 + k]);
                 }
             }
         }
     }
     if (col_ok) {
+        float * o = p.partial + (size_t)blockIdx.y * p.ncols + (size_t)b * QK;
 #pragma unroll
-        for (int t = 0; t < TT; t++) {
-            float * o = p.partial + ((size_t)blockIdx.y * p.T + t) * p.ncols + (size_t)b * QK;
-#pragma unroll
-            for (int j = 0; j < 32; j += 4)
-                *reinterpret_cast<float4 *>(o + j) = make_float4(acc[t][j], acc[t][j + 1], acc[t][j + 2], acc[t][j + 3]);
-        }
+        for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4 *>(o + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
     }
 }
 
@@ -302,24 +270,23 @@ int launch_axpy(const AxpyArgs & a, cudaStream_t st, int * groups_used) {
         if (rc != PI_ERR_UNSUPPORTED) return rc;
         if (groups_used) *groups_used = a.n_groups;
     }
+    if (a.T != 1) { set_error("axpy: %d tokens need coefficients by list position", a.T); return PI_ERR_UNSUPPORTED; }
     // CUDA-core kernels for the one-token shapes the kernel above declines.  Q4_0 rows read coefficient planes (int8 quant of
     // h per 32 neurons, block scale).
     if (q4) {
-        PI_REQUIRE(a.cq && a.cd, "axpy: Q4_0 needs coefficient planes");
-        const int rc = launch_neuron_q8(a.h, a.h_stride, a.h_stride, 1, const_cast<int8_t *>(a.cq), const_cast<float *>(a.cd), st);
+        PI_REQUIRE(a.cq && a.cd, "axpy: Q4_0 needs room for coefficient planes");
+        const int rc = launch_neuron_q8(a.h, a.h_stride, a.cq, a.cd, st);
         if (rc) return rc;
     }
-    if (a.T != 1) { set_error("axpy: %d tokens need coefficients by list position", a.T); return PI_ERR_UNSUPPORTED; }
     AxpyP p;
     p.Wt = (const uint8_t *)a.Wt; p.row_bytes = (int64_t)pi_row_bytes(a.wtype, a.ncols);
     p.nrows = (int)a.nrows; p.ncols = (int)a.ncols; p.nb = (int)(a.ncols / QK);
-    p.h_stride = a.h_stride; p.list = a.list; p.count = a.count; p.bucket = a.bucket;
-    p.idx_stride = a.idx_stride; p.threshold = a.threshold; p.c_stride = a.c_stride; p.T = 1;
+    p.list = a.list; p.count = a.count; p.bucket = a.bucket; p.threshold = a.threshold;
     p.h = a.h; p.idx = a.idx; p.cq = a.cq; p.cd = a.cd; p.partial = a.partial;
     const int tiles = q4 ? (p.nb + AXPY_Q4_THREADS - 1) / AXPY_Q4_THREADS : (p.ncols / 8 + AXPY_F16_THREADS - 1) / AXPY_F16_THREADS;
     const dim3 grid(tiles, a.n_groups);
-    if (q4) k_axpy_q4<1><<<grid, AXPY_Q4_THREADS, 0, st>>>(p);
-    else    k_axpy_f16<1><<<grid, AXPY_F16_THREADS, 0, st>>>(p);
+    if (q4) k_axpy_q4<<<grid, AXPY_Q4_THREADS, 0, st>>>(p);
+    else    k_axpy_f16<<<grid, AXPY_F16_THREADS, 0, st>>>(p);
     PI_LAUNCH_CHECK("k_axpy");
     return PI_OK;
 }
