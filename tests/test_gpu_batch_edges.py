@@ -274,3 +274,15 @@ def test_dense_product_in_a_workspace_for_the_activations_alone(ops, wtype, T):
     xr, w = rounded(ops, wtype, x), ops.dequantize(W).double()
     assert ((out.double() - xr @ w.T).abs() <= (cols + 8) * 2.0 ** -24 * (xr.abs() @ w.abs().T)).all()
     assert lib.pi_mul_mat(wtype, W.ptr, rows, cols, x.data_ptr(), T, None, out.data_ptr(), buf.data_ptr() + at, need - 1, st) == 3
+
+
+def test_operators_run_on_the_current_stream(ops, monkeypatch):
+    """With torch's private functions, and without them."""
+    side = torch.cuda.Stream()
+    for names in ((), ("_raw_stream",), ("_raw_device",)):
+        for name in names:
+            monkeypatch.setattr(ops, name, None)
+        assert ops._stream() == torch.cuda.current_stream().cuda_stream
+        with torch.cuda.stream(side):
+            assert ops._stream() == side.cuda_stream
+        monkeypatch.undo()
