@@ -37,7 +37,7 @@ class Weight:
 # An operator at one token lasts a few microseconds on the device, so what these wrappers do on the host is part of its time:
 # tensors that are float32 and contiguous already pass untouched, and sizes and addresses of the workspace are kept.
 
-# (torch.cuda.current_stream() makes an object: 3.3 us a call where the number alone takes 0.2, and the seven calls of an FFN's nodes 79
+# (torch.cuda.current_stream() makes an object: 3.3 us a call where the number alone takes 0.2, and the nodes of an FFN 79
 # instead of 64 us.  The number comes from private functions, so a torch without them gets the public one.)
 _raw_stream, _raw_device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
 

@@ -286,3 +286,78 @@ def test_operators_run_on_the_current_stream(ops, monkeypatch):
         with torch.cuda.stream(side):
             assert ops._stream() == side.cuda_stream
         monkeypatch.undo()
+
+
+@pytest.mark.parametrize("wtype", [synth.F16, synth.Q4_0])
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("T", [32, 33, 77, 129, 256, 261])
+def test_sparse_ffn_of_many_rows_per_cta(ops, wtype, gated, T):
+    """Every CTA's share of the rows takes several tiles (277 neurons, 554 rows with the gate), most of them full."""
+    F, d = 40960, 256
+    gen = generator(T)
+    up, gate, down = (weight(ops, wtype, F, d, gen) for _ in range(3))
+    x = torch.randn(T, d, device="cuda", generator=gen)
+    idx = torch.randn(T, F, device="cuda", generator=gen) + 0.5
+    idx[:, torch.rand(F, device="cuda", generator=gen) < 0.1] = -1.0                               # active for no token
+    bias = None if gated else torch.randn(F, device="cuda", generator=gen) * 0.1
+    got = ops.sparse_ffn(up, gate if gated else None, down, x, idx, up_bias=bias).double()
+    xr, keep = rounded(ops, wtype, x), (idx >= 0).double()
+    h = xr @ ops.dequantize(up).double().T
+    h = (torch.relu(xr @ ops.dequantize(gate).double().T) * h if gated else h + bias) * (keep if gated else 1.0)
+    if not gated:
+        h = torch.relu(torch.where(keep > 0, h, bias[None, :].double()))                            # an inactive neuron's block sees relu(bias)
+    ref = (rounded(ops, wtype, h.float()) * keep) @ ops.dequantize(down).double()
+    # hidden values in FP32 against float64: 2^-22 of them, which flips one rounding in 2^11 (FP16) or one of 127 levels in 2^14, each worth
+    # 2^-11 or 2^-7 of a term; FP16 factors of a rounded Q4_0 sum do not occur at this width.  A missing neuron moves the sum by 1 / 200.
+    assert (got - ref).norm() <= (4e-5 if wtype == synth.F16 else 1e-3) * ref.norm()
+
+
+@pytest.mark.parametrize("cols", [8, 24, 56])
+@pytest.mark.parametrize("T", [2, 33, 100, 200])
+def test_rows_shorter_than_a_tile(ops, cols, T):
+    rows = 77
+    gen = generator(cols + T)
+    W = weight(ops, synth.F16, rows, cols, gen)
+    x = torch.randn(T, cols, device="cuda", generator=gen)
+    xr, w = rounded(ops, synth.F16, x), ops.dequantize(W).double()
+    bound = (cols + 8) * 2.0 ** -24 * (xr.abs() @ w.abs().T)
+    assert ((ops.ggml_mul_mat(W, x).double() - xr @ w.T).abs() <= bound).all()
+    idx = torch.randn(T, rows, device="cuda", generator=gen)
+    assert ((ops.ggml_mul_mat_idx(W, x, idx).double() - (xr @ w.T) * (idx >= 0)).abs() <= bound).all()
+    c = rounded(ops, synth.F16, torch.rand(T, rows, device="cuda", generator=gen)) * (idx >= 0)
+    assert ((ops.ggml_axpy(W, c.float(), idx).double() - c @ w).abs() <= (rows + 8) * 2.0 ** -24 * (c.abs() @ w.abs())).all()
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("n_ctx", [1200, 3584, 3600])
+def test_attention_of_one_token_far_into_a_sequence(ops, hd, n_ctx):
+    """Positions around the ends of what a thread holds in flight (512 scores, 384 and 768 value rows), up to the last; equal scores make the
+    largest sum of numerators."""
+    gen = generator(hd + n_ctx)
+    heads, kv = 4, 2
+    kc, vc = (torch.randn(1, n_ctx, kv * hd, device="cuda", generator=gen).half() for _ in range(2))
+    for pos in (0, 383, 384, 511, 512, 767, 768, 1100, n_ctx - 1):
+        for scale in (1.0, 0.0):
+            q = torch.randn(1, heads * hd, device="cuda", generator=gen) * scale
+            k, v = (torch.randn(1, kv * hd, device="cuda", generator=gen) for _ in range(2))
+            got = ops.attention_decode(q, k, v, kc, vc, torch.tensor([pos], dtype=torch.int32, device="cuda"), heads, kv)
+            assert torch.equal(kc[0, pos], k[0].half()) and torch.equal(vc[0, pos], v[0].half())
+            ref, bound = attention_reference(q[0], kc[0, :pos + 1], vc[0, :pos + 1], heads, kv)
+            assert ((got.double().view(heads, hd) - ref).abs() <= bound).all(), (pos, scale)
+
+
+@pytest.mark.parametrize("heads,kv,hd,n_ctx", [(4, 2, 128, 2500), (16, 1, 128, 1920), (16, 1, 128, 2500), (16, 1, 64, 2500), (16, 1, 128, 3700), (20, 1, 64, 2100)])
+def test_attention_of_a_batch_in_a_long_context(ops, heads, kv, hd, n_ctx):
+    """Scores of 16 rows fit up to 1920 (head_dim 64: 2112) positions; longer contexts, and those beyond 3584, have a kernel each."""
+    gen = generator(heads + n_ctx)
+    pos = torch.tensor([n_ctx - 1, 700, 1300], dtype=torch.int32, device="cuda")
+    seq = torch.tensor([2, 0, 1], dtype=torch.int32, device="cuda")
+    kc, vc = (torch.randn(3, n_ctx, kv * hd, device="cuda", generator=gen).half() for _ in range(2))
+    q = torch.randn(3, heads * hd, device="cuda", generator=gen)
+    k, v = (torch.randn(3, kv * hd, device="cuda", generator=gen) for _ in range(2))
+    got = ops.attention_decode(q, k, v, kc, vc, pos, heads, kv, seq=seq).double().view(3, heads, hd)
+    for t in range(3):
+        s, n = int(seq[t]), int(pos[t]) + 1
+        assert torch.equal(kc[s, n - 1], k[t].half()) and torch.equal(vc[s, n - 1], v[t].half())
+        ref, bound = attention_reference(q[t], kc[s, :n], vc[s, :n], heads, kv)
+        assert ((got[t] - ref).abs() <= bound).all(), t

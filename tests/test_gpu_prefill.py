@@ -1,6 +1,6 @@
-"""Prompt processing through the engine: several consecutive tokens of ONE sequence per step (chunks of up to max_batch
-tokens), K / V of the whole chunk stored first, causal attention after, union list for reading and each token's own mask
-for writing.  Held against (1) the reference's llama.cpp logits after its own batched prompt (golden fixtures: the
+"""Prompt processing through the engine: several consecutive tokens of ONE sequence per step (chunks of up to 256
+tokens, of max_batch where predictor logits are traced), K / V of the whole chunk stored first, causal attention after, union list for
+reading and each token's own mask for writing.  Held against (1) the reference's llama.cpp logits after its own batched prompt (golden fixtures: the
 reference's batched and token-by-token prompts give identical logits at one thread) and (2) the same engine fed the prompt
 one token per step: the KV cache rows a chunk leaves behind must be what single steps leave."""
 import os
@@ -31,7 +31,7 @@ def test_prompt_in_chunks_matches_the_reference_after_its_batched_prompt(engine_
     g = np.load(os.path.join(GOLD, f"model_{name}.npz"))
     assert bool(g["single_equals_batch"])
     eng = engine_mod.DecodeEngine(spec, synth.build_model(spec), max_batch=max_batch)
-    toks = [int(v) for v in g["prompt"]]                       # 8 tokens: one chunk of 8, or chunks of 3 + 3 + 2
+    toks = [int(v) for v in g["prompt"]]                       # 8 tokens: one chunk, within a decode step's batch or larger than it
     logits, amax = eng.prefill(toks, seq=0, pos0=0)
     err = [float(np.abs(logits - g["logits"][0]).max())]
     assert amax == int(logits.argmax())
@@ -59,7 +59,7 @@ def test_chunked_prompt_leaves_the_kv_cache_single_steps_leave(engine_mod, name)
     ka, va = a.k_cache.clone(), a.v_cache.clone()
     a.close()
     b = engine_mod.DecodeEngine(spec, t, max_batch=8)
-    b.prefill(toks, seq=0, pos0=0, want_logits=False)           # 8 + 8 + 5, no lm head at all
+    b.prefill(toks, seq=0, pos0=0, want_logits=False)           # one chunk of 21, no lm head at all
     got_l, _ = b.decode([5], [len(toks)])
     kb = b.k_cache.view(spec.n_layer, 8, spec.n_ctx, -1)[:, 0, :len(toks) + 1]
     vb = b.v_cache.view(spec.n_layer, 8, spec.n_ctx, -1)[:, 0, :len(toks) + 1]
@@ -96,3 +96,67 @@ def test_decoding_goes_on_from_the_device_after_a_prompt(engine_mod, n):
         got.append(int(eng.device_view("argmax", 1).cpu()[0]))
     assert got == want
     eng.close()
+
+
+def apart(spec, t, seed):
+    """Second predictor matrices that keep every neuron's logit five standard deviations away from the threshold: kernels that add in another
+    order choose the same neurons."""
+    rng = np.random.default_rng(seed)
+    for il in range(spec.n_layer):
+        z = np.where(rng.random(spec.n_ff) < spec.firing, 5.0, -5.0)
+        w = rng.standard_normal((spec.n_ff, spec.rank)) * spec.sigma
+        t[f"blk.{il}.fc2.weight"] = (w + (spec.sigma / (0.564 * spec.rank ** 0.5) * z)[:, None]).astype(np.float16)
+    return t
+
+
+def against_single_steps(engine_mod, spec, lengths):
+    t = apart(spec, synth.build_model(spec), 17)
+    one, many = engine_mod.DecodeEngine(spec, t, max_batch=1), engine_mod.DecodeEngine(spec, t, max_batch=2)
+    rng = np.random.default_rng(18)
+    for n in lengths:
+        toks = rng.integers(0, spec.n_vocab, n).astype(np.int32)
+        for pos in range(n):
+            ref, _ = one.decode([toks[pos]], [pos])
+        got, got_id = many.prefill(toks, seq=1)
+        # the bound of test_gpu_batches.test_prompt_chunks: roundings between the nodes that flip by one level
+        assert np.linalg.norm(got - ref[0]) <= (24e-3 if spec.wtype == synth.Q4_0 else 3e-3) * np.linalg.norm(ref[0]), n
+        assert got_id == int(got.argmax())
+        a = one.k_cache.view(spec.n_layer, 1, spec.n_ctx, -1)[:, 0, :n].float()
+        b = many.k_cache.view(spec.n_layer, 2, spec.n_ctx, -1)[:, 1, :n].float()
+        assert (a - b).norm() <= (24e-3 if spec.wtype == synth.Q4_0 else 3e-3) * a.norm()
+    many.status()
+    one.close()
+    many.close()
+
+
+@pytest.mark.parametrize("wtype", [synth.F16, synth.Q4_0])
+def test_prompt_over_many_neurons_per_cta(engine_mod, wtype):
+    """277 neurons per CTA: the predictor's masks and the gather take several tiles of every token count."""
+    against_single_steps(engine_mod, synth.ModelSpec(arch=synth.ARCH_LLAMA, wtype=wtype, n_layer=1, d=256, n_ff=40960, n_head=4, n_head_kv=4, rank=64, n_vocab=256,
+                                                     n_ctx=256, firing=0.9, seed=6), (40, 77, 130, 256))
+
+
+@pytest.mark.parametrize("heads,kv,n_ctx", [(4, 4, 2048), (8, 2, 2304), (4, 2, 4096)])
+def test_prompt_in_a_long_context(engine_mod, heads, kv, n_ctx):
+    """Contexts whose scores do not fit the several-token attention (head_dim 128 from 1921, 64 from 2113 positions): a store pass, then one
+    CTA per head and token."""
+    against_single_steps(engine_mod, synth.ModelSpec(arch=synth.ARCH_LLAMA, wtype=synth.F16, n_layer=2, d=512, n_ff=1024, n_head=heads, n_head_kv=kv, rank=64, n_vocab=256,
+                                                     n_ctx=n_ctx, firing=0.2, seed=7), (2, 40, 300))
+
+
+@pytest.mark.parametrize("wtype", [synth.F16, synth.Q4_0])
+def test_prompt_in_chunks_of_the_batch(engine_mod, wtype):
+    """With a trace of the predictor logits a prompt goes through in steps of max_batch tokens (8 + 8 + 5: a plain run, a captured one, a
+    replay), and leaves what one chunk leaves."""
+    spec = synth.ModelSpec(arch=synth.ARCH_LLAMA, wtype=wtype, n_layer=2, d=512, n_ff=1024, n_head=4, n_head_kv=2, rank=64, n_vocab=256, n_ctx=128, firing=0.2, seed=8)
+    t = apart(spec, synth.build_model(spec), 8)
+    toks = np.random.default_rng(8).integers(0, spec.n_vocab, 21)
+    plain, traced = engine_mod.DecodeEngine(spec, t, max_batch=8), engine_mod.DecodeEngine(spec, t, max_batch=8)
+    traced.enable_trace()
+    want, want_id = plain.prefill(toks)
+    for _ in range(3):
+        got, got_id = traced.prefill(toks)
+        assert np.linalg.norm(got - want) <= (24e-3 if wtype == synth.Q4_0 else 3e-3) * np.linalg.norm(want)
+        assert got_id == int(got.argmax()) and want_id == int(want.argmax())
+    plain.close()
+    traced.close()
