@@ -437,18 +437,17 @@ def main():
         raise SystemExit(f"bench.py: {cfg_name} needs about {need / 2**30:.0f} GiB per GPU on {world} GPU(s), the device has "
                          f"{have / 2**30:.0f} GiB: run it with more GPUs (--gpus N under torch.distributed.run)")
     g, layers = synth_device.build_local_model(spec, world, rank, seed=0)
-    PB = 32                                           # prompt chunk: tokens of one sequence per step
-    eng = engine.DecodeEngine(spec, g, max_batch=max(T, PB), n_ranks=world, rank=rank, local_layers=layers)
+    B = max(T, 32)                                    # sequences of a step at most
+    PB = B if world > 1 else max(B, min(256, spec.n_ctx))   # prompt chunk: tokens of one sequence per step (pi_engine_prefill_host)
+    eng = engine.DecodeEngine(spec, g, max_batch=B, n_ranks=world, rank=rank, local_layers=layers)
     del layers
     if world > 1:
         eng.setup_exchange()
 
     # ---- prompt: through the engine's chunked prompt path (pi_engine_prefill_host), timed on its own
     prompt = np.random.default_rng(0).integers(0, spec.n_vocab, (T, P))
-    eng.prefill([int(v) for v in prompt[0, :PB]], seq=0, pos0=0, want_logits=True)       # warm-up: plain run + capture
-    eng.prefill([int(v) for v in prompt[0, :PB]], seq=0, pos0=0, want_logits=False)
-    eng.prefill([int(v) for v in prompt[0, :PB]], seq=0, pos0=0, want_logits=True)
-    eng.prefill([int(v) for v in prompt[0, :PB]], seq=0, pos0=0, want_logits=False)
+    for _ in range(3):                                # warm-up: every chunk of the prompt as a plain run, and captured where it is within the batch
+        eng.prefill([int(v) for v in prompt[0]], seq=0, pos0=0, want_logits=True)
     barrier()
     t0 = time.perf_counter()
     start_tokens = []

@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
 // quant of h in its block of 32 neurons times that block's FP16 scale (ggml.c:14575-14581, quantize_row_q8_0), rounded to FP16
 // or (exact mode) as it is, in F32; 0 where the token is inactive.  The block is the one of the GLOBAL ids.  Where a warp's rows are one
 // whole block (always without a bucket) its maximum is the warp's; any other bucket's rows read their blocks from h, which then holds
-// something at every neuron (h_uncleared only without a bucket).  One warp per 32 local rows (one word of the union masks); a
+// something at every neuron (BLOCKS: an instance of its own; in one kernel the look-up cost the calls that have no use for it 3 us).  One warp per 32 local rows (one word of the union masks); a
 // CTA takes 8 tokens, counts the rows named by the words before its own to find its list positions, and writes its part of the list.
 // Bound: the latency from the wait to the stores.  The hidden values are loaded before the count, whether the word names a row or
 // not, the count meets at one barrier, and the eight tokens' maxima and quotients run side by side: eight tokens, 28672 rows, 3 layers
@@ -366,18 +366,18 @@ __global__ void __launch_bounds__(AX_THREADS, 1) k_axpy_mm(const AxpyMmP p) {
 struct CoefP {
     const float * h; int64_t h_stride; const float * idx; int64_t idx_stride; float threshold;
     const int32_t * bucket; const uint32_t * masks; int32_t * list; int32_t * count; int n_local, T;
-    const float * fill_bias; int h_uncleared;
+    const float * fill_bias;
     void * coef; int64_t coef_stride; int exact;
 };
 
-template <bool Q4>
+template <bool Q4, bool BLOCKS>
 __global__ void __launch_bounds__(256) k_coef(const CoefP p) {
     __shared__ int s_pre[8], s_cnt[8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_chunks = (p.n_local + 31) / 32;
     const int c = blockIdx.x * 8 + warp, r = c * 32 + lane;
     const bool in = r < p.n_local;
     const int64_t g = in ? (p.bucket ? p.bucket[r] : r) : 0;
-    const float fill = Q4 && p.h_uncleared && p.fill_bias && in ? fmaxf(p.fill_bias[g], 0.f) : 0.f;
+    const float fill = Q4 && !BLOCKS && p.fill_bias && in ? fmaxf(p.fill_bias[g], 0.f) : 0.f;
     constexpr int UN = 8;
     pdl_launch();
     pdl_wait();
@@ -385,14 +385,13 @@ __global__ void __launch_bounds__(256) k_coef(const CoefP p) {
     const int t0 = blockIdx.y * UN;
     // (lanes past the last row stand for the rest of its block, which counts where h holds something there)
     const int64_t first = __shfl_sync(0xffffffffu, g, 0);
-    const bool tail = Q4 && !p.h_uncleared && !in && c < n_chunks;
-    const bool whole = !Q4 || p.h_uncleared || __all_sync(0xffffffffu, (first & 31) == 0 && (!in || g == first + lane));
+    const bool whole = !BLOCKS || __all_sync(0xffffffffu, (first & 31) == 0 && (!in || g == first + lane));
     float v[UN], l[UN];                                               // (on their way while the positions are counted)
 #pragma unroll
     for (int u = 0; u < UN; u++) {
         v[u] = 0.f; l[u] = 0.f;
         if (in && t0 + u < p.T) { v[u] = p.h[(size_t)(t0 + u) * p.h_stride + g]; l[u] = p.idx[(size_t)(t0 + u) * p.idx_stride + g]; }
-        if (tail && whole && t0 + u < p.T) v[u] = p.h[(size_t)(t0 + u) * p.h_stride + first + lane];
+        if (BLOCKS && whole && !in && c < n_chunks && t0 + u < p.T) v[u] = p.h[(size_t)(t0 + u) * p.h_stride + first + lane];
     }
     int sum = 0;
 #pragma unroll 4
@@ -416,7 +415,7 @@ __global__ void __launch_bounds__(256) k_coef(const CoefP p) {
     for (int u = 0; u < UN; u++) {
         const bool on = in && !(l[u] < p.threshold);                  // (a NaN logit counts as active)
         if (!Q4) { o[u] = on ? v[u] : 0.f; continue; }
-        o[u] = on || !p.h_uncleared ? v[u] : fill;                    // what the graph leaves at an inactive neuron
+        o[u] = on || BLOCKS ? v[u] : fill;                            // what the graph leaves at an inactive neuron
     }
     if (Q4) {
         float amax[UN];
@@ -426,7 +425,7 @@ __global__ void __launch_bounds__(256) k_coef(const CoefP p) {
         for (int s = 16; s > 0; s >>= 1)
 #pragma unroll
             for (int u = 0; u < UN; u++) { const float a = __shfl_xor_sync(0xffffffffu, amax[u], s); if (whole) amax[u] = fmaxf(amax[u], a); }
-        if (!whole && in) {                                           // a bucket that cuts blocks: every row looks its own up
+        if (BLOCKS && !whole && in) {                                 // a bucket that cuts blocks: every row looks its own up
 #pragma unroll
             for (int u = 0; u < UN; u++)
                 for (int k = 0; k < 32 && t0 + u < p.T; k++) amax[u] = fmaxf(amax[u], fabsf(p.h[(size_t)(t0 + u) * p.h_stride + (g & ~(int64_t)31) + k]));
@@ -451,17 +450,25 @@ int launch_coef(const CoefArgs & a, cudaStream_t st) {
     CoefP p;
     p.h = a.h; p.h_stride = a.h_stride; p.idx = a.idx; p.idx_stride = a.idx_stride; p.threshold = a.threshold;
     p.bucket = a.bucket; p.masks = a.masks; p.list = a.list_out; p.count = a.count_out; p.n_local = (int)a.n_local; p.T = a.T;
-    p.fill_bias = a.fill_bias; p.h_uncleared = a.h_uncleared ? 1 : 0; p.coef = a.coef; p.coef_stride = a.coef_stride; p.exact = a.exact ? 1 : 0;
+    p.fill_bias = a.fill_bias; p.coef = a.coef; p.coef_stride = a.coef_stride; p.exact = a.exact ? 1 : 0;
     const int n_chunks = (int)((a.n_local + 31) / 32);
     const dim3 grid((n_chunks + 7) / 8, (a.T + 7) / 8);
-    if (a.wtype == PI_TYPE_Q4_0) PI_CUDA(launch_k(k_coef<true>, grid, dim3(256), 0, st, a.pdl, p));
-    else                         PI_CUDA(launch_k(k_coef<false>, grid, dim3(256), 0, st, a.pdl, p));
+    if (a.wtype != PI_TYPE_Q4_0) PI_CUDA(launch_k(k_coef<false, false>, grid, dim3(256), 0, st, a.pdl, p));
+    else if (a.h_uncleared)      PI_CUDA(launch_k(k_coef<true, false>, grid, dim3(256), 0, st, a.pdl, p));
+    else                         PI_CUDA(launch_k(k_coef<true, true>, grid, dim3(256), 0, st, a.pdl, p));
     return PI_OK;
 }
 
 // ---------------------------------------------------------------------------------------------- launch
 // At most 16 CTAs per slice (a partial vector each): more would cost the reader of the pieces more than they save.
-static int axpy_mm_group(int T) {                                      // tokens of a group: 8, 16, 32, or the equal share of up to 64 rounded up
+// Tokens of a group: 8, 16, 32, or the equal share of up to 64 rounded up.  Few large groups expand a row's fragments less often, a group's
+// products are made for all of its columns.  us with the groups taken | the others, 11008 x 4096 FP16 and 28672 x 8192 Q4_0 (exact):
+//    40 tokens  1 x 40   43.2 |  1 x 48 44.4,   1 x 64  50.0,  2 x 32  48.6       233.6 |  272.7,  356.9,  371.3
+//    80         2 x 40   64.5 |  2 x 48 67.2,   2 x 64  78.2,  3 x 32  71.1       448.1 |  525.7,  690.2,  557.4
+//    96         2 x 48   71.9 |  3 x 40 82.0,   2 x 64  82.8,  3 x 32  74.1       536.3 |  652.5,  699.6,  565.9
+//   128         2 x 64   93.6 |  4 x 40 103.3,  3 x 48  95.5,  4 x 32  95.4       715.6 |  863.0,  783.4,  748.7
+//   256         4 x 64  163.6 |  7 x 40 168.5,  6 x 48 166.5,  8 x 32 172.4      1393.1 | 1504.3, 1545.9, 1478.7
+static int axpy_mm_group(int T) {
     if (T <= 32) return T <= 8 ? 8 : T <= 16 ? 16 : 32;
     const int n = (T + 63) / 64, share = (T + n - 1) / n;
     return share <= 40 ? 40 : share <= 48 ? 48 : 64;

@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(ARG_THREADS) k_argmax(const float * __restrict
 }
 
 // Tokens of a prompt that go through the layers together, whatever the engine's batch: a chunk reads the weights once, and 77 tokens of
-// the 7B shape in one chunk take 1.0 ms where three chunks of up to 32 took 3.5.  256: beyond it the products are all that is left.
+// eight layers of the 7B shape in one chunk take 1.98 ms, in three chunks of up to 32 3.08.  256: beyond it the products are all that is left.
 static constexpr int PROMPT_CHUNK = 256;
 
 // A step's token ids and positions travel as kernel arguments: one launch instead of two copies, and the caller's arrays are free again

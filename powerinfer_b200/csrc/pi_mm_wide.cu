@@ -497,7 +497,10 @@ static int mw_sel(const MwP & p, bool pdl, cudaStream_t st) {
     return mw_go<WT, WM, WN, NT, true, false>(p, pdl, st);
 }
 
-// the narrowest tile that holds the tokens
+// The narrowest tile that holds the tokens: the products of a tile are made for all of its columns.  us at this step | at the next wider one,
+// 12288 x 4096 FP16 and 10240 x 8192 Q4_0: 64 tokens 33.7 | 37.7, 69.2 | 81.7; 80 38.3 | 41.2, 82.8 | 96.0; 96 41.7 | 50.1, 96.5 | 113.7;
+// 128 50.5 | 59.6, 114.6 | 144.1; 192 58.1 | 74.9, 148.7 | 189.6.  (2..32 tokens go to k_mm.)  Steps at 112, 160 and 224 would give token
+// counts below them up to half of those differences, for six more instances each.
 template <int WT>
 static int mw_tokens(const MwP & p, bool pdl, cudaStream_t st) {
     if (p.T <= 64)  return mw_sel<WT, 6, 2, 4>(p, pdl, st);
