@@ -560,16 +560,18 @@ def main():
                        "GBps": round(gbs, 1), "frac_of_measured_peak": round(gbs / peak, 3),
                        "serialised_ms_per_step": round(stage_ms[st], 4)}
         dom = max(ops, key=lambda k: ops[k]["ms_per_step"])
-        roofline = {"bound": "hbm", "kernel": {"qkv": "k_gemv_ring_w (dense, QKV rows)", "out_proj": "k_gemv_ring_w (dense, out-proj)",
+        batch_kernels = {"qkv": "k_mm (dense, QKV rows)", "out_proj": "k_mm (dense, out-proj)", "predictor": "k_mm (dense F16, fc1 + fc2)",
+                         "up_gate": "k_mm (gather, up+gate)", "down": "k_axpy_mm (with its coefficients)", "lm_head": "k_mm (dense, lm head)"}
+        roofline = {"bound": "hbm", "kernel": (batch_kernels if T > 1 else {"qkv": "k_gemv_ring_w (dense, QKV rows)", "out_proj": "k_gemv_ring_w (dense, out-proj)",
                                                "predictor": "k_gemv_ring_g + k_gemv_ring_w (dense F16, fc1 + fc2)", "up_gate": "k_gather_rows (gather, up+gate)",
                                                "down": "k_axpy_rows",
-                                               "sparse_ffn": "k_ffn_rows (gather over up + gate rows, activation, axpy over down rows: one launch)", "lm_head": "k_gemv_ring_w (dense, lm head)"}[dom],
+                                               "sparse_ffn": "k_ffn_rows (gather over up + gate rows, activation, axpy over down rows: one launch)", "lm_head": "k_gemv_ring_w (dense, lm head)"})[dom],
                     "achieved": ops[dom]["GBps"], "peak": peak, "unit": "GB/s", "frac": round(ops[dom]["GBps"] / peak, 3),
                     "peak_source": f"of {peak_kind}", "launches_per_step": ops[dom]["launches_per_step"],
                     "bytes_per_launch": bytes_tok[dom] / world / ops[dom]["launches_per_step"],
                     "mean_launch_us": ops[dom]["us_per_launch"],
                     "how": "this stage's kernels for every layer, back to back in a CUDA graph as inside a step, CUDA events around 5 replays",
-                    "traffic": ncu_traffic(cfg_name).get(dom) if world == 1 else None}
+                    "traffic": ncu_traffic(cfg_name).get(dom) if world == 1 and T == 1 else None}
         step_bytes = bytes_tok["total"] / world
         line = {"metric": metric, "value": K * T / (ms * 1e-3), "unit": "tok/s", "n_gpus": world, "steps": K, "warmup": W,
                 "ms_per_step": ms / K, "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
