@@ -182,8 +182,11 @@ class DecodeEngine:
     def decode(self, tokens, pos, want_logits: bool = True):
         T = len(tokens)
         n_tokens, n_pos, n_logits, n_argmax, (p_tokens, p_pos, p_logits, p_argmax) = self._host_io
-        n_tokens[:T] = tokens.cpu() if isinstance(tokens, torch.Tensor) else tokens
-        n_pos[:T] = pos.cpu() if isinstance(pos, torch.Tensor) else pos
+        for staged, given in ((n_tokens, tokens), (n_pos, pos)):
+            try:
+                staged[:T] = given
+            except TypeError:                                     # tensors of the GPU, as a whole or in a list
+                staged[:T] = torch.as_tensor(given, dtype=torch.int32).cpu()
         check(lib.pi_engine_decode_host(self.handle, p_tokens, p_pos, T, p_logits if want_logits else None, p_argmax, self.st))
         return (n_logits[:T] if want_logits else None), n_argmax[:T]
 

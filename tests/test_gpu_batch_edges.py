@@ -361,3 +361,51 @@ def test_attention_of_a_batch_in_a_long_context(ops, heads, kv, hd, n_ctx):
         assert torch.equal(kc[s, n - 1], k[t].half()) and torch.equal(vc[s, n - 1], v[t].half())
         ref, bound = attention_reference(q[t], kc[s, :n], vc[s, :n], heads, kv)
         assert ((got[t] - ref).abs() <= bound).all(), t
+
+
+def test_decode_takes_ids_in_any_container(ops):
+    """Lists, arrays and tensors, of the GPU too, as a whole and one by one."""
+    from powerinfer_b200 import engine
+    spec = synth.ModelSpec(arch=synth.ARCH_LLAMA, wtype=synth.F16, n_layer=1, d=256, n_ff=512, n_head=2, n_head_kv=2, rank=64, n_vocab=64, n_ctx=32, seed=3)
+    eng = engine.DecodeEngine(spec, synth.build_model(spec), max_batch=2)
+    ref = eng.decode([5, 9], [0, 3])[0].copy()
+    ids, at = torch.tensor([5, 9]), torch.tensor([0, 3])
+    for tokens, pos in ((np.array([5, 9]), (0, 3)), (ids, at), (ids.cuda(), at.cuda()), (list(ids), list(at)), (list(ids.cuda()), list(at.cuda())), (ids.int().cuda(), [0, 3])):
+        assert np.array_equal(eng.decode(tokens, pos)[0], ref)
+    eng.close()
+
+
+@pytest.mark.parametrize("wtype", [synth.F16, synth.Q4_0])
+@pytest.mark.parametrize("T", [1, 4, 40])
+def test_operators_in_a_captured_graph(ops, wtype, T):
+    """Every operator of an FFN captured behind a copy and behind another stream's work, replayed with other inputs."""
+    gen = generator(T)
+    F, d = 1024, 512
+    up, gate, down = (weight(ops, wtype, F, d, gen) for _ in range(3))
+    fc1, fc2 = weight(ops, synth.F16, 64, d, gen), weight(ops, synth.F16, F, 64, gen)
+    x, src = torch.zeros(T, d, device="cuda"), torch.randn(T, d, device="cuda", generator=gen)
+    bucket = torch.arange(0, 512, device="cuda", dtype=torch.int32)
+    half = [weight(ops, wtype, 512, d, gen) for _ in range(2)]
+
+    def step():
+        x.copy_(src)
+        idx = ops.predictor(fc1, fc2, x)
+        h = torch.relu(ops.ggml_mul_mat_idx(gate, x, idx)) * ops.ggml_mul_mat_idx(up, x, idx)
+        return (idx, h, ops.ggml_axpy(down, h, idx), ops.sparse_ffn(up, gate, down, x, idx), ops.ggml_mul_mat(up, x),
+                ops.sparse_ffn(half[0], None, half[1], x, idx, gpu_bucket=bucket))
+
+    eager = step()                                                    # (the workspace has its size)
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            src.mul_(1.0)
+        torch.cuda.current_stream().wait_stream(side)
+        captured = step()
+    for scale in (1.0, -0.5):
+        src.mul_(scale)
+        graph.replay()
+        torch.cuda.synchronize()
+        for a, b in zip(captured, eager if scale == 1.0 else step()):
+            assert torch.equal(a, b)
