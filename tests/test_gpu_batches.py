@@ -13,7 +13,7 @@ from powerinfer_b200 import synth
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
-TOKENS = [2, 8, 9, 16, 17, 24, 25, 32, 33, 64, 65, 77, 128, 129, 256, 261]
+TOKENS = [2, 8, 9, 16, 17, 24, 25, 32, 33, 48, 64, 65, 77, 96, 128, 129, 256, 261]
 
 
 def weight(ops, wtype, rows, cols, gen):

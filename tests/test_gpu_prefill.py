@@ -136,6 +136,13 @@ def test_prompt_over_many_neurons_per_cta(engine_mod, wtype):
                                                      n_ctx=256, firing=0.9, seed=6), (40, 77, 130, 256))
 
 
+def test_prompt_with_rounded_factors(engine_mod):
+    """Q4_0 prompts of an engine for several sequences at a width of whole 1024 columns: the down projection's factors are rounded to FP16, in
+    token groups of 40, 48 and 64."""
+    against_single_steps(engine_mod, synth.ModelSpec(arch=synth.ARCH_LLAMA, wtype=synth.Q4_0, n_layer=1, d=1024, n_ff=2048, n_head=8, n_head_kv=8, rank=64, n_vocab=256,
+                                                     n_ctx=256, firing=0.5, seed=9), (40, 48, 90, 130))
+
+
 @pytest.mark.parametrize("heads,kv,n_ctx", [(4, 4, 2048), (8, 2, 2304), (4, 2, 4096)])
 def test_prompt_in_a_long_context(engine_mod, heads, kv, n_ctx):
     """Contexts whose scores do not fit the several-token attention (head_dim 128 from 1921, 64 from 2113 positions): a store pass, then one
