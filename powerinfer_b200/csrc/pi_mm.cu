@@ -195,7 +195,9 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
             s_src += 8 * MM_RINGS;
         }
     };
-    // The activation of a slice: 16-byte pieces, 8 (Q4_0: 4) tokens per instruction; tokens past the last one copy the last one again
+    // The activation of a slice: 16-byte pieces, 8 (Q4_0: 4) tokens per instruction.  Columns of tokens past the last one keep whatever shared
+    // memory holds, like the rows past a tile: no product mixes columns.  (Filled with the last token's bytes they cost what its lines
+    // cost at the L2, which every CTA asks for at once: 10240 x 8192 Q4_0, 2 tokens 30.7 us where it is 18.4, 8 tokens 18.9.)
     constexpr int XN = Q4 ? 2 * NT : NT, XT = Q4 ? 4 : 8;             // instructions, tokens of one
     const int xr = Q4 ? lane >> 3 : r8, xc = Q4 ? lane & 7 : c4;
     const uint32_t x_dst = Q4 ? (uint32_t)(xr * 128 + ((xc ^ xr) & 7) * 16) : (uint32_t)(xr * 64 + ((xc ^ (xr >> 1)) & 3) * 16);
@@ -204,9 +206,9 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
     const char * d_src = reinterpret_cast<const char *>(p.x.d) + (lane & 3) * 4;
     auto start_x = [&]() {
 #pragma unroll
-        for (int i = 0; i < XN; i++) x_at[i] = min(xr + i * XT, p.T - 1) * (Q4 ? p.nb * 16 : p.ncols * 2);
+        for (int i = 0; i < XN; i++) x_at[i] = (xr + i * XT) * (Q4 ? p.nb * 16 : p.ncols * 2);
 #pragma unroll
-        for (int i = 0; i < (Q4 ? NT : 0); i++) d_at[i] = min((lane >> 2) + i * 8, p.T - 1) * p.nb * 4;
+        for (int i = 0; i < (Q4 ? NT : 0); i++) d_at[i] = ((lane >> 2) + i * 8) * p.nb * 4;
     };
     auto issue_x = [&](int j, int slot) {
         const int s = me + j * MM_RINGS;
@@ -218,12 +220,12 @@ __global__ void __launch_bounds__(MM_THREADS, 1) k_mm(const MmP p) {
         } else {
             const char * src = x_src + s * 64;
 #pragma unroll
-            for (int i = 0; i < XN; i++) mm_cp16(Q4 && (i & 1) ? (to + i * 512) ^ 64u : to + i * 512, src + x_at[i]);      // (token + 4: piece ^ 4)
+            for (int i = 0; i < XN; i++) if (xr + i * XT < p.T) mm_cp16(Q4 && (i & 1) ? (to + i * 512) ^ 64u : to + i * 512, src + x_at[i]);      // (token + 4: piece ^ 4)
         }
         if (Q4) {
             const uint32_t dt = base + TP * 128 + rt * 8 + ((lane & 3) * TP + (lane >> 2)) * 4;
 #pragma unroll
-            for (int i = 0; i < (Q4 ? NT : 0); i++) mm_cp4(dt + i * 32, d_src + s * 16 + d_at[i]);
+            for (int i = 0; i < (Q4 ? NT : 0); i++) if ((lane >> 2) + i * 8 < p.T) mm_cp4(dt + i * 32, d_src + s * 16 + d_at[i]);
         }
     };
     auto start_tile = [&](int tile) {

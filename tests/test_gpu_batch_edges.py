@@ -409,3 +409,31 @@ def test_operators_in_a_captured_graph(ops, wtype, T):
         torch.cuda.synchronize()
         for a, b in zip(captured, eager if scale == 1.0 else step()):
             assert torch.equal(a, b)
+
+
+def test_fewer_tokens_cost_no_more(ops):
+    """2 and 8 tokens take the same instance of the same kernel, and the same bytes of weights: 2 may not take longer (they did, 1.6 times,
+    when the token columns without a token were filled with copies of the last one).  The margin is for the clock of the events."""
+    gen = generator(7)
+    W = weight(ops, synth.Q4_0, 10240, 8192, gen)
+
+    def best(T):
+        x = torch.randn(T, 8192, device="cuda", generator=gen)
+        g = torch.cuda.CUDAGraph()
+        ops.ggml_mul_mat(W, x)
+        torch.cuda.synchronize()
+        with torch.cuda.graph(g):
+            for _ in range(8):
+                ops.ggml_mul_mat(W, x)
+        times = []
+        for _ in range(10):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            g.replay()
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    two, eight = best(2), best(8)
+    assert two <= 1.2 * eight, (two, eight)
