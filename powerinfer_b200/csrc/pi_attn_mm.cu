@@ -329,9 +329,19 @@ static size_t attn_mm_smem(const AttnArgs & a, int * P, int * R) {
 }
 
 // Several tokens and head_dim 64 or 128 whose scores fit (16 rows: contexts of up to about 1900 positions); the others keep one
-// CTA per head and token.
+// CTA per head and token.  So do steps of several sequences whose CTAs per head and token fit the SMs at once: nothing is gained there
+// by reading a KV head once for all of its query heads, and a CTA of k_attention_row has more rows in flight.  us in k_attention_row | here,
+// 8 sequences of 8 heads of 64: 200 positions 5.5 | 7.1, 1000 8.5 | 16.3, 3500 19.8 | 44.3; 4 of 32 heads of 128, 1000 positions
+// 13.1 | 20.8.  With more CTAs than SMs: 32 sequences of 8 heads of 64 over 2 KV heads, 200 positions
+// 9.6 | 7.1, 1000 15.8 | 16.4; 8 of 64 heads of 128 over 8 KV heads, 500 positions 28.0 | 13.2.
+// Nor do steps with one or two query heads per KV head (one for 128) gain anything in long contexts: one or two rows of 16 are at work,
+// and the scores take the room of what could be in flight.  16 sequences of 12 heads of 64, 4000 of 8192 positions 81.6 | 103.6, of 4096
+// 81.0 | 75.9; 13 of 24 heads of 64 over 12 KV heads, 6000 of 8192 155.8 | 170.1; 13 of 12 heads of 128, 6000 of 12288 206 | 252, 32 of 32, 8000 of 8192
+// 1050 | 1070.
 bool attention_mm_takes(const AttnArgs & a) {
     int P, R;
+    if (a.store_mode == 0 && (int64_t)a.T * a.n_head <= sm_count()) return false;
+    if (a.store_mode == 0 && a.n_head / a.n_head_kv * a.head_dim <= 128 && a.n_ctx > 64 * a.head_dim) return false;
     return a.T >= 2 && (a.head_dim == 64 || a.head_dim == 128) && a.n_ctx > 0 && attn_mm_smem(a, &P, &R) <= AM_SMEM_MAX;
 }
 

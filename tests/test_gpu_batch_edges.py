@@ -138,7 +138,7 @@ def attention_reference(q, k, v, heads, kv):
 
 
 @pytest.mark.parametrize("hd", [64, 128])
-@pytest.mark.parametrize("T", [1, 3])
+@pytest.mark.parametrize("T", [1, 3, 40])
 def test_attention_result_at_any_float_address(ops, hd, T):
     """The F32 result goes to any address that is aligned to a float."""
     from powerinfer_b200._lib import check, lib
@@ -147,7 +147,7 @@ def test_attention_result_at_any_float_address(ops, hd, T):
     kc, vc = (torch.randn(T, n_ctx, kv * hd, device="cuda", generator=gen).half() for _ in range(2))
     q = torch.randn(T, heads * hd, device="cuda", generator=gen)
     k, v = (torch.randn(T, kv * hd, device="cuda", generator=gen) for _ in range(2))
-    pos = torch.tensor([40, 3, 63][:T], dtype=torch.int32, device="cuda")
+    pos = torch.tensor([(40, 3, 63)[t % 3] for t in range(T)], dtype=torch.int32, device="cuda")
     seq = torch.arange(T, dtype=torch.int32, device="cuda")
     buf = torch.zeros(T * heads * hd + 8, device="cuda")
     for off in (0, 1, 2, 3):
@@ -346,17 +346,20 @@ def test_attention_of_one_token_far_into_a_sequence(ops, hd, n_ctx):
             assert ((got.double().view(heads, hd) - ref).abs() <= bound).all(), (pos, scale)
 
 
-@pytest.mark.parametrize("heads,kv,hd,n_ctx", [(4, 2, 128, 2500), (16, 1, 128, 1920), (16, 1, 128, 2500), (16, 1, 64, 2500), (16, 1, 128, 3700), (20, 1, 64, 2100)])
-def test_attention_of_a_batch_in_a_long_context(ops, heads, kv, hd, n_ctx):
-    """Scores of 16 rows fit up to 1920 (head_dim 64: 2112) positions; longer contexts, and those beyond 3584, have a kernel each."""
+@pytest.mark.parametrize("heads,kv,hd,n_ctx", [(4, 2, 128, 2500), (16, 1, 128, 1920), (16, 1, 128, 2500), (16, 1, 64, 2500), (16, 1, 128, 3700), (20, 1, 64, 2100), (12, 12, 64, 4097)])
+@pytest.mark.parametrize("many", [False, True])
+def test_attention_of_a_batch_in_a_long_context(ops, heads, kv, hd, n_ctx, many):
+    """Scores of 16 rows fit up to 1920 (head_dim 64: 2112) positions; longer contexts, those beyond 3584, and steps whose CTAs per head and
+    token all fit the SMs at once have a kernel each."""
     gen = generator(heads + n_ctx)
-    pos = torch.tensor([n_ctx - 1, 700, 1300], dtype=torch.int32, device="cuda")
-    seq = torch.tensor([2, 0, 1], dtype=torch.int32, device="cuda")
-    kc, vc = (torch.randn(3, n_ctx, kv * hd, device="cuda", generator=gen).half() for _ in range(2))
-    q = torch.randn(3, heads * hd, device="cuda", generator=gen)
-    k, v = (torch.randn(3, kv * hd, device="cuda", generator=gen) for _ in range(2))
-    got = ops.attention_decode(q, k, v, kc, vc, pos, heads, kv, seq=seq).double().view(3, heads, hd)
-    for t in range(3):
+    T = torch.cuda.get_device_properties(0).multi_processor_count // heads + 1 if many else 3
+    pos = torch.tensor([(n_ctx - 1, 700, 1300)[t % 3] for t in range(T)], dtype=torch.int32, device="cuda")
+    seq = torch.arange(T, device="cuda").roll(1).int()
+    kc, vc = (torch.randn(T, n_ctx, kv * hd, device="cuda", generator=gen).half() for _ in range(2))
+    q = torch.randn(T, heads * hd, device="cuda", generator=gen)
+    k, v = (torch.randn(T, kv * hd, device="cuda", generator=gen) for _ in range(2))
+    got = ops.attention_decode(q, k, v, kc, vc, pos, heads, kv, seq=seq).double().view(T, heads, hd)
+    for t in range(T):
         s, n = int(seq[t]), int(pos[t]) + 1
         assert torch.equal(kc[s, n - 1], k[t].half()) and torch.equal(vc[s, n - 1], v[t].half())
         ref, bound = attention_reference(q[t], kc[s, :n], vc[s, :n], heads, kv)
