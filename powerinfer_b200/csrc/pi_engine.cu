@@ -8,6 +8,7 @@
 // replicated.  The two partial d_model vectors per layer (attention out-projection, FFN down-projection) are
 // exchanged by pi_exchange.cu; a rank never reads another rank's memory.
 #include "pi_common.cuh"
+#include "pi_step.cuh"
 
 #include <cmath>
 #include <cstdlib>
@@ -195,6 +196,9 @@ struct pi_engine {
     bool rows1;                              // one token: masks-only compaction + register-streaming sparse kernels (shape eligible)
     long long wait_cycles;                   // bound of the exchange waits (0: about a second)
     unsigned skip_mask;                      // set only inside pi_engine_time_stage: the stages left out of the captured sequence
+    StepPlan step;                           // the step of one sequence as one launch (step.ok)
+    StepP step_p;                            // ... and its arguments, but for those of a call
+    StepLayer * step_layers; char * step_words; unsigned int * step_ctl;
 };
 
 static constexpr int NORM_MAX_GROUPS = 48;      // partial vectors the norm adds itself; more go through k_reduce_partials first
@@ -244,8 +248,82 @@ static void carve(pi_engine * e, void * ws, size_t ws_bytes, bool dry, size_t * 
     e->act_q = cv.act(c.wtype, c.d, T);
     e->act_p = cv.act(PI_TYPE_F16, c.d, T);
     e->act_o = cv.act(c.wtype, e->dq, T);
+    if (e->step.ok) {
+        e->step_layers = cv.take<StepLayer>(c.n_layer); e->step_ctl = cv.take<unsigned int>(2); e->step_words = cv.take<char>(e->step.words);
+    }
     *need = (size_t)(cv.p - (char *)ws);
     if (!cv.ok && !dry) *need = (size_t)-1;
+}
+
+// The one-launch step takes one sequence of an unsharded model; where a diagnostic switch names a kernel of the launch sequence, that
+// sequence runs.
+static bool step_wanted() {
+    const char * v = getenv("PI_STEP");
+    if (v && v[0] == '0') return false;
+    for (const char * n : {"PI_PDL", "PI_ROWS", "PI_FFN_FUSED", "PI_FFN_CS", "PI_FC2_MASKS", "PI_QKV_PRE", "PI_RING_W", "PI_RING_G", "PI_RING_RW", "PI_RING_CPS", "PI_RING_KB",
+                           "PI_RING_SMALL", "PI_NORM_CLUSTER"})
+        if (getenv(n)) return false;
+    return true;
+}
+
+static void plan_step(pi_engine * e, bool tied) {
+    const pi_engine_config & c = e->c;
+    e->step = StepPlan();
+    if (c.n_ranks != 1 || !step_wanted()) return;
+    StepShape s;
+    s.wtype = c.wtype; s.head_type = tied ? PI_TYPE_F16 : c.wtype; s.falcon = c.arch == PI_ARCH_FALCON;
+    s.d = c.d; s.F = e->F; s.dkv = e->dkv; s.rank = c.rank; s.n_vocab = c.n_vocab; s.hd = e->hd; s.n_ctx = c.n_ctx;
+    step_plan(s, e->step);
+}
+
+// arguments of the one-launch step; leaves step.ok false where the model's weights do not allow it
+static int setup_step(pi_engine * e, cudaStream_t st) {
+    const pi_engine_config & c = e->c;
+    bool ok = rows_eligible(c.wtype, e->F, c.d);
+    std::vector<StepLayer> ly(c.n_layer);
+    const bool gated = e->layers[0].gate != nullptr;
+    auto al = [&](const void * p) { if (((uintptr_t)p & 15) != 0) ok = false; return p; };
+    for (int i = 0; i < c.n_layer; i++) {
+        const pi_layer_weights & L = e->layers[i];
+        const void * w[7] = {L.wqkv, L.wo, L.fc1, L.fc2, L.up, L.gate, L.down_t};
+        const bool falcon = c.arch == PI_ARCH_FALCON;
+        const float * f[8] = {L.attn_norm_w, L.attn_norm_b, falcon ? L.attn_norm2_w : L.ffn_norm_w, falcon ? L.attn_norm2_b : L.ffn_norm_b, L.bqkv, L.bo, L.up_b, L.down_b};
+        for (int k = 0; k < 7; k++) { ly[i].w[k] = (const uint8_t *)al(w[k]); if (!w[k] && k != ST_GATE) ok = false; }
+        for (int k = 0; k < 8; k++) ly[i].f[k] = (const float *)al(f[k]);
+        if ((L.gate != nullptr) != gated || (c.wtype == PI_TYPE_Q4_0 && L.up_b)) ok = false;
+        ly[i].pad = 0;
+    }
+    al(e->g.output); al(e->g.tok_embd); al(e->g.out_norm_w); al(e->g.out_norm_b); al(e->k_cache); al(e->v_cache);
+    if (!ok) { e->step.ok = false; return PI_OK; }
+    const StepPlan & pl = e->step;
+    StepP & p = e->step_p;
+    memset(&p, 0, sizeof p);
+    p.layers = e->step_layers; p.n_layer = c.n_layer;
+    p.d = c.d; p.F = e->F; p.rank = c.rank; p.dq = e->dq; p.dkv = e->dkv; p.n_head = c.n_head; p.n_head_kv = c.n_head_kv; p.hd = e->hd; p.n_ctx = c.n_ctx;
+    p.n_vocab = c.n_vocab; p.n_pos = c.n_pos; p.max_batch = c.max_batch;
+    p.q4 = c.wtype == PI_TYPE_Q4_0; p.falcon = c.arch == PI_ARCH_FALCON; p.rms = c.arch == PI_ARCH_LLAMA; p.neox = p.falcon;
+    p.relu = gated ? (e->gate_sym ? 1 : 0) : 1; p.head_type = e->g.output ? c.wtype : PI_TYPE_F16;
+    p.eps = c.norm_eps; p.threshold = c.threshold;
+    p.tok_embd = (const __half *)e->g.tok_embd; p.pos_embd = (const __half *)e->g.pos_embd; p.head = (const uint8_t *)(e->g.output ? e->g.output : e->g.tok_embd);
+    p.out_w = e->g.out_norm_w; p.out_b = e->g.out_norm_b;
+    p.cs = c.arch != PI_ARCH_OPT ? e->cs : nullptr; p.k_cache = e->k_cache; p.v_cache = e->v_cache;
+    char * w = e->step_words;
+    auto take = [&](size_t bytes) { char * r = w; w += up256(bytes); return r; };
+    const size_t d = c.d, F = e->F;
+    p.x = (unsigned long long *)take(2 * d * 8); p.x2 = (unsigned long long *)take(2 * d * 8); p.qkv = (unsigned long long *)take(2 * (d + 2 * e->dkv) * 8);
+    p.h = (unsigned long long *)take(2 * F * 8); p.part = (unsigned long long *)take(2 * (size_t)pl.groups * d * 8);
+    p.acto = (uint32_t *)take(2 * d * 4); p.acts = (uint32_t *)take(2 * (d / 32) * 4); p.hid = (uint32_t *)take(2 * (size_t)c.rank * 4); p.maskw = (uint32_t *)take(2 * (F / 8) * 4);
+    p.logits = e->logits; p.tokens = e->tokens; p.positions = e->pos; p.argmax = e->argmax;
+    p.step_no = e->step_ctl; p.abort = e->step_ctl + 1; p.status = e->status; p.ticket = e->amax_ticket; p.best = e->amax_best; p.rows_total = e->active_total;
+    p.row_bytes = (int64_t)pi_row_bytes(c.wtype, c.d);
+    for (int i = 0; i < ST_N_MAT; i++) p.mat[i] = pl.mat[i];
+    p.slot_bytes = pl.slot_bytes; p.n_slots = pl.n_slots; p.window = pl.window; p.groups = pl.groups; p.wpt = pl.wpt;
+    p.off_a = pl.off_a; p.off_b = pl.off_b; p.off_c = pl.off_c; p.off_h = pl.off_h; p.off_part = pl.off_part;
+    PI_CUDA(cudaMemcpyAsync(e->step_layers, ly.data(), ly.size() * sizeof(StepLayer), cudaMemcpyHostToDevice, st));
+    PI_CUDA(cudaMemsetAsync(e->step_ctl, 0, 8, st));
+    PI_CUDA(cudaMemsetAsync(e->step_words, 0, pl.words, st));       // (no layer has the number 0)
+    PI_CUDA(cudaStreamSynchronize(st));
+    return PI_OK;
 }
 
 // (a sharded run exchanges whole steps through mailboxes sized for the batch)
@@ -281,9 +359,13 @@ size_t pi_engine_workspace_bytes(const pi_engine_config * cfg) {
     e.hd = cfg->d / cfg->n_head; e.dq = cfg->d / cfg->n_ranks; e.dkv = e.hd * cfg->n_head_kv / cfg->n_ranks;
     e.F = cfg->n_ff / cfg->n_ranks; e.T_max = cfg->max_batch; e.P_max = prompt_chunk(*cfg);
     e.G = axpy_groups(cfg->wtype, cfg->d, cfg->max_batch);
-    size_t need = 0;
-    carve(&e, nullptr, 0, true, &need);
-    return need + 256;
+    size_t need = 0, most = 0;
+    for (int tied = 0; tied < 2; tied++) {                           // (whether the lm head is the embedding shows when the weights come)
+        plan_step(&e, tied);
+        carve(&e, nullptr, 0, true, &need);
+        most = std::max(most, need);
+    }
+    return most + 256;
 }
 
 size_t pi_engine_kv_bytes(const pi_engine_config * cfg) {
@@ -311,7 +393,9 @@ int pi_engine_create(const pi_engine_config * cfg, const pi_model_weights * gw, 
     e->F = cfg->n_ff / cfg->n_ranks; e->T_max = cfg->max_batch; e->P_max = prompt_chunk(*cfg);
     e->G = axpy_groups(cfg->wtype, cfg->d, cfg->max_batch);
     size_t need = 0;
+    plan_step(e, !gw->output);
     carve(e, workspace, workspace_bytes, false, &need);
+    if (need == (size_t)-1 && e->step.ok) { e->step = StepPlan(); carve(e, workspace, workspace_bytes, false, &need); }
     if (need == (size_t)-1) { delete e; set_error("engine_create: workspace of %zu bytes is too small", workspace_bytes); return PI_ERR_WORKSPACE; }
     e->k_cache = (__half *)k_cache; e->v_cache = (__half *)v_cache;
     memset(e->graphs, 0, sizeof e->graphs);
@@ -342,6 +426,7 @@ int pi_engine_create(const pi_engine_config * cfg, const pi_model_weights * gw, 
     if (ce == cudaSuccess) ce = cudaMemsetAsync(e->active_total, 0, 8, st);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);            // the host vectors above die at return
     if (ce != cudaSuccess) { delete e; return cuda_fail(ce, "engine_create"); }
+    if (e->step.ok && (rc = setup_step(e, st))) { delete e; return rc; }
     *out = e;
     return PI_OK;
 }
@@ -710,8 +795,20 @@ void * mapped(void * host) {
     return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
 }
 
+// one sequence's step as one launch; `feed`: its token, and where the results go besides the engine's own buffers (null: the token is
+// in the engine's buffers)
+int run_one(pi_engine * e, cudaStream_t st, const Feed * feed = nullptr) {
+    StepP p = e->step_p;
+    p.pred = e->pred_trace ? e->pred_trace : e->pred;
+    p.pred_stride = e->pred_trace ? (int64_t)e->c.max_batch * e->F : 0;
+    if (feed) { p.fed = 1; p.token = feed->token[0]; p.pos = feed->pos[0]; p.logits_host = feed->logits; p.argmax_host = feed->sink; }
+    e->launches = 1;
+    return launch_step(p, e->step, e->layers[0].gate != nullptr, st);
+}
+
 // first call for a batch size: one plain run (fills every per-kernel attribute cache), then capture
 int run_step(pi_engine * e, int T, cudaStream_t st, int mode = 0) {
+    if (T == 1 && mode == 0 && e->step.ok) return run_one(e, st);
     StageTimer tm;
     // A chunk beyond the batch: its length seldom comes again, and its kernels are longer than their launches
     if (T > e->T_max) return enqueue_step(e, T, st, tm, mode);
@@ -768,12 +865,16 @@ int pi_engine_decode_host(pi_engine * e, const int32_t * host_tokens, const int3
     f.sink = host_argmax ? (int32_t *)mapped(host_argmax) : nullptr;
     f.logits = host_logits ? (float *)mapped(host_logits) : nullptr;
     f.n_vocab = e->c.n_vocab;
+    const bool one = T == 1 && e->step.ok;
+    if (one) { if ((rc = run_one(e, st, &f))) return rc; }
+    else {
     k_feed<<<1, PI_MAX_BATCH, 0, st>>>(f, T, e->tokens, e->pos, e->sink, e->logits_sink);
     PI_LAUNCH_CHECK("k_feed");
     if ((rc = run_step(e, T, st))) {
         cudaMemsetAsync(e->sink, 0, (size_t)T * sizeof *e->sink, st);
         cudaMemsetAsync(e->logits_sink, 0, (size_t)T * sizeof *e->logits_sink, st);
         return rc;
+    }
     }
     if (host_argmax && !f.sink) PI_CUDA(cudaMemcpyAsync(host_argmax, e->argmax, (size_t)T * 4, cudaMemcpyDeviceToHost, st));
     if (host_logits && !f.logits) PI_CUDA(cudaMemcpyAsync(host_logits, e->logits, (size_t)T * e->c.n_vocab * 4, cudaMemcpyDeviceToHost, st));

@@ -1,11 +1,10 @@
 // Device helpers shared by the one-token sparse kernels: activity masks -> ranks of the active rows, the Q4_0 x Q8_0 block
 // dot, packed FP32 FMAs.
 #pragma once
-#include "pi_common.cuh"
+#include "pi_act.cuh"
 
 namespace pi {
 
-static constexpr int QK = 32;
 static constexpr int ROWS_THREADS = 512;
 static constexpr int ROWS_WARPS = ROWS_THREADS / 32;
 static constexpr int ROWS_MAX_CHUNKS = 4096;            // mask words one CTA scans (131072 neurons)
