@@ -573,6 +573,13 @@ def main():
                     "how": "this stage's kernels for every layer, back to back in a CUDA graph as inside a step, CUDA events around 5 replays",
                     "traffic": ncu_traffic(cfg_name).get(dom) if world == 1 and T == 1 else None}
         step_bytes = bytes_tok["total"] / world
+        one_launch = launches_per_step == 2 and T == 1                # the step and the feedback kernel
+        if one_launch:
+            gbs = step_bytes / (ms / K * 1e-3) / 1e9
+            roofline.update({"kernel": "k_step (the whole step of one token: one launch)", "achieved": round(gbs, 1), "frac": round(gbs / peak, 3), "launches_per_step": 1,
+                             "bytes_per_launch": step_bytes, "mean_launch_us": round(ms / K * 1e3, 2), "traffic": ncu_traffic(cfg_name).get("step"),
+                             "how": "the timed steps themselves, the feedback kernel between them included; `ops`, `latency_stages` and `stage_ms_profiled` "
+                                    "are the kernels of the launch sequence that sharded runs and batches take"})
         line = {"metric": metric, "value": K * T / (ms * 1e-3), "unit": "tok/s", "n_gpus": world, "steps": K, "warmup": W,
                 "ms_per_step": ms / K, "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
                 "dtype": "q4_0 x q8_0 int8 dot, f32 accumulate" if spec.wtype == 2 else "f16 weights, f32 accumulate",
