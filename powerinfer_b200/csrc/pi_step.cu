@@ -4,7 +4,7 @@
 // What bounds a step is the chain: every node needs the whole vector the node before it made, a layer's bytes are spread over
 // 8 dependent nodes of 5-60 MB, and a kernel per node drains and refills the memory pipeline at every boundary (a layer of the
 // 70B shape: 73 us for 207 MB, 32 us at the copy rate).  Here
-//   weights   a copying warp streams the dense rows of THIS SM (QKV, out-proj, fc1, fc2 of every layer, lm head) through one
+//   weights   copying warps stream the rows of THIS SM (QKV, out-proj, fc1, fc2, gathered rows of every layer, lm head) through one
 //             shared-memory ring, in the order the step needs them and without regard to where the arithmetic is: weights depend
 //             on nothing, so the ring fills while the computing warps wait for another CTA's values.  At most `window` slots are
 //             on their way at a time: the queue in front of the memory stays short, and with it the latency of the small reads

@@ -1,0 +1,122 @@
+"""The one-launch decode step (csrc/pi_step.cu) against the launch sequence it replaces, over the forms it takes: graphs, weight types, head
+sizes, ragged sizes, the edges of its ring plan, contexts beyond one pass of the attention, every / no neuron active.
+
+Two correct implementations differ in the order of their sums, which flips roundings of activations between the nodes (FP16, or the int8 of
+Q8_0): the bounds are those of perf/cases.py for whole steps, relative in the 2-norm: 3e-3 (FP16 weights), 3e-2 (Q4_0).  The predictors lie
+far from the threshold there, so both choose the same neurons."""
+import os
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(arch, wtype, n_layer, d, n_ff, n_head, n_head_kv, rank, n_vocab, n_ctx, firing, pos, batch=1):
+    return dict(kind="decode", arch=arch, wtype=wtype, n_layer=n_layer, d=d, n_ff=n_ff, n_head=n_head, n_head_kv=n_head_kv, rank=rank, n_vocab=n_vocab,
+                n_ctx=n_ctx, firing=firing, batch=batch, pos=pos)
+
+
+CASES = {
+    # d just above the narrowest model, a rank of one unit, a vocabulary that divides nothing, the first position
+    "llama_q4_narrow": _case("llama", "q4_0", 3, 768, 2016, 6, 6, 8, 509, 96, 0.2, 0),
+    "llama_f16_gqa_64": _case("llama", "f16", 2, 1024, 1312, 16, 1, 1368, 1001, 160, 0.3, 158),
+    "llama_f16_pieces": _case("llama", "f16", 2, 5120, 3456, 40, 8, 488, 777, 128, 0.1, 77),
+    "llama_q4_pieces": _case("llama", "q4_0", 1, 12544, 1600, 98, 7, 256, 515, 64, 0.2, 63),
+    "llama_f16_wide": _case("llama", "f16", 1, 9216, 1376, 72, 8, 520, 300, 64, 0.2, 20),
+    "falcon_q4": _case("falcon", "q4_0", 2, 1280, 3904, 20, 5, 552, 600, 200, 0.15, 130),
+    "falcon_f16": _case("falcon", "f16", 3, 2048, 4096, 32, 2, 144, 901, 96, 0.1, 50),
+    "opt_f16": _case("opt", "f16", 2, 1536, 4032, 12, 12, 200, 1003, 128, 0.1, 90),
+    "bamboo_q4": _case("bamboo", "q4_0", 2, 2560, 7776, 20, 20, 208, 1500, 96, 0.2, 33),
+    "bamboo_f16": _case("bamboo", "f16", 2, 1024, 2080, 8, 4, 808, 640, 96, 0.2, 95),
+    "long_context": _case("llama", "q4_0", 2, 1024, 2048, 8, 2, 64, 512, 3584, 0.2, 3583),
+    "all_active": _case("llama", "q4_0", 2, 1024, 8192, 8, 2, 64, 512, 64, 0.9999, 5),
+    "few_active": _case("llama", "f16", 2, 1024, 4096, 8, 2, 64, 512, 64, 1e-5, 5),
+    "row_of_a_batch_engine": _case("llama", "f16", 2, 1024, 2048, 8, 2, 64, 512, 64, 0.2, 9, batch=3),
+}
+
+
+def _engine(case, one, seed=5):
+    cases = pytest.importorskip("perf.cases")
+    old = os.environ.get("PI_STEP")
+    os.environ["PI_STEP"] = "1" if one else "0"
+    try:
+        return cases._prepare_engine(case, seed)["eng"]
+    finally:
+        if old is None:
+            del os.environ["PI_STEP"]
+        else:
+            os.environ["PI_STEP"] = old
+
+
+def _steps(eng, case, n=3):
+    out = []
+    for i in range(n):
+        pos = max(0, min(case["pos"] - (n - 1) + i, case["n_ctx"] - 1))
+        logits, ids = eng.decode([(7 + 31 * i) % case["n_vocab"]], [pos])
+        out.append(np.array(logits[0]))
+        assert int(ids[0]) == int(np.argmax(out[-1]))
+    eng.status()
+    return np.stack(out)
+
+
+def _close(got, want, wtype):
+    rel = np.linalg.norm(got.astype(np.float64) - want) / np.linalg.norm(want.astype(np.float64))
+    assert np.isfinite(got).all() and rel <= (3e-2 if wtype == "q4_0" else 3e-3), rel
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_step_matches_the_launch_sequence(name):
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    case = CASES[name]
+    ref = _engine(case, False)
+    want = _steps(ref, case)
+    assert ref.launches() > 1
+    keys, values, total = ref.k_cache.float().cpu().numpy(), ref.v_cache.float().cpu().numpy(), ref.active_total()
+    ref.close()
+    eng = _engine(case, True)
+    got = _steps(eng, case)
+    assert eng.launches() == 1
+    _close(got, want, case["wtype"])
+    _close(eng.k_cache.float().cpu().numpy(), keys, case["wtype"])
+    _close(eng.v_cache.float().cpu().numpy(), values, case["wtype"])
+    assert eng.active_total() == total
+    # the same bits again, fed from the device as well as from the host, and with the predictor's logits kept
+    eng.enable_trace()
+    again = _steps(eng, case)
+    assert np.array_equal(again[-1], got[-1])
+    assert (eng.predictor_trace(1)[:, 0] != 0).any()
+    pos = max(0, min(case["pos"], case["n_ctx"] - 1))
+    eng.set_inputs_device([(7 + 31 * 2) % case["n_vocab"]], [pos])
+    eng.step_device(1)
+    torch.cuda.synchronize()
+    assert np.array_equal(eng.device_view("logits", 1)[0].cpu().numpy(), got[-1])
+    eng.status()
+    eng.close()
+
+
+def test_steps_of_two_engines_in_two_threads():
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    cs = [CASES["llama_f16_gqa_64"], CASES["falcon_q4"]]
+    engs = [_engine(c, True) for c in cs]
+    want = [_steps(e, c) for e, c in zip(engs, cs)]
+    bad = []
+
+    def work(e, c, w):
+        try:
+            for _ in range(30):
+                if not np.array_equal(_steps(e, c), w):
+                    bad.append("other bits")
+        except Exception as ex:
+            bad.append(repr(ex))
+
+    ts = [threading.Thread(target=work, args=a) for a in zip(engs, cs, want)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    assert not bad, bad[:3]
+    [e.close() for e in engs]
