@@ -273,7 +273,7 @@ static void plan_step(pi_engine * e, bool tied) {
     StepShape s;
     s.wtype = c.wtype; s.head_type = tied ? PI_TYPE_F16 : c.wtype; s.falcon = c.arch == PI_ARCH_FALCON;
     s.d = c.d; s.F = e->F; s.dkv = e->dkv; s.rank = c.rank; s.n_vocab = c.n_vocab; s.hd = e->hd; s.n_ctx = c.n_ctx;
-    step_plan(s, e->step);
+    step_plan(s, step_device(), e->step);
 }
 
 // arguments of the one-launch step; leaves step.ok false where the model's weights do not allow it

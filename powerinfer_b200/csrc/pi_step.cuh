@@ -1,30 +1,15 @@
 // Interface of the one-launch decode step (pi_step.cu) to the engine.
 #pragma once
 #include "pi_common.cuh"
+#include "pi_step_plan.h"
 
 namespace pi {
 
-static constexpr int ST_QKV = 0, ST_WO = 1, ST_FC1 = 2, ST_FC2 = 3, ST_HEAD = 4, ST_GATHER = 5, ST_N_MAT = 6;   // what goes through the ring: dense matrices, the rows of the gather
 static constexpr int ST_UP = 4, ST_GATE = 5, ST_DOWN = 6;                                           // places in StepLayer::w (those of the dense ones are the numbers above)
 static constexpr int ST_N1W = 0, ST_N1B = 1, ST_N2W = 2, ST_N2B = 3, ST_BQKV = 4, ST_BO = 5, ST_BUP = 6, ST_BDOWN = 7;
-static constexpr int ST_MAX_SLOTS = 48;
 
 // a layer's pointers, as the kernel reads them (n2: the FFN's norm; falcon: attn_norm2)
 struct StepLayer { const uint8_t * w[7]; const float * f[8]; uint64_t pad; };
-
-// a matrix cut for the ring: rows in units of `gran` dealt evenly to the CTAs; a slot holds `rps` rows (1, 2 or 4), or one of `pieces` pieces of
-// a row (`punits` units; a unit is 8 columns of F16, a block of Q4_0) and is the work of a team of `wpr` warps, whose lanes take `upt` units
-// each; `chunk` rows have room for their sums
-struct StepMat { int rows, gran, units, rps, pieces, punits, wpr, upt, chunk, q4; int64_t row_bytes; };
-
-struct StepShape { int wtype, head_type, falcon; int64_t d, F, dkv, rank, n_vocab; int hd, n_ctx; };
-struct StepPlan {
-    bool ok = false;
-    StepMat mat[ST_N_MAT];
-    int slot_bytes = 0, n_slots = 0, window = 0, grid = 0, groups = 0, wpt = 0;
-    int off_a = 0, off_b = 0, off_c = 0, off_h = 0, off_part = 0;
-    size_t smem = 0, words = 0;                                      // shared memory; bytes of the words passed between CTAs
-};
 
 struct StepP {
     const StepLayer * layers; int n_layer;
@@ -44,7 +29,7 @@ struct StepP {
     int slot_bytes, n_slots, window, groups, wpt, off_a, off_b, off_c, off_h, off_part;
 };
 
-bool step_plan(const StepShape & s, StepPlan & pl);                  // false: the shape is not eligible
+StepDevice step_device();                                             // the current device, as the plan sees it (no device: no SMs)
 int launch_step(const StepP & p, const StepPlan & pl, bool gated, cudaStream_t st);
 
 }  // namespace pi

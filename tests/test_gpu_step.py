@@ -10,6 +10,8 @@ import threading
 import numpy as np
 import pytest
 
+from powerinfer_b200 import synth
+
 pytestmark = pytest.mark.gpu
 
 
@@ -96,6 +98,51 @@ def test_step_matches_the_launch_sequence(name):
     assert np.array_equal(eng.device_view("logits", 1)[0].cpu().numpy(), got[-1])
     eng.status()
     eng.close()
+
+
+# rows whose pieces have unequal lengths, and predictors of such ranks
+UNEVEN = {
+    "f16_d_8320": dict(wtype=synth.F16, d=8320, n_ff=1088, n_head=65, n_head_kv=5, rank=72),
+    "f16_d_8512": dict(wtype=synth.F16, d=8512, n_ff=1056, n_head=133, n_head_kv=7, rank=64),
+    "f16_rank_4104": dict(wtype=synth.F16, d=1024, n_ff=2080, n_head=8, n_head_kv=2, rank=4104),
+    "q4_rank_1552": dict(wtype=synth.Q4_0, d=5120, n_ff=1184, n_head=40, n_head_kv=8, rank=1552),
+    "q4_rank_3080": dict(wtype=synth.Q4_0, d=4096, n_ff=1376, n_head=32, n_head_kv=4, rank=3080),
+}
+
+
+def _against_checker(spec, steps=2, launches=None):
+    """Steps of an engine and of the CPU checker under the engine's own active sets: predictor logits and logits."""
+    from oracle import pio
+    from powerinfer_b200 import engine
+    tensors = synth.build_model(spec)
+    eng = engine.DecodeEngine(spec, tensors, max_batch=1)
+    eng.enable_trace()
+    om = pio.OracleModel(spec, tensors)
+    wtype = "q4_0" if spec.wtype == synth.Q4_0 else "f16"
+    active = []
+    for pos in range(steps):
+        tok = (7 + 31 * pos) % spec.n_vocab
+        logits, ids = eng.decode([tok], [pos])
+        got = eng.predictor_trace(1)[:, 0]
+        want, pred = om.decode_imposed(tok, pos, got)
+        _close(got, pred, wtype)
+        _close(logits[0], want, wtype)
+        assert int(ids[0]) == int(np.argmax(logits[0]))
+        active.append(int((got >= spec.threshold).sum()))
+    if launches is not None:
+        assert eng.launches() == launches
+    eng.status()
+    eng.close()
+    om.close()
+    return active
+
+
+@pytest.mark.parametrize("name", list(UNEVEN))
+def test_rows_cut_into_unequal_pieces(name):
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    _against_checker(synth.ModelSpec(arch=synth.ARCH_LLAMA, n_layer=1, n_vocab=320, n_ctx=64, firing=0.2, seed=3, **UNEVEN[name]))
 
 
 def test_steps_of_two_engines_in_two_threads():
