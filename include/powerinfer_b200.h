@@ -302,7 +302,7 @@ int  pi_engine_time_stage(pi_engine * e, int T, int stage, int reps, float * hos
  * delivered, a bulk copy that never landed); the step that hit it still ran to its end.  The word is cleared once it has
  * been reported, and the engine stays usable.  Synchronises `stream`. */
 int  pi_engine_status(pi_engine * e, void * stream);
-/* Bound of the exchange waits in SM clock cycles (0: the default, about a second). */
+/* Bound of the exchange waits, and of the waits inside the step of one sequence, in SM clock cycles (0: the default, about a second). */
 int  pi_engine_set_wait_cycles(pi_engine * e, long long cycles);
 
 /* For tests: device pointers of the predictor logits F32 [T, n_ff/n_ranks] that the LAST layer of the last step left

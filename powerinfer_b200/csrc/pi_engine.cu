@@ -194,7 +194,7 @@ struct pi_engine {
     int qkv_pre;                             // ring stages the QKV mat-vec requests before its dependency wait after a norm that collects vectors (-1: all)
     bool fc2_masks;                          // ... with the activity masks written by the predictor's second mat-vec itself (no mask kernel)
     bool rows1;                              // one token: masks-only compaction + register-streaming sparse kernels (shape eligible)
-    long long wait_cycles;                   // bound of the exchange waits (0: about a second)
+    long long wait_cycles;                   // bound of the exchange waits and of those in the one-launch step (0: about a second)
     unsigned skip_mask;                      // set only inside pi_engine_time_stage: the stages left out of the captured sequence
     StepPlan step;                           // the step of one sequence as one launch (step.ok)
     StepP step_p;                            // ... and its arguments, but for those of a call
@@ -802,6 +802,8 @@ int run_one(pi_engine * e, cudaStream_t st, const Feed * feed = nullptr) {
     p.pred = e->pred_trace ? e->pred_trace : e->pred;
     p.pred_stride = e->pred_trace ? (int64_t)e->c.max_batch * e->F : 0;
     if (feed) { p.fed = 1; p.token = feed->token[0]; p.pos = feed->pos[0]; p.logits_host = feed->logits; p.argmax_host = feed->sink; }
+    p.limit = e->wait_cycles > 0 ? e->wait_cycles : 2000000000LL;
+    p.look = p.limit < 1000000 ? 0 : 63;                              // (64 polls take about 20 us)
     e->launches = 1;
     return launch_step(p, e->step, e->layers[0].gate != nullptr, st);
 }

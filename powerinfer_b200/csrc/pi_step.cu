@@ -19,7 +19,10 @@
 // A word is overwritten two layers later at the earliest (buffers alternate by the parity of the layer).  By then every CTA has
 // read it: each CTA owns at least one row of the out-projection, whose whole output every later layer's words depend on, and it
 // computes that row behind all its reads of the layer before.
-// Every wait is bounded (about a second): on expiry the step finishes with wrong values and bit 3 of the status word.
+// Every wait is bounded (pi_engine_set_wait_cycles; about a second): one that runs out ends the others of the step, which finishes with
+// wrong values and bit 3 of the status word.  From then on nobody waits: the computing warps overwrite lists and scratch whose readers they
+// no longer wait for, and whatever is read there may be anything.  So the copying warps read a count once and derive the rest from it, and
+// bound every row number before it becomes an address; ring slots, the lists' places and all stores depend on no such value.
 #include "pi_rows.cuh"
 #include "pi_step.cuh"
 
@@ -36,8 +39,6 @@ __device__ long long g_stl[160][16][32];
 #else
 #define MARK(i) do { } while (0)
 #endif
-
-static constexpr long long ST_LIMIT = 2000000000LL;                 // cycles of a wait, about a second
 
 // ------------------------------------------------------------------------------------------------ words that carry their own validity
 __device__ __forceinline__ void ld2(const u64 * p, u64 & a, u64 & b) {
@@ -98,20 +99,24 @@ __device__ __forceinline__ float * sh_part() { return reinterpret_cast<float *>(
 // Waits.  The kernel's code is walked through once per layer and has to stay in the instruction cache (at 170 KB a layer, every phase ran at
 // a third of its speed): what is not there at the first look goes to a function.
 __device__ __forceinline__ bool wait_over(int & spins, long long & t0) {
-    if ((++spins & 63) != 0) return false;
     if (s_dead) return true;
+    if ((++spins & s_p.look) != 0) return false;
     const long long now = clock64();
-    if (spins == 64) { t0 = now; return false; }
-    if (now - t0 < ST_LIMIT && ldw(s_p.abort) != s_step + 1u) return false;
-    s_dead = 1;
+    if (t0 == 0) { t0 = now; return false; }
+    if (now - t0 < s_p.limit && ldw(s_p.abort) != s_step + 1u) return false;
     stw(s_p.abort, s_step + 1u);
     atomicOr(s_p.status, 8u);
+    __threadfence();
+    s_dead = 1;
     return true;
 }
 __device__ __noinline__ bool wait_bar_slow(uint64_t * bar, unsigned parity) {
     int spins = 0; long long t0 = 0;
-    while (!mbar_try_wait(bar, parity)) if (wait_over(spins, t0)) return false;
-    return true;
+    while (!s_dead) {                                                 // (a try may put the warp to sleep for a while)
+        if (mbar_try_wait(bar, parity)) return true;
+        if (wait_over(spins, t0)) break;
+    }
+    return false;
 }
 __device__ __forceinline__ bool wait_bar(uint64_t * bar, unsigned parity) { return mbar_test(bar, parity) || wait_bar_slow(bar, parity); }
 // until each of the n words carries the number; returns the last one
@@ -1110,13 +1115,15 @@ __device__ __noinline__ void head_phase(unsigned kbase) {
 
 struct Copier { unsigned k, s, par, bs, bpar; };                     // this copier's next slot, its place, the round's parity; the slot `window` places back
 
-// the slots below kbase + s_slots[mi] that are this copier's (k % ST_COPY == me); false: a wait ran out
+// the slots of `nrow` rows from kbase on that are this copier's (k % ST_COPY == me); false: a wait ran out
 template <bool GATED>
-__device__ __noinline__ bool issue(int mi, const uint8_t * W, const uint8_t * W2, unsigned kbase, Copier & cp) {
-    const int nslots = s_slots[mi], nrow = s_rows[mi], rps = s_p.mat[mi].rps, pieces = s_p.mat[mi].pieces, units = s_p.mat[mi].units, punits = s_p.mat[mi].punits, q4 = s_p.mat[mi].q4;
+__device__ __noinline__ bool issue(int mi, const uint8_t * W, const uint8_t * W2, unsigned kbase, int nrow, int nslots, Copier & cp) {
+    const int rps = s_p.mat[mi].rps, pieces = s_p.mat[mi].pieces, units = s_p.mat[mi].units, punits = s_p.mat[mi].punits, q4 = s_p.mat[mi].q4;
     const unsigned row_bytes = (unsigned)s_p.mat[mi].row_bytes, ring = (unsigned)s_p.n_slots, back = (unsigned)s_p.window * ST_COPY, slot = (unsigned)s_p.slot_bytes;
     const uint8_t * src = W + (size_t)(mi == ST_GATHER ? 0 : s_first[mi]) * row_bytes;
-    const int * rows = sh_list() + 4 * ST_LIST;
+    const volatile int * rows = sh_list() + 4 * ST_LIST;
+    const unsigned top = (unsigned)s_p.F - 1u;
+    auto row_at = [&](int i) { return min((unsigned)rows[i], top); };   // (a list being overwritten after a wait ran out: any number)
     const bool gather = mi == ST_GATHER;
     unsigned k = cp.k, s = cp.s, par = cp.par, bs = cp.bs, bpar = cp.bpar;
     bool ok = true;
@@ -1132,7 +1139,7 @@ __device__ __noinline__ bool issue(int mi, const uint8_t * W, const uint8_t * W2
         uint64_t * bar = s_full + s;
         if (pieces > 1) {                                             // one piece of a row: Q4_0 nibbles, then their scales
             const int row = i / pieces, first = (i - row * pieces) * punits, nu = min(punits, units - first);
-            const uint8_t * from = gather ? (GATED && (row & 1) ? W2 : src) + (size_t)rows[GATED ? row >> 1 : row] * row_bytes : src + (size_t)row * row_bytes;
+            const uint8_t * from = gather ? (GATED && (row & 1) ? W2 : src) + (size_t)row_at(GATED ? row >> 1 : row) * row_bytes : src + (size_t)row * row_bytes;
             const unsigned nb = (unsigned)nu * 16u, ns = q4 ? (unsigned)nu * 2u : 0u;
             mbar_expect_tx(bar, nb + ns);
             bulk_g2s(dst, from + (size_t)first * 16, nb, bar);
@@ -1145,7 +1152,7 @@ __device__ __noinline__ bool issue(int mi, const uint8_t * W, const uint8_t * W2
 #pragma unroll 1
                 for (int r = 0; r < n; r++) {                         // up and gate rows in turn
                     const int v = i * rps + r;
-                    bulk_g2s(dst + (unsigned)r * row_bytes, (GATED && (v & 1) ? W2 : src) + (size_t)rows[GATED ? v >> 1 : v] * row_bytes, row_bytes, bar);
+                    bulk_g2s(dst + (unsigned)r * row_bytes, (GATED && (v & 1) ? W2 : src) + (size_t)row_at(GATED ? v >> 1 : v) * row_bytes, row_bytes, bar);
                 }
             }
         }
@@ -1170,8 +1177,9 @@ __device__ __noinline__ void copy_weights(unsigned me) {
         const int mi = i == n ? ST_HEAD : (m == 0 ? ST_QKV : (m == 1 ? second : (m == 2 ? third : (m == 3 ? fourth : ST_GATHER))));
         const uint8_t * W = i == n ? s_p.head : L.w[m == 4 ? ST_UP : mi], * W2 = L.w[ST_GATE];
         if (m == 4 && !wait_bar(&s_listed, (unsigned)l & 1u)) { ok = false; break; }
-        ok = issue<GATED>(mi, W, W2, kbase, cp);
-        kbase += s_slots[mi];
+        const int nrow = *(volatile int *)&s_rows[mi], nslots = mat_slots(s_p.mat[mi], nrow);   // (read once: see the head of the file)
+        ok = issue<GATED>(mi, W, W2, kbase, nrow, nslots, cp);
+        kbase += (unsigned)nslots;
         if (m == 4 && ok) mbar_arrive(&s_taken);
         if (++m == 5) { m = 0; l++; }
     }

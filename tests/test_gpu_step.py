@@ -145,6 +145,31 @@ def test_rows_cut_into_unequal_pieces(name):
     _against_checker(synth.ModelSpec(arch=synth.ARCH_LLAMA, n_layer=1, n_vocab=320, n_ctx=64, firing=0.2, seed=3, **UNEVEN[name]))
 
 
+@pytest.mark.parametrize("name", ["llama_q4_narrow", "llama_f16_gqa_64", "llama_f16_pieces", "falcon_q4", "opt_f16", "bamboo_q4", "all_active"])
+def test_waits_that_run_out_are_reported_and_the_next_step_is_right(name):
+    """A bound of one cycle: whichever wait finds its value missing twice gives up, at any place of the step, and ends the others.  The step
+    comes to its end, the host reads the status, and the next step with the usual bound gives the bits of a run without any of this."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from powerinfer_b200._lib import lib
+    case = CASES[name]
+    eng = _engine(case, True)
+    want = _steps(eng, case)
+    pos = max(0, min(case["pos"], case["n_ctx"] - 1))
+    for _ in range(4):
+        eng.set_wait_cycles(1)
+        for _ in range(5):
+            eng.set_inputs_device([(7 + 31 * 2) % case["n_vocab"]], [pos])
+            eng.step_device(1)
+            assert lib.pi_engine_status(eng.handle, eng.st) == 5 and b"status 8" in lib.pi_last_error()     # PI_ERR_TIMEOUT
+            assert lib.pi_engine_status(eng.handle, eng.st) == 0                                            # reported once
+        eng.set_wait_cycles(0)
+        assert np.array_equal(_steps(eng, case), want)
+    assert eng.launches() == 1
+    eng.close()
+
+
 def test_steps_of_two_engines_in_two_threads():
     torch = pytest.importorskip("torch")
     if not torch.cuda.is_available():
