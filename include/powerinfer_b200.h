@@ -250,7 +250,7 @@ void pi_engine_destroy(pi_engine * e);
 int  pi_engine_set_exchange(pi_engine * e, const pi_exchange * x);
 
 /* Device-side I/O of a step: tokens int32 [max_batch], pos int32 [max_batch] (position of each sequence's new token),
- * logits F32 [max_batch, n_vocab], argmax int32 [max_batch] (llama_sample_token_greedy, llama.cpp:8617). */
+ * logits F32 [max_batch, n_vocab], argmax int32 [max_batch] (llama_sample_token_greedy, llama.cpp:8617; -1 after a step that gave up). */
 int  pi_engine_io(pi_engine * e, int32_t ** tokens, int32_t ** pos, float ** logits, int32_t ** argmax);
 
 /* Enqueue one step for T sequences on `stream`; inputs are read from / results left in the pi_engine_io buffers. */
@@ -262,7 +262,8 @@ int  pi_engine_advance(pi_engine * e, int T, void * stream);
 
 /* llama_decode + llama_get_logits with HOST buffers (llama.cpp:10672, 6960-6978): copies T token ids and positions to the
  * device, runs the step, copies back T*n_vocab logits (host_logits != NULL) and T greedy ids (host_argmax != NULL), and
- * synchronises `stream`. */
+ * synchronises `stream`.  PI_ERR_TIMEOUT: a wait inside the step of one sequence ran out (see pi_engine_set_wait_cycles); the results
+ * are not valid, the greedy id is -1, and pi_engine_status has nothing more to report. */
 int  pi_engine_decode_host(pi_engine * e, const int32_t * host_tokens, const int32_t * host_pos, int T,
                            float * host_logits, int32_t * host_argmax, void * stream);
 
@@ -302,7 +303,8 @@ int  pi_engine_time_stage(pi_engine * e, int T, int stage, int reps, float * hos
  * delivered, a bulk copy that never landed); the step that hit it still ran to its end.  The word is cleared once it has
  * been reported, and the engine stays usable.  Synchronises `stream`. */
 int  pi_engine_status(pi_engine * e, void * stream);
-/* Bound of the exchange waits, and of the waits inside the step of one sequence, in SM clock cycles (0: the default, about a second). */
+/* Bound of the exchange waits, and of the waits inside the step of one sequence, in SM clock cycles (0: the default, about a second).
+ * The step of one sequence takes all SMs at once; while kernels of other streams hold some of them, its waits last up to 64 times as long. */
 int  pi_engine_set_wait_cycles(pi_engine * e, long long cycles);
 
 /* For tests: device pointers of the predictor logits F32 [T, n_ff/n_ranks] that the LAST layer of the last step left

@@ -249,7 +249,7 @@ static void carve(pi_engine * e, void * ws, size_t ws_bytes, bool dry, size_t * 
     e->act_p = cv.act(PI_TYPE_F16, c.d, T);
     e->act_o = cv.act(c.wtype, e->dq, T);
     if (e->step.ok) {
-        e->step_layers = cv.take<StepLayer>(c.n_layer); e->step_ctl = cv.take<unsigned int>(2); e->step_words = cv.take<char>(e->step.words);
+        e->step_layers = cv.take<StepLayer>(c.n_layer); e->step_ctl = cv.take<unsigned int>(3); e->step_words = cv.take<char>(e->step.words);
     }
     *need = (size_t)(cv.p - (char *)ws);
     if (!cv.ok && !dry) *need = (size_t)-1;
@@ -314,13 +314,13 @@ static int setup_step(pi_engine * e, cudaStream_t st) {
     p.h = (unsigned long long *)take(2 * F * 8); p.part = (unsigned long long *)take(2 * (size_t)pl.groups * d * 8);
     p.acto = (uint32_t *)take(2 * d * 4); p.acts = (uint32_t *)take(2 * (d / 32) * 4); p.hid = (uint32_t *)take(2 * (size_t)c.rank * 4); p.maskw = (uint32_t *)take(2 * (F / 8) * 4);
     p.logits = e->logits; p.tokens = e->tokens; p.positions = e->pos; p.argmax = e->argmax;
-    p.step_no = e->step_ctl; p.abort = e->step_ctl + 1; p.status = e->status; p.ticket = e->amax_ticket; p.best = e->amax_best; p.rows_total = e->active_total;
+    p.step_no = e->step_ctl; p.abort = e->step_ctl + 1; p.arrived = e->step_ctl + 2; p.status = e->status; p.ticket = e->amax_ticket; p.best = e->amax_best; p.rows_total = e->active_total;
     p.row_bytes = (int64_t)pi_row_bytes(c.wtype, c.d);
     for (int i = 0; i < ST_N_MAT; i++) p.mat[i] = pl.mat[i];
     p.slot_bytes = pl.slot_bytes; p.n_slots = pl.n_slots; p.window = pl.window; p.groups = pl.groups; p.wpt = pl.wpt;
-    p.off_a = pl.off_a; p.off_b = pl.off_b; p.off_c = pl.off_c; p.off_h = pl.off_h; p.off_part = pl.off_part;
+    p.off_a = pl.off_a; p.off_b = pl.off_b; p.off_c = pl.off_c; p.off_h = pl.off_h; p.off_part = pl.off_part; p.off_rows = pl.off_rows;
     PI_CUDA(cudaMemcpyAsync(e->step_layers, ly.data(), ly.size() * sizeof(StepLayer), cudaMemcpyHostToDevice, st));
-    PI_CUDA(cudaMemsetAsync(e->step_ctl, 0, 8, st));
+    PI_CUDA(cudaMemsetAsync(e->step_ctl, 0, 12, st));
     PI_CUDA(cudaMemsetAsync(e->step_words, 0, pl.words, st));       // (no layer has the number 0)
     PI_CUDA(cudaStreamSynchronize(st));
     return PI_OK;
@@ -802,8 +802,8 @@ int run_one(pi_engine * e, cudaStream_t st, const Feed * feed = nullptr) {
     p.pred = e->pred_trace ? e->pred_trace : e->pred;
     p.pred_stride = e->pred_trace ? (int64_t)e->c.max_batch * e->F : 0;
     if (feed) { p.fed = 1; p.token = feed->token[0]; p.pos = feed->pos[0]; p.logits_host = feed->logits; p.argmax_host = feed->sink; }
-    p.limit = e->wait_cycles > 0 ? e->wait_cycles : 2000000000LL;
-    p.look = p.limit < 1000000 ? 0 : 63;                              // (64 polls take about 20 us)
+    p.limit = e->wait_cycles > 0 ? std::min(e->wait_cycles, 1LL << 40) : 2000000000LL;
+    p.look = p.limit < 1000000 ? 0 : 63;
     e->launches = 1;
     return launch_step(p, e->step, e->layers[0].gate != nullptr, st);
 }
@@ -880,7 +880,15 @@ int pi_engine_decode_host(pi_engine * e, const int32_t * host_tokens, const int3
     }
     if (host_argmax && !f.sink) PI_CUDA(cudaMemcpyAsync(host_argmax, e->argmax, (size_t)T * 4, cudaMemcpyDeviceToHost, st));
     if (host_logits && !f.logits) PI_CUDA(cudaMemcpyAsync(host_logits, e->logits, (size_t)T * e->c.n_vocab * 4, cudaMemcpyDeviceToHost, st));
+    int32_t id = 0;
+    if (one && !host_argmax) PI_CUDA(cudaMemcpyAsync(&id, e->argmax, 4, cudaMemcpyDeviceToHost, st));
     PI_CUDA(cudaStreamSynchronize(st));
+    if (one && host_argmax) id = host_argmax[0];
+    if (id < 0) {                                                     // the one-launch step gave up (see pi_step.cu)
+        if ((rc = pi_engine_status(e, stream))) return rc;
+        set_error("a wait inside the step ran out");
+        return PI_ERR_TIMEOUT;
+    }
     return PI_OK;
 }
 

@@ -19,10 +19,11 @@
 // A word is overwritten two layers later at the earliest (buffers alternate by the parity of the layer).  By then every CTA has
 // read it: each CTA owns at least one row of the out-projection, whose whole output every later layer's words depend on, and it
 // computes that row behind all its reads of the layer before.
-// Every wait is bounded (pi_engine_set_wait_cycles; about a second): one that runs out ends the others of the step, which finishes with
-// wrong values and bit 3 of the status word.  From then on nobody waits: the computing warps overwrite lists and scratch whose readers they
-// no longer wait for, and whatever is read there may be anything.  So the copying warps read a count once and derive the rest from it, and
-// bound every row number before it becomes an address; ring slots, the lists' places and all stores depend on no such value.
+// Every wait ends (pi_engine_set_wait_cycles): where a copying warp has waited for about a second since the last CTA of the step was seen to
+// run, or 64 times as long before that (a kernel of another stream may hold an SM), it ends the waits of all, and the step finishes with
+// wrong values, the greedy id -1 and bit 3 of the status word (12 ms for 8 layers of the 70B shape).  From then on the computing warps go on
+// without the copying warps' leave.  So what an address is made from holds whoever is late: the gather's rows have a place of their own, in
+// which nothing but row numbers stands, and the copying warps get the number of rows and that of slots in one word.
 #include "pi_rows.cuh"
 #include "pi_step.cuh"
 
@@ -83,56 +84,62 @@ extern __shared__ __align__(128) unsigned char smem[];                // ring | 
 static __shared__ StepP s_p;
 static __shared__ StepLayer s_layer[2];                               // this layer's and the next one's
 static __shared__ int s_first[ST_N_MAT], s_rows[ST_N_MAT], s_slots[ST_N_MAT];   // this CTA's rows of every matrix, and the ring slots they take
-static __shared__ __align__(8) uint64_t s_full[ST_MAX_SLOTS], s_empty[ST_MAX_SLOTS], s_listed, s_taken;   // s_listed: the gather's rows of this layer are listed; s_taken: the copying warps have read them
+static __shared__ __align__(8) uint64_t s_full[ST_MAX_SLOTS], s_empty[ST_MAX_SLOTS], s_listed, s_taken, s_done;   // s_done: the computing warps have waited for the last time; s_listed: the gather's rows of this layer are listed; s_taken: the copying warps have read them
 static __shared__ double s_dred[ST_WARPS];
 static __shared__ int s_warp[ST_WARPS];
 static __shared__ int s_kb, s_ke, s_kz, s_col0, s_ncol;                 // s_col0, s_ncol: the columns of the residual stream that this CTA adds up
-static __shared__ volatile int s_dead;                                // a wait ran out: nobody waits any more
+static __shared__ volatile int s_dead;                                // 1: a wait ran out, nobody waits any more; 2: all waits of this CTA ended well
 static __shared__ unsigned int s_step;
+static __shared__ volatile unsigned int s_gather;                     // rows and slots (in the upper half) of the gather, for the copying warps
 
 __device__ __forceinline__ int mat_slots(const StepMat & m, int nrow) { return m.pieces > 1 ? nrow * m.pieces : (nrow + m.rps - 1) / m.rps; }
 __device__ __forceinline__ uint32_t * sh_mask() { return reinterpret_cast<uint32_t *>(smem + s_p.off_b); }
 __device__ __forceinline__ int * sh_pref() { return reinterpret_cast<int *>(smem + s_p.off_b) + s_p.F / 32; }
-__device__ __forceinline__ int * sh_list() { return sh_pref() + s_p.F / 32 + 1; }                    // [4][ST_LIST], then this CTA's rows of the gather
+__device__ __forceinline__ int * sh_list() { return sh_pref() + s_p.F / 32 + 1; }                    // [4][ST_LIST]
+__device__ __forceinline__ int * sh_rows() { return reinterpret_cast<int *>(smem + s_p.off_rows); }      // this CTA's rows of the gather
 __device__ __forceinline__ float * sh_part() { return reinterpret_cast<float *>(smem + s_p.off_part); }
 
 // Waits.  The kernel's code is walked through once per layer and has to stay in the instruction cache (at 170 KB a layer, every phase ran at
 // a third of its speed): what is not there at the first look goes to a function.
-__device__ __forceinline__ bool wait_over(int & spins, long long & t0) {
-    if (s_dead) return true;
-    if ((++spins & s_p.look) != 0) return false;
-    const long long now = clock64();
-    if (t0 == 0) { t0 = now; return false; }
-    if (now - t0 < s_p.limit && ldw(s_p.abort) != s_step + 1u) return false;
-    stw(s_p.abort, s_step + 1u);
-    atomicOr(s_p.status, 8u);
-    __threadfence();
-    s_dead = 1;
+// Only the copying warps' waits have a clock: where the step does not go on, the ring stays full and they wait.  The computing warps look
+// whether the step has been ended: a clock in the dozen places where they wait cost up to 4 % of a step (registers spill, polls get longer).
+__device__ __forceinline__ bool wait_over(int & polls) { return (++polls & 63) == 0 && s_dead; }
+__device__ __noinline__ bool wait_bar_slow(uint64_t * bar, unsigned parity) {
+    int tries = 0;
+    while (!mbar_try_wait(bar, parity)) if ((++tries & 7) == 0 && s_dead) return false;
     return true;
 }
-__device__ __noinline__ bool wait_bar_slow(uint64_t * bar, unsigned parity) {
-    int spins = 0; long long t0 = 0;
-    while (!s_dead) {                                                 // (a try may put the warp to sleep for a while)
-        if (mbar_try_wait(bar, parity)) return true;
-        if (wait_over(spins, t0)) break;
-    }
-    return false;
-}
 __device__ __forceinline__ bool wait_bar(uint64_t * bar, unsigned parity) { return mbar_test(bar, parity) || wait_bar_slow(bar, parity); }
+__device__ __forceinline__ void end_step() { stw(s_p.abort, s_step + 1u); atomicOr(s_p.status, 8u); }
+__device__ __noinline__ bool timed_bar_slow(uint64_t * bar, unsigned parity) {
+    long long from = clock64();
+    bool placed = false;                                              // all CTAs of the step run
+    for (int i = 1; !mbar_try_wait(bar, parity); i++) {
+        if (s_dead) return false;
+        if ((i & s_p.look) != 0) continue;
+        const long long now = clock64();
+        if (!placed && ldw(s_p.arrived) == (s_step + 1u) * gridDim.x) { placed = true; from = now; }
+        if (now - from <= (placed ? s_p.limit : 64 * s_p.limit) && ldw(s_p.abort) != s_step + 1u) continue;
+        if (atomicCAS(const_cast<int *>(&s_dead), 0, 1) == 0) end_step();
+        return false;
+    }
+    return true;
+}
+__device__ __forceinline__ bool timed_bar(uint64_t * bar, unsigned parity) { return mbar_test(bar, parity) || timed_bar_slow(bar, parity); }
 // until each of the n words carries the number; returns the last one
 __device__ __noinline__ u64 wait_words(const u64 * p, int n, unsigned tag) {
     u64 x = 0ull;
     for (int i = 0; i < n; i++) {
-        int spins = 0; long long t0 = 0;
-        for (x = ld1(p + i); !fresh(x, tag); x = ld1(p + i)) if (wait_over(spins, t0)) break;
+        int polls = 0;
+        for (x = ld1(p + i); !fresh(x, tag); x = ld1(p + i)) if (wait_over(polls)) break;
     }
     return x;
 }
 // the same for four 4-byte words whose number stands above the lowest `bits` bits
 __device__ __noinline__ uint4 wait_words4(const uint32_t * p, int bits, unsigned tag) {
-    int spins = 0; long long t0 = 0;
+    int polls = 0;
     uint4 v = ld4(p);
-    while (((v.x ^ tag) | (v.y ^ tag) | (v.z ^ tag) | (v.w ^ tag)) >> bits) { if (wait_over(spins, t0)) break; v = ld4(p); }
+    while (((v.x ^ tag) | (v.y ^ tag) | (v.z ^ tag) | (v.w ^ tag)) >> bits) { if (wait_over(polls)) break; v = ld4(p); }
     return v;
 }
 __device__ __forceinline__ float wait_val(const u64 * s, unsigned tag) {
@@ -256,7 +263,7 @@ __device__ __noinline__ void consume_t(int mi, unsigned k0, int nrow, const unsi
     x.load(xs, units, first + u0, step, last_ok);
     const int pshift = __popc(P - 1);
     float * s_part = sh_part() + pc * wpr + part;
-    const int nslots = P > 1 ? nrow * P : (nrow + R - 1) / R;
+    const int nslots = P > 1 ? nrow * P : (nrow + R - 1) / R;   // (a wait ran out: nothing comes any more)
     const unsigned k = k0 + team, round = k / ring;
     unsigned s = k - round * ring, par = round & 1u;
     if (team < nslots) wait_bar(s_full + s, par);
@@ -362,7 +369,7 @@ __device__ __noinline__ void norm_phase(const u64 * src, unsigned tag, const Nor
     for (int k0 = 0; k0 < NC; k0 += 2) {
         u64 r[2][8];
         const int c = (k0 * ST_CT + tid) * 8;
-        int spins = 0; long long t0 = 0;
+        int polls = 0;
         while (true) {
             unsigned off = 0u;
 #pragma unroll
@@ -375,7 +382,7 @@ __device__ __noinline__ void norm_phase(const u64 * src, unsigned tag, const Nor
                         off |= ((unsigned)(r[k][j] >> 32) ^ tag) | ((unsigned)(r[k][j + 1] >> 32) ^ tag);
                     }
                 }
-            if (!off || wait_over(spins, t0)) break;
+            if (!off || wait_over(polls)) break;
             // every CTA polls this vector: where it is more than a word pair a thread, one word until it is there (8 layers of d 8192: 603
             // us, 617 without; 12 layers of d 4096: 743 us with it, 726 without)
             if (n > ST_CT * 8) wait_words(src + c, 1, tag);
@@ -744,10 +751,11 @@ template <bool GATED>
 __device__ __forceinline__ void gather_list(int layer, int n) {
     if (layer) wait_bar(&s_taken, (unsigned)(layer - 1) & 1u);
     const int first = (int)(blockIdx.x * (unsigned)n / gridDim.x), mj = (int)((blockIdx.x + 1) * (unsigned)n / gridDim.x) - first;
-    list_rows(first, first + mj, sh_list() + 4 * ST_LIST);
+    list_rows(first, first + mj, sh_rows());
     if (threadIdx.x == 0) {
         s_rows[ST_GATHER] = GATED ? 2 * mj : mj;
         s_slots[ST_GATHER] = mat_slots(s_p.mat[ST_GATHER], GATED ? 2 * mj : mj);
+        s_gather = (unsigned)s_rows[ST_GATHER] | (unsigned)s_slots[ST_GATHER] << 16;
         s_kb = s_p.F / 32; s_ke = s_p.F / 32;                         // (axpy_phase looks for its range)
     }
     bar_ct();
@@ -759,7 +767,7 @@ template <int WT, bool GATED>
 __device__ __noinline__ void gather_phase(int layer, unsigned kbase, unsigned tag) {
     constexpr int NM = GATED ? 2 : 1;
     const int n = s_rows[ST_GATHER], chunk = s_p.mat[ST_GATHER].chunk;   // (an even number of rows)
-    const int * rows = sh_list() + 4 * ST_LIST;
+    const int * rows = sh_rows();
     const float * bias = s_layer[layer & 1].f[ST_BUP];
     u64 * out = s_p.h + (size_t)(layer & 1) * s_p.F;
 #pragma unroll 1
@@ -1095,18 +1103,20 @@ __device__ __noinline__ void head_phase(unsigned kbase) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) { const u64 k = __shfl_xor_sync(0xffffffffu, key, o); key = k > key ? k : key; }
     u64 * s_key = reinterpret_cast<u64 *>(s_dred);
-    if ((tid & 31) == 0) s_key[tid >> 5] = key;
+    if ((tid & 31) == 0) { s_key[tid >> 5] = key; mbar_arrive(&s_done); }
     bar_ct();
     if (tid != 0) return;
+    if (atomicCAS(const_cast<int *>(&s_dead), 0, 2) == 1) end_step();  // (a copying warp has said so or is about to: the last CTA shall see it)
     for (int w = 1; w < ST_WARPS; w++) key = s_key[w] > key ? s_key[w] : key;
     if (key) atomicMax(s_p.best, key);
     __threadfence();
     if (atomicAdd(s_p.ticket, 1u) != gridDim.x - 1u) return;
     __threadfence();
     const u64 k = atomicExch(s_p.best, 0ull);
+    const bool ended = ldw(s_p.abort) == s_step + 1u;
     *s_p.ticket = 0u;
     *s_p.step_no = s_step + 1u;                                       // every CTA has read it: all have taken a ticket
-    const int32_t i = k ? (int32_t)~(unsigned)k : 0;
+    const int32_t i = ended ? -1 : (k ? (int32_t)~(unsigned)k : 0);
     *s_p.argmax = i;
     if (s_p.argmax_host) *s_p.argmax_host = i;
 }
@@ -1121,25 +1131,23 @@ __device__ __noinline__ bool issue(int mi, const uint8_t * W, const uint8_t * W2
     const int rps = s_p.mat[mi].rps, pieces = s_p.mat[mi].pieces, units = s_p.mat[mi].units, punits = s_p.mat[mi].punits, q4 = s_p.mat[mi].q4;
     const unsigned row_bytes = (unsigned)s_p.mat[mi].row_bytes, ring = (unsigned)s_p.n_slots, back = (unsigned)s_p.window * ST_COPY, slot = (unsigned)s_p.slot_bytes;
     const uint8_t * src = W + (size_t)(mi == ST_GATHER ? 0 : s_first[mi]) * row_bytes;
-    const volatile int * rows = sh_list() + 4 * ST_LIST;
-    const unsigned top = (unsigned)s_p.F - 1u;
-    auto row_at = [&](int i) { return min((unsigned)rows[i], top); };   // (a list being overwritten after a wait ran out: any number)
+    const int * rows = sh_rows();
     const bool gather = mi == ST_GATHER;
     unsigned k = cp.k, s = cp.s, par = cp.par, bs = cp.bs, bpar = cp.bpar;
     bool ok = true;
 #pragma unroll 1
     for (int i = (int)(k - kbase); i < nslots; i += ST_COPY) {
         if (k >= back) {
-            if (!wait_bar(s_full + bs, bpar)) { ok = false; break; }
+            if (!timed_bar(s_full + bs, bpar)) { ok = false; break; }
             bs += ST_COPY;
             if (bs >= ring) { bs -= ring; bpar ^= 1u; }
         }
-        if (k >= ring && !wait_bar(s_empty + s, par ^ 1u)) { ok = false; break; }
+        if (k >= ring && !timed_bar(s_empty + s, par ^ 1u)) { ok = false; break; }
         unsigned char * dst = smem + s * slot;
         uint64_t * bar = s_full + s;
         if (pieces > 1) {                                             // one piece of a row: Q4_0 nibbles, then their scales
             const int row = i / pieces, first = (i - row * pieces) * punits, nu = min(punits, units - first);
-            const uint8_t * from = gather ? (GATED && (row & 1) ? W2 : src) + (size_t)row_at(GATED ? row >> 1 : row) * row_bytes : src + (size_t)row * row_bytes;
+            const uint8_t * from = gather ? (GATED && (row & 1) ? W2 : src) + (size_t)rows[GATED ? row >> 1 : row] * row_bytes : src + (size_t)row * row_bytes;
             const unsigned nb = (unsigned)nu * 16u, ns = q4 ? (unsigned)nu * 2u : 0u;
             mbar_expect_tx(bar, nb + ns);
             bulk_g2s(dst, from + (size_t)first * 16, nb, bar);
@@ -1152,7 +1160,7 @@ __device__ __noinline__ bool issue(int mi, const uint8_t * W, const uint8_t * W2
 #pragma unroll 1
                 for (int r = 0; r < n; r++) {                         // up and gate rows in turn
                     const int v = i * rps + r;
-                    bulk_g2s(dst + (unsigned)r * row_bytes, (GATED && (v & 1) ? W2 : src) + (size_t)row_at(GATED ? v >> 1 : v) * row_bytes, row_bytes, bar);
+                    bulk_g2s(dst + (unsigned)r * row_bytes, (GATED && (v & 1) ? W2 : src) + (size_t)rows[GATED ? v >> 1 : v] * row_bytes, row_bytes, bar);
                 }
             }
         }
@@ -1176,8 +1184,9 @@ __device__ __noinline__ void copy_weights(unsigned me) {
         const StepLayer & L = s_p.layers[min(l, s_p.n_layer - 1)];
         const int mi = i == n ? ST_HEAD : (m == 0 ? ST_QKV : (m == 1 ? second : (m == 2 ? third : (m == 3 ? fourth : ST_GATHER))));
         const uint8_t * W = i == n ? s_p.head : L.w[m == 4 ? ST_UP : mi], * W2 = L.w[ST_GATE];
-        if (m == 4 && !wait_bar(&s_listed, (unsigned)l & 1u)) { ok = false; break; }
-        const int nrow = *(volatile int *)&s_rows[mi], nslots = mat_slots(s_p.mat[mi], nrow);   // (read once: see the head of the file)
+        if (m == 4 && !timed_bar(&s_listed, (unsigned)l & 1u)) { ok = false; break; }
+        int nrow = s_rows[mi], nslots = s_slots[mi];
+        if (m == 4) { const unsigned g = s_gather; nrow = (int)(g & 0xffffu); nslots = (int)(g >> 16); }   // (one word: see the head of the file)
         ok = issue<GATED>(mi, W, W2, kbase, nrow, nslots, cp);
         kbase += (unsigned)nslots;
         if (m == 4 && ok) mbar_arrive(&s_taken);
@@ -1190,6 +1199,7 @@ __device__ __noinline__ void copy_weights(unsigned me) {
         int spins = 0;
         while (!mbar_try_wait(s_full + (j - ST_COPY) % ring, ((j - ST_COPY) / ring) & 1u) && ++spins < (1 << 16)) {}
     }
+    if (ok && me == 0) timed_bar(&s_done, 0u);                        // the clock runs to the end
 }
 
 // ------------------------------------------------------------------------------------------------ the kernel
@@ -1208,13 +1218,14 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_step(const __grid_constant__ 
         s_slots[tid] = mat_slots(m, r1 - r0);
     }
     if (tid == 0) {
-        s_dead = 0;
+        s_dead = 0; s_gather = 0u;
         const unsigned c8n = (unsigned)args.d / 8u;
         s_col0 = (int)(blockIdx.x * c8n / gridDim.x) * 8;
         s_ncol = (int)((blockIdx.x + 1) * c8n / gridDim.x) * 8 - s_col0;
         s_step = *args.step_no;                                       // raised by the CTA that finishes the step last
+        atomicAdd(args.arrived, 1u);
         for (int s = 0; s < args.n_slots; s++) { mbar_init(s_full + s, 1); mbar_init(s_empty + s, ST_WARPS); }
-        mbar_init(&s_listed, 1); mbar_init(&s_taken, ST_COPY);
+        mbar_init(&s_listed, 1); mbar_init(&s_taken, ST_COPY); mbar_init(&s_done, ST_WARPS);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }

@@ -23,11 +23,11 @@ struct StepP {
     float * pred; int64_t pred_stride; float * logits;
     int32_t * tokens, * positions, * argmax; int fed, token, pos;    // fed: this step's token comes with the launch
     float * logits_host; int32_t * argmax_host;
-    long long limit; int look, pad;                                  // cycles of a wait; it looks at the clock where its polls & look == 0
-    unsigned int * step_no, * abort, * status, * ticket; unsigned long long * best, * rows_total;
+    long long limit; int look, pad;                                  // cycles of a wait; it looks at the clock where its tries & look == 0
+    unsigned int * step_no, * abort, * arrived, * status, * ticket; unsigned long long * best, * rows_total;
     int64_t row_bytes;                                               // of up / gate / down_t
     StepMat mat[ST_N_MAT];
-    int slot_bytes, n_slots, window, groups, wpt, off_a, off_b, off_c, off_h, off_part;
+    int slot_bytes, n_slots, window, groups, wpt, off_a, off_b, off_c, off_h, off_part, off_rows;
 };
 
 StepDevice step_device();                                             // the current device, as the plan sees it (no device: no SMs)

@@ -34,7 +34,7 @@ struct StepPlan {
     bool ok = false;
     StepMat mat[ST_N_MAT];
     int slot_bytes = 0, n_slots = 0, window = 0, grid = 0, groups = 0, wpt = 0;
-    int off_a = 0, off_b = 0, off_c = 0, off_h = 0, off_part = 0;
+    int off_a = 0, off_b = 0, off_c = 0, off_h = 0, off_part = 0, off_rows = 0;
     size_t smem = 0, words = 0;                                      // shared memory; bytes of the words passed between CTAs
 };
 
@@ -87,11 +87,11 @@ inline bool step_plan(const StepShape & s, const StepDevice & dev, StepPlan & pl
     const size_t a = step_up128(std::max(std::max(act, act_head), (size_t)ST_RED));
     const size_t att = (size_t)s.n_ctx * 6 + (size_t)ST_WARPS * s.hd * 4 + (size_t)3 * s.hd * 2 + ST_WARPS * 8 + 64;
     const int64_t myrow = (s.F + grid - 1) / grid + 1;
-    const size_t lists = (size_t)(2 * (s.F / 32) + 1) * 4 + (size_t)4 * ST_LIST * 4 + (size_t)myrow * 4 + 64;
+    const size_t lists = (size_t)(2 * (s.F / 32) + 1) * 4 + (size_t)4 * ST_LIST * 4 + 64, rows = step_up128((size_t)myrow * 4);
     const size_t b = step_up128(std::max(std::max((size_t)s.d * 2, att), lists));
     const size_t c = s.falcon ? step_up128(act) : 0;                  // else the first region serves: it is free until the FFN's norm
     const size_t h = step_up128((size_t)s.rank * 2), part = step_up128((size_t)ST_PART * 4);
-    const size_t fixed = a + b + c + h + part, room = dev.smem > ST_STATIC ? dev.smem - ST_STATIC : 0;
+    const size_t fixed = a + b + c + h + part + rows, room = dev.smem > ST_STATIC ? dev.smem - ST_STATIC : 0;
     if (fixed >= room) return false;
     // Slots of about 8 KB (F16) or 4.6 KB (Q4_0: whole rows where they fit): smaller ones cost the copying warps more than they save, larger
     // ones leave teams without work at the end of a matrix (steps of the 7B, 40B and 70B shapes in 4, 8, 16 and 36 KB slots: 1030, 729, 785,
@@ -121,7 +121,7 @@ inline bool step_plan(const StepShape & s, const StepDevice & dev, StepPlan & pl
     if (cols > ST_CT || pl.groups * cols > ST_PART) return false;
     const size_t ring = step_up128((size_t)pl.n_slots * pl.slot_bytes);
     pl.off_a = (int)ring; pl.off_b = (int)(ring + a); pl.off_c = s.falcon ? (int)(ring + a + b) : pl.off_a;
-    pl.off_h = (int)(ring + a + b + c); pl.off_part = (int)(ring + a + b + c + h);
+    pl.off_h = (int)(ring + a + b + c); pl.off_part = (int)(ring + a + b + c + h); pl.off_rows = (int)(ring + a + b + c + h + part);
     pl.smem = ring + fixed;
     pl.wpt = s.F / 32 > 2 * ST_CT ? 4 : (s.F / 32 > ST_CT ? 2 : 1);
     // words: x, x2 [2][d] u64; qkv [2][d + 2 dkv] u64; h [2][F] u64; part [2][groups][d] u64; acto [2][d], acts [2][d / 32], hid [2][rank],

@@ -4,7 +4,9 @@ sizes, ragged sizes, the edges of its ring plan, contexts beyond one pass of the
 Two correct implementations differ in the order of their sums, which flips roundings of activations between the nodes (FP16, or the int8 of
 Q8_0): the bounds are those of perf/cases.py for whole steps, relative in the 2-norm: 3e-3 (FP16 weights), 3e-2 (Q4_0).  The predictors lie
 far from the threshold there, so both choose the same neurons."""
+import ctypes
 import os
+import subprocess
 import threading
 
 import numpy as np
@@ -147,8 +149,9 @@ def test_rows_cut_into_unequal_pieces(name):
 
 @pytest.mark.parametrize("name", ["llama_q4_narrow", "llama_f16_gqa_64", "llama_f16_pieces", "falcon_q4", "opt_f16", "bamboo_q4", "all_active"])
 def test_waits_that_run_out_are_reported_and_the_next_step_is_right(name):
-    """A bound of one cycle: whichever wait finds its value missing twice gives up, at any place of the step, and ends the others.  The step
-    comes to its end, the host reads the status, and the next step with the usual bound gives the bits of a run without any of this."""
+    """A bound of one cycle: the first copying warp that has to wait gives up and ends the others' waits.  With larger bounds it is one that
+    waits longer, in the middle of the step (for a slot, for the rows of the gather), or none.  The step comes to its end, the host reads the
+    status, and the next step with the usual bound gives the bits of a run without any of this."""
     torch = pytest.importorskip("torch")
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
@@ -157,16 +160,82 @@ def test_waits_that_run_out_are_reported_and_the_next_step_is_right(name):
     eng = _engine(case, True)
     want = _steps(eng, case)
     pos = max(0, min(case["pos"], case["n_ctx"] - 1))
-    for _ in range(4):
-        eng.set_wait_cycles(1)
+    for cycles in (1, 2000, 4000, 7000, 10000, 15000, 20000, 30000, 45000, 70000, 100000):
         for _ in range(5):
+            eng.set_wait_cycles(cycles)
             eng.set_inputs_device([(7 + 31 * 2) % case["n_vocab"]], [pos])
             eng.step_device(1)
-            assert lib.pi_engine_status(eng.handle, eng.st) == 5 and b"status 8" in lib.pi_last_error()     # PI_ERR_TIMEOUT
+            rc = lib.pi_engine_status(eng.handle, eng.st)
+            assert rc == 5 or (rc == 0 and cycles > 1), cycles                                              # PI_ERR_TIMEOUT
+            assert (int(eng.device_view("argmax", 1)[0]) == -1) == (rc == 5)
+            assert rc == 0 or b"status 8" in lib.pi_last_error()
             assert lib.pi_engine_status(eng.handle, eng.st) == 0                                            # reported once
         eng.set_wait_cycles(0)
         assert np.array_equal(_steps(eng, case), want)
     assert eng.launches() == 1
+    eng.close()
+
+
+def test_a_step_that_gives_up_is_an_error_of_the_call():
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from powerinfer_b200._lib import lib
+    case = CASES["llama_f16_gqa_64"]
+    eng = _engine(case, True)
+    want = _steps(eng, case)
+    for want_logits in (True, False):
+        eng.set_wait_cycles(1)
+        with pytest.raises(RuntimeError, match="ran out"):
+            eng.decode([3], [case["pos"]], want_logits=want_logits)      # (what it leaves in the cache is overwritten below)
+        assert int(eng.h_argmax[0]) == -1
+        assert lib.pi_engine_decode_host(eng.handle, eng.h_tokens.data_ptr(), eng.h_pos.data_ptr(), 1, None, None, eng.st) == 5
+        eng.set_wait_cycles(0)
+        eng.status()                                              # the call has reported it
+        assert np.array_equal(_steps(eng, case), want)
+    eng.close()
+
+
+HOLD = r"""
+#include <cuda_runtime.h>
+__global__ void hold(unsigned long long ns) {
+    unsigned long long t0, t1;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    for (int i = 0; i < 10000000; i++) {
+        __nanosleep(1000);
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
+        if (t1 - t0 >= ns) break;
+    }
+}
+extern "C" int hold_sm(unsigned long long ns, void * stream) {
+    if (cudaFuncSetAttribute(hold, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess) return 1;
+    hold<<<1, 32, 200 * 1024, (cudaStream_t)stream>>>(ns);
+    return (int)cudaGetLastError();
+}
+"""
+
+
+def test_a_kernel_of_another_stream_may_hold_an_sm(tmp_path):
+    """An SM is taken for 0.4 s, far longer than a wait's bound of about 20 ms: the step waits for it and is right."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from powerinfer_b200 import build
+    src, so = tmp_path / "hold.cu", tmp_path / "libhold.so"
+    src.write_text(HOLD)
+    subprocess.run([build.NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xcompiler", "-fPIC", "-o", str(so), str(src)], check=True)
+    hold = ctypes.CDLL(str(so)).hold_sm
+    hold.argtypes = [ctypes.c_ulonglong, ctypes.c_void_p]
+    case = CASES["llama_f16_gqa_64"]
+    eng = _engine(case, True)
+    want = _steps(eng, case)
+    eng.set_wait_cycles(40_000_000)
+    other = torch.cuda.Stream()
+    for _ in range(2):
+        assert hold(400_000_000, other.cuda_stream) == 0
+        got = _steps(eng, case)                                   # (asserts a clean status)
+        other.synchronize()
+        assert np.array_equal(got, want)
     eng.close()
 
 
