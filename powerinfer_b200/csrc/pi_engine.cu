@@ -276,10 +276,10 @@ static void plan_step(pi_engine * e, bool tied) {
     step_plan(s, step_device(), e->step);
 }
 
-// arguments of the one-launch step; leaves step.ok false where the model's weights do not allow it
+// arguments of the one-launch step; leaves step.ok false where the model's weights or the context do not allow it
 static int setup_step(pi_engine * e, cudaStream_t st) {
     const pi_engine_config & c = e->c;
-    bool ok = rows_eligible(c.wtype, e->F, c.d);
+    bool ok = rows_eligible(c.wtype, e->F, c.d) && step_fits(e->step, c.wtype == PI_TYPE_Q4_0, e->layers[0].gate != nullptr);
     std::vector<StepLayer> ly(c.n_layer);
     const bool gated = e->layers[0].gate != nullptr;
     auto al = [&](const void * p) { if (((uintptr_t)p & 15) != 0) ok = false; return p; };
@@ -796,7 +796,7 @@ void * mapped(void * host) {
 }
 
 // one sequence's step as one launch; `feed`: its token, and where the results go besides the engine's own buffers (null: the token is
-// in the engine's buffers)
+// in the engine's buffers).  STEP_REFUSED: the launch sequence has to run it
 int run_one(pi_engine * e, cudaStream_t st, const Feed * feed = nullptr) {
     StepP p = e->step_p;
     p.pred = e->pred_trace ? e->pred_trace : e->pred;
@@ -804,13 +804,13 @@ int run_one(pi_engine * e, cudaStream_t st, const Feed * feed = nullptr) {
     if (feed) { p.fed = 1; p.token = feed->token[0]; p.pos = feed->pos[0]; p.logits_host = feed->logits; p.argmax_host = feed->sink; }
     p.limit = e->wait_cycles > 0 ? std::min(e->wait_cycles, 1LL << 40) : 2000000000LL;
     p.look = p.limit < 1000000 ? 0 : 63;
-    e->launches = 1;
-    return launch_step(p, e->step, e->layers[0].gate != nullptr, st);
+    const int rc = launch_step(p, e->step, e->layers[0].gate != nullptr, st);
+    if (rc == PI_OK) e->launches = 1;
+    return rc;
 }
 
 // first call for a batch size: one plain run (fills every per-kernel attribute cache), then capture
-int run_step(pi_engine * e, int T, cudaStream_t st, int mode = 0) {
-    if (T == 1 && mode == 0 && e->step.ok) return run_one(e, st);
+int run_sequence(pi_engine * e, int T, cudaStream_t st, int mode = 0) {
     StageTimer tm;
     // A chunk beyond the batch: its length seldom comes again, and its kernels are longer than their launches
     if (T > e->T_max) return enqueue_step(e, T, st, tm, mode);
@@ -833,6 +833,11 @@ int run_step(pi_engine * e, int T, cudaStream_t st, int mode = 0) {
     e->graphs[mode][T] = exec; e->graph_nodes[mode][T] = e->launches;
     PI_CUDA(cudaGraphLaunch(exec, st));
     return PI_OK;
+}
+
+int run_step(pi_engine * e, int T, cudaStream_t st, int mode = 0) {
+    const int rc = T == 1 && mode == 0 && e->step.ok ? run_one(e, st) : STEP_REFUSED;
+    return rc == STEP_REFUSED ? run_sequence(e, T, st, mode) : rc;
 }
 
 }  // namespace
@@ -867,16 +872,17 @@ int pi_engine_decode_host(pi_engine * e, const int32_t * host_tokens, const int3
     f.sink = host_argmax ? (int32_t *)mapped(host_argmax) : nullptr;
     f.logits = host_logits ? (float *)mapped(host_logits) : nullptr;
     f.n_vocab = e->c.n_vocab;
-    const bool one = T == 1 && e->step.ok;
-    if (one) { if ((rc = run_one(e, st, &f))) return rc; }
-    else {
-    k_feed<<<1, PI_MAX_BATCH, 0, st>>>(f, T, e->tokens, e->pos, e->sink, e->logits_sink);
-    PI_LAUNCH_CHECK("k_feed");
-    if ((rc = run_step(e, T, st))) {
-        cudaMemsetAsync(e->sink, 0, (size_t)T * sizeof *e->sink, st);
-        cudaMemsetAsync(e->logits_sink, 0, (size_t)T * sizeof *e->logits_sink, st);
-        return rc;
-    }
+    rc = T == 1 && e->step.ok ? run_one(e, st, &f) : STEP_REFUSED;
+    const bool one = rc != STEP_REFUSED;
+    if (one && rc) return rc;
+    if (!one) {
+        k_feed<<<1, PI_MAX_BATCH, 0, st>>>(f, T, e->tokens, e->pos, e->sink, e->logits_sink);
+        PI_LAUNCH_CHECK("k_feed");
+        if ((rc = run_sequence(e, T, st))) {
+            cudaMemsetAsync(e->sink, 0, (size_t)T * sizeof *e->sink, st);
+            cudaMemsetAsync(e->logits_sink, 0, (size_t)T * sizeof *e->logits_sink, st);
+            return rc;
+        }
     }
     if (host_argmax && !f.sink) PI_CUDA(cudaMemcpyAsync(host_argmax, e->argmax, (size_t)T * 4, cudaMemcpyDeviceToHost, st));
     if (host_logits && !f.logits) PI_CUDA(cudaMemcpyAsync(host_logits, e->logits, (size_t)T * e->c.n_vocab * 4, cudaMemcpyDeviceToHost, st));

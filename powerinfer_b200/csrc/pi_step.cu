@@ -27,6 +27,8 @@
 #include "pi_rows.cuh"
 #include "pi_step.cuh"
 
+#include <cuda.h>
+
 #include <algorithm>
 #include <cstdlib>
 
@@ -1333,31 +1335,60 @@ StepDevice step_device() {
     return r;
 }
 
-template <int WT, bool GATED>
-static int step_go(const StepP & p, const StepPlan & pl, cudaStream_t st) {
-    auto kern = k_step<WT, GATED>;
-    static bool attr_done[16] = {false};
-    int dev = 0;
-    PI_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 16 || !attr_done[dev]) {
-        int most = 0;
-        PI_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        PI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most - ST_STATIC));
-        if (dev >= 0 && dev < 16) attr_done[dev] = true;
-    }
+typedef void (*StepKernel)(const StepP);
+static StepKernel step_kernel(bool q4, bool gated) {
+    if (q4) return gated ? k_step<PI_TYPE_Q4_0, true> : k_step<PI_TYPE_Q4_0, false>;
+    return gated ? k_step<PI_TYPE_F16, true> : k_step<PI_TYPE_F16, false>;
+}
+
+// A context or a stream can have a part of the device only (a green context).  No answer counts as the whole.
+template <typename F> static F driver_call(const char * name) {
+    void * f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion(name, &f, 12040, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) { cudaGetLastError(); return nullptr; }
+    return (F)f;
+}
+static int context_sms() {
+    static const auto current = driver_call<CUresult (*)(CUcontext *)>("cuCtxGetCurrent");
+    static const auto resource = driver_call<CUresult (*)(CUcontext, CUdevResource *, CUdevResourceType)>("cuCtxGetDevResource");
+    CUcontext ctx = nullptr;
+    CUdevResource r;
+    if (!current || !resource || current(&ctx) != CUDA_SUCCESS || !ctx || resource(ctx, &r, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS) return sm_count();
+    return (int)r.sm.smCount;
+}
+static bool stream_has_sms(cudaStream_t st, int need) {
+    static const auto green = driver_call<CUresult (*)(CUstream, CUgreenCtx *)>("cuStreamGetGreenCtx");
+    static const auto resource = driver_call<CUresult (*)(CUgreenCtx, CUdevResource *, CUdevResourceType)>("cuGreenCtxGetDevResource");
+    CUgreenCtx g = nullptr;
+    CUdevResource r;
+    if (!st || !green || !resource || green(st, &g) != CUDA_SUCCESS || !g || resource(g, &r, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS) return true;
+    return (int)r.sm.smCount >= need;
+}
+
+bool step_fits(const StepPlan & pl, bool q4, bool gated) {
+    const StepKernel kern = step_kernel(q4, gated);
+    int dev = 0, cooperative = 0, per_sm = 0;
+    cudaFuncAttributes at;
+    const bool ok = cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && cooperative &&
+                    cudaFuncGetAttributes(&at, kern) == cudaSuccess && at.sharedSizeBytes <= (size_t)ST_STATIC &&
+                    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(step_device().smem - ST_STATIC)) == cudaSuccess &&
+                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, ST_THREADS, pl.smem) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    return ok && per_sm * context_sms() >= pl.grid;
+}
+
+int launch_step(const StepP & p, const StepPlan & pl, bool gated, cudaStream_t st) {
+    if (!stream_has_sms(st, pl.grid)) return STEP_REFUSED;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(pl.grid); cfg.blockDim = dim3(ST_THREADS); cfg.dynamicSmemBytes = pl.smem; cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;                      // the CTAs wait for one another: all are resident, or the launch fails
     attr[0].val.cooperative = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    PI_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, step_kernel(p.q4, gated), p);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported) { cudaGetLastError(); return STEP_REFUSED; }
+    PI_CUDA(e);
     return PI_OK;
-}
-
-int launch_step(const StepP & p, const StepPlan & pl, bool gated, cudaStream_t st) {
-    if (p.q4) return gated ? step_go<PI_TYPE_Q4_0, true>(p, pl, st) : step_go<PI_TYPE_Q4_0, false>(p, pl, st);
-    return gated ? step_go<PI_TYPE_F16, true>(p, pl, st) : step_go<PI_TYPE_F16, false>(p, pl, st);
 }
 
 }  // namespace pi

@@ -31,6 +31,8 @@ struct StepP {
 };
 
 StepDevice step_device();                                             // the current device, as the plan sees it (no device: no SMs)
+bool step_fits(const StepPlan & pl, bool q4, bool gated);             // the current context runs all CTAs of the plan at once; readies the kernel for launches
+static constexpr int STEP_REFUSED = -1;                               // launch_step: these CTAs cannot run at once on this stream, nothing was launched
 int launch_step(const StepP & p, const StepPlan & pl, bool gated, cudaStream_t st);
 
 }  // namespace pi

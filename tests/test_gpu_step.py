@@ -239,6 +239,64 @@ def test_a_kernel_of_another_stream_may_hold_an_sm(tmp_path):
     eng.close()
 
 
+def test_a_stream_with_a_part_of_the_device_runs_the_launch_sequence():
+    """All CTAs of the step run at once; where a stream has too few SMs for them (a green context), the launch sequence takes the step."""
+    torch = pytest.importorskip("torch")
+    driver = pytest.importorskip("cuda.bindings.driver")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from powerinfer_b200._lib import check, lib
+    case = CASES["llama_f16_gqa_64"]
+    eng = _engine(case, False)
+    want = _steps(eng, case)
+    eng.close()
+    eng = _engine(case, True)
+    one = _steps(eng, case)
+    assert eng.launches() == 1
+
+    def ok(r):
+        if r[0] != driver.CUresult.CUDA_SUCCESS:
+            pytest.skip(f"no green context here: {r[0]}")
+        return r[1:] if len(r) > 2 else (r[1] if len(r) == 2 else None)
+
+    dev = ok(driver.cuDeviceGet(0))
+    sms = ok(driver.cuDeviceGetDevResource(dev, driver.CUdevResourceType.CU_DEV_RESOURCE_TYPE_SM))
+    groups, _, _ = ok(driver.cuDevSmResourceSplitByCount(1, sms, 0, 32))
+    green = ok(driver.cuGreenCtxCreate(ok(driver.cuDevResourceGenerateDesc([groups[0]], 1)), dev, driver.CUgreenCtxCreate_flags.CU_GREEN_CTX_DEFAULT_STREAM))
+    stream = ok(driver.cuGreenCtxStreamCreate(green, driver.CUstream_flags.CU_STREAM_NON_BLOCKING, 0))
+    for i in range(3):                                            # plain launch, graph capture, graph replay
+        eng.h_tokens[0], eng.h_pos[0] = (7 + 31 * 2) % case["n_vocab"], case["pos"]
+        check(lib.pi_engine_decode_host(eng.handle, eng.h_tokens.data_ptr(), eng.h_pos.data_ptr(), 1, eng.h_logits.data_ptr(), eng.h_argmax.data_ptr(), int(stream)))
+        assert eng.launches() > 1
+        _close(eng.h_logits[0].numpy(), want[-1], case["wtype"])
+    assert np.array_equal(_steps(eng, case)[-1], one[-1]) and eng.launches() == 1
+    eng.close()
+    ok(driver.cuStreamDestroy(stream))
+    ok(driver.cuGreenCtxDestroy(green))
+
+
+def test_a_step_inside_a_captured_graph():
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    case = CASES["llama_f16_gqa_64"]
+    eng = _engine(case, True)
+    want = _steps(eng, case)
+    graph = torch.cuda.CUDAGraph()
+    pos = max(0, min(case["pos"], case["n_ctx"] - 1))
+    eng.set_inputs_device([(7 + 31 * 2) % case["n_vocab"]], [pos])
+    with torch.cuda.graph(graph, stream=eng.stream, capture_error_mode="thread_local"):
+        eng.step_device(1)
+    for _ in range(3):
+        eng.device_view("logits", 1).zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(eng.device_view("logits", 1)[0].cpu().numpy(), want[-1])
+    eng.status()
+    del graph
+    eng.close()
+
+
 def test_steps_of_two_engines_in_two_threads():
     torch = pytest.importorskip("torch")
     if not torch.cuda.is_available():
