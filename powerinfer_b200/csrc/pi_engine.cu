@@ -187,7 +187,8 @@ struct pi_engine {
     cudaGraphExec_t graphs[3][PI_MAX_BATCH + 1];   // [0] decode, [1] prompt chunk, [2] prompt chunk without the lm head
     bool warmed[3][PI_MAX_BATCH + 1];
     int graph_nodes[3][PI_MAX_BATCH + 1];          // kernel nodes of each captured graph
-    int launches;                            // kernels enqueued by the last enqueue_step
+    int launches;                            // kernels enqueued by the last step
+    int seq_launches;                        // ... by the last complete enqueue_step (0: none yet)
     float * pred_trace;                      // optional [n_layer, max_batch, F]: keeps every layer's predictor logits
     bool pdl;                                // programmatic dependent launch between the kernels of a step
     bool gate_sym;                           // bamboo: relu on the gated product as well
@@ -402,7 +403,7 @@ int pi_engine_create(const pi_engine_config * cfg, const pi_model_weights * gw, 
     memset(e->warmed, 0, sizeof e->warmed);
     memset(e->graph_nodes, 0, sizeof e->graph_nodes);
     memset(&e->xch, 0, sizeof e->xch);
-    e->pred_trace = nullptr; e->launches = 0;
+    e->pred_trace = nullptr; e->launches = e->seq_launches = 0;
     { const char * v = getenv("PI_PDL"); e->pdl = !(v && v[0] == '0'); }
     e->skip_mask = 0u; e->wait_cycles = 0;
     e->rows1 = rows_eligible(cfg->wtype, e->F, cfg->d) && axpy_rows_groups(e->F, cfg->d) <= e->G;
@@ -762,6 +763,7 @@ int enqueue_step(pi_engine * e, int T, cudaStream_t st, StageTimer & tm, int mod
             pend.vec = e->ffn_vec;
         }
     }
+    if (!e->skip_mask) e->seq_launches = e->launches;
     return PI_OK;
 }
 
@@ -939,14 +941,16 @@ int pi_engine_profile_step(pi_engine * e, int T, float * host_ms, int * host_lau
     StageTimer tm;
     tm.on = true; tm.st = st;
     tm.pool.reserve(4096);
-    for (int i = 0; i < 2 * (e->launches > 0 ? e->launches + 8 : 2048); i++) tm.next();   // create the events before the clock starts
+    const int n = e->seq_launches, saved_launches = e->launches;     // of the sequence that runs here, whatever a step is
+    for (int i = 0; i < 2 * (n > 0 ? n + 8 : 2048); i++) tm.next();   // create the events before the clock starts
     tm.used = 0;
-    const unsigned long long hold_ns = (unsigned long long)(e->launches > 0 ? e->launches : 1000) * 12000ull;
+    const unsigned long long hold_ns = (unsigned long long)(n > 0 ? n : 1000) * 12000ull;
     k_hold<<<1, 1, 0, st>>>(hold_ns < 30000000ull ? hold_ns : 30000000ull);
     PI_LAUNCH_CHECK("k_hold");
     rc = enqueue_step(e, T, st, tm);
     if (rc) { cudaStreamSynchronize(st); return rc; }
     if (host_launches) *host_launches = e->launches;
+    if (T == 1 && e->step.ok) e->launches = saved_launches;
     return tm.collect(host_ms);
 }
 

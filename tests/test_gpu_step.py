@@ -275,6 +275,26 @@ def test_a_stream_with_a_part_of_the_device_runs_the_launch_sequence():
     ok(driver.cuGreenCtxDestroy(green))
 
 
+def test_a_profiled_step_is_held_until_its_launches_are_queued():
+    """The stream is held while the host queues the launch sequence: 12 us a launch, 12 ms where none was counted yet, whatever a step
+    launches by itself."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import time
+    eng = _engine(_case("llama", "f16", 24, 768, 2048, 6, 6, 64, 512, 64, 0.2, 3), True)
+    eng.decode([5], [3])
+    assert eng.launches() == 1
+    for least in (lambda n: 1000, lambda n: n):
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        ms, n = eng.profile_step(1)
+        assert time.perf_counter() - t0 >= least(n) * 12e-6
+        assert n > 8 * 24 and ms["qkv"] > 0 and eng.launches() == 1
+    eng.status()
+    eng.close()
+
+
 def test_a_step_inside_a_captured_graph():
     torch = pytest.importorskip("torch")
     if not torch.cuda.is_available():
