@@ -181,7 +181,7 @@ struct pi_engine {
     __half * k_cache, * v_cache;             // [n_layer, max_batch, n_ctx, dkv]
     unsigned long long * amax_best; unsigned int * amax_ticket;   // k_argmax: a word per row, 0 between steps
     int32_t ** sink; float ** logits_sink;   // per row: where the step's greedy id and logits go as well (null for steps fed on the device)
-    unsigned int * status;                   // device word: bit 0 = an exchange wait ran out, any other = a wait for a kernel's own copies
+    unsigned int * status;                   // device word: bit 0 = an exchange wait ran out, bit 3 = one inside the one-launch step, any other = a wait for a kernel's own copies
     unsigned long long * active_total;       // device counter: sum of active-list lengths over layers and steps
     pi_exchange xch;
     cudaGraphExec_t graphs[3][PI_MAX_BATCH + 1];   // [0] decode, [1] prompt chunk, [2] prompt chunk without the lm head
@@ -1000,6 +1000,7 @@ int pi_engine_status(pi_engine * e, void * stream) {
     if (s) PI_CUDA(cudaMemsetAsync(e->status, 0, 4, (cudaStream_t)stream));      // reported once
     PI_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
     if (s & 1u) { set_error("an exchange wait ran out: a peer rank did not deliver its partial vector"); return PI_ERR_TIMEOUT; }
+    if (s & 8u) { set_error("a wait inside the one-launch step ran out: for a copy, for another CTA's values, or for an SM that other work held (status %u)", s); return PI_ERR_TIMEOUT; }
     if (s) { set_error("a copy's wait ran out in a weight-streaming kernel (status %u)", s); return PI_ERR_TIMEOUT; }
     return PI_OK;
 }

@@ -624,7 +624,7 @@ __device__ __noinline__ void attention_head(int h, int layer, int pos, int seq, 
     for (int j = tid; j <= pos; j += ST_CT) {
         const float e = round_f16(expf(round_f16(sc[j] - mx)));
         sc[j] = e;
-        part += (unsigned)(e * 16777216.0f);                          // exact; 2^24 at most, for up to 7 positions of a thread (step_eligible)
+        part += (unsigned)(e * 16777216.0f);                          // exact; 2^24 at most, for up to 7 positions of a thread (step_plan)
     }
     const unsigned ws = __reduce_add_sync(0xffffffffu, part);
     if (lane == 0) s_sum[wid] = ws;

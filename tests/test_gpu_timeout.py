@@ -84,5 +84,6 @@ def test_every_status_bit_is_reported(bit):
     word.fill_(bit)
     torch.cuda.synchronize()
     assert lib.pi_engine_status(eng.handle, eng.st) == 5 and b"status %d" % bit in lib.pi_last_error()
+    assert (b"one-launch step" in lib.pi_last_error()) == (bit == 8) and (b"weight-streaming" in lib.pi_last_error()) == (bit != 8)
     assert word.item() == 0 and lib.pi_engine_status(eng.handle, eng.st) == 0
     eng.close()
