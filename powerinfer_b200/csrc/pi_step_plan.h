@@ -93,11 +93,21 @@ inline bool step_plan(const StepShape & s, const StepDevice & dev, StepPlan & pl
     const size_t h = step_up128((size_t)s.rank * 2), part = step_up128((size_t)ST_PART * 4);
     const size_t fixed = a + b + c + h + part + rows, room = dev.smem > ST_STATIC ? dev.smem - ST_STATIC : 0;
     if (fixed >= room) return false;
-    // Slots of about 8 KB (F16) or 4.6 KB (Q4_0: whole rows where they fit): smaller ones cost the copying warps more than they save, larger
-    // ones leave teams without work at the end of a matrix (steps of the 7B, 40B and 70B shapes in 4, 8, 16 and 36 KB slots: 1030, 729, 785,
-    // 856; 724, 574, 807, 591; 622, 639, 690, 736 us).
-    const int64_t row = step_row_bytes(s.wtype, s.d);
-    const int64_t slot64 = q4 ? (row <= 4608 ? row * std::max<int64_t>(1, 4608 / row) : std::min<int64_t>(row, 6912)) : 8192;
+    // Slots of about 8 KB (F16) or 4.6 KB (Q4_0): smaller ones cost the copying warps more than they save, larger ones leave teams without
+    // work at the end of a matrix (steps of the 7B, 40B and 70B shapes in 4, 8, 16 and 36 KB slots: 1030, 729, 785, 856; 724, 574, 807, 591;
+    // 622, 639, 690, 736 us).  A row that is larger goes whole or in even pieces that fill the slot: what a slot does not hold is missing in
+    // the ring, and a piece of half a slot costs the copying warps as much as a whole one.  Layers in 8 KB slots, in slots that the pieces fill,
+    // by the launch sequence: F16, 3 of d 4352 265, 235, 261 us; 3 of d 5120 295, 265, 330; 3 of d 6656 357, 336, 417; 1 of d 9216 305, 242, 265;
+    // 1 of d 10240 327, 272, 376 (12 KB slots: 3 of d 5632 311, in pieces of 5.5 KB 291).  Q4_0, in 6.9 KB slots, whole rows, by the
+    // sequence: d 12544 341, 181, 198; d 13312 361, 186, 209.
+    const int64_t row = step_row_bytes(s.wtype, s.d), units = s.d / (q4 ? 32 : 8), unit_bytes = q4 ? 18 : 16;
+    if (q4 && row > 7680) return false;                               // (1 layer of d 14336, F 39936: 244 us in two pieces, 199 by the sequence)
+    int64_t slot64 = q4 ? (row <= 4608 ? row * std::max<int64_t>(1, 4608 / row) : row) : 8192;
+    if (!q4 && row > slot64) {
+        int64_t pieces = 1;
+        while (row > pieces * 10240) pieces *= 2;
+        slot64 = ((units + pieces - 1) / pieces + 7) / 8 * 8 * unit_bytes;
+    }
     const int slot = (int)((slot64 + 127) / 128 * 128);
     bool found = false;
     const int most_slots = (int)std::min<size_t>(ST_MAX_SLOTS, (room - fixed) / slot);

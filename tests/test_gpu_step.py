@@ -29,6 +29,10 @@ CASES = {
     "llama_f16_pieces": _case("llama", "f16", 2, 5120, 3456, 40, 8, 488, 777, 128, 0.1, 77),
     "llama_q4_pieces": _case("llama", "q4_0", 1, 12544, 1600, 98, 7, 256, 515, 64, 0.2, 63),
     "llama_f16_wide": _case("llama", "f16", 1, 9216, 1376, 72, 8, 520, 300, 64, 0.2, 20),
+    # rows just above a ring slot's usual size: whole, and in two pieces that fill the slot
+    "llama_f16_whole_rows": _case("llama", "f16", 1, 4352, 1376, 34, 2, 96, 300, 64, 0.2, 20),
+    "falcon_f16_two_pieces": _case("falcon", "f16", 1, 8448, 1376, 66, 22, 96, 300, 64, 0.2, 20),
+    "llama_q4_whole_rows": _case("llama", "q4_0", 1, 13312, 1376, 104, 8, 96, 300, 64, 0.2, 20),
     "falcon_q4": _case("falcon", "q4_0", 2, 1280, 3904, 20, 5, 552, 600, 200, 0.15, 130),
     "falcon_f16": _case("falcon", "f16", 3, 2048, 4096, 32, 2, 144, 901, 96, 0.1, 50),
     "opt_f16": _case("opt", "f16", 2, 1536, 4032, 12, 12, 200, 1003, 128, 0.1, 90),

@@ -65,6 +65,8 @@ static bool check(const StepShape & s, const StepDevice & dev) {
                          : m.rps * m.row_bytes > p.slot_bytes) return fail("slot", s, i, m);
         if (m.row_bytes % 16 || m.chunk < 1 || m.chunk % m.gran || m.chunk % m.rps || m.chunk * m.wpr * m.pieces > ST_PART) return fail("sums", s, i, m);
     }
+    const StepMat & qkv = p.mat[ST_QKV];                              // rows in pieces fill the slot but for a share of the last one
+    if (qkv.pieces > 1 && (qkv.q4 || qkv.punits * 16 + 127 < p.slot_bytes)) return fail("pieces smaller than a slot", s, ST_QKV, qkv);
     if (p.n_slots > ST_MAX_SLOTS || p.n_slots % ST_COPY || p.window < 1 || p.window * ST_COPY > p.n_slots || p.slot_bytes % 128) return fail("ring", s, 0, p.mat[0]);
     if (p.smem + ST_STATIC > dev.smem || p.off_part + ST_PART * 4 > p.off_rows || p.off_rows + (int)((s.F + p.grid - 1) / p.grid) * 4 > (int)p.smem || p.off_a < p.n_slots * p.slot_bytes) return fail("shared memory", s, 0, p.mat[0]);
     if (p.grid > dev.sms || p.grid * 8 > s.d || p.grid * 8 > s.F || p.groups < 1 || p.wpt * ST_CT * 32 < s.F) return fail("grid", s, 0, p.mat[0]);
