@@ -36,13 +36,6 @@ namespace pi {
 
 typedef unsigned long long u64;
 
-#ifdef PI_STEP_TL                                                     // timeline builds, never the shipped library: when thread 0 of a CTA passes a mark
-__device__ long long g_stl[160][16][32];
-#define MARK(i) do { if (threadIdx.x == 0 && layer < 16) g_stl[blockIdx.x][layer][i] = clock64(); } while (0)
-#else
-#define MARK(i) do { } while (0)
-#endif
-
 // ------------------------------------------------------------------------------------------------ words that carry their own validity
 __device__ __forceinline__ void ld2(const u64 * p, u64 & a, u64 & b) {
     asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
@@ -995,7 +988,6 @@ __device__ __noinline__ void wo_phase(int layer, unsigned kbase, unsigned tag) {
     if (tid < n) { if (bias) b = bias[tid]; if (x) res = val(ld1(x + tid)); }
     if (WT == PI_TYPE_F16) stage_f16(s_p.acto + (size_t)par * s_p.dq, s_p.dq, tag, smem + s_p.off_c);
     else                   stage_q8(s_p.acto + (size_t)par * s_p.dq, s_p.acts + (size_t)par * (s_p.dq / QK), s_p.dq, tag, smem + s_p.off_c);
-    MARK(5);
     u64 * out = s_p.x2 + (size_t)par * s_p.d + first;
     rows_of<WT>(ST_WO, kbase, smem + s_p.off_c, [&](int t, float o) {
         if (bias) o += t == tid ? b : bias[t];
@@ -1013,7 +1005,6 @@ __device__ __noinline__ void fc1_phase(int layer, unsigned kbase, unsigned tag) 
 // the predictor's logits and masks (llama.cpp:4692-4695)
 __device__ __noinline__ void fc2_phase(int layer, unsigned kbase, unsigned tag) {
     stage_f16(s_p.hid + (size_t)(layer & 1) * s_p.rank, s_p.rank, tag, smem + s_p.off_h);
-    MARK(10);
     const int n = s_rows[ST_FC2], first = s_first[ST_FC2], chunk = s_p.mat[ST_FC2].chunk;    // (chunks of whole groups of 8 rows)
     float * pred = s_p.pred + (size_t)layer * s_p.pred_stride + first;
     uint32_t * out = s_p.maskw + (size_t)(layer & 1) * (s_p.F / 8) + first / 8;
@@ -1247,7 +1238,6 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_step(const __grid_constant__ 
     unsigned kbase = 0;
 #pragma unroll 1
     for (int l = 0; l < s_p.n_layer; l++) {
-        const int layer = l;
         const StepLayer & L = s_layer[l & 1];
         const unsigned tag = ep0 + (unsigned)l;
         const u64 * x_in = s_p.x + (size_t)(l & 1) * s_p.d;
@@ -1256,7 +1246,6 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_step(const __grid_constant__ 
             const float * f = i < lines * 4 ? L.f[i / lines] : nullptr;
             if (f) asm volatile("prefetch.global.L2 [%0];" :: "l"(f + (size_t)(i % lines) * 32));
         }
-        MARK(0);
         auto attention = [&]() {
 #pragma unroll 1
             for (int h = blockIdx.x; h < s_p.n_head; h += gridDim.x) {
@@ -1270,52 +1259,38 @@ __global__ void __launch_bounds__(ST_THREADS, 1) k_step(const __grid_constant__ 
         } else {
             norm_any(x_in, tag, {L.f[ST_N1W], L.f[ST_N1B], smem + s_p.off_c, nullptr, nullptr, nullptr, nullptr, WT});
         }
-        MARK(1);
         qkv_phase<WT>(l, kbase, tag);
         kbase += s_slots[ST_QKV];
-        MARK(2);
         if (l + 1 < s_p.n_layer && wid == ST_WARPS - 1 && lane < (int)(sizeof(StepLayer) / 8))
             reinterpret_cast<u64 *>(&s_layer[(l + 1) & 1])[lane] = reinterpret_cast<const u64 *>(s_p.layers + l + 1)[lane];
         if (s_p.falcon) {
             // the two branches do not depend on each other: the predictor's first product before the attention, which hides its hand-over
             fc1_phase(l, kbase, tag);
             kbase += s_slots[ST_FC1];
-            MARK(4);
             attention();
-            MARK(5);
             fc2_phase(l, kbase, tag);
             kbase += s_slots[ST_FC2];
-            MARK(6);
             wo_phase<WT>(l, kbase, tag);
             kbase += s_slots[ST_WO];
         } else {
             attention();
-            MARK(4);
             wo_phase<WT>(l, kbase, tag);
             kbase += s_slots[ST_WO];
-            MARK(6);
             // ---- ffn_inp = attention + x: its norm, and ffn_inp itself for the predictor
             norm_any(s_p.x2 + (size_t)(l & 1) * s_p.d, tag, {L.f[ST_N2W], L.f[ST_N2B], smem + s_p.off_a, nullptr, nullptr, nullptr, smem + s_p.off_b, WT});
-            MARK(8);
             fc1_phase(l, kbase, tag);
             kbase += s_slots[ST_FC1];
-            MARK(9);
             fc2_phase(l, kbase, tag);
             kbase += s_slots[ST_FC2];
         }
-        MARK(11);
         // ---- the sparse FFN
         const int n = scan_words(s_p.maskw + (size_t)(l & 1) * (s_p.F / 8), tag);
         if (s_p.rows_total && blockIdx.x == 0 && tid == 0 && n) atomicAdd(s_p.rows_total, (u64)n);
         gather_list<GATED>(l, n);
-        MARK(13);
         gather_phase<WT, GATED>(l, kbase, tag);
         kbase += s_slots[ST_GATHER];
-        MARK(15);
         axpy_phase<WT>(l, n, tag);
-        MARK(16);
         reduce_phase(l, tag);
-        MARK(18);
     }
     // ---- output norm, lm head, greedy choice
     norm_any(s_p.x + (size_t)(s_p.n_layer & 1) * s_p.d, ep0 + (unsigned)s_p.n_layer, {s_p.out_w, s_p.out_b, smem + s_p.off_a, nullptr, nullptr, nullptr, nullptr, s_p.head_type});
@@ -1392,6 +1367,3 @@ int launch_step(const StepP & p, const StepPlan & pl, bool gated, cudaStream_t s
 }
 
 }  // namespace pi
-#ifdef PI_STEP_TL
-extern "C" __attribute__((visibility("default"))) int pi_stl_read(long long * host) { cudaDeviceSynchronize(); return (int)cudaMemcpyFromSymbol(host, pi::g_stl, sizeof(pi::g_stl)); }
-#endif
