@@ -1,9 +1,11 @@
-"""The one-launch decode step (csrc/pi_step.cu) against the launch sequence it replaces, over the forms it takes: graphs, weight types, head
-sizes, ragged sizes, the edges of its ring plan, contexts beyond one pass of the attention, every / no neuron active.
+"""The one-launch decode step (csrc/pi_step.cu) over the forms it takes.  Against the launch sequence it replaces: graphs, weight types, head
+sizes, ragged sizes, rows in pieces, contexts beyond one pass of the attention, nearly all and few neurons active.  Against the CPU checker:
+pieces of unequal length, exactly no and exactly every neuron active, more rows than one pass of the axpy, of the mask scan or of a phase's
+sums takes.  (What its ring plan does at all other sizes is walked on the CPU: test_step_plan_cpu.py.)
 
 Two correct implementations differ in the order of their sums, which flips roundings of activations between the nodes (FP16, or the int8 of
 Q8_0): the bounds are those of perf/cases.py for whole steps, relative in the 2-norm: 3e-3 (FP16 weights), 3e-2 (Q4_0).  The predictors lie
-far from the threshold there, so both choose the same neurons."""
+far from the threshold against the launch sequence, so both choose the same neurons; the CPU checker is given the engine's choice."""
 import ctypes
 import os
 import subprocess
@@ -117,7 +119,7 @@ UNEVEN = {
 
 
 def _against_checker(spec, steps=2, launches=None):
-    """Steps of an engine and of the CPU checker under the engine's own active sets: predictor logits and logits."""
+    """Steps of an engine and of the CPU checker under the engine's own active sets: predictor logits and logits.  Active neurons of each step."""
     from oracle import pio
     from powerinfer_b200 import engine
     tensors = synth.build_model(spec)
@@ -149,6 +151,29 @@ def test_rows_cut_into_unequal_pieces(name):
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     _against_checker(synth.ModelSpec(arch=synth.ARCH_LLAMA, n_layer=1, n_vocab=320, n_ctx=64, firing=0.2, seed=3, **UNEVEN[name]))
+
+
+# the threshold below or above every logit.  every_*: more than 512 rows in a group of the axpy, 2 and 4 mask words a thread (more than 16384,
+# 32768 neurons), more rows of the gather, of fc2 and of the lm head in a CTA than have room for their sums at once
+EXTREMES = {
+    "none_llama_q4": (0, dict(arch=synth.ARCH_LLAMA, wtype=synth.Q4_0, d=1024, n_ff=2048, n_head=8, n_head_kv=2, rank=64, n_vocab=320)),
+    "none_llama_f16": (0, dict(arch=synth.ARCH_LLAMA, wtype=synth.F16, d=1024, n_ff=2048, n_head=8, n_head_kv=2, rank=64, n_vocab=320)),
+    "none_falcon_q4": (0, dict(arch=synth.ARCH_FALCON, wtype=synth.Q4_0, d=1024, n_ff=2048, n_head=16, n_head_kv=2, rank=64, n_vocab=320)),
+    "none_opt_f16": (0, dict(arch=synth.ARCH_OPT, wtype=synth.F16, d=1024, n_ff=2048, n_head=8, n_head_kv=8, rank=64, n_vocab=320)),
+    "every_q4_20480": (20480, dict(arch=synth.ARCH_LLAMA, wtype=synth.Q4_0, d=1024, n_ff=20480, n_head=8, n_head_kv=2, rank=64, n_vocab=320)),
+    "every_q4_40960": (40960, dict(arch=synth.ARCH_FALCON, wtype=synth.Q4_0, d=1024, n_ff=40960, n_head=8, n_head_kv=2, rank=64, n_vocab=320)),
+    "every_q4_wide": (4096, dict(arch=synth.ARCH_LLAMA, wtype=synth.Q4_0, d=8192, n_ff=4096, n_head=64, n_head_kv=8, rank=64, n_vocab=320)),
+    "every_f16_65536": (65536, dict(arch=synth.ARCH_LLAMA, wtype=synth.F16, d=768, n_ff=65536, n_head=6, n_head_kv=2, rank=4096, n_vocab=100000)),
+}
+
+
+@pytest.mark.parametrize("name", list(EXTREMES))
+def test_no_neuron_and_every_neuron_active(name):
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    active, spec = EXTREMES[name]
+    assert _against_checker(synth.ModelSpec(n_layer=1, n_ctx=64, seed=9, threshold=-1e30 if active else 1e30, **spec), launches=1) == [active, active]
 
 
 @pytest.mark.parametrize("name", ["llama_q4_narrow", "llama_f16_gqa_64", "llama_f16_pieces", "falcon_q4", "opt_f16", "bamboo_q4", "all_active"])
