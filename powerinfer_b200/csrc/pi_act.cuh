@@ -6,6 +6,7 @@ namespace pi {
 
 static constexpr int QK = 32;
 
+// (put_act of the one-launch step does the same into shared memory.)
 // Emit 8 consecutive values (chunk index c8 = first column / 8) of token t as activation planes.
 // Must be called by every lane of a warp (it shuffles); `valid` gates the stores.  With n % 32 == 0 the 4 lanes that
 // share a Q8 block are valid or invalid together.

@@ -705,6 +705,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) k_attention(const AttnP p) {
 //   values   the first 12 rows of a thread are requested before the softmax and travel while it runs.
 //   sums     the numerators are FP16 numbers, i.e. multiples of 2^-24: their sum is exact in integers (redux.sync), as it is in double.
 //   planes   a warp owns one block of 32 columns and quantises it itself.
+// (attention_head of the one-launch step repeats it, with 6 value rows on their way and keys of 256 positions before the query.)
 template <int HC>                                                     // head_dim / 32
 __global__ void __launch_bounds__(ATTN_THREADS) k_attention_row(const AttnP p) {
     constexpr int HD = HC * 32, HALF = HD / 2, CH = HD / 8, SL = ATTN_THREADS / CH, NW = ATTN_THREADS / 32;

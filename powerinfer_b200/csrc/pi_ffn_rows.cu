@@ -234,6 +234,7 @@ __global__ void __launch_bounds__(ROWS_THREADS, 1) k_ffn_rows(const FfnRowsP p) 
     // Coefficient = what the CPU path multiplies the row by: FP16(h) for FP16 rows; for Q4_0 the int8 quant of h within its
     // block of 32 neurons times that block's FP16 scale (ggml.c:14575-14581, quantize_row_q8_0).  Inactive neurons of the
     // block count as 0, so the largest |h| is taken over the block's active rows, which are neighbours in rank order.
+    // (axpy_phase of the one-launch step makes the same coefficients and sums.)
     if (tid == 0) s_cnt = 0;
     __syncthreads();
     for (int t0 = 0; t0 < m; t0 += ROWS_THREADS) {

@@ -24,6 +24,10 @@
 // wrong values, the greedy id -1 and bit 3 of the status word (12 ms for 8 layers of the 70B shape).  From then on the computing warps go on
 // without the copying warps' leave.  So what an address is made from holds whoever is late: the gather's rows have a place of their own, in
 // which nothing but row numbers stands, and the copying warps get the number of rows and that of slots in one word.
+//
+// The arithmetic of four nodes stands here a second time, with other inputs and outputs: attention_head (k_attention_row), norm_phase
+// (k_norm), put_act (emit_act8), axpy_phase (k_ffn_rows, k_axpy_rows).  A change of one is a change of both; steps by this kernel and by
+// the launch sequence are compared in the tests.
 #include "pi_rows.cuh"
 #include "pi_step.cuh"
 
