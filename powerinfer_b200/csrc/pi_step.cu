@@ -101,8 +101,16 @@ __device__ __forceinline__ float * sh_part() { return reinterpret_cast<float *>(
 // Waits.  The kernel's code is walked through once per layer and has to stay in the instruction cache (at 170 KB a layer, every phase ran at
 // a third of its speed): what is not there at the first look goes to a function.
 // Only the copying warps' waits have a clock: where the step does not go on, the ring stays full and they wait.  The computing warps look
-// whether the step has been ended: a clock in the dozen places where they wait cost up to 4 % of a step (registers spill, polls get longer).
-__device__ __forceinline__ bool wait_over(int & polls) { return (++polls & 63) == 0 && s_dead; }
+// whether the step has been ended, by their CTA or another: a clock and a count of the running CTAs in the dozen places where they wait cost
+// up to 4 % of a step (registers spill, polls get longer).
+// (The look at the word in L2 costs nothing: 80 layers of the 70B shape 180.8 tok/s with it, 178.8 where only s_dead is read.)
+__device__ __forceinline__ bool wait_over(int & polls) {
+    if ((++polls & 63) != 0) return false;
+    if (s_dead) return true;
+    if (ldw(s_p.abort) != s_step + 1u) return false;
+    s_dead = 1;
+    return true;
+}
 __device__ __noinline__ bool wait_bar_slow(uint64_t * bar, unsigned parity) {
     int tries = 0;
     while (!mbar_try_wait(bar, parity)) if ((++tries & 7) == 0 && s_dead) return false;
