@@ -133,7 +133,8 @@ int launch_gemv(const GemvArgs & a, cudaStream_t st);
 // PI_ERR_UNSUPPORTED: not eligible; *wrote_masks: the kernel that ran honoured masks_out itself
 int launch_gemv_ring(const GemvArgs & a, unsigned int * status, bool pdl, cudaStream_t st, bool * wrote_masks = nullptr);
 int launch_mm(const GemvArgs & a, cudaStream_t st);                                           // 2+ tokens; PI_ERR_UNSUPPORTED: not eligible
-int launch_mm_wide(const GemvArgs & a, cudaStream_t st);                                      // 33+ tokens (called by launch_mm)
+int launch_mm_wide(const GemvArgs & a, cudaStream_t st);                                      // 33+ tokens, Q4_0 rows (called by launch_mm)
+int launch_mm_tc(const GemvArgs & a, cudaStream_t st);                                        // the same for FP16 rows
 static constexpr int64_t MM_MAX_ROWS = 262144;                                                // rows a gather of launch_mm can choose from
 
 // predictor logits -> compacted list of LOCAL rows active for >= 1 token; also writes zeros (or relu(bias)) into

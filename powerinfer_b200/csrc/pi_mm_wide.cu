@@ -1,25 +1,23 @@
-// Mat-mat over FP16 and planar Q4_0 rows for MORE than 32 tokens (prompt chunks of up to 256): the same operators, row selection and
-// epilogue as pi_mm.cu, another split of the work.
+// Mat-mat over planar Q4_0 rows for MORE than 32 tokens (prompt chunks of up to 256): the same operators, row selection and epilogue as
+// pi_mm.cu, another split of the work.  (FP16 rows: pi_mm_tc.cu.)
 //
-// Bound: with 77 FP16 tokens the tensor pipe and HBM are about even (12288 x 4096: 17 us of mma.sync at 955 multiply-adds per clock
-// and SM, 15 us of weights); above that the products.  Q4_0 is bound by the scaling of its blocks: an mma of 16 rows x 32 columns x
-// 8 tokens takes 8 clocks of a scheduler, the eight fused multiply-adds that apply its scales another 8 (as four packed ones they were
-// slower, 259 us where these take 208: packed operations have half the pipes, and every row scale needed a copy).
-// What must not cost extra is shared memory: every warp reads its own fragments of both operands.
+// Bound: the scaling of the Q4_0 blocks.  An mma of 16 rows x 32 columns x 8 tokens takes 8 clocks of a scheduler, the eight fused
+// multiply-adds that apply its scales another 8 (as four packed ones they were slower, 259 us where these take 208: packed operations
+// have half the pipes, and every row scale needed a copy).  What must not cost extra is shared memory: every warp reads its own
+// fragments of both operands.
 //
 // Work split: as in pi_mm.cu every CTA takes an equal contiguous range of rows, in tiles of 192 (96), and producer warps (4) copy for the
 // consumers (12) (a computing warp that issues cp.async waits while the SM's queue of outstanding loads is full: 700 to 2900 of the
-// clocks of a stage).  Here all consumers share a stage (128 bytes of every activation, 128 or 64 of every row) and split the TILE:
+// clocks of a stage).  Here all consumers share a stage (128 columns: 128 bytes of every activation, 64 of every row) and split the TILE:
 // no partial sums, so the accumulators of a tile exist once and the tile can be 96 x 256.  Up to 128 tokens 6 x 2 consumers, beyond that 3 x 4,
 // of 2 x 16 rows, the second of which a tile of up to half its height goes without; the token count of a consumer is a template argument in steps of 8 or 16, because a branch
 // around every pair of products costs more than the products that it leaves out.
 // Copies: the activations and dense rows come as TMA tiles (one instruction of one thread; with 16-byte cp.async the producers' own
-// instruction rate, 50 clocks per warp and copy, bound every launch of few rows), gathered rows and the Q4_0 rows' scales by cp.async.
+// instruction rate, 50 clocks per warp and copy, bound every launch of few rows), gathered rows and the rows' scales by cp.async.
 // The accumulators go straight to global memory: the ring runs on across tiles.
 // Every wait is bounded, as in pi_mm.cu.
-#include "pi_common.cuh"
+#include "pi_tc.cuh"
 
-#include <cuda.h>
 #include <type_traits>
 
 namespace pi {
@@ -31,7 +29,7 @@ static constexpr int MW_SMAX = 6;                       // stages at most
 static constexpr int MW_TOKENS = 256;                   // of a launch
 
 struct alignas(64) MwP {
-    CUtensorMap m_w, m_x, m_x2, m_d;                    // dense rows; activation (Q4_0: its low and high planes, its scales)
+    CUtensorMap m_w, m_x, m_x2, m_d;                    // dense rows; activation: its low and high planes, its scales
     int per_tile;                                       // dense: rows of a tile
     const uint8_t * W; const uint8_t * W2; int64_t row_bytes; int nrows, ncols, nb;
     Act x; int T;
@@ -47,19 +45,9 @@ struct alignas(64) MwP {
 
 __device__ __forceinline__ void mw_cp16(uint32_t dst, const void * src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory"); }
 __device__ __forceinline__ void mw_cp8(uint32_t dst, const void * src)  { asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" :: "r"(dst), "l"(src) : "memory"); }
-// the tile of `map` at columns x.., rows y.. (x times the element size a multiple of 16 bytes)
-__device__ __forceinline__ void mw_tma(void * dst, const CUtensorMap * map, int x, int y, uint64_t * bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 :: "r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mw_zero16(uint32_t dst) { asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" :: "r"(dst), "r"(0u) : "memory"); }
 __device__ __forceinline__ void mw_arrive_copies(uint64_t * bar) { asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" :: "r"(smem_u32(bar)) : "memory"); }
 __device__ __forceinline__ void mw_ldsm4(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void mw_hmma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 // (the C operand: four registers of their own, kept: as one value four times over it was copied into place for every product)
 __device__ __forceinline__ void mw_imma(uint32_t (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, const uint32_t (&c)[4]) {
@@ -70,28 +58,24 @@ __device__ __forceinline__ void mw_imma(uint32_t (&d)[4], const uint32_t (&a)[4]
 __device__ __forceinline__ void mw_scale_add(float & acc, uint32_t v, float dd, float md, float d4) { acc = fmaf(fmaf(__uint_as_float(v), dd, md), d4, acc); }
 
 // WM x WN consumers of MT x 16 rows and NT x 8 tokens
-template <int WT, int WM, int WN, int NT>
+template <int WM, int WN, int NT>
 struct MwShape {
-    static constexpr bool Q4 = WT == PI_TYPE_Q4_0;
     static constexpr int TM = WM * MW_MT * 16, TN = WN * NT * 8;       // rows and tokens of a tile
     // 384 consumers + 128 producers share the 512 x 128 registers of the launch; producers of 192 gathered rows keep 12 addresses each
     static constexpr int REGS_C = WM == 6 ? 152 : 160, REGS_P = WM == 6 ? 56 : 32;
-    static constexpr int KS = Q4 ? 128 : 64;                          // columns of a stage
-    static constexpr int WB = Q4 ? 64 : 128;                          // bytes of a row in a stage (Q4_0: of its nibbles)
-    // a stage: rows [TM][WB], activations [TN][128], Q4_0: rows' scales [TM][4 halves], activation scales [4][TN] floats
-    // (Q4_0: low plane [TN][64], high plane [TN][64]; activation scales [TN][4]).  TMA writes and ldmatrix reads with the 16-byte pieces of a
+    static constexpr int KS = 128, WB = 64;                           // columns of a stage, bytes of a row's nibbles in it
+    // a stage: rows [TM][64], activations' low plane [TN][64] and high plane [TN][64], rows' scales [TM][4 halves], activation
+    // scales [TN][4 floats].  TMA writes and ldmatrix reads with the 16-byte pieces of a
     // row permuted by the row's number in groups of 8 (64-byte rows: pairs of rows in groups of 4), counted from 1024-byte boundaries.
-    static constexpr int X_OFF = TM * WB, S_OFF = X_OFF + TN * 128, D_OFF = S_OFF + (Q4 ? TM * 8 : 0), STAGE = (D_OFF + (Q4 ? TN * 16 : 0) + 1023) / 1024 * 1024;
+    static constexpr int X_OFF = TM * WB, S_OFF = X_OFF + TN * 128, D_OFF = S_OFF + TM * 8, STAGE = (D_OFF + TN * 16 + 1023) / 1024 * 1024;
     static_assert(WM * WN == MW_CONS && X_OFF % 1024 == 0 && D_OFF % 128 == 0 && TN % 8 == 0 && TN <= 256, "split");
 };
 
-template <int WT, int WM, int WN, int NT, bool SPARSE, bool GATED>
+template <int WM, int WN, int NT, bool SPARSE, bool GATED>
 __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant__ MwP p) {
-    using Z = MwShape<WT, WM, WN, NT>;
-    constexpr bool Q4 = Z::Q4;
+    using Z = MwShape<WM, WN, NT>;
     constexpr int TM = Z::TM, WB = Z::WB, MT = MW_MT;
     const int IT = GATED ? TM / 2 : SPARSE ? TM : p.per_tile;         // items (rows / neurons) of a tile
-    constexpr bool COPIES = SPARSE || Q4;                             // some of a stage comes by cp.async
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     __shared__ int s_warp[MW_THREADS / 32];
@@ -105,7 +89,7 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
     const uint32_t ring = smem_u32(smem);
     constexpr uint32_t x_off = Z::X_OFF, s_off = Z::S_OFF, d_off = Z::D_OFF;
     if (tid < 8) s_any[tid] = 0u;
-    if (tid < MW_SMAX) { mbar_init(s_full + tid, COPIES ? MW_PROD + 1 : 1); mbar_init(s_empty + tid, MW_CONS); }
+    if (tid < MW_SMAX) { mbar_init(s_full + tid, MW_PROD + 1); mbar_init(s_empty + tid, MW_CONS); }
     if (tid == 0) { mbar_init(s_bits, MW_CONS); mbar_init(s_bits + 1, MW_CONS); s_dead = 0; }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncthreads();
@@ -139,9 +123,8 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
         ok = r < TM && lo + k < hi;
         return (GATED && (r & 8) ? p.W2 : p.W) + (ok ? (size_t)(SPARSE ? rows[k] : lo + k) * p.row_bytes : 0);
     };
-    const bool ragged = !Q4 && p.ncols % 64 != 0;                     // the last slice of a row is not whole
     const int wr = pt / CW;
-    const uint32_t w_to = (uint32_t)(wr * WB + (Q4 ? (cw ^ (wr >> 1)) & 3 : (cw ^ wr) & 7) * 16);
+    const uint32_t w_to = (uint32_t)(wr * WB + ((cw ^ (wr >> 1)) & 3) * 16);
     auto issue_w = [&](int slot) {                                    // cp.async: addresses are kept and moved along
         if (i_slice == 0) {
             w_ok = 0u;
@@ -152,22 +135,21 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
                 if (ok) w_ok |= 1u << j;
             }
 #pragma unroll
-            for (int j = 0; j < (Q4 ? 2 : 0); j++) {
+            for (int j = 0; j < 2; j++) {
                 bool ok;
                 sp[j] = row_ptr(pt + j * MW_PROD, ok) + (size_t)p.nb * 16;
                 if (ok) w_ok |= 1u << (NW + j);
             }
         }
         const uint32_t base = ring + (uint32_t)(slot * Z::STAGE);
-        const bool in = !ragged || i_slice * 64 + cw * 8 < p.ncols;   // past the end of a row: zeros
 #pragma unroll
         for (int j = 0; j < (SPARSE ? NW : 0); j++) {
             const uint32_t to = base + w_to + j * WS * WB;
-            if (w_ok >> j & 1u) { if (in) mw_cp16(to, wp[j]); else mw_zero16(to); }
+            if (w_ok >> j & 1u) mw_cp16(to, wp[j]);
             wp[j] += WB;
         }
 #pragma unroll
-        for (int j = 0; j < (Q4 ? 2 : 0); j++) {
+        for (int j = 0; j < 2; j++) {
             if (w_ok >> (NW + j) & 1u) mw_cp8(base + s_off + (pt + j * MW_PROD) * 8, sp[j]);
             sp[j] += 8;
         }
@@ -175,13 +157,11 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
     auto issue_tma = [&](int slot) {                                  // one thread
         unsigned char * base = smem + (size_t)slot * Z::STAGE;
         uint64_t * bar = s_full + slot;
-        mbar_expect_tx(bar, (unsigned)(Z::TN * 128 + (Q4 ? Z::TN * 16 : 0) + (SPARSE ? 0 : p.per_tile * WB)));
-        if (!SPARSE) mw_tma(base, &p.m_w, i_slice * 64, lo + i_tile * IT, bar);
-        mw_tma(base + x_off, &p.m_x, i_slice * 64, 0, bar);
-        if (Q4) {
-            mw_tma(base + x_off + Z::TN * 64, &p.m_x2, i_slice * 64, 0, bar);
-            mw_tma(base + d_off, &p.m_d, i_slice * 4, 0, bar);
-        }
+        mbar_expect_tx(bar, (unsigned)(Z::TN * 128 + Z::TN * 16 + (SPARSE ? 0 : p.per_tile * WB)));
+        if (!SPARSE) tma_tile(smem_u32(base), &p.m_w, i_slice * 64, lo + i_tile * IT, bar);
+        tma_tile(smem_u32(base + x_off), &p.m_x, i_slice * 64, 0, bar);
+        tma_tile(smem_u32(base + x_off + Z::TN * 64), &p.m_x2, i_slice * 64, 0, bar);
+        tma_tile(smem_u32(base + d_off), &p.m_d, i_slice * 4, 0, bar);
     };
     auto advance = [&]() { if (++i_slice == p.n_slices) { i_slice = 0; i_tile++; } };
 
@@ -245,15 +225,11 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(Z::REGS_P));
         int slot = 0;
         unsigned phase = 1u;                                          // parity of the hand-back to wait for (first round: none)
-        if (!COPIES && warp > MW_CONS) return;
         for (int i = 0; i < n_units; i++) {
             if (!wait(s_empty + slot, phase)) break;
             if (pt == 0) issue_tma(slot);
-            if (COPIES) {
-                issue_w(slot);
-                if (ragged && i_slice == p.n_slices - 1) __threadfence_block();  // zeros were stored, not copied
-                mw_arrive_copies(s_full + slot);
-            }
+            issue_w(slot);
+            mw_arrive_copies(s_full + slot);
             advance();
             if (++slot == S) { slot = 0; phase ^= 1u; }
         }
@@ -285,11 +261,11 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
     constexpr int MS = APART ? WM * 16 : 16;
     const int row0 = wm * (APART ? 16 : 32), tok0 = wn * NT * 8;
     // ldmatrix row addresses inside a stage (fragment layouts of mma.m16n8k16 / m16n8k32); the piece is added per step
-    const uint32_t a_row = (uint32_t)((row0 + (lane & 15) + (Q4 ? (lane >> 4) * MS : 0)) * WB);
-    constexpr int XB = Q4 ? 64 : 128;                                 // bytes of a token (Q4_0: of a plane)
-    const uint32_t plane = Q4 ? ((lane >> 3) & 1) * Z::TN * 64 : 0;
+    const uint32_t a_row = (uint32_t)((row0 + (lane & 15) + (lane >> 4) * MS) * WB);
+    constexpr int XB = 64;                                            // bytes of a token in a plane
+    const uint32_t plane = ((lane >> 3) & 1) * Z::TN * 64;
     const uint32_t b_row = x_off + plane + (uint32_t)((tok0 + (lane & 7) + (lane >> 4) * 8) * XB), b_last = x_off + plane + (uint32_t)((tok0 + (NT - 1) * 8 + (lane & 7)) * XB);
-    const int a_swz = Q4 ? (lane >> 1) & 3 : lane & 7, b_swz = Q4 ? (lane & 7) >> 1 : lane & 7;
+    const int a_swz = (lane >> 1) & 3, b_swz = (lane & 7) >> 1;
 
     int tile = 0, slice = 0, slot = 0;
     unsigned phase = 0u;
@@ -300,62 +276,43 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
         const bool busy = (GATED ? row0 / 2 : row0) < n_tile && tok0 < p.T;       // my rows and tokens exist
         auto multiply = [&](auto mc) {                                // MC fragments of 16 rows
             constexpr int MC = decltype(mc)::value;
-            if (!Q4) {
 #pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    uint32_t a[MC][4];
+            for (int k = 0; k < 4; k++) {                         // block by block
+                uint32_t w[4], a[MC][4];
+                mw_ldsm4(w, base + a_row + ((k ^ a_swz) & 3) * 16);
+                float d4[MC][2];                                  // (the nibbles stand for 16 times their value)
 #pragma unroll
-                    for (int m = 0; m < MC; m++) mw_ldsm4(a[m], base + a_row + m * MS * WB + (((2 * k + (lane >> 4)) ^ a_swz) & 7) * 16);
+                for (int m = 0; m < MC; m++) {
+                    const uint32_t w0 = w[2 * m], wh = w[2 * m + 1];
+                    a[m][0] = ((w0 << 4) & 0xF0F0F0F0u) ^ 0x80808080u; a[m][1] = ((wh << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
+                    a[m][2] = (w0 & 0xF0F0F0F0u) ^ 0x80808080u;        a[m][3] = (wh & 0xF0F0F0F0u) ^ 0x80808080u;
 #pragma unroll
-                    for (int n = 0; n < NT; n += 2) {
-                        uint32_t b[4];
-                        mw_ldsm4(b, base + (n + 1 < NT ? b_row + n * 8 * XB : b_last) + (((2 * k + ((lane >> 3) & 1)) ^ b_swz) & 7) * 16);
-#pragma unroll
-                        for (int m = 0; m < MC; m++) {
-                            mw_hmma(acc[m][n], a[m], b[0], b[1]);
-                            if (n + 1 < NT) mw_hmma(acc[m][(n + 1) % NT], a[m], b[2], b[3]);
-                        }
+                    for (int h = 0; h < 2; h++) {
+                        unsigned short s;
+                        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(s) : "r"(base + s_off + (row0 + m * MS + g + h * 8) * 8 + k * 2));
+                        d4[m][h] = __half2float(__ushort_as_half(s)) * 0.0625f;
                     }
                 }
-            } else {
 #pragma unroll
-                for (int k = 0; k < (Q4 ? 4 : 0); k++) {              // block by block
-                    uint32_t w[4], a[MC][4];
-                    mw_ldsm4(w, base + a_row + ((k ^ a_swz) & 3) * 16);
-                    float d4[MC][2];                                  // (the nibbles stand for 16 times their value)
+                for (int n = 0; n < NT; n += 2) {
+                    uint32_t b[4];
+                    mw_ldsm4(b, base + (n + 1 < NT ? b_row + n * 8 * XB : b_last) + ((k ^ b_swz) & 3) * 16);
 #pragma unroll
-                    for (int m = 0; m < MC; m++) {
-                        const uint32_t w0 = w[2 * m], wh = w[2 * m + 1];
-                        a[m][0] = ((w0 << 4) & 0xF0F0F0F0u) ^ 0x80808080u; a[m][1] = ((wh << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
-                        a[m][2] = (w0 & 0xF0F0F0F0u) ^ 0x80808080u;        a[m][3] = (wh & 0xF0F0F0F0u) ^ 0x80808080u;
+                    for (int u = 0; u < 2; u++) {
+                        if (n + u >= NT) break;
+                        float t0, t1;                             // scales of tokens 2q, 2q + 1
+                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t0) : "r"(base + d_off + (tok0 + (n + u) * 8 + 2 * q) * 16 + k * 4));
+                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t1) : "r"(base + d_off + (tok0 + (n + u) * 8 + 2 * q + 1) * 16 + k * 4));
+                        const float m0 = t0 * -12582912.0f, m1 = t1 * -12582912.0f;
 #pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            unsigned short s;
-                            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(s) : "r"(base + s_off + (row0 + m * MS + g + h * 8) * 8 + k * 2));
-                            d4[m][h] = __half2float(__ushort_as_half(s)) * 0.0625f;
-                        }
-                    }
-#pragma unroll
-                    for (int n = 0; n < NT; n += 2) {
-                        uint32_t b[4];
-                        mw_ldsm4(b, base + (n + 1 < NT ? b_row + n * 8 * XB : b_last) + ((k ^ b_swz) & 3) * 16);
-#pragma unroll
-                        for (int u = 0; u < 2; u++) {
-                            if (n + u >= NT) break;
-                            float t0, t1;                             // scales of tokens 2q, 2q + 1
-                            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t0) : "r"(base + d_off + (tok0 + (n + u) * 8 + 2 * q) * 16 + k * 4));
-                            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t1) : "r"(base + d_off + (tok0 + (n + u) * 8 + 2 * q + 1) * 16 + k * 4));
-                            const float m0 = t0 * -12582912.0f, m1 = t1 * -12582912.0f;
-#pragma unroll
-                            for (int m = 0; m < MC; m++) {
-                                uint32_t c[4];
-                                mw_imma(c, a[m], b[2 * u], b[2 * u + 1], MAGIC);
-                                float (&o)[4] = acc[m][(n + u) % NT];
-                                mw_scale_add(o[0], c[0], t0, m0, d4[m][0]);
-                                mw_scale_add(o[1], c[1], t1, m1, d4[m][0]);
-                                mw_scale_add(o[2], c[2], t0, m0, d4[m][1]);
-                                mw_scale_add(o[3], c[3], t1, m1, d4[m][1]);
-                            }
+                        for (int m = 0; m < MC; m++) {
+                            uint32_t c[4];
+                            mw_imma(c, a[m], b[2 * u], b[2 * u + 1], MAGIC);
+                            float (&o)[4] = acc[m][(n + u) % NT];
+                            mw_scale_add(o[0], c[0], t0, m0, d4[m][0]);
+                            mw_scale_add(o[1], c[1], t1, m1, d4[m][0]);
+                            mw_scale_add(o[2], c[2], t0, m0, d4[m][1]);
+                            mw_scale_add(o[3], c[3], t1, m1, d4[m][1]);
                         }
                     }
                 }
@@ -433,8 +390,7 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
 typedef CUresult (*MwEncode)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
                              CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// rows of `cols` elements, `pitch` bytes apart, in boxes of box_cols x box_rows; what lies past the ends reads as zeros
-static int mw_map(CUtensorMap * m, CUtensorMapDataType type, const void * base, int64_t cols, int64_t rows, int64_t pitch, int box_cols, int box_rows, CUtensorMapSwizzle swizzle) {
+int tensor_map(CUtensorMap * m, CUtensorMapDataType type, const void * base, int64_t cols, int64_t rows, int64_t pitch, int box_cols, int box_rows, CUtensorMapSwizzle swizzle) {
     static MwEncode encode = nullptr;
     if (!encode) {
         void * f = nullptr;
@@ -451,9 +407,9 @@ static int mw_map(CUtensorMap * m, CUtensorMapDataType type, const void * base, 
     return PI_OK;
 }
 
-template <int WT, int WM, int WN, int NT, bool SPARSE, bool GATED>
+template <int WM, int WN, int NT, bool SPARSE, bool GATED>
 static int mw_go(MwP p, bool pdl, cudaStream_t st) {
-    using Z = MwShape<WT, WM, WN, NT>;
+    using Z = MwShape<WM, WN, NT>;
     p.n_slices = (p.ncols + Z::KS - 1) / Z::KS;
     const int G = (int)imin64(sm_count(), (p.nrows + 7) / 8);
     const int list = SPARSE ? ((p.nrows + G - 1) / G + 1) * 4 : 0;    // bytes
@@ -467,21 +423,16 @@ static int mw_go(MwP p, bool pdl, cudaStream_t st) {
         const int share = (p.nrows + G - 1) / G + (p.masks_out ? 8 : 0), tiles = (share + Z::TM - 1) / Z::TM;
         p.per_tile = p.masks_out ? (share / tiles + 8) / 8 * 8 : (share + tiles - 1) / tiles;
         if (p.per_tile > Z::TM) p.per_tile = Z::TM;
-        if (Z::Q4) rc = mw_map(&p.m_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.W, (int64_t)p.nb * 16, p.nrows, p.row_bytes, 64, p.per_tile, CU_TENSOR_MAP_SWIZZLE_64B);
-        else       rc = mw_map(&p.m_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, p.W, p.ncols, p.nrows, p.row_bytes, 64, p.per_tile, CU_TENSOR_MAP_SWIZZLE_128B);
+        rc = tensor_map(&p.m_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.W, (int64_t)p.nb * 16, p.nrows, p.row_bytes, 64, p.per_tile, CU_TENSOR_MAP_SWIZZLE_64B);
         if (rc != PI_OK) return rc;
     }
-    if (Z::Q4) {
-        if ((rc = mw_map(&p.m_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.x.lo, (int64_t)p.nb * 16, p.T, (int64_t)p.nb * 16, 64, Z::TN, CU_TENSOR_MAP_SWIZZLE_64B)) != PI_OK) return rc;
-        if ((rc = mw_map(&p.m_x2, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.x.hi, (int64_t)p.nb * 16, p.T, (int64_t)p.nb * 16, 64, Z::TN, CU_TENSOR_MAP_SWIZZLE_64B)) != PI_OK) return rc;
-        if ((rc = mw_map(&p.m_d, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, p.x.d, p.nb, p.T, (int64_t)p.nb * 4, 4, Z::TN, CU_TENSOR_MAP_SWIZZLE_NONE)) != PI_OK) return rc;
-    } else {
-        if ((rc = mw_map(&p.m_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, p.x.h16, p.ncols, p.T, (int64_t)p.ncols * 2, 64, Z::TN, CU_TENSOR_MAP_SWIZZLE_128B)) != PI_OK) return rc;
-    }
+    if ((rc = tensor_map(&p.m_x, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.x.lo, (int64_t)p.nb * 16, p.T, (int64_t)p.nb * 16, 64, Z::TN, CU_TENSOR_MAP_SWIZZLE_64B)) != PI_OK) return rc;
+    if ((rc = tensor_map(&p.m_x2, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.x.hi, (int64_t)p.nb * 16, p.T, (int64_t)p.nb * 16, 64, Z::TN, CU_TENSOR_MAP_SWIZZLE_64B)) != PI_OK) return rc;
+    if ((rc = tensor_map(&p.m_d, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, p.x.d, p.nb, p.T, (int64_t)p.nb * 4, 4, Z::TN, CU_TENSOR_MAP_SWIZZLE_NONE)) != PI_OK) return rc;
     static bool attr_done[16] = {false};
     int dev = 0;
     PI_CUDA(cudaGetDevice(&dev));
-    auto kern = k_mm_wide<WT, WM, WN, NT, SPARSE, GATED>;
+    auto kern = k_mm_wide<WM, WN, NT, SPARSE, GATED>;
     if (dev >= 0 && dev < 16 && !attr_done[dev]) {
         PI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MW_SMEM_MAX));
         attr_done[dev] = true;
@@ -490,40 +441,33 @@ static int mw_go(MwP p, bool pdl, cudaStream_t st) {
     return PI_OK;
 }
 
-template <int WT, int WM, int WN, int NT>
+template <int WM, int WN, int NT>
 static int mw_sel(const MwP & p, bool pdl, cudaStream_t st) {
-    if (!p.masks) return mw_go<WT, WM, WN, NT, false, false>(p, pdl, st);
-    if (p.W2)     return mw_go<WT, WM, WN, NT, true, true>(p, pdl, st);
-    return mw_go<WT, WM, WN, NT, true, false>(p, pdl, st);
+    if (!p.masks) return mw_go<WM, WN, NT, false, false>(p, pdl, st);
+    if (p.W2)     return mw_go<WM, WN, NT, true, true>(p, pdl, st);
+    return mw_go<WM, WN, NT, true, false>(p, pdl, st);
 }
 
 // The narrowest tile that holds the tokens: the products of a tile are made for all of its columns.  us at this step | at the next wider one,
-// 12288 x 4096 FP16 and 10240 x 8192 Q4_0: 64 tokens 33.7 | 37.7, 69.2 | 81.7; 80 38.3 | 41.2, 82.8 | 96.0; 96 41.7 | 50.1, 96.5 | 113.7;
-// 128 50.5 | 59.6, 114.6 | 144.1; 192 58.1 | 74.9, 148.7 | 189.6.  (2..32 tokens go to k_mm.)  Steps at 112, 160 and 224 would give token
+// 10240 x 8192: 64 tokens 69.2 | 81.7; 80 82.8 | 96.0; 96 96.5 | 113.7; 128 114.6 | 144.1; 192 148.7 | 189.6.  (2..32 tokens go to k_mm.)  Steps at 112, 160 and 224 would give token
 // counts below them up to half of those differences, for six more instances each.
-template <int WT>
 static int mw_tokens(const MwP & p, bool pdl, cudaStream_t st) {
-    if (p.T <= 64)  return mw_sel<WT, 6, 2, 4>(p, pdl, st);
-    if (p.T <= 80)  return mw_sel<WT, 6, 2, 5>(p, pdl, st);
-    if (p.T <= 96)  return mw_sel<WT, 6, 2, 6>(p, pdl, st);
-    if (p.T <= 128) return mw_sel<WT, 6, 2, 8>(p, pdl, st);
-    if (p.T <= 192) return mw_sel<WT, 3, 4, 6>(p, pdl, st);
-    return mw_sel<WT, 3, 4, 8>(p, pdl, st);
+    if (p.T <= 64)  return mw_sel<6, 2, 4>(p, pdl, st);
+    if (p.T <= 80)  return mw_sel<6, 2, 5>(p, pdl, st);
+    if (p.T <= 96)  return mw_sel<6, 2, 6>(p, pdl, st);
+    if (p.T <= 128) return mw_sel<6, 2, 8>(p, pdl, st);
+    if (p.T <= 192) return mw_sel<3, 4, 6>(p, pdl, st);
+    return mw_sel<3, 4, 8>(p, pdl, st);
 }
 
 // Called by launch_mm, which has checked the arguments.  Tokens go in launches of at most 256.
 int launch_mm_wide(const GemvArgs & a, cudaStream_t st) {
-    const bool q4 = a.wtype == PI_TYPE_Q4_0;
     for (int t0 = 0; t0 < a.T; t0 += MW_TOKENS) {
         MwP p;
         p.W = (const uint8_t *)a.W; p.W2 = (const uint8_t *)a.W2; p.row_bytes = (int64_t)pi_row_bytes(a.wtype, a.ncols);
         p.nrows = (int)a.nrows; p.ncols = (int)a.ncols; p.nb = (int)(a.ncols / 32);
         p.T = a.T - t0 < MW_TOKENS ? a.T - t0 : MW_TOKENS;
-        if (q4) {
-            p.x.lo = a.x.lo + (size_t)t0 * p.nb; p.x.hi = a.x.hi + (size_t)t0 * p.nb; p.x.d = a.x.d + (size_t)t0 * p.nb;
-        } else {
-            p.x.h16 = a.x.h16 + (size_t)t0 * a.ncols;
-        }
+        p.x.lo = a.x.lo + (size_t)t0 * p.nb; p.x.hi = a.x.hi + (size_t)t0 * p.nb; p.x.d = a.x.d + (size_t)t0 * p.nb;
         p.masks = a.masks; p.bucket = a.bucket; p.list = a.list_out; p.count = a.count_out; p.rows_total = t0 == 0 ? a.rows_total : nullptr;
         p.idx = a.idx ? a.idx + (size_t)t0 * a.idx_stride : nullptr; p.idx_stride = a.idx_stride; p.threshold = a.threshold;
         p.bias = a.bias; p.relu = a.relu;
@@ -531,7 +475,7 @@ int launch_mm_wide(const GemvArgs & a, cudaStream_t st) {
         p.dst16 = a.dst16 ? a.dst16 + (size_t)t0 * a.dst_stride : nullptr; p.dst_stride = a.dst_stride;
         p.coef = a.coef ? a.coef + (size_t)t0 * a.coef_stride : nullptr; p.coef_stride = a.coef_stride;
         p.masks_out = a.masks_out; p.masks_threshold = a.masks_threshold; p.masks_or = t0 > 0; p.status = a.status;
-        const int rc = q4 ? mw_tokens<PI_TYPE_Q4_0>(p, a.pdl, st) : mw_tokens<PI_TYPE_F16>(p, a.pdl, st);
+        const int rc = mw_tokens(p, a.pdl, st);
         if (rc != PI_OK) return rc;
     }
     return PI_OK;
