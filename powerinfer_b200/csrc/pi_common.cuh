@@ -174,7 +174,10 @@ int axpy_groups(int wtype, int64_t ncols, int T);                     // row gro
 int launch_axpy(const AxpyArgs & a, cudaStream_t st, int * groups_used = nullptr);   // groups_used: partial vectors written
 int launch_axpy_mm(const AxpyArgs & a, cudaStream_t st, int * groups_used);          // 2+ tokens, needs coef; PI_ERR_UNSUPPORTED: not eligible
 bool axpy_mm_exact(int wtype, int64_t nrows, int64_t ncols, int T);                  // the batch's coefficients are to be F32, else FP16
-int axpy_mm_pieces(int64_t ncols, int T);                                            // partial vectors launch_axpy_mm writes
+int axpy_mm_pieces(int64_t ncols, int T);                                            // partial vectors launch_axpy_mm writes with room for as many
+int axpy_mm_least_pieces(int64_t ncols, int T);                                      // ... that it can do with
+int launch_axpy_tc(const AxpyArgs & a, cudaStream_t st, int * groups_used);          // many tokens, FP16 coefficients, zeros behind them to the next multiple of 64
+int axpy_tc_pieces(int64_t ncols);
 // axpy coefficients by list position (pi_axpy_mm.cu): [T, coef_stride], FP16 or (exact) F32, from h F32 [T, h_stride] by global neuron id
 struct CoefArgs {
     int wtype = PI_TYPE_F16;

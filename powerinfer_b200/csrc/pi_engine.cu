@@ -170,6 +170,7 @@ struct pi_engine {
     int hd, dq, dkv, F, T_max;
     int P_max;                               // tokens of a prompt chunk (>= T_max)
     int G;                                   // axpy row groups (one token)
+    bool few_pieces;                         // the workspace has room for the least partial vectors of a batch only
     // device buffers carved from the caller's workspace
     int32_t * tokens, * pos, * seq_ids, * seq_pf, * argmax;   // seq_pf: the sequence of every token of a prompt chunk
     float * x, * x2, * attn_out, * ffn_vec, * qkv, * pred, * h, * partial, * logits, * cs;
@@ -235,7 +236,7 @@ static void carve(pi_engine * e, void * ws, size_t ws_bytes, bool dry, size_t * 
     e->qkv = cv.take<float>((size_t)T * (e->dq + 2 * e->dkv));
     e->pred = cv.take<float>(T * F); e->h = cv.take<float>(T * F);
     size_t vecs = 0;                                                 // partial vectors of 2+ tokens, of one token
-    for (int t = 2; t <= T; t++) vecs = std::max(vecs, (size_t)axpy_mm_pieces(c.d, t) * t);
+    for (int t = 2; t <= T; t++) vecs = std::max(vecs, (size_t)(e->few_pieces ? axpy_mm_least_pieces(c.d, t) : axpy_mm_pieces(c.d, t)) * t);
     e->partial = cv.take<float>((vecs > (size_t)e->G ? vecs : (size_t)e->G) * d);
     e->logits = cv.take<float>((size_t)B * c.n_vocab);
     e->cs = cv.take<float>((size_t)c.n_ctx * e->hd);
@@ -396,6 +397,7 @@ int pi_engine_create(const pi_engine_config * cfg, const pi_model_weights * gw, 
     size_t need = 0;
     plan_step(e, !gw->output);
     carve(e, workspace, workspace_bytes, false, &need);
+    if (need == (size_t)-1) { e->few_pieces = true; carve(e, workspace, workspace_bytes, false, &need); }      // (room for fewer partial vectors)
     if (need == (size_t)-1 && e->step.ok) { e->step = StepPlan(); carve(e, workspace, workspace_bytes, false, &need); }
     if (need == (size_t)-1) { delete e; set_error("engine_create: workspace of %zu bytes is too small", workspace_bytes); return PI_ERR_WORKSPACE; }
     e->k_cache = (__half *)k_cache; e->v_cache = (__half *)v_cache;
@@ -747,7 +749,7 @@ int enqueue_step(pi_engine * e, int T, cudaStream_t st, StageTimer & tm, int mod
                 a.wtype = wt; a.Wt = L->down_t; a.nrows = F; a.ncols = d; a.h = e->h; a.h_stride = F; a.T = T;
                 if (T == 1 && rows1) { a.masks = e->masks; a.h_uncleared = masks1; } else { a.list = e->list; a.count = e->count; }
                 a.idx = pred; a.idx_stride = F; a.threshold = c.threshold;
-                a.cq = e->cq; a.cd = e->cd; a.partial = e->partial; a.n_groups = T == 1 ? e->G : axpy_mm_pieces(d, T); a.status = e->status;
+                a.cq = e->cq; a.cd = e->cd; a.partial = e->partial; a.n_groups = T == 1 ? e->G : e->few_pieces ? axpy_mm_least_pieces(d, T) : axpy_mm_pieces(d, T); a.status = e->status;
                 if (T > 1) { a.coef = e->coef; a.coef_stride = e->coef_stride; a.exact = exact; }
                 STAGE(PI_STAGE_DOWN, 1, launch_axpy(a, st, &used));
             }

@@ -79,6 +79,11 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
             if (p.rows_total && total) atomicAdd(p.rows_total, (unsigned long long)total);      // statistics
         }
         if (p.list) for (int k = tid; k < hi - lo; k += MT_THREADS) p.list[lo + k] = rows[k];
+        if (p.coef && cta == G - 1) {                                 // zeros behind the last position (k_axpy_tc reads stages of 64)
+            const int64_t end = (total + 63) / 64 * 64 < p.coef_stride ? (total + 63) / 64 * 64 : p.coef_stride;
+            for (int e = tid; e < p.T * 64; e += MT_THREADS)
+                if (total + e % 64 < end) p.coef[(size_t)(e / 64) * p.coef_stride + total + e % 64] = __ushort_as_half((unsigned short)0);
+        }
     } else {
         const int al = p.masks_out ? 8 : 1, gr = (p.nrows + al - 1) / al;          // (a byte of the masks has one writer)
         lo = min(p.nrows, (int)((long long)gr * cta / G) * al);

@@ -59,3 +59,27 @@ def test_gathered_products(ops, rows, cols, T, share):
     y = ops.sparse_ffn(up, gate, down, x, idx).double()
     assert ((y - h @ d).abs() <= (rows * share + 8) * 2.0 ** -23 * (h.abs() @ d.abs()) + 1e-30).all()
     assert ops.last_op_status() == 0
+
+
+# list ranges that end inside a stage of 64, no and every row, columns in parts of a range, one accumulator and several, a second launch
+@pytest.mark.parametrize("share", [0.0, 0.01, 0.7, 1.0])
+@pytest.mark.parametrize("rows,cols,T", [(40, 1024, 65), (1500, 3072, 77), (3001, 2056, 129), (700, 1032, 128), (900, 520, 256), (5000, 4096, 261), (300, 8, 70)])
+def test_axpy_of_many_tokens(ops, rows, cols, T, share):
+    gen = generator(rows + T)
+    W = weight(ops, synth.F16, rows, cols, gen)
+    idx = torch.where((torch.rand(1, rows, device="cuda", generator=gen) < share) & (torch.rand(T, rows, device="cuda", generator=gen) < 0.7), 1.0, -1.0)
+    h = torch.randn(T, rows, device="cuda", generator=gen).relu()
+    c, w = h.half().double() * (idx >= 0), ops.dequantize(W).double()
+    got = ops.ggml_axpy(W, h, idx)
+    assert ((got.double() - c @ w).abs() <= (rows * share + 8) * 2.0 ** -23 * (c.abs() @ w.abs()) + 1e-30).all()
+    assert torch.equal(got, ops.ggml_axpy(W, h, idx))
+    assert ops.last_op_status() == 0
+
+
+def test_prompt_with_rounded_factors_of_256_columns():
+    """Q4_0 rows go to k_axpy_tc within prompts only, where their factors are rounded to FP16: a prompt against the same prompt token by
+    token, at a width of two ranges of 256 columns and more (1024 columns, in ranges of 128: test_gpu_prefill)."""
+    from powerinfer_b200 import engine
+    from test_gpu_prefill import against_single_steps
+    against_single_steps(engine, synth.ModelSpec(arch=synth.ARCH_LLAMA, wtype=synth.Q4_0, n_layer=1, d=2048, n_ff=5024, n_head=16, n_head_kv=4, rank=64, n_vocab=256,
+                                                 n_ctx=256, firing=0.6, seed=9), (77, 129, 200))
