@@ -134,6 +134,8 @@ int launch_gemv(const GemvArgs & a, cudaStream_t st);
 int launch_gemv_ring(const GemvArgs & a, unsigned int * status, bool pdl, cudaStream_t st, bool * wrote_masks = nullptr);
 int launch_mm(const GemvArgs & a, cudaStream_t st);                                           // 2+ tokens; PI_ERR_UNSUPPORTED: not eligible
 int launch_mm_wide(const GemvArgs & a, cudaStream_t st);                                      // 33+ tokens, Q4_0 rows (called by launch_mm)
+bool mm_q4_takes(const GemvArgs & a);                                                         // ... of which these go to launch_mm_q4
+int launch_mm_q4(const GemvArgs & a, cudaStream_t st);
 int launch_mm_tc(const GemvArgs & a, cudaStream_t st);                                        // the same for FP16 rows
 static constexpr int64_t MM_MAX_ROWS = 262144;                                                // rows a gather of launch_mm can choose from
 

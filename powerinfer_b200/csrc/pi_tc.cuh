@@ -36,6 +36,11 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t d, uint64_t a, uint64_t b, u
     asm volatile("{\n .reg .pred e, p;\n elect.sync _|e, 0xffffffff;\n setp.ne.u32 p, %4, 0;\n @e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
                  :: "r"(d), "l"(a), "l"(b), "r"(idesc), "r"((unsigned)accumulate) : "memory");
 }
+// the same with A in tensor memory: 128 lanes x 8 columns of two halves
+__device__ __forceinline__ void tc_mma_f16_ta(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, bool accumulate) {
+    asm volatile("{\n .reg .pred e, p;\n elect.sync _|e, 0xffffffff;\n setp.ne.u32 p, %4, 0;\n @e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+                 :: "r"(d), "r"(a), "l"(b), "r"(idesc), "r"((unsigned)accumulate) : "memory");
+}
 // the barrier completes when all products that this warp's elected lane has issued are done
 __device__ __forceinline__ void tc_commit(uint64_t * bar) {
     asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n @e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" :: "r"(smem_u32(bar)) : "memory");
@@ -57,6 +62,17 @@ __device__ __forceinline__ void tc_ld16(float (&v)[16], uint32_t addr) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\ttcgen05.wait::ld.sync.aligned;"
                  : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]) : "r"(addr));
 }
+
+__device__ __forceinline__ void tc_ld8(float (&v)[8], uint32_t addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\ttcgen05.wait::ld.sync.aligned;"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "r"(addr));
+}
+// 16 columns back; tc_wait_st: this warp's stores are there
+__device__ __forceinline__ void tc_st16(uint32_t addr, const uint32_t (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 :: "r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
+}
+__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // ---- The rows that the masks name, dealt to `groups` in equal contiguous ranges by rank: rank range [lo, hi) of group `grp`, its row
 // numbers to rows[0 .. hi - lo).  All THREADS threads call it, s_warp holds THREADS / 32 words; returns the number of active rows.

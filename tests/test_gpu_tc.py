@@ -7,7 +7,7 @@ import pytest
 
 from powerinfer_b200 import synth
 from test_gpu_batch_edges import generator
-from test_gpu_batches import weight
+from test_gpu_batches import rounded, weight
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -83,3 +83,56 @@ def test_prompt_with_rounded_factors_of_256_columns():
     from test_gpu_prefill import against_single_steps
     against_single_steps(engine, synth.ModelSpec(arch=synth.ARCH_LLAMA, wtype=synth.Q4_0, n_layer=1, d=2048, n_ff=5024, n_head=16, n_head_kv=4, rank=64, n_vocab=256,
                                                  n_ctx=256, firing=0.6, seed=9), (77, 129, 200))
+
+
+def close_q4(got, x, w, keep=None):
+    """Each product of halves is exact, the dropped ones lie below 2^-24 of their term, a drain of 64 terms is cut up to 12 times at 2^-23 of what it
+    holds then, and the drains are added in FP32: far within one unit of 2^-23 per 4 terms, which is asserted."""
+    ref, mass = x @ w.T, x.abs() @ w.abs().T
+    err = (got.double() - ref).abs()
+    if keep is not None:
+        err = err * keep
+    assert (err <= (x.shape[1] / 4 + 16) * 2.0 ** -23 * mass + 1e-30).all()
+    ref, err = (ref, err) if keep is None else (ref * keep, err)
+    assert err.norm() <= 4e-7 * ref.norm() + 1e-30
+
+
+# 9.. rows per CTA, tiles of 16, 96, 160 rows and several of them, sizes around every line of mm_q4_takes, a second launch
+@pytest.mark.parametrize("rows,cols,T", [(8, 2048, 193), (1000, 2304, 256), (2370, 4352, 200), (10000, 2048, 97), (24000, 2048, 128), (12100, 2048, 256), (5000, 2048, 261)])
+def test_q4_products(ops, rows, cols, T):
+    gen = generator(rows + T)
+    W, x = weight(ops, synth.Q4_0, rows, cols, gen), torch.randn(T, cols, device="cuda", generator=gen) * torch.exp(torch.randn(1, cols, device="cuda", generator=gen))
+    bias = torch.randn(rows, device="cuda", generator=gen)
+    got = ops.ggml_mul_mat(W, x)
+    close_q4(got, rounded(ops, synth.Q4_0, x), ops.dequantize(W).double())
+    assert torch.equal(ops.ggml_mul_mat(W, x, bias), got + bias)
+    assert ops.last_op_status() == 0
+
+
+@pytest.mark.parametrize("share", [0.0, 0.004, 0.6, 1.0])
+@pytest.mark.parametrize("rows,cols,T", [(640, 2048, 97), (5000, 2304, 128), (24000, 2048, 129), (3001, 4096, 256)])
+def test_q4_gathers(ops, rows, cols, T, share):
+    gen = generator(rows + T)
+    up, gate = weight(ops, synth.Q4_0, rows, cols, gen), weight(ops, synth.Q4_0, rows, cols, gen)
+    x = torch.randn(T, cols, device="cuda", generator=gen)
+    idx = torch.where((torch.rand(1, rows, device="cuda", generator=gen) < share) & (torch.rand(T, rows, device="cuda", generator=gen) < 0.7), 1.0, -1.0)
+    on, xr = idx >= 0, rounded(ops, synth.Q4_0, x)
+    got = ops.ggml_mul_mat_idx(up, x, idx)
+    assert (got[~on] == 0).all()
+    close_q4(got, xr, ops.dequantize(up).double(), on)
+    if rows % 32 == 0:                                                # the gated gather of the whole FFN: its hidden values are those of the two nodes
+        h, down = torch.relu(ops.ggml_mul_mat_idx(gate, x, idx)) * got, weight(ops, synth.Q4_0, rows, cols, gen)
+        assert torch.equal(ops.sparse_ffn(up, gate, down, x, idx), ops.ggml_axpy(down, h, idx))
+    assert ops.last_op_status() == 0
+
+
+def test_q4_tokens_above_the_halves_range(ops):
+    """Blocks of a token whose scale times 127 is above 65504, beside tokens and blocks with small ones."""
+    rows, cols, T = 1000, 2048, 200
+    gen = generator(3)
+    W, x = weight(ops, synth.Q4_0, rows, cols, gen), torch.randn(T, cols, device="cuda", generator=gen)
+    x[3] *= 3e4
+    x[70, 64:96] *= 1e6
+    x[71, ::3] *= 1e-4
+    x[199] *= 2e6
+    close_q4(ops.ggml_mul_mat(W, x), rounded(ops, synth.Q4_0, x), ops.dequantize(W).double())
