@@ -28,7 +28,7 @@ static constexpr int MT_PASS = MT_OUT / 8;              // rows of a pass of the
 struct alignas(64) MtP {
     CUtensorMap m_w, m_x;
     const uint8_t * W; const uint8_t * W2; int64_t row_bytes; int nrows, ncols;
-    int T, nt, x_rows, per_tile, ring;                   // token tiles (1, 2), rows of an activation box, rows of a dense box, bytes of the ring
+    int T, nt, n_tt, x_rows, per_tile, ring;             // token tiles of a CTA (1, 2), CTAs that share rows, rows of an activation box, of a dense box, bytes of the ring
     const uint32_t * masks; const int32_t * bucket; int32_t * list; int32_t * count; unsigned long long * rows_total;
     const float * idx; int64_t idx_stride; float threshold;
     const float * bias; int relu;
@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
     float * const epi = reinterpret_cast<float *>(smem_raw + (ring - smem_u32(smem_raw)) + p.ring);
     int * const rows = reinterpret_cast<int *>(epi + MT_OUT / 32 * (MT_EPI / 4));      // rows of this CTA (sparse only)
-    const int G = gridDim.x, cta = blockIdx.x;
+    const int G = gridDim.x / p.n_tt, cta = blockIdx.x / p.n_tt, tok_first = (int)(blockIdx.x % p.n_tt) * 128;
     if (tid < 8) s_any[tid] = 0u;
     if (tid < MT_SMAX) { mbar_init(s_full + tid, SPARSE ? 1 + MT_OUT / 32 : 1); mbar_init(s_empty + tid, 1); }
     if (tid < 2) { mbar_init(s_dfull + tid, 1); mbar_init(s_dempty + tid, MT_OUT / 32); }
@@ -74,12 +74,12 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
     pdl_wait();
     if (SPARSE) {
         const int total = tc_active_rows<MT_THREADS>(p.masks, p.nrows, cta, G, s_warp, rows, lo, hi);
-        if (cta == 0 && tid == 0) {
+        if (blockIdx.x == 0 && tid == 0) {
             if (p.count) *p.count = total;
             if (p.rows_total && total) atomicAdd(p.rows_total, (unsigned long long)total);      // statistics
         }
-        if (p.list) for (int k = tid; k < hi - lo; k += MT_THREADS) p.list[lo + k] = rows[k];
-        if (p.coef && cta == G - 1) {                                 // zeros behind the last position (k_axpy_tc reads stages of 64)
+        if (p.list && tok_first == 0) for (int k = tid; k < hi - lo; k += MT_THREADS) p.list[lo + k] = rows[k];
+        if (p.coef && cta == G - 1 && tok_first == 0) {                                 // zeros behind the last position (k_axpy_tc reads stages of 64)
             const int64_t end = (total + 63) / 64 * 64 < p.coef_stride ? (total + 63) / 64 * 64 : p.coef_stride;
             for (int e = tid; e < p.T * 64; e += MT_THREADS)
                 if (total + e % 64 < end) p.coef[(size_t)(e / 64) * p.coef_stride + total + e % 64] = __ushort_as_half((unsigned short)0);
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
                 mbar_expect_tx(s_full + slot, (unsigned)(su * (p.nt * p.x_rows + (SPARSE ? 0 : p.per_tile)) * 128));
                 for (int u = 0; u < su; u++) {
                     const uint32_t base = ring + (uint32_t)slot * stage + (uint32_t)u * slice_bytes;
-                    for (int t = 0; t < p.nt; t++) tma_tile(base + t * 16384, &p.m_x, (slice + u) * 64, t * 128, s_full + slot);
+                    for (int t = 0; t < p.nt; t++) tma_tile(base + t * 16384, &p.m_x, (slice + u) * 64, tok_first + t * 128, s_full + slot);
                     if (!SPARSE) tma_tile(base + w_off, &p.m_w, (slice + u) * 64, row, s_full + slot);
                 }
             }
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
             const int n_tile = min(items, hi - lo - tile * items);
             constexpr int PER = GATED ? 8 : 16;                       // items of 16 columns
             for (int t = 0; t < p.nt; t++) {
-                const int tok0 = t * 128 + quarter * 32;
+                const int tok0 = tok_first + t * 128 + quarter * 32;
                 if (tok0 >= p.T) break;
                 for (int c = third * 16; c < N; c += 48) {
                     const int k0 = GATED ? c / 2 : c;
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
 // ---------------------------------------------------------------------------------------------- launch
 template <bool SPARSE, bool GATED>
 static int mt_go(MtP & p, bool pdl, cudaStream_t st) {
-    const int G = (int)imin64(sm_count(), (p.nrows + 7) / 8);
+    const int G = (int)imin64(sm_count() / p.n_tt, (p.nrows + 7) / 8);
     const int list = SPARSE ? ((p.nrows + G - 1) / G + 1) * 4 : 0;    // bytes
     p.ring = (MT_SMEM_MAX - 1024 - MT_OUT / 32 * MT_EPI - list) / 1024 * 1024;
     if (p.ring < 2 * (p.nt * 16384 + 256 * 128)) return PI_ERR_UNSUPPORTED;        // two stages of the largest kind (more than MM_MAX_ROWS rows)
@@ -329,7 +329,7 @@ static int mt_go(MtP & p, bool pdl, cudaStream_t st) {
         PI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MT_SMEM_MAX));
         attr_done[dev] = true;
     }
-    PI_CUDA(launch_k(kern, dim3(G), dim3(MT_THREADS), (size_t)MT_SMEM_MAX, st, pdl, p));
+    PI_CUDA(launch_k(kern, dim3(G * p.n_tt), dim3(MT_THREADS), (size_t)MT_SMEM_MAX, st, pdl, p));
     return PI_OK;
 }
 
@@ -340,7 +340,12 @@ int launch_mm_tc(const GemvArgs & a, cudaStream_t st) {
         p.W = (const uint8_t *)a.W; p.W2 = (const uint8_t *)a.W2; p.row_bytes = a.ncols * 2;
         p.nrows = (int)a.nrows; p.ncols = (int)a.ncols;
         p.T = a.T - t0 < 256 ? a.T - t0 : 256;
-        p.nt = (p.T + 127) / 128; p.x_rows = p.nt > 1 ? 128 : (p.T + 7) / 8 * 8;
+        // More than 128 tokens: a CTA has all of them and its share r of the rows, or every other CTA has half of them and 2 r rows.  What it
+        // brings in is 256 + r or 128 + 2 r rows of K: half the tokens below 128 dense rows a CTA (us, 256 tokens, all | half: 1024 x 8192 54 | 37,
+        // 4096 x 4096 33 | 24, 12288 x 4096 42 | 38, 16000 x 4096 47 | 46).  Gathered rows go through the CTA's registers, so that doing it twice
+        // costs more (idx, 72 % of 2048 x 2048 40 | 35, 4096 x 4096 64 | 50, 11008 x 1024 54 | 57).  Masks are the union over ALL tokens.
+        p.n_tt = p.T > 128 && !a.masks_out && a.nrows * (a.W2 ? 2 : 1) < (a.masks ? 6000 : 128 * (int64_t)sm_count()) ? 2 : 1;
+        p.nt = p.n_tt > 1 ? 1 : (p.T + 127) / 128; p.x_rows = p.T > 128 ? 128 : (p.T + 7) / 8 * 8;
         int rc = tensor_map(&p.m_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a.x.h16 + (size_t)t0 * a.ncols, p.ncols, p.T, (int64_t)p.ncols * 2, 64, p.x_rows, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc != PI_OK) return rc;
         p.masks = a.masks; p.bucket = a.bucket; p.list = a.list_out; p.count = a.count_out; p.rows_total = t0 == 0 ? a.rows_total : nullptr;
