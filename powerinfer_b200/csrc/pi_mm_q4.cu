@@ -11,7 +11,7 @@
 // ones cut anything, half a unit each on the average, which the drain gives back (a factor of 1 + 2^-23).  Error against 64 bits, one FP32
 // chain of all blocks (pi_mm_wide.cu) | here: 8192 columns 2.8e-7 | 2.2e-7, 4096 2.1e-7 | 1.7e-7, 2048 1.4e-7 | 1.3e-7, 1024 1.1e-7 | 1.1e-7, 256
 // 0.5e-7 | 0.9e-7: shorter sums stay there (mm_q4_takes).
-// Scales of rows above 8188 would leave the halves' range: weights above 65504, which FP16 rows cannot hold either.
+// A row with a scale above 8188 may leave the halves' range, 65504: its sums are not finite then, and are made anew block by block.
 //
 // Tokens are the 128 lanes (M), rows the columns (N, steps of 16): every CTA takes its equal contiguous range of rows, in tiles of up to 160.
 // More than 128 tokens: neighbouring CTAs take the same rows for other tokens (the second finds them in L2).
@@ -52,11 +52,38 @@ struct alignas(64) TsP {
 __device__ __forceinline__ uint32_t ts_mul2(uint32_t a, uint32_t b) { uint32_t r; asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
 __device__ __forceinline__ uint32_t ts_add2(uint32_t a, uint32_t b) { uint32_t r; asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
 __device__ __forceinline__ uint32_t ts_fma2(uint32_t a, uint32_t b, uint32_t c) { uint32_t r; asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c)); return r; }
+__device__ __forceinline__ uint32_t ts_neg2(uint32_t a) { uint32_t r; asm("neg.f16x2 %0, %1;" : "=r"(r) : "r"(a)); return r; }     // (folds into the next one)
 // a * b = hi + lo, exactly
-__device__ __forceinline__ void ts_split(uint32_t a, uint32_t b, uint32_t & hi, uint32_t & lo) { hi = ts_mul2(a, b); lo = ts_fma2(a, b, hi ^ 0x80008000u); }
+__device__ __forceinline__ void ts_split(uint32_t a, uint32_t b, uint32_t & hi, uint32_t & lo) { hi = ts_mul2(a, b); lo = ts_fma2(a, b, ts_neg2(hi)); }
 // Token scales above 256 (products with 127 above the halves' range) are brought below by a power of two per token and stage, which the
 // drain takes back: its exponent
 __device__ __forceinline__ int ts_down(float d0, float d1) { const int e = (int)(__float_as_uint(fmaxf(d0, d1)) >> 23) - 127; return max(0, e - 7); }
+
+// The rare rows whose scales times 8 are above the halves' range: found, and summed block by block for one token
+__device__ __forceinline__ bool ts_beyond(unsigned short s) { return (s & 0x7FFFu) > 0x6FFFu; }      // |s| > 8188, infinite or NaN
+__device__ __forceinline__ bool ts_row_beyond(const uint8_t * row, int nb, int lane) {               // (the same row in all lanes)
+    const unsigned short * s = reinterpret_cast<const unsigned short *>(row + (size_t)nb * 16);
+    bool any = false;
+    for (int b = lane; b < nb; b += 32) any |= ts_beyond(s[b]);
+    return __any_sync(0xffffffffu, any);
+}
+__device__ __forceinline__ float ts_row_sum(const uint8_t * row, const uint4 * lo, const uint4 * hi, const float * d, int nb) {
+    const unsigned short * s = reinterpret_cast<const unsigned short *>(row + (size_t)nb * 16);
+    float acc = 0.f;
+#pragma unroll 1
+    for (int b = 0; b < nb; b++) {
+        const uint4 q = reinterpret_cast<const uint4 *>(row)[b], l = lo[b], h = hi[b];
+        const uint32_t qs[4] = {q.x, q.y, q.z, q.w}, ls[4] = {l.x, l.y, l.z, l.w}, hs[4] = {h.x, h.y, h.z, h.w};
+        int sum = 0;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {                                 // (q - 8: nibbles as signed bytes)
+            sum = __dp4a((int)__vsub4(qs[j] & 0x0F0F0F0Fu, 0x08080808u), (int)ls[j], sum);
+            sum = __dp4a((int)__vsub4(qs[j] >> 4 & 0x0F0F0F0Fu, 0x08080808u), (int)hs[j], sum);
+        }
+        acc = fmaf((float)sum, __half2float(__ushort_as_half(s[b])) * d[b], acc);
+    }
+    return acc;
+}
 
 template <bool SPARSE, bool GATED>
 __global__ void __launch_bounds__(TS_THREADS, 1) k_mm_q4(const __grid_constant__ TsP p) {
@@ -185,8 +212,8 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_mm_q4(const __grid_constant__
                 int l_i = pw / tasks, l_st = l_i, l_tile = 0;         // the stage that is requested next, of all and of the tile
                 while (l_st >= n_st) { l_st -= n_st; l_tile++; }
                 auto rows_of = [&](int tile) {
-                    const int k = GATED ? r >> 1 : r, item = tile * items + k;
-                    const size_t row = k < items && lo + item < hi ? (size_t)(SPARSE ? rows[item] : lo + item) : 0;    // (a column of no row: any row)
+                    const int item = min(tile * items + (GATED ? r >> 1 : r), hi - lo - 1);       // (a column of no row: the last)
+                    const size_t row = (size_t)(SPARSE ? rows[item] : lo + item);
                     const uint8_t * at = (GATED && (r & 1) ? p.W2 : p.W) + row * p.row_bytes;
                     src = at + (size_t)(l_st * 2 + blk) * 16;
                     scale = at + (size_t)p.nb * 16 + (size_t)(l_st * 2 + blk) * 2;
@@ -309,7 +336,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_mm_q4(const __grid_constant__
         for (int j = 0; j < TS_NC; j++) acc[j] = 0.f;
         int db = 0;
         unsigned dphase = 0u;
-        bool ok = true;
+        bool ok = true, odd = false;                                  // (a sum that is not finite)
         const uint32_t mine_at = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(g * nc);
         const float2 * xd = reinterpret_cast<const float2 *>(p.x.d + (size_t)(tok0 + min(wq * 32 + lane, Tt - 1)) * p.nb);
         const float UP = __uint_as_float(0x3F800001u);                // 1 + 2^-23: what cutting four times takes on the average
@@ -346,6 +373,8 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_mm_q4(const __grid_constant__
             // ---- the tile is complete: a thread holds one token's rows; 16 items at a time become lanes
             const int n_tile = min(items, hi - lo - tile * items), half = items / 2;
             float * mine = epi + (warp - 12) * (TS_EPI / 4);
+#pragma unroll
+            for (int j = 0; j < TS_NC; j++) odd |= !(fabsf(acc[j]) < __int_as_float(0x7F800000));
 #pragma unroll 1
             for (int c = 0; c < half; c += 16) {                      // (one copy of the body: only the selection is unrolled)
                 const int k0 = g * half + c;                          // item of the tile
@@ -394,6 +423,27 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_mm_q4(const __grid_constant__
             }
 #pragma unroll
             for (int j = 0; j < TS_NC; j++) acc[j] = 0.f;
+        }
+        // ---- rows beyond the halves' range, by the warp that wrote their results: a lane has a token
+        if (live && ok && __any_sync(0xffffffffu, odd)) {
+            const int tok = tok0 + wq * 32 + lane;
+            const size_t xb = (size_t)min(tok, p.T - 1) * p.nb;
+#pragma unroll 1
+            for (int item = lo; item < hi; item++) {
+                if ((item - lo) % items / (items / 2) != g) continue;
+                const int r = SPARSE ? rows[item - lo] : item;
+                const uint8_t * const row = p.W + (size_t)r * p.row_bytes, * const row2 = GATED ? p.W2 + (size_t)r * p.row_bytes : nullptr;
+                if (!ts_row_beyond(row, p.nb, lane) && !(GATED && ts_row_beyond(row2, p.nb, lane))) continue;
+                const int64_t gid = SPARSE && p.bucket ? p.bucket[r] : r;
+                if (tok >= p.T || (SPARSE && p.idx[(size_t)tok * p.idx_stride + gid] < p.threshold)) continue;
+                float o = ts_row_sum(row, p.x.lo + xb, p.x.hi + xb, p.x.d + xb, p.nb);
+                if (GATED) o *= fmaxf(ts_row_sum(row2, p.x.lo + xb, p.x.hi + xb, p.x.d + xb, p.nb), 0.f);
+                if (p.bias) o += p.bias[gid];
+                if (p.relu) o = fmaxf(o, 0.f);
+                if (p.dst)   p.dst[(size_t)tok * p.dst_stride + gid] = o;
+                if (p.dst16) p.dst16[(size_t)tok * p.dst_stride + gid] = __float2half_rn(o);
+                if (p.coef)  p.coef[(size_t)tok * p.coef_stride + item] = __float2half_rn(o);
+            }
         }
     }
     tc_fence_before();

@@ -136,3 +136,25 @@ def test_q4_tokens_above_the_halves_range(ops):
     x[71, ::3] *= 1e-4
     x[199] *= 2e6
     close_q4(ops.ggml_mul_mat(W, x), rounded(ops, synth.Q4_0, x), ops.dequantize(W).double())
+
+
+def test_q4_rows_above_the_halves_range(ops):
+    """Rows with weights above 65504, single blocks of them among others, in a dense product and a gather with gate."""
+    rows, cols, T = 1024, 2048, 200
+    gen = generator(4)
+    w = torch.randn(rows, cols, device="cuda", generator=gen) * 0.05
+    w[5] *= 2e6
+    w[700, 320:352] *= 2e6
+    w[1023, ::7] *= 1.5e6
+    W = ops.upload_weight(synth.quantize_q4_0(w.cpu().numpy()), synth.Q4_0, rows, cols)
+    x, wd = torch.randn(T, cols, device="cuda", generator=gen), ops.dequantize(W).double()
+    assert (wd.abs() > 65504).any(1).sum() == 3 and wd.isfinite().all()
+    close_q4(ops.ggml_mul_mat(W, x), rounded(ops, synth.Q4_0, x), wd)
+    idx = torch.where(torch.rand(T, rows, device="cuda", generator=gen) < 0.7, 1.0, -1.0)
+    got = ops.ggml_mul_mat_idx(W, x, idx)
+    close_q4(got, rounded(ops, synth.Q4_0, x), wd, idx >= 0)
+    x, down = x * 0.0001, weight(ops, synth.Q4_0, rows, cols, gen)       # (hidden values within the range of Q8_0's scales; up and gate the same rows)
+    got = ops.ggml_mul_mat_idx(W, x, idx)
+    y = ops.ggml_axpy(down, torch.relu(got) * got, idx)
+    assert y.isfinite().all() and torch.equal(ops.sparse_ffn(W, W, down, x, idx), y)
+    assert ops.last_op_status() == 0
