@@ -6,6 +6,8 @@
 // (92 MB of keys and values), 125 us for 32 prompt tokens with 64 heads.
 //
 // Bound: the bytes of the cached rows for batches, the chain scores -> maximum -> probabilities -> values for chunks.
+// A probability takes the place of a score, and the output sums that of the values: what shared memory holds decides how many CTAs an SM has (256
+// tokens with 64 heads in a context of 768: 113 KB and one CTA an SM before, 89 KB and two now, the longest ones first: 48 -> 45 us).
 // Scores: mma.m16n8k16 with the keys straight from global memory: a lane loads 16 bytes (8 columns) of a row, which serve
 // as B operands of two mma whose k order is permuted in the same way on the query side; four tiles of 8 positions in
 // flight per warp, or two where more than two CTAs per SM have work (attn_mm_go).  Values travel to shared memory by cp.async (tiles of 64 positions, two in flight) while the scores are made and
@@ -45,19 +47,18 @@ __global__ void __launch_bounds__(AM_THREADS, UN == 2 ? 4 : HC == 2 ? 3 : 2) k_a
     __shared__ int s_pos[16];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
     const int group = p.n_head / p.n_head_kv, dkv = p.n_head_kv * HD;
-    // shared-memory map: scores [R][P + 4] F32 (later the output sums) | probabilities [R][P + 8] FP16 | queries [16][Q_PITCH] | values 2 x [64][V_PITCH]
-    const int S_PITCH = p.P + 4, P_PITCH = p.P + 8;
+    // shared-memory map: scores [R][P + 4] F32, later the probabilities as FP16 in their place | queries [16][Q_PITCH] | values 2 x [64][V_PITCH], later the output sums
+    const int S_PITCH = p.P + 4, P_PITCH = 2 * S_PITCH;
     float * sc = reinterpret_cast<float *>(smem);
-    const size_t s_bytes = (size_t)max(p.R * S_PITCH * 4, KSPL * 16 * HD * 4);
-    __half * p16 = reinterpret_cast<__half *>(smem + (s_bytes + 127) / 128 * 128);
-    __half * qs = reinterpret_cast<__half *>(reinterpret_cast<unsigned char *>(p16) + ((size_t)p.R * P_PITCH * 2 + 127) / 128 * 128);
+    __half * p16 = reinterpret_cast<__half *>(smem);
+    __half * qs = reinterpret_cast<__half *>(smem + ((size_t)p.R * S_PITCH * 4 + 127) / 128 * 128);
     __half * vs = qs + 16 * Q_PITCH;
 
     pdl_launch();
     // ---- before the wait: positions, and L2 hints for the cached rows (earlier steps wrote them)
     int t0, n_rows, head0, hk;
     if (p.chunk) {
-        head0 = blockIdx.x; hk = head0 / group; t0 = blockIdx.y * 16; n_rows = min(16, p.T - t0);
+        head0 = blockIdx.x; hk = head0 / group; t0 = (gridDim.y - 1 - blockIdx.y) * 16; n_rows = min(16, p.T - t0);
     } else {
         const int ng = (group + 15) / 16, gi = blockIdx.x % ng;
         hk = blockIdx.x / ng; head0 = hk * group + gi * 16; t0 = blockIdx.y; n_rows = min(16, group - gi * 16);
@@ -207,8 +208,14 @@ __global__ void __launch_bounds__(AM_THREADS, UN == 2 ? 4 : HC == 2 ? 3 : 2) k_a
             part += (double)e;
         }
         const float inv = (float)(1.0 / warp_sum_d(part));
-#pragma unroll 4
-        for (int j = lane; j < k_end; j += 32) p16[r * P_PITCH + j] = __float2half_rn(j <= last ? row[j] * inv : 0.f);
+        for (int j0 = lane; j0 < k_end + lane; j0 += 128) {            // (a probability takes the place of a score of its own step or an earlier one)
+            float e[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) e[u] = j0 + 32 * u <= last ? row[j0 + 32 * u] * inv : 0.f;
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < 4; u++) if (j0 + 32 * u < k_end) p16[r * P_PITCH + j0 + 32 * u] = __float2half_rn(e[u]);
+        }
     }
 
     // ---- values
@@ -243,8 +250,9 @@ __global__ void __launch_bounds__(AM_THREADS, UN == 2 ? 4 : HC == 2 ? 3 : 2) k_a
         }
         if (tile + 2 < n_vt) { __syncthreads(); issue_v(tile + 2); }
     }
-    // ---- the output rows (scores are dead: their place takes the sums of each position share)
-    float * o = sc;
+    // ---- the output rows (the values are dead: their place takes the sums of each position share)
+    __syncthreads();
+    float * o = reinterpret_cast<float *>(vs);
 #pragma unroll
     for (int cg = 0; cg < NCG; cg++)
 #pragma unroll
@@ -320,16 +328,16 @@ static constexpr size_t AM_SMEM_MAX = 220 * 1024;
 // rows and positions that shared memory holds, and its size
 static size_t attn_mm_smem(const AttnArgs & a, int * P, int * R) {
     const int hd = a.head_dim, group = a.n_head / a.n_head_kv;
-    const int nwc = hd / 16 < AM_WARPS ? hd / 16 : AM_WARPS, kspl = AM_WARPS / nwc;
     *P = (a.n_ctx + 63) / 64 * 64;
     *R = a.store_mode != 0 || group > 16 ? 16 : group;
     auto up = [](size_t v) { return (v + 127) / 128 * 128; };
-    const size_t scores = (size_t)*R * (*P + 4) * 4, sums = (size_t)kspl * 16 * hd * 4;
-    return up(scores > sums ? scores : sums) + up((size_t)*R * (*P + 8) * 2) + (size_t)16 * (hd + 8) * 2 + (size_t)2 * AM_VT * (hd + 8) * 2;
+    return up((size_t)*R * (*P + 4) * 4) + (size_t)16 * (hd + 8) * 2 + (size_t)2 * AM_VT * (hd + 8) * 2;
 }
 
-// Several tokens and head_dim 64 or 128 whose scores fit (16 rows: contexts of up to about 1900 positions); the others keep one
-// CTA per head and token.  So do steps of several sequences whose CTAs per head and token fit the SMs at once: nothing is gained there
+// Several tokens and head_dim 64 or 128 whose scores fit; the others keep one CTA per head and token.  For prompt chunks of 32 tokens and more
+// that is contexts of up to 2880 positions (256 tokens at the end of 2048, 32 heads of 128, 4 layers 4952 | 1276 us, of 2560 5611 | 1366); for
+// the rest the line stays where scores and probabilities apart would fit (16 rows: about 1900 positions; 16 tokens at the end of 2304, 16 heads
+// of 64, 314 | 346, of 2560, 32 heads of 128 699 | 538).  So do steps of several sequences whose CTAs per head and token fit the SMs at once: nothing is gained there
 // by reading a KV head once for all of its query heads, and a CTA of k_attention_row has more rows in flight.  us in k_attention_row | here,
 // 8 sequences of 8 heads of 64: 200 positions 5.5 | 7.1, 1000 8.5 | 16.3, 3500 19.8 | 44.3; 4 of 32 heads of 128, 1000 positions
 // 13.1 | 20.8.  With more CTAs than SMs: 32 sequences of 8 heads of 64 over 2 KV heads, 200 positions
@@ -342,7 +350,9 @@ bool attention_mm_takes(const AttnArgs & a) {
     int P, R;
     if (a.store_mode == 0 && (int64_t)a.T * a.n_head <= sm_count()) return false;
     if (a.store_mode == 0 && a.n_head / a.n_head_kv * a.head_dim <= 128 && a.n_ctx > 64 * a.head_dim) return false;
-    return a.T >= 2 && (a.head_dim == 64 || a.head_dim == 128) && a.n_ctx > 0 && attn_mm_smem(a, &P, &R) <= AM_SMEM_MAX;
+    if (!(a.T >= 2 && (a.head_dim == 64 || a.head_dim == 128) && a.n_ctx > 0)) return false;
+    const size_t smem = attn_mm_smem(a, &P, &R);
+    return smem + (a.store_mode != 0 && a.T >= 32 ? 0 : (size_t)R * (P + 8) * 2) <= AM_SMEM_MAX;
 }
 
 // UN = 4 takes 126 registers with head_dim 128, two CTAs per SM.  Where the grid and shared memory give an SM more than two, half
@@ -372,9 +382,12 @@ int launch_attention_mm(const AttnArgs & a, cudaStream_t st) {
     p.out = a.out; p.out_act = a.out_act; p.out_act_type = a.out_act_type;
     p.chunk = a.store_mode != 0;
     p.stored = p.chunk && a.T > AM_OWN_STORE;
-    const size_t smem = attn_mm_smem(a, &p.P, &p.R);
+    size_t smem = attn_mm_smem(a, &p.P, &p.R);
     if (p.stored) PI_CUDA(launch_k(k_kv_store, dim3((unsigned)((a.n_head_kv * a.head_dim / 2 + 255) / 256), a.T), dim3(256), 0, st, a.pdl, p, a.head_dim));
     const dim3 grid = p.chunk ? dim3(a.n_head, (a.T + 15) / 16) : dim3(a.n_head_kv * ((a.n_head / a.n_head_kv + 15) / 16), a.T);
+    // CTAs that can have an SM each do: placed early, while the kernel before this one holds other SMs, two would share one (eight sequences of the
+    // 70B shape, three layers 536 -> 525 us a step; 32 tokens at position 991, 32 heads of 128, four layers 533 -> 486).
+    if ((int64_t)grid.x * grid.y <= sm_count() && smem < AM_SMEM_MAX / 2 + 8192) smem = AM_SMEM_MAX / 2 + 8192;
     if (a.head_dim == 64) return attn_mm_go<2, 4>(p, grid, smem, a.pdl, st);
     return smem <= AM_SMEM_MAX / 3 && (int64_t)grid.x * grid.y > 2 * sm_count() ? attn_mm_go<4, 2>(p, grid, smem, a.pdl, st) : attn_mm_go<4, 4>(p, grid, smem, a.pdl, st);
 }
