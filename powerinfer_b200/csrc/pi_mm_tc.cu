@@ -50,7 +50,8 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
     float * const epi = reinterpret_cast<float *>(smem_raw + (ring - smem_u32(smem_raw)) + p.ring);
     int * const rows = reinterpret_cast<int *>(epi + MT_OUT / 32 * (MT_EPI / 4));      // rows of this CTA (sparse only)
-    const int G = gridDim.x / p.n_tt, cta = blockIdx.x / p.n_tt, tok_first = (int)(blockIdx.x % p.n_tt) * 128;
+    const int G = gridDim.x / p.n_tt, cta = blockIdx.x / p.n_tt, tok_first = (int)(blockIdx.x % p.n_tt) * p.x_rows;
+    const int tok_end = p.n_tt > 1 ? min(p.T, tok_first + p.x_rows) : p.T;
     if (tid < 8) s_any[tid] = 0u;
     if (tid < MT_SMAX) { mbar_init(s_full + tid, SPARSE ? 1 + MT_OUT / 32 : 1); mbar_init(s_empty + tid, 1); }
     if (tid < 2) { mbar_init(s_dfull + tid, 1); mbar_init(s_dempty + tid, MT_OUT / 32); }
@@ -170,7 +171,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
             constexpr int PER = GATED ? 8 : 16;                       // items of 16 columns
             for (int t = 0; t < p.nt; t++) {
                 const int tok0 = tok_first + t * 128 + quarter * 32;
-                if (tok0 >= p.T) break;
+                if (tok0 >= tok_end) break;
                 for (int c = third * 16; c < N; c += 48) {
                     const int k0 = GATED ? c / 2 : c;
                     if (k0 >= n_tile) break;
@@ -195,7 +196,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
 #pragma unroll
                         for (int u = 0; u < PER; u++) {
                             const int tok = tok0 + u * (32 / PER) + lane / PER;
-                            l[u] = SPARSE && tok < p.T ? p.idx[(size_t)tok * p.idx_stride + gid] : 0.f;
+                            l[u] = SPARSE && tok < tok_end ? p.idx[(size_t)tok * p.idx_stride + gid] : 0.f;
                         }
 #pragma unroll
                         for (int u = 0; u < PER; u++) {
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
                             float o = off ? 0.f : mine[kl * 34 + tw];
                             if (p.bias && !(off && p.coef)) o += bias;                // (a coefficient of an inactive token is 0 whatever the bias)
                             if (p.relu) o = fmaxf(o, 0.f);
-                            if (tok < p.T) {
+                            if (tok < tok_end) {
                                 if (p.dst)   p.dst[(size_t)tok * p.dst_stride + gid] = o;
                                 if (p.dst16) p.dst16[(size_t)tok * p.dst_stride + gid] = __float2half_rn(o);
                                 if (p.coef)  p.coef[(size_t)tok * p.coef_stride + item] = __float2half_rn(o);
@@ -235,11 +236,13 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
         if (!SPARSE) {
             for (int tile = 0; tile < n_tiles; tile++) write(tile);
         } else {
-            // ---- gathered rows: 8 threads a row, 48 rows a pass.  A thread requests 8 pieces at once, of U slices, while the 8 before are
-            // stored: 48 KB on their way per SM whatever the number of rows (with 96 KB slower: 8600 of 11008 rows of 8 KB, gated, 77 tokens
-            // 71 against 60 us).
-            auto gather = [&](auto slices) {
-                constexpr int U = decltype(slices)::value, PJ = 8 / U, SETS = 2;
+            // ---- gathered rows: 8 threads a row, 48 rows a pass, as many passes as the tile has rows for.  A thread requests 6 .. 9 pieces at once, of U
+            // slices, while those before are stored: 36 .. 54 KB on their way per SM (with 96 KB slower: 8600 of 11008 rows of 8 KB, gated, 77 tokens
+            // 71 against 60 us).  Nothing is requested for a column of no row: with two, four or eight passes, and some row in the place of
+            // those beyond the tile, every CTA asked the L2 for the same lines, up to half of its requests (us, before | here, 77, 128 and 256
+            // tokens: idx, 72 % of 4096 x 4096 33.9 | 26.9, 41.9 | 32.5, 50.4 | 43.6; the FFN of 36 % of 11008 x 4096 76.9 | 71.0, 85.0 | 78.1, 123.1 | 117.9).
+            auto gather = [&](auto slices, auto passes) {
+                constexpr int U = decltype(slices)::value, PJ = decltype(passes)::value, SETS = 2;
                 const int piece = pt & 7, r0 = pt >> 3;
                 const uint32_t to = (uint32_t)(r0 * 128 + (piece ^ (r0 & 7)) * 16);       // (48 is a multiple of 8: the same place in every pass)
                 const int n_steps = (n_stages * su + U - 1) / U;
@@ -249,21 +252,21 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
                 for (int tile = 0; tile < n_tiles && ok; tile++) {
                     const uint8_t * src[PJ];
 #pragma unroll
-                    for (int j = 0; j < PJ; j++) {                    // (columns of no row: any row)
+                    for (int j = 0; j < PJ; j++) {
                         const int r = r0 + j * MT_PASS, k = GATED ? r >> 1 : r, item = tile * items + k;
-                        src[j] = (GATED && (r & 1) ? p.W2 : p.W) + (k < items && lo + item < hi ? (size_t)rows[item] * p.row_bytes : 0) + piece * 16;
+                        src[j] = k < items && lo + item < hi ? (GATED && (r & 1) ? p.W2 : p.W) + (size_t)rows[item] * p.row_bytes + piece * 16 : nullptr;
                     }
-                    uint4 v[SETS][8];
-                    auto load = [&](int step, uint4 (&b)[8]) {
+                    uint4 v[SETS][U * PJ];
+                    auto load = [&](int step, uint4 (&b)[U * PJ]) {
                         if (step >= n_steps) return;
                         const int x = step * U * 64 + piece * 8;      // (a row's end: zeros)
 #pragma unroll
                         for (int u = 0; u < U; u++)
 #pragma unroll
-                            for (int j = 0; j < PJ; j++) b[u * PJ + j] = x + u * 64 < p.ncols ? ldg_stream(src[j] + (size_t)(step * U + u) * 128) : make_uint4(0u, 0u, 0u, 0u);
+                            for (int j = 0; j < PJ; j++) b[u * PJ + j] = src[j] && x + u * 64 < p.ncols ? ldg_stream(src[j] + (size_t)(step * U + u) * 128) : make_uint4(0u, 0u, 0u, 0u);
                     };
                     int part = 0;                                     // slice of the stage
-                    auto store = [&](int step, const uint4 (&b)[8]) {
+                    auto store = [&](int step, const uint4 (&b)[U * PJ]) {
                         if (step >= n_steps) return;
 #pragma unroll
                         for (int u = 0; u < U; u++) {
@@ -295,9 +298,11 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
                     write(tile);
                 }
             };
-            if (N <= 2 * MT_PASS)      gather(std::integral_constant<int, 4>());
-            else if (N <= 4 * MT_PASS) gather(std::integral_constant<int, 2>());
-            else                       gather(std::integral_constant<int, 1>());
+            if (N <= MT_PASS)          gather(std::integral_constant<int, 8>(), std::integral_constant<int, 1>());
+            else if (N <= 2 * MT_PASS) gather(std::integral_constant<int, 4>(), std::integral_constant<int, 2>());
+            else if (N <= 3 * MT_PASS) gather(std::integral_constant<int, 3>(), std::integral_constant<int, 3>());
+            else if (N <= 4 * MT_PASS) gather(std::integral_constant<int, 2>(), std::integral_constant<int, 4>());
+            else                       gather(std::integral_constant<int, 1>(), std::integral_constant<int, 6>());
         }
         tc_fence_before();
     }
@@ -345,7 +350,10 @@ int launch_mm_tc(const GemvArgs & a, cudaStream_t st) {
         // 4096 x 4096 33 | 24, 12288 x 4096 42 | 38, 16000 x 4096 47 | 46).  Gathered rows go through the CTA's registers, so that doing it twice
         // costs more (idx, 72 % of 2048 x 2048 40 | 35, 4096 x 4096 64 | 50, 11008 x 1024 54 | 57).  Masks are the union over ALL tokens.
         p.n_tt = p.T > 128 && !a.masks_out && a.nrows * (a.W2 ? 2 : 1) < (a.masks ? 6000 : 128 * (int64_t)sm_count()) ? 2 : 1;
-        p.nt = p.n_tt > 1 ? 1 : (p.T + 127) / 128; p.x_rows = p.T > 128 ? 128 : (p.T + 7) / 8 * 8;
+        p.x_rows = ((p.T + p.n_tt - 1) / p.n_tt + 7) / 8 * 8;
+        if (p.x_rows > 128) p.x_rows = 128;
+        p.nt = p.n_tt > 1 ? 1 : (p.T + 127) / 128;
+        if (p.n_tt > 1) p.n_tt = (p.T + p.x_rows - 1) / p.x_rows;
         int rc = tensor_map(&p.m_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a.x.h16 + (size_t)t0 * a.ncols, p.ncols, p.T, (int64_t)p.ncols * 2, 64, p.x_rows, CU_TENSOR_MAP_SWIZZLE_128B);
         if (rc != PI_OK) return rc;
         p.masks = a.masks; p.bucket = a.bucket; p.list = a.list_out; p.count = a.count_out; p.rows_total = t0 == 0 ? a.rows_total : nullptr;
