@@ -345,11 +345,18 @@ int launch_mm_tc(const GemvArgs & a, cudaStream_t st) {
         p.W = (const uint8_t *)a.W; p.W2 = (const uint8_t *)a.W2; p.row_bytes = a.ncols * 2;
         p.nrows = (int)a.nrows; p.ncols = (int)a.ncols;
         p.T = a.T - t0 < 256 ? a.T - t0 : 256;
-        // More than 128 tokens: a CTA has all of them and its share r of the rows, or every other CTA has half of them and 2 r rows.  What it
-        // brings in is 256 + r or 128 + 2 r rows of K: half the tokens below 128 dense rows a CTA (us, 256 tokens, all | half: 1024 x 8192 54 | 37,
-        // 4096 x 4096 33 | 24, 12288 x 4096 42 | 38, 16000 x 4096 47 | 46).  Gathered rows go through the CTA's registers, so that doing it twice
-        // costs more (idx, 72 % of 2048 x 2048 40 | 35, 4096 x 4096 64 | 50, 11008 x 1024 54 | 57).  Masks are the union over ALL tokens.
-        p.n_tt = p.T > 128 && !a.masks_out && a.nrows * (a.W2 ? 2 : 1) < (a.masks ? 6000 : 128 * (int64_t)sm_count()) ? 2 : 1;
+        // Dense rows: all CTAs have all of the tokens, or groups of n neighbours have a part of them each (64 at least) and n times the rows.  What a
+        // CTA brings in decides: its tokens, and its r rows one and a half times (us, 256 tokens, n = 1 | 2 | 3 | 4: 1024 x 8192 54 | 38 | 31 | 31, 2048 x 2048
+        // 20.1 | 14.7 | 15.0 | 14.5, 4096 x 4096 32.7 | 24.3 | 24.8 | 26.2, 12288 x 4096 41.5 | 37.5 | 45.7 | 55.8; 128 tokens, n = 1 | 2: 1024 x 8192
+        // 35.2 | 28.5, 4096 x 4096 22.3 | 20.8, 12288 x 4096 29.9 | 35.1).  Two token tiles in one CTA cost their products, too: 44 more.
+        // Gathered rows go through the CTA's registers, so that doing it twice costs more (idx, 72 % of 2048 x 2048 40 | 35, 4096 x 4096 64 | 50, 11008 x
+        // 1024 54 | 57).  Masks are the union over ALL tokens.
+        p.n_tt = 1;
+        if (a.masks) p.n_tt = p.T > 128 && a.nrows * (a.W2 ? 2 : 1) < 6000 ? 2 : 1;
+        else if (!a.masks_out) {
+            auto brought = [&](int n) { return (n == 1 && p.T > 128 ? 300 : ((p.T + n - 1) / n + 7) / 8 * 8) + 3 * a.nrows * n / (2 * sm_count()); };
+            for (int n = 2; n <= p.T / 64; n++) if (brought(n) < brought(p.n_tt)) p.n_tt = n;
+        }
         p.x_rows = ((p.T + p.n_tt - 1) / p.n_tt + 7) / 8 * 8;
         if (p.x_rows > 128) p.x_rows = 128;
         p.nt = p.n_tt > 1 ? 1 : (p.T + 127) / 128;
