@@ -11,10 +11,11 @@
 // one launch of 8600 of 11008 gated rows of 8 KB: 49 us; rows by cp.async, 50 clocks per warp and copy, 70 in the kernel before this one; by
 // tile::gather4, 90 clocks per four rows of 128 bytes, 94).
 //
-// us, mma.sync | here, 77, 128 and 256 tokens: 12288 x 4096 38.7 | 26.0, 51.5 | 30.2, 74.4 | 41.8; 1024 x 4096 30.2 | 17.6, 38.1 | 21.1, 42.9 | 30.8;
+// us, mma.sync | here, 77, 128 and 256 tokens: 12288 x 4096 38.7 | 26.0, 51.5 | 30.2, 74.4 | 37.6; 1024 x 4096 30.2 | 11.5, 38.1 | 11.7, 42.9 | 12.7;
 // the FFN of 72 % of 11008 x 4096 119 | 95, 175 | 120, 290 | 185 (half of it the down projection).
 #include "pi_tc.cuh"
 
+#include <atomic>
 #include <type_traits>
 
 namespace pi {
@@ -23,6 +24,7 @@ static constexpr int MT_THREADS = 512, MT_OUT = 384;    // threads 128 .. 511 co
 static constexpr int MT_EPI = 16 * 34 * 4;               // a warp's transposition of 16 rows x 32 tokens
 static constexpr int MT_SMAX = 8;                        // stages at most
 static constexpr int MT_SMEM_MAX = 226 * 1024;
+static constexpr int MT_RANKS = 4;                       // CTAs that share the columns of a range of rows (SPLIT)
 static constexpr int MT_PASS = MT_OUT / 8;              // rows of a pass of the copying threads
 
 struct alignas(64) MtP {
@@ -38,7 +40,7 @@ struct alignas(64) MtP {
     unsigned int * status;
 };
 
-template <bool SPARSE, bool GATED>
+template <bool SPARSE, bool GATED, bool SPLIT>
 __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__ MtP p) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ int s_warp[MT_THREADS / 32];
@@ -50,7 +52,9 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
     float * const epi = reinterpret_cast<float *>(smem_raw + (ring - smem_u32(smem_raw)) + p.ring);
     int * const rows = reinterpret_cast<int *>(epi + MT_OUT / 32 * (MT_EPI / 4));      // rows of this CTA (sparse only)
-    const int G = gridDim.x / p.n_tt, cta = blockIdx.x / p.n_tt, tok_first = (int)(blockIdx.x % p.n_tt) * p.x_rows;
+    constexpr int ks = SPLIT ? MT_RANKS : 1;
+    const int rank = SPLIT ? (int)(blockIdx.x % ks) : 0, block = blockIdx.x / ks;       // ranges of columns, this CTA's
+    const int G = gridDim.x / (p.n_tt * ks), cta = block / p.n_tt, tok_first = (int)(block % p.n_tt) * p.x_rows;
     const int tok_end = p.n_tt > 1 ? min(p.T, tok_first + p.x_rows) : p.T;
     if (tid < 8) s_any[tid] = 0u;
     if (tid < MT_SMAX) { mbar_init(s_full + tid, SPARSE ? 1 + MT_OUT / 32 : 1); mbar_init(s_empty + tid, 1); }
@@ -62,6 +66,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
+    if (SPLIT) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // (waited for before the first store into a neighbour's memory)
     pdl_launch();
     auto wait = [&](uint64_t * bar, unsigned parity) -> bool {        // warp-uniform; false: the wait ran out, here or elsewhere
         bool ok = false;
@@ -95,7 +100,8 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
     const int n_tiles = SPARSE ? (n_cols + 255) / 256 : (n_cols + p.per_tile - 1) / p.per_tile;
     const int N = SPARSE ? (n_tiles ? ((n_cols + n_tiles - 1) / n_tiles + 15) / 16 * 16 : 16) : (p.per_tile + 15) / 16 * 16;
     const int items = GATED ? N / 2 : SPARSE ? N : p.per_tile;        // of a tile
-    const int n_slices = (p.ncols + 63) / 64;
+    const int all_slices = (p.ncols + 63) / 64, slice0 = all_slices * rank / ks;
+    const int n_slices = all_slices * (rank + 1) / ks - slice0;
     const int n_bufs = p.nt * N <= 256 ? 2 : 1;
     // A stage is `su` slices of 64 columns, as many as leave three stages: a hand-over costs each of the three parties 200 .. 400 clocks,
     // a slice of few rows less (1024 x 4096, 77 tokens: one slice a stage 23.9 us, four 17.0).
@@ -114,8 +120,9 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
                 mbar_expect_tx(s_full + slot, (unsigned)(su * (p.nt * p.x_rows + (SPARSE ? 0 : p.per_tile)) * 128));
                 for (int u = 0; u < su; u++) {
                     const uint32_t base = ring + (uint32_t)slot * stage + (uint32_t)u * slice_bytes;
-                    for (int t = 0; t < p.nt; t++) tma_tile(base + t * 16384, &p.m_x, (slice + u) * 64, tok_first + t * 128, s_full + slot);
-                    if (!SPARSE) tma_tile(base + w_off, &p.m_w, (slice + u) * 64, row, s_full + slot);
+                    const int col = (SPLIT && slice + u >= n_slices ? all_slices : slice0 + slice + u) * 64;       // (behind the last slice: zeros)
+                    for (int t = 0; t < p.nt; t++) tma_tile(base + t * 16384, &p.m_x, col, tok_first + t * 128, s_full + slot);
+                    if (!SPARSE) tma_tile(base + w_off, &p.m_w, col, row, s_full + slot);
                 }
             }
             __syncwarp();
@@ -160,23 +167,36 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
     } else if (warp >= 4) {
         const int pt = tid - (MT_THREADS - MT_OUT), quarter = warp & 3, third = (warp >> 2) - 1;
         float * const mine = epi + (warp - 4) * (MT_EPI / 4);
+        // (SPLIT) sums of 16 rows x 32 tokens: [rank they come from][group of 16 rows of this CTA][quarter of the tokens][row][token]
+        float * const red = epi + MT_OUT / 32 * (MT_EPI / 4);
+        const int quarters = (p.x_rows + 31) / 32, red_rank = (N / 16 + ks - 1) / ks * quarters * 512;
         int buf = 0;
         unsigned dphase = 0u;
         bool ok = true;
         // ---- the results of a tile
         auto write = [&](int tile) {
-            ok = wait(s_dfull + buf, dphase) && ok;
+            if (!SPLIT) ok = wait(s_dfull + buf, dphase) && ok;
             tc_fence_after();
             const int n_tile = min(items, hi - lo - tile * items);
             constexpr int PER = GATED ? 8 : 16;                       // items of 16 columns
             for (int t = 0; t < p.nt; t++) {
                 const int tok0 = tok_first + t * 128 + quarter * 32;
                 if (tok0 >= tok_end) break;
-                for (int c = third * 16; c < N; c += 48) {
+                for (int c = (SPLIT ? third * ks + rank : third) * 16; c < N; c += 48 * ks) {
                     const int k0 = GATED ? c / 2 : c;
                     if (k0 >= n_tile) break;
                     float v[16];
-                    tc_ld16(v, tmem + (uint32_t)(quarter * 32 << 16) + (uint32_t)(buf * 256 + t * N + c));
+                    if (SPLIT) {                                      // the cluster's sums, in the order of their columns
+                        const float * part = red + ((c / 16 / ks) * quarters + quarter) * 512 + lane;
+#pragma unroll
+                        for (int j = 0; j < 16; j++) v[j] = part[j * 32];
+#pragma unroll
+                        for (int k = 1; k < ks; k++) {
+                            part += red_rank;
+#pragma unroll
+                            for (int j = 0; j < 16; j++) v[j] += part[j * 32];
+                        }
+                    } else tc_ld16(v, tmem + (uint32_t)(quarter * 32 << 16) + (uint32_t)(buf * 256 + t * N + c));
                     if (GATED) {
 #pragma unroll
                         for (int j = 0; j < 8; j++) mine[j * 34 + lane] = fmaxf(v[2 * j + 1], 0.f) * v[2 * j];
@@ -233,7 +253,25 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
                 asm volatile("bar.sync 1, 384;" ::: "memory");
             }
         };
-        if (!SPARSE) {
+        if (SPLIT) {
+            // ---- a tile's sums go to the CTA of the cluster that writes these rows
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+            if (n_tiles) {
+                ok = wait(s_dfull, 0u);
+                tc_fence_after();
+                for (int c = third; c < N / 16 && quarter < quarters; c += 3) {
+                    float v[16];
+                    tc_ld16(v, tmem + (uint32_t)(quarter * 32 << 16) + (uint32_t)(c * 16));
+                    uint32_t to;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(smem_u32(red + rank * red_rank + ((c / ks) * quarters + quarter) * 512 + lane)), "r"(c % ks));
+#pragma unroll
+                    for (int j = 0; j < 16; j++) asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(to + (uint32_t)j * 128u), "f"(v[j]) : "memory");
+                }
+            }
+            __syncwarp();
+            asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+            if (n_tiles && ok) write(0);
+        } else if (!SPARSE) {
             for (int tile = 0; tile < n_tiles; tile++) write(tile);
         } else {
             // ---- gathered rows: 8 threads a row, 48 rows a pass, as many passes as the tile has rows for.  A thread requests 6 .. 9 pieces at once, of U
@@ -306,15 +344,48 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
         }
         tc_fence_before();
     }
+    if (SPLIT && warp < 4) {                                          // (the two barriers of the cluster, for the warps that write nothing)
+        __syncwarp();
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
     __syncthreads();
     tc_fence_after();
     if (warp == 0) tc_dealloc(tmem, 512);
 }
 
 // ---------------------------------------------------------------------------------------------- launch
-template <bool SPARSE, bool GATED>
+static cudaLaunchConfig_t mt_config(int clusters, cudaLaunchAttribute * attr, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(clusters * MT_RANKS); cfg.blockDim = dim3(MT_THREADS); cfg.dynamicSmemBytes = MT_SMEM_MAX; cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = MT_RANKS; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    return cfg;
+}
+
+// clusters that this device keeps resident at once (B200: 33)
+static int mt_clusters() {
+    static std::atomic<int> known[16];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return 0;
+    if ((n = known[dev].load()) > 0) return n;
+    auto kern = k_mm_tc<false, false, true>;
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg = mt_config(1, attr, nullptr);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MT_SMEM_MAX) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    known[dev].store(n);
+    return n;
+}
+
+template <bool SPARSE, bool GATED, bool SPLIT>
 static int mt_go(MtP & p, bool pdl, cudaStream_t st) {
-    const int G = (int)imin64(sm_count() / p.n_tt, (p.nrows + 7) / 8);
+    const int G = SPLIT ? mt_clusters() / p.n_tt : (int)imin64(sm_count() / p.n_tt, (p.nrows + 7) / 8);
     const int list = SPARSE ? ((p.nrows + G - 1) / G + 1) * 4 : 0;    // bytes
     p.ring = (MT_SMEM_MAX - 1024 - MT_OUT / 32 * MT_EPI - list) / 1024 * 1024;
     if (p.ring < 2 * (p.nt * 16384 + 256 * 128)) return PI_ERR_UNSUPPORTED;        // two stages of the largest kind (more than MM_MAX_ROWS rows)
@@ -326,15 +397,20 @@ static int mt_go(MtP & p, bool pdl, cudaStream_t st) {
         if (p.per_tile > 256) p.per_tile = 256;
         if ((rc = tensor_map(&p.m_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, p.W, p.ncols, p.nrows, p.row_bytes, 64, p.per_tile, CU_TENSOR_MAP_SWIZZLE_128B)) != PI_OK) return rc;
     }
+    if (SPLIT) p.ring -= ((p.per_tile + 15) / 16 + MT_RANKS) * ((p.x_rows + 31) / 32) * 2048 / 1024 * 1024;      // what comes from the cluster
     static bool attr_done[16] = {false};
     int dev = 0;
     PI_CUDA(cudaGetDevice(&dev));
-    auto kern = k_mm_tc<SPARSE, GATED>;
+    auto kern = k_mm_tc<SPARSE, GATED, SPLIT>;
     if (dev >= 0 && dev < 16 && !attr_done[dev]) {
         PI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MT_SMEM_MAX));
         attr_done[dev] = true;
     }
-    PI_CUDA(launch_k(kern, dim3(G * p.n_tt), dim3(MT_THREADS), (size_t)MT_SMEM_MAX, st, pdl, p));
+    if (!SPLIT) { PI_CUDA(launch_k(kern, dim3(G * p.n_tt), dim3(MT_THREADS), (size_t)MT_SMEM_MAX, st, pdl, p)); return PI_OK; }
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg = mt_config(G * p.n_tt, attr, st);
+    cfg.numAttrs = pdl ? 2 : 1;
+    PI_CUDA(cudaLaunchKernelEx(&cfg, kern, (const MtP &)p));
     return PI_OK;
 }
 
@@ -346,16 +422,26 @@ int launch_mm_tc(const GemvArgs & a, cudaStream_t st) {
         p.nrows = (int)a.nrows; p.ncols = (int)a.ncols;
         p.T = a.T - t0 < 256 ? a.T - t0 : 256;
         // Dense rows: all CTAs have all of the tokens, or groups of n neighbours have a part of them each (64 at least) and n times the rows.  What a
-        // CTA brings in decides: its tokens, and its r rows one and a half times (us, 256 tokens, n = 1 | 2 | 3 | 4: 1024 x 8192 54 | 38 | 31 | 31, 2048 x 2048
-        // 20.1 | 14.7 | 15.0 | 14.5, 4096 x 4096 32.7 | 24.3 | 24.8 | 26.2, 12288 x 4096 41.5 | 37.5 | 45.7 | 55.8; 128 tokens, n = 1 | 2: 1024 x 8192
-        // 35.2 | 28.5, 4096 x 4096 22.3 | 20.8, 12288 x 4096 29.9 | 35.1).  Two token tiles in one CTA cost their products, too: 44 more.
+        // CTA brings in decides: its tokens, and its r rows one and a half times (us, 256 tokens, n = 1 | 2 | 3 | 4: 4096 x 4096 32.7 | 24.3 | 24.8 | 26.2,
+        // 12288 x 4096 41.5 | 37.5 | 45.7 | 55.8; 128 tokens, n = 1 | 2: 8192 x 8192 38.0 | 37.6, 12288 x 4096 29.9 | 35.1).  Two token tiles in one
+        // CTA cost their products, too: 44 more.
+        // Few rows leave a CTA the activations and a chain of column slices, 0.2 us each whatever they hold: four CTAs of a cluster then take a
+        // quarter of the columns each, of four times the rows, up to 160 in a CTA (so that a part of the tokens still is 64 or more), and add up their
+        // sums through each other's shared memory.  us, in a graph, alone | in fours, 77, 128, 256 tokens: 1024 x 4096 16.5 | 11.5, 16.6 | 11.7, 17.2 |
+        // 12.7; 1024 x 8192 26.8 | 15.0, 27.1 | 15.2, 29.1 | 17.8; 2048 x 2048 11.3 | 10.1, 11.6 | 11.0, 13.3 | 12.3; 4096 x 4096 16.9 | 14.4, 18.4 | 14.8; 5120 x
+        // 5120 19.8 | 16.5, 25.5 | 19.4; no gain below 2048 columns (2048 x 1024 8.7 | 9.1).  In pairs 13.0 for the first, 8192 x 8192 36.2 | 35.3, 38.0 | 39.4.
         // Gathered rows go through the CTA's registers, so that doing it twice costs more (idx, 72 % of 2048 x 2048 40 | 35, 4096 x 4096 64 | 50, 11008 x
         // 1024 54 | 57).  Masks are the union over ALL tokens.
         p.n_tt = 1;
+        bool split = false;
         if (a.masks) p.n_tt = p.T > 128 && a.nrows * (a.W2 ? 2 : 1) < 6000 ? 2 : 1;
         else if (!a.masks_out) {
+            for (int n = p.T > 128 ? p.T / 64 : 1; n >= (p.T + 127) / 128 && a.ncols >= 2048 && !split; n--) {
+                const int G = mt_clusters() / n;
+                if (G > 0 && (a.nrows + G - 1) / G <= 160) { split = true; p.n_tt = n; }
+            }
             auto brought = [&](int n) { return (n == 1 && p.T > 128 ? 300 : ((p.T + n - 1) / n + 7) / 8 * 8) + 3 * a.nrows * n / (2 * sm_count()); };
-            for (int n = 2; n <= p.T / 64; n++) if (brought(n) < brought(p.n_tt)) p.n_tt = n;
+            for (int n = 2; n <= p.T / 64 && !split; n++) if (brought(n) < brought(p.n_tt)) p.n_tt = n;
         }
         p.x_rows = ((p.T + p.n_tt - 1) / p.n_tt + 7) / 8 * 8;
         if (p.x_rows > 128) p.x_rows = 128;
@@ -370,7 +456,7 @@ int launch_mm_tc(const GemvArgs & a, cudaStream_t st) {
         p.dst16 = a.dst16 ? a.dst16 + (size_t)t0 * a.dst_stride : nullptr; p.dst_stride = a.dst_stride;
         p.coef = a.coef ? a.coef + (size_t)t0 * a.coef_stride : nullptr; p.coef_stride = a.coef_stride;
         p.masks_out = a.masks_out; p.masks_threshold = a.masks_threshold; p.masks_or = t0 > 0; p.status = a.status;
-        rc = !p.masks ? mt_go<false, false>(p, a.pdl, st) : p.W2 ? mt_go<true, true>(p, a.pdl, st) : mt_go<true, false>(p, a.pdl, st);
+        rc = split ? mt_go<false, false, true>(p, a.pdl, st) : !p.masks ? mt_go<false, false, false>(p, a.pdl, st) : p.W2 ? mt_go<true, true, false>(p, a.pdl, st) : mt_go<true, false, false>(p, a.pdl, st);
         if (rc != PI_OK) return rc;
     }
     return PI_OK;
