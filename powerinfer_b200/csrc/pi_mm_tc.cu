@@ -8,11 +8,11 @@
 //
 // Warps: 0 brings activations and dense rows as TMA tiles, 1 issues the products, 4..15 write the results: a thread holds ONE token's rows
 // after tcgen05.ld, 16 columns at a time become lanes through shared memory.  Gathered rows these warps copy first, through registers (in
-// one launch of 8600 of 11008 gated rows of 8 KB: 49 us; rows by cp.async, 50 clocks per warp and copy, 70 in the kernel before this one; by
+// one launch of 8600 of 11008 gated rows of 8 KB: 47 us; rows by cp.async, 50 clocks per warp and copy, 70 in the kernel before this one; by
 // tile::gather4, 90 clocks per four rows of 128 bytes, 94).
 //
 // us, mma.sync | here, 77, 128 and 256 tokens: 12288 x 4096 38.7 | 26.0, 51.5 | 30.2, 74.4 | 37.6; 1024 x 4096 30.2 | 11.5, 38.1 | 11.7, 42.9 | 12.7;
-// the FFN of 72 % of 11008 x 4096 119 | 95, 175 | 120, 290 | 185 (half of it the down projection).
+// the FFN of 72 % of 11008 x 4096, down projection included, 119 | 71, 175 | 78, 290 | 118.
 #include "pi_tc.cuh"
 
 #include <atomic>
@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
             // slices, while those before are stored: 36 .. 54 KB on their way per SM (with 96 KB slower: 8600 of 11008 rows of 8 KB, gated, 77 tokens
             // 71 against 60 us).  Nothing is requested for a column of no row: with two, four or eight passes, and some row in the place of
             // those beyond the tile, every CTA asked the L2 for the same lines, up to half of its requests (us, before | here, 77, 128 and 256
-            // tokens: idx, 72 % of 4096 x 4096 33.9 | 26.9, 41.9 | 32.5, 50.4 | 43.6; the FFN of 36 % of 11008 x 4096 76.9 | 71.0, 85.0 | 78.1, 123.1 | 117.9).
+            // tokens: idx, 72 % of 4096 x 4096 33.9 | 26.9, 41.9 | 32.5, 50.4 | 43.6; the FFN of 72 % of 11008 x 4096 76.9 | 71.0, 85.0 | 78.1, 123.1 | 117.9).
             auto gather = [&](auto slices, auto passes) {
                 constexpr int U = decltype(slices)::value, PJ = decltype(passes)::value, SETS = 2;
                 const int piece = pt & 7, r0 = pt >> 3;
