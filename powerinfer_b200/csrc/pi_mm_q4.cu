@@ -1,16 +1,20 @@
-// Mat-mat over planar Q4_0 rows for MORE than 32 tokens (prompt chunks) on tcgen05: the operators, row selection and epilogue of pi_mm.cu.
+// Mat-mat over planar Q4_0 rows of many columns for MORE than 96 tokens (prompt chunks; the lines: mm_q4_takes) on tcgen05: the operators, row
+// selection and epilogue of pi_mm.cu.
 //
 // A term is (q - 8) * w * v * d: an integer and an FP16 scale of the row's block, an int8 and an FP16 scale of the token's block.  (q - 8) * w has 15
 // significant bits, v * d 18, and both are multiples of 2^-24: each is exactly the sum of TWO halves, its rounding and the rest.  Of
-// the four products of halves the two rests' (below 2^-24 of the term) is left out; the other three are exact in FP32.  So the scales ride on
-// the operands and the tensor cores do all of the work; as integers per block, scaled one by one, 2.7e9 sums of 256 tokens and a 70B-shape gather
-// take two FP32 instructions each (mma.sync 770 us, here 530; tcgen05 kind::i8 with that scaling 600 .. 700).
+// the four products of halves the two rests' (up to 2^-22 of the term, each rest up to 2^-11 of its value) is left out; the other three are exact
+// in FP32.  So the scales ride on the operands and the tensor cores do all of the work; as integers per block, scaled one by one, 2.7e9 sums of 256
+// tokens and a 70B-shape gather take two FP32 instructions each (mma.sync 770 us, here 530; tcgen05 kind::i8 with that scaling 600 .. 700).  The
+// fourth product costs 4 .. 5 % (10240 x 8192, 256 tokens 128 -> 134 us) for 2 % of the error.
 //
 // Precision: the tensor cores cut FP32 sums at every step, so a sum must not stay with them.  After 64 columns
 // it is drained and added with rounding in registers; the small products of a drain come first, so that only the four large
-// ones cut anything, half a unit each on the average, which the drain gives back (a factor of 1 + 2^-23).  Error against 64 bits, one FP32
-// chain of all blocks (pi_mm_wide.cu) | here: 8192 columns 2.8e-7 | 2.2e-7, 4096 2.1e-7 | 1.7e-7, 2048 1.4e-7 | 1.3e-7, 1024 1.1e-7 | 1.1e-7, 256
-// 0.5e-7 | 0.9e-7: shorter sums stay there (mm_q4_takes).
+// ones cut anything.  A sum that fits FP32 at every step (whole numbers at scales that are powers of two) is exact.  Error against 64 bits, one FP32
+// chain of all blocks (pi_mm_wide.cu) | here: random values in 8192 columns 2.86e-7 | 2.32e-7, 4096 2.03e-7 | 1.84e-7, 3072 1.77e-7 | 1.69e-7, 2816
+// 1.69e-7 | 1.65e-7, 2560 1.61e-7 | 1.61e-7, 2048 1.44e-7 | 1.53e-7: shorter sums stay there (mm_q4_takes).  A token with one feature that is not zero
+// 2.5e-8 | 5.5e-8 (what is left out, and a cut in the place of a rounding), with 16 6.8e-8 | 8.9e-8, with every 16th 2.6e-7 | 2.1e-7.  (A drain
+// times 1 + 2^-23, what cutting four times takes on the average, would halve the bias of random sums, 2.18e-7 in 8192 columns, and move exact ones.)
 // A row with a scale above 8188 may leave the halves' range, 65504: its sums are not finite then, and are made anew block by block.
 //
 // Tokens are the 128 lanes (M), rows the columns (N, steps of 16): every CTA takes its equal contiguous range of rows, in tiles of up to 160.
@@ -339,13 +343,12 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_mm_q4(const __grid_constant__
         bool ok = true, odd = false;                                  // (a sum that is not finite)
         const uint32_t mine_at = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(g * nc);
         const float2 * xd = reinterpret_cast<const float2 *>(p.x.d + (size_t)(tok0 + min(wq * 32 + lane, Tt - 1)) * p.nb);
-        const float UP = __uint_as_float(0x3F800001u);                // 1 + 2^-23: what cutting four times takes on the average
         auto tile_sums = [&](auto pieces) {                           // up to 32, 64 or 80 columns (what lies beyond nc is some other warp's, and dropped)
             constexpr int C = decltype(pieces)::value;
 #pragma unroll 1
             for (int st = 0; st < n_st; st++) {
-                float up = UP;
-                if (large) { const float2 d = xd[st]; up = __uint_as_float(((uint32_t)(127 + ts_down(d.x, d.y)) << 23) + 1u); }
+                float up = 1.f;
+                if (large) { const float2 d = xd[st]; up = __uint_as_float((uint32_t)(127 + ts_down(d.x, d.y)) << 23); }
                 ok = wait(s_dfull + db, dphase) && ok;
                 tc_fence_after();
                 const uint32_t src = mine_at + (uint32_t)db * TS_N;
@@ -473,15 +476,15 @@ static int ts_go(TsP & p, bool pdl, cudaStream_t st) {
     return PI_OK;
 }
 
-// Sums of fewer than 2048 columns are more precise in one chain (see above).  A CTA's time per 64 columns hardly depends on its rows and not at
+// Sums of fewer than 2816 columns are more precise in one chain, or no less (see above).  A CTA's time per 64 columns hardly depends on its rows and not at
 // all on its tokens up to 128 (hand-overs; the kernel with mma.sync takes steps of 64, 80, 96, 128, 192 and 256 tokens).  us, pi_mm_wide.cu | here:
 //   gathers (whose results it writes token by token, too)   97 tokens 4096 x 4096 60 | 52, 8192 x 8192 120 | 93; 256 tokens 88 | 67, 193 | 124
-//   dense, 193 .. 256 tokens   1000 x 2048 32.0 | 27.6, 4096 x 4096 61.6 | 54.2, 10240 x 8192 193 | 129
-//   dense, 129 .. 192          8192 x 2048 36.5 | 41.6, 8192 x 8192 114 | 114, 5120 x 5120 75 | 69: stays there
-//   dense, 97 .. 128           4096 x 4096 41.8 | 45.5, 8192 x 2048 30.0 | 31.9, 8192 x 8192 93 | 90, 10240 x 8192 114 | 103, 22016 x 2304 66 | 51
+//   dense, 193 .. 256 tokens   4096 x 4096 61.6 | 54.2, 10240 x 8192 193 | 129
+//   dense, 129 .. 192          8192 x 8192 114 | 114, 5120 x 5120 75 | 69: stays there
+//   dense, 97 .. 128           4096 x 4096 41.8 | 45.5, 8192 x 8192 93 | 90, 10240 x 8192 114 | 103
 //   fewer                      10240 x 8192, 77 tokens 83 | 102
 bool mm_q4_takes(const GemvArgs & a) {
-    if (a.ncols < 2048 || a.masks_out) return false;
+    if (a.ncols < 2816 || a.masks_out) return false;
     const int T = a.T > 256 ? 256 : a.T;
     return a.masks ? T > 96 : T > 192 || (T > 96 && T <= 128 && a.nrows >= 10000);
 }

@@ -87,8 +87,8 @@ def test_prompt_with_rounded_factors_of_256_columns():
 
 
 def close_q4(got, x, w, keep=None):
-    """Each product of halves is exact, the dropped ones lie below 2^-24 of their term, a drain of 64 terms is cut up to 12 times at 2^-23 of what it
-    holds then, and the drains are added in FP32: far within one unit of 2^-23 per 4 terms, which is asserted."""
+    """Each product of halves is exact, the dropped ones lie below 2^-22 of their term, a drain of 64 terms is cut up to 12 times at 2^-23 of what it
+    holds then, and the drains are added in FP32: within one unit of 2^-23 per 4 terms, which is asserted."""
     ref, mass = x @ w.T, x.abs() @ w.abs().T
     err = (got.double() - ref).abs()
     if keep is not None:
@@ -98,8 +98,9 @@ def close_q4(got, x, w, keep=None):
     assert err.norm() <= 4e-7 * ref.norm() + 1e-30
 
 
-# 9.. rows per CTA, tiles of 16, 96, 160 rows and several of them, sizes around every line of mm_q4_takes, a second launch
-@pytest.mark.parametrize("rows,cols,T", [(8, 2048, 193), (1000, 2304, 256), (2370, 4352, 200), (10000, 2048, 97), (24000, 2048, 128), (12100, 2048, 256), (5000, 2048, 261)])
+# 9.. rows per CTA, tiles of 16, 96, 160 rows and several of them, sizes around every line of mm_q4_takes (below 2816 columns: k_mm_wide), a second launch
+@pytest.mark.parametrize("rows,cols,T", [(8, 2048, 193), (1000, 2304, 256), (2370, 4352, 200), (10000, 2048, 97), (24000, 2048, 128), (12100, 2048, 256), (5000, 2048, 261),
+                                         (8, 2816, 193), (1000, 3072, 256), (10000, 2816, 97), (24000, 2816, 128), (12100, 3072, 256), (5000, 2816, 261), (5000, 2560, 200)])
 def test_q4_products(ops, rows, cols, T):
     gen = generator(rows + T)
     W, x = weight(ops, synth.Q4_0, rows, cols, gen), torch.randn(T, cols, device="cuda", generator=gen) * torch.exp(torch.randn(1, cols, device="cuda", generator=gen))
@@ -111,7 +112,8 @@ def test_q4_products(ops, rows, cols, T):
 
 
 @pytest.mark.parametrize("share", [0.0, 0.004, 0.6, 1.0])
-@pytest.mark.parametrize("rows,cols,T", [(640, 2048, 97), (5000, 2304, 128), (24000, 2048, 129), (3001, 4096, 256)])
+@pytest.mark.parametrize("rows,cols,T", [(640, 2048, 97), (5000, 2304, 128), (24000, 2048, 129), (3001, 4096, 256),
+                                         (640, 2816, 97), (5000, 3072, 128), (24000, 2816, 129)])
 def test_q4_gathers(ops, rows, cols, T, share):
     gen = generator(rows + T)
     up, gate = weight(ops, synth.Q4_0, rows, cols, gen), weight(ops, synth.Q4_0, rows, cols, gen)
@@ -159,3 +161,38 @@ def test_q4_rows_above_the_halves_range(ops):
     y = ops.ggml_axpy(down, torch.relu(got) * got, idx)
     assert y.isfinite().all() and torch.equal(ops.sparse_ffn(W, W, down, x, idx), y)
     assert ops.last_op_status() == 0
+
+
+def q4_of(ops, rows, cols, gen, exponents):
+    """Random whole weights (-8 .. 7), a power of two as every block's scale."""
+    raw = torch.randint(0, 256, (rows, cols // 32, 18), dtype=torch.uint8, device="cuda", generator=gen)
+    scale = 2.0 ** torch.randint(exponents[0], exponents[1] + 1, (rows, cols // 32, 1), device="cuda", generator=gen)
+    raw[..., :2] = scale.half().view(torch.uint8)
+    return ops.upload_weight(raw.reshape(-1).cpu().numpy(), synth.Q4_0, rows, cols)
+
+
+@pytest.mark.parametrize("rows,cols,T", [(1000, 2816, 256), (2370, 8192, 200), (12100, 3072, 128), (1000, 2048, 256)])
+def test_q4_sums_that_fit_fp32_are_exact(ops, rows, cols, T):
+    """Whole numbers at scales that are powers of two: a sum is a multiple of 2^-6 and stays below 2^18 (asserted of the results), so that 24 bits hold
+    it at every step: nothing may be cut or rounded."""
+    gen = generator(rows)
+    W = q4_of(ops, rows, cols, gen, (-6, -2))
+    x = torch.randint(-20, 21, (T, cols), device="cuda", generator=gen).float()
+    x[:, ::32] = 127.0                                                # (a block's largest value: scales of 1)
+    ref = x.double() @ ops.dequantize(W).double().T
+    assert ref.abs().max() < 2.0 ** 18 and torch.equal(rounded(ops, synth.Q4_0, x), x.double())
+    assert torch.equal(ops.ggml_mul_mat(W, x).double(), ref)
+    idx = torch.where(torch.rand(T, rows, device="cuda", generator=gen) < 0.7, 1.0, -1.0)
+    assert torch.equal(ops.ggml_mul_mat_idx(W, x, idx).double(), ref * (idx >= 0))
+
+
+@pytest.mark.parametrize("rows,cols,T", [(1000, 2816, 256), (12100, 8192, 128)])
+def test_q4_tokens_of_one_feature(ops, rows, cols, T):
+    """One term: the product of the rests, 2^-22 of it, is left out, and the others are cut once each at 2^-23 of their sum."""
+    gen = generator(cols)
+    W, x = weight(ops, synth.Q4_0, rows, cols, gen), torch.zeros(T, cols, device="cuda")
+    x[torch.arange(T, device="cuda"), torch.randint(0, cols, (T,), device="cuda", generator=gen)] = torch.randn(T, device="cuda", generator=gen)
+    ref = rounded(ops, synth.Q4_0, x) @ ops.dequantize(W).double().T
+    err = (ops.ggml_mul_mat(W, x).double() - ref).abs()
+    assert (err <= (2.0 ** -22 + 2 * 2.0 ** -23) * ref.abs() + 1e-30).all()
+    assert err.norm() <= 7e-8 * ref.norm()
