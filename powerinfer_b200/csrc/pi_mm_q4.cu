@@ -59,9 +59,10 @@ __device__ __forceinline__ uint32_t ts_fma2(uint32_t a, uint32_t b, uint32_t c) 
 __device__ __forceinline__ uint32_t ts_neg2(uint32_t a) { uint32_t r; asm("neg.f16x2 %0, %1;" : "=r"(r) : "r"(a)); return r; }     // (folds into the next one)
 // a * b = hi + lo, exactly
 __device__ __forceinline__ void ts_split(uint32_t a, uint32_t b, uint32_t & hi, uint32_t & lo) { hi = ts_mul2(a, b); lo = ts_fma2(a, b, ts_neg2(hi)); }
-// Token scales above 256 (products with 127 above the halves' range) are brought below by a power of two per token and stage, which the
-// drain takes back: its exponent
-__device__ __forceinline__ int ts_down(float d0, float d1) { const int e = (int)(__float_as_uint(fmaxf(d0, d1)) >> 23) - 127; return max(0, e - 7); }
+// Token scales above 256 (products with 127 above the halves' range) are brought below by a power of two per token and block, which the
+// drain takes back: its exponent.  A CTA with such a token drains every block by itself (one power for two blocks would make a subnormal
+// half of the smaller scale, and lose what the row's result consists of where its weights in the larger one are 0).
+__device__ __forceinline__ int ts_down(float d) { const int e = (int)(__float_as_uint(d) >> 23) - 127; return max(0, e - 7); }
 
 // The rare rows whose scales times 8 are above the halves' range: found, and summed block by block for one token
 __device__ __forceinline__ bool ts_beyond(unsigned short s) { return (s & 0x7FFFu) > 0x6FFFu; }      // |s| > 8188, infinite or NaN
@@ -164,19 +165,27 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_mm_q4(const __grid_constant__
                 if (!wait(s_full + slot, phase)) break;               // rows and tokens (one barrier: a wait that is over costs 150 clocks)
                 const uint32_t a = tmem + TS_A + (uint32_t)ab * 64u;
                 const uint64_t w = tc_desc_k(ring + (uint32_t)slot * slot_bytes), w_rest = tc_desc_k(ring + (uint32_t)slot * slot_bytes + (uint32_t)N * 128u);
-                wait(s_dempty + db, dphase);
-                tc_fence_after();
-                const uint32_t d = tmem + (uint32_t)db * TS_N;
+                auto drained = [&](auto first, auto last) {           // products of columns 16 first .. 16 last
+                    constexpr int K0 = decltype(first)::value, K1 = decltype(last)::value;
+                    wait(s_dempty + db, dphase);
+                    tc_fence_after();
+                    const uint32_t d = tmem + (uint32_t)db * TS_N;
 #pragma unroll
-                for (int k = 0; k < 4; k++) {                         // the rests first (see above)
-                    tc_mma_f16_ta(d, a + 32u + 8u * k, w + 2 * k, idesc, k > 0);
-                    tc_mma_f16_ta(d, a + 8u * k, w_rest + 2 * k, idesc, true);
+                    for (int k = K0; k < K1; k++) {                   // the rests first (see above)
+                        tc_mma_f16_ta(d, a + 32u + 8u * k, w + 2 * k, idesc, k > K0);
+                        tc_mma_f16_ta(d, a + 8u * k, w_rest + 2 * k, idesc, true);
+                    }
+#pragma unroll
+                    for (int k = K0; k < K1; k++) tc_mma_f16_ta(d, a + 8u * k, w + 2 * k, idesc, true);
+                    tc_commit(s_dfull + db);
+                    db ^= 1;
+                    if (db == 0) dphase ^= 1u;
+                };
+                if (!large) drained(std::integral_constant<int, 0>(), std::integral_constant<int, 4>());
+                else {
+                    drained(std::integral_constant<int, 0>(), std::integral_constant<int, 2>());
+                    drained(std::integral_constant<int, 2>(), std::integral_constant<int, 4>());
                 }
-#pragma unroll
-                for (int k = 0; k < 4; k++) tc_mma_f16_ta(d, a + 8u * k, w + 2 * k, idesc, true);
-                tc_commit(s_dfull + db);
-                db ^= 1;
-                if (db == 0) dphase ^= 1u;
                 tc_commit(s_empty + slot);
                 if (++slot == S) { slot = 0; phase ^= 1u; }
                 ab ^= 1;
@@ -292,13 +301,13 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_mm_q4(const __grid_constant__
                 const float d[4] = {__uint_as_float(d4.x), __uint_as_float(d4.y), __uint_as_float(d4.z), __uint_as_float(d4.w)};
 #pragma unroll
                 for (int h = 0; h < 2; h++) {                         // two stages
-                    const float down = large ? __uint_as_float((uint32_t)(127 - ts_down(d[2 * h], d[2 * h + 1])) << 23) : 1.f;
                     const uint32_t a = tmem + ((uint32_t)(wq * 32) << 16) + TS_A + (uint32_t)ab * 64u;
 #pragma unroll
                     for (int b = 0; b < 2; b++) {
                         const uint32_t at = from + row * 64u + (uint32_t)(((2 * h + b) ^ (row >> 1 & 3u)) * 16u);   // (as TMA permutes rows of 64 bytes)
                         const uint4 xl = lds(at), xh = lds(at + TS_TOK * 64);
                         const uint32_t w[8] = {xl.x, xh.x, xl.y, xh.y, xl.z, xh.z, xl.w, xh.w};
+                        const float down = large ? __uint_as_float((uint32_t)(127 - ts_down(d[2 * h + b])) << 23) : 1.f;
                         const uint32_t s2 = (uint32_t)__half_as_ushort(__float2half_rn(d[2 * h + b] * down)) * 0x10001u;
                         uint32_t hi16[16], lo16[16];
 #pragma unroll
@@ -339,16 +348,16 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_mm_q4(const __grid_constant__
 #pragma unroll
         for (int j = 0; j < TS_NC; j++) acc[j] = 0.f;
         int db = 0;
+        const int n_drains = large ? p.nb : n_st;                     // of a tile
         unsigned dphase = 0u;
         bool ok = true, odd = false;                                  // (a sum that is not finite)
         const uint32_t mine_at = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(g * nc);
-        const float2 * xd = reinterpret_cast<const float2 *>(p.x.d + (size_t)(tok0 + min(wq * 32 + lane, Tt - 1)) * p.nb);
+        const float * xd = p.x.d + (size_t)(tok0 + min(wq * 32 + lane, Tt - 1)) * p.nb;
         auto tile_sums = [&](auto pieces) {                           // up to 32, 64 or 80 columns (what lies beyond nc is some other warp's, and dropped)
             constexpr int C = decltype(pieces)::value;
 #pragma unroll 1
-            for (int st = 0; st < n_st; st++) {
-                float up = 1.f;
-                if (large) { const float2 d = xd[st]; up = __uint_as_float((uint32_t)(127 + ts_down(d.x, d.y)) << 23); }
+            for (int st = 0; st < n_drains; st++) {
+                const float up = large ? __uint_as_float((uint32_t)(127 + ts_down(xd[st])) << 23) : 1.f;
                 ok = wait(s_dfull + db, dphase) && ok;
                 tc_fence_after();
                 const uint32_t src = mine_at + (uint32_t)db * TS_N;

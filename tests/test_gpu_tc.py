@@ -129,9 +129,10 @@ def test_q4_gathers(ops, rows, cols, T, share):
     assert ops.last_op_status() == 0
 
 
-def test_q4_tokens_above_the_halves_range(ops):
+@pytest.mark.parametrize("cols", [2048, 3072])
+def test_q4_tokens_above_the_halves_range(ops, cols):
     """Blocks of a token whose scale times 127 is above 65504, beside tokens and blocks with small ones."""
-    rows, cols, T = 1000, 2048, 200
+    rows, T = 1000, 200
     gen = generator(3)
     W, x = weight(ops, synth.Q4_0, rows, cols, gen), torch.randn(T, cols, device="cuda", generator=gen)
     x[3] *= 3e4
@@ -141,9 +142,25 @@ def test_q4_tokens_above_the_halves_range(ops):
     close_q4(ops.ggml_mul_mat(W, x), rounded(ops, synth.Q4_0, x), ops.dequantize(W).double())
 
 
-def test_q4_rows_above_the_halves_range(ops):
+@pytest.mark.parametrize("rows,T", [(1000, 200), (12100, 128)])
+def test_q4_blocks_beside_one_above_the_halves_range(ops, rows, T):
+    """Scales around 0.0002 beside scales of up to 30000 in blocks where a row's weights are 0: the result is that of the small ones alone."""
+    cols, gen = 3072, generator(rows)
+    raw = torch.from_numpy(synth.quantize_q4_0((torch.randn(rows, cols, device="cuda", generator=gen) * 0.05).cpu().numpy()).reshape(rows, cols // 32, 18).copy())
+    raw[:, ::2, 2:] = 0x88
+    W = ops.upload_weight(raw.reshape(-1).numpy(), synth.Q4_0, rows, cols)
+    x = torch.randn(T, cols, device="cuda", generator=gen) * 0.01
+    x.view(T, -1, 2, 32)[::3, :, 0] *= 10.0 ** (3 + 5 * torch.rand((T + 2) // 3, cols // 64, 1, device="cuda", generator=gen))
+    close_q4(ops.ggml_mul_mat(W, x), rounded(ops, synth.Q4_0, x), ops.dequantize(W).double())
+    idx = torch.where(torch.rand(T, rows, device="cuda", generator=gen) < 0.7, 1.0, -1.0)
+    close_q4(ops.ggml_mul_mat_idx(W, x, idx), rounded(ops, synth.Q4_0, x), ops.dequantize(W).double(), idx >= 0)
+    assert ops.last_op_status() == 0
+
+
+@pytest.mark.parametrize("cols", [2048, 3072])
+def test_q4_rows_above_the_halves_range(ops, cols):
     """Rows with weights above 65504, single blocks of them among others, in a dense product and a gather with gate."""
-    rows, cols, T = 1024, 2048, 200
+    rows, T = 1024, 200
     gen = generator(4)
     w = torch.randn(rows, cols, device="cuda", generator=gen) * 0.05
     w[5] *= 2e6
