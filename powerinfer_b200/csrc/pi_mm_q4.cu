@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_mm_q4(const __grid_constant__
             const int n_tile = min(items, hi - lo - tile * items), half = items / 2;
             float * mine = epi + (warp - 12) * (TS_EPI / 4);
 #pragma unroll
-            for (int j = 0; j < TS_NC; j++) odd |= !(fabsf(acc[j]) < __int_as_float(0x7F800000));
+            for (int j = 0; j < TS_NC; j++) odd |= j < nc && !(fabsf(acc[j]) < __int_as_float(0x7F800000));        // (behind nc: what an earlier kernel left)
 #pragma unroll 1
             for (int c = 0; c < half; c += 16) {                      // (one copy of the body: only the selection is unrolled)
                 const int k0 = g * half + c;                          // item of the tile

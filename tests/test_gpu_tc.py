@@ -213,3 +213,26 @@ def test_q4_tokens_of_one_feature(ops, rows, cols, T):
     err = (ops.ggml_mul_mat(W, x).double() - ref).abs()
     assert (err <= (2.0 ** -22 + 2 * 2.0 ** -23) * ref.abs() + 1e-30).all()
     assert err.norm() <= 7e-8 * ref.norm()
+
+
+def test_q4_products_take_no_notice_of_what_tensor_memory_held(ops):
+    """Ranges of 144 rows are read from tensor memory in pieces of 80 columns, so that 8 of the last piece are an earlier kernel's.  Infinite sums
+    there started a search through the scales of all rows: the same product after infinite and after finite ones takes the same time."""
+    sms, cols, T = torch.cuda.get_device_properties(0).multi_processor_count, 2816, 128
+    gen = generator(11)
+    raw = torch.randint(0, 256, (sms * 160, cols // 32, 18), dtype=torch.uint8, device="cuda", generator=gen)
+    x, ws = torch.randn(T, cols, device="cuda", generator=gen), []
+    for scale, rows in ((float("inf"), 160), (0.01, 160), (0.01, 144)):
+        raw[..., :2] = torch.full((1, 1, 1), scale, device="cuda").half().view(torch.uint8)
+        ws.append(ops.upload_weight(raw[:sms * rows].reshape(-1).cpu().numpy(), synth.Q4_0, sms * rows, cols))
+    times = []
+    for before in ws[:2] * 5:
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        ops.ggml_mul_mat(before, x)
+        a.record()
+        y = ops.ggml_mul_mat(ws[2], x)
+        b.record()
+        torch.cuda.synchronize()
+        times.append(a.elapsed_time(b))
+        assert y.isfinite().all()
+    assert min(times[0::2]) < 1.3 * min(times[1::2]), times
