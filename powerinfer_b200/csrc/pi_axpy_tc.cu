@@ -76,7 +76,8 @@ __global__ void __launch_bounds__(XT_THREADS, 1) k_axpy_tc(const __grid_constant
         // ================================================================= coefficients
         int slot = 0;
         unsigned phase = 1u;                                          // parity of the hand-back to wait for (first round: none)
-        for (int i = 0; i < n_st; i++) {
+        int i = 0;
+        for (; i < n_st; i++) {
             if (!wait(s_empty + slot, phase)) break;
             if (lane == 0) {
                 mbar_expect_tx(s_full + slot, (unsigned)(p.nt * p.c_rows * 128));
@@ -85,8 +86,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) k_axpy_tc(const __grid_constant
             __syncwarp();
             if (++slot == S) { slot = 0; phase ^= 1u; }
         }
-        if (s_dead && lane == 0)                                      // do not exit with tiles still landing in shared memory
-            for (int t = 0; t < S; t++) { int spins = 0; while (!mbar_try_wait(s_full + t, 0) && !mbar_try_wait(s_full + t, 1) && ++spins < (1 << 16)) {} }
+        if (lane == 0) ring_land(s_full, i, S);
         __syncwarp();
     } else if (warp == 1) {
         // ================================================================= products

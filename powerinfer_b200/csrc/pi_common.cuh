@@ -7,6 +7,7 @@
 #include <stddef.h>
 
 #include "../../include/powerinfer_b200.h"
+#include "pi_ring.h"
 
 namespace pi {
 
@@ -322,6 +323,15 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t * bar, unsigned parity) {
     asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
                  : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return ok != 0;
+}
+// One thread, at the end of a kernel: waits (bounded) until the copies of the last use of every slot have landed, so that no CTA ends with copies
+// on their way into shared memory that another may own by then.  A phase that also counts threads which have given up never completes:
+// one bound for all slots, long enough for any copy.
+__device__ __forceinline__ void ring_land(uint64_t * full, int issued, int slots) {
+    for (int s = 0, spins = 0; s < slots; s++) {
+        const int parity = ring_last_parity(issued, slots, s);
+        while (parity >= 0 && spins < (1 << 16) && !mbar_try_wait(full + s, (unsigned)parity)) spins++;
+    }
 }
 // Weights are read once per step and a step streams far more of them than L2 holds: they are marked evict-first, so what
 // IS re-used between kernels (kernel code, activations, partial vectors, masks) is not pushed out of L2 by them.

@@ -163,7 +163,9 @@ __global__ void __launch_bounds__(RING_THREADS) k_gemv_ring(const RingP p) {
     // stage st of this CTA covers items [ (cta + st*G) * R, +R ) of the row / list sequence
     int n_items, n_stages;
     auto stage_first = [&](int st) { return (cta + st * G) * R; };
+    int issued = 0;                                                 // stages, in order
     auto issue = [&](int st) {                                       // all lanes of warp 0
+        issued++;
         const int s = st % S;
         const int first = stage_first(st);
         const int n = min(R, n_items - first);
@@ -270,9 +272,7 @@ __global__ void __launch_bounds__(RING_THREADS) k_gemv_ring(const RingP p) {
             if (p.dst16) p.dst16[g] = __float2half_rn(o);
         }
     }
-    if (__syncthreads_or(dead) && tid == 0) {                       // do not exit with copies still landing in shared memory
-        for (int s = 0; s < S; s++) { int spins = 0; while (!mbar_try_wait(full + s, 0) && !mbar_try_wait(full + s, 1) && ++spins < (1 << 16)) {} }
-    }
+    if (__syncthreads_or(dead) && tid == 0) ring_land(full, issued, S);
 }
 
 // Dense matrices whose stage holds at least one row per warp (R >= 8): every warp owns whole rows of the stage, so nothing
@@ -304,7 +304,9 @@ __global__ void __launch_bounds__(RING_THREADS) k_gemv_ring_w(const RingP p) {
     const int total_stages = (n_items + R - 1) / R;
     const int n_stages = cta < total_stages ? (total_stages - cta + G - 1) / G : 0;
     auto stage_first = [&](int st) { return (cta + st * G) * R; };
+    int issued = 0;                                                 // stages, in order
     auto issue = [&](int st) {                                       // lane 0 of warp 0
+        issued++;
         const int s = st % S, first = stage_first(st), n = min(R, n_items - first);
         mbar_expect_tx(full + s, (unsigned)(n * p.row_bytes));
         bulk_g2s(ring + (size_t)s * p.stage_bytes, p.W + (size_t)first * p.row_bytes, (unsigned)(n * p.row_bytes), full + s);
@@ -379,7 +381,7 @@ __global__ void __launch_bounds__(RING_THREADS) k_gemv_ring_w(const RingP p) {
             int spins = 0;
             bool gave_up = false;
             while (!mbar_try_wait(empty + s, parity)) { if (++spins > (1 << 20)) { gave_up = true; break; } }
-            if (gave_up) { if (lane == 0) atomicOr(p.status, 4u); }
+            if (__any_sync(0xffffffffu, gave_up)) { dead = true; if (lane == 0) atomicOr(p.status, 4u); }      // (nothing is issued from here on)
             else if (lane == 0 && !dead) {
                 if (p.masks_out) {
                     unsigned long long m = 0ull;
@@ -394,9 +396,7 @@ __global__ void __launch_bounds__(RING_THREADS) k_gemv_ring_w(const RingP p) {
             }
         }
     }
-    if (__syncthreads_or(dead) && tid == 0) {                       // do not exit with copies still landing in shared memory
-        for (int s = 0; s < S; s++) { int spins = 0; while (!mbar_try_wait(full + s, 0) && !mbar_try_wait(full + s, 1) && ++spins < (1 << 16)) {} }
-    }
+    if (__syncthreads_or(dead) && tid == 0) ring_land(full, issued, S);
 }
 
 // The same hand-off for stages of fewer than 8 vectors (the gather mat-vec with the gate rows riding along, matrices with
@@ -427,7 +427,9 @@ __global__ void __launch_bounds__(RING_THREADS) k_gemv_ring_g(const RingP p) {
     __syncthreads();
     int n_items, n_stages;
     auto stage_first = [&](int st) { return (cta + st * G) * R; };
+    int issued = 0;                                                 // stages, in order
     auto issue = [&](int st) {                                       // all lanes of warp 0
+        issued++;
         const int s = st % S, first = stage_first(st), n = min(R, n_items - first);
         unsigned char * dstp = ring + (size_t)s * p.stage_bytes;
         if (!SPARSE) {
@@ -538,13 +540,11 @@ __global__ void __launch_bounds__(RING_THREADS) k_gemv_ring_g(const RingP p) {
             int spins = 0;
             bool gave_up = false;
             while (!mbar_try_wait(empty + s, parity)) { if (++spins > (1 << 20)) { gave_up = true; break; } }
-            if (gave_up) { if (lane == 0) atomicOr(p.status, 4u); }
+            if (__any_sync(0xffffffffu, gave_up)) { dead = true; if (lane == 0) atomicOr(p.status, 4u); }      // (nothing is issued from here on)
             else if (!dead) issue(st + S);
         }
     }
-    if (__syncthreads_or(dead) && tid == 0) {
-        for (int s = 0; s < S; s++) { int spins = 0; while (!mbar_try_wait(full + s, 0) && !mbar_try_wait(full + s, 1) && ++spins < (1 << 16)) {} }
-    }
+    if (__syncthreads_or(dead) && tid == 0) ring_land(full, issued, S);
 }
 
 struct RingPlan { bool ok; int R, split, rw, stages, ctas_per_sm; size_t stage_bytes, smem; int max_items; };

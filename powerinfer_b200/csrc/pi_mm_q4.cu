@@ -197,7 +197,8 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_mm_q4(const __grid_constant__
             // ============================================================= activations
             int xb = 0, pair = 0;
             unsigned xphase = 1u;
-            for (int i = 0; i < n_tiles * (n_st / 2); i++) {
+            int i = 0;
+            for (; i < n_tiles * (n_st / 2); i++) {
                 if (!wait(s_xempty + xb, xphase)) break;
                 if (lane == 0) {
                     const uint32_t to = xbufs + (uint32_t)xb * TS_XBUF;
@@ -211,8 +212,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_mm_q4(const __grid_constant__
                 xb ^= 1;
                 if (xb == 0) xphase ^= 1u;
             }
-            if (s_dead && lane == 0)                                  // do not exit with tiles still landing in shared memory
-                for (int t = 0; t < 2; t++) { int spins = 0; while (!mbar_try_wait(s_xfull + t, 0) && !mbar_try_wait(s_xfull + t, 1) && ++spins < (1 << 16)) {} }
+            if (lane == 0) ring_land(s_xfull, i, 2);
             __syncwarp();
         } else {
             // ============================================================= rows: a block a lane, 16 rows x 2 blocks

@@ -114,7 +114,8 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
         // ================================================================= TMA tiles
         int slot = 0, slice = 0, row = lo;
         unsigned phase = 1u;                                          // parity of the hand-back to wait for (first round: none)
-        for (int i = 0; i < n_tiles * n_stages; i++) {
+        int i = 0;
+        for (; i < n_tiles * n_stages; i++) {
             if (!wait(s_empty + slot, phase)) break;
             if (lane == 0) {
                 mbar_expect_tx(s_full + slot, (unsigned)(su * (p.nt * p.x_rows + (SPARSE ? 0 : p.per_tile)) * 128));
@@ -130,8 +131,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
             if (slice >= n_slices) { slice = 0; row += items; }
             if (++slot == S) { slot = 0; phase ^= 1u; }
         }
-        if (s_dead && lane == 0)                                      // do not exit with tiles still landing in shared memory
-            for (int t = 0; t < S; t++) { int spins = 0; while (!mbar_try_wait(s_full + t, 0) && !mbar_try_wait(s_full + t, 1) && ++spins < (1 << 16)) {} }
+        if (lane == 0) ring_land(s_full, i, S);
         __syncwarp();
     } else if (warp == 1) {
         // ================================================================= products

@@ -225,7 +225,8 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(Z::REGS_P));
         int slot = 0;
         unsigned phase = 1u;                                          // parity of the hand-back to wait for (first round: none)
-        for (int i = 0; i < n_units; i++) {
+        int i = 0;
+        for (; i < n_units; i++) {
             if (!wait(s_empty + slot, phase)) break;
             if (pt == 0) issue_tma(slot);
             issue_w(slot);
@@ -234,8 +235,7 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
             if (++slot == S) { slot = 0; phase ^= 1u; }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
-        if (s_dead && pt == 0)                                        // do not exit with tiles still landing in shared memory
-            for (int t = 0; t < S; t++) { int spins = 0; while (!mbar_try_wait(s_full + t, 0) && !mbar_try_wait(s_full + t, 1) && ++spins < (1 << 16)) {} }
+        if (pt == 0) ring_land(s_full, i, S);
         return;
     }
     // ===================================================================== consumers
