@@ -108,7 +108,9 @@ __global__ void __launch_bounds__(XT_THREADS, 1) k_axpy_tc(const __grid_constant
             tc_commit(s_empty + slot);
             if (++slot == S) { slot = 0; phase ^= 1u; }
         }
-        tc_commit(&s_done);
+        tc_commit(&s_done);                                           // nothing is in flight when tensor memory is given back
+        for (int spins = 0; spins < (1 << 20) && !mbar_try_wait(&s_done, 0u); spins++) {}
+        __syncwarp();
     } else {
         // ================================================================= rows
         const int pw = warp - 2, n_tasks = n_st * TASKS;

@@ -46,3 +46,15 @@ def test_no_kernel_waits_for_either_parity():
     for name in sorted(os.listdir(CSRC)):
         text = open(os.path.join(CSRC, name)).read()
         assert not re.search(r"try_wait\([^;]*, 0u?\) *&& *!mbar_try_wait\([^;]*, 1u?\)", text), name
+
+
+def test_tensor_memory_is_given_back_when_no_product_is_in_flight():
+    """Every kernel that gives tensor memory back lets the issuing warp wait for its last products, also after a wait ran out (no look at s_dead)."""
+    seen = 0
+    for name in sorted(os.listdir(CSRC)):
+        text = open(os.path.join(CSRC, name)).read()
+        if "tc_dealloc(tmem" not in text:
+            continue
+        seen += 1
+        assert re.search(r"tc_commit\(&(\w+)\);[^\n]*\n *for \(int spins = 0; spins < \(1 << 20\) && !mbar_try_wait\(&\1, 0u\); spins\+\+\) \{\}\n *__syncwarp\(\);", text), name
+    assert seen == 3
