@@ -545,7 +545,8 @@ static int axpy_mm_tokens(const AxpyMmP & p, int grid, bool pdl, cudaStream_t st
 int launch_axpy_mm(const AxpyArgs & a, cudaStream_t st, int * pieces_used) {
     const bool q4 = a.wtype == PI_TYPE_Q4_0;
     if (!a.coef || a.coef_stride % 8 != 0 || !a.list || (q4 ? a.ncols % 256 != 0 : a.ncols % 8 != 0)) return PI_ERR_UNSUPPORTED;
-    if (a.T > AXPY_TC_TOKENS && !(q4 && a.exact)) return launch_axpy_tc(a, st, pieces_used);
+    // (room for fewer partial vectors, an engine in a workspace of its earlier size: fewer and longer chains in tensor memory than here)
+    if (a.T > AXPY_TC_TOKENS && !(q4 && a.exact) && a.n_groups >= axpy_tc_pieces(a.ncols)) return launch_axpy_tc(a, st, pieces_used);
     AxpyMmP p;
     int grid;
     axpy_mm_shape(a.ncols, a.T, &p.n_cs, &p.n_tg, &grid, &p.n_pieces);

@@ -278,9 +278,9 @@ static int xt_go(const XtP & p, bool pdl, cudaStream_t st) {
     return PI_OK;
 }
 
-// Called by launch_axpy_mm, which has checked the arguments.  Tokens go in launches of at most 256.
+// Called by launch_axpy_mm, which has checked the arguments and the room for axpy_tc_pieces partial vectors.  Tokens go in launches of at most 256.
 int launch_axpy_tc(const AxpyArgs & a, cudaStream_t st, int * pieces_used) {
-    const int split = (int)imin64(axpy_tc_pieces(a.ncols), a.n_groups), cw = xt_columns(a.ncols);
+    const int split = axpy_tc_pieces(a.ncols), cw = xt_columns(a.ncols);
     if (pieces_used) *pieces_used = split;
     for (int t0 = 0; t0 < a.T; t0 += 256) {
         XtP p;

@@ -170,7 +170,7 @@ struct pi_engine {
     int hd, dq, dkv, F, T_max;
     int P_max;                               // tokens of a prompt chunk (>= T_max)
     int G;                                   // axpy row groups (one token)
-    bool few_pieces;                         // the workspace has room for the least partial vectors of a batch only
+    bool few_pieces;                         // the workspace has room for the least partial vectors of a batch only: no k_axpy_tc
     // device buffers carved from the caller's workspace
     int32_t * tokens, * pos, * seq_ids, * seq_pf, * argmax;   // seq_pf: the sequence of every token of a prompt chunk
     float * x, * x2, * attn_out, * ffn_vec, * qkv, * pred, * h, * partial, * logits, * cs;

@@ -152,6 +152,47 @@ def test_prompt_in_a_long_context(engine_mod, heads, kv, n_ctx):
 
 
 @pytest.mark.parametrize("wtype", [synth.F16, synth.Q4_0])
+def test_prompt_in_a_workspace_with_room_for_fewer_partial_vectors(engine_mod, monkeypatch, wtype):
+    """A workspace of the size that engines had before k_axpy_tc is taken, and their down projections are k_axpy_mm's: against the same prompts
+    token by token."""
+    from powerinfer_b200._lib import PiError
+    spec = synth.ModelSpec(arch=synth.ARCH_LLAMA, wtype=wtype, n_layer=1, d=2048, n_ff=2048, n_head=16, n_head_kv=4, rank=64, n_vocab=256, n_ctx=256, firing=0.6, seed=9)
+    t = apart(spec, synth.build_model(spec), 17)
+    query = engine_mod.lib.pi_engine_workspace_bytes
+
+    def engine_of(less):
+        monkeypatch.setattr(engine_mod.lib, "pi_engine_workspace_bytes", lambda cfg: query(cfg) - less)
+        try:
+            return engine_mod.DecodeEngine(spec, t, max_batch=2)
+        finally:
+            monkeypatch.setattr(engine_mod.lib, "pi_engine_workspace_bytes", query)
+
+    whole = engine_of(0)
+    lo, hi = 0, query(engine_mod.C.byref(whole.cfg))                  # the most bytes that can be left out lie between
+    whole.close()
+    while hi - lo > 65536:
+        mid = (lo + hi) // 2
+        try:
+            engine_of(mid).close()
+            lo = mid
+        except PiError:
+            hi = mid
+    assert lo > 1 << 20                                               # (some partial vectors of 256 tokens)
+    small = engine_of(lo)
+    one = engine_mod.DecodeEngine(spec, t, max_batch=1)
+    rng = np.random.default_rng(18)
+    for n in (50, 77, 200):
+        toks = rng.integers(0, spec.n_vocab, n).astype(np.int32)
+        for pos in range(n):
+            ref, _ = one.decode([toks[pos]], [pos])
+        got, _ = small.prefill(toks, seq=1)
+        assert np.linalg.norm(got - ref[0]) <= (24e-3 if wtype == synth.Q4_0 else 3e-3) * np.linalg.norm(ref[0]), n
+    small.status()
+    one.close()
+    small.close()
+
+
+@pytest.mark.parametrize("wtype", [synth.F16, synth.Q4_0])
 def test_prompt_in_chunks_of_the_batch(engine_mod, wtype):
     """With a trace of the predictor logits a prompt goes through in steps of max_batch tokens (8 + 8 + 5: a plain run, a captured one, a
     replay), and leaves what one chunk leaves."""
