@@ -335,9 +335,11 @@ static size_t attn_mm_smem(const AttnArgs & a, int * P, int * R) {
 }
 
 // Several tokens and head_dim 64 or 128 whose scores fit; the others keep one CTA per head and token.  For prompt chunks of 32 tokens and more
-// that is contexts of up to 2880 positions (256 tokens at the end of 2048, 32 heads of 128, 4 layers 4952 | 1276 us, of 2560 5611 | 1366); for
-// the rest the line stays where scores and probabilities apart would fit (16 rows: about 1900 positions; 16 tokens at the end of 2304, 16 heads
-// of 64, 314 | 346, of 2560, 32 heads of 128 699 | 538).  So do steps of several sequences whose CTAs per head and token fit the SMs at once: nothing is gained there
+// and at least 24 CTAs that is contexts of up to 2880 positions (256 tokens at the end of 2048, 32 heads of 128, 4 layers 4952 | 1276 us, of 2560
+// 5611 | 1366; fewer CTAs leave the chip idle: at the end of 2560, 4 layers, 4 heads of 128 and 32 tokens, 8 CTAs, 296 | 417, 8 heads of 64 and
+// 32 tokens, 16, 319 | 356; 40 tokens, 24, gain 4 .. 6 %, 16 heads of 64 and 32 tokens, 32, 14 .. 18 %); for the rest the line stays where
+// scores and probabilities apart would fit (16 rows: about 1900 positions; 16 tokens at the end of 2304, 16 heads of 64, 314 | 346, of 2560, 32
+// heads of 128 699 | 538).  So do steps of several sequences whose CTAs per head and token fit the SMs at once: nothing is gained there
 // by reading a KV head once for all of its query heads, and a CTA of k_attention_row has more rows in flight.  us in k_attention_row | here,
 // 8 sequences of 8 heads of 64: 200 positions 5.5 | 7.1, 1000 8.5 | 16.3, 3500 19.8 | 44.3; 4 of 32 heads of 128, 1000 positions
 // 13.1 | 20.8.  With more CTAs than SMs: 32 sequences of 8 heads of 64 over 2 KV heads, 200 positions
@@ -352,7 +354,8 @@ bool attention_mm_takes(const AttnArgs & a) {
     if (a.store_mode == 0 && a.n_head / a.n_head_kv * a.head_dim <= 128 && a.n_ctx > 64 * a.head_dim) return false;
     if (!(a.T >= 2 && (a.head_dim == 64 || a.head_dim == 128) && a.n_ctx > 0)) return false;
     const size_t smem = attn_mm_smem(a, &P, &R);
-    return smem + (a.store_mode != 0 && a.T >= 32 ? 0 : (size_t)R * (P + 8) * 2) <= AM_SMEM_MAX;
+    const bool many = a.store_mode != 0 && a.T >= 32 && (int64_t)a.n_head * ((a.T + 15) / 16) >= 24;
+    return smem + (many ? 0 : (size_t)R * (P + 8) * 2) <= AM_SMEM_MAX;
 }
 
 // UN = 4 takes 126 registers with head_dim 128, two CTAs per SM.  Where the grid and shared memory give an SM more than two, half
