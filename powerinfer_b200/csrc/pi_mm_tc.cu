@@ -11,6 +11,9 @@
 // one launch of 8600 of 11008 gated rows of 8 KB: 47 us; rows by cp.async, 50 clocks per warp and copy, 70 in the kernel before this one; by
 // tile::gather4, 90 clocks per four rows of 128 bytes, 94).
 //
+// Short rows are the launch's fixed part: what a CTA finds out before its first request (ranges come from the host, no 64-bit division), the first
+// trip to memory, and the results' way out.  us, mma.sync | here, 64 tokens: 1024 x 64 4.4 | 4.7, 512 x 128 4.7 | 4.7, 1024 x 256 5.4 | 5.3.
+//
 // us, mma.sync | here, 77, 128 and 256 tokens: 12288 x 4096 38.7 | 26.0, 51.5 | 30.2, 74.4 | 37.6; 1024 x 4096 30.2 | 11.5, 38.1 | 11.7, 42.9 | 12.7;
 // the FFN of 72 % of 11008 x 4096, down projection included, 119 | 71, 175 | 78, 290 | 118.
 #include "pi_tc.cuh"
@@ -30,6 +33,7 @@ static constexpr int MT_PASS = MT_OUT / 8;              // rows of a pass of the
 struct alignas(64) MtP {
     CUtensorMap m_w, m_x;
     const uint8_t * W; const uint8_t * W2; int64_t row_bytes; int nrows, ncols;
+    int groups, share, more;                                     // groups of CTAs along the rows; dense: rows (masks_out: bytes of the masks) of a group, groups that have one more
     int T, nt, n_tt, x_rows, per_tile, ring;             // token tiles of a CTA (1, 2), CTAs that share rows, rows of an activation box, of a dense box, bytes of the ring
     const uint32_t * masks; const int32_t * bucket; int32_t * list; int32_t * count; unsigned long long * rows_total;
     const float * idx; int64_t idx_stride; float threshold;
@@ -54,8 +58,9 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
     int * const rows = reinterpret_cast<int *>(epi + MT_OUT / 32 * (MT_EPI / 4));      // rows of this CTA (sparse only)
     constexpr int ks = SPLIT ? MT_RANKS : 1;
     const int rank = SPLIT ? (int)(blockIdx.x % ks) : 0, block = blockIdx.x / ks;       // ranges of columns, this CTA's
-    const int G = gridDim.x / (p.n_tt * ks), cta = block / p.n_tt, tok_first = (int)(block % p.n_tt) * p.x_rows;
+    const int cta = p.n_tt == 1 ? block : (int)((unsigned)block / (unsigned)p.n_tt), tok_first = (block - cta * p.n_tt) * p.x_rows;
     const int tok_end = p.n_tt > 1 ? min(p.T, tok_first + p.x_rows) : p.T;
+    if (tid == 32) { tma_map(&p.m_x); if (!SPARSE) tma_map(&p.m_w); }
     if (tid < 8) s_any[tid] = 0u;
     if (tid < MT_SMAX) { mbar_init(s_full + tid, SPARSE ? 1 + MT_OUT / 32 : 1); mbar_init(s_empty + tid, 1); }
     if (tid < 2) { mbar_init(s_dfull + tid, 1); mbar_init(s_dempty + tid, MT_OUT / 32); }
@@ -77,27 +82,27 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
     };
 
     int lo, hi;
-    pdl_wait();
     if (SPARSE) {
-        const int total = tc_active_rows<MT_THREADS>(p.masks, p.nrows, cta, G, s_warp, rows, lo, hi);
+        pdl_wait();
+        const int total = tc_active_rows<MT_THREADS>(p.masks, p.nrows, cta, p.groups, s_warp, rows, lo, hi);
         if (blockIdx.x == 0 && tid == 0) {
             if (p.count) *p.count = total;
             if (p.rows_total && total) atomicAdd(p.rows_total, (unsigned long long)total);      // statistics
         }
         if (p.list && tok_first == 0) for (int k = tid; k < hi - lo; k += MT_THREADS) p.list[lo + k] = rows[k];
-        if (p.coef && cta == G - 1 && tok_first == 0) {                                 // zeros behind the last position (k_axpy_tc reads stages of 64)
+        if (p.coef && cta == p.groups - 1 && tok_first == 0) {                                 // zeros behind the last position (k_axpy_tc reads stages of 64)
             const int64_t end = (total + 63) / 64 * 64 < p.coef_stride ? (total + 63) / 64 * 64 : p.coef_stride;
             for (int e = tid; e < p.T * 64; e += MT_THREADS)
                 if (total + e % 64 < end) p.coef[(size_t)(e / 64) * p.coef_stride + total + e % 64] = __ushort_as_half((unsigned short)0);
         }
     } else {
-        const int al = p.masks_out ? 8 : 1, gr = (p.nrows + al - 1) / al;          // (a byte of the masks has one writer)
-        lo = min(p.nrows, (int)((long long)gr * cta / G) * al);
-        hi = min(p.nrows, (int)((long long)gr * (cta + 1) / G) * al);
+        const int al = p.masks_out ? 8 : 1;                           // (a byte of the masks has one writer)
+        lo = min(p.nrows, (p.share * cta + min(cta, p.more)) * al);
+        hi = min(p.nrows, (p.share * (cta + 1) + min(cta + 1, p.more)) * al);
     }
     // tiles of equal height, N columns each (gated: column pairs, up and gate of one item)
     const int n_cols = (hi - lo) * (GATED ? 2 : 1);
-    const int n_tiles = SPARSE ? (n_cols + 255) / 256 : (n_cols + p.per_tile - 1) / p.per_tile;
+    const int n_tiles = SPARSE ? (n_cols + 255) / 256 : n_cols <= p.per_tile ? n_cols > 0 : (int)((unsigned)(n_cols + p.per_tile - 1) / (unsigned)p.per_tile);
     const int N = SPARSE ? (n_tiles ? ((n_cols + n_tiles - 1) / n_tiles + 15) / 16 * 16 : 16) : (p.per_tile + 15) / 16 * 16;
     const int items = GATED ? N / 2 : SPARSE ? N : p.per_tile;        // of a tile
     const int all_slices = (p.ncols + 63) / 64, slice0 = all_slices * rank / ks;
@@ -106,9 +111,10 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
     // A stage is `su` slices of 64 columns, as many as leave three stages: a hand-over costs each of the three parties 200 .. 400 clocks,
     // a slice of few rows less (1024 x 4096, 77 tokens: one slice a stage 23.9 us, four 17.0).
     const uint32_t w_off = p.nt > 1 ? 32768u : (uint32_t)p.x_rows * 128u, slice_bytes = w_off + (uint32_t)N * 128u;
-    const int fit = p.ring / (int)slice_bytes, deep = SPARSE ? (N <= 2 * MT_PASS ? 4 : N <= 4 * MT_PASS ? 2 : 1) : 4;   // (gathered: slices that a thread copies at once)
-    const int su = min(deep, fit >= 12 ? 4 : fit >= 6 ? 2 : 1), S = min(MT_SMAX, fit / su), n_stages = (n_slices + su - 1) / su;
+    const int fit = (int)((unsigned)p.ring / slice_bytes), deep = SPARSE ? (N <= 2 * MT_PASS ? 4 : N <= 4 * MT_PASS ? 2 : 1) : 4;   // (gathered: slices that a thread copies at once)
+    const int su = min(min(deep, n_slices), fit >= 12 ? 4 : fit >= 6 ? 2 : 1), S = min(MT_SMAX, (int)((unsigned)fit / (unsigned)su)), n_stages = n_slices <= su ? 1 : su == 1 ? n_slices : (int)((unsigned)(n_slices + su - 1) / (unsigned)su);
     const uint32_t stage = slice_bytes * (uint32_t)su;
+    if (!SPARSE) pdl_wait();
 
     if (warp == 0) {
         // ================================================================= TMA tiles
@@ -212,24 +218,47 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
                         const int r = SPARSE ? rows[tile * items + k] : item;
                         const int64_t gid = SPARSE && p.bucket ? p.bucket[r] : r;
                         const float bias = p.bias ? p.bias[gid] : 0.f;
-                        float l[PER];                                 // (predictor logits: all on their way before the first is looked at)
+                        if (SPARSE) {
+                            float l[PER];                             // (predictor logits: all on their way before the first is looked at)
 #pragma unroll
-                        for (int u = 0; u < PER; u++) {
-                            const int tok = tok0 + u * (32 / PER) + lane / PER;
-                            l[u] = SPARSE && tok < tok_end ? p.idx[(size_t)tok * p.idx_stride + gid] : 0.f;
-                        }
+                            for (int u = 0; u < PER; u++) {
+                                const int tok = tok0 + u * (32 / PER) + lane / PER;
+                                l[u] = tok < tok_end ? p.idx[(size_t)tok * p.idx_stride + gid] : 0.f;
+                            }
 #pragma unroll
-                        for (int u = 0; u < PER; u++) {
-                            const int tw = u * (32 / PER) + lane / PER, tok = tok0 + tw;
-                            const bool off = SPARSE && l[u] < p.threshold;            // (a NaN logit counts as active)
-                            float o = off ? 0.f : mine[kl * 34 + tw];
-                            if (p.bias && !(off && p.coef)) o += bias;                // (a coefficient of an inactive token is 0 whatever the bias)
-                            if (p.relu) o = fmaxf(o, 0.f);
-                            if (tok < tok_end) {
-                                if (p.dst)   p.dst[(size_t)tok * p.dst_stride + gid] = o;
-                                if (p.dst16) p.dst16[(size_t)tok * p.dst_stride + gid] = __float2half_rn(o);
-                                if (p.coef)  p.coef[(size_t)tok * p.coef_stride + item] = __float2half_rn(o);
-                                any |= !(o < p.masks_threshold);
+                            for (int u = 0; u < PER; u++) {
+                                const int tw = u * (32 / PER) + lane / PER, tok = tok0 + tw;
+                                const bool off = l[u] < p.threshold;          // (a NaN logit counts as active)
+                                float o = off ? 0.f : mine[kl * 34 + tw];
+                                if (p.bias && !(off && p.coef)) o += bias;    // (a coefficient of an inactive token is 0 whatever the bias)
+                                if (p.relu) o = fmaxf(o, 0.f);
+                                if (tok < tok_end) {
+                                    if (p.dst)   p.dst[(size_t)tok * p.dst_stride + gid] = o;
+                                    if (p.dst16) p.dst16[(size_t)tok * p.dst_stride + gid] = __float2half_rn(o);
+                                    if (p.coef)  p.coef[(size_t)tok * p.coef_stride + item] = __float2half_rn(o);
+                                }
+                            }
+                        } else {
+                            // Eight values are there before the first is stored, because a load of shared memory does not pass a store through a
+                            // pointer (16 rows of 64 tokens, clocks: one by one 2600, here 900; the gathers, with more to keep, 1.2 times slower so)
+#pragma unroll 1
+                            for (int u0 = 0; u0 < 32; u0 += 16) {
+                                const int tw0 = u0 + (lane >> 4), first = tok0 + tw0, n_tok = tok_end - first;
+                                float o[8];
+#pragma unroll
+                                for (int u = 0; u < 8; u++) {
+                                    o[u] = mine[kl * 34 + tw0 + 2 * u];
+                                    if (p.bias) o[u] += bias;
+                                    if (p.relu) o[u] = fmaxf(o[u], 0.f);
+                                    any |= 2 * u < n_tok && !(o[u] < p.masks_threshold);
+                                }
+                                auto put = [&](auto * to, auto as) {
+                                    to += (size_t)first * p.dst_stride + gid;
+#pragma unroll
+                                    for (int u = 0; u < 8; u++, to += 2 * p.dst_stride) if (2 * u < n_tok) *to = as(o[u]);
+                                };
+                                if (p.dst)   put(p.dst, [](float v) { return v; });
+                                if (p.dst16) put(p.dst16, [](float v) { return __float2half_rn(v); });
                             }
                         }
                         if (!SPARSE && p.masks_out && any) atomicOr(&s_any[k / 32], 1u << (k % 32));
@@ -389,9 +418,12 @@ static int mt_go(MtP & p, bool pdl, cudaStream_t st) {
     const int list = SPARSE ? ((p.nrows + G - 1) / G + 1) * 4 : 0;    // bytes
     p.ring = (MT_SMEM_MAX - 1024 - MT_OUT / 32 * MT_EPI - list) / 1024 * 1024;
     if (p.ring < 2 * (p.nt * 16384 + 256 * 128)) return PI_ERR_UNSUPPORTED;        // two stages of the largest kind (more than MM_MAX_ROWS rows)
-    p.per_tile = 0;
+    p.groups = G; p.per_tile = 0;
     int rc;
     if (!SPARSE) {                                                    // equal tiles; whole bytes of the masks
+        // (dealt out here: a division of 64 bits takes a CTA 0.2 us)
+        const int units = p.masks_out ? (p.nrows + 7) / 8 : p.nrows;
+        p.share = units / G; p.more = units % G;
         const int share = (p.nrows + G - 1) / G + (p.masks_out ? 8 : 0), tiles = (share + 255) / 256;
         p.per_tile = p.masks_out ? (share / tiles + 8) / 8 * 8 : (share + tiles - 1) / tiles;
         if (p.per_tile > 256) p.per_tile = 256;

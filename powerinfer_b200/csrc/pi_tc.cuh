@@ -17,6 +17,8 @@ __device__ __forceinline__ void tma_tile(uint32_t dst, const CUtensorMap * map, 
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  :: "r"(dst), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
 }
+// the map itself on its way to the SM
+__device__ __forceinline__ void tma_map(const CUtensorMap * map) { asm volatile("prefetch.tensormap [%0];" :: "l"(map) : "memory"); }
 // ---- tensor memory: allocated by one whole warp, which writes the address to shared memory; given back by the same warp
 __device__ __forceinline__ void tc_alloc(uint32_t * slot, unsigned columns) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(slot)), "r"(columns) : "memory");
@@ -104,8 +106,8 @@ __device__ __forceinline__ int tc_active_rows(const uint32_t * masks, int nrows,
 #pragma unroll
     for (int w = 0; w < THREADS / 32; w++) { if (w < warp) before += s_warp[w]; total += s_warp[w]; }
     total = __shfl_sync(0xffffffffu, total, 0);
-    lo = (int)((long long)total * grp / groups);
-    hi = (int)((long long)total * (grp + 1) / groups);
+    lo = (int)((unsigned)total * (unsigned)grp / (unsigned)groups);   // (up to 262144 rows, 148 groups: 32 bits)
+    hi = (int)((unsigned)total * (unsigned)(grp + 1) / (unsigned)groups);
     int rank = before + incl - mine;
     for (int c = c0; c < c1 && rank < hi; c++) {
         uint32_t m = c - c0 < KEEP ? mw[0] : word(c);

@@ -27,9 +27,10 @@ def close(got, x, w, terms):
 
 
 # 38040 rows: two tiles of rows per CTA; 1184 rows: 8 per CTA; 8, 24, 520, 1032 columns: parts of a slice, of a stage of several slices.  2048 columns and
-# more, up to 5280 rows: four CTAs share the columns (33, 34 or 65 slices), clusters without rows, the line itself
+# more, up to 5280 rows: four CTAs share the columns (33, 34 or 65 slices), clusters without rows, the line itself; rows of two and three slices, all in one stage
 @pytest.mark.parametrize("T", [33, 128, 129, 261])
-@pytest.mark.parametrize("rows,cols", [(8, 8), (1184, 1032), (3001, 520), (38040, 64), (8, 2048), (1001, 2120), (5120, 2056), (5290, 2048), (2100, 4104)])
+@pytest.mark.parametrize("rows,cols", [(8, 8), (1184, 1032), (3001, 520), (38040, 64), (8, 2048), (1001, 2120), (5120, 2056), (5290, 2048), (2100, 4104),
+                                       (700, 136), (9001, 192), (300, 72)])
 def test_dense_products(ops, rows, cols, T):
     gen = generator(rows + T)
     W, x = weight(ops, synth.F16, rows, cols, gen), torch.randn(T, cols, device="cuda", generator=gen)
