@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_mm_q4(const __grid_constant__
     if (tid < 2) { mbar_init(s_dfull + tid, 1); mbar_init(s_dempty + tid, (unsigned)live_quarters * 2); }
     if (tid < 2) { mbar_init(s_xfull + tid, 1); mbar_init(s_xempty + tid, (unsigned)live_quarters); }
     if (tid == 0) mbar_init(&s_fin, 1);
-    {                                                                 // a scale above 256? (ts_down; NaN too)
+    if (n_tiles) {                                                    // a scale above 256? (ts_down; NaN too)
         bool large = false;
         const float4 * d4 = reinterpret_cast<const float4 *>(p.x.d + (size_t)tok0 * p.nb);
         for (int e = tid; e < Tt * p.nb / 4; e += TS_THREADS) { const float4 v = d4[e]; large |= !(fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)) <= 256.f); }
