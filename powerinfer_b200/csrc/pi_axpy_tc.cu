@@ -19,7 +19,8 @@
 // (Q4_0: 64 blocks), 16 (8) a stage of 256 columns, dealt to the warps in turn, the next two on their way while one is stored.
 //
 // us, mma.sync | here: 28672 x 8192 Q4_0, 78 % of the rows, 256 tokens 375 | 104 (470 MB through L2 in 80 us: every range of columns reads all
-// coefficients); 11008 x 4096 FP16, 72 %, 77 tokens 38 | 24, 128 81 | 53, 256 138 | 70 (these two as operators, with 12 us of preparation and sum).
+// coefficients); 11008 x 4096 FP16, 72 %, 77 tokens 38 | 24; 75 %, as operators with 12 us of
+// preparation and sum, 77 tokens 52 | 33, 128 79 | 39, 256 138 | 66.
 #include "pi_tc.cuh"
 
 namespace pi {
@@ -225,11 +226,14 @@ __global__ void __launch_bounds__(XT_THREADS, 1) k_axpy_tc(const __grid_constant
             }
         }
         // ================================================================= sums: a thread has one token's columns
+        // Four lanes store 64 bytes of a token, through the ring, which is free (a lane its own token's 16 bytes at a time: 13824 x 5120, 256 tokens, 3 % of
+        // the rows, 63 us where mma.sync takes 58; so 53; 75 % 92 -> 83)
         if (warp >= 4) wait(&s_done, 0u);
+        float * const turn = reinterpret_cast<float *>(smem_raw + (ring - smem_u32(smem_raw))) + (warp - 4) * (32 * 20);
         tc_fence_after();
         for (int t = 0; t < p.nt && warp >= 4; t++) {
-            const int tok = t * 128 + (warp & 3) * 32 + lane;
-            if (t * 128 + (warp & 3) * 32 >= p.T) break;
+            const int tok0 = t * 128 + (warp & 3) * 32;
+            if (tok0 >= p.T) break;
             for (int c = ((warp >> 2) - 1) * 16; c < CW; c += 48) {
                 if (col0 + c >= p.ncols) break;
                 float v[16];
@@ -241,12 +245,15 @@ __global__ void __launch_bounds__(XT_THREADS, 1) k_axpy_tc(const __grid_constant
 #pragma unroll
                     for (int j = 0; j < 16; j++) v[j] += w[j];
                 }
-                if (tok < p.T) {
-                    float * o = p.partial + (size_t)mine * p.piece + (size_t)tok * p.ncols + col0 + c;
+                __syncwarp();
 #pragma unroll
-                    for (int j = 0; j < 16; j += 4)                   // (a multiple of 8 columns)
-                        if (col0 + c + j < p.ncols) *reinterpret_cast<float4 *>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                }
+                for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4 *>(turn + lane * 20 + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                __syncwarp();
+                const int part = (lane & 3) * 4;
+                float * o = p.partial + (size_t)mine * p.piece + (size_t)(tok0 + (lane >> 2)) * p.ncols + col0 + c + part;
+#pragma unroll
+                for (int j = 0; j < 32; j += 8, o += 8 * (size_t)p.ncols)           // (a multiple of 8 columns)
+                    if (tok0 + j + (lane >> 2) < p.T && col0 + c + part < p.ncols) *reinterpret_cast<float4 *>(o) = *reinterpret_cast<const float4 *>(turn + (j + (lane >> 2)) * 20 + part);
             }
         }
         tc_fence_before();
