@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(256) k_coef(const CoefP p) {
 #pragma unroll
     for (int w = 0; w < 8; w++) { base += s_pre[w] + (w < warp ? s_cnt[w] : 0); total += s_pre[w] + s_cnt[w]; }
     if (blockIdx.x == gridDim.x - 1 && blockIdx.y == 0 && tid == 0) *p.count = total;
-    if (blockIdx.x == gridDim.x - 1 && !p.exact) {                    // zeros behind the last position (k_axpy_tc reads stages of 64)
+    if (blockIdx.x == gridDim.x - 1 && !p.exact && p.T > AXPY_TC_TOKENS) {      // zeros behind the last position (k_axpy_tc reads stages of 64)
         const int64_t end = (total + 63) / 64 * 64 < p.coef_stride ? (total + 63) / 64 * 64 : p.coef_stride;
         for (int e = tid; e < UN * 64; e += 256)
             if (t0 + e / 64 < p.T && total + e % 64 < end) reinterpret_cast<__half *>(p.coef)[(size_t)(t0 + e / 64) * p.coef_stride + total + e % 64] = __ushort_as_half((unsigned short)0);
@@ -501,11 +501,6 @@ static void axpy_mm_shape(int64_t ncols, int T, int * n_cs, int * n_tg, int * gr
 bool axpy_mm_exact(int wtype, int64_t nrows, int64_t ncols, int T) {
     return wtype == PI_TYPE_Q4_0 && (T < 2 || T > 32 || ncols % 1024 != 0 || nrows * ncols > (int64_t)1 << 28);
 }
-
-// FP16 coefficients: more tokens than these go to k_axpy_tc.  Up to 64 they are one group here, and its sums, cut by the tensor cores at every
-// step, have as many chains as tensor memory has room for there: no gain in precision, and little in time (11008 x 4096, 33 tokens 35 us | 43;
-// 77 tokens 54 | 46, 128 tokens 81 | 53 and half the error, with two groups here).
-static constexpr int AXPY_TC_TOKENS = 64;
 
 int axpy_mm_least_pieces(int64_t ncols, int T) { int cs, tg, g, np; axpy_mm_shape(ncols, T, &cs, &tg, &g, &np); return np; }
 int axpy_mm_pieces(int64_t ncols, int T) {

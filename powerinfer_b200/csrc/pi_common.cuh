@@ -181,6 +181,10 @@ int axpy_mm_pieces(int64_t ncols, int T);                                       
 int axpy_mm_least_pieces(int64_t ncols, int T);                                      // ... that it can do with
 int launch_axpy_tc(const AxpyArgs & a, cudaStream_t st, int * groups_used);          // many tokens, FP16 coefficients, zeros behind them to the next multiple of 64
 int axpy_tc_pieces(int64_t ncols);
+// FP16 coefficients: more tokens than these go to k_axpy_tc.  Up to 64 they are one group in k_axpy_mm, and k_axpy_tc's sums, cut by the tensor cores at every
+// step, have as many chains as tensor memory has room for: no gain in precision, and little in time (11008 x 4096, 33 tokens 35 us | 43;
+// 77 tokens 54 | 46, 128 tokens 81 | 53 and half the error, with two groups there).
+static constexpr int AXPY_TC_TOKENS = 64;
 // axpy coefficients by list position (pi_axpy_mm.cu): [T, coef_stride], FP16 or (exact) F32, from h F32 [T, h_stride] by global neuron id
 struct CoefArgs {
     int wtype = PI_TYPE_F16;

@@ -39,7 +39,7 @@ struct alignas(64) MtP {
     const float * idx; int64_t idx_stride; float threshold;
     const float * bias; int relu;
     float * dst; __half * dst16; int64_t dst_stride;
-    __half * coef; int64_t coef_stride;
+    __half * coef; int64_t coef_stride; bool coef_tail;           // zeros behind the last position (k_axpy_tc reads stages of 64)
     uint32_t * masks_out; float masks_threshold; int masks_or;
     unsigned int * status;
 };
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
             if (p.rows_total && total) atomicAdd(p.rows_total, (unsigned long long)total);      // statistics
         }
         if (p.list && tok_first == 0) for (int k = tid; k < hi - lo; k += MT_THREADS) p.list[lo + k] = rows[k];
-        if (p.coef && cta == p.groups - 1 && tok_first == 0) {                                 // zeros behind the last position (k_axpy_tc reads stages of 64)
+        if (p.coef_tail && cta == p.groups - 1 && tok_first == 0) {
             const int64_t end = (total + 63) / 64 * 64 < p.coef_stride ? (total + 63) / 64 * 64 : p.coef_stride;
             for (int e = tid; e < p.T * 64; e += MT_THREADS)
                 if (total + e % 64 < end) p.coef[(size_t)(e / 64) * p.coef_stride + total + e % 64] = __ushort_as_half((unsigned short)0);
@@ -486,7 +486,7 @@ int launch_mm_tc(const GemvArgs & a, cudaStream_t st) {
         p.bias = a.bias; p.relu = a.relu;
         p.dst = a.dst ? a.dst + (size_t)t0 * a.dst_stride : nullptr;
         p.dst16 = a.dst16 ? a.dst16 + (size_t)t0 * a.dst_stride : nullptr; p.dst_stride = a.dst_stride;
-        p.coef = a.coef ? a.coef + (size_t)t0 * a.coef_stride : nullptr; p.coef_stride = a.coef_stride;
+        p.coef = a.coef ? a.coef + (size_t)t0 * a.coef_stride : nullptr; p.coef_stride = a.coef_stride; p.coef_tail = a.coef && a.T > AXPY_TC_TOKENS;
         p.masks_out = a.masks_out; p.masks_threshold = a.masks_threshold; p.masks_or = t0 > 0; p.status = a.status;
         rc = split ? mt_go<false, false, true>(p, a.pdl, st) : !p.masks ? mt_go<false, false, false>(p, a.pdl, st) : p.W2 ? mt_go<true, true, false>(p, a.pdl, st) : mt_go<true, false, false>(p, a.pdl, st);
         if (rc != PI_OK) return rc;
