@@ -488,14 +488,18 @@ static int ts_go(TsP & p, bool pdl, cudaStream_t st) {
 // Sums of fewer than 2816 columns are more precise in one chain, or no less (see above).  A CTA's time per 64 columns hardly depends on its rows and not at
 // all on its tokens up to 128 (hand-overs; the kernel with mma.sync takes steps of 64, 80, 96, 128, 192 and 256 tokens).  us, pi_mm_wide.cu | here:
 //   gathers (whose results it writes token by token, too)   97 tokens 4096 x 4096 60 | 52, 8192 x 8192 120 | 93; 256 tokens 88 | 67, 193 | 124
-//   dense, 193 .. 256 tokens   4096 x 4096 61.6 | 54.2, 10240 x 8192 193 | 129
+//   dense, 193 .. 256 tokens   4096 x 4096 61.6 | 54.2, 10240 x 8192 193 | 129; where the rows of a CTA pair are just more than one tile here and those of
+//                              a CTA just less than one there (two tiles take twice the time of one, however high) 13824 x 4096 101 | 108,
+//                              13824 x 8192 192 | 195: stays there; the next tile there, 14300 x 4096, 151 | 118
 //   dense, 129 .. 192          8192 x 8192 114 | 114, 5120 x 5120 75 | 69: stays there
 //   dense, 97 .. 128           4096 x 4096 41.8 | 45.5, 8192 x 8192 93 | 90, 10240 x 8192 114 | 103
 //   fewer                      10240 x 8192, 77 tokens 83 | 102
 bool mm_q4_takes(const GemvArgs & a) {
     if (a.ncols < 2816 || a.masks_out) return false;
     const int T = a.T > 256 ? 256 : a.T;
-    return a.masks ? T > 96 : T > 192 || (T > 96 && T <= 128 && a.nrows >= 10000);
+    if (a.masks) return T > 96;
+    if (T > 192) return a.nrows <= sm_count() / 2 * TS_N || a.nrows > sm_count() * 96;
+    return T > 96 && T <= 128 && a.nrows >= 10000;
 }
 
 // Called by launch_mm, which has checked the arguments.  Tokens go in launches of at most 256.

@@ -237,3 +237,14 @@ def test_q4_products_take_no_notice_of_what_tensor_memory_held(ops):
         times.append(a.elapsed_time(b))
         assert y.isfinite().all()
     assert min(times[0::2]) < 1.3 * min(times[1::2]), times
+
+
+@pytest.mark.parametrize("more", [0, 1])
+@pytest.mark.parametrize("share", [80, 96])
+def test_q4_products_around_one_tile_a_cta(ops, share, more):
+    """Rows on both sides of the lines between k_mm_q4 (one tile, several) and k_mm_wide (two tiles there, one here)."""
+    rows, cols, T = torch.cuda.get_device_properties(0).multi_processor_count * share + more, 2816, 200
+    gen = generator(rows)
+    W, x = weight(ops, synth.Q4_0, rows, cols, gen), torch.randn(T, cols, device="cuda", generator=gen)
+    close_q4(ops.ggml_mul_mat(W, x), rounded(ops, synth.Q4_0, x), ops.dequantize(W).double())
+    assert ops.last_op_status() == 0
