@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) k_axpy_tc(const __grid_constant
         __syncwarp();
     } else if (warp == 1) {
         // ================================================================= products
-        constexpr uint32_t idesc = tc_idesc(CW, true, false);
+        constexpr uint32_t idesc = tc_idesc(CW, true);
         int slot = 0, acc = 0;
         unsigned phase = 0u;
         for (int i = 0; i < n_st; i++) {

@@ -564,6 +564,7 @@ int launch_mm(const GemvArgs & a, cudaStream_t st) {
     const bool q4 = a.wtype == PI_TYPE_Q4_0;
     if (q4 ? !a.x.lo || a.ncols % 256 != 0 : !a.x.h16 || a.ncols % 8 != 0) return PI_ERR_UNSUPPORTED;
     if (a.nrows > (a.masks ? MM_MAX_ROWS : (1 << 26)) || (a.W2 && !a.masks) || (a.list && !a.masks)) return PI_ERR_UNSUPPORTED;
+    if (a.T > 32 && q4 && (a.masks_out || a.coef)) return PI_ERR_UNSUPPORTED;           // (predictors and coefficients as products are FP16 rows')
     if (a.T > 32) return !q4 ? launch_mm_tc(a, st) : mm_q4_takes(a) ? launch_mm_q4(a, st) : launch_mm_wide(a, st);
     MmP p;
     p.W = (const uint8_t *)a.W; p.W2 = (const uint8_t *)a.W2; p.row_bytes = (int64_t)pi_row_bytes(a.wtype, a.ncols);

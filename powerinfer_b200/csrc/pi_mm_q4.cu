@@ -49,7 +49,6 @@ struct alignas(64) TsP {
     const float * idx; int64_t idx_stride; float threshold;
     const float * bias; int relu;
     float * dst; __half * dst16; int64_t dst_stride;
-    __half * coef; int64_t coef_stride;
     unsigned int * status;
 };
 
@@ -158,7 +157,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_mm_q4(const __grid_constant__
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(TS_REGS_S));
         if (warp == 0) {
             // ============================================================= products
-            const uint32_t idesc = tc_idesc(N, false, false);
+            const uint32_t idesc = tc_idesc(N, false);
             int slot = 0, ab = 0, db = 0;
             unsigned phase = 0u, dphase = 1u;                         // (the first round's buffers of sums are free)
             for (int i = 0; i < n_tiles * n_st; i++) {
@@ -420,12 +419,11 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_mm_q4(const __grid_constant__
                                 const int tw = (u0 + u) * 2 + (lane >> 4), tok = tok0 + wq * 32 + tw;
                                 const bool off = SPARSE && l[u] < p.threshold;        // (a NaN logit counts as active)
                                 float o = off ? 0.f : mine[(lane & 15) * 34 + tw];
-                                if (p.bias && !(off && p.coef)) o += bias;            // (a coefficient of an inactive token is 0 whatever the bias)
+                                if (p.bias) o += bias;
                                 if (p.relu) o = fmaxf(o, 0.f);
                                 if (tok < p.T) {
                                     if (p.dst)   p.dst[(size_t)tok * p.dst_stride + gid] = o;
                                     if (p.dst16) p.dst16[(size_t)tok * p.dst_stride + gid] = __float2half_rn(o);
-                                    if (p.coef)  p.coef[(size_t)tok * p.coef_stride + item] = __float2half_rn(o);
                                 }
                             }
                         }
@@ -454,7 +452,6 @@ __global__ void __launch_bounds__(TS_THREADS, 1) k_mm_q4(const __grid_constant__
                 if (p.relu) o = fmaxf(o, 0.f);
                 if (p.dst)   p.dst[(size_t)tok * p.dst_stride + gid] = o;
                 if (p.dst16) p.dst16[(size_t)tok * p.dst_stride + gid] = __float2half_rn(o);
-                if (p.coef)  p.coef[(size_t)tok * p.coef_stride + item] = __float2half_rn(o);
             }
         }
     }
@@ -495,7 +492,7 @@ static int ts_go(TsP & p, bool pdl, cudaStream_t st) {
 //   dense, 97 .. 128           4096 x 4096 41.8 | 45.5, 8192 x 8192 93 | 90, 10240 x 8192 114 | 103
 //   fewer                      10240 x 8192, 77 tokens 83 | 102
 bool mm_q4_takes(const GemvArgs & a) {
-    if (a.ncols < 2816 || a.masks_out) return false;
+    if (a.ncols < 2816) return false;
     const int T = a.T > 256 ? 256 : a.T;
     if (a.masks) return T > 96;
     if (T > 192) return a.nrows <= sm_count() / 2 * TS_N || a.nrows > sm_count() * 96;
@@ -515,7 +512,6 @@ int launch_mm_q4(const GemvArgs & a, cudaStream_t st) {
         p.bias = a.bias; p.relu = a.relu;
         p.dst = a.dst ? a.dst + (size_t)t0 * a.dst_stride : nullptr;
         p.dst16 = a.dst16 ? a.dst16 + (size_t)t0 * a.dst_stride : nullptr; p.dst_stride = a.dst_stride;
-        p.coef = a.coef ? a.coef + (size_t)t0 * a.coef_stride : nullptr; p.coef_stride = a.coef_stride;
         p.status = a.status;
         int rc;
         if ((rc = tensor_map(&p.m_lo, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.x.lo, (int64_t)p.nb * 16, p.T, (int64_t)p.nb * 16, 64, TS_TOK, CU_TENSOR_MAP_SWIZZLE_64B)) != PI_OK) return rc;

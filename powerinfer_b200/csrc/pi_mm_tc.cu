@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) k_mm_tc(const __grid_constant__
         __syncwarp();
     } else if (warp == 1) {
         // ================================================================= products
-        const uint32_t idesc = tc_idesc(N, false, false);
+        const uint32_t idesc = tc_idesc(N, false);
         int slot = 0, buf = 0;
         unsigned phase = 0u, dphase = 1u;                             // (the first tiles' buffers are free)
         bool ok = true;

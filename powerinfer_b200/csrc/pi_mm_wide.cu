@@ -37,8 +37,6 @@ struct alignas(64) MwP {
     const float * idx; int64_t idx_stride; float threshold;
     const float * bias; int relu;
     float * dst; __half * dst16; int64_t dst_stride;
-    __half * coef; int64_t coef_stride;
-    uint32_t * masks_out; float masks_threshold; int masks_or;
     unsigned int * status;
     int n_slices, S;                                    // column slices of a row; stages
 };
@@ -79,8 +77,7 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     __shared__ int s_warp[MW_THREADS / 32];
-    __shared__ unsigned s_any[8];
-    __shared__ uint64_t s_full[MW_SMAX], s_empty[MW_SMAX], s_bits[2];
+    __shared__ uint64_t s_full[MW_SMAX], s_empty[MW_SMAX];
     __shared__ volatile int s_dead;
     int * rows = reinterpret_cast<int *>(smem + (size_t)p.S * Z::STAGE);          // rows of this CTA (sparse only)
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);    // (a shuffle: uniform for the compiler too; a branch it takes for divergent costs every mma behind it)
@@ -88,9 +85,8 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
     const int G = gridDim.x, cta = blockIdx.x, S = p.S;
     const uint32_t ring = smem_u32(smem);
     constexpr uint32_t x_off = Z::X_OFF, s_off = Z::S_OFF, d_off = Z::D_OFF;
-    if (tid < 8) s_any[tid] = 0u;
     if (tid < MW_SMAX) { mbar_init(s_full + tid, MW_PROD + 1); mbar_init(s_empty + tid, MW_CONS); }
-    if (tid == 0) { mbar_init(s_bits, MW_CONS); mbar_init(s_bits + 1, MW_CONS); s_dead = 0; }
+    if (tid == 0) s_dead = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncthreads();
     pdl_launch();
@@ -104,10 +100,8 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
 
     int lo = 0, hi = 0, n_units = 0;
     auto set_range = [&](int n) {
-        const int al = !SPARSE && p.masks_out ? 8 : 1;                // (a byte of the masks has one writer)
-        const int gr = (n + al - 1) / al;
-        lo = min(n, (int)((long long)gr * cta / G) * al);
-        hi = min(n, (int)((long long)gr * (cta + 1) / G) * al);
+        lo = (int)((long long)n * cta / G);
+        hi = (int)((long long)n * (cta + 1) / G);
         n_units = (hi - lo + IT - 1) / IT * p.n_slices;
     };
     // ---- copies: a thread's pieces of a stage lie in the same rows for a whole tile
@@ -335,7 +329,6 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
 #pragma unroll
                     for (int h = 0; h < (GATED ? 1 : 2); h++) {
                         const int k = GATED ? (row0 + m * MS) / 2 + g : row0 + m * MS + g + h * 8;     // item of the tile
-                        bool any = false;
                         if (k < n_tile) {
                             const int item = lo + tile * IT + k;
                             const int r = SPARSE ? rows[tile * IT + k] : item;
@@ -350,36 +343,18 @@ __global__ void __launch_bounds__(MW_THREADS, 1) k_mm_wide(const __grid_constant
                                     const float v[2] = {acc[m][n][j], acc[m][n][2 + j]};
                                     float o = GATED ? fmaxf(v[1], 0.f) * v[0] : v[h];
                                     const bool off = SPARSE && p.idx[(size_t)t * p.idx_stride + gid] < p.threshold;   // (a NaN logit counts as active)
-                                    if (off && p.coef) { p.coef[(size_t)t * p.coef_stride + item] = __ushort_as_half((unsigned short)0); continue; }
                                     if (off) o = 0.f;
                                     if (p.bias) o += bias;
                                     if (p.relu) o = fmaxf(o, 0.f);
                                     if (p.dst)   p.dst[(size_t)t * p.dst_stride + gid] = o;
                                     if (p.dst16) p.dst16[(size_t)t * p.dst_stride + gid] = __float2half_rn(o);
-                                    if (p.coef)  p.coef[(size_t)t * p.coef_stride + item] = __float2half_rn(o);
-                                    any |= !(o < p.masks_threshold);
                                 }
                             }
                         }
-                        if (!SPARSE && p.masks_out && any) atomicOr(&s_any[k / 32], 1u << (k % 32));
                     }
                 }
             }
-            if (!SPARSE && p.masks_out) {                             // the union over the tokens of !(result < threshold), one bit per row
-                __syncwarp();
-                if (lane == 0) mbar_arrive(s_bits);
-                if (!wait(s_bits, (unsigned)tile & 1u)) break;
-                if (tid < TM / 8 && tid * 8 < n_tile) {               // the range starts at a multiple of 8 rows
-                    unsigned char * o = reinterpret_cast<unsigned char *>(p.masks_out) + (lo + tile * IT) / 8 + tid;
-                    const unsigned char bits = (unsigned char)(s_any[tid / 4] >> (tid % 4 * 8));
-                    *o = p.masks_or ? (unsigned char)(*o | bits) : bits;
-                }
-                __syncwarp();
-                if (tid < 8) s_any[tid] = 0u;
-                __syncwarp();
-                if (lane == 0) mbar_arrive(s_bits + 1);
-                if (!wait(s_bits + 1, (unsigned)tile & 1u)) break;
-            }
+            __syncwarp();                                             // (keeps the compiler from folding what follows into the loop: 9000 x 4096, 128 tokens 65 us, so 50)
             clear();
         }
         if (++slice == p.n_slices) { slice = 0; tile++; }
@@ -419,10 +394,9 @@ static int mw_go(MwP p, bool pdl, cudaStream_t st) {
     static_assert(2 * Z::STAGE <= MW_SMEM_MAX - 1024 - 8192, "two stages");
     p.per_tile = 0;
     int rc;
-    if (!SPARSE) {                                                    // equal tiles; whole bytes of the masks
-        const int share = (p.nrows + G - 1) / G + (p.masks_out ? 8 : 0), tiles = (share + Z::TM - 1) / Z::TM;
-        p.per_tile = p.masks_out ? (share / tiles + 8) / 8 * 8 : (share + tiles - 1) / tiles;
-        if (p.per_tile > Z::TM) p.per_tile = Z::TM;
+    if (!SPARSE) {                                                    // equal tiles
+        const int share = (p.nrows + G - 1) / G, tiles = (share + Z::TM - 1) / Z::TM;
+        p.per_tile = (share + tiles - 1) / tiles;
         rc = tensor_map(&p.m_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.W, (int64_t)p.nb * 16, p.nrows, p.row_bytes, 64, p.per_tile, CU_TENSOR_MAP_SWIZZLE_64B);
         if (rc != PI_OK) return rc;
     }
@@ -473,8 +447,7 @@ int launch_mm_wide(const GemvArgs & a, cudaStream_t st) {
         p.bias = a.bias; p.relu = a.relu;
         p.dst = a.dst ? a.dst + (size_t)t0 * a.dst_stride : nullptr;
         p.dst16 = a.dst16 ? a.dst16 + (size_t)t0 * a.dst_stride : nullptr; p.dst_stride = a.dst_stride;
-        p.coef = a.coef ? a.coef + (size_t)t0 * a.coef_stride : nullptr; p.coef_stride = a.coef_stride;
-        p.masks_out = a.masks_out; p.masks_threshold = a.masks_threshold; p.masks_or = t0 > 0; p.status = a.status;
+        p.status = a.status;
         const int rc = mw_tokens(p, a.pdl, st);
         if (rc != PI_OK) return rc;
     }

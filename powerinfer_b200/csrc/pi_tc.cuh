@@ -47,9 +47,9 @@ __device__ __forceinline__ void tc_mma_f16_ta(uint32_t d, uint32_t a, uint64_t b
 __device__ __forceinline__ void tc_commit(uint64_t * bar) {
     asm volatile("{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n @e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" :: "r"(smem_u32(bar)) : "memory");
 }
-// instruction descriptor: 128 x n, halves (or BF16), FP32 sums; b_mn: B lies with its columns, not K, contiguous
-__host__ __device__ constexpr uint32_t tc_idesc(int n, bool b_mn, bool bf16) {
-    return (1u << 4) | (bf16 ? 1u << 7 | 1u << 10 : 0u) | (b_mn ? 1u << 16 : 0u) | ((uint32_t)(n >> 3) << 17) | (8u << 24);
+// instruction descriptor: 128 x n, halves, FP32 sums; b_mn: B lies with its columns, not K, contiguous
+__host__ __device__ constexpr uint32_t tc_idesc(int n, bool b_mn) {
+    return (1u << 4) | (b_mn ? 1u << 16 : 0u) | ((uint32_t)(n >> 3) << 17) | (8u << 24);
 }
 // Operands in 128-byte rows whose 16-byte pieces are permuted by the row's number in groups of 8 (piece ^ row: the 128-byte swizzle), from
 // 1024-byte boundaries.  K-major: a row is 64 values of K; a step of 16 in K is 32 bytes on.  MN-major: a row is 64 values of M or N at
