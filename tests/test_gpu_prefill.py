@@ -143,12 +143,17 @@ def test_prompt_with_rounded_factors(engine_mod):
                                                      n_ctx=256, firing=0.5, seed=9), (40, 48, 90, 130))
 
 
-@pytest.mark.parametrize("heads,kv,n_ctx", [(4, 4, 2048), (8, 2, 2304), (4, 2, 4096), (4, 4, 2880), (4, 4, 2881), (8, 2, 3136), (8, 2, 3137)])
+@pytest.mark.parametrize("heads,kv,n_ctx", [(4, 4, 2048), (8, 2, 2304), (4, 2, 4096)])
 def test_prompt_in_a_long_context(engine_mod, heads, kv, n_ctx):
     """Contexts beyond 1920 positions (heads of 64: 2112): chunks of 32 tokens and more with 24 CTAs and more (here 40 tokens of 8 heads, and 256) take the
     several-token attention up to 2880 (3136), all others and the longer contexts a store pass, then one CTA per head and token."""
     against_single_steps(engine_mod, synth.ModelSpec(arch=synth.ARCH_LLAMA, wtype=synth.F16, n_layer=2, d=512, n_ff=1024, n_head=heads, n_head_kv=kv, rank=64, n_vocab=256,
                                                      n_ctx=n_ctx, firing=0.2, seed=7), (2, 40, 300))
+
+
+@pytest.mark.parametrize("heads,kv,n_ctx", [(4, 4, 2880), (4, 4, 2881), (8, 2, 3136), (8, 2, 3137)])
+def test_prompt_in_a_context_at_the_line(engine_mod, heads, kv, n_ctx):
+    test_prompt_in_a_long_context(engine_mod, heads, kv, n_ctx)
 
 
 @pytest.mark.parametrize("wtype", [synth.F16, synth.Q4_0])

@@ -27,10 +27,9 @@ def close(got, x, w, terms):
 
 
 # 38040 rows: two tiles of rows per CTA; 1184 rows: 8 per CTA; 8, 24, 520, 1032 columns: parts of a slice, of a stage of several slices.  2048 columns and
-# more, up to 5280 rows: four CTAs share the columns (33, 34 or 65 slices), clusters without rows, the line itself; rows of two and three slices, all in one stage
+# more, up to 5280 rows: four CTAs share the columns (33, 34 or 65 slices), clusters without rows, the line itself
 @pytest.mark.parametrize("T", [33, 128, 129, 261])
-@pytest.mark.parametrize("rows,cols", [(8, 8), (1184, 1032), (3001, 520), (38040, 64), (8, 2048), (1001, 2120), (5120, 2056), (5290, 2048), (2100, 4104),
-                                       (700, 136), (9001, 192), (300, 72)])
+@pytest.mark.parametrize("rows,cols", [(8, 8), (1184, 1032), (3001, 520), (38040, 64), (8, 2048), (1001, 2120), (5120, 2056), (5290, 2048), (2100, 4104)])
 def test_dense_products(ops, rows, cols, T):
     gen = generator(rows + T)
     W, x = weight(ops, synth.F16, rows, cols, gen), torch.randn(T, cols, device="cuda", generator=gen)
@@ -99,9 +98,8 @@ def close_q4(got, x, w, keep=None):
     assert err.norm() <= 4e-7 * ref.norm() + 1e-30
 
 
-# 9.. rows per CTA, tiles of 16, 96, 160 rows and several of them, sizes around every line of mm_q4_takes (below 2816 columns: k_mm_wide), a second launch
-@pytest.mark.parametrize("rows,cols,T", [(8, 2048, 193), (1000, 2304, 256), (2370, 4352, 200), (10000, 2048, 97), (24000, 2048, 128), (12100, 2048, 256), (5000, 2048, 261),
-                                         (8, 2816, 193), (1000, 3072, 256), (10000, 2816, 97), (24000, 2816, 128), (12100, 3072, 256), (5000, 2816, 261), (5000, 2560, 200)])
+# 9.. rows per CTA, tiles of 16, 96, 160 rows and several of them, sizes around every line of mm_q4_takes, a second launch
+@pytest.mark.parametrize("rows,cols,T", [(8, 2048, 193), (1000, 2304, 256), (2370, 4352, 200), (10000, 2048, 97), (24000, 2048, 128), (12100, 2048, 256), (5000, 2048, 261)])
 def test_q4_products(ops, rows, cols, T):
     gen = generator(rows + T)
     W, x = weight(ops, synth.Q4_0, rows, cols, gen), torch.randn(T, cols, device="cuda", generator=gen) * torch.exp(torch.randn(1, cols, device="cuda", generator=gen))
@@ -113,8 +111,7 @@ def test_q4_products(ops, rows, cols, T):
 
 
 @pytest.mark.parametrize("share", [0.0, 0.004, 0.6, 1.0])
-@pytest.mark.parametrize("rows,cols,T", [(640, 2048, 97), (5000, 2304, 128), (24000, 2048, 129), (3001, 4096, 256),
-                                         (640, 2816, 97), (5000, 3072, 128), (24000, 2816, 129)])
+@pytest.mark.parametrize("rows,cols,T", [(640, 2048, 97), (5000, 2304, 128), (24000, 2048, 129), (3001, 4096, 256)])
 def test_q4_gathers(ops, rows, cols, T, share):
     gen = generator(rows + T)
     up, gate = weight(ops, synth.Q4_0, rows, cols, gen), weight(ops, synth.Q4_0, rows, cols, gen)
@@ -130,10 +127,9 @@ def test_q4_gathers(ops, rows, cols, T, share):
     assert ops.last_op_status() == 0
 
 
-@pytest.mark.parametrize("cols", [2048, 3072])
-def test_q4_tokens_above_the_halves_range(ops, cols):
+def test_q4_tokens_above_the_halves_range(ops):
     """Blocks of a token whose scale times 127 is above 65504, beside tokens and blocks with small ones."""
-    rows, T = 1000, 200
+    rows, cols, T = 1000, 2048, 200
     gen = generator(3)
     W, x = weight(ops, synth.Q4_0, rows, cols, gen), torch.randn(T, cols, device="cuda", generator=gen)
     x[3] *= 3e4
@@ -143,25 +139,9 @@ def test_q4_tokens_above_the_halves_range(ops, cols):
     close_q4(ops.ggml_mul_mat(W, x), rounded(ops, synth.Q4_0, x), ops.dequantize(W).double())
 
 
-@pytest.mark.parametrize("rows,T", [(1000, 200), (12100, 128)])
-def test_q4_blocks_beside_one_above_the_halves_range(ops, rows, T):
-    """Scales around 0.0002 beside scales of up to 30000 in blocks where a row's weights are 0: the result is that of the small ones alone."""
-    cols, gen = 3072, generator(rows)
-    raw = torch.from_numpy(synth.quantize_q4_0((torch.randn(rows, cols, device="cuda", generator=gen) * 0.05).cpu().numpy()).reshape(rows, cols // 32, 18).copy())
-    raw[:, ::2, 2:] = 0x88
-    W = ops.upload_weight(raw.reshape(-1).numpy(), synth.Q4_0, rows, cols)
-    x = torch.randn(T, cols, device="cuda", generator=gen) * 0.01
-    x.view(T, -1, 2, 32)[::3, :, 0] *= 10.0 ** (3 + 5 * torch.rand((T + 2) // 3, cols // 64, 1, device="cuda", generator=gen))
-    close_q4(ops.ggml_mul_mat(W, x), rounded(ops, synth.Q4_0, x), ops.dequantize(W).double())
-    idx = torch.where(torch.rand(T, rows, device="cuda", generator=gen) < 0.7, 1.0, -1.0)
-    close_q4(ops.ggml_mul_mat_idx(W, x, idx), rounded(ops, synth.Q4_0, x), ops.dequantize(W).double(), idx >= 0)
-    assert ops.last_op_status() == 0
-
-
-@pytest.mark.parametrize("cols", [2048, 3072])
-def test_q4_rows_above_the_halves_range(ops, cols):
+def test_q4_rows_above_the_halves_range(ops):
     """Rows with weights above 65504, single blocks of them among others, in a dense product and a gather with gate."""
-    rows, T = 1024, 200
+    rows, cols, T = 1024, 2048, 200
     gen = generator(4)
     w = torch.randn(rows, cols, device="cuda", generator=gen) * 0.05
     w[5] *= 2e6
@@ -178,6 +158,21 @@ def test_q4_rows_above_the_halves_range(ops, cols):
     got = ops.ggml_mul_mat_idx(W, x, idx)
     y = ops.ggml_axpy(down, torch.relu(got) * got, idx)
     assert y.isfinite().all() and torch.equal(ops.sparse_ffn(W, W, down, x, idx), y)
+    assert ops.last_op_status() == 0
+
+
+@pytest.mark.parametrize("rows,T", [(1000, 200), (12100, 128)])
+def test_q4_blocks_beside_one_above_the_halves_range(ops, rows, T):
+    """Scales around 0.0002 beside scales of up to 30000 in blocks where a row's weights are 0: the result is that of the small ones alone."""
+    cols, gen = 3072, generator(rows)
+    raw = torch.from_numpy(synth.quantize_q4_0((torch.randn(rows, cols, device="cuda", generator=gen) * 0.05).cpu().numpy()).reshape(rows, cols // 32, 18).copy())
+    raw[:, ::2, 2:] = 0x88
+    W = ops.upload_weight(raw.reshape(-1).numpy(), synth.Q4_0, rows, cols)
+    x = torch.randn(T, cols, device="cuda", generator=gen) * 0.01
+    x.view(T, -1, 2, 32)[::3, :, 0] *= 10.0 ** (3 + 5 * torch.rand((T + 2) // 3, cols // 64, 1, device="cuda", generator=gen))
+    close_q4(ops.ggml_mul_mat(W, x), rounded(ops, synth.Q4_0, x), ops.dequantize(W).double())
+    idx = torch.where(torch.rand(T, rows, device="cuda", generator=gen) < 0.7, 1.0, -1.0)
+    close_q4(ops.ggml_mul_mat_idx(W, x, idx), rounded(ops, synth.Q4_0, x), ops.dequantize(W).double(), idx >= 0)
     assert ops.last_op_status() == 0
 
 
@@ -248,3 +243,90 @@ def test_q4_products_around_one_tile_a_cta(ops, share, more):
     W, x = weight(ops, synth.Q4_0, rows, cols, gen), torch.randn(T, cols, device="cuda", generator=gen)
     close_q4(ops.ggml_mul_mat(W, x), rounded(ops, synth.Q4_0, x), ops.dequantize(W).double())
     assert ops.last_op_status() == 0
+
+
+# ---- the same at sizes that take other paths today.  Short rows: two and three slices, all in one stage
+@pytest.mark.parametrize("T", [33, 128, 129, 261])
+@pytest.mark.parametrize("rows,cols", [(700, 136), (9001, 192), (300, 72)])
+def test_dense_products_of_short_rows(ops, rows, cols, T):
+    test_dense_products(ops, rows, cols, T)
+
+
+# (below 2816 columns: k_mm_wide)
+@pytest.mark.parametrize("rows,cols,T", [(8, 2816, 193), (1000, 3072, 256), (10000, 2816, 97), (24000, 2816, 128), (12100, 3072, 256), (5000, 2816, 261), (5000, 2560, 200)])
+def test_q4_products_of_2816_columns_and_more(ops, rows, cols, T):
+    test_q4_products(ops, rows, cols, T)
+
+
+@pytest.mark.parametrize("share", [0.0, 0.004, 0.6, 1.0])
+@pytest.mark.parametrize("rows,cols,T", [(640, 2816, 97), (5000, 3072, 128), (24000, 2816, 129)])
+def test_q4_gathers_of_2816_columns_and_more(ops, rows, cols, T, share):
+    test_q4_gathers(ops, rows, cols, T, share)
+
+
+def test_wide_q4_tokens_above_the_halves_range(ops):
+    """test_q4_tokens_above_the_halves_range at a width of k_mm_q4."""
+    rows, cols, T = 1000, 3072, 200
+    gen = generator(3)
+    W, x = weight(ops, synth.Q4_0, rows, cols, gen), torch.randn(T, cols, device="cuda", generator=gen)
+    x[3] *= 3e4
+    x[70, 64:96] *= 1e6
+    x[71, ::3] *= 1e-4
+    x[199] *= 2e6
+    close_q4(ops.ggml_mul_mat(W, x), rounded(ops, synth.Q4_0, x), ops.dequantize(W).double())
+
+
+@pytest.mark.parametrize("T", [97, 200])
+def test_wide_q4_rows_above_the_halves_range(ops, T):
+    """test_q4_rows_above_the_halves_range at a width of k_mm_q4; the FFN with gate, and without it but with a bias: the sums of such rows, made anew,
+    take the same epilogue."""
+    rows, cols = 1024, 3072
+    gen = generator(4)
+    w = torch.randn(rows, cols, device="cuda", generator=gen) * 0.05
+    w[5] *= 2e6
+    w[700, 320:352] *= 2e6
+    w[1023, ::7] *= 1.5e6
+    W = ops.upload_weight(synth.quantize_q4_0(w.cpu().numpy()), synth.Q4_0, rows, cols)
+    x, wd = torch.randn(T, cols, device="cuda", generator=gen), ops.dequantize(W).double()
+    assert (wd.abs() > 65504).any(1).sum() == 3 and wd.isfinite().all()
+    close_q4(ops.ggml_mul_mat(W, x), rounded(ops, synth.Q4_0, x), wd)
+    idx = torch.where(torch.rand(T, rows, device="cuda", generator=gen) < 0.7, 1.0, -1.0)
+    idx[:, 64:200] = -1.0                                             # active for no token
+    close_q4(ops.ggml_mul_mat_idx(W, x, idx), rounded(ops, synth.Q4_0, x), wd, idx >= 0)
+    x, down = x * 0.0001, weight(ops, synth.Q4_0, rows, cols, gen)       # (hidden values within the range of Q8_0's scales; up and gate the same rows)
+    got = ops.ggml_mul_mat_idx(W, x, idx)
+    close_q4(got, rounded(ops, synth.Q4_0, x), wd, idx >= 0)
+    y = ops.ggml_axpy(down, torch.relu(got) * got, idx)
+    assert y.isfinite().all() and torch.equal(ops.sparse_ffn(W, W, down, x, idx), y)
+    bias = torch.randn(rows, device="cuda", generator=gen)
+    y = ops.ggml_axpy(down, torch.relu(got + bias), idx)
+    assert y.isfinite().all() and torch.equal(ops.sparse_ffn(W, None, down, x, idx, up_bias=bias), y)
+    assert ops.last_op_status() == 0
+
+
+def within_steps(got, ref, terms):
+    """The error of a whole result, as a 2-norm: the tensor cores cut a sum at every step of 16 terms, each time by at most 2^-23 of what it holds
+    then, which in the mean over the results is no more than the result itself; 20 more for partial sums added in FP32.  (Partial sums passed on
+    in FP16 would be 2^-13 of the results off, four to a hundred times this.)"""
+    assert (got.double() - ref).norm() <= (terms / 16 + 20) * 2.0 ** -23 * ref.norm()
+
+
+# one chain, two tiles, chains in a cluster of four (2048 columns and more)
+@pytest.mark.parametrize("rows,cols,T", [(300, 72, 33), (38040, 64, 128), (1184, 1032, 77), (1001, 2120, 261), (5290, 2048, 128), (2100, 4104, 77), (512, 4096, 256)])
+def test_dense_products_keep_fp32_sums(ops, rows, cols, T):
+    gen = generator(rows + T)
+    W, x = weight(ops, synth.F16, rows, cols, gen), torch.randn(T, cols, device="cuda", generator=gen)
+    within_steps(ops.ggml_mul_mat(W, x), x.half().double() @ ops.dequantize(W).double().T, cols)
+    idx = torch.where(torch.rand(T, rows, device="cuda", generator=gen) < 0.6, 1.0, -1.0)
+    within_steps(ops.ggml_mul_mat_idx(W, x, idx), (x.half().double() @ ops.dequantize(W).double().T) * (idx >= 0), cols)
+
+
+# one accumulator and several, list ranges of one stage and of many
+@pytest.mark.parametrize("share", [0.05, 0.7])
+@pytest.mark.parametrize("rows,cols,T", [(1500, 3072, 77), (3001, 2056, 129), (900, 520, 256), (5000, 4096, 256)])
+def test_axpy_of_many_tokens_keeps_fp32_sums(ops, rows, cols, T, share):
+    gen = generator(rows + T)
+    W = weight(ops, synth.F16, rows, cols, gen)
+    idx = torch.where((torch.rand(1, rows, device="cuda", generator=gen) < share) & (torch.rand(T, rows, device="cuda", generator=gen) < 0.7), 1.0, -1.0)
+    h = torch.randn(T, rows, device="cuda", generator=gen)
+    within_steps(ops.ggml_axpy(W, h, idx), (h.half().double() * (idx >= 0)) @ ops.dequantize(W).double(), rows * share)
