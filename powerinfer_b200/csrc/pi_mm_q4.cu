@@ -1,5 +1,5 @@
 // Mat-mat over planar Q4_0 rows of many columns for MORE than 96 tokens (prompt chunks; the lines: mm_q4_takes) on tcgen05: the operators, row
-// selection and epilogue of pi_mm.cu.
+// selection and results of pi_mm.cu (masks and coefficients are FP16 rows' alone).
 //
 // A term is (q - 8) * w * v * d: an integer and an FP16 scale of the row's block, an int8 and an FP16 scale of the token's block.  (q - 8) * w has 15
 // significant bits, v * d 18, and both are multiples of 2^-24: each is exactly the sum of TWO halves, its rounding and the rest.  Of

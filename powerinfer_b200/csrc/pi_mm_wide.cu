@@ -1,5 +1,5 @@
-// Mat-mat over planar Q4_0 rows for MORE than 32 tokens (prompt chunks of up to 256): the same operators, row selection and epilogue as
-// pi_mm.cu, another split of the work.  (FP16 rows: pi_mm_tc.cu.)
+// Mat-mat over planar Q4_0 rows for MORE than 32 tokens (prompt chunks of up to 256): the same operators, row selection and results as
+// pi_mm.cu (masks and coefficients are FP16 rows' alone), another split of the work.  (FP16 rows: pi_mm_tc.cu.)
 //
 // Bound: the scaling of the Q4_0 blocks.  An mma of 16 rows x 32 columns x 8 tokens takes 8 clocks of a scheduler, the eight fused
 // multiply-adds that apply its scales another 8 (as four packed ones they were slower, 259 us where these take 208: packed operations
